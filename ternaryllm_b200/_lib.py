@@ -110,6 +110,24 @@ def lib():
     return _lib
 
 
+_binding = None
+
+
+def binding():
+    """The CPython extension that carries the per-call path (csrc/binding.cpp); like the library, it has no fallback."""
+    global _binding
+    if _binding is None:
+        lib()                                # the library first: the extension resolves its symbols from the same copy
+        path = os.path.join(HERE, "_binding.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -m ternaryllm_b200.build`")
+        import torch  # noqa: F401  (the extension links torch's libraries)
+        from . import _binding as b
+
+        _binding = b
+    return _binding
+
+
 def check(rc: int, what: str = "libtllm"):
     if rc != 0:
         msg = lib().tllm_last_error()

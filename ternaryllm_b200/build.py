@@ -1,8 +1,9 @@
-"""Build libtllm.so (the C-ABI shared library) in-tree with nvcc for sm_100a.
+"""Build libtllm.so (the C-ABI shared library) in-tree with nvcc for sm_100a, and `_binding.so` (the CPython extension that
+calls it from torch tensors) with g++.
 
     python -m ternaryllm_b200.build [--force] [--verbose]
 
-The library has no dependency on torch; the Python modules of this package bind it with ctypes.
+The library has no dependency on torch; the extension has, and links the library from its own folder.
 """
 from __future__ import annotations
 
@@ -20,30 +21,54 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC,-O2", "--shared", "-Xptxas", "-v",
 ]
 
+BINDING = os.path.join(HERE, "_binding.so")
+BINDING_DEPS = ["binding.cpp", os.path.join("..", "..", "include", "tllm.h")]
 
-def _stale() -> bool:
-    if not os.path.exists(LIB):
+
+def _stale(target: str, deps) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in SOURCES + DEPS)
+    t = os.path.getmtime(target)
+    return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in deps)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not _stale():
-        return LIB
-    nvcc = os.environ.get("NVCC", "nvcc")
-    cmd = [nvcc] + NVCC_FLAGS + [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB]
+def _run(cmd, verbose: bool, log_mode: str) -> None:
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     log = os.path.join(HERE, "build.log")
-    with open(log, "w") as f:
+    with open(log, log_mode) as f:
         f.write(" ".join(cmd) + "\n" + r.stdout)
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
-        raise RuntimeError("nvcc failed; see " + log)
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed; see " + log)
     if verbose:
         print(r.stdout)
+
+
+def build_binding(force: bool = False, verbose: bool = False) -> str:
+    if not force and not _stale(BINDING, BINDING_DEPS):
+        return BINDING
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+           os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           os.path.join(CSRC, "binding.cpp")] + ["-I" + i for i in inc] + \
+        ["-L" + HERE, "-l:libtllm.so", "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+         "-Wl,-rpath,$ORIGIN", "-o", BINDING]
+    _run(cmd, verbose, "a")
+    return BINDING
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    if force or _stale(LIB, SOURCES + DEPS):
+        nvcc = os.environ.get("NVCC", "nvcc")
+        _run([nvcc] + NVCC_FLAGS + [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB], verbose, "w")
+    build_binding(force, verbose)
     return LIB
 
 

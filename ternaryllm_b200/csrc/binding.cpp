@@ -1,0 +1,257 @@
+// binding.cpp -- the per-call half of the Python package as a CPython extension (module `_binding`): tensor checks, result
+// allocation, stream lookup and the call into libtllm.so (include/tllm.h), without a Python-level attribute walk or a
+// ctypes argument conversion per call.
+//
+// A decode product runs 3 to 10 us on the GPU; the same call through ctypes took 16 us of host time (info struct to dict,
+// device context manager, stream object, torch.empty, nine converted arguments), so a decode loop that is not captured in
+// a graph was bound by the host.  Here a call costs the checks (tens of ns), one allocation from torch's caching
+// allocator and the launch.  Only host plumbing lives here; kernels, dispatch and handles are libtllm's.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
+
+#include "../../include/tllm.h"
+
+namespace {
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kFloat: return TLLM_F32;
+        case at::kHalf: return TLLM_F16;
+        case at::kBFloat16: return TLLM_BF16;
+        case at::kChar: return TLLM_I8;
+        case at::kInt: return TLLM_I32;
+        default: return -1;
+    }
+}
+
+PyObject* raise(const std::string& msg) {
+    PyErr_SetString(PyExc_RuntimeError, msg.c_str());
+    return nullptr;
+}
+
+PyObject* raise_rc(const char* what, int rc) {
+    const char* m = tllm_last_error();
+    return raise(std::string(what) + ": " + (m && *m ? m : "error") + " (code " + std::to_string(rc) + ")");
+}
+
+const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+bool int_of(PyObject* o, long long* v) {
+    *v = PyLong_AsLongLong(o);
+    return !(*v == -1 && PyErr_Occurred());
+}
+
+// makes `device` current for the scope of a call; nothing when it already is
+struct DeviceScope {
+    c10::cuda::OptionalCUDAGuard g;
+    explicit DeviceScope(c10::DeviceIndex device) {
+        if (c10::cuda::current_device() != device) g.set_index(device);
+    }
+};
+
+std::string shape_text(const at::Tensor& t) {
+    std::string s = "torch.Size([";
+    for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+    return s + "])";
+}
+
+#define NEED_ARGS(n, who)                                                        \
+    if (nargs != (n)) {                                                           \
+        PyErr_SetString(PyExc_TypeError, who ": wrong number of arguments");      \
+        return nullptr;                                                           \
+    }
+// C++ exceptions (allocation failure, bad stream) become Python errors
+#define BINDING_TRY try {
+#define BINDING_CATCH                  \
+    }                                  \
+    catch (const std::exception& e) {  \
+        return raise(e.what());        \
+    }
+
+// matmul(handle, x, out | None, col_major, device, inners, columns) -> tensor
+PyObject* matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    NEED_ARGS(7, "matmul")
+    BINDING_TRY
+    long long handle, device, inners, columns;
+    if (!int_of(a[0], &handle) || !int_of(a[4], &device) || !int_of(a[5], &inners) || !int_of(a[6], &columns)) return nullptr;
+    const at::Tensor* xp = tensor_of(a[1]);
+    if (!xp) return raise("matmul expects a tensor");
+    const int col_major = PyObject_IsTrue(a[3]);
+    if (col_major < 0) return nullptr;
+    if (!xp->is_cuda() || xp->get_device() != device) return raise("activation must be on the CUDA device that holds the packed weight");
+    if (xp->dim() != 2) return raise("matmul expects a 2-D activation");
+    at::Tensor xc;
+    if (!xp->is_contiguous()) xc = xp->contiguous(), xp = &xc;
+    const int64_t rows = xp->size(col_major ? 1 : 0);
+    if (xp->size(col_major ? 0 : 1) != inners) return raise("activation has " + shape_text(*xp) + " but the weight has " + std::to_string(inners) + " inners");
+    if (rows > INT32_MAX) return raise("matmul: too many rows");
+    const at::ScalarType xt = xp->scalar_type(), yt = xt == at::kChar ? at::kInt : xt;
+    const int xcode = dtype_code(xt);
+    if (xcode < 0) {
+        PyErr_SetString(PyExc_KeyError, c10::toString(xt));
+        return nullptr;
+    }
+    DeviceScope scope((c10::DeviceIndex)device);
+    at::Tensor y;
+    if (a[2] == Py_None) {
+        y = at::empty({rows, columns}, xp->options().dtype(yt));
+    } else {
+        const at::Tensor* op = tensor_of(a[2]);
+        if (!op) return raise("out must be a tensor");
+        const at::ScalarType ot = op->scalar_type();
+        if ((ot != yt && !(ot == at::kFloat && yt != at::kInt)) || op->dim() != 2 || op->size(0) != rows || op->size(1) != columns || !op->is_contiguous())
+            return raise("out has the wrong dtype, shape or strides");
+        y = *op;
+    }
+    void* st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    const void* X = xp->const_data_ptr();
+    void* Y = y.data_ptr();
+    const int ycode = dtype_code(y.scalar_type());
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = tllm_spmm((tllm_weight*)handle, X, xcode, col_major ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR, (int)rows, Y, ycode, st);
+    Py_END_ALLOW_THREADS
+    if (rc) return raise_rc("tllm_spmm", rc);
+    if (a[2] != Py_None) {
+        Py_INCREF(a[2]);
+        return a[2];
+    }
+    return THPVariable_Wrap(std::move(y));
+    BINDING_CATCH
+}
+
+// mlp_forward(handle, x, out | None, h | None, hidden, inter) -> tensor
+PyObject* mlp_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    NEED_ARGS(6, "mlp_forward")
+    BINDING_TRY
+    long long handle, hidden, inter;
+    if (!int_of(a[0], &handle) || !int_of(a[4], &hidden) || !int_of(a[5], &inter)) return nullptr;
+    const at::Tensor* xp = tensor_of(a[1]);
+    if (!xp || !xp->is_cuda() || xp->dim() != 2 || xp->size(1) != hidden) return raise("PackedMLP.forward expects a 2-D CUDA activation [rows, hidden]");
+    at::Tensor xc;
+    if (!xp->is_contiguous()) xc = xp->contiguous(), xp = &xc;
+    const int64_t rows = xp->size(0);
+    if (rows > INT32_MAX) return raise("PackedMLP.forward: too many rows");
+    const at::ScalarType xt = xp->scalar_type();
+    const int xcode = dtype_code(xt);
+    if (xcode < 0) {
+        PyErr_SetString(PyExc_KeyError, c10::toString(xt));
+        return nullptr;
+    }
+    DeviceScope scope(xp->get_device());
+    at::Tensor y, h;
+    if (a[2] == Py_None) {
+        y = at::empty({rows, hidden}, xp->options());
+    } else {
+        const at::Tensor* op = tensor_of(a[2]);
+        if (!op) return raise("out must be a tensor");
+        if ((op->scalar_type() != xt && op->scalar_type() != at::kFloat) || op->dim() != 2 || op->size(0) != rows || op->size(1) != hidden || !op->is_contiguous())
+            return raise("out has the wrong dtype, shape or strides");
+        y = *op;
+    }
+    if (a[3] != Py_None) {
+        const at::Tensor* hp = tensor_of(a[3]);
+        if (!hp) return raise("h must be a tensor");
+        h = *hp;
+    } else if (rows > 16) {
+        h = at::empty({rows, inter}, xp->options());
+    }
+    void* st = c10::cuda::getCurrentCUDAStream(xp->get_device()).stream();
+    const void* X = xp->const_data_ptr();
+    void *Y = y.data_ptr(), *H = h.defined() ? h.data_ptr() : nullptr;
+    const int ycode = dtype_code(y.scalar_type());
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = tllm_mlp_forward_ex((tllm_mlp*)handle, X, xcode, (int)rows, Y, ycode, H, st);
+    Py_END_ALLOW_THREADS
+    if (rc) return raise_rc("tllm_mlp_forward", rc);
+    if (a[2] != Py_None) {
+        Py_INCREF(a[2]);
+        return a[2];
+    }
+    return THPVariable_Wrap(std::move(y));
+    BINDING_CATCH
+}
+
+// ter_spmm(X, row_idx, col_off, tile_idx | None, batch, rows, columns, inners, uniformed, padded, scale, out | None, tile_k) -> tensor
+PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    NEED_ARGS(13, "ter_spmm")
+    BINDING_TRY
+    const at::Tensor *xp = tensor_of(a[0]), *ip = tensor_of(a[1]), *op = tensor_of(a[2]);
+    long long batch, rows, columns, inners, tile_k;
+    if (!int_of(a[4], &batch) || !int_of(a[5], &rows) || !int_of(a[6], &columns) || !int_of(a[7], &inners) || !int_of(a[12], &tile_k)) return nullptr;
+    const int uniformed = PyObject_IsTrue(a[8]), padded = PyObject_IsTrue(a[9]);
+    const double scale = PyFloat_AsDouble(a[10]);
+    if (uniformed < 0 || padded < 0 || (scale == -1.0 && PyErr_Occurred())) return nullptr;
+    const at::Tensor* three[3] = {xp, ip, op};
+    const char* names[3] = {"X", "row indices", "col offsets"};
+    for (int i = 0; i < 3; ++i)
+        if (!three[i] || !three[i]->is_cuda()) return raise(std::string("ter_spmm: ") + names[i] + " must be a CUDA tensor");
+    if (ip->scalar_type() != at::kShort) return raise("ter_spmm: row indices must be int16");
+    if (op->scalar_type() != at::kInt) return raise("ter_spmm: col offsets must be int32");
+    const at::ScalarType xt = xp->scalar_type(), yt = xt == at::kChar ? at::kInt : xt;
+    if (xt != at::kFloat && xt != at::kHalf && xt != at::kBFloat16 && xt != at::kChar)
+        return raise(std::string("ter_spmm: unsupported activation dtype torch.") + c10::toString(xt));
+    at::Tensor xc;
+    if (!xp->is_contiguous()) xc = xp->contiguous(), xp = &xc;
+    const int64_t d = xp->dim();
+    const int layout = d >= 1 && xp->size(d - 1) == inners ? TLLM_ROW_MAJOR : TLLM_COL_MAJOR;
+    if (layout == TLLM_COL_MAJOR && !(d >= 2 && xp->size(d - 2) == inners))
+        return raise("ter_spmm: activation of shape " + shape_text(*xp) + " has no dimension of " + std::to_string(inners) + " inners");
+    if (batch > 0 && xp->numel() != batch * rows * inners) return raise("ter_spmm: activation size does not match batch_size*rows*inners");
+    if (tile_k <= 0) return raise("ter_spmm: TILE_K must be positive");
+    const int64_t tiles = (inners + tile_k - 1) / tile_k;
+    if (op->numel() != columns * tiles * 4) return raise("ter_spmm: col offsets do not have columns*ceil(inners/TILE_K)*4 entries");
+    DeviceScope scope(xp->get_device());
+    at::Tensor y;
+    if (a[11] == Py_None) {
+        y = at::empty({batch, rows, columns}, xp->options().dtype(yt));
+    } else {
+        const at::Tensor* o = tensor_of(a[11]);
+        if (!o || o->scalar_type() != yt || o->numel() != batch * rows * columns || !o->is_contiguous())
+            return raise("ter_spmm: out has the wrong dtype, size or strides");
+        y = *o;
+    }
+    if (batch != 0) {   // the reference launches nothing for an empty batch (TernaryLinear.py:168)
+        const at::Tensor* tp = tensor_of(a[3]);
+        const int16_t* tile_ptr = tp && tp->numel() ? (const int16_t*)tp->const_data_ptr() : nullptr;
+        void* st = c10::cuda::getCurrentCUDAStream(xp->get_device()).stream();
+        const void* X = xp->const_data_ptr();
+        void* Y = y.data_ptr();
+        const int xcode = dtype_code(xt), ycode = dtype_code(yt);
+        const int16_t* idx = (const int16_t*)ip->const_data_ptr();
+        const int32_t* off = (const int32_t*)op->const_data_ptr();
+        int rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = tllm_ter_spmm(X, xcode, layout, idx, off, tile_ptr, Y, ycode, (int)batch, (int)rows, (int)columns, (int)inners, (int)tile_k, (float)scale,
+                           uniformed, padded, st);
+        Py_END_ALLOW_THREADS
+        if (rc) return raise_rc("ter_spmm", rc);
+    }
+    if (a[11] != Py_None) {
+        Py_INCREF(a[11]);
+        return a[11];
+    }
+    return THPVariable_Wrap(std::move(y));
+    BINDING_CATCH
+}
+
+PyMethodDef methods[] = {
+    {"matmul", (PyCFunction)(void (*)(void))matmul, METH_FASTCALL, "matmul(handle, x, out, col_major, device, inners, columns)"},
+    {"mlp_forward", (PyCFunction)(void (*)(void))mlp_forward, METH_FASTCALL, "mlp_forward(handle, x, out, h, hidden, inter)"},
+    {"ter_spmm", (PyCFunction)(void (*)(void))ter_spmm, METH_FASTCALL,
+     "ter_spmm(X, row_idx, col_off, tile_idx, batch, rows, columns, inners, uniformed, padded, scale, out, tile_k)"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", "per-call path of ternaryllm_b200 (see csrc/binding.cpp)", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__binding(void) { return PyModule_Create(&module); }

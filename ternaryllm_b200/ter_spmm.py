@@ -101,44 +101,15 @@ def ter_spmm(X, w_tiled_merged_row_indice, w_tiled_merged_col_offset, w_col_tile
     tensor is not on a CUDA device or has the wrong dtype, like the reference's TORCH_INTERNAL_ASSERT /
     data_ptr<T>() checks (:326-333).
     """
-    import torch
-
-    for t, name in ((X, "X"), (w_tiled_merged_row_indice, "row indices"), (w_tiled_merged_col_offset, "col offsets")):
-        if t.device.type != "cuda":
-            raise RuntimeError(f"ter_spmm: {name} must be a CUDA tensor")
-    if w_tiled_merged_row_indice.dtype != torch.int16:
-        raise RuntimeError("ter_spmm: row indices must be int16")
-    if w_tiled_merged_col_offset.dtype != torch.int32:
-        raise RuntimeError("ter_spmm: col offsets must be int32")
-    if X.dtype not in (torch.float32, torch.float16, torch.bfloat16, torch.int8):
-        raise RuntimeError(f"ter_spmm: unsupported activation dtype {X.dtype}")
-    X = X.contiguous()
-    y_dtype = torch.int32 if X.dtype == torch.int8 else X.dtype
-    layout = _lib.ROW_MAJOR if X.shape[-1] == inners else _lib.COL_MAJOR
-    if layout == _lib.COL_MAJOR and not (X.dim() >= 2 and X.shape[-2] == inners):
-        raise RuntimeError(f"ter_spmm: activation of shape {tuple(X.shape)} has no dimension of {inners} inners")
-    if X.numel() != max(batch_size, 0) * rows * inners and batch_size > 0:
-        raise RuntimeError("ter_spmm: activation size does not match batch_size*rows*inners")
     if tile_k is None:
         tile_k = tile_size_for(inners)
-    tiles = -(-inners // tile_k)
-    if w_tiled_merged_col_offset.numel() != columns * tiles * 4:
-        raise RuntimeError("ter_spmm: col offsets do not have columns*ceil(inners/TILE_K)*4 entries")
-    if out is None:
-        out = torch.empty((batch_size, rows, columns), device=X.device, dtype=y_dtype)
-    elif out.dtype != y_dtype or out.numel() != batch_size * rows * columns or not out.is_contiguous():
-        raise RuntimeError("ter_spmm: out has the wrong dtype, size or strides")
-    if batch_size == 0:
-        return out                      # the reference launches nothing for an empty batch (TernaryLinear.py:168)
-    tile_ptr = w_col_tile_indices.data_ptr() if w_col_tile_indices is not None and w_col_tile_indices.numel() else None
-    if AUTO_PREPARE and not torch.cuda.is_current_stream_capturing():
-        prepare(w_tiled_merged_row_indice, w_tiled_merged_col_offset, columns, inners, tile_k)
-    with torch.cuda.device(X.device):
-        check(lib().tllm_ter_spmm(X.data_ptr(), _lib.torch_dtype_code(X.dtype), layout, w_tiled_merged_row_indice.data_ptr(),
-                                  w_tiled_merged_col_offset.data_ptr(), tile_ptr, out.data_ptr(), _lib.torch_dtype_code(y_dtype),
-                                  int(batch_size), int(rows), int(columns), int(inners), int(tile_k), float(scale),
-                                  int(bool(uniformed)), int(bool(padded)), torch.cuda.current_stream().cuda_stream), "ter_spmm")
-    return out
+    if AUTO_PREPARE and batch_size != 0 and w_tiled_merged_row_indice.is_cuda and w_tiled_merged_col_offset.is_cuda:
+        import torch
+
+        if not torch.cuda.is_current_stream_capturing():
+            prepare(w_tiled_merged_row_indice, w_tiled_merged_col_offset, columns, inners, tile_k)
+    return _lib.binding().ter_spmm(X, w_tiled_merged_row_indice, w_tiled_merged_col_offset, w_col_tile_indices, batch_size, rows, columns,
+                                   inners, uniformed, padded, scale, out, tile_k)
 
 
 def prepare(w_tiled_merged_row_indice, w_tiled_merged_col_offset, columns, inners, tile_k=None):

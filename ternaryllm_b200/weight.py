@@ -29,6 +29,7 @@ class PackedWeight:
 
     def __init__(self, handle, device_index):
         self._h = handle
+        self._call = None                    # (entry point, handle as an integer, device, inners, columns): made on first use
         self.device_index = device_index
 
     # ---- constructors -------------------------------------------------------------------------------
@@ -108,27 +109,13 @@ class PackedWeight:
 
     def matmul(self, x, out=None, col_major=False):
         """y = x @ W * s for a 2-D CUDA tensor x [rows, inners] (or [inners, rows] with col_major)."""
-        import torch
+        c = self._call or self._bind()
+        return c[0](c[1], x, out, col_major, c[2], c[3], c[4])
 
-        if x.device.type != "cuda" or x.device.index != self.device_index:
-            raise RuntimeError("activation must be on the CUDA device that holds the packed weight")
-        if x.dim() != 2:
-            raise RuntimeError("matmul expects a 2-D activation")
-        x = x.contiguous()
+    def _bind(self):
         info = self.info
-        rows = x.shape[1] if col_major else x.shape[0]
-        if (x.shape[0] if col_major else x.shape[1]) != info["inners"]:
-            raise RuntimeError(f"activation has {x.shape} but the weight has {info['inners']} inners")
-        ydt = torch.int32 if x.dtype == torch.int8 else x.dtype
-        if out is None:
-            out = torch.empty((rows, info["columns"]), device=x.device, dtype=ydt)
-        elif (out.dtype != ydt and not (out.dtype == torch.float32 and ydt != torch.int32)) or \
-                tuple(out.shape) != (rows, info["columns"]) or not out.is_contiguous():
-            raise RuntimeError("out has the wrong dtype, shape or strides")
-        with torch.cuda.device(x.device):
-            check(lib().tllm_spmm(self._h, x.data_ptr(), _lib.torch_dtype_code(x.dtype), _lib.COL_MAJOR if col_major else _lib.ROW_MAJOR,
-                                  rows, out.data_ptr(), _lib.torch_dtype_code(out.dtype), torch.cuda.current_stream().cuda_stream), "tllm_spmm")
-        return out
+        self._call = (_lib.binding().matmul, self._h.value, self.device_index, info["inners"], info["columns"])
+        return self._call
 
     def matmul_host(self, x, col_major=False, y_col_major=False):
         """Same on numpy host arrays (copies in, runs, copies out, synchronises): the CPU entry points' form."""
@@ -149,7 +136,7 @@ class PackedWeight:
     def close(self):
         if self._h:
             lib().tllm_weight_destroy(self._h)
-            self._h = None
+            self._h = self._call = None
 
     def __del__(self):
         try:
@@ -191,6 +178,7 @@ class PackedMLP:
             check(lib().tllm_mlp_create(np_ptr(g), np_ptr(u), np_ptr(d), hidden, inter, float(s_gate), float(s_up), float(s_down),
                                         C.byref(o), C.byref(h)), "PackedMLP")
         self._h = h
+        self._handle, self._forward = h.value, _lib.binding().mlp_forward
 
     @property
     def info(self):
@@ -199,28 +187,13 @@ class PackedMLP:
         return a.as_dict(), b.as_dict()
 
     def forward(self, x, out=None, h=None):
-        import torch
-
-        if x.device.type != "cuda" or x.dim() != 2 or x.shape[1] != self.hidden:
-            raise RuntimeError("PackedMLP.forward expects a 2-D CUDA activation [rows, hidden]")
-        x = x.contiguous()
-        rows = x.shape[0]
-        if out is None:
-            out = torch.empty((rows, self.hidden), device=x.device, dtype=x.dtype)
-        elif out.dtype not in (x.dtype, torch.float32) or tuple(out.shape) != (rows, self.hidden) or not out.is_contiguous():
-            raise RuntimeError("out has the wrong dtype, shape or strides")
-        if h is None and rows > 16:
-            h = torch.empty((rows, self.inter), device=x.device, dtype=x.dtype)
-        with torch.cuda.device(x.device):
-            check(lib().tllm_mlp_forward_ex(self._h, x.data_ptr(), _lib.torch_dtype_code(x.dtype), rows, out.data_ptr(),
-                                            _lib.torch_dtype_code(out.dtype), h.data_ptr() if h is not None else None,
-                                            torch.cuda.current_stream().cuda_stream), "tllm_mlp_forward")
-        return out
+        return self._forward(self._handle, x, out, h, self.hidden, self.inter)
 
     def close(self):
         if self._h:
             lib().tllm_mlp_destroy(self._h)
             self._h = None
+            self._handle = 0                 # the library refuses a null handle
 
     def __del__(self):
         try:
