@@ -1,0 +1,94 @@
+// bits.cu -- instantiations and launches of bits_spmm_kernel (bits_kernel.cuh), in a translation unit of their own so that
+// they compile beside the rest.
+#include <mutex>
+
+#include "bits_kernel.cuh"
+#include "util.h"
+
+namespace tllm {
+namespace {
+
+#define BT_TRY(expr)                                                                                       \
+    do {                                                                                                   \
+        cudaError_t e_ = (expr);                                                                           \
+        if (e_ != cudaSuccess) return fail(TLLM_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_)); \
+    } while (0)
+
+template <int XT, int NB, int GR, bool ASYNC>
+int launch(const BitsParams& p, int grid, size_t smem, int device, cudaStream_t st) {
+    auto kern = bits_spmm_kernel<XT, NB, GR, ASYNC>;
+    static std::once_flag once[64];
+    cudaError_t err = cudaSuccess;
+    std::call_once(once[device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+    BT_TRY(err);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(BT_WARPS * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    BT_TRY(cudaLaunchKernelEx(&cfg, kern, p));
+    note_launch();
+    return TLLM_OK;
+}
+
+template <int XT, bool ASYNC>
+int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device, cudaStream_t st) {
+    if (nb == 1 && gr == 1) return launch<XT, 1, 1, ASYNC>(p, grid, smem, device, st);
+    if (nb == 1 && gr == 2) return launch<XT, 1, 2, ASYNC>(p, grid, smem, device, st);
+    if (nb == 1 && gr == 3) return launch<XT, 1, 3, ASYNC>(p, grid, smem, device, st);
+    if (nb == 2 && gr == 1) return launch<XT, 2, 1, ASYNC>(p, grid, smem, device, st);
+    if (nb == 2 && gr == 2) return launch<XT, 2, 2, ASYNC>(p, grid, smem, device, st);
+    if constexpr (XT == TLLM_F32) {
+        if (nb == 3 && gr == 1) return launch<XT, 3, 1, ASYNC>(p, grid, smem, device, st);
+        if (nb == 3 && gr == 2) return launch<XT, 3, 2, ASYNC>(p, grid, smem, device, st);
+    }
+    return fail(TLLM_ERR_ARG, "bits_launch: no kernel for %d x %d", nb, gr);
+}
+
+}  // namespace
+
+int bits_launch(BitsParams& p, int sms, int device, void* stream) {
+    const int cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, nb = (cols + 7) / 8;     // fp32: three bf16 columns a row
+    const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
+    const bool async = p.x_layout == TLLM_ROW_MAJOR && (uintptr_t)p.X % 16 == 0 && (size_t)p.x_ld * e % 16 == 0;
+    const int groups = (p.N + 15) / 16, grid = sms;
+    p.own = groups / grid, p.own_more = groups % grid;
+    p.mul4 = 4, p.mul16 = 16;
+    p.m_inv = (uint32_t)(((1ull << 32) + p.M - 1) / p.M);
+    // One pass over the widest block's columns if GR = 3 (two for more than eight columns of B: 64 and 128 registers) and a split
+    // of up to four allow it; the narrowest split that does, because every part of a split fetches the activations anew.
+    const int most = nb > 1 ? 2 : 3, own = p.own + (p.own_more ? 1 : 0);
+    p.split_log = own <= most ? 0 : own <= 2 * most ? 1 : 2;
+    const int split = 1 << p.split_log, passes = (own + split * most - 1) / (split * most);
+    p.per_pass = (own + passes - 1) / passes;
+    const int gr = (p.per_pass + split - 1) / split;
+    p.slot_bytes = (uint32_t)(gr * 512 + p.M * 128 * e);
+    // Pairs in flight: as many as a warp has to fetch and half of the shared memory holds (so that the next launch fits
+    // beside this one); where not even two fit there, up to all of it.
+    const int kparts = BT_WARPS / split, pairs = ((p.KB + 1) / 2 + kparts - 1) / kparts * passes;
+    const size_t red = (size_t)kparts * p.per_pass * cols * 80;
+    auto slots = [&](int d) { return pairs <= d ? pairs : d + 1; };
+    auto total = [&](int d) { return (size_t)BT_WARPS * slots(d) * p.slot_bytes + red; };
+    p.depth = 8;
+    while (p.depth > 1 && (p.depth / 2 >= pairs || total(p.depth) > BT_SMEM_SHARED)) p.depth /= 2;
+    if (p.depth == 1 && pairs > 1 && total(2) <= 220u * 1024u) p.depth = 2;
+    p.slots = slots(p.depth);
+    const size_t smem = total(p.depth);
+    if (smem > 227u * 1024u) return fail(TLLM_ERR_ARG, "bits_launch: %zu bytes of shared memory", smem);
+    cudaStream_t st = (cudaStream_t)stream;
+#define BT_PICK(XT) (async ? pick<XT, true>(p, nb, gr, grid, smem, device, st) : pick<XT, false>(p, nb, gr, grid, smem, device, st))
+    switch (p.x_dtype) {
+        case TLLM_F32: return BT_PICK(TLLM_F32);
+        case TLLM_F16: return BT_PICK(TLLM_F16);
+        case TLLM_BF16: return BT_PICK(TLLM_BF16);
+        default: return BT_PICK(TLLM_I8);
+    }
+#undef BT_PICK
+}
+
+}  // namespace tllm

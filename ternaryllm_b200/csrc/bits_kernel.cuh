@@ -1,0 +1,424 @@
+// bits_kernel.cuh -- the product on few activation rows: two-bit tiles of W streamed from HBM, decoded in registers and
+// multiplied with mma.sync.
+//
+//   D[n, m] = sum_k Wt[n, k] * X[m, k]      A = sixteen columns of W (decoded in registers), B = eight activation rows
+//
+// What bounds it.  At 0.25 bytes per entry the stream is the smallest form of W this library has (a 4096 x 11008 matrix is
+// 11.3 MB, 1.7 us at the measured copy bandwidth), so on all but the largest matrices the time of a launch is its chain
+// of latencies: launch, first bytes of W, activations once the preceding kernel has left, sum over the warps, store.
+// Hence:
+//   * no tensor memory, no operand tiles in shared memory, no role hand-over: a lane decodes what it loaded (a shift and
+//     an AND per two entries, bittile_format.h) straight into the A fragment of mma.sync.m16n8k16.  tcgen05 would need the
+//     decoded tile written to shared memory or tensor memory first, and its rate is not what limits eight rows;
+//   * a block owns whole columns (groups of sixteen, dealt out evenly) over all of K; its sixteen warps cut K, and the
+//     columns two or four ways where it owns many: no scratch, no counters, no second pass over global memory.  The warps'
+//     partial sums meet in shared memory and are added in warp order, so results do not depend on scheduling;
+//   * W and X travel by cp.async, several pairs of slices ahead, into slots that belong to one warp: no block barrier in
+//     the main loop, and W is in flight before the preceding kernel has finished (griddepcontrol.wait);
+//   * sixteen warps (four per scheduler hide the latency of shared-memory load -> decode -> MMA; with two per scheduler the
+//     loop issued 0.49 instructions per clock) of <= 64 registers, so that the next launch's block fits beside this one
+//     and starts streaming;
+//   * the shifts of the decode are multiplications by a value in a register: they run on the FMA pipe beside the ANDs on the
+//     ALU pipe, both of which take two clocks per warp instruction.
+//
+// Measured, fp16, CUDA-graph chain of distinct weights from HBM (us; before = the fastest of the other kernels):
+//   2048 x 2048    1 row  2.3 (gather 3.9)      8 rows  2.6 (batched 11.5)
+//   4096 x 11008   1 row  6.2 (gather 8.3, 75 % zeros; four-bit planes 10.5)   8 rows  7.0 (17.2)   16 rows 13.3 (19.5)
+//   8192 x 10240   1 row 10.8 (four-bit planes 15.4)     8 rows 12.1 (22.7)
+// Of the 6.2 us, 3.3 are there without any decode or MMA (launch chain, activations from L2, sums); the rest is instruction
+// issue, 0.55 per scheduler and clock.
+//
+// Precision.  fp16 / bf16 activations are multiplied as they are; int8 becomes fp16 (exact); an fp32 value is cut into
+// three bf16 values of eight significant bits each (truncation, so the three add up to it exactly), three columns of B
+// whose sums are added at the end.  W is 0 / +-2 (the factor two is taken back with the scale), products are exact, sums
+// are fp32; integer activations give exact sums below 2^24.
+#pragma once
+#include <type_traits>
+
+#include "bittile_format.h"
+#include "kernels.cuh"
+
+namespace tllm {
+
+#define BT_WARPS 16
+#define BT_SMEM_SHARED (112u * 1024u)   // two blocks of this size share an SM
+#define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks)
+#define BT_MASK 0xC000C000u             // the two codes at the top of a word's halves: 16-bit floats 0 / +-2
+
+struct BitsParams {
+    const uint4* bits;
+    const void* X;
+    void* Y;
+    int x_dtype, x_layout, x_ld;   // row-major X: elements between rows; column-major X: elements between k
+    int y_dtype, y_ld, epilogue;   // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
+    int M, K, N, KB;               // KB = ceil(K / 64) slices
+    int own, own_more;             // groups of sixteen columns per block; the first own_more blocks have one more
+    int per_pass;                  // groups per pass (<= split * GR)
+    int split_log;                 // the warps cut the block's columns 1 << split_log ways (1, 2 or 4); 16 >> split_log warps cut K
+    int slots, depth;              // pairs of slices a warp has room for, pairs in flight (1, 2, 4 or 8; < slots unless no slot is used twice)
+    uint32_t slot_bytes;           // shared memory of one pair of slices: GR * 512 + M * 128 * E
+    uint32_t m_inv;                // ceil(2^32 / M): idx / M = umulhi(idx, m_inv) for M > 1
+    uint32_t mul4, mul16;          // 4 and 16
+    float scale, scale2;
+};
+
+template <int XT>
+struct BitsAct;   // E: bytes of an activation; P: columns of B (16-bit values) it becomes
+template <>
+struct BitsAct<TLLM_F32> { static constexpr int E = 4, P = 3; };
+template <>
+struct BitsAct<TLLM_F16> { static constexpr int E = 2, P = 1; };
+template <>
+struct BitsAct<TLLM_BF16> { static constexpr int E = 2, P = 1; };
+template <>
+struct BitsAct<TLLM_I8> { static constexpr int E = 1, P = 1; };
+
+template <bool BF16>
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if (BF16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// waits until at most `left` of the newest groups are in flight (7, 3, 1 or 0)
+__device__ __forceinline__ void cp_wait(int left) {
+    if (left >= 7) asm volatile("cp.async.wait_group 7;" ::: "memory");
+    else if (left >= 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
+    else if (left >= 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+__device__ __forceinline__ uint4 bt_lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 bt_lds64(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void bt_sts128(uint32_t addr, const uint4& v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+// Sixteen bytes of a row that starts on any address: the one or two aligned vectors that hold them, shifted; bytes past the
+// row's end are zero.  Only vectors that hold at least one byte of the row are read.
+__device__ __forceinline__ uint4 bt_load_unaligned(const char* row, int off, int row_bytes) {
+    const int left = row_bytes - off;
+    if (left <= 0) return make_uint4(0u, 0u, 0u, 0u);
+    const char* p = row + off;
+    const uint32_t sh = (uint32_t)((uintptr_t)p & 15u);
+    const uint4* v = (const uint4*)(p - sh);
+    const uint4 a = __ldcg(v), b = sh && left > (int)(16u - sh) ? __ldcg(v + 1) : make_uint4(0u, 0u, 0u, 0u);
+    uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (sh & 8u) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+    }
+    if (sh & 4u) {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+    }
+    const uint32_t bs = (sh & 3u) * 8u;
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o[i] = __funnelshift_r(w[i], w[i + 1], bs);
+        const int keep = left - 4 * i;                    // bytes of this word inside the row
+        if (keep < 4) o[i] = keep <= 0 ? 0u : o[i] & (0xFFFFFFFFu >> (8 * (4 - keep)));
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+// the same sixteen bytes of a column-major X (elements of one row are x_ld apart)
+template <int E>
+__device__ __forceinline__ uint4 bt_load_strided(const void* X, int m, int k, int K, size_t ld) {
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int j = 0; j < 4 / E; ++j) {
+            const int kk = k + i * (4 / E) + j;
+            if (kk < K) {
+                const size_t at = (size_t)kk * ld + m;
+                const uint32_t x = E == 4 ? __ldcg((const unsigned int*)X + at) : E == 2 ? (uint32_t)__ldcg((const unsigned short*)X + at) : (uint32_t)__ldcg((const unsigned char*)X + at);
+                v |= x << (8 * E * j);
+            }
+        }
+        o[i] = v;
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// Where the 16-byte chunk `ch` of a pair of slices of row m lies in the row's 128 * E bytes: the four lanes that multiply one
+// row and the rows of two neighbouring groups of four then read eight different bank groups.  (The copy writes whole rows
+// in order but for this: chunks scattered by lane instead made cp.async four times slower, 57 against 15 us for sixteen rows
+// of a 4096 x 11008 matrix.)
+template <int XT>
+__device__ __forceinline__ uint32_t bt_chunk(uint32_t ch, uint32_t m) {
+    if (XT == TLLM_F32) return ch ^ (((ch >> 3) & 1u) | ((m & 1u) << 1));
+    if (XT == TLLM_I8) return ch ^ ((m & 1u) << 2);
+    return ch ^ (m & 1u);
+}
+// Offset of the lane's first chunk of slice 0 in row m; the other chunks are an addition (slice) and an exclusive or (chunk) away.
+template <int XT>
+__device__ __forceinline__ uint32_t bt_lane_chunk(uint32_t t, uint32_t m) { return bt_chunk<XT>(t * BitsAct<XT>::E, m) * 16u; }
+// The lane's sixteen activations of slice h (rows 16t .. 16t+15) -> the eight words of a B fragment (word p = rows 2p, 2p+1);
+// `at` is the address of the lane's first chunk of slice 0.  fp32: the `piece`-th of the three bf16 values that add up to
+// each of them.
+template <int XT>
+__device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, uint32_t (&b)[8]) {
+    constexpr uint32_t CS = BitsAct<XT>::E;
+    uint32_t w[4 * CS];
+    const uint32_t a0 = XT == TLLM_I8 ? at ^ (h * 64u) : at + h * (CS * 64u);
+#pragma unroll
+    for (uint32_t c = 0; c < CS; ++c) {
+        const uint4 v = bt_lds128(a0 ^ (c * 16u));
+        w[4 * c] = v.x, w[4 * c + 1] = v.y, w[4 * c + 2] = v.z, w[4 * c + 3] = v.w;
+    }
+    if constexpr (XT == TLLM_F32) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {       // what the upper half (eight significant bits) leaves, exactly
+                const float rest = __uint_as_float(w[i]) - __uint_as_float(w[i] & 0xFFFF0000u);
+                if (p < piece) w[i] = __float_as_uint(rest);
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x7632);
+    } else if constexpr (XT == TLLM_I8) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t u = w[i >> 1] ^ 0x80808080u;                                     // 0..255: x + 128
+            const uint32_t v = __byte_perm(u, 0x64646464u, i & 1 ? 0x4342 : 0x4140);        // fp16 1024 + (x + 128)
+            const uint32_t bias = 0x64806480u;                                              // 1152 twice
+            const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&bias));
+            b[i] = *reinterpret_cast<const uint32_t*>(&d);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] = w[i];
+    }
+}
+
+// A warp multiplies up to GR groups of sixteen columns by NB blocks of eight columns of B (activation rows; fp32: pieces of
+// rows).  A block with more than split * GR groups makes several passes.
+// ASYNC: the rows of X start on 16 bytes and are copied by cp.async; otherwise they pass through registers.
+//
+// The code is kept short (rolled loops, no divisions): a warp of a small product runs the loop body once or twice, and then
+// fetching instructions costs more than executing them.
+template <int XT, int NB, int GR, bool ASYNC>
+__global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_spmm_kernel(const __grid_constant__ BitsParams p) {
+    extern __shared__ __align__(128) unsigned char bt_smem[];
+    using Act = BitsAct<XT>;
+    constexpr bool BF16 = XT == TLLM_BF16 || XT == TLLM_F32;
+    constexpr int CPR = 8 * Act::E, RPI = 32 / CPR, KPC = 16 / Act::E;     // chunks per row (and pair of slices), rows per warp copy, values per chunk
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
+    const int KB = p.KB, KP = (KB + 1) >> 1, D = p.depth, S = p.slots, M = p.M, SL = p.split_log;
+    const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = warp & ((1 << SL) - 1);
+    const int np = kw < KP ? (KP - kw + kstep - 1) >> klog : 0;      // pairs of this warp: kw, kw + kstep, ...
+    const uint32_t ring = smem_u32(bt_smem) + (uint32_t)warp * (uint32_t)S * p.slot_bytes;
+    float* red = (float*)(bt_smem + (size_t)BT_WARPS * S * p.slot_bytes);          // [warp][group][column of B][20] partial sums
+    const uint32_t group_bytes = (uint32_t)KB * 256u;
+    pdl_launch_dependents();
+    // There is a block for every SM even where there are fewer groups: with free SMs the next launch's blocks would be placed
+    // two to an SM there (8192 x 2048, one row: 10.5 us instead of 5), so the spare ones hold their place until it is settled.
+    if (own == 0) {
+        pdl_wait();
+        return;
+    }
+
+    // A pass covers groups [q0, q0 + n) of the block; this warp's share is [n * cw / split, n * (cw + 1) / split) of them.
+    // ---- copies: the warp's step s (its pairs in order, pass after pass) goes to slot s % S ---------------------------
+    const char* wsrc;                                                // first group of the pass being fetched, this warp's next pair
+    uint32_t last;                                                   // offset of the last group from it
+    int fpass = 0, fi = 0, fs = 0;                                   // next copy: first group of the pass, pair, slot
+    auto open_pass = [&]() {
+        const int n = min(p.per_pass, own - fpass), a = (n * cw) >> SL, e = (n * (cw + 1)) >> SL;
+        wsrc = (const char*)p.bits + (size_t)(c0 + fpass + a) * group_bytes + (size_t)kw * 512u;
+        last = (uint32_t)max(e - a - 1, 0) * group_bytes;
+    };
+    auto copy_w = [&](uint32_t slot) {
+        const uint32_t dst = slot + (uint32_t)lane * 16u;
+        if (2 * (kw + (fi << klog)) + 2 <= KB) {
+#pragma unroll
+            for (int j = 0; j < GR; ++j) cp_async16(dst + (uint32_t)j * 512u, wsrc + min((uint32_t)j * group_bytes, last) + lane * 16);
+        } else {                                                     // an odd last slice
+#pragma unroll
+            for (int j = 0; j < GR; ++j) {
+                cp_async8(dst + (uint32_t)j * 512u, wsrc + min((uint32_t)j * group_bytes, last) + lane * 8);
+                asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(dst + (uint32_t)j * 512u + 8u), "r"(0u) : "memory");
+            }
+        }
+    };
+    auto advance = [&]() {
+        wsrc += (uint32_t)kstep * 512u;
+        if (++fi == np) {
+            fi = 0, fpass += p.per_pass;
+            open_pass();
+        }
+        if (++fs == S) fs = 0;
+    };
+    // X: the lanes copy whole rows, 16 bytes each (the caller's pair i of this warp)
+    const uint32_t xm = (uint32_t)lane / CPR, xch = (uint32_t)lane % CPR;
+    auto copy_x = [&](int i, uint32_t slot) {
+        const int k = (kw + (i << klog)) * 128 + (int)xch * KPC;
+        const char* src = (const char*)p.X + ((size_t)xm * p.x_ld + k) * Act::E;
+        const uint32_t xb = slot + GR * 512u;
+#pragma unroll 1
+        for (uint32_t m = xm; m < (uint32_t)M; m += RPI, src += (size_t)RPI * p.x_ld * Act::E) {
+            const uint32_t dst = xb + (m * CPR + bt_chunk<XT>(xch, m)) * 16u;
+            if (ASYNC) {
+                if (k < p.K) cp_async16(dst, src);
+                else bt_sts128(dst, make_uint4(0u, 0u, 0u, 0u));
+            } else if (p.x_layout == TLLM_ROW_MAJOR) {
+                bt_sts128(dst, bt_load_unaligned((const char*)p.X + (size_t)m * p.x_ld * Act::E, k * Act::E, p.K * Act::E));
+            } else {
+                bt_sts128(dst, bt_load_strided<Act::E>(p.X, (int)m, k, p.K, (size_t)p.x_ld));
+            }
+        }
+    };
+    open_pass();
+#pragma unroll 1
+    for (int s = 0; s < D; ++s)                                     // W does not depend on the preceding kernel
+        if (fpass < own && np) {
+            copy_w(ring + (uint32_t)fs * p.slot_bytes);
+            advance();
+        }
+    const int pre_pass = fpass, pre_i = fi;
+    pdl_wait();
+    {
+        int i = 0, pass = 0;
+#pragma unroll 1
+        for (int s = 0; s < D; ++s) {
+            if (np && (pass < pre_pass || i < pre_i)) {
+                copy_x(i, ring + (uint32_t)s * p.slot_bytes);
+                if (++i == np) i = 0, pass += p.per_pass;
+            }
+            cp_commit();
+        }
+    }
+
+    // This lane's column of B in block nb: a row of X (any row, past the last column: those sums are not used) and its piece.
+    uint32_t bat[NB];
+    int bpiece[NB];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+        const uint32_t c = (uint32_t)(nb * 8 + g), m = min(c / Act::P, (uint32_t)M - 1u);
+        bpiece[nb] = (int)(c % Act::P);
+        bat[nb] = GR * 512u + m * (CPR * 16u) + bt_lane_chunk<XT>((uint32_t)t, m);
+    }
+    // Multipliers in registers: a shift by an immediate would run on the ALU pipe, which the ANDs already fill.
+    uint32_t m4, m16;
+    asm volatile("mov.b32 %0, %2;\n\tmov.b32 %1, %3;" : "=r"(m4), "=r"(m16) : "r"(p.mul4), "r"(p.mul16));
+    int cs = 0;                                                      // slot being consumed
+#pragma unroll 1
+    for (int q0 = 0; q0 < own; q0 += p.per_pass) {
+        const int ng = min(p.per_pass, own - q0), w0 = (ng * cw) >> SL, mine = ((ng * (cw + 1)) >> SL) - w0;    // this warp's groups of the pass
+        float acc[GR][NB][4];
+#pragma unroll
+        for (int j = 0; j < GR; ++j)
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[j][nb][i] = 0.f;
+#pragma unroll 1
+        for (int i = 0; i < np; ++i) {
+            cp_wait(D - 1);
+            __syncwarp();                                            // other lanes' chunks of X are here, and they have read the slot before
+            const uint32_t slot = ring + (uint32_t)cs * p.slot_bytes;
+            if (fpass < own) {                                       // into the slot that was consumed one step ago
+                const uint32_t dst = ring + (uint32_t)fs * p.slot_bytes;
+                copy_w(dst);
+                copy_x(fi, dst);
+                advance();
+            }
+            cp_commit();
+#pragma unroll 1
+            for (uint32_t h = 0; h < 2; ++h) {
+                uint32_t bf[NB][8];
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb) bt_fragment<XT>(slot + bat[nb], h, bpiece[nb], bf[nb]);
+                auto half = [&](auto first, auto end) {              // groups [lo, hi) of the warp
+                    constexpr int lo = decltype(first)::value, hi = decltype(end)::value;
+                    uint2 a[GR];
+#pragma unroll
+                    for (int j = lo; j < hi; ++j) a[j] = bt_lds64(slot + (uint32_t)j * 512u + (uint32_t)lane * 16u + h * 8u);
+                    // consecutive MMAs go to different accumulators: a chain of dependent ones costs their full latency each
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)
+#pragma unroll
+                        for (int j = lo; j < hi; ++j) {
+                            const uint32_t a0 = a[j].x & BT_MASK, a1 = a[j].y & BT_MASK, a2 = (a[j].x * m4) & BT_MASK, a3 = (a[j].y * m4) & BT_MASK;
+                            if (s < 3) a[j].x *= m16, a[j].y *= m16;
+#pragma unroll
+                            for (int nb = 0; nb < NB; ++nb) mma_16816<BF16>(acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                        }
+                };
+                // a warp's share of a pass is GR groups or one less (or none: GR = 1)
+                if constexpr (GR > 1) half(std::integral_constant<int, 0>{}, std::integral_constant<int, GR - 1>{});
+                if (mine == GR) half(std::integral_constant<int, GR - 1>{}, std::integral_constant<int, GR>{});
+            }
+            if (++cs == S) cs = 0;
+        }
+        // ---- sum over the warps that share columns: lane (g, t) holds columns g, g + 8 of W for columns 2t, 2t + 1 of B (20
+        // floats apart: no bank conflicts)
+        const int MC = M * Act::P;
+        const int kw_step = p.per_pass * MC * 20;
+        if (q0 > 0) __syncthreads();                                 // the previous pass has been read
+#pragma unroll
+        for (int j = 0; j < GR; ++j)
+            if (j < mine) {
+                float* r = red + (size_t)kw * kw_step + (w0 + j) * MC * 20 + g;
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb) {
+                    const int m = nb * 8 + 2 * t;
+                    if (m < MC) r[m * 20] = acc[j][nb][0], r[m * 20 + 8] = acc[j][nb][2];
+                    if (m + 1 < MC) r[(m + 1) * 20] = acc[j][nb][1], r[(m + 1) * 20 + 8] = acc[j][nb][3];
+                }
+            }
+        __syncthreads();
+        // half a warp per group and row; idx = group * M + row
+        const int c = lane & 15;
+#pragma unroll 1
+        for (int i0 = warp * 2; i0 < ng * M; i0 += BT_WARPS * 2) {
+            const int idx = i0 + (lane >> 4), j = M > 1 ? (int)__umulhi((uint32_t)idx, p.m_inv) : idx, m = idx - j * M;
+            const bool valid = idx < ng * M;
+            float v = 0.f;
+            if (valid) {
+                const float* r = red + (j * MC + m * Act::P) * 20 + c;
+#pragma unroll
+                for (int pc = Act::P - 1; pc >= 0; --pc)            // fp32: the small pieces first
+#pragma unroll 4
+                    for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
+            }
+            const int n = (c0 + q0 + j) * 16 + c;
+            if (p.epilogue == 0) {
+                if (valid && n < p.N) {
+                    if (p.y_dtype == TLLM_I32) ((int*)p.Y)[(size_t)m * p.y_ld + n] = (int)(v * 0.5f);
+                    else store_out(p.Y, p.y_dtype, (size_t)m * p.y_ld + n, v * p.scale);
+                }
+            } else {
+                const float u = __shfl_xor_sync(0xffffffffu, v, 1);
+                if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_ld + (n >> 1), silu_mul(v * p.scale, u * p.scale2));
+            }
+        }
+    }
+}
+
+// one launch of up to BT_MAX_ROWS rows (half of it fp32); fills in everything from `own` to `mul16` (bits.cu)
+int bits_launch(BitsParams& p, int sms, int device, void* stream);
+
+}  // namespace tllm

@@ -1,17 +1,35 @@
-// bittile_format.h -- the dense two-bit copy of W that the tensor-core kernel reads ("bit tiles"), shared by
-// the host packer and mma_kernel.cuh.
+// bittile_format.h -- the dense two-bit copy of W ("bit tiles") that the register-decode kernel (bits_kernel.cuh) and the
+// batched tensor-core kernel (mma_kernel.cuh) read, shared by the host packer and the device code.
 //
-// For output-column tile nt (128 columns) and K-slice kb (64 rows): 128 consecutive 16-byte records, one per
-// column, each holding 64 codes (0: zero, 1: +1, 2: -1).  Row k_local of the slice sits in 32-bit word
-// k_local/16 at bit mm_code_bit(k_local%16); the positions are chosen so that one shift, one mask and one byte
-// permute turn two codes into two fp16 / bf16 values.  The tiles of one column tile are contiguous along K.
+// A code is two bits, nz | neg << 1: 0 = zero, 1 = +1, 3 = -1.  Put into the top two bits of a 16-bit float -- sign and
+// highest exponent bit -- it IS the number: 0, +2.0 or -2.0 in fp16 and in bf16 alike.  One word holds sixteen
+// consecutive rows of one column; the pair of rows (2p, 2p+1) sits so that a left shift by 2p brings its two codes to the
+// top of the word's two halves: one shift and one AND decode two entries (mm_code_bit below).
+//
+// Order: columns in groups of sixteen (N padded to 128), a group's slices of 64 rows one after the other along K, so a
+// group is one contiguous stream of KB * 256 bytes (KB = ceil(K / 64)).  Slices come in pairs of 512 bytes = 16 bytes for
+// each lane of a warp; lane 4g + t holds { slice 0: column g, column g + 8; slice 1: column g, column g + 8 }, rows
+// 16t .. 16t + 15 of the slice -- the places that mma.sync.m16n8k16 wants lane 4g + t to fill, so a warp loads 16 bytes per
+// lane, coalesced, and decodes in registers.  An odd last slice is 256 bytes, 8 per lane.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
-inline int mm_code_bit(int kk) {            // kk = 0..15
-    const int j = kk >> 1, h = kk & 1;       // output word (two values) and half within it
-    return (j < 4 ? 2 * j : 16 + 2 * (j - 4)) + 8 * h;
+#ifdef __CUDACC__
+#define MM_FMT_HD __host__ __device__
+#else
+#define MM_FMT_HD
+#endif
+MM_FMT_HD inline int mm_code_bit(int kk) {            // kk = 0..15, row within the word
+    return 14 - 2 * (kk >> 1) + 16 * (kk & 1);
+}
+// index of the word that holds rows 16t .. 16t+15 of slice kb, column n
+MM_FMT_HD inline size_t mm_word_index(int n, int kb, int t, int KB) {
+    const size_t base = (size_t)(n >> 4) * KB * 64;
+    const int g = n & 7, hi = (n >> 3) & 1, lane = 4 * g + t;
+    if ((kb | 1) < KB) return base + (size_t)(kb >> 1) * 128 + lane * 4 + (kb & 1) * 2 + hi;
+    return base + (size_t)kb * 64 + lane * 2 + hi;
 }
 void mm_pack_bits(const int8_t* w, int inners, int columns, std::vector<uint32_t>* bits, int* n_tiles, int* kb);
 void mm_unpack_bits(const std::vector<uint32_t>& bits, int inners, int columns, int8_t* w);

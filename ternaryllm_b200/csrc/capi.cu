@@ -10,6 +10,7 @@
 
 #include <cudaTypedefs.h>
 
+#include "bits_kernel.cuh"
 #include "bstream_kernel.cuh"
 #include "kernels.cuh"
 #include "mma_kernel.cuh"
@@ -153,10 +154,6 @@ struct tllm_weight {
     unsigned int* d_nr_counters = nullptr;
     CUtensorMap nr_map[4];
     int nb_k_pad = 0, nr_grid = 0;
-    // the activation tensor map of the last tensor-core launch (encoding one costs more than a short launch)
-    CUtensorMap tmap;
-    const void* tmap_x = nullptr;
-    int tmap_dtype = -1, tmap_rows = 0, tmap_ld = 0, tmap_nt = 0;
 };
 
 struct tllm_mlp {
@@ -241,100 +238,239 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// true when the tensor-core kernel can take this call: fp16 / bf16 row-major activations whose rows TMA can address
+// true when TMA can read the activations where they are (rows on 16 bytes; a box is 64 values wide)
+bool mm_direct(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld) {
+    return (x_dtype == TLLM_F16 || x_dtype == TLLM_BF16) && x_layout == TLLM_ROW_MAJOR && (uintptr_t)X % 16 == 0 && (size_t)x_ld * 2 % 16 == 0 &&
+           w->lay.inners >= MM_TILE_K;
+}
+
+// true when the tensor-core kernel is pinned, or the cost model of the older kernels prefers it, for fp16 / bf16 row-major
+// activations whose rows TMA can address
 bool mm_usable(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows) {
-    // (a TMA box is 64 values wide: narrower matrices stay on the gather kernel)
-    if (!w->d_bits || (x_dtype != TLLM_F16 && x_dtype != TLLM_BF16) || x_layout != TLLM_ROW_MAJOR || ((uintptr_t)X % 16) || ((size_t)x_ld * 2 % 16) ||
-        w->lay.inners < MM_TILE_K || tensor_map_encoder() == nullptr)
-        return false;
+    if (!w->d_bits || !mm_direct(w, X, x_dtype, x_layout, x_ld) || tensor_map_encoder() == nullptr) return false;
     const int thr = mm_min_rows();
     if (thr == 0) return false;
     if (thr > 0) return rows >= thr;
     return mm_model_prefers_tensor(w->lay.nnz, (int64_t)w->lay.inners * w->lay.columns, rows);
 }
 
-// the whole product of `rows` activation rows in one launch of the tensor-core kernel
-int run_mm(tllm_weight* w, const void* X, int x_dtype, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
-           float scale2, cudaStream_t st) {
+// ---- workspace of one call ---------------------------------------------------------------------------------------------
+// Stream-ordered allocations from a pool of the library's own (one per device): a call takes what it needs, frees it behind its
+// last kernel in stream order, and the next call on the stream gets the same memory without a synchronisation.  The pool
+// is thread-safe, keeps at most WS_KEEP_BYTES across synchronisations and is trimmed to nothing when the last handle goes.
+constexpr uint64_t WS_KEEP_BYTES = 256ull << 20;
+std::mutex g_ws_mu;
+cudaMemPool_t g_ws_pool[64] = {};
+std::atomic<int> g_handles{0};
+
+int ws_pool(int device, cudaMemPool_t* out) {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    if (device < 0 || device >= 64) return fail(TLLM_ERR_ARG, "device ordinal %d out of range", device);
+    if (!g_ws_pool[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        CU_TRY(cudaMemPoolCreate(&pool, &props));
+        uint64_t keep = WS_KEEP_BYTES;
+        CU_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        g_ws_pool[device] = pool;
+    }
+    *out = g_ws_pool[device];
+    return TLLM_OK;
+}
+void ws_trim() {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    for (cudaMemPool_t pool : g_ws_pool)
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+struct Workspace {
+    void* ptr = nullptr;
+    cudaStream_t st = nullptr;
+    int take(int device, size_t bytes, cudaStream_t stream) {
+        cudaMemPool_t pool = nullptr;
+        const int rc = ws_pool(device, &pool);
+        if (rc) return rc;
+        st = stream;
+        CU_TRY(cudaMallocFromPoolAsync(&ptr, bytes, pool, stream));
+        return TLLM_OK;
+    }
+    ~Workspace() {
+        if (ptr) cudaFreeAsync(ptr, st);
+    }
+};
+
+// How a product of `rows` rows (in `planes` planes) is cut: row tiles of Nt rows each, whole tiles or equal ranges of units, chosen
+// by an estimate in SM clocks.  An MMA of 128 x Nt x 16 takes Nt / 2 clocks of the tensor core and its operands 32 + Nt / 4 of
+// shared memory, a slice of 64 rows of W four of them per plane and never less than the 150 of its decode.  A tile's epilogue is
+// hidden behind the next one except at the end.  In a tile that `parts` blocks share the last one to arrive reads the other
+// parts, a round trip to L2 for every sixteen rows of each.
+struct MmPlan {
+    int Nt, m_tiles, split;
+    double clocks;
+};
+int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_NT : MM_MAX_NT / 2; }     // two accumulators each with three planes
+MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
+    MmPlan best{0, 0, 0, 0};
+    const int kbu = (kb + 1) / 2;
+    for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
+        const int mt = (rows + nt - 1) / nt;
+        if (mt > MM_MAX_M_TILES) continue;
+        const double tiles = (double)n_tiles * mt, units = tiles * kbu;
+        const double slice = std::max(150.0, planes * 4 * std::max(nt / 2.0, 32.0 + nt / 4.0)), epilogue = nt / 16 * 150.0;
+        const double whole = std::ceil(tiles / sms) * kb * slice + epilogue;
+        const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
+        const double split = std::ceil(units / blocks) * 2 * slice + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
+        if (best.Nt == 0 || whole < best.clocks) best = MmPlan{nt, mt, 0, whole};
+        if (split < best.clocks) best = MmPlan{nt, mt, 1, split};
+        if (nt >= rows) break;
+    }
+    return best;
+}
+
+int encode_rows_map(CUtensorMap* map, const void* base, bool bf16, int k, int rows, size_t pitch_bytes, int box_rows) {
+    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch_bytes};
+    const cuuint32_t box[2] = {MM_TILE_K, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult cr = tensor_map_encoder()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides,
+                                             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
+    return TLLM_OK;
+}
+
+cudaLaunchAttribute pdl_attribute() {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    return at;
+}
+
+int stage_pad(int k) { return (k + 63) / 64 * 64; }
+
+int run_stage(const void* X, int x_dtype, int x_layout, int x_ld, int rows, int K, unsigned short* out, cudaStream_t st) {
+    StageParams q{X, out, x_dtype, x_layout, x_ld, rows, K, stage_pad(K)};
+    void (*kern)(StageParams) = x_dtype == TLLM_F32 ? stage_acts_kernel<TLLM_F32> : x_dtype == TLLM_I8 ? stage_acts_kernel<TLLM_I8> : stage_acts_kernel<TLLM_F16>;
+    cudaLaunchConfig_t cfg{};
+    const long long blocks = x_layout == TLLM_ROW_MAJOR ? ((long long)rows * (q.k_pad / 8) + 255) / 256 : (long long)(q.k_pad / 64) * ((rows + 31) / 32);
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1] = {pdl_attribute()};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU_TRY(cudaLaunchKernelEx(&cfg, kern, q));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TLLM_OK;
+}
+
+// X of one launch as the kernel reads it: `planes` planes of 16-bit rows, plane_rows apart, pitch bytes per row
+struct MmActs {
+    const void* base;
+    bool bf16;
+    int planes, plane_rows;
+    size_t pitch;
+};
+struct MmOut {
+    void* Y;
+    int dtype, ld, epilogue;
+    float scale, scale2;
+    bool col_major;          // Y[n * ld + m]
+    bool planes;             // three bf16 planes, plane elements apart, instead of dtype
+    long long plane;
+};
+
+// rows [0, rows) of `x` (at most MM_MAX_M_TILES tiles) in one launch of the tensor-core kernel
+int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStream_t st) {
     const BsLayout& L = w->lay;
+    const MmPlan plan = mm_plan(rows, x.planes, w->mm_n_tiles, w->mm_kb, w->mm_grid);
     MmParams p{};
     p.bits = w->d_bits;
-    p.Y = Y;
-    p.partial = w->d_mm_partial;
+    p.Y = o.Y;
     p.counters = w->d_mm_counters;
     p.status = w->d_status;
-    p.M = rows;
-    p.K = L.inners;
-    p.N = L.columns;
-    p.KB = w->mm_kb;
-    p.n_tiles = w->mm_n_tiles;
-    p.Nt = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
-    p.m_tiles = (rows + p.Nt - 1) / p.Nt;
-    p.y_dtype = y_dtype;
-    p.epilogue = epilogue;
-    p.y_ld = y_ld;
-    // slices per unit and ring depths: narrow activation tiles take four slices per hand-over and a deep ring of
-    // bit tiles (the stream from HBM is what matters there), wide ones keep the operand ring deep instead
-    p.UK = p.Nt <= 64 ? 4 : 2;
-    p.S = p.Nt == 128 ? 3 : 2;
-    p.R = p.Nt == 64 ? 4 : 8;
-    p.KBU = (p.KB + p.UK - 1) / p.UK;
-    p.split = p.Nt <= MM_SPLIT_MAX_NT ? 1 : 0;
-    const uint32_t fmt = x_dtype == TLLM_BF16 ? 1u : 0u;
+    p.M = rows, p.K = L.inners, p.N = L.columns;
+    p.KB = w->mm_kb, p.KBU = (p.KB + 1) / 2;
+    p.n_tiles = w->mm_n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split;
+    p.P = x.planes, p.plane_rows = x.plane_rows;
+    p.y_dtype = o.dtype, p.epilogue = o.epilogue, p.y_ld = o.ld, p.y_planes = o.planes, p.plane_y = o.plane;
+    p.y_col = !o.col_major ? 0 : (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0 ? 2 : 1;
+    // Rings within 208 KiB: four units of bit tiles (eight for narrow tiles, which are bound by the stream of W), then as many
+    // units of A and B as fit; with three planes B turns over three times as fast and gets what two or three units of A leave.
+    p.R = p.Nt <= 64 ? 8 : 4;
+    const int room = 208 * 1024 - p.R * MM_UNIT_BYTES, b_unit = p.Nt * 256;
+    p.SA = x.planes == 1 ? std::min(MM_MAX_STAGES, room / (MM_A_UNIT + b_unit)) : p.Nt <= 64 ? 3 : 2;
+    p.SB = x.planes == 1 ? p.SA : std::min(MM_MAX_STAGES, (room - p.SA * MM_A_UNIT) / b_unit);
+    p.mul4 = 4, p.mul16 = 16;
+    const uint32_t fmt = x.bf16 ? 1u : 0u;
     // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B formats (bits 7-9, 10-12), both K-major,
     // N / 8 in bits 17-22, M / 16 in bits 24-28
     p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.Nt >> 3) << 17) | ((uint32_t)(MM_TILE_N >> 4) << 24);
-    p.tmem_cols = 2u * (uint32_t)p.Nt < 32u ? 32u : 2u * (uint32_t)p.Nt;
-    // fp16 holds +-1.0 (0x3C00 / 0xBC00); bf16 holds +-2.0 (0x4000 / 0xC000, whose low byte is zero like fp16's)
-    // and the factor 1/2 moves into the scale
-    p.pool = fmt ? 0x00C04000u : 0x00BC3C00u;
-    p.scale = fmt ? scale * 0.5f : scale;
-    p.scale2 = fmt ? scale2 * 0.5f : scale2;
+    p.tmem_cols = 32;
+    while (p.tmem_cols < (x.planes == 1 ? 2u : 4u) * (uint32_t)p.Nt) p.tmem_cols *= 2;
+    p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
 
-    if (w->tmap_x != X || w->tmap_dtype != x_dtype || w->tmap_rows != rows || w->tmap_ld != x_ld || w->tmap_nt != p.Nt) {
-        const cuuint64_t dims[2] = {(cuuint64_t)L.inners, (cuuint64_t)rows};
-        const cuuint64_t strides[1] = {(cuuint64_t)x_ld * 2u};
-        const cuuint32_t box[2] = {MM_TILE_K, (cuuint32_t)p.Nt};
-        const cuuint32_t estr[2] = {1, 1};
-        const CUresult cr = tensor_map_encoder()(&w->tmap, fmt ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(X), dims,
-                                                 strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (cr != CUDA_SUCCESS) {
-            w->tmap_x = nullptr;
-            return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
-        }
-        w->tmap_x = X, w->tmap_dtype = x_dtype, w->tmap_rows = rows, w->tmap_ld = x_ld, w->tmap_nt = p.Nt;
-    }
-
-    const size_t smem = 1024 + (size_t)p.S * p.UK * (MM_A_STAGE_BYTES + (size_t)p.Nt * 128) + (size_t)p.R * p.UK * MM_CHUNK_BYTES + 512;
+    CUtensorMap map;
+    int rc = encode_rows_map(&map, x.base, x.bf16, L.inners, (x.planes - 1) * x.plane_rows + rows, x.pitch, p.Nt);
+    if (rc) return rc;
+    const size_t smem = 1024 + (size_t)p.SA * MM_A_UNIT + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512;
     if (smem > 227 * 1024) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
-    void (*kern)(CUtensorMap, MmParams) = p.UK == 4 ? mma_spmm_kernel<4> : mma_spmm_kernel<2>;
-    static std::mutex mu;
-    static bool configured[64][2] = {};
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        const int slot = p.UK == 4 ? 1 : 0;
-        if (w->device < 64 && !configured[w->device][slot]) {
-            CU_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-            configured[w->device][slot] = true;
-        }
+    static std::once_flag once[64];
+    cudaError_t err = cudaSuccess;
+    std::call_once(once[w->device & 63], [&] { err = cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+    CU_TRY(err);
+    // never more blocks than items: the hand-over between the blocks that share a tile counts on every block in a
+    // tile's range of owners holding at least one unit of it
+    const long long items = (long long)p.n_tiles * p.m_tiles * (p.split ? p.KBU : 1);
+    const int grid = (int)(items < w->mm_grid ? items : w->mm_grid);
+    Workspace ws;
+    if (p.Nt <= MM_OWN_NT || !p.split) p.partial = w->d_mm_partial;
+    else {
+        rc = ws.take(w->device, (size_t)2 * grid * MM_TILE_N * p.Nt * sizeof(float), st);
+        if (rc) return rc;
+        p.partial = (float*)ws.ptr;
     }
     cudaLaunchConfig_t cfg{};
-    // never more blocks than work items: the hand-over between the blocks that share a tile counts on every
-    // block in a tile's range of owners holding at least one unit of it
-    const long long tiles = (long long)p.n_tiles * p.m_tiles, items = p.split ? tiles * p.KBU : tiles;
-    cfg.gridDim = dim3((unsigned)(items < w->mm_grid ? items : w->mm_grid));
+    cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(MM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[1] = {pdl_attribute()};
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CU_TRY(cudaLaunchKernelEx(&cfg, kern, w->tmap, p));
+    CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
+    return TLLM_OK;
+}
+
+// the whole product on the tensor-core kernel: activations that TMA cannot read as they are go through planes in a workspace
+int run_mm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
+           float scale2, cudaStream_t st, bool y_col = false) {
+    const int K = w->lay.inners;
+    const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
+    const bool direct = mm_direct(w, X, x_dtype, x_layout, x_ld);
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
+    Workspace ws;
+    if (!direct) {
+        const int rc = ws.take(w->device, (size_t)planes * std::min(rows, per) * stage_pad(K) * 2, st);
+        if (rc) return rc;
+    }
+    for (int r0 = 0; r0 < rows; r0 += per) {
+        const int m = std::min(rows - r0, per);
+        const char* xp = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
+        MmActs a{xp, x_dtype == TLLM_BF16 || x_dtype == TLLM_F32, planes, m, (size_t)x_ld * 2};
+        if (!direct) {
+            const int rc = run_stage(xp, x_dtype, x_layout, x_ld, m, K, (unsigned short*)ws.ptr, st);
+            if (rc) return rc;
+            a.base = ws.ptr, a.pitch = (size_t)stage_pad(K) * 2;
+        }
+        const int rc = launch_mm(w, a, m, MmOut{(char*)Y + (y_col ? (size_t)r0 : (size_t)r0 * y_ld) * ye, y_dtype, y_ld, epilogue, scale, scale2, y_col, false, 0}, st);
+        if (rc) return rc;
+    }
     return TLLM_OK;
 }
 
@@ -541,15 +677,62 @@ int run_nb(tllm_weight* w, const void* X, int x_dtype, int x_ld, int rows, void*
     return TLLM_OK;
 }
 
-enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE };
+// ---- two-bit tiles decoded in registers ----------------------------------------------------------------------------
+// rows one launch takes: 16, fp32 (three bf16 values each) 8
+int bt_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? BT_MAX_ROWS / 2 : BT_MAX_ROWS; }
+
+int run_bits(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
+             float scale2, cudaStream_t st) {
+    BitsParams p{};
+    p.bits = w->d_bits;
+    p.x_dtype = x_dtype, p.x_layout = x_layout, p.x_ld = x_ld;
+    p.y_dtype = y_dtype, p.y_ld = y_ld, p.epilogue = epilogue;
+    p.K = w->lay.inners, p.N = w->lay.columns, p.KB = w->mm_kb;
+    p.scale = scale * 0.5f, p.scale2 = scale2 * 0.5f;            // the decoded weights are +-2
+    const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
+    const int per = bt_rows_per_launch(x_dtype);
+    for (int r0 = 0; r0 < rows; r0 += per) {
+        p.M = rows - r0 < per ? rows - r0 : per;
+        p.X = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
+        p.Y = (char*)Y + (size_t)r0 * y_ld * ye;
+        const int rc = bits_launch(p, w->mm_grid, w->device, st);
+        if (rc) return rc;
+    }
+    if (rows > 4) g_mm_launches.fetch_add((rows + per - 1) / per, std::memory_order_relaxed);   // counted with the batched products
+    return TLLM_OK;
+}
+
+// Cost models of the two kernels that read the two-bit tiles, microseconds.  Register decode: a launch chain of 2 us and, per
+// million entries, 0.1 (one block of eight columns of B), 0.25 (two) or 0.35 (three).  Batched: 6 us of start-up and
+// hand-over, the plan's clocks at 1.8 GHz, and 2.5 us for planes that have to be made first.
+double bt_model_us(int64_t entries, int x_dtype, int rows) {
+    static const double per_mentry[4] = {0, 0.105, 0.25, 0.35};
+    const int per = bt_rows_per_launch(x_dtype), p = x_dtype == TLLM_F32 ? 3 : 1;
+    double t = 0;
+    for (int r0 = 0; r0 < rows; r0 += per) t += 2.0 + entries * 1e-6 * per_mentry[(std::min(rows - r0, per) * p + 7) / 8];
+    return t;
+}
+double mm_tiles_model_us(const tllm_weight* w, bool direct, int x_dtype, int rows) {
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
+    double t = 0;
+    for (int r0 = 0; r0 < rows; r0 += per)
+        t += 6.0 + mm_plan(std::min(rows - r0, per), planes, w->mm_n_tiles, w->mm_kb, w->mm_grid).clocks / 1800.0 + (direct ? 0.0 : 2.5);
+    return t;
+}
+
+enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
 KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows) {
     const bool nb = nb_usable(w, x_dtype, x_layout, rows), mm = mm_usable(w, X, x_dtype, x_layout, x_ld, rows);
     if (nb && g_nb_max_rows.load(std::memory_order_relaxed) > 0) return KERNEL_NIBBLE;     // pinned
     if (mm && mm_min_rows() > 0) return KERNEL_MMA;                                         // pinned
-    if (nb && mm) {
-        const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
-        return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
+    const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
+    // int8 sums are exact in fp32 while K * 128 stays within 2^24
+    if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
+        if (rows <= 8) return KERNEL_BITS;
+        if (rows > 8 * BT_MAX_ROWS) return KERNEL_MMA;
+        return bt_model_us(entries, x_dtype, rows) <= mm_tiles_model_us(w, mm_direct(w, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
+    if (nb && mm) return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
     return nb ? KERNEL_NIBBLE : (mm ? KERNEL_MMA : KERNEL_GATHER);
 }
 
@@ -625,6 +808,17 @@ int run_gather(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_l
     return TLLM_OK;
 }
 
+// the product of `rows` rows on the kernel that choose_kernel names
+int run_product(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
+                float scale2, cudaStream_t st) {
+    switch (choose_kernel(w, X, x_dtype, x_layout, x_ld, rows)) {
+        case KERNEL_BITS: return run_bits(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
+        case KERNEL_NIBBLE: return run_nb(w, X, x_dtype, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
+        case KERNEL_MMA: return run_mm(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
+        default: return run_gather(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, Scratch{w->d_partial, w->d_counters}, st);
+    }
+}
+
 int upload(tllm_weight* w, const BsHostImage& img, float scale, int max_rows) {
     w->lay = img.lay;
     w->scale = scale;
@@ -657,8 +851,8 @@ int upload_bit_tiles(tllm_weight* w, const std::vector<uint32_t>& bits, int sms)
     w->mm_grid = sms;
     CU_TRY(cudaMalloc(&w->d_bits, w->bits_bytes));
     CU_TRY(cudaMemcpy(w->d_bits, bits.data(), w->bits_bytes, cudaMemcpyHostToDevice));
-    const size_t partial_bytes = (size_t)2 * sms * MM_TILE_N * MM_SPLIT_MAX_NT * sizeof(float);
-    const size_t counter_bytes = (size_t)w->mm_n_tiles * 4 * sizeof(unsigned int);
+    const size_t partial_bytes = (size_t)2 * sms * MM_TILE_N * MM_OWN_NT * sizeof(float);
+    const size_t counter_bytes = (size_t)w->mm_n_tiles * MM_MAX_M_TILES * 4 * sizeof(unsigned int);
     CU_TRY(cudaMalloc(&w->d_mm_partial, partial_bytes));
     CU_TRY(cudaMalloc(&w->d_mm_counters, counter_bytes));
     CU_TRY(cudaMemset(w->d_mm_counters, 0, counter_bytes));
@@ -696,6 +890,7 @@ int create_from_dense(const int8_t* dense, int inners, int columns, float scale,
     int max_rows = (opts && opts->max_rows > 0) ? opts->max_rows : 4;
     if (max_rows > 4) max_rows = 4;
     tllm_weight* w = new tllm_weight();
+    g_handles.fetch_add(1, std::memory_order_relaxed);
     rc = upload(w, img, scale, max_rows);
     if (rc == TLLM_OK && !(opts && opts->no_bit_tiles)) rc = upload_bits(w, dense, inners, columns, sms);
     if (rc == TLLM_OK && !(opts && opts->no_nibbles)) rc = upload_nibbles(w, dense, inners, columns, sms);
@@ -860,23 +1055,18 @@ int tllm_ter_spmm(const void* X, int x_dtype, int x_layout, const int16_t* row_i
     if (batch > 65535) return fail(TLLM_ERR_ARG, "tllm_ter_spmm: batch too large");
     if (tllm_weight* w = ter_cache_find(row_idx, col_off, columns, inners, tile_k)) {
         // these arrays were repacked by tllm_ter_spmm_prepare: the product runs on the packed copy
-        const BsLayout& L = w->lay;
         cudaStream_t st = (cudaStream_t)stream;
         const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
         if (x_layout == TLLM_ROW_MAJOR) {
             const long long m = (long long)batch * rows;      // the batch is contiguous: one product of batch * rows rows
             if (m > 0x7fffffffLL) return fail(TLLM_ERR_ARG, "tllm_ter_spmm: batch * rows too large");
-            const KernelChoice kc = choose_kernel(w, X, x_dtype, x_layout, inners, (int)m);
-            if (kc == KERNEL_NIBBLE) return run_nb(w, X, x_dtype, inners, (int)m, Y, y_dtype, columns, 0, scale, 0.f, st);
-            if (kc == KERNEL_MMA) return run_mm(w, X, x_dtype, inners, (int)m, Y, y_dtype, columns, 0, scale, 0.f, st);
-            return run_gather(w, X, x_dtype, x_layout, inners, (int)m, Y, y_dtype, columns, 0, scale, 0.f, Scratch{w->d_partial, w->d_counters}, st);
+            return run_product(w, X, x_dtype, x_layout, inners, (int)m, Y, y_dtype, columns, 0, scale, 0.f, st);
         }
         for (int b = 0; b < batch; ++b) {
-            const int rc2 = run_gather(w, (const char*)X + (size_t)b * rows * inners * xe, x_dtype, x_layout, rows, rows,
-                                       (char*)Y + (size_t)b * rows * columns * ye, y_dtype, columns, 0, scale, 0.f, Scratch{w->d_partial, w->d_counters}, st);
+            const int rc2 = run_product(w, (const char*)X + (size_t)b * rows * inners * xe, x_dtype, x_layout, rows, rows,
+                                        (char*)Y + (size_t)b * rows * columns * ye, y_dtype, columns, 0, scale, 0.f, st);
             if (rc2) return rc2;
         }
-        (void)L;
         return TLLM_OK;
     }
     constexpr int MC = 4;
@@ -968,6 +1158,7 @@ int tllm_weight_destroy(tllm_weight* w) {
     if (w->h_status) cudaFreeHost(w->h_status);
     if (w->own_stream) cudaStreamDestroy(w->own_stream);
     delete w;
+    if (g_handles.fetch_sub(1, std::memory_order_relaxed) == 1) ws_trim();
     return TLLM_OK;
 }
 
@@ -988,7 +1179,7 @@ int tllm_weight_get_info(const tllm_weight* w, tllm_weight_info* info) {
 // ---- packed-weight files: header, column ranges, block descriptors, index stream, block tables, bit tiles ----------
 namespace {
 struct WeightFileHeader {
-    char magic[8];                // "TLLMW002"
+    char magic[8];                // "TLLMW003"; "TLLMW002" files hold the bit tiles in another order
     int32_t inners, columns, tile_rows, tiles, col_blocks, k_splits, tiles_per_cta, num_ctas, max_cols_per_block, max_rows, mm_n_tiles, mm_kb;
     int64_t nnz, total_vecs, units, meta_words, bits_words;
     float scale;
@@ -1002,7 +1193,7 @@ int tllm_weight_save(const tllm_weight* w, const char* path) {
     if (!w || !path) return fail(TLLM_ERR_ARG, "tllm_weight_save: NULL argument");
     const BsLayout& L = w->lay;
     WeightFileHeader h{};
-    std::memcpy(h.magic, "TLLMW002", 8);
+    std::memcpy(h.magic, "TLLMW003", 8);
     h.inners = L.inners, h.columns = L.columns, h.tile_rows = L.tile_rows, h.tiles = L.tiles, h.col_blocks = L.col_blocks;
     h.k_splits = L.k_splits, h.tiles_per_cta = L.tiles_per_cta, h.num_ctas = L.num_ctas, h.max_cols_per_block = L.max_cols_per_block;
     h.max_rows = w->max_rows, h.mm_n_tiles = w->mm_n_tiles, h.mm_kb = w->mm_kb;
@@ -1035,7 +1226,7 @@ int tllm_weight_load(const char* path, tllm_weight** out) {
     WeightFileHeader h{};
     BsHostImage img;
     std::vector<uint32_t> bits;
-    bool ok = read_exact(f, &h, sizeof h) && std::memcmp(h.magic, "TLLMW002", 8) == 0;
+    bool ok = read_exact(f, &h, sizeof h) && (std::memcmp(h.magic, "TLLMW003", 8) == 0 || std::memcmp(h.magic, "TLLMW002", 8) == 0);
     ok = ok && h.num_ctas > 0 && h.num_ctas <= BS_MAX_BLOCKS && h.col_blocks > 0 && h.col_blocks <= h.num_ctas && h.total_vecs >= 0 && h.meta_words >= 0 &&
          h.bits_words >= 0 && h.total_vecs < ((int64_t)1 << 32) && h.meta_words < ((int64_t)1 << 34) && h.bits_words < ((int64_t)1 << 38);
     if (ok) {
@@ -1062,17 +1253,22 @@ int tllm_weight_load(const char* path, tllm_weight** out) {
     int rc = device_sms(&sms);
     if (rc) return rc;
     tllm_weight* w = new tllm_weight();
+    g_handles.fetch_add(1, std::memory_order_relaxed);
     rc = upload(w, img, h.scale, h.max_rows > 0 && h.max_rows <= 4 ? h.max_rows : 4);
-    if (rc == TLLM_OK && h.bits_words) {
-        w->mm_n_tiles = h.mm_n_tiles;
-        w->mm_kb = h.mm_kb;
-        rc = upload_bit_tiles(w, bits, sms);
-    }
-    if (rc == TLLM_OK) {   // the four-bit planes are not stored: they are rebuilt from the lists
-        std::vector<int8_t> dense((size_t)h.inners * h.columns);
+    // the four-bit planes are not stored, and older files keep the bit tiles in another order: both are rebuilt from the lists
+    std::vector<int8_t> dense;
+    if (rc == TLLM_OK) {
+        dense.resize((size_t)h.inners * h.columns);
         bs_unpack_dense(img, dense.data());
-        rc = upload_nibbles(w, dense.data(), h.inners, h.columns, sms);
     }
+    if (rc == TLLM_OK && h.bits_words) {
+        if (h.magic[7] == '3') {
+            w->mm_n_tiles = h.mm_n_tiles;
+            w->mm_kb = h.mm_kb;
+            rc = upload_bit_tiles(w, bits, sms);
+        } else rc = upload_bits(w, dense.data(), h.inners, h.columns, sms);
+    }
+    if (rc == TLLM_OK) rc = upload_nibbles(w, dense.data(), h.inners, h.columns, sms);
     if (rc != TLLM_OK) {
         tllm_weight_destroy(w);
         return rc;
@@ -1094,7 +1290,7 @@ int tllm_weight_check(tllm_weight* w) {
     if (st != 0) {
         cudaMemset(w->d_status, 0, sizeof(int));
         cudaMemset(w->d_counters, 0, (size_t)w->lay.col_blocks * sizeof(unsigned int));
-        if (w->d_mm_counters) cudaMemset(w->d_mm_counters, 0, (size_t)w->mm_n_tiles * 4 * sizeof(unsigned int));
+        if (w->d_mm_counters) cudaMemset(w->d_mm_counters, 0, (size_t)w->mm_n_tiles * MM_MAX_M_TILES * 4 * sizeof(unsigned int));
         if (w->d_nb_counters) cudaMemset(w->d_nb_counters, 0, (size_t)w->nb_tiles * 4 * sizeof(unsigned int));
         if (w->d_nr_counters) cudaMemset(w->d_nr_counters, 0, (size_t)w->nb_tiles * 4 * sizeof(unsigned int));
         return fail(TLLM_ERR_KERNEL, "a bounded wait ran out inside the kernel (code %d: %s)", st,
@@ -1113,11 +1309,7 @@ int tllm_spmm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows
     if (rc) return rc;
     const BsLayout& L = w->lay;
     const int x_ld = x_layout == TLLM_ROW_MAJOR ? L.inners : rows;
-    const KernelChoice kc = choose_kernel(w, X, x_dtype, x_layout, x_ld, rows);
-    if (kc == KERNEL_NIBBLE) return run_nb(w, X, x_dtype, x_ld, rows, Y, y_dtype, L.columns, 0, w->scale, 0.f, (cudaStream_t)stream);
-    if (kc == KERNEL_MMA) return run_mm(w, X, x_dtype, x_ld, rows, Y, y_dtype, L.columns, 0, w->scale, 0.f, (cudaStream_t)stream);
-    return run_gather(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, L.columns, 0, w->scale, 0.f, Scratch{w->d_partial, w->d_counters},
-                      (cudaStream_t)stream);
+    return run_product(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, L.columns, 0, w->scale, 0.f, (cudaStream_t)stream);
 }
 
 int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows, const void* bias, void* Y, int y_dtype, int y_layout) {
@@ -1322,17 +1514,9 @@ int tllm_mlp_forward_ex(tllm_mlp* m, const void* X, int x_dtype, int rows, void*
     char* h = (char*)(H ? H : m->d_h);
     cudaStream_t st = (cudaStream_t)stream;
     // the two products pick their kernel independently (gate and up share the first one: its epilogue applies SiLU and the product)
-    const KernelChoice k1 = choose_kernel(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows);
-    if (k1 == KERNEL_NIBBLE) rc = run_nb(m->gate_up, X, x_dtype, m->hidden, rows, h, x_dtype, m->inter, 1, m->s_gate, m->s_up, st);
-    else if (k1 == KERNEL_MMA) rc = run_mm(m->gate_up, X, x_dtype, m->hidden, rows, h, x_dtype, m->inter, 1, m->s_gate, m->s_up, st);
-    else rc = run_gather(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows, h, x_dtype, m->inter, 1, m->s_gate, m->s_up,
-                         Scratch{m->gate_up->d_partial, m->gate_up->d_counters}, st);
+    rc = run_product(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows, h, x_dtype, m->inter, 1, m->s_gate, m->s_up, st);
     if (rc) return rc;
-    const KernelChoice k2 = choose_kernel(m->down, h, x_dtype, TLLM_ROW_MAJOR, m->inter, rows);
-    if (k2 == KERNEL_NIBBLE) return run_nb(m->down, h, x_dtype, m->inter, rows, Y, y_dtype, m->hidden, 0, m->down->scale, 0.f, st);
-    if (k2 == KERNEL_MMA) return run_mm(m->down, h, x_dtype, m->inter, rows, Y, y_dtype, m->hidden, 0, m->down->scale, 0.f, st);
-    return run_gather(m->down, h, x_dtype, TLLM_ROW_MAJOR, m->inter, rows, Y, y_dtype, m->hidden, 0, m->down->scale, 0.f,
-                      Scratch{m->down->d_partial, m->down->d_counters}, st);
+    return run_product(m->down, h, x_dtype, TLLM_ROW_MAJOR, m->inter, rows, Y, y_dtype, m->hidden, 0, m->down->scale, 0.f, st);
 }
 
 // [a][b] -> [b][a] for elements of `e` bytes

@@ -133,17 +133,6 @@ __device__ __forceinline__ void nb_emit_pieces(uint32_t (&hw)[8], int n, F dst) 
     }
 }
 
-// true in exactly one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xFFFFFFFF;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred != 0;
-}
-
 #ifdef NB_DEBUG
 __device__ long long* g_nb_trace = nullptr;
 #define NB_STAMP(slot)                                               \

@@ -395,19 +395,29 @@ extern "C" int tllm_ternarize(const float* w, int inners, int columns, float thr
 void mm_pack_bits(const int8_t* w, int inners, int columns, std::vector<uint32_t>* bits, int* n_tiles, int* kb_out) {
     const int NT = (columns + 127) / 128, KB = (inners + 63) / 64;
     bits->assign((size_t)NT * KB * 128 * 4, 0u);
-    for (int kb = 0; kb < KB; ++kb) {
-        const int k1 = std::min(inners, (kb + 1) * 64);
-        for (int k = kb * 64; k < k1; ++k) {
-            const int kl = k - kb * 64, word = kl >> 4, bit = mm_code_bit(kl & 15);
-            const int8_t* row = w + (size_t)k * columns;
-            for (int n = 0; n < columns; ++n) {
-                const int8_t v = row[n];
-                if (!v) continue;
-                const size_t rec = ((size_t)(n >> 7) * KB + kb) * 128 + (n & 127);
-                (*bits)[rec * 4 + word] |= (v > 0 ? 1u : 2u) << bit;
+    uint32_t* out = bits->data();
+    std::atomic<int> next{0};
+    // one tile of 128 columns at a time: its words are private to the thread that builds them
+    auto work = [&]() {
+        for (;;) {
+            const int nt = next.fetch_add(1);
+            if (nt >= NT) return;
+            const int n0 = nt * 128, n1 = std::min(columns, n0 + 128);
+            for (int k = 0; k < inners; ++k) {
+                const int kb = k >> 6, t = (k >> 4) & 3, bit = mm_code_bit(k & 15);
+                const int8_t* row = w + (size_t)k * columns;
+                for (int n = n0; n < n1; ++n) {
+                    const int8_t v = row[n];
+                    if (v) out[mm_word_index(n, kb, t, KB)] |= (v > 0 ? 1u : 3u) << bit;
+                }
             }
         }
-    }
+    };
+    const unsigned nthreads = std::min<unsigned>(std::max(1u, std::min(std::thread::hardware_concurrency(), 32u)), (unsigned)NT);
+    std::vector<std::thread> pool;
+    for (unsigned i = 1; i < nthreads; ++i) pool.emplace_back(work);
+    work();
+    for (std::thread& th : pool) th.join();
     *n_tiles = NT;
     *kb_out = KB;
 }
@@ -415,11 +425,10 @@ void mm_pack_bits(const int8_t* w, int inners, int columns, std::vector<uint32_t
 void mm_unpack_bits(const std::vector<uint32_t>& bits, int inners, int columns, int8_t* w) {
     const int KB = (inners + 63) / 64;
     for (int k = 0; k < inners; ++k) {
-        const int kb = k >> 6, kl = k & 63, word = kl >> 4, bit = mm_code_bit(kl & 15);
+        const int kb = k >> 6, t = (k >> 4) & 3, bit = mm_code_bit(k & 15);
         for (int n = 0; n < columns; ++n) {
-            const size_t rec = ((size_t)(n >> 7) * KB + kb) * 128 + (n & 127);
-            const uint32_t c = (bits[rec * 4 + word] >> bit) & 3u;
-            w[(size_t)k * columns + n] = c == 1 ? 1 : c == 2 ? -1 : 0;
+            const uint32_t c = (bits[mm_word_index(n, kb, t, KB)] >> bit) & 3u;
+            w[(size_t)k * columns + n] = c == 1 ? 1 : c == 3 ? -1 : 0;
         }
     }
 }

@@ -1,0 +1,64 @@
+"""The batched tensor-core product on every form of activations (csrc/mma_kernel.cuh): fp32 as three bf16 planes, int8 as fp16,
+column-major and unaligned rows, at row counts around the edges of its row tiles; tiles that many blocks share.
+
+Exact on integers (sums below 2^24); on N(0,1) within 1e-5 of the largest output, the bound of the other tensor-core kernels
+(fp32 sums of exact products).
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from conftest import random_ternary
+from ternaryllm_b200 import PackedMLP, PackedWeight
+
+pytestmark = pytest.mark.gpu
+DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16, "i8": torch.int8}
+
+
+@pytest.mark.parametrize("dtype", list(DT))
+@pytest.mark.parametrize("K,N,s", [(40, 17, 0.3), (64, 130, 0.5), (1003, 517, 0.6), (4100, 128, 0.5)])
+def test_exact_on_integer_activations(K, N, s, dtype):
+    rng = np.random.default_rng(K + N)
+    w = random_ternary(rng, K, N, s)
+    pw = PackedWeight.from_dense(w)
+    top = {"f32": 512, "f16": 512, "bf16": 127, "i8": 127}[dtype]
+    for M in (129, 257, 300, 1200):
+        xs = rng.integers(-top, top + 1, size=(M, K)).astype(np.float64)
+        X = torch.tensor(xs, dtype=DT[dtype], device="cuda")
+        out = torch.full((M, N), -1, dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+        want = oracle.dense_f64(xs, w)
+        assert np.array_equal(pw.matmul(X, out=out).double().cpu().numpy(), want), M
+        out.fill_(-1)
+        assert np.array_equal(pw.matmul(X.t().contiguous(), out=out, col_major=True).double().cpu().numpy(), want), M
+    pw.check()
+    pw.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+def test_gaussian_activations(dtype):
+    rng = np.random.default_rng(5)
+    K, N = 4096, 2816
+    w = random_ternary(rng, K, N, 0.6)
+    pw = PackedWeight.from_dense(w, scale=0.03125)
+    for M in (20, 64, 200, 512):
+        X = torch.tensor(rng.standard_normal((M, K)), dtype=DT[dtype], device="cuda")
+        ref = oracle.dense_f64(X.double().cpu().numpy(), w, 0.03125)
+        Y = pw.matmul(X, out=torch.empty((M, N), dtype=torch.float32, device="cuda"))
+        assert np.max(np.abs(Y.double().cpu().numpy() - ref)) <= 1e-5 * np.max(np.abs(ref)), M
+    pw.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("hidden,inter", [(520, 1416), (768, 1027)])
+def test_fused_mlp(dtype, hidden, inter):
+    rng = np.random.default_rng(6)
+    wg, wu, wd = (random_ternary(rng, *shape, 0.6) for shape in ((hidden, inter), (hidden, inter), (inter, hidden)))
+    mlp = PackedMLP(wg, wu, wd, 0.021, 0.034, 0.027)
+    for M in (40, 130, 300):
+        X = torch.tensor(rng.standard_normal((M, hidden)), dtype=DT[dtype], device="cuda")
+        ref = oracle.mlp_f64(X.double().cpu().numpy(), wg, wu, wd, 0.021, 0.034, 0.027, h_round={"f32": 3, "f16": 1, "bf16": 2}[dtype])
+        err = np.max(np.abs(mlp.forward(X).double().cpu().numpy() - ref)) / np.max(np.abs(ref))
+        # fp32 sums, and up to one last place of the type in h and in the result
+        assert err <= 1e-5 + {"f32": 2.0 ** -22, "f16": 2.0 ** -10, "bf16": 2.0 ** -7}[dtype], (M, err)
+    mlp.close()

@@ -1,0 +1,74 @@
+"""The register-decode product (two-bit tiles of W decoded into mma.sync fragments, csrc/bits_kernel.cuh) against the
+oracle, through the calls that reach it by default: few activation rows of any type and layout.
+
+Integer-valued activations are exact (products and partial sums are integers below 2^24); on N(0,1) the fp32 sums of
+exact products stay within 1e-5 of the largest output, the bound the other tensor-core kernels are held to.
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from conftest import random_ternary
+from ternaryllm_b200 import PackedMLP, PackedWeight
+
+pytestmark = pytest.mark.gpu
+DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16, "i8": torch.int8}
+
+# one slice, an odd last slice, K and N multiples of nothing (rows of X on odd addresses), fewer pairs of slices than
+# warps, several passes per block (more than eight groups of sixteen columns per SM)
+SHAPES = [(1, 1, 0.0), (40, 17, 0.3), (64, 16, 0.5), (77, 5, 0.3), (192, 48, 0.5), (1003, 517, 0.6), (1000, 70, 0.6), (2056, 386, 0.9), (4099, 33, 0.5), (520, 21000, 0.5)]
+
+
+@pytest.mark.parametrize("dtype", list(DT))
+@pytest.mark.parametrize("K,N,s", SHAPES)
+def test_exact_on_integer_activations(K, N, s, dtype):
+    rng = np.random.default_rng(K + N)
+    w = random_ternary(rng, K, N, s)
+    pw = PackedWeight.from_dense(w)
+    top = {"f32": 512, "f16": 512, "bf16": 127, "i8": 127}[dtype]
+    for M in (1, 2, 3, 7, 8, 9, 16, 17, 32):
+        xs = rng.integers(-top, top + 1, size=(M, K)).astype(np.float64)
+        X = torch.tensor(xs, dtype=DT[dtype], device="cuda")
+        out = torch.full((M, N), -1, dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+        want = oracle.dense_f64(xs, w)
+        assert np.array_equal(pw.matmul(X, out=out).double().cpu().numpy(), want), M
+        out.fill_(-1)
+        assert np.array_equal(pw.matmul(X.t().contiguous(), out=out, col_major=True).double().cpu().numpy(), want), M
+        # rows that start inside a wider buffer, on an address that is a multiple of the element size only
+        buf = torch.zeros(M * K + 1, dtype=DT[dtype], device="cuda")
+        buf[1:] = X.reshape(-1)
+        assert np.array_equal(pw.matmul(buf[1:].view(M, K), out=out).double().cpu().numpy(), want), M
+    pw.check()
+    pw.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+def test_gaussian_activations_and_result_types(dtype):
+    rng = np.random.default_rng(5)
+    K, N, s = 4096, 2816, 0.6
+    w = random_ternary(rng, K, N, s)
+    pw = PackedWeight.from_dense(w, scale=0.03125)
+    for M in (1, 5, 16, 32):
+        X = torch.tensor(rng.standard_normal((M, K)), dtype=DT[dtype], device="cuda")
+        ref = oracle.dense_f64(X.double().cpu().numpy(), w, 0.03125)
+        Y = pw.matmul(X, out=torch.empty((M, N), dtype=torch.float32, device="cuda"))
+        assert np.max(np.abs(Y.double().cpu().numpy() - ref)) <= 1e-5 * np.max(np.abs(ref))
+        eps = {"f32": 2.0 ** -23, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dtype]          # one rounding to the result's type
+        assert np.max(np.abs(pw.matmul(X).double().cpu().numpy() - ref)) <= (1e-5 + eps) * np.max(np.abs(ref))
+    pw.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+def test_fused_mlp(dtype):
+    rng = np.random.default_rng(6)
+    hidden, inter = 520, 1416
+    wg, wu, wd = (random_ternary(rng, *shape, 0.6) for shape in ((hidden, inter), (hidden, inter), (inter, hidden)))
+    mlp = PackedMLP(wg, wu, wd, 0.021, 0.034, 0.027)
+    for M in (1, 8, 13):
+        X = torch.tensor(rng.standard_normal((M, hidden)), dtype=DT[dtype], device="cuda")
+        ref = oracle.mlp_f64(X.double().cpu().numpy(), wg, wu, wd, 0.021, 0.034, 0.027, h_round={"f32": 3, "f16": 1, "bf16": 2}[dtype])
+        err = np.max(np.abs(mlp.forward(X).double().cpu().numpy() - ref)) / np.max(np.abs(ref))
+        # fp32 sums, and up to one last place of the type in h and in the result
+        assert err <= 1e-5 + {"f32": 2.0 ** -22, "f16": 2.0 ** -10, "bf16": 2.0 ** -7}[dtype], (M, err)
+    mlp.close()
