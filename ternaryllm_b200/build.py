@@ -18,7 +18,7 @@ SOURCES = ["capi.cu", "bits.cu", "comm.cu", "packer.cpp", "bstream_pack.cpp", "s
 DEPS = ["kernels.cuh", "bits_kernel.cuh", "mma_kernel.cuh", "bstream_kernel.cuh", "nibble_kernel.cuh", "nibble_rows_kernel.cuh", "nibble_format.h", "bstream_format.h", "bittile_format.h", "column_lists.h", "util.h", os.path.join("..", "..", "include", "tllm.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC,-O2", "--shared", "-Xptxas", "-v", "-t", "0", "-split-compile=0",
+    "-Xcompiler", "-fPIC,-O2", "--shared", "-Xptxas", "-v", "-t", "0",
 ]
 
 BINDING = os.path.join(HERE, "_binding.so")

@@ -127,12 +127,12 @@ PyObject* matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     BINDING_CATCH
 }
 
-// mlp_forward(handle, x, out | None, h | None, hidden, inter) -> tensor
+// mlp_forward(handle, x, out | None, h | None, hidden) -> tensor
 PyObject* mlp_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-    NEED_ARGS(6, "mlp_forward")
+    NEED_ARGS(5, "mlp_forward")
     BINDING_TRY
-    long long handle, hidden, inter;
-    if (!int_of(a[0], &handle) || !int_of(a[4], &hidden) || !int_of(a[5], &inter)) return nullptr;
+    long long handle, hidden;
+    if (!int_of(a[0], &handle) || !int_of(a[4], &hidden)) return nullptr;
     const at::Tensor* xp = tensor_of(a[1]);
     if (!xp || !xp->is_cuda() || xp->dim() != 2 || xp->size(1) != hidden) return raise("PackedMLP.forward expects a 2-D CUDA activation [rows, hidden]");
     at::Tensor xc;
@@ -160,8 +160,6 @@ PyObject* mlp_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const at::Tensor* hp = tensor_of(a[3]);
         if (!hp) return raise("h must be a tensor");
         h = *hp;
-    } else if (rows > 16) {
-        h = at::empty({rows, inter}, xp->options());
     }
     void* st = c10::cuda::getCurrentCUDAStream(xp->get_device()).stream();
     const void* X = xp->const_data_ptr();
@@ -245,7 +243,7 @@ PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
 PyMethodDef methods[] = {
     {"matmul", (PyCFunction)(void (*)(void))matmul, METH_FASTCALL, "matmul(handle, x, out, col_major, device, inners, columns)"},
-    {"mlp_forward", (PyCFunction)(void (*)(void))mlp_forward, METH_FASTCALL, "mlp_forward(handle, x, out, h, hidden, inter)"},
+    {"mlp_forward", (PyCFunction)(void (*)(void))mlp_forward, METH_FASTCALL, "mlp_forward(handle, x, out, h, hidden)"},
     {"ter_spmm", (PyCFunction)(void (*)(void))ter_spmm, METH_FASTCALL,
      "ter_spmm(X, row_idx, col_off, tile_idx, batch, rows, columns, inners, uniformed, padded, scale, out, tile_k)"},
     {nullptr, nullptr, 0, nullptr}};

@@ -250,12 +250,14 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
         wsrc = (const char*)p.bits + (size_t)(c0 + fpass + a) * group_bytes + (size_t)kw * 512u;
         last = (uint32_t)max(e - a - 1, 0) * group_bytes;
     };
+    const uint32_t wchunk = (uint32_t)mm_chunk(g, t) * 16u;          // where this lane's chunk of a pair lies
     auto copy_w = [&](uint32_t slot) {
-        const uint32_t dst = slot + (uint32_t)lane * 16u;
+        uint32_t dst = slot + (uint32_t)lane * 16u;
         if (2 * (kw + (fi << klog)) + 2 <= KB) {
 #pragma unroll
             for (int j = 0; j < GR; ++j) cp_async16(dst + (uint32_t)j * 512u, wsrc + min((uint32_t)j * group_bytes, last) + lane * 16);
         } else {                                                     // an odd last slice
+            dst = slot + wchunk;
 #pragma unroll
             for (int j = 0; j < GR; ++j) {
                 cp_async8(dst + (uint32_t)j * 512u, wsrc + min((uint32_t)j * group_bytes, last) + lane * 8);
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                     constexpr int lo = decltype(first)::value, hi = decltype(end)::value;
                     uint2 a[GR];
 #pragma unroll
-                    for (int j = lo; j < hi; ++j) a[j] = bt_lds64(slot + (uint32_t)j * 512u + (uint32_t)lane * 16u + h * 8u);
+                    for (int j = lo; j < hi; ++j) a[j] = bt_lds64(slot + (uint32_t)j * 512u + wchunk + h * 8u);
                     // consecutive MMAs go to different accumulators: a chain of dependent ones costs their full latency each
 #pragma unroll
                     for (int s = 0; s < 4; ++s)

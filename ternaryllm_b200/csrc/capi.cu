@@ -138,6 +138,7 @@ struct tllm_weight {
     float* d_mm_partial = nullptr;
     unsigned int* d_mm_counters = nullptr;
     size_t bits_bytes = 0;
+    CUtensorMap bits_map;             // rows = groups of sixteen columns, KB * 64 words each; box = 8 groups x four slices
     int mm_n_tiles = 0, mm_kb = 0, mm_grid = 0;
     // decode tensor-core kernel: transposed four-bit copy of W, its tensor map, schedule and hand-over scratch
     uint8_t* d_nib = nullptr;
@@ -303,26 +304,26 @@ struct Workspace {
 };
 
 // How a product of `rows` rows (in `planes` planes) is cut: row tiles of Nt rows each, whole tiles or equal ranges of units, chosen
-// by an estimate in SM clocks.  An MMA of 128 x Nt x 16 takes Nt / 2 clocks of the tensor core and its operands 32 + Nt / 4 of
-// shared memory, a slice of 64 rows of W four of them per plane and never less than the 150 of its decode.  A tile's epilogue is
-// hidden behind the next one except at the end.  In a tile that `parts` blocks share the last one to arrive reads the other
-// parts, a round trip to L2 for every sixteen rows of each.
+// by an estimate in SM clocks.  A slice of 64 rows of W is four MMAs of 128 x Nt x 16 per plane, 2.4 * Nt clocks (measured) and
+// never less than the 260 of their issue.  A tile's epilogue is hidden behind the next one except at the end, or where there
+// is no room for two sets of accumulators.  In a tile
+// that `parts` blocks share the last one to arrive reads the other parts, a round trip to L2 for every sixteen rows of each, 3000 clocks in all at least.
 struct MmPlan {
     int Nt, m_tiles, split;
     double clocks;
 };
-int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_NT : MM_MAX_NT / 2; }     // two accumulators each with three planes
 MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
     MmPlan best{0, 0, 0, 0};
-    const int kbu = (kb + 1) / 2;
-    for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
+    const int kbu = (kb + MM_UK - 1) / MM_UK;
+    for (int nt = 16; nt <= MM_MAX_NT; nt += 16) {
         const int mt = (rows + nt - 1) / nt;
         if (mt > MM_MAX_M_TILES) continue;
         const double tiles = (double)n_tiles * mt, units = tiles * kbu;
-        const double slice = std::max(150.0, planes * 4 * std::max(nt / 2.0, 32.0 + nt / 4.0)), epilogue = nt / 16 * 150.0;
-        const double whole = std::ceil(tiles / sms) * kb * slice + epilogue;
+        const double slice = planes * std::max(260.0, 2.4 * nt), epilogue = nt / 16 * 500.0;
+        const bool two = (planes == 1 ? 2 : 4) * nt <= MM_A_COL;
+        const double whole = std::ceil(tiles / sms) * (kb * slice + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
-        const double split = std::ceil(units / blocks) * 2 * slice + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
+        const double split = std::ceil(units / blocks) * MM_UK * slice + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
         if (best.Nt == 0 || whole < best.clocks) best = MmPlan{nt, mt, 0, whole};
         if (split < best.clocks) best = MmPlan{nt, mt, 1, split};
         if (nt >= rows) break;
@@ -379,7 +380,7 @@ struct MmOut {
     int dtype, ld, epilogue;
     float scale, scale2;
     bool col_major;          // Y[n * ld + m]
-    bool planes;             // three bf16 planes, plane elements apart, instead of dtype
+    bool planes;             // epilogue 1: three bf16 planes, plane elements apart, instead of dtype
     long long plane;
 };
 
@@ -388,35 +389,36 @@ int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStr
     const BsLayout& L = w->lay;
     const MmPlan plan = mm_plan(rows, x.planes, w->mm_n_tiles, w->mm_kb, w->mm_grid);
     MmParams p{};
-    p.bits = w->d_bits;
     p.Y = o.Y;
     p.counters = w->d_mm_counters;
     p.status = w->d_status;
     p.M = rows, p.K = L.inners, p.N = L.columns;
-    p.KB = w->mm_kb, p.KBU = (p.KB + 1) / 2;
+    p.KB = w->mm_kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
     p.n_tiles = w->mm_n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split;
     p.P = x.planes, p.plane_rows = x.plane_rows;
-    p.y_dtype = o.dtype, p.epilogue = o.epilogue, p.y_ld = o.ld, p.y_planes = o.planes, p.plane_y = o.plane;
-    p.y_col = !o.col_major ? 0 : (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0 ? 2 : 1;
-    // Rings within 208 KiB: four units of bit tiles (eight for narrow tiles, which are bound by the stream of W), then as many
-    // units of A and B as fit; with three planes B turns over three times as fast and gets what two or three units of A leave.
-    p.R = p.Nt <= 64 ? 8 : 4;
-    const int room = 208 * 1024 - p.R * MM_UNIT_BYTES, b_unit = p.Nt * 256;
-    p.SA = x.planes == 1 ? std::min(MM_MAX_STAGES, room / (MM_A_UNIT + b_unit)) : p.Nt <= 64 ? 3 : 2;
-    p.SB = x.planes == 1 ? p.SA : std::min(MM_MAX_STAGES, (room - p.SA * MM_A_UNIT) / b_unit);
+    p.epilogue = o.epilogue, p.y_ld = o.ld, p.plane_y = o.plane;
+    p.y_step_n = o.col_major ? o.ld : 1, p.y_step_m = o.col_major ? 1 : o.ld;
+    p.out = o.planes ? MM_OUT_PLANES : o.dtype == TLLM_F32 ? MM_OUT_F32 : o.dtype == TLLM_I32 ? MM_OUT_I32 : o.dtype == TLLM_F16 ? MM_OUT_F16 : MM_OUT_BF16;
+    if (o.epilogue == 0 && !o.planes) {
+        const bool wide = o.dtype == TLLM_F32 || o.dtype == TLLM_I32;
+        if (wide && o.col_major && (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0) p.out = o.dtype == TLLM_F32 ? MM_OUT_F32_COL4 : MM_OUT_I32_COL4;
+        if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && L.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
+    }
+    // rings: four units of bit tiles, and as many of B as 192 KiB hold (three at 128 rows)
+    p.R = 4;
+    const int b_unit = p.Nt * 128 * MM_UK;
+    p.SB = std::min(MM_MAX_STAGES, 192 * 1024 / b_unit);
     p.mul4 = 4, p.mul16 = 16;
     const uint32_t fmt = x.bf16 ? 1u : 0u;
     // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B formats (bits 7-9, 10-12), both K-major,
     // N / 8 in bits 17-22, M / 16 in bits 24-28
     p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.Nt >> 3) << 17) | ((uint32_t)(MM_TILE_N >> 4) << 24);
-    p.tmem_cols = 32;
-    while (p.tmem_cols < (x.planes == 1 ? 2u : 4u) * (uint32_t)p.Nt) p.tmem_cols *= 2;
     p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
 
     CUtensorMap map;
     int rc = encode_rows_map(&map, x.base, x.bf16, L.inners, (x.planes - 1) * x.plane_rows + rows, x.pitch, p.Nt);
     if (rc) return rc;
-    const size_t smem = 1024 + (size_t)p.SA * MM_A_UNIT + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512;
+    const size_t smem = 1024 + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512;
     if (smem > 227 * 1024) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
     static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
@@ -441,19 +443,30 @@ int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStr
     cudaLaunchAttribute at[1] = {pdl_attribute()};
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, p));
+    CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, w->bits_map, p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
 }
 
+// fp32 activations that are three planes already ([3][rows][pitch / 2], pitch bytes per row)
+int run_mm_planes(tllm_weight* w, const unsigned short* planes, int plane_rows, size_t pitch, int rows, void* Y, int y_dtype, int y_ld, float scale, cudaStream_t st) {
+    const int per = MM_MAX_M_TILES * MM_MAX_NT;
+    for (int r0 = 0; r0 < rows; r0 += per) {
+        const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch}, std::min(rows - r0, per),
+                                 MmOut{(char*)Y + (size_t)r0 * y_ld * dtype_size(y_dtype), y_dtype, y_ld, 0, scale, 0.f, false, false, 0}, st);
+        if (rc) return rc;
+    }
+    return TLLM_OK;
+}
+
 // the whole product on the tensor-core kernel: activations that TMA cannot read as they are go through planes in a workspace
 int run_mm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
-           float scale2, cudaStream_t st, bool y_col = false) {
+           float scale2, cudaStream_t st, bool y_col = false, bool y_planes = false, long long plane_y = 0) {
     const int K = w->lay.inners;
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const bool direct = mm_direct(w, X, x_dtype, x_layout, x_ld);
-    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * MM_MAX_NT;
     Workspace ws;
     if (!direct) {
         const int rc = ws.take(w->device, (size_t)planes * std::min(rows, per) * stage_pad(K) * 2, st);
@@ -468,7 +481,7 @@ int run_mm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, i
             if (rc) return rc;
             a.base = ws.ptr, a.pitch = (size_t)stage_pad(K) * 2;
         }
-        const int rc = launch_mm(w, a, m, MmOut{(char*)Y + (y_col ? (size_t)r0 : (size_t)r0 * y_ld) * ye, y_dtype, y_ld, epilogue, scale, scale2, y_col, false, 0}, st);
+        const int rc = launch_mm(w, a, m, MmOut{(char*)Y + (y_col ? (size_t)r0 : (size_t)r0 * y_ld) * (y_planes ? 2 : ye), y_dtype, y_ld, epilogue, scale, scale2, y_col, y_planes, plane_y}, st);
         if (rc) return rc;
     }
     return TLLM_OK;
@@ -713,7 +726,7 @@ double bt_model_us(int64_t entries, int x_dtype, int rows) {
     return t;
 }
 double mm_tiles_model_us(const tllm_weight* w, bool direct, int x_dtype, int rows) {
-    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * MM_MAX_NT;
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
         t += 6.0 + mm_plan(std::min(rows - r0, per), planes, w->mm_n_tiles, w->mm_kb, w->mm_grid).clocks / 1800.0 + (direct ? 0.0 : 2.5);
@@ -728,6 +741,8 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
     // int8 sums are exact in fp32 while K * 128 stays within 2^24
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
+        // very sparse weights: the index lists are shorter than two bits an entry (the gather model is a fifth low at 90 % zeros)
+        if (rows <= 4 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(entries, x_dtype, rows)) return KERNEL_GATHER;
         if (rows <= 8) return KERNEL_BITS;
         if (rows > 8 * BT_MAX_ROWS) return KERNEL_MMA;
         return bt_model_us(entries, x_dtype, rows) <= mm_tiles_model_us(w, mm_direct(w, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
@@ -851,6 +866,14 @@ int upload_bit_tiles(tllm_weight* w, const std::vector<uint32_t>& bits, int sms)
     w->mm_grid = sms;
     CU_TRY(cudaMalloc(&w->d_bits, w->bits_bytes));
     CU_TRY(cudaMemcpy(w->d_bits, bits.data(), w->bits_bytes, cudaMemcpyHostToDevice));
+    if (tensor_map_encoder() != nullptr) {
+        const cuuint64_t dims[2] = {(cuuint64_t)w->mm_kb * 64, (cuuint64_t)w->mm_n_tiles * 8};
+        const cuuint64_t strides[1] = {(cuuint64_t)w->mm_kb * 256};
+        const cuuint32_t box[2] = {MM_UK * 64, 8}, estr[2] = {1, 1};
+        const CUresult cr = tensor_map_encoder()(&w->bits_map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->d_bits, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (cr != CUDA_SUCCESS) return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled (bit tiles) failed with code %d", (int)cr);
+    }
     const size_t partial_bytes = (size_t)2 * sms * MM_TILE_N * MM_OWN_NT * sizeof(float);
     const size_t counter_bytes = (size_t)w->mm_n_tiles * MM_MAX_M_TILES * 4 * sizeof(unsigned int);
     CU_TRY(cudaMalloc(&w->d_mm_partial, partial_bytes));
@@ -1508,12 +1531,28 @@ int tllm_mlp_forward_ex(tllm_mlp* m, const void* X, int x_dtype, int rows, void*
     if (y_dtype != TLLM_F32 && y_dtype != TLLM_F16 && y_dtype != TLLM_BF16) return fail(TLLM_ERR_ARG, "tllm_mlp_forward: unsupported y_dtype");
     if (rows <= 0) return fail(TLLM_ERR_ARG, "tllm_mlp_forward: rows must be positive");
     if (x_dtype != TLLM_F32 && x_dtype != TLLM_F16 && x_dtype != TLLM_BF16) return fail(TLLM_ERR_ARG, "tllm_mlp_forward: unsupported dtype");
-    if (!H && (size_t)rows * m->inter * dtype_size(x_dtype) > m->h_cap) return fail(TLLM_ERR_ARG, "tllm_mlp_forward: pass H for more than 16 rows");
     int rc = check_device(m->gate_up, "tllm_mlp_forward");
     if (rc) return rc;
-    char* h = (char*)(H ? H : m->d_h);
     cudaStream_t st = (cudaStream_t)stream;
     // the two products pick their kernel independently (gate and up share the first one: its epilogue applies SiLU and the product)
+    Workspace ws;
+    if (!H && x_dtype == TLLM_F32 && choose_kernel(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows) == KERNEL_MMA &&
+        choose_kernel(m->down, X, x_dtype, TLLM_ROW_MAJOR, m->inter, rows) == KERNEL_MMA) {
+        // the intermediate result goes from one kernel to the other as the three planes that the second one reads
+        const int ld = (m->inter + 7) / 8 * 8;
+        rc = ws.take(m->gate_up->device, (size_t)3 * rows * ld * 2, st);
+        if (rc) return rc;
+        rc = run_mm(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows, ws.ptr, x_dtype, ld, 1, m->s_gate, m->s_up, st, false, true, (long long)rows * ld);
+        if (rc) return rc;
+        return run_mm_planes(m->down, (const unsigned short*)ws.ptr, rows, (size_t)ld * 2, rows, Y, y_dtype, m->hidden, m->down->scale, st);
+    }
+    char* h = (char*)(H ? H : m->d_h);
+    const size_t h_bytes = (size_t)rows * m->inter * dtype_size(x_dtype);
+    if (!H && h_bytes > m->h_cap) {
+        rc = ws.take(m->gate_up->device, h_bytes, st);
+        if (rc) return rc;
+        h = (char*)ws.ptr;
+    }
     rc = run_product(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows, h, x_dtype, m->inter, 1, m->s_gate, m->s_up, st);
     if (rc) return rc;
     return run_product(m->down, h, x_dtype, TLLM_ROW_MAJOR, m->inter, rows, Y, y_dtype, m->hidden, 0, m->down->scale, 0.f, st);

@@ -1,9 +1,13 @@
 // mma_kernel.cuh -- the batched product on the tcgen05 tensor cores of sm_100a.
 //
 // The two-bit copy of W ("bit tiles") is expanded one slice of 128 columns x 64 rows at a time into fp16 / bf16 values in
-// shared memory and multiplied on the tensor cores:  D[n, m] = sum_k Wt[n, k] * X[m, k],  A = Wt slice (K-major, 128-byte
-// swizzle, written by decoder warps), B = X slice (K-major, the same swizzle, written by TMA), D in tensor memory (fp32).
-// The ternary values are exact in both formats and products are exact; sums are accumulated in fp32.
+// tensor memory and multiplied on the tensor cores:  D[n, m] = sum_k Wt[n, k] * X[m, k],  A = Wt slice (tensor memory, written
+// by decoder warps with tcgen05.st), B = X slice (shared memory, K-major, 128-byte swizzle, written by TMA), D in tensor
+// memory (fp32).  The ternary values are exact in both formats and products are exact; sums are accumulated in fp32.
+//
+// Why tensor memory for A: with the expanded slice in shared memory a slice of 64 rows and Nt activation rows moved
+// 32 KiB of A (written and read) and Nt * 256 bytes of B through a shared memory of 128 bytes per clock -- 768 clocks at
+// Nt = 256 for the 512 that the MMAs take, 320 for 64 at Nt = 32.  Without A it is Nt * 2 clocks beside MMAs of Nt * 2.
 //
 // X comes in one or three planes of 16-bit values.  fp16 / bf16 activations whose rows TMA can address are read where they
 // are (one plane).  Everything else passes through stage_acts_kernel: int8 becomes fp16 (exact), rows on odd addresses and
@@ -13,15 +17,17 @@
 // every step would cut bits (1e-5 of the result at K = 4096, against 1e-7).
 //
 // One persistent block per SM, twenty-three warps:
-//   warp 0        streams this block's range of bit tiles into a shared-memory ring (bulk copies)
+//   warp 0        streams this block's range of bit tiles into a shared-memory ring (TMA)
 //   warp 1        owns tensor memory and issues tcgen05.mma (one lane)
 //   warps 2..5    epilogue: tensor memory -> registers -> Y (or partial sums)
 //   warp 6        loads the activation slices by TMA
-//   warps 7..22   decoders: bit tile -> swizzled fp16 / bf16 slices (two groups of eight warps, alternate units; with four
-//                 warps a group the latency of load -> decode -> store -> fence, 1500 clocks a unit, set the pace)
-// A unit is two consecutive slices of K: one hand-over between the roles for eight MMAs.  (With one for four the barriers, not
-// the tensor core, set the pace: 244 against 159 us without any of them at 5120 x 15360, 2048 rows.)  A has a ring of
-// units, B one of (unit, plane); with one plane they are the same ring and one commit frees both.
+//   warps 7..22   decoders: bit tile -> tensor memory, one slice of 32 columns per warp and unit (a warp can only write the 32
+//                 lanes of tensor memory that its number modulo 4 selects)
+// A unit is four consecutive slices of K: the issuer's waits, commits and loop cost 500 clocks whatever it issues in between, and an
+// MMA 40 to issue, so that sixteen MMAs of 128 x 128 x 16 (1270 clocks) hide it and eight do not (measured at 5120 x 15360, 2048
+// rows: 285 us with two slices per unit, 183 with the MMAs alone).  A has a ring of two units (256 columns of tensor memory;
+// the accumulators have the other 256: two of them where they fit, so that the epilogue of one tile runs beside the next),
+// B one of (unit, plane).
 // Work is either whole output tiles or, where those would leave SMs idle, the flattened list of (output tile, unit) pairs
 // cut into equal contiguous ranges, one per block.  Tiles that straddle two or more blocks are summed in block order by the
 // last block to arrive, which makes the result independent of scheduling; a block does its two shared tiles first, so that
@@ -37,38 +43,47 @@
 namespace tllm {
 
 #define MM_TILE_N 128                 // output columns per tile  (the MMA's M)
-#define MM_TILE_K 64                  // rows of W per slice      (four MMAs of K = 16); a unit is two slices
-#define MM_UNIT_BYTES 4096            // bit tiles of one unit: eight groups of sixteen columns, 512 bytes each
-#define MM_A_BYTES (MM_TILE_N * MM_TILE_K * 2)
-#define MM_A_UNIT (2 * MM_A_BYTES)
+#define MM_TILE_K 64                  // rows of W per slice      (four MMAs of K = 16); a unit is four slices
+#define MM_UNIT_BYTES 8192            // bit tiles of one unit: eight groups of sixteen columns, 1024 bytes each
+#define MM_UK 4
+#define MM_A_UNITS 2                  // ring of expanded units in tensor memory: 128 columns each, behind 256 columns of accumulators
+#define MM_A_COL 256
 #define MM_MAX_STAGES 8
 #define MM_THREADS (23 * 32)
-#define MM_MAX_NT 256                 // activation rows per tile (the MMA's N), a multiple of sixteen; half of it with three planes
+#define MM_MAX_NT 128                 // activation rows per tile (the MMA's N), a multiple of sixteen
 #define MM_OWN_NT 64                  // a handle's own hand-over scratch is for tiles of up to this many rows
 #define MM_MAX_M_TILES 16             // row tiles of one launch
+// what a result is stored as
+#define MM_OUT_F32 0
+#define MM_OUT_I32 1
+#define MM_OUT_F16 2
+#define MM_OUT_BF16 3
+#define MM_OUT_F16_PAIRS 4            // row-major, whole tiles of columns, rows on 4 bytes: two columns per store
+#define MM_OUT_BF16_PAIRS 5
+#define MM_OUT_F32_COL4 6             // column-major on 16 bytes: four rows per store
+#define MM_OUT_I32_COL4 7
+#define MM_OUT_PLANES 8               // the three bf16 values that add up to an fp32 result (see stage_acts_kernel)
 #define MM_ERR_WAIT 3                 // status word: a bounded wait of the tensor-core kernel ran out
 
 struct MmParams {
-    const uint4* bits;        // bit tiles: groups of sixteen columns, KB slices of 256 bytes each (bittile_format.h)
     void* Y;
     float* partial;           // [2 * gridDim.x][Nt / 4][128][4] fp32: a block's first and last (partial) tile
     unsigned int* counters;   // [tiles][4], zero between launches
     int* status;
     int M, K, N;
     int KB;                   // ceil(K / 64): slices
-    int KBU;                  // ceil(KB / 2): units per tile
+    int KBU;                  // ceil(KB / 4): units per tile
     int n_tiles, m_tiles;
     int Nt;                   // activation rows per tile
     int split;                // 1: equal unit ranges, tiles may be shared; 0: whole tiles
     int P, plane_rows;        // planes of X; rows from one plane to the next in the tensor map
-    int y_dtype, epilogue, y_ld;
-    int y_col;                // 1: Y is column-major, y_ld elements from column to column (epilogue 0); 2: and 16-byte stores reach it
-    int y_planes;             // 1: Y is three planes of bf16 (the pieces of an fp32 result), plane_y elements apart
-    long long plane_y;
-    int SA, SB, R;            // ring lengths: units of A, (unit, plane) pairs of B (SA = SB with one plane), units of bit tiles
+    int out;                  // MM_OUT_*
+    int epilogue, y_ld;       // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
+    long long y_step_n, y_step_m;   // elements from column to column and from row to row (epilogue 0)
+    long long plane_y;        // MM_OUT_PLANES: elements from plane to plane
+    int SB, R;                // ring lengths: (unit, plane) pairs of B, units of bit tiles
     uint32_t idesc;           // tcgen05 instruction descriptor
     uint32_t mul4, mul16;     // 4 and 16
-    uint32_t tmem_cols;       // power of two >= 2 * Nt (4 * Nt with three planes)
     float scale, scale2;      // half the product's scales: the decoded weights are 0 / +-2
 };
 
@@ -82,15 +97,29 @@ __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], issued by one thread
-__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem], issued by one thread; A: lane = row, 32-bit column c = values 2c, 2c + 1 of K.  B is given by the
+// low word of its shared-memory descriptor (start address >> 4; the upper word -- K-major, 128-byte swizzle, eight-row
+// groups 1024 bytes apart, version 1 -- is a constant).
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "mov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "r"(b_lo | (1u << 16)), "r"(idesc), "r"(accumulate), "r"(0x40004040u)
         : "memory");
 }
+// 32 columns of the calling warp's 32 lanes
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
+        "%23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+        "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]),
+        "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // the barrier receives one arrival when every MMA issued so far by this thread has completed
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -112,15 +141,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
-// Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes, groups of
-// eight rows 1024 bytes apart (stride byte offset), descriptor version 1, layout type 2 (SWIZZLE_128B).
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-
 // Sixteen two-bit codes -> eight words of two 16-bit floats 0 / +-2 (bittile_format.h).  The shifts are multiplications by
 // values in registers: they run on the FMA pipe beside the ANDs on the ALU pipe.
-__device__ __forceinline__ void mm_decode_word(uint32_t x, uint32_t m4, uint32_t m16, uint32_t (&o)[8]) {
+__device__ __forceinline__ void mm_decode_word(uint32_t x, uint32_t m4, uint32_t m16, uint32_t* o) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         o[2 * p] = x & 0xC000C000u;
@@ -165,13 +188,8 @@ __device__ __forceinline__ bool bounded_spin(uint32_t bar, uint32_t parity, vola
     }
 }
 
-// single-lane roles (producers, MMA issuer) spin on the non-blocking probe; warps that wait with all their
-// lanes use the blocking try_wait of bounded_wait, which parks them instead of spending issue slots
-#define MM_WAIT(bar, par)                                   \
-    do {                                                    \
-        if (!bounded_spin((bar), (par), abort_flag)) goto done; \
-    } while (0)
-#define MM_WAIT_BLOCK(bar, par)                             \
+// waiting roles are parked (bounded_wait): spinning ones took issue slots from the epilogue
+#define MM_WAIT(bar, par)                             \
     do {                                                    \
         if (!bounded_wait((bar), (par), abort_flag)) goto done; \
     } while (0)
@@ -195,6 +213,9 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// column (of the 32 of a quarter tile) that lane `lane` of tensor memory's quarter holds
+__device__ __forceinline__ int mm_column(int lane) { return ((lane >> 1) & 1) * 16 + (lane & 1) * 8 + (lane >> 2); }
+
 // The segments of a block's unit range [u0, u1): one per output tile it touches; the first and the last, which other blocks may
 // share, come first.
 struct MmSegs {
@@ -210,7 +231,104 @@ struct MmSegs {
     }
 };
 
-__global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ MmParams p) {
+// ---- results: sixteen rows m .. m+15 of column n, called by whole warps.  The kind of store is looked at once per sixteen
+// rows and the stores of a kind are straight-line code: with the choice inside the loop a store took 220 to 390 clocks, and a
+// tile of 128 rows spent longer in its epilogue than in its MMAs.
+template <bool BF16>
+__device__ __forceinline__ unsigned short mm_16bit(float v) {
+    return BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+}
+template <bool BF16>
+__device__ __forceinline__ void mm_emit_16(const MmParams& p, const float (&f)[16], int n, int m) {
+    unsigned short* y = (unsigned short*)p.Y + (size_t)n * p.y_step_n + (size_t)m * p.y_step_m;
+#pragma unroll
+    for (int t = 0; t < 16; ++t)
+        if (n < p.N && m + t < p.M) y[t * p.y_step_m] = mm_16bit<BF16>(f[t] * p.scale);
+}
+// the lanes of neighbouring columns trade one value per pair of rows, so that every lane writes two adjacent columns of one row
+template <bool BF16>
+__device__ __forceinline__ void mm_emit_pairs(const MmParams& p, const float (&f)[16], int n, int m) {
+    const bool odd = n & 1;
+    unsigned short* y = (unsigned short*)p.Y + (size_t)(m + (odd ? 1 : 0)) * p.y_step_m + (n & ~1);
+#pragma unroll
+    for (int t = 0; t < 16; t += 2) {
+        const float e0 = f[t] * p.scale, e1 = f[t + 1] * p.scale;
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? e0 : e1, 4);
+        const uint32_t w = (uint32_t)mm_16bit<BF16>(odd ? got : e0) | ((uint32_t)mm_16bit<BF16>(odd ? e1 : got) << 16);
+        if (m + t + (odd ? 1 : 0) < p.M) *(uint32_t*)(y + t * p.y_step_m) = w;
+    }
+}
+__device__ __forceinline__ void mm_emit(const MmParams& p, const float (&f)[16], int n, int m) {
+    uint32_t* y = (uint32_t*)p.Y + (size_t)n * p.y_step_n + (size_t)m * p.y_step_m;
+    switch (p.out) {
+        case MM_OUT_F32:
+#pragma unroll
+            for (int t = 0; t < 16; ++t)
+                if (n < p.N && m + t < p.M) y[t * p.y_step_m] = __float_as_uint(f[t] * p.scale);
+            break;
+        case MM_OUT_I32:
+#pragma unroll
+            for (int t = 0; t < 16; ++t)
+                if (n < p.N && m + t < p.M) y[t * p.y_step_m] = (uint32_t)(int)(f[t] * 0.5f);
+            break;
+        case MM_OUT_F16: mm_emit_16<false>(p, f, n, m); break;
+        case MM_OUT_BF16: mm_emit_16<true>(p, f, n, m); break;
+        case MM_OUT_F16_PAIRS: mm_emit_pairs<false>(p, f, n, m); break;
+        case MM_OUT_BF16_PAIRS: mm_emit_pairs<true>(p, f, n, m); break;
+        default:                     // MM_OUT_F32_COL4, MM_OUT_I32_COL4
+#pragma unroll
+            for (int t = 0; t < 16; t += 4) {
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = p.out == MM_OUT_F32_COL4 ? __float_as_uint(f[t + j] * p.scale) : (uint32_t)(int)(f[t + j] * 0.5f);
+                if (n < p.N && m + t + 4 <= p.M) *(uint4*)(y + t) = make_uint4(w[0], w[1], w[2], w[3]);
+                else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (n < p.N && m + t + j < p.M) y[t + j] = w[j];
+                }
+            }
+    }
+}
+// Gate and up columns sit in neighbouring lanes: the even one takes row t, the odd one row t + 1.
+__device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)[16], int n, int m) {
+    const bool odd = n & 1;
+    const int row = m + (odd ? 1 : 0);
+    const size_t at = (size_t)row * p.y_ld + (n >> 1);
+    float y[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? f[2 * t] : f[2 * t + 1], 4);
+        y[t] = silu_mul((odd ? got : f[2 * t]) * p.scale, (odd ? f[2 * t + 1] : got) * p.scale2);
+    }
+    const bool ok = (n | 1) < p.N;
+    const size_t step = 2 * (size_t)p.y_ld;
+    if (p.out == MM_OUT_F32) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            if (ok && row + 2 * t < p.M) ((float*)p.Y)[at + t * step] = y[t];
+    } else if (p.out == MM_OUT_PLANES) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            uint32_t w = __float_as_uint(y[t]);
+#pragma unroll
+            for (int pl = 0; pl < 3; ++pl) {
+                if (ok && row + 2 * t < p.M) ((unsigned short*)p.Y)[(size_t)pl * p.plane_y + at + t * step] = (unsigned short)(w >> 16);
+                w = __float_as_uint(__uint_as_float(w) - __uint_as_float(w & 0xFFFF0000u));
+            }
+        }
+    } else {
+        const bool bf = p.out == MM_OUT_BF16;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const unsigned short w = bf ? mm_16bit<true>(y[t]) : mm_16bit<false>(y[t]);
+            if (ok && row + 2 * t < p.M) ((unsigned short*)p.Y)[at + t * step] = w;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap,
+                                                                 const __grid_constant__ MmParams p) {
     extern __shared__ unsigned char mm_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -225,10 +343,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     // ---- shared memory ---------------------------------------------------------------------------------
     const uint32_t raw0 = smem_u32(mm_smem);
     const uint32_t base = (raw0 + 1023u) & ~1023u;                 // swizzled tiles need 1024-byte alignment
-    const uint32_t SA = (uint32_t)p.SA, SB = (uint32_t)p.SB, R = (uint32_t)p.R;
+    const uint32_t SB = (uint32_t)p.SB, R = (uint32_t)p.R;
     const int Nt = p.Nt;
-    const uint32_t b_slice = (uint32_t)Nt * 128u, b_unit = 2u * b_slice;
-    const uint32_t a_base = base, b_base = a_base + SA * MM_A_UNIT, r_base = b_base + SB * b_unit;
+    const uint32_t b_slice = (uint32_t)Nt * 128u, b_unit = MM_UK * b_slice;
+    const uint32_t b_base = base, r_base = b_base + SB * b_unit;
     const uint32_t bar_base = r_base + R * MM_UNIT_BYTES;
     volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 52);   // [0] tensor-memory address, [1] abort
     volatile int* abort_flag = flags + 1;
@@ -243,12 +361,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 
     if (tid == 0) {
         for (int s = 0; s < MM_MAX_STAGES; ++s) {
-            mbar_init(A_FULL(s), 8);       // the eight decoder warps of a group
+            mbar_init(A_FULL(s), 16);      // the decoder warps
             mbar_init(A_EMPTY(s), 1);      // tcgen05.commit
             mbar_init(B_FULL(s), 1);       // the TMA thread's expect_tx arrival
             mbar_init(B_EMPTY(s), 1);      // tcgen05.commit
             mbar_init(RAW_FULL(s), 1);
-            mbar_init(RAW_EMPTY(s), 8);    // the eight decoder warps of the group that took the unit
+            mbar_init(RAW_EMPTY(s), 16);   // the decoder warps
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(ACC_FULL(a), 1);
@@ -260,57 +378,63 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
-    if (warp == 1) tmem_alloc(smem_u32((const void*)flags), p.tmem_cols);
+    if (warp == 1) tmem_alloc(smem_u32((const void*)flags), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = (uint32_t)flags[0];
     const uint32_t acc_cols = p.P == 1 ? (uint32_t)Nt : 2u * (uint32_t)Nt;
+    const uint32_t accs = 2u * acc_cols <= MM_A_COL ? 2u : 1u;
     pdl_launch_dependents();
 
     // Every role walks the same list of segments.
     if (warp == 0) {
-        // ---- bit-tile producer: the weights do not depend on the preceding kernel, so this starts at once.  A tile's eight
-        // groups of sixteen columns are eight streams along K: lanes 0..7 copy one each.
+        // ---- bit-tile producer: the weights do not depend on the preceding kernel, so this starts at once.  A tile's eight groups
+        // of sixteen columns are eight streams along K; the tensor map sees them as eight rows, and one box of 8 x 1024 bytes is
+        // a unit.  (Eight bulk copies instead, one per lane, took 820 clocks a unit to issue.)
         uint32_t r = 0, rph = 0;
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
-            const char* src = (const char*)p.bits + ((size_t)(tile / p.m_tiles * 8 + (lane & 7)) * KB + (size_t)ua * 2) * 256u;
-            for (int ku = ua; ku < ub; ++ku, src += 512) {
-                if (!__all_sync(0xffffffffu, bounded_wait(RAW_EMPTY(r), rph ^ 1u, abort_flag))) goto done;
-                const uint32_t bytes = (uint32_t)min(2, KB - ku * 2) * 256u;
-                if (lane == 0) mbar_expect_tx(RAW_FULL(r), 8u * bytes);
+            const int row0 = tile / p.m_tiles * 8;
+            for (int ku = ua; ku < ub; ++ku) {
+                MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
+                if (elect_one()) {
+                    mbar_expect_tx(RAW_FULL(r), MM_UNIT_BYTES);          // past the end of K the box is filled with zeros, which count
+                    tma_load_2d(r_base + r * MM_UNIT_BYTES, &wmap, ku * (MM_UK * 64), row0, RAW_FULL(r));
+                }
                 __syncwarp();
-                if (lane < 8) bulk_g2s(r_base + r * MM_UNIT_BYTES + (uint32_t)lane * 512u, src, bytes, RAW_FULL(r));
                 MM_ADVANCE(r, rph, R);
             }
         }
     } else if (warp == 6) {
-        // ---- activation producer: a unit and plane is two TMA boxes on one barrier
-        if (lane == 0) {
-            pdl_wait();
-            uint32_t b = 0, bph = 0;
-            for (int i = 0; i < segs.n; ++i) {
-                int tile, ua, ub, sl;
-                segs.get(i, tile, ua, ub, sl);
-                const int row0 = (tile % p.m_tiles) * Nt;
-                for (int ku = ua; ku < ub; ++ku) {
-                    const int nk = min(2, KB - ku * 2);
-                    for (int pl = 0; pl < p.P; ++pl) {
-                        MM_WAIT(p.P == 1 ? A_EMPTY(b) : B_EMPTY(b), bph ^ 1u);
+        // ---- activation producer: a unit and plane is four TMA boxes on one barrier (whole warp converged, one elected lane per
+        // instruction: addresses and coordinates then are warp-uniform values)
+        pdl_wait();
+        uint32_t b = 0, bph = 0;
+        for (int i = 0; i < segs.n; ++i) {
+            int tile, ua, ub, sl;
+            segs.get(i, tile, ua, ub, sl);
+            const int row0 = (tile % p.m_tiles) * Nt;
+            for (int ku = ua; ku < ub; ++ku) {
+                const int nk = min(MM_UK, KB - ku * MM_UK);
+                for (int pl = 0; pl < p.P; ++pl) {
+                    MM_WAIT(B_EMPTY(b), bph ^ 1u);
+                    if (elect_one()) {
                         mbar_expect_tx(B_FULL(b), (uint32_t)nk * b_slice);
-                        for (int h = 0; h < nk; ++h)
-                            tma_load_2d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * 2 + h) * MM_TILE_K, pl * p.plane_rows + row0, B_FULL(b));
-                        MM_ADVANCE(b, bph, SB);
+#pragma unroll
+                        for (int h = 0; h < MM_UK; ++h)
+                            if (h < nk) tma_load_2d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * MM_UK + h) * MM_TILE_K, pl * p.plane_rows + row0, B_FULL(b));
                     }
+                    __syncwarp();
+                    MM_ADVANCE(b, bph, SB);
                 }
             }
         }
     } else if (warp == 1) {
         // ---- MMA issuer (whole warp converged, one elected lane per instruction)
         const uint32_t idesc = p.idesc;
-        const uint64_t ad0 = umma_desc_sw128(a_base), bd0 = umma_desc_sw128(b_base);
+        const uint32_t b_lo0 = (b_base >> 4) & 0x3FFFu;
         uint32_t sa = 0, saph = 0, sb = 0, sbph = 0, a = 0, aph = 0;
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
@@ -320,135 +444,99 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             const uint32_t d = tmem + a * acc_cols;
             uint32_t acc = 0;
             for (int ku = ua; ku < ub; ++ku) {
-                const bool two = ku * 2 + 1 < KB;
+                const int nk = min(MM_UK, KB - ku * MM_UK);
                 MM_WAIT(A_FULL(sa), saph);
-                const uint64_t ad = ad0 + sa * (MM_A_UNIT >> 4);
+                const uint32_t at = tmem + MM_A_COL + sa * (MM_UK * 32u);
                 for (int pl = 0; pl < p.P; ++pl) {
                     MM_WAIT(B_FULL(sb), sbph);
                     tc_fence_after();
-                    const uint64_t bd = bd0 + sb * (b_unit >> 4);
+                    const uint32_t b_lo = b_lo0 + sb * (b_unit >> 4);
                     const uint32_t dp = pl == 0 ? d : d + (uint32_t)Nt, keep = pl < 2 ? acc : 1u;
                     if (elect_one()) {
 #pragma unroll
-                        for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)      // 16 values = 32 bytes = 2 descriptor address units
-                            umma_f16(dp, ad + 2u * k4, bd + 2u * k4, idesc, k4 == 0 ? keep : 1u);
-                        if (two) {
+                        for (uint32_t h = 0; h < MM_UK; ++h)
+                            if ((int)h < nk) {
 #pragma unroll
-                            for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
-                                umma_f16(dp, ad + (MM_A_BYTES >> 4) + 2u * k4, bd + (b_slice >> 4) + 2u * k4, idesc, 1u);
-                        }
-                        if (p.P > 1) umma_commit(B_EMPTY(sb));
-                        if (pl == p.P - 1) umma_commit(A_EMPTY(sa));          // with one plane this frees the unit of B too
+                                for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)  // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
+                                    umma_f16_ts(dp, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, (h | k4) == 0 ? keep : 1u);
+                            }
+                        umma_commit(B_EMPTY(sb));
+                        if (pl == p.P - 1) umma_commit(A_EMPTY(sa));
                     }
                     __syncwarp();
                     MM_ADVANCE(sb, sbph, SB);
                 }
                 acc = 1;
-                MM_ADVANCE(sa, saph, SA);
+                MM_ADVANCE(sa, saph, MM_A_UNITS);
             }
             if (elect_one()) umma_commit(ACC_FULL(a));
             __syncwarp();
-            a ^= 1u;
-            aph ^= (a == 0);
+            MM_ADVANCE(a, aph, accs);
         }
     } else if (warp >= 7) {
-        // ---- decoders: group 0 (warps 7..14) takes even units, group 1 (warps 15..22) odd units; warp dw of a group takes sixteen
-        // columns: a lane decodes the words it would feed to mma.sync
-        const int dw = (warp - 7) & 7, group = (warp - 7) >> 3;
-        const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u;
-        const uint32_t ch0 = ((2u * t) ^ g) << 4, ch1 = ((2u * t + 1u) ^ g) << 4;      // swizzled 16-byte chunks of rows 16t .. 16t+15
+        // ---- decoders: a warp expands slice h of every unit, 32 columns of W, into its 32 lanes of tensor memory.  Lane 4g + u
+        // holds column 16 * (u >> 1) + 8 * (u & 1) + g of them (see mm_column).
+        const int q = warp & 3, h = (warp - 7) >> 2;
+        const uint32_t g = (uint32_t)lane >> 2, u = (uint32_t)lane & 3u;
+        const uint32_t raw_lane = (uint32_t)(2 * q + (u >> 1)) * 1024u + (uint32_t)(h >> 1) * 512u;
+        const uint32_t a_lane = tmem + MM_A_COL + ((uint32_t)(q * 32) << 16) + (uint32_t)h * 32u;
         uint32_t m4, m16;
         asm volatile("mov.b32 %0, %2;\n\tmov.b32 %1, %3;" : "=r"(m4), "=r"(m16) : "r"(p.mul4), "r"(p.mul16));
-        uint32_t sa = 0, saph = 0, r = 0, rph = 0, turn = 0;
+        uint32_t sa = 0, saph = 0, r = 0, rph = 0;
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
-            for (int ku = ua; ku < ub; ++ku, turn ^= 1u) {
-                if ((int)turn == group) {
-                    const bool two = ku * 2 + 1 < KB;
-                    const uint32_t at = r_base + r * MM_UNIT_BYTES + (uint32_t)dw * 512u;
-                    MM_WAIT_BLOCK(RAW_FULL(r), rph);
-                    uint4 rw;
-                    if (two) rw = ld_shared_v4(at + (uint32_t)lane * 16u);
-                    else asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(rw.x), "=r"(rw.y) : "r"(at + (uint32_t)lane * 8u) : "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(RAW_EMPTY(r));
-                    MM_WAIT_BLOCK(A_EMPTY(sa), saph ^ 1u);
+            for (int ku = ua; ku < ub; ++ku) {
+                const int slice = ku * MM_UK + h;
+                const uint32_t at = r_base + r * MM_UNIT_BYTES + raw_lane;
+                MM_WAIT(RAW_FULL(r), rph);
+                uint32_t w[4];
+                if ((slice | 1) < KB) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        if (h == 0 || two) {
-                            const uint32_t arow = a_base + sa * MM_A_UNIT + (uint32_t)h * MM_A_BYTES + ((uint32_t)(dw * 16) + g) * 128u;
+                    for (int t = 0; t < 4; ++t) {
+                        uint32_t lo, hi;
+                        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(at + (uint32_t)mm_chunk((int)g, t) * 16u + (uint32_t)(h & 1) * 8u) : "memory");
+                        w[t] = u & 1u ? hi : lo;
+                    }
+                } else if (slice < KB) {                      // an odd last slice
 #pragma unroll
-                            for (int hi = 0; hi < 2; ++hi) {
-                                uint32_t o[8];
-                                mm_decode_word(h ? (hi ? rw.w : rw.z) : (hi ? rw.y : rw.x), m4, m16, o);
-                                st_shared_v4(arow + (uint32_t)hi * 1024u + ch0, o[0], o[1], o[2], o[3]);
-                                st_shared_v4(arow + (uint32_t)hi * 1024u + ch1, o[4], o[5], o[6], o[7]);
-                            }
-                        }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // make the slices visible to the tensor core's reads
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(A_FULL(sa));
+                    for (int t = 0; t < 4; ++t)
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[t]) : "r"(at + (4u * g + (uint32_t)t) * 8u + (u & 1u) * 4u) : "memory");
                 }
-                MM_ADVANCE(sa, saph, SA);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(RAW_EMPTY(r));
+                MM_WAIT(A_EMPTY(sa), saph ^ 1u);
+                if (slice < KB) {
+                    tc_fence_after();
+                    uint32_t o[32];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) mm_decode_word(w[t], m4, m16, o + 8 * t);
+                    tmem_st32(a_lane + sa * (MM_UK * 32u), o);
+                    tmem_wait_st();
+                    tc_fence_before();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(A_FULL(sa));
+                MM_ADVANCE(sa, saph, MM_A_UNITS);
                 MM_ADVANCE(r, rph, R);
             }
         }
     } else {
         // ---- epilogue (warps 2..5): a warp may read the 32 tensor-memory lanes selected by warp % 4
-        const int q = warp & 3, nl = q * 32 + lane;
+        const int q = warp & 3, nl = q * 32 + lane, ncol = q * 32 + mm_column(lane);
         pdl_wait();
         uint32_t a = 0, aph = 0;
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
             const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
-            MM_WAIT_BLOCK(ACC_FULL(a), aph);
+            MM_WAIT(ACC_FULL(a), aph);
             tc_fence_after();
             const bool full = ua == 0 && ub == KBU;
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + a * acc_cols;
             const size_t slot_floats = (size_t)MM_TILE_N * Nt;
             float* slot = p.partial + (size_t)(2 * cta + sl) * slot_floats + nl * 4;
-            const int n = nt * MM_TILE_N + nl;
-            const bool in_n = n < p.N;
-            // four consecutive rows m .. m+3 of this lane's column
-            auto emit4 = [&](const float (&v)[4], int m) {
-                if (p.y_col == 2 && in_n && m + 4 <= p.M && p.y_dtype != TLLM_F16 && p.y_dtype != TLLM_BF16) {
-                    // column-major results of four bytes: the rows are neighbours
-                    uint4 w;
-                    if (p.y_dtype == TLLM_I32) w = make_uint4((uint32_t)(int)(v[0] * 0.5f), (uint32_t)(int)(v[1] * 0.5f), (uint32_t)(int)(v[2] * 0.5f), (uint32_t)(int)(v[3] * 0.5f));
-                    else w = make_uint4(__float_as_uint(v[0] * p.scale), __float_as_uint(v[1] * p.scale), __float_as_uint(v[2] * p.scale), __float_as_uint(v[3] * p.scale));
-                    *(uint4*)((uint32_t*)p.Y + (size_t)n * p.y_ld + m) = w;
-                    return;
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float y;
-                    bool ok;
-                    size_t at;
-                    if (p.epilogue == 0) {
-                        y = v[j] * p.scale;
-                        ok = in_n;
-                        at = p.y_col ? (size_t)n * p.y_ld + m + j : (size_t)(m + j) * p.y_ld + n;
-                    } else {
-                        const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
-                        y = silu_mul(v[j] * p.scale, other * p.scale2);
-                        ok = !(nl & 1) && n + 1 < p.N;
-                        at = (size_t)(m + j) * p.y_ld + (n >> 1);
-                    }
-                    if (!ok || m + j >= p.M) continue;
-                    if (p.y_planes) {
-                        // the three bf16 values that add up to y (see stage_acts_kernel)
-                        uint32_t w = __float_as_uint(y);
-#pragma unroll
-                        for (int pl = 0; pl < 3; ++pl) {
-                            ((unsigned short*)p.Y)[(size_t)pl * p.plane_y + at] = (unsigned short)(w >> 16);
-                            w = __float_as_uint(__uint_as_float(w) - __uint_as_float(w & 0xFFFF0000u));
-                        }
-                    } else if (p.y_dtype == TLLM_I32) ((int*)p.Y)[at] = (int)(v[j] * 0.5f);
-                    else store_out(p.Y, p.y_dtype, at, y);
-                }
-            };
+            const int n = nt * MM_TILE_N + ncol;
             // sixteen accumulator columns (rows of X) of this lane's column of W
             auto load16 = [&](int c16, float (&f)[16]) {
                 uint32_t v[16];
@@ -495,8 +583,6 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 // A part lies in its block's slot 0, except that the first block may have come from an earlier tile.
                 const float* part0 = p.partial + (size_t)(2 * cf + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * cf + 2) * slot_floats + nl * 4;
-                const bool pairs = p.epilogue == 0 && !p.y_planes && !p.y_col && (p.y_dtype == TLLM_F16 || p.y_dtype == TLLM_BF16) && !(p.y_ld & 1) &&
-                                   ((uintptr_t)p.Y & 3u) == 0 && nt * MM_TILE_N + MM_TILE_N <= p.N;
                 for (int c16 = 0; c16 < Nt; c16 += 16) {
                     float f[16];
                     if (full) load16(c16, f);
@@ -520,37 +606,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                             ps = rest + (size_t)(cc - cf) * 2 * slot_floats + (size_t)c16 * MM_TILE_N;
                         }
                     }
-                    if (pairs) {
-                        // 16-bit outputs: neighbouring lanes trade one value per pair of rows, so that every lane
-                        // writes two adjacent columns of one row with a single 4-byte store
-#pragma unroll
-                        for (int t = 0; t < 16; t += 2) {
-                            const float e0 = f[t] * p.scale, e1 = f[t + 1] * p.scale;
-                            const float mine = (lane & 1) ? e1 : e0, send = (lane & 1) ? e0 : e1;
-                            const float got = __shfl_xor_sync(0xffffffffu, send, 1);
-                            const int m = mt * Nt + c16 + t + (lane & 1);
-                            const float lo = (lane & 1) ? got : mine, hi = (lane & 1) ? mine : got;
-                            if (m < p.M) {
-                                uint32_t w;
-                                if (p.y_dtype == TLLM_F16) w = (uint32_t)__half_as_ushort(__float2half_rn(lo)) | ((uint32_t)__half_as_ushort(__float2half_rn(hi)) << 16);
-                                else w = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) | ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
-                                *(uint32_t*)((char*)p.Y + ((size_t)m * p.y_ld + (n & ~1)) * 2) = w;
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int t = 0; t < 16; t += 4) {
-                            const float e[4] = {f[t], f[t + 1], f[t + 2], f[t + 3]};
-                            emit4(e, mt * Nt + c16 + t);
-                        }
-                    }
+                    if (p.epilogue == 0) mm_emit(p, f, n, mt * Nt + c16);
+                    else mm_emit_silu(p, f, n, mt * Nt + c16);
                 }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(ACC_EMPTY(a));
-            a ^= 1u;
-            aph ^= (a == 0);
+            MM_ADVANCE(a, aph, accs);
         }
     }
 done:
@@ -559,7 +622,7 @@ done:
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, p.tmem_cols);
+        tmem_dealloc(tmem, 512);
     }
     if (tid == 0 && flags[1]) atomicExch(p.status, MM_ERR_WAIT);
 #undef A_FULL
@@ -572,7 +635,6 @@ done:
 #undef ACC_EMPTY
 }
 #undef MM_WAIT
-#undef MM_WAIT_BLOCK
 #undef MM_ADVANCE
 
 // ---- activations as planes of 16-bit values for the kernel above: rows of k_pad values, zero beyond K ------------------

@@ -187,7 +187,7 @@ class PackedMLP:
         return a.as_dict(), b.as_dict()
 
     def forward(self, x, out=None, h=None):
-        return self._forward(self._handle, x, out, h, self.hidden, self.inter)
+        return self._forward(self._handle, x, out, h, self.hidden)
 
     def close(self):
         if self._h:

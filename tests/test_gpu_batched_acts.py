@@ -62,3 +62,24 @@ def test_fused_mlp(dtype, hidden, inter):
         # fp32 sums, and up to one last place of the type in h and in the result
         assert err <= 1e-5 + {"f32": 2.0 ** -22, "f16": 2.0 ** -10, "bf16": 2.0 ** -7}[dtype], (M, err)
     mlp.close()
+
+
+def test_calls_with_a_workspace_replay_from_a_graph():
+    rng = np.random.default_rng(7)
+    K, N, M = 1024, 640, 200
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w)
+    X = torch.zeros((M, K), device="cuda")
+    pw.matmul(X)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        Y = pw.matmul(X)
+        Z = pw.matmul(X * 2)
+    for seed in range(3):
+        xs = np.random.default_rng(seed).integers(-9, 10, size=(M, K)).astype(np.float64)
+        X.copy_(torch.tensor(xs, dtype=torch.float32))
+        g.replay()
+        want = oracle.dense_f64(xs, w)
+        assert np.array_equal(Y.double().cpu().numpy(), want) and np.array_equal(Z.double().cpu().numpy(), 2 * want)
+    pw.close()
