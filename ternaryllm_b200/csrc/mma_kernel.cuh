@@ -38,6 +38,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace tllm {
@@ -242,55 +244,61 @@ template <bool BF16>
 __device__ __forceinline__ void mm_emit_16(const MmParams& p, const float (&f)[16], int n, int m) {
     unsigned short* y = (unsigned short*)p.Y + (size_t)n * p.y_step_n + (size_t)m * p.y_step_m;
 #pragma unroll
-    for (int t = 0; t < 16; ++t)
-        if (n < p.N && m + t < p.M) y[t * p.y_step_m] = mm_16bit<BF16>(f[t] * p.scale);
+    for (int t = 0; t < 16; ++t) {
+        if (n < p.N && m + t < p.M) *y = mm_16bit<BF16>(f[t] * p.scale);
+        y += p.y_step_m;
+    }
 }
 // the lanes of neighbouring columns trade one value per pair of rows, so that every lane writes two adjacent columns of one row
 template <bool BF16>
 __device__ __forceinline__ void mm_emit_pairs(const MmParams& p, const float (&f)[16], int n, int m) {
     const bool odd = n & 1;
-    unsigned short* y = (unsigned short*)p.Y + (size_t)(m + (odd ? 1 : 0)) * p.y_step_m + (n & ~1);
+    uint32_t* y = (uint32_t*)((unsigned short*)p.Y + (size_t)(m + (odd ? 1 : 0)) * p.y_step_m + (n & ~1));
 #pragma unroll
     for (int t = 0; t < 16; t += 2) {
-        const float e0 = f[t] * p.scale, e1 = f[t + 1] * p.scale;
-        const float got = __shfl_xor_sync(0xffffffffu, odd ? e0 : e1, 4);
-        const uint32_t w = (uint32_t)mm_16bit<BF16>(odd ? got : e0) | ((uint32_t)mm_16bit<BF16>(odd ? e1 : got) << 16);
-        if (m + t + (odd ? 1 : 0) < p.M) *(uint32_t*)(y + t * p.y_step_m) = w;
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? f[t] : f[t + 1], 4);
+        const float lo = (odd ? got : f[t]) * p.scale, hi = (odd ? f[t + 1] : got) * p.scale;
+        uint32_t w;
+        if (BF16) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+            w = *reinterpret_cast<const uint32_t*>(&h);
+        } else {
+            const __half2 h = __floats2half2_rn(lo, hi);
+            w = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        if (m + t + (odd ? 1 : 0) < p.M) *y = w;
+        y += p.y_step_m;                       // two rows of 16-bit values = y_step_m words
     }
 }
+template <int OUT>
 __device__ __forceinline__ void mm_emit(const MmParams& p, const float (&f)[16], int n, int m) {
     uint32_t* y = (uint32_t*)p.Y + (size_t)n * p.y_step_n + (size_t)m * p.y_step_m;
-    switch (p.out) {
-        case MM_OUT_F32:
+    if constexpr (OUT == MM_OUT_F16 || OUT == MM_OUT_BF16) mm_emit_16<OUT == MM_OUT_BF16>(p, f, n, m);
+    else if constexpr (OUT == MM_OUT_F16_PAIRS || OUT == MM_OUT_BF16_PAIRS) mm_emit_pairs<OUT == MM_OUT_BF16_PAIRS>(p, f, n, m);
+    else if constexpr (OUT == MM_OUT_F32 || OUT == MM_OUT_I32) {
 #pragma unroll
-            for (int t = 0; t < 16; ++t)
-                if (n < p.N && m + t < p.M) y[t * p.y_step_m] = __float_as_uint(f[t] * p.scale);
-            break;
-        case MM_OUT_I32:
+        for (int t = 0; t < 16; ++t) {
+            const uint32_t w = OUT == MM_OUT_F32 ? __float_as_uint(f[t] * p.scale) : (uint32_t)(int)(f[t] * 0.5f);
+            if (n < p.N && m + t < p.M) *y = w;
+            y += p.y_step_m;
+        }
+    } else {
 #pragma unroll
-            for (int t = 0; t < 16; ++t)
-                if (n < p.N && m + t < p.M) y[t * p.y_step_m] = (uint32_t)(int)(f[t] * 0.5f);
-            break;
-        case MM_OUT_F16: mm_emit_16<false>(p, f, n, m); break;
-        case MM_OUT_BF16: mm_emit_16<true>(p, f, n, m); break;
-        case MM_OUT_F16_PAIRS: mm_emit_pairs<false>(p, f, n, m); break;
-        case MM_OUT_BF16_PAIRS: mm_emit_pairs<true>(p, f, n, m); break;
-        default:                     // MM_OUT_F32_COL4, MM_OUT_I32_COL4
+        for (int t = 0; t < 16; t += 4) {
+            uint32_t w[4];
 #pragma unroll
-            for (int t = 0; t < 16; t += 4) {
-                uint32_t w[4];
+            for (int j = 0; j < 4; ++j) w[j] = OUT == MM_OUT_F32_COL4 ? __float_as_uint(f[t + j] * p.scale) : (uint32_t)(int)(f[t + j] * 0.5f);
+            if (n < p.N && m + t + 4 <= p.M) *(uint4*)(y + t) = make_uint4(w[0], w[1], w[2], w[3]);
+            else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) w[j] = p.out == MM_OUT_F32_COL4 ? __float_as_uint(f[t + j] * p.scale) : (uint32_t)(int)(f[t + j] * 0.5f);
-                if (n < p.N && m + t + 4 <= p.M) *(uint4*)(y + t) = make_uint4(w[0], w[1], w[2], w[3]);
-                else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (n < p.N && m + t + j < p.M) y[t + j] = w[j];
-                }
+                for (int j = 0; j < 4; ++j)
+                    if (n < p.N && m + t + j < p.M) y[t + j] = w[j];
             }
+        }
     }
 }
 // Gate and up columns sit in neighbouring lanes: the even one takes row t, the odd one row t + 1.
+template <int OUT>
 __device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)[16], int n, int m) {
     const bool odd = n & 1;
     const int row = m + (odd ? 1 : 0);
@@ -303,11 +311,11 @@ __device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)
     }
     const bool ok = (n | 1) < p.N;
     const size_t step = 2 * (size_t)p.y_ld;
-    if (p.out == MM_OUT_F32) {
+    if constexpr (OUT == MM_OUT_F32) {
 #pragma unroll
         for (int t = 0; t < 8; ++t)
             if (ok && row + 2 * t < p.M) ((float*)p.Y)[at + t * step] = y[t];
-    } else if (p.out == MM_OUT_PLANES) {
+    } else if constexpr (OUT == MM_OUT_PLANES) {
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
             uint32_t w = __float_as_uint(y[t]);
@@ -318,11 +326,34 @@ __device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)
             }
         }
     } else {
-        const bool bf = p.out == MM_OUT_BF16;
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            const unsigned short w = bf ? mm_16bit<true>(y[t]) : mm_16bit<false>(y[t]);
+            const unsigned short w = mm_16bit<OUT == MM_OUT_BF16>(y[t]);
             if (ok && row + 2 * t < p.M) ((unsigned short*)p.Y)[at + t * step] = w;
+        }
+    }
+}
+
+// runs `f` with the kind of store as a type
+template <typename F>
+__device__ __forceinline__ void mm_with_out(const MmParams& p, F f) {
+    if (p.epilogue == 0) {
+        switch (p.out) {
+            case MM_OUT_F32: f(std::integral_constant<int, MM_OUT_F32>{}, std::false_type{}); break;
+            case MM_OUT_I32: f(std::integral_constant<int, MM_OUT_I32>{}, std::false_type{}); break;
+            case MM_OUT_F16: f(std::integral_constant<int, MM_OUT_F16>{}, std::false_type{}); break;
+            case MM_OUT_BF16: f(std::integral_constant<int, MM_OUT_BF16>{}, std::false_type{}); break;
+            case MM_OUT_F16_PAIRS: f(std::integral_constant<int, MM_OUT_F16_PAIRS>{}, std::false_type{}); break;
+            case MM_OUT_BF16_PAIRS: f(std::integral_constant<int, MM_OUT_BF16_PAIRS>{}, std::false_type{}); break;
+            case MM_OUT_F32_COL4: f(std::integral_constant<int, MM_OUT_F32_COL4>{}, std::false_type{}); break;
+            default: f(std::integral_constant<int, MM_OUT_I32_COL4>{}, std::false_type{});
+        }
+    } else {
+        switch (p.out) {
+            case MM_OUT_F32: f(std::integral_constant<int, MM_OUT_F32>{}, std::true_type{}); break;
+            case MM_OUT_F16: f(std::integral_constant<int, MM_OUT_F16>{}, std::true_type{}); break;
+            case MM_OUT_BF16: f(std::integral_constant<int, MM_OUT_BF16>{}, std::true_type{}); break;
+            default: f(std::integral_constant<int, MM_OUT_PLANES>{}, std::true_type{});
         }
     }
 }
@@ -443,31 +474,48 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             tc_fence_after();
             const uint32_t d = tmem + a * acc_cols;
             uint32_t acc = 0;
+            MM_WAIT(A_FULL(sa), saph);
+            MM_WAIT(B_FULL(sb), sbph);
+            tc_fence_after();
             for (int ku = ua; ku < ub; ++ku) {
                 const int nk = min(MM_UK, KB - ku * MM_UK);
-                MM_WAIT(A_FULL(sa), saph);
                 const uint32_t at = tmem + MM_A_COL + sa * (MM_UK * 32u);
                 for (int pl = 0; pl < p.P; ++pl) {
-                    MM_WAIT(B_FULL(sb), sbph);
-                    tc_fence_after();
-                    const uint32_t b_lo = b_lo0 + sb * (b_unit >> 4);
+                    const uint32_t b_lo = b_lo0 + sb * (b_unit >> 4), sb0 = sb, sa0 = sa;
                     const uint32_t dp = pl == 0 ? d : d + (uint32_t)Nt, keep = pl < 2 ? acc : 1u;
+                    const bool unit_done = pl == p.P - 1;
+                    // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
                     if (elect_one()) {
 #pragma unroll
-                        for (uint32_t h = 0; h < MM_UK; ++h)
+                        for (uint32_t h = 0; h < MM_UK - 1; ++h)
                             if ((int)h < nk) {
 #pragma unroll
-                                for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)  // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
+                                for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
                                     umma_f16_ts(dp, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, (h | k4) == 0 ? keep : 1u);
                             }
-                        umma_commit(B_EMPTY(sb));
-                        if (pl == p.P - 1) umma_commit(A_EMPTY(sa));
                     }
                     __syncwarp();
                     MM_ADVANCE(sb, sbph, SB);
+                    if (unit_done) MM_ADVANCE(sa, saph, MM_A_UNITS);
+                    // what comes next is waited for before the last slice goes out: the tensor core works on what is queued meanwhile
+                    if (!unit_done || ku + 1 < ub) {
+                        if (unit_done) MM_WAIT(A_FULL(sa), saph);
+                        MM_WAIT(B_FULL(sb), sbph);
+                        tc_fence_after();
+                    }
+                    if (elect_one()) {
+                        if (nk == MM_UK) {
+                            constexpr uint32_t h = MM_UK - 1;
+#pragma unroll
+                            for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
+                                umma_f16_ts(dp, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, 1u);
+                        }
+                        umma_commit(B_EMPTY(sb0));
+                        if (unit_done) umma_commit(A_EMPTY(sa0));
+                    }
+                    __syncwarp();
                 }
                 acc = 1;
-                MM_ADVANCE(sa, saph, MM_A_UNITS);
             }
             if (elect_one()) umma_commit(ACC_FULL(a));
             __syncwarp();
@@ -583,6 +631,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 // A part lies in its block's slot 0, except that the first block may have come from an earlier tile.
                 const float* part0 = p.partial + (size_t)(2 * cf + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * cf + 2) * slot_floats + nl * 4;
+                mm_with_out(p, [&](auto out, auto silu) {
                 for (int c16 = 0; c16 < Nt; c16 += 16) {
                     float f[16];
                     if (full) load16(c16, f);
@@ -606,9 +655,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                             ps = rest + (size_t)(cc - cf) * 2 * slot_floats + (size_t)c16 * MM_TILE_N;
                         }
                     }
-                    if (p.epilogue == 0) mm_emit(p, f, n, mt * Nt + c16);
-                    else mm_emit_silu(p, f, n, mt * Nt + c16);
+                    if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, mt * Nt + c16);
+                    else mm_emit<decltype(out)::value>(p, f, n, mt * Nt + c16);
                 }
+                });
             }
             tc_fence_before();
             __syncwarp();
