@@ -30,7 +30,7 @@ int launch(const BitsParams& p, int grid, size_t smem, int device, cudaStream_t 
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p.pdl ? 1 : 0;
     BT_TRY(cudaLaunchKernelEx(&cfg, kern, p));
     note_launch();
     return TLLM_OK;

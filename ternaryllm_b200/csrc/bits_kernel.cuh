@@ -59,6 +59,7 @@ struct BitsParams {
     uint32_t slot_bytes;           // shared memory of one pair of slices: GR * 512 + M * 128 * E
     uint32_t m_inv;                // ceil(2^32 / M): idx / M = umulhi(idx, m_inv) for M > 1
     uint32_t mul4, mul16;          // 4 and 16
+    bool pdl;                      // host: launch beside the preceding kernel
     float scale, scale2;
 };
 

@@ -13,6 +13,7 @@
 #include "bits_kernel.cuh"
 #include "bstream_kernel.cuh"
 #include "kernels.cuh"
+#include "lists_kernel.cuh"
 #include "mma_kernel.cuh"
 #include "nibble_format.h"
 #include "nibble_kernel.cuh"
@@ -138,7 +139,7 @@ struct tllm_weight {
     float* d_mm_partial = nullptr;
     unsigned int* d_mm_counters = nullptr;
     size_t bits_bytes = 0;
-    CUtensorMap bits_map;             // rows = groups of sixteen columns, KB * 64 words each; box = 8 groups x four slices
+    CUtensorMap bits_map;
     int mm_n_tiles = 0, mm_kb = 0, mm_grid = 0;
     // decode tensor-core kernel: transposed four-bit copy of W, its tensor map, schedule and hand-over scratch
     uint8_t* d_nib = nullptr;
@@ -155,6 +156,17 @@ struct tllm_weight {
     unsigned int* d_nr_counters = nullptr;
     CUtensorMap nr_map[4];
     int nb_k_pad = 0, nr_grid = 0;
+};
+
+// What the two kernels that read bit tiles need of a weight: a handle's, or one made for a single call (tllm_ter_spmm).
+struct BitsView {
+    const uint4* bits;
+    const CUtensorMap* map;
+    int inners, columns, n_tiles, kb, sms, device;
+    float* partial;               // 2 * sms hand-over slots for row tiles of up to MM_OWN_NT, or NULL
+    unsigned int* counters;       // n_tiles * MM_MAX_M_TILES * 4, zero between launches
+    int* status;
+    bool pdl;                     // the weight was there before the preceding kernel in the stream: the product may start beside it
 };
 
 struct tllm_mlp {
@@ -239,16 +251,20 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
+BitsView bits_view(const tllm_weight* w) {
+    return BitsView{w->d_bits, &w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, true};
+}
+
 // true when TMA can read the activations where they are (rows on 16 bytes; a box is 64 values wide)
-bool mm_direct(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld) {
+bool mm_direct(int inners, const void* X, int x_dtype, int x_layout, int x_ld) {
     return (x_dtype == TLLM_F16 || x_dtype == TLLM_BF16) && x_layout == TLLM_ROW_MAJOR && (uintptr_t)X % 16 == 0 && (size_t)x_ld * 2 % 16 == 0 &&
-           w->lay.inners >= MM_TILE_K;
+           inners >= MM_TILE_K;
 }
 
 // true when the tensor-core kernel is pinned, or the cost model of the older kernels prefers it, for fp16 / bf16 row-major
 // activations whose rows TMA can address
 bool mm_usable(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows) {
-    if (!w->d_bits || !mm_direct(w, X, x_dtype, x_layout, x_ld) || tensor_map_encoder() == nullptr) return false;
+    if (!w->d_bits || !mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld) || tensor_map_encoder() == nullptr) return false;
     const int thr = mm_min_rows();
     if (thr == 0) return false;
     if (thr > 0) return rows >= thr;
@@ -343,6 +359,17 @@ int encode_rows_map(CUtensorMap* map, const void* base, bool bf16, int k, int ro
     return TLLM_OK;
 }
 
+// bit tiles as rows = groups of sixteen columns of KB * 64 words; a box is a unit: eight groups x four slices
+int encode_bits_map(CUtensorMap* map, const void* bits, int n_tiles, int kb) {
+    const cuuint64_t dims[2] = {(cuuint64_t)kb * 64, (cuuint64_t)n_tiles * 8};
+    const cuuint64_t strides[1] = {(cuuint64_t)kb * 256};
+    const cuuint32_t box[2] = {MM_UK * 64, 8}, estr[2] = {1, 1};
+    const CUresult cr = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(bits), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled (bit tiles) failed with code %d", (int)cr);
+    return TLLM_OK;
+}
+
 cudaLaunchAttribute pdl_attribute() {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -385,16 +412,15 @@ struct MmOut {
 };
 
 // rows [0, rows) of `x` (at most MM_MAX_M_TILES tiles) in one launch of the tensor-core kernel
-int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStream_t st) {
-    const BsLayout& L = w->lay;
-    const MmPlan plan = mm_plan(rows, x.planes, w->mm_n_tiles, w->mm_kb, w->mm_grid);
+int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cudaStream_t st) {
+    const MmPlan plan = mm_plan(rows, x.planes, w.n_tiles, w.kb, w.sms);
     MmParams p{};
     p.Y = o.Y;
-    p.counters = w->d_mm_counters;
-    p.status = w->d_status;
-    p.M = rows, p.K = L.inners, p.N = L.columns;
-    p.KB = w->mm_kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
-    p.n_tiles = w->mm_n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split;
+    p.counters = w.counters;
+    p.status = w.status;
+    p.M = rows, p.K = w.inners, p.N = w.columns;
+    p.KB = w.kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
+    p.n_tiles = w.n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split;
     p.P = x.planes, p.plane_rows = x.plane_rows;
     p.epilogue = o.epilogue, p.y_ld = o.ld, p.plane_y = o.plane;
     p.y_step_n = o.col_major ? o.ld : 1, p.y_step_m = o.col_major ? 1 : o.ld;
@@ -402,7 +428,7 @@ int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStr
     if (o.epilogue == 0 && !o.planes) {
         const bool wide = o.dtype == TLLM_F32 || o.dtype == TLLM_I32;
         if (wide && o.col_major && (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0) p.out = o.dtype == TLLM_F32 ? MM_OUT_F32_COL4 : MM_OUT_I32_COL4;
-        if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && L.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
+        if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && w.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
     }
     // rings: four units of bit tiles, and as many of B as 192 KiB hold (three at 128 rows)
     p.R = 4;
@@ -416,22 +442,22 @@ int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStr
     p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
 
     CUtensorMap map;
-    int rc = encode_rows_map(&map, x.base, x.bf16, L.inners, (x.planes - 1) * x.plane_rows + rows, x.pitch, p.Nt);
+    int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, (x.planes - 1) * x.plane_rows + rows, x.pitch, p.Nt);
     if (rc) return rc;
     const size_t smem = 1024 + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512;
     if (smem > 227 * 1024) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
     static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[w->device & 63], [&] { err = cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+    std::call_once(once[w.device & 63], [&] { err = cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
     CU_TRY(err);
     // never more blocks than items: the hand-over between the blocks that share a tile counts on every block in a
     // tile's range of owners holding at least one unit of it
     const long long items = (long long)p.n_tiles * p.m_tiles * (p.split ? p.KBU : 1);
-    const int grid = (int)(items < w->mm_grid ? items : w->mm_grid);
+    const int grid = (int)(items < w.sms ? items : w.sms);
     Workspace ws;
-    if (p.Nt <= MM_OWN_NT || !p.split) p.partial = w->d_mm_partial;
+    if ((p.Nt <= MM_OWN_NT && w.partial) || !p.split) p.partial = w.partial;
     else {
-        rc = ws.take(w->device, (size_t)2 * grid * MM_TILE_N * p.Nt * sizeof(float), st);
+        rc = ws.take(w.device, (size_t)2 * grid * MM_TILE_N * p.Nt * sizeof(float), st);
         if (rc) return rc;
         p.partial = (float*)ws.ptr;
     }
@@ -442,15 +468,15 @@ int launch_mm(tllm_weight* w, const MmActs& x, int rows, const MmOut& o, cudaStr
     cfg.stream = st;
     cudaLaunchAttribute at[1] = {pdl_attribute()};
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, w->bits_map, p));
+    cfg.numAttrs = w.pdl ? 1 : 0;
+    CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, *w.map, p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
 }
 
 // fp32 activations that are three planes already ([3][rows][pitch / 2], pitch bytes per row)
-int run_mm_planes(tllm_weight* w, const unsigned short* planes, int plane_rows, size_t pitch, int rows, void* Y, int y_dtype, int y_ld, float scale, cudaStream_t st) {
+int run_mm_planes(const BitsView& w, const unsigned short* planes, int plane_rows, size_t pitch, int rows, void* Y, int y_dtype, int y_ld, float scale, cudaStream_t st) {
     const int per = MM_MAX_M_TILES * MM_MAX_NT;
     for (int r0 = 0; r0 < rows; r0 += per) {
         const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch}, std::min(rows - r0, per),
@@ -461,15 +487,15 @@ int run_mm_planes(tllm_weight* w, const unsigned short* planes, int plane_rows, 
 }
 
 // the whole product on the tensor-core kernel: activations that TMA cannot read as they are go through planes in a workspace
-int run_mm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
+int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
            float scale2, cudaStream_t st, bool y_col = false, bool y_planes = false, long long plane_y = 0) {
-    const int K = w->lay.inners;
+    const int K = w.inners;
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
-    const bool direct = mm_direct(w, X, x_dtype, x_layout, x_ld);
+    const bool direct = mm_direct(w.inners, X, x_dtype, x_layout, x_ld);
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * MM_MAX_NT;
     Workspace ws;
     if (!direct) {
-        const int rc = ws.take(w->device, (size_t)planes * std::min(rows, per) * stage_pad(K) * 2, st);
+        const int rc = ws.take(w.device, (size_t)planes * std::min(rows, per) * stage_pad(K) * 2, st);
         if (rc) return rc;
     }
     for (int r0 = 0; r0 < rows; r0 += per) {
@@ -694,13 +720,14 @@ int run_nb(tllm_weight* w, const void* X, int x_dtype, int x_ld, int rows, void*
 // rows one launch takes: 16, fp32 (three bf16 values each) 8
 int bt_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? BT_MAX_ROWS / 2 : BT_MAX_ROWS; }
 
-int run_bits(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
+int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
              float scale2, cudaStream_t st) {
     BitsParams p{};
-    p.bits = w->d_bits;
+    p.pdl = w.pdl;
+    p.bits = w.bits;
     p.x_dtype = x_dtype, p.x_layout = x_layout, p.x_ld = x_ld;
     p.y_dtype = y_dtype, p.y_ld = y_ld, p.epilogue = epilogue;
-    p.K = w->lay.inners, p.N = w->lay.columns, p.KB = w->mm_kb;
+    p.K = w.inners, p.N = w.columns, p.KB = w.kb;
     p.scale = scale * 0.5f, p.scale2 = scale2 * 0.5f;            // the decoded weights are +-2
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const int per = bt_rows_per_launch(x_dtype);
@@ -708,7 +735,7 @@ int run_bits(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld,
         p.M = rows - r0 < per ? rows - r0 : per;
         p.X = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
         p.Y = (char*)Y + (size_t)r0 * y_ld * ye;
-        const int rc = bits_launch(p, w->mm_grid, w->device, st);
+        const int rc = bits_launch(p, w.sms, w.device, st);
         if (rc) return rc;
     }
     if (rows > 4) g_mm_launches.fetch_add((rows + per - 1) / per, std::memory_order_relaxed);   // counted with the batched products
@@ -725,12 +752,17 @@ double bt_model_us(int64_t entries, int x_dtype, int rows) {
     for (int r0 = 0; r0 < rows; r0 += per) t += 2.0 + entries * 1e-6 * per_mentry[(std::min(rows - r0, per) * p + 7) / 8];
     return t;
 }
-double mm_tiles_model_us(const tllm_weight* w, bool direct, int x_dtype, int rows) {
+double mm_tiles_model_us(int n_tiles, int kb, int sms, bool direct, int x_dtype, int rows) {
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * MM_MAX_NT;
     double t = 0;
-    for (int r0 = 0; r0 < rows; r0 += per)
-        t += 6.0 + mm_plan(std::min(rows - r0, per), planes, w->mm_n_tiles, w->mm_kb, w->mm_grid).clocks / 1800.0 + (direct ? 0.0 : 2.5);
+    for (int r0 = 0; r0 < rows; r0 += per) t += 6.0 + mm_plan(std::min(rows - r0, per), planes, n_tiles, kb, sms).clocks / 1800.0 + (direct ? 0.0 : 2.5);
     return t;
+}
+// which of the two: true = decode in registers
+bool bits_prefer_registers(int inners, int columns, int sms, bool direct, int x_dtype, int rows) {
+    if (rows <= 8) return true;
+    if (rows > 8 * BT_MAX_ROWS) return false;
+    return bt_model_us((int64_t)inners * columns, x_dtype, rows) <= mm_tiles_model_us((columns + 127) / 128, (inners + 63) / 64, sms, direct, x_dtype, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
@@ -743,9 +775,7 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
         // very sparse weights: the index lists are shorter than two bits an entry (the gather model is a fifth low at 90 % zeros)
         if (rows <= 4 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(entries, x_dtype, rows)) return KERNEL_GATHER;
-        if (rows <= 8) return KERNEL_BITS;
-        if (rows > 8 * BT_MAX_ROWS) return KERNEL_MMA;
-        return bt_model_us(entries, x_dtype, rows) <= mm_tiles_model_us(w, mm_direct(w, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
+        return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
     if (nb && mm) return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
     return nb ? KERNEL_NIBBLE : (mm ? KERNEL_MMA : KERNEL_GATHER);
@@ -827,9 +857,9 @@ int run_gather(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_l
 int run_product(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
                 float scale2, cudaStream_t st) {
     switch (choose_kernel(w, X, x_dtype, x_layout, x_ld, rows)) {
-        case KERNEL_BITS: return run_bits(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
+        case KERNEL_BITS: return run_bits(bits_view(w), X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
         case KERNEL_NIBBLE: return run_nb(w, X, x_dtype, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
-        case KERNEL_MMA: return run_mm(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
+        case KERNEL_MMA: return run_mm(bits_view(w), X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
         default: return run_gather(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, Scratch{w->d_partial, w->d_counters}, st);
     }
 }
@@ -867,12 +897,8 @@ int upload_bit_tiles(tllm_weight* w, const std::vector<uint32_t>& bits, int sms)
     CU_TRY(cudaMalloc(&w->d_bits, w->bits_bytes));
     CU_TRY(cudaMemcpy(w->d_bits, bits.data(), w->bits_bytes, cudaMemcpyHostToDevice));
     if (tensor_map_encoder() != nullptr) {
-        const cuuint64_t dims[2] = {(cuuint64_t)w->mm_kb * 64, (cuuint64_t)w->mm_n_tiles * 8};
-        const cuuint64_t strides[1] = {(cuuint64_t)w->mm_kb * 256};
-        const cuuint32_t box[2] = {MM_UK * 64, 8}, estr[2] = {1, 1};
-        const CUresult cr = tensor_map_encoder()(&w->bits_map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->d_bits, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (cr != CUDA_SUCCESS) return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled (bit tiles) failed with code %d", (int)cr);
+        const int rc = encode_bits_map(&w->bits_map, w->d_bits, w->mm_n_tiles, w->mm_kb);
+        if (rc) return rc;
     }
     const size_t partial_bytes = (size_t)2 * sms * MM_TILE_N * MM_OWN_NT * sizeof(float);
     const size_t counter_bytes = (size_t)w->mm_n_tiles * MM_MAX_M_TILES * 4 * sizeof(unsigned int);
@@ -947,6 +973,77 @@ int add_bias(void* Y, const void* bias, int y_dtype, int rows, int columns, cuda
     CU_TRY(cudaGetLastError());
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
+}
+
+int device_sms_cached(int dev, int* sms) {
+    static std::atomic<int> known[64];
+    int v = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (!v) {
+        const int rc = device_sms(&v);
+        if (rc) return rc;
+        if (dev < 64) known[dev].store(v, std::memory_order_relaxed);
+    }
+    *sms = v;
+    return TLLM_OK;
+}
+
+// ---- the product on the reference's arrays as they are --------------------------------------------------------------
+// one warp per column; with `flags`, `blocks` thread blocks that do it only if one of the nflags words is not zero
+int run_mcsc(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, const int32_t* col_off, void* Y, int y_dtype, int batch, int rows, int columns,
+             int inners, int tile_k, float scale, const int* flags, int nflags, int blocks, cudaStream_t st) {
+    const dim3 grid((columns + 7) / 8, (rows + MCSC_ROWS - 1) / MCSC_ROWS, batch);
+#define MCSC_ARGS rows, columns, inners, tile_k, scale
+    if (flags) {
+        if (x_dtype == TLLM_I8)
+            mcsc_spmm_if_kernel<int, MCSC_ROWS><<<blocks, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, MCSC_ARGS, flags, nflags);
+        else mcsc_spmm_if_kernel<float, MCSC_ROWS><<<blocks, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, MCSC_ARGS, flags, nflags);
+    } else {
+        if (grid.y > 65535) return fail(TLLM_ERR_ARG, "tllm_ter_spmm: too many rows for one call");
+        if (x_dtype == TLLM_I8) mcsc_spmm_kernel<int, MCSC_ROWS><<<grid, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, MCSC_ARGS);
+        else mcsc_spmm_kernel<float, MCSC_ROWS><<<grid, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, MCSC_ARGS);
+    }
+#undef MCSC_ARGS
+    CU_TRY(cudaGetLastError());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TLLM_OK;
+}
+
+// Whether the arrays are turned into bit tiles first, on every call.  The per-column kernel reads the lists again for every four
+// rows: 27 us a time at 2048 x 8192, 80 % zeros, fp32; the conversion and what follows it cost 15 us and 1.2e-6 us an entry
+// (35 us there, 57 with 256 rows).  The two meet at about 6e6 entries times passes.
+bool lists_worth_converting(long long entries, int rows) { return rows > MCSC_ROWS && entries * ((rows + MCSC_ROWS - 1) / MCSC_ROWS) >= 6000000; }
+
+int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, const int32_t* col_off, void* Y, int y_dtype, int batch, int rows, int columns,
+              int inners, int tile_k, float scale, int dev, int sms, cudaStream_t st) {
+    const int n_tiles = (columns + 127) / 128, kb = (inners + 63) / 64, groups = n_tiles * 8;
+    const size_t bits_bytes = (size_t)groups * kb * 256, counter_words = (size_t)n_tiles * MM_MAX_M_TILES * 4;
+    Workspace ws;
+    int rc = ws.take(dev, bits_bytes + (counter_words + groups + 1) * 4, st);
+    if (rc) return rc;
+    uint32_t* bits = (uint32_t*)ws.ptr;
+    unsigned int* counters = (unsigned int*)((char*)ws.ptr + bits_bytes);
+    int* flags = (int*)(counters + counter_words);          // one per group of columns, then the status word of the product
+    lists_to_bits_kernel<<<(unsigned)groups, LB_THREADS, 0, st>>>(row_idx, col_off, bits, counters, (int)counter_words, flags, columns, inners, tile_k, kb);
+    CU_TRY(cudaGetLastError());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    CUtensorMap map;
+    rc = encode_bits_map(&map, bits, n_tiles, kb);
+    if (rc) return rc;
+    // not beside the preceding kernel: that is the one that writes the tiles
+    const BitsView view{(const uint4*)bits, &map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, false};
+    const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
+    const bool one = x_layout == TLLM_ROW_MAJOR && (long long)batch * rows <= 0x7fffffffLL;      // the batch is contiguous: one product
+    const int parts = one ? 1 : batch, m = one ? batch * rows : rows, x_ld = x_layout == TLLM_ROW_MAJOR ? inners : rows;
+    for (int b = 0; b < parts; ++b) {
+        const char* xp = (const char*)X + (size_t)b * rows * inners * xe;
+        char* yp = (char*)Y + (size_t)b * rows * columns * ye;
+        if (bits_prefer_registers(inners, columns, sms, mm_direct(inners, xp, x_dtype, x_layout, x_ld), x_dtype, m))
+            rc = run_bits(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
+        else rc = run_mm(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
+        if (rc) return rc;
+    }
+    // lists that two bits an entry cannot hold (an entry named twice) are computed as before
+    return run_mcsc(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, rows, columns, inners, tile_k, scale, flags, groups + 1, 2 * sms, st);
 }
 
 }  // namespace
@@ -1076,6 +1173,7 @@ int tllm_ter_spmm(const void* X, int x_dtype, int x_layout, const int16_t* row_i
     const int rc = check_types(x_dtype, y_dtype, "tllm_ter_spmm");
     if (rc) return rc;
     if (batch > 65535) return fail(TLLM_ERR_ARG, "tllm_ter_spmm: batch too large");
+    if (rows == 1) x_layout = TLLM_ROW_MAJOR;        // one row per batch item: both layouts are the same memory
     if (tllm_weight* w = ter_cache_find(row_idx, col_off, columns, inners, tile_k)) {
         // these arrays were repacked by tllm_ter_spmm_prepare: the product runs on the packed copy
         cudaStream_t st = (cudaStream_t)stream;
@@ -1092,17 +1190,15 @@ int tllm_ter_spmm(const void* X, int x_dtype, int x_layout, const int16_t* row_i
         }
         return TLLM_OK;
     }
-    constexpr int MC = 4;
-    dim3 grid((columns + 7) / 8, (rows + MC - 1) / MC, batch), block(256);
-    if (grid.y > 65535) return fail(TLLM_ERR_ARG, "tllm_ter_spmm: too many rows for one call");
     cudaStream_t st = (cudaStream_t)stream;
-    if (x_dtype == TLLM_I8)
-        mcsc_spmm_kernel<int, MC><<<grid, block, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, rows, columns, inners, tile_k, scale);
-    else
-        mcsc_spmm_kernel<float, MC><<<grid, block, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, rows, columns, inners, tile_k, scale);
-    CU_TRY(cudaGetLastError());
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return TLLM_OK;
+    int dev = 0, sms = 0;
+    CU_TRY(cudaGetDevice(&dev));
+    if (mm_min_rows() == -1 && lists_worth_converting((long long)columns * inners, x_layout == TLLM_ROW_MAJOR ? (int)std::min(rows * (long long)batch, 0x7fffffffLL) : rows) && (x_dtype != TLLM_I8 || inners <= 131072) && tensor_map_encoder() != nullptr) {
+        const int rc2 = device_sms_cached(dev, &sms);
+        if (rc2) return rc2;
+        return run_lists(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, rows, columns, inners, tile_k, scale, dev, sms, st);
+    }
+    return run_mcsc(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, rows, columns, inners, tile_k, scale, nullptr, 0, 0, st);
 }
 
 int tllm_weight_create_dense(const int8_t* w, int inners, int columns, float scale, const tllm_pack_opts* opts, tllm_weight** out) {
@@ -1542,9 +1638,9 @@ int tllm_mlp_forward_ex(tllm_mlp* m, const void* X, int x_dtype, int rows, void*
         const int ld = (m->inter + 7) / 8 * 8;
         rc = ws.take(m->gate_up->device, (size_t)3 * rows * ld * 2, st);
         if (rc) return rc;
-        rc = run_mm(m->gate_up, X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows, ws.ptr, x_dtype, ld, 1, m->s_gate, m->s_up, st, false, true, (long long)rows * ld);
+        rc = run_mm(bits_view(m->gate_up), X, x_dtype, TLLM_ROW_MAJOR, m->hidden, rows, ws.ptr, x_dtype, ld, 1, m->s_gate, m->s_up, st, false, true, (long long)rows * ld);
         if (rc) return rc;
-        return run_mm_planes(m->down, (const unsigned short*)ws.ptr, rows, (size_t)ld * 2, rows, Y, y_dtype, m->hidden, m->down->scale, st);
+        return run_mm_planes(bits_view(m->down), (const unsigned short*)ws.ptr, rows, (size_t)ld * 2, rows, Y, y_dtype, m->hidden, m->down->scale, st);
     }
     char* h = (char*)(H ? H : m->d_h);
     const size_t h_bytes = (size_t)rows * m->inter * dtype_size(x_dtype);

@@ -153,17 +153,13 @@ __device__ __forceinline__ int staged_act<int>(const unsigned char* st, int dtyp
 __device__ __forceinline__ uint32_t act_bytes(int dtype) { return dtype == TLLM_F32 ? 4u : (dtype == TLLM_I8 ? 1u : 2u); }
 
 // ---------------------------------------------------------------------------------------------------
-// product on the reference's merged tiled CSC arrays: one warp per column, MC rows per pass
+// product on the reference's merged tiled CSC arrays: one warp per column, MC rows per pass (grid: columns / 8, rows / MC, batch)
 // ---------------------------------------------------------------------------------------------------
+#define MCSC_ROWS 4
 template <typename ACC, int MC>
-__global__ void __launch_bounds__(256) mcsc_spmm_kernel(const void* __restrict__ X, int x_dtype, int x_layout,
-                                                         const int16_t* __restrict__ idx, const int32_t* __restrict__ off,
-                                                         void* __restrict__ Y, int y_dtype, int M, int N, int K, int T, float scale) {
-    const int warp_in_block = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = blockIdx.x * (blockDim.x >> 5) + warp_in_block;
-    const int m0 = blockIdx.y * MC;
-    const size_t batch = blockIdx.z;
-    if (n >= N) return;
+__device__ __forceinline__ void mcsc_item(const void* __restrict__ X, int x_dtype, int x_layout, const int16_t* __restrict__ idx, const int32_t* __restrict__ off,
+                                          void* __restrict__ Y, int y_dtype, int M, int N, int K, int T, float scale, int n, int m0, size_t batch) {
+    const int lane = threadIdx.x & 31;
     const int tiles = (K + T - 1) / T;
     const size_t xb = batch * (size_t)M * K;
     auto xat = [&](int m, int k) -> ACC {
@@ -203,6 +199,31 @@ __global__ void __launch_bounds__(256) mcsc_spmm_kernel(const void* __restrict__
             if (y_dtype == TLLM_I32) ((int*)Y)[at] = (int)v;
             else store_out(Y, y_dtype, at, (float)v * scale);
         }
+    }
+}
+template <typename ACC, int MC>
+__global__ void __launch_bounds__(256) mcsc_spmm_kernel(const void* __restrict__ X, int x_dtype, int x_layout,
+                                                         const int16_t* __restrict__ idx, const int32_t* __restrict__ off,
+                                                         void* __restrict__ Y, int y_dtype, int M, int N, int K, int T, float scale) {
+    const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (n < N) mcsc_item<ACC, MC>(X, x_dtype, x_layout, idx, off, Y, y_dtype, M, N, K, T, scale, n, blockIdx.y * MC, blockIdx.z);
+}
+// the same on a grid of any size, and only if one of the nflags words is not zero (lists_kernel.cuh found lists that bit tiles
+// cannot hold, or the product on them gave up)
+template <typename ACC, int MC>
+__global__ void __launch_bounds__(256) mcsc_spmm_if_kernel(const void* __restrict__ X, int x_dtype, int x_layout,
+                                                            const int16_t* __restrict__ idx, const int32_t* __restrict__ off,
+                                                            void* __restrict__ Y, int y_dtype, int B, int M, int N, int K, int T, float scale, const int* flags,
+                                                            int nflags) {
+    int any = 0;
+    for (int i = threadIdx.x; i < nflags; i += blockDim.x) any |= __ldcg(flags + i);
+    if (!__syncthreads_or(any)) return;
+    const long long blocks_n = (N + 7) / 8, blocks_m = (M + MC - 1) / MC;
+    for (long long item = blockIdx.x; item < blocks_n * blocks_m * B; item += gridDim.x) {
+        const int n = (int)(item % blocks_n) * 8 + (int)(threadIdx.x >> 5);
+        if (n < N)
+            mcsc_item<ACC, MC>(X, x_dtype, x_layout, idx, off, Y, y_dtype, M, N, K, T, scale, n, (int)(item / blocks_n % blocks_m) * MC,
+                               (size_t)(item / (blocks_n * blocks_m)));
     }
 }
 

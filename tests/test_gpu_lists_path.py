@@ -1,0 +1,57 @@
+"""ter_spmm on the reference's arrays with enough rows: the lists are turned into two-bit tiles on the device first
+(csrc/lists_kernel.cuh).  Pinned by the oracle's product on the arrays themselves, exact on integers; lists that bit tiles
+cannot hold (an entry named twice, a pair that cancels across lists) fall back to the per-column kernel inside the same call."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from conftest import random_ternary
+from ternaryllm_b200 import ter_spmm
+
+pytestmark = pytest.mark.gpu
+DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16, "i8": torch.int8}
+
+
+def call(x, idx, off, N, K, T, dtype, col_major=False):
+    B, M = x.shape[:2]
+    X = torch.tensor(x, dtype=DT[dtype], device="cuda")
+    if col_major:
+        X = X.transpose(1, 2).contiguous()
+    ri = torch.tensor(np.asarray(idx).astype(np.int16), device="cuda")
+    co = torch.tensor(np.asarray(off).astype(np.int32), device="cuda")
+    return ter_spmm.ter_spmm(X, ri, co, None, B, M, N, K, False, False, tile_k=T).double().cpu().numpy()
+
+
+# one slice, odd slices, tiles of many sizes, several images per block (K > 8192), no full tile of columns
+@pytest.mark.parametrize("K,N,T,s", [(40, 3, 16, 0.3), (64, 16, 64, 0.5), (200, 130, 64, 0.6), (1000, 70, 256, 0.5), (2048, 300, 256, 0.9), (9000, 40, 512, 0.6),
+                                     (8256, 20, 100, 0.5)])
+@pytest.mark.parametrize("padding", [0, 4])
+def test_exact_on_integer_activations(K, N, T, s, padding):
+    rng = np.random.default_rng(K + N)
+    w = random_ternary(rng, K, N, s).astype(np.int32)
+    idx, off, _ = ter_spmm.convert_to_ter_tiled_mcsc(w, N, K, int((w == 1).sum()), int((w == -1).sum()), T, bool(padding), padding or 4, as_numpy=True)
+    for dtype, top in (("f32", 100), ("bf16", 1), ("i8", 127)):
+        for B, M in ((1, 8), (3, 3), (2, 1200)) if K * N < 100000 else ((1, 80), (3, 30)):
+            x = rng.integers(-top, top + 1, size=(B, M, K)).astype(np.float64)
+            want = np.stack([oracle.dense_f64(x[b], w.astype(np.int8)) for b in range(B)])
+            if dtype == "bf16":
+                want = oracle.round_to(want, 2)
+            assert np.array_equal(call(x, idx, off, N, K, T, dtype), want), (dtype, B, M)
+            if M != K:
+                assert np.array_equal(call(x, idx, off, N, K, T, dtype, col_major=True), want), (dtype, B, M)
+
+
+def test_lists_that_bit_tiles_cannot_hold():
+    rng = np.random.default_rng(3)
+    K, N, T, M = 512, 64, 64, 800
+    w = random_ternary(rng, K, N, 0.5).astype(np.int32)
+    idx, off, _ = ter_spmm.convert_to_ter_tiled_mcsc(w, N, K, int((w == 1).sum()), int((w == -1).sum()), T, False, 4, as_numpy=True)
+    x = rng.integers(-50, 51, size=(1, M, K)).astype(np.float64)
+    o = off.reshape(N, K // T, 4)
+    for column, tile in ((0, 0), (17, 3), (63, 7)):
+        bad = idx.copy()
+        bad[o[column, tile, 0]] = bad[o[column, tile, 0] + 2]          # the first two pairs name the same +1 row
+        want = oracle.mcsc_product_f64(x[0], bad, off, N, K, T)
+        assert not np.array_equal(want, oracle.dense_f64(x[0], w.astype(np.int8)))
+        assert np.array_equal(call(x, bad, off, N, K, T, "f32")[0], want)
