@@ -50,7 +50,8 @@ struct BitsParams {
     const void* X;
     void* Y;
     int x_dtype, x_layout, x_ld;   // row-major X: elements between rows; column-major X: elements between k
-    int y_dtype, y_ld, epilogue;   // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
+    int y_dtype, epilogue;         // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
+    long long y_step_n, y_step_m;  // elements from column to column and from row to row of Y
     int M, K, N, KB;               // KB = ceil(K / 64) slices
     int own, own_more;             // groups of sixteen columns per block; the first own_more blocks have one more
     int per_pass;                  // groups per pass (<= split * GR)
@@ -410,12 +411,13 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
             const int n = (c0 + q0 + j) * 16 + c;
             if (p.epilogue == 0) {
                 if (valid && n < p.N) {
-                    if (p.y_dtype == TLLM_I32) ((int*)p.Y)[(size_t)m * p.y_ld + n] = (int)(v * 0.5f);
-                    else store_out(p.Y, p.y_dtype, (size_t)m * p.y_ld + n, v * p.scale);
+                    const size_t at = (size_t)m * p.y_step_m + (size_t)n * p.y_step_n;
+                    if (p.y_dtype == TLLM_I32) ((int*)p.Y)[at] = (int)(v * 0.5f);
+                    else store_out(p.Y, p.y_dtype, at, v * p.scale);
                 }
             } else {
                 const float u = __shfl_xor_sync(0xffffffffu, v, 1);
-                if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_ld + (n >> 1), silu_mul(v * p.scale, u * p.scale2));
+                if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(v * p.scale, u * p.scale2));
             }
         }
     }

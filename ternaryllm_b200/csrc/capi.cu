@@ -130,9 +130,8 @@ struct tllm_weight {
     void* d_x = nullptr;
     void* d_y = nullptr;
     void* d_bias = nullptr;
-    void* h_pin = nullptr;
     int* h_status = nullptr;        // pinned copy of the status word, read back with every host-buffer call
-    size_t x_cap = 0, y_cap = 0, bias_cap = 0, pin_cap = 0;
+    size_t x_cap = 0, y_cap = 0, bias_cap = 0;
     cudaStream_t own_stream = nullptr;
     // tensor-core kernel: dense two-bit copy of W and its split scratch
     uint4* d_bits = nullptr;
@@ -721,12 +720,13 @@ int run_nb(tllm_weight* w, const void* X, int x_dtype, int x_ld, int rows, void*
 int bt_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? BT_MAX_ROWS / 2 : BT_MAX_ROWS; }
 
 int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
-             float scale2, cudaStream_t st) {
+             float scale2, cudaStream_t st, bool y_col = false) {
     BitsParams p{};
     p.pdl = w.pdl;
     p.bits = w.bits;
     p.x_dtype = x_dtype, p.x_layout = x_layout, p.x_ld = x_ld;
-    p.y_dtype = y_dtype, p.y_ld = y_ld, p.epilogue = epilogue;
+    p.y_dtype = y_dtype, p.epilogue = epilogue;
+    p.y_step_n = y_col ? y_ld : 1, p.y_step_m = y_col ? 1 : y_ld;
     p.K = w.inners, p.N = w.columns, p.KB = w.kb;
     p.scale = scale * 0.5f, p.scale2 = scale2 * 0.5f;            // the decoded weights are +-2
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
@@ -734,7 +734,7 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
     for (int r0 = 0; r0 < rows; r0 += per) {
         p.M = rows - r0 < per ? rows - r0 : per;
         p.X = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
-        p.Y = (char*)Y + (size_t)r0 * y_ld * ye;
+        p.Y = (char*)Y + (size_t)r0 * p.y_step_m * ye;
         const int rc = bits_launch(p, w.sms, w.device, st);
         if (rc) return rc;
     }
@@ -853,15 +853,36 @@ int run_gather(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_l
     return TLLM_OK;
 }
 
-// the product of `rows` rows on the kernel that choose_kernel names
+// [rows][columns] -> [columns][ld], elements of e bytes, on the device
+int turn_out(const void* src, void* dst, int rows, int columns, int ld, int e, cudaStream_t st) {
+    const dim3 grid((columns + 31) / 32, (rows + 31) / 32), block(32, 8);
+    if (e == 4) turn_kernel<uint32_t><<<grid, block, 0, st>>>((const uint32_t*)src, (uint32_t*)dst, rows, columns, ld);
+    else turn_kernel<uint16_t><<<grid, block, 0, st>>>((const uint16_t*)src, (uint16_t*)dst, rows, columns, ld);
+    CU_TRY(cudaGetLastError());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TLLM_OK;
+}
+
+// the product of `rows` rows on the kernel that choose_kernel names.  y_col: Y is column-major (y_ld elements from column to
+// column), which the two kernels on bit tiles write themselves; for the others it is turned out of a workspace.
 int run_product(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
-                float scale2, cudaStream_t st) {
-    switch (choose_kernel(w, X, x_dtype, x_layout, x_ld, rows)) {
-        case KERNEL_BITS: return run_bits(bits_view(w), X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
-        case KERNEL_NIBBLE: return run_nb(w, X, x_dtype, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
-        case KERNEL_MMA: return run_mm(bits_view(w), X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st);
-        default: return run_gather(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, Scratch{w->d_partial, w->d_counters}, st);
+                float scale2, cudaStream_t st, bool y_col = false) {
+    const KernelChoice kc = choose_kernel(w, X, x_dtype, x_layout, x_ld, rows);
+    if (kc == KERNEL_BITS) return run_bits(bits_view(w), X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st, y_col);
+    if (kc == KERNEL_MMA) return run_mm(bits_view(w), X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, y_ld, epilogue, scale, scale2, st, y_col);
+    Workspace ws;
+    void* out = Y;
+    int ld = y_ld;
+    if (y_col) {
+        ld = w->lay.columns;
+        const int rc = ws.take(w->device, (size_t)rows * ld * dtype_size(y_dtype), st);
+        if (rc) return rc;
+        out = ws.ptr;
     }
+    const int rc = kc == KERNEL_NIBBLE ? run_nb(w, X, x_dtype, x_ld, rows, out, y_dtype, ld, epilogue, scale, scale2, st)
+                                       : run_gather(w, X, x_dtype, x_layout, x_ld, rows, out, y_dtype, ld, epilogue, scale, scale2, Scratch{w->d_partial, w->d_counters}, st);
+    if (rc || !y_col) return rc;
+    return turn_out(out, Y, rows, ld, y_ld, (int)dtype_size(y_dtype), st);
 }
 
 int upload(tllm_weight* w, const BsHostImage& img, float scale, int max_rows) {
@@ -1273,7 +1294,6 @@ int tllm_weight_destroy(tllm_weight* w) {
     cudaFree(w->d_x);
     cudaFree(w->d_y);
     cudaFree(w->d_bias);
-    if (w->h_pin) cudaFreeHost(w->h_pin);
     if (w->h_status) cudaFreeHost(w->h_status);
     if (w->own_stream) cudaStreamDestroy(w->own_stream);
     delete w;
@@ -1452,28 +1472,30 @@ int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout
         if (r) return r;
         CU_TRY(cudaMemcpyAsync(w->d_bias, bias, (size_t)L.columns * dtype_size(y_dtype), cudaMemcpyHostToDevice, w->own_stream));
     }
-    r = tllm_spmm(w, w->d_x, x_dtype, x_layout, rows, w->d_y, y_dtype, w->own_stream);
-    if (r) return r;
-    if (bias) {
-        r = add_bias(w->d_y, w->d_bias, y_dtype, rows, L.columns, w->own_stream);
+    // A column-major result leaves the kernels in that layout; a bias is added to rows first.
+    const bool y_col = y_layout != TLLM_ROW_MAJOR && rows > 1;
+    const int x_ld = x_layout == TLLM_ROW_MAJOR ? L.inners : rows;
+    void* out = w->d_y;
+    if (!bias) {
+        r = run_product(w, w->d_x, x_dtype, x_layout, x_ld, rows, out, y_dtype, y_col ? rows : L.columns, 0, w->scale, 0.f, w->own_stream, y_col);
         if (r) return r;
-    }
-    if (y_layout == TLLM_ROW_MAJOR) {
-        CU_TRY(cudaMemcpyAsync(Y, w->d_y, yb, cudaMemcpyDeviceToHost, w->own_stream));
-        CU_TRY(cudaMemcpyAsync(w->h_status, w->d_status, sizeof(int), cudaMemcpyDeviceToHost, w->own_stream));
-        CU_TRY(cudaStreamSynchronize(w->own_stream));
     } else {
-        r = ensure(&w->h_pin, &w->pin_cap, yb, true);
+        r = run_product(w, w->d_x, x_dtype, x_layout, x_ld, rows, out, y_dtype, L.columns, 0, w->scale, 0.f, w->own_stream);
         if (r) return r;
-        CU_TRY(cudaMemcpyAsync(w->h_pin, w->d_y, yb, cudaMemcpyDeviceToHost, w->own_stream));
-        CU_TRY(cudaMemcpyAsync(w->h_status, w->d_status, sizeof(int), cudaMemcpyDeviceToHost, w->own_stream));
-        CU_TRY(cudaStreamSynchronize(w->own_stream));
-        const size_t e = dtype_size(y_dtype);
-        const char* src = (const char*)w->h_pin;
-        char* dst = (char*)Y;
-        for (int m = 0; m < rows; ++m)
-            for (int n = 0; n < L.columns; ++n) std::memcpy(dst + ((size_t)n * rows + m) * e, src + ((size_t)m * L.columns + n) * e, e);
+        r = add_bias(out, w->d_bias, y_dtype, rows, L.columns, w->own_stream);
+        if (r) return r;
     }
+    Workspace ws;
+    if (bias && y_col) {
+        r = ws.take(w->device, yb, w->own_stream);
+        if (r) return r;
+        r = turn_out(out, ws.ptr, rows, L.columns, rows, (int)dtype_size(y_dtype), w->own_stream);
+        if (r) return r;
+        out = ws.ptr;
+    }
+    CU_TRY(cudaMemcpyAsync(w->h_status, w->d_status, sizeof(int), cudaMemcpyDeviceToHost, w->own_stream));
+    CU_TRY(cudaMemcpyAsync(Y, out, yb, cudaMemcpyDeviceToHost, w->own_stream));
+    CU_TRY(cudaStreamSynchronize(w->own_stream));
     // the status word came back with the result; only a non-zero one needs the (synchronising) full check
     return *w->h_status ? tllm_weight_check(w) : TLLM_OK;
 }

@@ -227,6 +227,20 @@ __global__ void __launch_bounds__(256) mcsc_spmm_if_kernel(const void* __restric
     }
 }
 
+// dst[c][r] = src[r][c] (ld elements from c to c), 32 x 32 tiles through shared memory; block (32, 8)
+template <typename T>
+__global__ void __launch_bounds__(256) turn_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int columns, int ld) {
+    __shared__ T tile[32][33];
+    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, x = threadIdx.x;
+#pragma unroll
+    for (int i = threadIdx.y; i < 32; i += 8)
+        if (r0 + i < rows && c0 + x < columns) tile[i][x] = src[(size_t)(r0 + i) * columns + c0 + x];
+    __syncthreads();
+#pragma unroll
+    for (int i = threadIdx.y; i < 32; i += 8)
+        if (c0 + i < columns && r0 + x < rows) dst[(size_t)(c0 + i) * ld + r0 + x] = tile[x][i];
+}
+
 // g[i] = silu(g[i]) * u[i]
 static __global__ void silu_mul_kernel(void* g, const void* u, int dtype, long long n) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

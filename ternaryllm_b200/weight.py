@@ -24,6 +24,9 @@ def _dense_i8(w):
     return w
 
 
+_HOST_CODES = {np.dtype(np.float32): _lib.F32, np.dtype(np.float16): _lib.F16, np.dtype(np.int8): _lib.I8}
+
+
 class PackedWeight:
     """A ternary matrix W [inners, columns] packed into the bank-stream format on the current CUDA device."""
 
@@ -119,19 +122,14 @@ class PackedWeight:
 
     def matmul_host(self, x, col_major=False, y_col_major=False):
         """Same on numpy host arrays (copies in, runs, copies out, synchronises): the CPU entry points' form."""
-        import torch
-
         x = np.ascontiguousarray(x)
-        code = {np.dtype(np.float32): _lib.F32, np.dtype(np.float16): _lib.F16, np.dtype(np.int8): _lib.I8}[x.dtype]
-        info = self.info
+        code = _HOST_CODES[x.dtype]
+        c = self._call or self._bind()
         rows = x.shape[1] if col_major else x.shape[0]
-        ydt = np.int32 if x.dtype == np.int8 else x.dtype
-        y = np.empty((info["columns"], rows) if y_col_major else (rows, info["columns"]), ydt)
-        with torch.cuda.device(self.device_index):
-            check(lib().tllm_spmm_host(self._h, np_ptr(x), code, _lib.COL_MAJOR if col_major else _lib.ROW_MAJOR, rows, np_ptr(y),
-                                       _lib.I32 if x.dtype == np.int8 else code, _lib.COL_MAJOR if y_col_major else _lib.ROW_MAJOR),
-                  "tllm_spmm_host")
-        return y
+        if x.ndim != 2 or x.shape[0 if col_major else 1] != c[3]:
+            raise RuntimeError(f"activation has {x.shape} but the weight has {c[3]} inners")
+        y_rows, y_cols = (c[4], rows) if y_col_major else (rows, c[4])
+        return _lib.binding().matmul_host(c[1], x, code, bool(col_major), rows, y_rows, y_cols, _lib.I32 if code == _lib.I8 else code, bool(y_col_major), c[2]).numpy()
 
     def close(self):
         if self._h:
