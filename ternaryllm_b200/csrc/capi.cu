@@ -1741,10 +1741,9 @@ int tllm_add_rmsnorm(void* x, const void* delta, const void* weight, void* h, in
         return fail(TLLM_ERR_ARG, "tllm_add_rmsnorm: hidden must be a multiple of %d and the pointers 16-byte aligned", vec);
     if (rows == 0) return TLLM_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    if (dtype == TLLM_F32) add_rmsnorm_kernel<float><<<(unsigned)rows, 256, 0, st>>>((float*)x, (const float*)delta, (const float*)weight, (float*)h, hidden, eps);
-    else if (dtype == TLLM_F16) add_rmsnorm_kernel<__half><<<(unsigned)rows, 256, 0, st>>>((__half*)x, (const __half*)delta, (const __half*)weight, (__half*)h, hidden, eps);
-    else add_rmsnorm_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>((__nv_bfloat16*)x, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)weight, (__nv_bfloat16*)h, hidden, eps);
-    CU_TRY(cudaGetLastError());
+    if (dtype == TLLM_F32) CU_TRY((launch_add_rmsnorm<float, float>(x, delta, weight, h, rows, hidden, eps, st)));
+    else if (dtype == TLLM_F16) CU_TRY((launch_add_rmsnorm<__half, __half>(x, delta, weight, h, rows, hidden, eps, st)));
+    else CU_TRY((launch_add_rmsnorm<__nv_bfloat16, __nv_bfloat16>(x, delta, weight, h, rows, hidden, eps, st)));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
 }

@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/tllm.h"
 
 namespace tllm {
@@ -261,8 +263,8 @@ static __global__ void bias_add_kernel(void* y, const void* bias, int dtype, lon
 // Residual add and RMS normalisation of one row per block, the glue between two ternary products of a decoder
 // layer:  x[r] += delta[r] (when delta is given, rounded once to x's type);  h[r] = x[r] * rsqrt(mean(x[r]^2) + eps)
 // * weight (weight = 1 when absent).  Sums in fp32; x, delta, h and weight share one 16-bit or 32-bit float type.
-// A thread keeps up to four 16-byte vectors of its row in registers between the two passes (rows of up to
-// 8192 16-bit or 4096 32-bit values are read once); longer rows re-read the remainder.
+// A thread keeps up to two 16-byte vectors of its row in registers between the two passes (rows of up to 8192 16-bit or
+// 4096 32-bit values are read once); longer rows re-read the remainder.
 template <typename T>
 struct RmsVec;   // 16 bytes of T as floats
 template <>
@@ -318,20 +320,46 @@ struct RmsVec<__nv_bfloat16> {
     static __device__ __forceinline__ float round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 };
 
-// hidden must be a multiple of the vector width and all pointers 16-byte aligned (checked by the caller)
-template <typename T>
-__global__ void __launch_bounds__(256) add_rmsnorm_kernel(T* x, const T* delta, const T* weight, T* h, int hidden, float eps) {
-    constexpr int N = RmsVec<T>::N, KEEP = 4;
-    __shared__ float red[8];
+// N consecutive values of delta: of x's type, or fp32 sums
+template <typename T, typename D>
+__device__ __forceinline__ void rms_load_delta(const D* p, float (&v)[8]) {
+    if constexpr (std::is_same<T, D>::value) RmsVec<T>::load(p, v);
+    else {
+#pragma unroll
+        for (int i = 0; i < RmsVec<T>::N; i += 4) {
+            const float4 a = __ldcg((const float4*)(p + i));
+            v[i] = a.x, v[i + 1] = a.y, v[i + 2] = a.z, v[i + 3] = a.w;
+        }
+    }
+}
+
+// hidden must be a multiple of the vector width and all pointers 16-byte aligned (checked by the caller).  D: type of delta.
+// Bound by latency (a row is a few KiB): one load round trip, one block reduction, one store; blocks of 256 threads for rows of up
+// to 256 vectors, 512 above, so that a thread holds one or two vectors.
+#define RMS_MAX_THREADS 512
+template <typename T, typename D>
+__global__ void __launch_bounds__(RMS_MAX_THREADS) add_rmsnorm_kernel(T* x, const D* delta, const T* weight, T* h, int hidden, float eps) {
+    constexpr int N = RmsVec<T>::N, KEEP = 2;
+    __shared__ float red[RMS_MAX_THREADS / 32];
+    const int nt = blockDim.x;
     const size_t row = (size_t)blockIdx.x * hidden;
     const int nvec = hidden / N;
-    float keep[KEEP][8];
+    float keep[KEEP][8], gain[KEEP][8];
     float ss = 0.f;
+    pdl_launch_dependents();
+    if (weight) {                       // does not depend on the preceding kernel
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int vi = threadIdx.x + k * nt;
+            if (vi < nvec) RmsVec<T>::load(weight + (size_t)vi * N, gain[k]);
+        }
+    }
+    pdl_wait();
     auto first_pass = [&](int vi, float (&v)[8]) {
+        float d[8];
         RmsVec<T>::load(x + row + (size_t)vi * N, v);
         if (delta) {
-            float d[8];
-            RmsVec<T>::load(delta + row + (size_t)vi * N, d);
+            rms_load_delta<T, D>(delta + row + (size_t)vi * N, d);
 #pragma unroll
             for (int i = 0; i < N; ++i) v[i] = RmsVec<T>::round(v[i] + d[i]);
             RmsVec<T>::store(x + row + (size_t)vi * N, v);
@@ -341,10 +369,10 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(T* x, const T* delta, 
     };
 #pragma unroll
     for (int k = 0; k < KEEP; ++k) {
-        const int vi = threadIdx.x + k * 256;
+        const int vi = threadIdx.x + k * nt;
         if (vi < nvec) first_pass(vi, keep[k]);
     }
-    for (int vi = threadIdx.x + KEEP * 256; vi < nvec; vi += 256) {
+    for (int vi = threadIdx.x + KEEP * nt; vi < nvec; vi += nt) {
         float v[8];
         first_pass(vi, v);
     }
@@ -353,31 +381,38 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(T* x, const T* delta, 
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
     float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) tot += red[w];
+    for (int w = 0; w < nt / 32; ++w) tot += red[w];
     const float inv = rsqrtf(tot / (float)hidden + eps);
-    auto second_pass = [&](int vi, float (&v)[8]) {
-        if (weight) {
-            float g[8];
-            RmsVec<T>::load(weight + (size_t)vi * N, g);
+    auto second_pass = [&](int vi, float (&v)[8], const float (&g)[8]) {
 #pragma unroll
-            for (int i = 0; i < N; ++i) v[i] = v[i] * inv * g[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < N; ++i) v[i] = v[i] * inv;
-        }
+        for (int i = 0; i < N; ++i) v[i] = weight ? v[i] * inv * g[i] : v[i] * inv;
         RmsVec<T>::store(h + row + (size_t)vi * N, v);
     };
 #pragma unroll
     for (int k = 0; k < KEEP; ++k) {
-        const int vi = threadIdx.x + k * 256;
-        if (vi < nvec) second_pass(vi, keep[k]);
+        const int vi = threadIdx.x + k * nt;
+        if (vi < nvec) second_pass(vi, keep[k], gain[k]);
     }
-    for (int vi = threadIdx.x + KEEP * 256; vi < nvec; vi += 256) {
-        float v[8];
+    for (int vi = threadIdx.x + KEEP * nt; vi < nvec; vi += nt) {
+        float v[8], g[8] = {};
         RmsVec<T>::load(x + row + (size_t)vi * N, v);     // written by this thread in the first pass, or untouched
-        second_pass(vi, v);
+        if (weight) RmsVec<T>::load(weight + (size_t)vi * N, g);
+        second_pass(vi, v, g);
     }
+}
+
+template <typename T, typename D>
+inline cudaError_t launch_add_rmsnorm(void* x, const void* delta, const void* weight, void* h, int rows, int hidden, float eps, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)rows);
+    cfg.blockDim = dim3(hidden / RmsVec<T>::N <= 256 ? 256 : RMS_MAX_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, add_rmsnorm_kernel<T, D>, (T*)x, (const D*)delta, (const T*)weight, (T*)h, hidden, eps);
 }
 
 }  // namespace tllm
