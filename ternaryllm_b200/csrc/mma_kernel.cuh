@@ -12,9 +12,10 @@
 // X comes in one or three planes of 16-bit values.  fp16 / bf16 activations whose rows TMA can address are read where they
 // are (one plane).  Everything else passes through stage_acts_kernel: int8 becomes fp16 (exact), rows on odd addresses and
 // column-major activations are copied straight, and an fp32 value becomes three bf16 values of eight significant bits that
-// add up to it exactly; the three planes of a slice are multiplied with the same expanded slice of W, the first into one
-// accumulator, the two small ones into another: the tensor core truncates its sums, and with all three in one accumulator
-// every step would cut bits (1e-5 of the result at K = 4096, against 1e-7).
+// add up to it exactly.  The planes of a row tile are rows of one B operand, 3 * Nt of them, each with its own columns of D, so
+// an MMA does the three at once (three MMAs of Nt columns each instead were bound by their issue: 20 us against 12 for 256 rows
+// of 2048 x 2048); D's planes are added in the epilogue, the small ones first.  (The tensor core truncates its sums: with the
+// planes in one accumulator every step would cut bits, 1e-5 of the result at K = 4096 against 1e-7.)
 //
 // One persistent block per SM, twenty-three warps:
 //   warp 0        streams this block's range of bit tiles into a shared-memory ring (TMA)
@@ -27,7 +28,7 @@
 // MMA 40 to issue, so that sixteen MMAs of 128 x 128 x 16 (1270 clocks) hide it and eight do not (measured at 5120 x 15360, 2048
 // rows: 285 us with two slices per unit, 183 with the MMAs alone).  A has a ring of two units (256 columns of tensor memory;
 // the accumulators have the other 256: two of them where they fit, so that the epilogue of one tile runs beside the next),
-// B one of (unit, plane).
+// B one of units.
 // Work is either whole output tiles or, where those would leave SMs idle, the flattened list of (output tile, unit) pairs
 // cut into equal contiguous ranges, one per block.  Tiles that straddle two or more blocks are summed in block order by the
 // last block to arrive, which makes the result independent of scheduling; a block does its two shared tiles first, so that
@@ -52,7 +53,7 @@ namespace tllm {
 #define MM_A_COL 256
 #define MM_MAX_STAGES 8
 #define MM_THREADS (23 * 32)
-#define MM_MAX_NT 128                 // activation rows per tile (the MMA's N), a multiple of sixteen
+#define MM_MAX_COLS 192               // columns of D of a tile = planes * Nt, Nt (activation rows) a multiple of sixteen
 #define MM_OWN_NT 64                  // a handle's own hand-over scratch is for tiles of up to this many rows
 #define MM_MAX_M_TILES 16             // row tiles of one launch
 // what a result is stored as
@@ -76,14 +77,14 @@ struct MmParams {
     int KB;                   // ceil(K / 64): slices
     int KBU;                  // ceil(KB / 4): units per tile
     int n_tiles, m_tiles;
-    int Nt;                   // activation rows per tile
+    int Nt;                   // activation rows per tile; planes * Nt is the MMA's N
     int split;                // 1: equal unit ranges, tiles may be shared; 0: whole tiles
-    int P, plane_rows;        // planes of X; rows from one plane to the next in the tensor map
+    int P;                    // planes of X
     int out;                  // MM_OUT_*
     int epilogue, y_ld;       // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
     long long y_step_n, y_step_m;   // elements from column to column and from row to row (epilogue 0)
     long long plane_y;        // MM_OUT_PLANES: elements from plane to plane
-    int SB, R;                // ring lengths: (unit, plane) pairs of B, units of bit tiles
+    int SB, R;                // ring lengths: units of B, units of bit tiles
     uint32_t idesc;           // tcgen05 instruction descriptor
     uint32_t mul4, mul16;     // 4 and 16
     float scale, scale2;      // half the product's scales: the decoded weights are 0 / +-2
@@ -139,6 +140,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
                  "l"(map), "r"(bar), "r"(c0), "r"(c1)
+                 : "memory");
+}
+// coordinates (element along K, activation row, plane)
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                 "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
                  : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -376,7 +383,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     const uint32_t base = (raw0 + 1023u) & ~1023u;                 // swizzled tiles need 1024-byte alignment
     const uint32_t SB = (uint32_t)p.SB, R = (uint32_t)p.R;
     const int Nt = p.Nt;
-    const uint32_t b_slice = (uint32_t)Nt * 128u, b_unit = MM_UK * b_slice;
+    const uint32_t acc_cols = (uint32_t)(p.P * Nt), b_slice = acc_cols * 128u, b_unit = MM_UK * b_slice;
     const uint32_t b_base = base, r_base = b_base + SB * b_unit;
     const uint32_t bar_base = r_base + R * MM_UNIT_BYTES;
     volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 52);   // [0] tensor-memory address, [1] abort
@@ -414,7 +421,6 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = (uint32_t)flags[0];
-    const uint32_t acc_cols = p.P == 1 ? (uint32_t)Nt : 2u * (uint32_t)Nt;
     const uint32_t accs = 2u * acc_cols <= MM_A_COL ? 2u : 1u;
     pdl_launch_dependents();
 
@@ -439,7 +445,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             }
         }
     } else if (warp == 6) {
-        // ---- activation producer: a unit and plane is four TMA boxes on one barrier (whole warp converged, one elected lane per
+        // ---- activation producer: a unit is four TMA boxes (all planes of a slice each) on one barrier (whole warp converged, one elected lane per
         // instruction: addresses and coordinates then are warp-uniform values)
         pdl_wait();
         uint32_t b = 0, bph = 0;
@@ -449,17 +455,23 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             const int row0 = (tile % p.m_tiles) * Nt;
             for (int ku = ua; ku < ub; ++ku) {
                 const int nk = min(MM_UK, KB - ku * MM_UK);
-                for (int pl = 0; pl < p.P; ++pl) {
-                    MM_WAIT(B_EMPTY(b), bph ^ 1u);
-                    if (elect_one()) {
-                        mbar_expect_tx(B_FULL(b), (uint32_t)nk * b_slice);
+                MM_WAIT(B_EMPTY(b), bph ^ 1u);
+                if (elect_one()) {
+                    mbar_expect_tx(B_FULL(b), (uint32_t)nk * b_slice);
+                    // (three planes as three boxes a slice would be twelve instructions to issue; one plane as a box of three dimensions
+                    // measured 4 % slower than one of two)
+                    if (p.P == 1) {
 #pragma unroll
                         for (int h = 0; h < MM_UK; ++h)
-                            if (h < nk) tma_load_2d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * MM_UK + h) * MM_TILE_K, pl * p.plane_rows + row0, B_FULL(b));
+                            if (h < nk) tma_load_2d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * MM_UK + h) * MM_TILE_K, row0, B_FULL(b));
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < MM_UK; ++h)
+                            if (h < nk) tma_load_3d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * MM_UK + h) * MM_TILE_K, row0, 0, B_FULL(b));
                     }
-                    __syncwarp();
-                    MM_ADVANCE(b, bph, SB);
                 }
+                __syncwarp();
+                MM_ADVANCE(b, bph, SB);
             }
         }
     } else if (warp == 1) {
@@ -479,42 +491,37 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             tc_fence_after();
             for (int ku = ua; ku < ub; ++ku) {
                 const int nk = min(MM_UK, KB - ku * MM_UK);
-                const uint32_t at = tmem + MM_A_COL + sa * (MM_UK * 32u);
-                for (int pl = 0; pl < p.P; ++pl) {
-                    const uint32_t b_lo = b_lo0 + sb * (b_unit >> 4), sb0 = sb, sa0 = sa;
-                    const uint32_t dp = pl == 0 ? d : d + (uint32_t)Nt, keep = pl < 2 ? acc : 1u;
-                    const bool unit_done = pl == p.P - 1;
-                    // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
-                    if (elect_one()) {
+                const uint32_t at = tmem + MM_A_COL + sa * (MM_UK * 32u), b_lo = b_lo0 + sb * (b_unit >> 4), sb0 = sb, sa0 = sa;
+                // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
+                if (elect_one()) {
 #pragma unroll
-                        for (uint32_t h = 0; h < MM_UK - 1; ++h)
-                            if ((int)h < nk) {
-#pragma unroll
-                                for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
-                                    umma_f16_ts(dp, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, (h | k4) == 0 ? keep : 1u);
-                            }
-                    }
-                    __syncwarp();
-                    MM_ADVANCE(sb, sbph, SB);
-                    if (unit_done) MM_ADVANCE(sa, saph, MM_A_UNITS);
-                    // what comes next is waited for before the last slice goes out: the tensor core works on what is queued meanwhile
-                    if (!unit_done || ku + 1 < ub) {
-                        if (unit_done) MM_WAIT(A_FULL(sa), saph);
-                        MM_WAIT(B_FULL(sb), sbph);
-                        tc_fence_after();
-                    }
-                    if (elect_one()) {
-                        if (nk == MM_UK) {
-                            constexpr uint32_t h = MM_UK - 1;
+                    for (uint32_t h = 0; h < MM_UK - 1; ++h)
+                        if ((int)h < nk) {
 #pragma unroll
                             for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
-                                umma_f16_ts(dp, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, 1u);
+                                umma_f16_ts(d, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, (h | k4) == 0 ? acc : 1u);
                         }
-                        umma_commit(B_EMPTY(sb0));
-                        if (unit_done) umma_commit(A_EMPTY(sa0));
-                    }
-                    __syncwarp();
                 }
+                __syncwarp();
+                MM_ADVANCE(sb, sbph, SB);
+                MM_ADVANCE(sa, saph, MM_A_UNITS);
+                // what comes next is waited for before the last slice goes out: the tensor core works on what is queued meanwhile
+                if (ku + 1 < ub) {
+                    MM_WAIT(A_FULL(sa), saph);
+                    MM_WAIT(B_FULL(sb), sbph);
+                    tc_fence_after();
+                }
+                if (elect_one()) {
+                    if (nk == MM_UK) {
+                        constexpr uint32_t h = MM_UK - 1;
+#pragma unroll
+                        for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
+                            umma_f16_ts(d, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, 1u);
+                    }
+                    umma_commit(B_EMPTY(sb0));
+                    umma_commit(A_EMPTY(sa0));
+                }
+                __syncwarp();
                 acc = 1;
             }
             if (elect_one()) umma_commit(ACC_FULL(a));
@@ -592,9 +599,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 #pragma unroll
                 for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]);
                 if (p.P > 1) {
+                    uint32_t u[16];
                     tmem_ld16(taddr + (uint32_t)(Nt + c16), v);
+                    tmem_ld16(taddr + (uint32_t)(2 * Nt + c16), u);
 #pragma unroll
-                    for (int t = 0; t < 16; ++t) f[t] += __uint_as_float(v[t]);
+                    for (int t = 0; t < 16; ++t) f[t] += __uint_as_float(v[t]) + __uint_as_float(u[t]);
                 }
             };
             bool sum = false;                    // this block adds up the parts of a shared tile
