@@ -8,7 +8,8 @@ are this library's work; rotary embedding, softmax and the value product are pla
 * the three input projections run as **one** product on a packed weight whose columns are q | k | v (`fused_qkv`,
   default on; the reference issues three calls, :73-75) -- bias-free projections only;
 * the attention core is `scaled_dot_product_attention` (same arithmetic up to summation order), causal when no mask
-  is given and more than one query position is passed;
+  is given and more than one query position is passed -- or, for a plain prompt (no mask, cache or rotary embedding), the
+  library's own one-launch kernel;
 * the key / value cache is a plain `(k, v)` tuple passed in and returned, not a transformers `Cache` object;
 * rotary position embeddings are applied only when `position_embeddings=(cos, sin)` is passed; no rotary module is
   instantiated here.
@@ -21,9 +22,13 @@ import numpy as np
 import torch
 from torch import nn
 
+from . import _lib
 from .configuration_ternary import TernaryConfig
 from .TernaryLinear import TernaryLinear
 from .weight import PackedWeight
+
+
+_OWN_CORE_16BIT = 256 * 256 * 2048        # batch * positions^2 * heads * head_dim
 
 
 def _rotate_half(x):
@@ -64,6 +69,14 @@ class LlamaTernaryAttention(nn.Module):
             self._qkv[idx] = pw
         return pw
 
+    def _own_core(self, dtype, bsz, q_len) -> bool:
+        """Whether a plain causal prompt goes to the library's one-launch attention (fp32 arithmetic on the CUDA cores, from the
+        q | k | v product as it lies).  fp32: always, the stock path is a dozen launches.  16-bit: while the arithmetic is less than
+        the stock path's launches and copies cost; the tensor-core kernels behind it are faster on long prompts."""
+        if self.head_dim not in (64, 128) or bsz > 65535:
+            return False
+        return dtype == torch.float32 or bsz * q_len * q_len * self.num_heads * self.head_dim <= _OWN_CORE_16BIT
+
     def forward(self, hidden_states: torch.Tensor, attention_mask: Optional[torch.Tensor] = None,
                 position_embeddings: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
                 past_key_value: Optional[Tuple[torch.Tensor, torch.Tensor]] = None, use_cache: bool = False, **kwargs):
@@ -71,6 +84,10 @@ class LlamaTernaryAttention(nn.Module):
         nq, nkv = self.num_heads * self.head_dim, self.num_key_value_heads * self.head_dim
         if self.fused_qkv:
             qkv = self.packed_qkv(hidden_states.device).matmul(hidden_states.reshape(bsz * q_len, self.hidden_size))
+            if attention_mask is None and position_embeddings is None and past_key_value is None and not use_cache and \
+                    not (self.training and self.attention_dropout > 0.0) and self._own_core(qkv.dtype, bsz, q_len):
+                out = _lib.binding().causal_attention(qkv, bsz, q_len, self.num_heads, self.num_key_value_heads, self.head_dim)
+                return self.o_proj(out.view(bsz, q_len, nq)), None, None
             q, k, v = qkv.split([nq, nkv, nkv], dim=1)
         else:
             q, k, v = self.q_proj(hidden_states), self.k_proj(hidden_states), self.v_proj(hidden_states)

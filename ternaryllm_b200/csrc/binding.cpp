@@ -267,6 +267,25 @@ PyObject* mlp_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     BINDING_CATCH
 }
 
+// causal_attention(qkv [batch * rows, (heads + 2 * kv_heads) * head_dim], batch, rows, heads, kv_heads, head_dim) -> [batch * rows, heads * head_dim]
+PyObject* causal_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    NEED_ARGS(6, "causal_attention")
+    BINDING_TRY
+    long long v[6];
+    for (int i = 1; i < 6; ++i)
+        if (!int_of(a[i], &v[i])) return nullptr;
+    const at::Tensor* x = tensor_of(a[0]);
+    if (!x || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous() || x->size(0) != v[1] * v[2] || x->size(1) != (v[3] + 2 * v[4]) * v[5])
+        return raise("causal_attention expects a contiguous CUDA tensor [batch * rows, (heads + 2 * kv_heads) * head_dim]");
+    DeviceScope scope(x->get_device());
+    at::Tensor y = at::empty({x->size(0), v[3] * v[5]}, x->options());
+    void* st = c10::cuda::getCurrentCUDAStream(x->get_device()).stream();
+    const int rc = tllm_causal_attention(x->const_data_ptr(), y.data_ptr(), dtype_code(x->scalar_type()), (int)v[1], (int)v[2], (int)v[3], (int)v[4], (int)v[5], st);
+    if (rc) return raise_rc("tllm_causal_attention", rc);
+    return THPVariable_Wrap(std::move(y));
+    BINDING_CATCH
+}
+
 // ter_spmm(X, row_idx, col_off, tile_idx | None, batch, rows, columns, inners, uniformed, padded, scale, out | None, tile_k) -> tensor
 PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     NEED_ARGS(13, "ter_spmm")
@@ -335,6 +354,7 @@ PyMethodDef methods[] = {
     {"matmul_host", (PyCFunction)(void (*)(void))matmul_host, METH_FASTCALL,
      "matmul_host(handle, x, x_code, x_col_major, rows, y_rows, y_columns, y_code, y_col_major, device)"},
     {"mlp_forward", (PyCFunction)(void (*)(void))mlp_forward, METH_FASTCALL, "mlp_forward(handle, x, out, h, hidden)"},
+    {"causal_attention", (PyCFunction)(void (*)(void))causal_attention, METH_FASTCALL, "causal_attention(qkv, batch, rows, heads, kv_heads, head_dim)"},
     {"ter_spmm", (PyCFunction)(void (*)(void))ter_spmm, METH_FASTCALL,
      "ter_spmm(X, row_idx, col_off, tile_idx, batch, rows, columns, inners, uniformed, padded, scale, out, tile_k)"},
     {nullptr, nullptr, 0, nullptr}};

@@ -1,5 +1,6 @@
 // capi.cu -- the C ABI of libtllm (declared in include/tllm.h): handles, launches, host staging.
 #include <atomic>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -10,6 +11,7 @@
 
 #include <cudaTypedefs.h>
 
+#include "attn_kernel.cuh"
 #include "bits_kernel.cuh"
 #include "bstream_kernel.cuh"
 #include "kernels.cuh"
@@ -319,23 +321,24 @@ struct Workspace {
 };
 
 // How a product of `rows` rows (in `planes` planes) is cut: row tiles of Nt rows each, whole tiles or equal ranges of units, chosen
-// by an estimate in SM clocks.  A slice of 64 rows of W is four MMAs of 128 x Nt x 16 per plane, 2.4 * Nt clocks (measured) and
-// never less than the 260 of their issue.  A tile's epilogue is hidden behind the next one except at the end, or where there
-// is no room for two sets of accumulators.  In a tile
-// that `parts` blocks share the last one to arrive reads the other parts, a round trip to L2 for every sixteen rows of each, 3000 clocks in all at least.
+// by an estimate in SM clocks.  A slice of 64 rows of W is four MMAs of 128 x (planes * Nt) x 16, 2.5 clocks a column (measured)
+// and never less than the 255 of their issue.  A tile's epilogue is hidden behind the next one except at the end, or where
+// there is no room for two sets of accumulators.  In a tile that `parts` blocks share the last one to arrive reads the other
+// parts, a round trip to L2 for every sixteen rows of each, 3000 clocks in all at least.
 struct MmPlan {
     int Nt, m_tiles, split;
     double clocks;
 };
+int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
 MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
     MmPlan best{0, 0, 0, 0};
     const int kbu = (kb + MM_UK - 1) / MM_UK;
-    for (int nt = 16; nt <= MM_MAX_NT; nt += 16) {
+    for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
         const int mt = (rows + nt - 1) / nt;
         if (mt > MM_MAX_M_TILES) continue;
         const double tiles = (double)n_tiles * mt, units = tiles * kbu;
-        const double slice = planes * std::max(260.0, 2.4 * nt), epilogue = nt / 16 * 500.0;
-        const bool two = (planes == 1 ? 2 : 4) * nt <= MM_A_COL;
+        const double slice = std::max(255.0, 2.5 * planes * nt), epilogue = nt / 16 * 350.0;
+        const bool two = 2 * planes * nt <= MM_A_COL;
         const double whole = std::ceil(tiles / sms) * (kb * slice + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
         const double split = std::ceil(units / blocks) * MM_UK * slice + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
@@ -346,12 +349,13 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
     return best;
 }
 
-int encode_rows_map(CUtensorMap* map, const void* base, bool bf16, int k, int rows, size_t pitch_bytes, int box_rows) {
-    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)pitch_bytes};
-    const cuuint32_t box[2] = {MM_TILE_K, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult cr = tensor_map_encoder()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides,
+// X as planes of rows of K values (one plane: two dimensions); a box is 64 values of box_rows rows of every plane
+int encode_rows_map(CUtensorMap* map, const void* base, bool bf16, int k, int rows, int planes, size_t pitch_bytes, size_t plane_bytes, int box_rows) {
+    const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)rows, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch_bytes, (cuuint64_t)plane_bytes};
+    const cuuint32_t box[3] = {MM_TILE_K, (cuuint32_t)box_rows, (cuuint32_t)planes};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult cr = tensor_map_encoder()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, planes == 1 ? 2 : 3, const_cast<void*>(base), dims, strides,
                                              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
@@ -420,7 +424,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     p.M = rows, p.K = w.inners, p.N = w.columns;
     p.KB = w.kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
     p.n_tiles = w.n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split;
-    p.P = x.planes, p.plane_rows = x.plane_rows;
+    p.P = x.planes;
     p.epilogue = o.epilogue, p.y_ld = o.ld, p.plane_y = o.plane;
     p.y_step_n = o.col_major ? o.ld : 1, p.y_step_m = o.col_major ? 1 : o.ld;
     p.out = o.planes ? MM_OUT_PLANES : o.dtype == TLLM_F32 ? MM_OUT_F32 : o.dtype == TLLM_I32 ? MM_OUT_I32 : o.dtype == TLLM_F16 ? MM_OUT_F16 : MM_OUT_BF16;
@@ -429,19 +433,19 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
         if (wide && o.col_major && (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0) p.out = o.dtype == TLLM_F32 ? MM_OUT_F32_COL4 : MM_OUT_I32_COL4;
         if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && w.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
     }
-    // rings: four units of bit tiles, and as many of B as 192 KiB hold (three at 128 rows)
+    // rings: four units of bit tiles, and as many of B as 192 KiB hold (three at 128 columns of D, two at 192)
     p.R = 4;
-    const int b_unit = p.Nt * 128 * MM_UK;
+    const int b_unit = x.planes * p.Nt * 128 * MM_UK;
     p.SB = std::min(MM_MAX_STAGES, 192 * 1024 / b_unit);
     p.mul4 = 4, p.mul16 = 16;
     const uint32_t fmt = x.bf16 ? 1u : 0u;
     // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B formats (bits 7-9, 10-12), both K-major,
     // N / 8 in bits 17-22, M / 16 in bits 24-28
-    p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.Nt >> 3) << 17) | ((uint32_t)(MM_TILE_N >> 4) << 24);
+    p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(x.planes * p.Nt >> 3) << 17) | ((uint32_t)(MM_TILE_N >> 4) << 24);
     p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
 
     CUtensorMap map;
-    int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, (x.planes - 1) * x.plane_rows + rows, x.pitch, p.Nt);
+    int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, rows, x.planes, x.pitch, (size_t)x.plane_rows * x.pitch, p.Nt);
     if (rc) return rc;
     const size_t smem = 1024 + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512;
     if (smem > 227 * 1024) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
@@ -476,7 +480,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
 
 // fp32 activations that are three planes already ([3][rows][pitch / 2], pitch bytes per row)
 int run_mm_planes(const BitsView& w, const unsigned short* planes, int plane_rows, size_t pitch, int rows, void* Y, int y_dtype, int y_ld, float scale, cudaStream_t st) {
-    const int per = MM_MAX_M_TILES * MM_MAX_NT;
+    const int per = MM_MAX_M_TILES * mm_max_nt(3);
     for (int r0 = 0; r0 < rows; r0 += per) {
         const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch}, std::min(rows - r0, per),
                                  MmOut{(char*)Y + (size_t)r0 * y_ld * dtype_size(y_dtype), y_dtype, y_ld, 0, scale, 0.f, false, false, 0}, st);
@@ -491,7 +495,7 @@ int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld
     const int K = w.inners;
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const bool direct = mm_direct(w.inners, X, x_dtype, x_layout, x_ld);
-    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * MM_MAX_NT;
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     Workspace ws;
     if (!direct) {
         const int rc = ws.take(w.device, (size_t)planes * std::min(rows, per) * stage_pad(K) * 2, st);
@@ -753,7 +757,7 @@ double bt_model_us(int64_t entries, int x_dtype, int rows) {
     return t;
 }
 double mm_tiles_model_us(int n_tiles, int kb, int sms, bool direct, int x_dtype, int rows) {
-    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * MM_MAX_NT;
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per) t += 6.0 + mm_plan(std::min(rows - r0, per), planes, n_tiles, kb, sms).clocks / 1800.0 + (direct ? 0.0 : 2.5);
     return t;
@@ -1746,6 +1750,48 @@ int tllm_add_rmsnorm(void* x, const void* delta, const void* weight, void* h, in
     else CU_TRY((launch_add_rmsnorm<__nv_bfloat16, __nv_bfloat16>(x, delta, weight, h, rows, hidden, eps, st)));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
+}
+
+}  // extern "C"
+
+namespace {
+template <typename T, int HD>
+int launch_attention(const void* qkv, void* out, int batch, int rows, int heads, int kv_heads, int ld, cudaStream_t st) {
+    auto kern = causal_attention_kernel<T, HD>;
+    int dev = 0;
+    CU_TRY(cudaGetDevice(&dev));
+    static std::once_flag once[64];
+    cudaError_t err = cudaSuccess;
+    std::call_once(once[dev & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)at_smem_bytes<HD>()); });
+    CU_TRY(err);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((rows + AT_ROWS - 1) / AT_ROWS), (unsigned)heads, (unsigned)batch);
+    cfg.blockDim = dim3(AT_THREADS);
+    cfg.dynamicSmemBytes = at_smem_bytes<HD>();
+    cfg.stream = st;
+    cudaLaunchAttribute at[1] = {pdl_attribute()};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU_TRY(cudaLaunchKernelEx(&cfg, kern, (const T*)qkv, (T*)out, rows, heads, kv_heads, ld, 1.0f / sqrtf((float)HD)));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TLLM_OK;
+}
+}  // namespace
+
+extern "C" {
+
+int tllm_causal_attention(const void* qkv, void* out, int dtype, int batch, int rows, int heads, int kv_heads, int head_dim, void* stream) {
+    if (!qkv || !out || batch <= 0 || rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads) return fail(TLLM_ERR_ARG, "tllm_causal_attention: bad argument");
+    if (head_dim != 64 && head_dim != 128) return fail(TLLM_ERR_ARG, "tllm_causal_attention: heads of %d values (64 and 128 are built)", head_dim);
+    if (batch > 65535 || heads > 65535 || ((uintptr_t)qkv | (uintptr_t)out) % 16) return fail(TLLM_ERR_ARG, "tllm_causal_attention: too many heads or unaligned pointers");
+    const int ld = (heads + 2 * kv_heads) * head_dim;
+    cudaStream_t st = (cudaStream_t)stream;
+#define AT_LAUNCH(T) (head_dim == 64 ? launch_attention<T, 64>(qkv, out, batch, rows, heads, kv_heads, ld, st) : launch_attention<T, 128>(qkv, out, batch, rows, heads, kv_heads, ld, st))
+    if (dtype == TLLM_F32) return AT_LAUNCH(float);
+    if (dtype == TLLM_F16) return AT_LAUNCH(__half);
+    if (dtype == TLLM_BF16) return AT_LAUNCH(__nv_bfloat16);
+#undef AT_LAUNCH
+    return fail(TLLM_ERR_ARG, "tllm_causal_attention: unsupported dtype");
 }
 
 int tllm_silu_mul(void* g, const void* u, int dtype, int64_t n, void* stream) {
