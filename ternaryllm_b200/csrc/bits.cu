@@ -52,25 +52,46 @@ int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device,
 
 }  // namespace
 
+// How a product is cut.  One pass over the widest block's columns if GR = 3 (two for more than eight columns of B: 64 and 128
+// registers) and a split of up to four allow it; the narrowest split that does, because every part of a split fetches the
+// activations anew.
+namespace {
+struct BitsPlan {
+    int nb, own, own_more, split_log, per_pass, gr, pairs;     // pairs: pairs of slices a warp goes through, all passes together
+};
+BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
+    BitsPlan q;
+    const int cols = x_dtype == TLLM_F32 ? 3 * rows : rows, groups = (columns + 15) / 16;     // fp32: three bf16 columns a row
+    q.nb = (cols + 7) / 8, q.own = groups / sms, q.own_more = groups % sms;
+    const int most = q.nb > 1 ? 2 : 3, own = q.own + (q.own_more ? 1 : 0);
+    q.split_log = own <= most ? 0 : own <= 2 * most ? 1 : 2;
+    const int split = 1 << q.split_log, passes = (own + split * most - 1) / (split * most), kparts = BT_WARPS / split;
+    q.per_pass = (own + passes - 1) / passes;
+    q.gr = (q.per_pass + split - 1) / split;
+    q.pairs = ((kb + 1) / 2 + kparts - 1) / kparts * passes;
+    return q;
+}
+}  // namespace
+
+// Microseconds of a launch: a chain of 2 us, and per pair of slices that a warp goes through what it takes sixteen warps to fetch and
+// turn the activations and to decode and multiply the columns.  Measured at 1 to 16 rows of 2048 x 2048 .. 8192 x 10240.
+double bits_estimate_us(int x_dtype, int rows, int columns, int kb, int sms) {
+    const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
+    const double step = x_dtype == TLLM_F32 ? q.nb * (0.6 + 0.18 * q.gr) : 0.25 + q.nb * (0.15 + 0.2 * q.gr);
+    return 2.0 + q.pairs * step;
+}
+
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {
-    const int cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, nb = (cols + 7) / 8;     // fp32: three bf16 columns a row
     const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
     const bool async = p.x_layout == TLLM_ROW_MAJOR && (uintptr_t)p.X % 16 == 0 && (size_t)p.x_ld * e % 16 == 0;
-    const int groups = (p.N + 15) / 16, grid = sms;
-    p.own = groups / grid, p.own_more = groups % grid;
+    const BitsPlan q = bits_plan(p.x_dtype, p.M, p.N, p.KB, sms);
+    const int nb = q.nb, gr = q.gr, grid = sms, kparts = BT_WARPS >> q.split_log, cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, pairs = q.pairs;
+    p.own = q.own, p.own_more = q.own_more, p.split_log = q.split_log, p.per_pass = q.per_pass;
     p.mul4 = 4, p.mul16 = 16;
     p.m_inv = (uint32_t)(((1ull << 32) + p.M - 1) / p.M);
-    // One pass over the widest block's columns if GR = 3 (two for more than eight columns of B: 64 and 128 registers) and a split
-    // of up to four allow it; the narrowest split that does, because every part of a split fetches the activations anew.
-    const int most = nb > 1 ? 2 : 3, own = p.own + (p.own_more ? 1 : 0);
-    p.split_log = own <= most ? 0 : own <= 2 * most ? 1 : 2;
-    const int split = 1 << p.split_log, passes = (own + split * most - 1) / (split * most);
-    p.per_pass = (own + passes - 1) / passes;
-    const int gr = (p.per_pass + split - 1) / split;
     p.slot_bytes = (uint32_t)(gr * 512 + p.M * 128 * e);
     // Pairs in flight: as many as a warp has to fetch and half of the shared memory holds (so that the next launch fits
     // beside this one); where not even two fit there, up to all of it.
-    const int kparts = BT_WARPS / split, pairs = ((p.KB + 1) / 2 + kparts - 1) / kparts * passes;
     const size_t red = (size_t)kparts * p.per_pass * cols * 80;
     auto slots = [&](int d) { return pairs <= d ? pairs : d + 1; };
     auto total = [&](int d) { return (size_t)BT_WARPS * slots(d) * p.slot_bytes + red; };

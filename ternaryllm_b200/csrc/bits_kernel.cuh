@@ -425,5 +425,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
 
 // one launch of up to BT_MAX_ROWS rows (half of it fp32); fills in everything from `own` to `mul16` (bits.cu)
 int bits_launch(BitsParams& p, int sms, int device, void* stream);
+// its time, for the choice between kernels
+double bits_estimate_us(int x_dtype, int rows, int columns, int kb, int sms);
 
 }  // namespace tllm

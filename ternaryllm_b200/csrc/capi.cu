@@ -746,27 +746,26 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
     return TLLM_OK;
 }
 
-// Cost models of the two kernels that read the two-bit tiles, microseconds.  Register decode: a launch chain of 2 us and, per
-// million entries, 0.1 (one block of eight columns of B), 0.25 (two) or 0.35 (three).  Batched: 6 us of start-up and
-// hand-over, the plan's clocks at 1.8 GHz, and 2.5 us for planes that have to be made first.
-double bt_model_us(int64_t entries, int x_dtype, int rows) {
-    static const double per_mentry[4] = {0, 0.105, 0.25, 0.35};
-    const int per = bt_rows_per_launch(x_dtype), p = x_dtype == TLLM_F32 ? 3 : 1;
+// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 4 us of start-up and hand-over, the plan's
+// clocks at 1.8 GHz, and 3 us for planes that have to be made first.
+double bt_model_us(int inners, int columns, int sms, int x_dtype, int rows) {
+    const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
-    for (int r0 = 0; r0 < rows; r0 += per) t += 2.0 + entries * 1e-6 * per_mentry[(std::min(rows - r0, per) * p + 7) / 8];
+    for (int r0 = 0; r0 < rows; r0 += per) t += bits_estimate_us(x_dtype, std::min(rows - r0, per), columns, (inners + 63) / 64, sms);
     return t;
 }
-double mm_tiles_model_us(int n_tiles, int kb, int sms, bool direct, int x_dtype, int rows) {
+double mm_tiles_model_us(int inners, int columns, int sms, bool direct, int x_dtype, int rows) {
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
-    for (int r0 = 0; r0 < rows; r0 += per) t += 6.0 + mm_plan(std::min(rows - r0, per), planes, n_tiles, kb, sms).clocks / 1800.0 + (direct ? 0.0 : 2.5);
+    for (int r0 = 0; r0 < rows; r0 += per)
+        t += 4.0 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms).clocks / 1800.0 + (direct ? 0.0 : 3.0);
     return t;
 }
 // which of the two: true = decode in registers
 bool bits_prefer_registers(int inners, int columns, int sms, bool direct, int x_dtype, int rows) {
-    if (rows <= 8) return true;
+    if (rows == 1) return true;
     if (rows > 8 * BT_MAX_ROWS) return false;
-    return bt_model_us((int64_t)inners * columns, x_dtype, rows) <= mm_tiles_model_us((columns + 127) / 128, (inners + 63) / 64, sms, direct, x_dtype, rows);
+    return bt_model_us(inners, columns, sms, x_dtype, rows) <= mm_tiles_model_us(inners, columns, sms, direct, x_dtype, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
@@ -778,7 +777,7 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     // int8 sums are exact in fp32 while K * 128 stays within 2^24
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
         // very sparse weights: the index lists are shorter than two bits an entry (the gather model is a fifth low at 90 % zeros)
-        if (rows <= 4 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(entries, x_dtype, rows)) return KERNEL_GATHER;
+        if (rows <= 4 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_GATHER;
         return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
     if (nb && mm) return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
