@@ -78,6 +78,7 @@ SIGNATURES = {
     "tllm_mlp_create_cpu_format": (_I, [_I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _I, _I, _P, _P]),
     "tllm_mlp_get_info": (_I, [_P, _P, _P]),
     "tllm_causal_attention": (_I, [_P, _P, _I, _I, _I, _I, _I, _I, _P]),
+    "tllm_decode_attention": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _L, _P]),
     "tllm_silu_mul": (_I, [_P, _P, _I, _L, _P]),
     "tllm_add_rmsnorm": (_I, [_P, _P, _P, _P, _I, _I, _I, _F, _P]),
     "tllm_comm_create": (_I, [_I, _I, _I, _I, _P]),

@@ -286,6 +286,28 @@ PyObject* causal_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     BINDING_CATCH
 }
 
+// decode_attention(qkv [rows, (heads + 2 * kv_heads) * head_dim], k_cache, v_cache [>= rows, kv_heads, positions, head_dim], heads, len) -> [rows, heads * head_dim];
+// the caches' position len is written
+PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    NEED_ARGS(5, "decode_attention")
+    BINDING_TRY
+    long long heads, len;
+    if (!int_of(a[3], &heads) || !int_of(a[4], &len)) return nullptr;
+    const at::Tensor *x = tensor_of(a[0]), *k = tensor_of(a[1]), *v = tensor_of(a[2]);
+    if (!x || !k || !v || !x->is_cuda() || x->dim() != 2 || !x->is_contiguous() || k->dim() != 4 || !k->is_contiguous() || !v->is_contiguous() || k->sizes() != v->sizes() ||
+        k->device() != x->device() || v->device() != x->device() || k->scalar_type() != x->scalar_type() || v->scalar_type() != x->scalar_type() || k->size(0) < x->size(0) ||
+        len < 0 || len >= k->size(2) || x->size(1) != (heads + 2 * k->size(1)) * k->size(3))
+        return raise("decode_attention expects contiguous CUDA tensors qkv [rows, (heads + 2 * kv_heads) * head_dim] and caches [>= rows, kv_heads, > len, head_dim] of one type");
+    DeviceScope scope(x->get_device());
+    at::Tensor y = at::empty({x->size(0), heads * k->size(3)}, x->options());
+    void* st = c10::cuda::getCurrentCUDAStream(x->get_device()).stream();
+    const int rc = tllm_decode_attention(x->const_data_ptr(), k->data_ptr(), v->data_ptr(), y.data_ptr(), dtype_code(x->scalar_type()), (int)x->size(0), (int)heads, (int)k->size(1),
+                                         (int)k->size(3), (int)len, k->stride(0), k->stride(1), st);
+    if (rc) return raise_rc("tllm_decode_attention", rc);
+    return THPVariable_Wrap(std::move(y));
+    BINDING_CATCH
+}
+
 // ter_spmm(X, row_idx, col_off, tile_idx | None, batch, rows, columns, inners, uniformed, padded, scale, out | None, tile_k) -> tensor
 PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     NEED_ARGS(13, "ter_spmm")
@@ -354,6 +376,7 @@ PyMethodDef methods[] = {
     {"matmul_host", (PyCFunction)(void (*)(void))matmul_host, METH_FASTCALL,
      "matmul_host(handle, x, x_code, x_col_major, rows, y_rows, y_columns, y_code, y_col_major, device)"},
     {"mlp_forward", (PyCFunction)(void (*)(void))mlp_forward, METH_FASTCALL, "mlp_forward(handle, x, out, h, hidden)"},
+    {"decode_attention", (PyCFunction)(void (*)(void))decode_attention, METH_FASTCALL, "decode_attention(qkv, k_cache, v_cache, heads, len)"},
     {"causal_attention", (PyCFunction)(void (*)(void))causal_attention, METH_FASTCALL, "causal_attention(qkv, batch, rows, heads, kv_heads, head_dim)"},
     {"ter_spmm", (PyCFunction)(void (*)(void))ter_spmm, METH_FASTCALL,
      "ter_spmm(X, row_idx, col_off, tile_idx, batch, rows, columns, inners, uniformed, padded, scale, out, tile_k)"},

@@ -1754,26 +1754,51 @@ int tllm_add_rmsnorm(void* x, const void* delta, const void* weight, void* h, in
 }  // extern "C"
 
 namespace {
-template <typename T, int HD>
-int launch_attention(const void* qkv, void* out, int batch, int rows, int heads, int kv_heads, int ld, cudaStream_t st) {
-    auto kern = causal_attention_kernel<T, HD>;
+// one launch of an attention kernel; `parts` blocks in x form a cluster
+template <typename... P, typename... A>
+int launch_attention(void (*kern)(P...), std::once_flag (&once)[64], dim3 grid, int threads, size_t smem, int parts, cudaStream_t st, A... args) {
     int dev = 0;
     CU_TRY(cudaGetDevice(&dev));
-    static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[dev & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)at_smem_bytes<HD>()); });
+    std::call_once(once[dev & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
     CU_TRY(err);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)((rows + AT_ROWS - 1) / AT_ROWS), (unsigned)heads, (unsigned)batch);
-    cfg.blockDim = dim3(AT_THREADS);
-    cfg.dynamicSmemBytes = at_smem_bytes<HD>();
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1] = {pdl_attribute()};
+    cudaLaunchAttribute at[2] = {pdl_attribute(), {}};
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)parts, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CU_TRY(cudaLaunchKernelEx(&cfg, kern, (const T*)qkv, (T*)out, rows, heads, kv_heads, ld, 1.0f / sqrtf((float)HD)));
+    cfg.numAttrs = parts > 1 ? 2 : 1;
+    CU_TRY(cudaLaunchKernelEx(&cfg, kern, args...));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
+}
+constexpr float LOG2E = 1.44269504f;
+
+template <int HD>
+int causal_f32(const void* qkv, void* out, int batch, int rows, int heads, int kv_heads, cudaStream_t st) {
+    static std::once_flag once[64];
+    return launch_attention(prompt_attention_f32_kernel<HD>, once, dim3((unsigned)((rows + AM_KEYS - 1) / AM_KEYS), (unsigned)heads, (unsigned)batch), AM_THREADS,
+                            am_f32_smem<HD>(), 1, st, (const float*)qkv, (float*)out, rows, heads, kv_heads, (heads + 2 * kv_heads) * HD, LOG2E / sqrtf((float)HD));
+}
+template <typename T, int HD>
+int causal_16bit(const void* qkv, void* out, int batch, int rows, int heads, int kv_heads, cudaStream_t st) {
+    static std::once_flag once[64];
+    return launch_attention(prompt_attention_kernel<T, HD>, once, dim3((unsigned)((rows + AM_KEYS - 1) / AM_KEYS), (unsigned)heads, (unsigned)batch), AM_THREADS,
+                            am_prompt_smem<HD>(), 1, st, (const T*)qkv, (T*)out, rows, heads, kv_heads, (heads + 2 * kv_heads) * HD, LOG2E / sqrtf((float)HD));
+}
+// A cluster of up to eight blocks per key head, as many as still fit two to an SM, with 128 keys each at least.  (Twice as many blocks than
+// that, in a second wave: 11 us instead of AM_DECODE_US at 16 sequences of 1024 keys, 8 key heads of 64.)
+template <typename T, int HD>
+int decode_16bit(const void* qkv, void* k, void* v, void* out, int rows, int heads, int kv_heads, int len, int64_t seq_step, int64_t head_step, int sms, cudaStream_t st) {
+    static std::once_flag once[64];
+    int parts = 1;
+    while (parts < 8 && (long long)rows * kv_heads * parts <= sms && len / (2 * parts) >= 128) parts *= 2;
+    return launch_attention(decode_attention_kernel<T, HD>, once, dim3((unsigned)parts, (unsigned)kv_heads, (unsigned)rows), AM_THREADS, am_decode_smem<HD>(), parts, st,
+                            (const T*)qkv, (T*)k, (T*)v, (T*)out, heads, kv_heads, len, (long long)seq_step, (long long)head_step, LOG2E / sqrtf((float)HD));
 }
 }  // namespace
 
@@ -1783,14 +1808,30 @@ int tllm_causal_attention(const void* qkv, void* out, int dtype, int batch, int 
     if (!qkv || !out || batch <= 0 || rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads) return fail(TLLM_ERR_ARG, "tllm_causal_attention: bad argument");
     if (head_dim != 64 && head_dim != 128) return fail(TLLM_ERR_ARG, "tllm_causal_attention: heads of %d values (64 and 128 are built)", head_dim);
     if (batch > 65535 || heads > 65535 || ((uintptr_t)qkv | (uintptr_t)out) % 16) return fail(TLLM_ERR_ARG, "tllm_causal_attention: too many heads or unaligned pointers");
-    const int ld = (heads + 2 * kv_heads) * head_dim;
     cudaStream_t st = (cudaStream_t)stream;
-#define AT_LAUNCH(T) (head_dim == 64 ? launch_attention<T, 64>(qkv, out, batch, rows, heads, kv_heads, ld, st) : launch_attention<T, 128>(qkv, out, batch, rows, heads, kv_heads, ld, st))
-    if (dtype == TLLM_F32) return AT_LAUNCH(float);
-    if (dtype == TLLM_F16) return AT_LAUNCH(__half);
-    if (dtype == TLLM_BF16) return AT_LAUNCH(__nv_bfloat16);
-#undef AT_LAUNCH
+    const bool narrow = head_dim == 64;
+    if (dtype == TLLM_F32) return narrow ? causal_f32<64>(qkv, out, batch, rows, heads, kv_heads, st) : causal_f32<128>(qkv, out, batch, rows, heads, kv_heads, st);
+    if (dtype == TLLM_F16) return narrow ? causal_16bit<__half, 64>(qkv, out, batch, rows, heads, kv_heads, st) : causal_16bit<__half, 128>(qkv, out, batch, rows, heads, kv_heads, st);
+    if (dtype == TLLM_BF16)
+        return narrow ? causal_16bit<__nv_bfloat16, 64>(qkv, out, batch, rows, heads, kv_heads, st) : causal_16bit<__nv_bfloat16, 128>(qkv, out, batch, rows, heads, kv_heads, st);
     return fail(TLLM_ERR_ARG, "tllm_causal_attention: unsupported dtype");
+}
+
+int tllm_decode_attention(const void* qkv, void* k_cache, void* v_cache, void* out, int dtype, int rows, int heads, int kv_heads, int head_dim, int len, int64_t seq_step,
+                          int64_t head_step, void* stream) {
+    if (!qkv || !k_cache || !v_cache || !out || rows <= 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || len < 0) return fail(TLLM_ERR_ARG, "tllm_decode_attention: bad argument");
+    if ((head_dim != 64 && head_dim != 128) || heads / kv_heads > AM_MAX_GROUP || (dtype != TLLM_F16 && dtype != TLLM_BF16))
+        return fail(TLLM_ERR_ARG, "tllm_decode_attention: 16-bit heads of 64 or 128 values, at most %d query heads per key head", AM_MAX_GROUP);
+    if (rows > 65535 || kv_heads > 65535 || ((uintptr_t)qkv | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16 || seq_step % 8 || head_step % 8)
+        return fail(TLLM_ERR_ARG, "tllm_decode_attention: too many sequences or unaligned pointers");
+    int dev = 0, sms = 0;
+    CU_TRY(cudaGetDevice(&dev));
+    CU_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    cudaStream_t st = (cudaStream_t)stream;
+#define AM_DECODE(T) (head_dim == 64 ? decode_16bit<T, 64>(qkv, k_cache, v_cache, out, rows, heads, kv_heads, len, seq_step, head_step, sms, st) \
+                                     : decode_16bit<T, 128>(qkv, k_cache, v_cache, out, rows, heads, kv_heads, len, seq_step, head_step, sms, st))
+    return dtype == TLLM_F16 ? AM_DECODE(__half) : AM_DECODE(__nv_bfloat16);
+#undef AM_DECODE
 }
 
 int tllm_silu_mul(void* g, const void* u, int dtype, int64_t n, void* stream) {

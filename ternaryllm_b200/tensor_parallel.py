@@ -228,9 +228,9 @@ def kv_cache(seed, kv_head, max_batch, kv_len, head_dim):
 class TernaryDecoderLayerTP(nn.Module):
     """One Llama-shaped decoder layer for single-token decode with ternary linears, tensor-parallel.
 
-    Only the linears and the reduction glue are this library's work; the attention core (scaled-dot-product over a
-    synthetic KV cache, grouped-query) is stock PyTorch, as in the reference, whose attention is stock Hugging Face
-    code (ternaryLLM_GPU/TernaryLLM/TernaryAttn.py:78-120).
+    The attention core (scaled-dot-product over a synthetic KV cache, grouped-query), stock code in the reference
+    (ternaryLLM_GPU/TernaryLLM/TernaryAttn.py:78-120), is one launch of this library (tllm_decode_attention) for 16-bit heads of
+    64 and 128, which appends the new key and value too, and stock PyTorch otherwise.
 
     reduce: "peer" -- tllm_allreduce_add_rmsnorm (one launch per reduction, fp32 partial sums over peer memory);
             "nccl" -- NCCL all-reduce of the bf16 partial result + tllm_add_rmsnorm.
@@ -271,6 +271,9 @@ class TernaryDecoderLayerTP(nn.Module):
         self._part2 = torch.empty((max_batch, hidden), dtype=torch.float32, device=self.device)   # down projection's
 
     def attention(self, qkv, M):
+        # one launch instead of two copies, a flash kernel and its reduction; the stock core takes what it is not built for
+        if self.dtype in (torch.float16, torch.bfloat16) and self.hd in (64, 128) and self.hq <= 16 * self.hkv and qkv.is_cuda:
+            return _lib.binding().decode_attention(qkv, self.k_cache, self.v_cache, self.hq, self.kv_len)
         q, k, v = qkv.split([self.hq * self.hd, self.hkv * self.hd, self.hkv * self.hd], dim=1)
         q = q.view(M, self.hq, 1, self.hd)
         kc, vc = self.k_cache[:M], self.v_cache[:M]

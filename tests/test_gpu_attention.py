@@ -1,6 +1,6 @@
-"""The one-launch causal attention (csrc/attn_kernel.cuh) and the module path that uses it, against the same attention in fp64.
-Bounds: fp32 arithmetic on values of order one, sums of up to a few hundred terms: 1e-5 of the largest output; 16-bit types add
-the rounding of the result (eps)."""
+"""The one-launch attention kernels (csrc/attn_kernel.cuh) and the module path that uses them, against the same
+attention in fp64.  Bounds: fp32 sums of up to a thousand terms of order one: 1e-5 of the largest output; 16-bit types add the
+rounding of the result (eps of it) and of the probabilities (each off by eps of itself at most: eps of the largest value)."""
 import pytest
 import torch
 
@@ -19,14 +19,33 @@ def reference(qkv, B, M, H, KV, D):
 
 
 @pytest.mark.parametrize("dtype", list(DT))
-@pytest.mark.parametrize("B,M,H,KV,D", [(1, 1, 4, 4, 64), (1, 31, 4, 1, 64), (2, 32, 8, 2, 128), (1, 33, 4, 2, 64), (3, 100, 2, 1, 128), (1, 257, 8, 8, 64)])
+@pytest.mark.parametrize("B,M,H,KV,D", [(1, 1, 4, 4, 64), (1, 31, 4, 1, 64), (2, 32, 8, 2, 128), (1, 33, 4, 2, 64), (3, 100, 2, 1, 128), (1, 257, 8, 8, 64), (2, 64, 4, 1, 128), (1, 65, 4, 4, 128)])
 def test_kernel(B, M, H, KV, D, dtype):
     dt, eps = DT[dtype]
     g = torch.Generator(device="cuda").manual_seed(M)
     qkv = (torch.randn((B * M, (H + 2 * KV) * D), device="cuda", generator=g) * 2).to(dt)
     y = _lib.binding().causal_attention(qkv, B, M, H, KV, D)
     ref = reference(qkv, B, M, H, KV, D)
-    assert float((y.double() - ref).abs().max()) <= (1e-5 + eps) * float(ref.abs().max())
+    assert float((y.double() - ref).abs().max()) <= (1e-5 + eps) * float(ref.abs().max()) + eps * float(qkv.abs().max())
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("B,H,KV,D,n", [(1, 4, 4, 64, 0), (1, 16, 1, 64, 31), (3, 8, 2, 128, 15), (2, 8, 8, 128, 16), (5, 24, 8, 64, 129), (1, 8, 1, 128, 1023),
+                                        (2, 16, 2, 64, 1024), (40, 16, 8, 128, 300)])
+def test_decode(B, H, KV, D, n, dtype):
+    """Positions 0 .. n, the new one included, at the edges of tiles (32 and 16 keys), of parts (128 keys, up to 8) and of groups."""
+    dt, eps = DT[dtype]
+    g = torch.Generator(device="cuda").manual_seed(n + B)
+    qkv = (torch.randn((B, (H + 2 * KV) * D), device="cuda", generator=g) * 2).to(dt)
+    kc, vc = ((torch.randn((B + 1, KV, n + 3, D), device="cuda", generator=g) * 2).to(dt) for _ in range(2))
+    wk, wv = kc.clone(), vc.clone()
+    wk[:B, :, n], wv[:B, :, n] = qkv[:, H * D:(H + KV) * D].view(B, KV, D), qkv[:, (H + KV) * D:].view(B, KV, D)
+    y = _lib.binding().decode_attention(qkv, kc, vc, H, n)
+    assert torch.equal(kc, wk) and torch.equal(vc, wv)
+    q = qkv[:, :H * D].double().view(B, KV, H // KV, D)
+    s = (q @ wk[:B, :, :n + 1].double().transpose(2, 3) / D ** 0.5).softmax(-1)
+    ref = (s @ wv[:B, :, :n + 1].double()).reshape(B, H * D)
+    assert float((y.double() - ref).abs().max()) <= (1e-5 + eps) * float(ref.abs().max()) + eps * float(wv.abs().max())
 
 
 @pytest.mark.parametrize("dtype", list(DT))
