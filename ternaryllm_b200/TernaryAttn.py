@@ -28,7 +28,7 @@ from .TernaryLinear import TernaryLinear
 from .weight import PackedWeight
 
 
-_OWN_CORE_16BIT = 256 * 256 * 2048        # batch * positions^2 * heads * head_dim
+_OWN_CORE_16BIT = 704 * 704 * 2048      # positions^2 * heads * head_dim
 
 
 def _rotate_half(x):
@@ -70,9 +70,9 @@ class LlamaTernaryAttention(nn.Module):
         return pw
 
     def _own_core(self, dtype, bsz, q_len) -> bool:
-        """Whether a plain causal prompt goes to the library's one-launch attention (fp32 arithmetic on the CUDA cores, from the
-        q | k | v product as it lies).  fp32: always, the stock path is a dozen launches.  16-bit: while the arithmetic is less than
-        the stock path's launches and copies cost; the tensor-core kernels behind it are faster on long prompts."""
+        """Whether a plain causal prompt goes to the library's one-launch attention, which reads the q | k | v product as it lies.
+        fp32: always, the stock path is a dozen launches.  16-bit: while it takes less than the host needs for the stock path's launches
+        (40 us: 14 us here at 512 positions of 16 heads of 128, 39 at 1024); the kernels behind that are faster on long prompts."""
         if self.head_dim not in (64, 128) or bsz > 65535:
             return False
         return dtype == torch.float32 or bsz * q_len * q_len * self.num_heads * self.head_dim <= _OWN_CORE_16BIT

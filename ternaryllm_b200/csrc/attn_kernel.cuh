@@ -8,8 +8,9 @@
 // runs along with the tiles of keys, in fp32 and in powers of two.  Keys and values come by cp.async into rows whose 16-byte
 // chunks are xor-ed with the row number, which makes every ldmatrix free of bank conflicts.
 //
-// The kernels differ in who shares a tile of keys: in a prompt the four warps of a block hold 64 queries and go through the
-// same tiles; in a decode step there is one query a head, the query heads of one key head are the rows of the one operand, and
+// The kernels differ in who shares a tile of keys: in a prompt four warps hold 64 queries and go through the same tiles, and a second group of four takes
+// every other tile: the prompts served here fill an SM with one block, and one warp per scheduler spends two thirds
+// of its time waiting.  In a decode step there is one query a head, the query heads of one key head are the rows of the one operand, and
 // every warp goes through keys of its own.
 #pragma once
 #include <type_traits>
@@ -19,7 +20,9 @@
 namespace tllm {
 
 #define AM_THREADS 128
-#define AM_KEYS 64                    // keys per tile of the prompt kernel, and queries per block
+#define AM_KEYS 64                    // keys per tile of the 16-bit prompt kernel, and queries per block
+#define AM_SHARES 2                   // groups of four warps that share the tiles of a block of queries
+#define AM_P_THREADS (AM_THREADS * AM_SHARES)
 #define AM_RING 3                     // tiles per warp on the way in the decode kernel
 #define AM_MAX_GROUP 16               // query heads per key head of the decode kernel: the rows of one operand
 
@@ -151,24 +154,50 @@ struct AmQueries {
     }
 };
 
+// one group's barrier
+__device__ __forceinline__ void am_group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory"); }
+// The second group's results join the first's.  buf: [4 warps][N * 4 + 4][32 lanes]; called by the whole block.
+template <int N>
+__device__ __forceinline__ void am_join(float (&o)[N][4], float (&mx)[2], float (&sum)[2], float* buf, int warp, int lane) {
+    __syncthreads();
+    float* at = buf + (warp & 3) * (N * 4 + 4) * 32 + lane;
+    if (warp >= 4) {
+#pragma unroll
+        for (int j = 0; j < N * 4; ++j) at[32 * j] = o[j >> 2][j & 3];
+        at[32 * N * 4] = mx[0], at[32 * (N * 4 + 1)] = mx[1], at[32 * (N * 4 + 2)] = sum[0], at[32 * (N * 4 + 3)] = sum[1];
+    }
+    __syncthreads();
+    if (warp < 4) {
+        float f[2], g[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float m1 = at[32 * (N * 4 + r)], m = fmaxf(mx[r], m1);         // the first group has seen key 0
+            f[r] = exp2f(mx[r] - m), g[r] = exp2f(m1 - m);
+            sum[r] = sum[r] * f[r] + at[32 * (N * 4 + 2 + r)] * g[r];
+        }
+#pragma unroll
+        for (int j = 0; j < N * 4; ++j) o[j >> 2][j & 3] = o[j >> 2][j & 3] * f[(j >> 1) & 1] + at[32 * j] * g[(j >> 1) & 1];
+    }
+}
+
 // ---- a prompt: out[b, m, h] from the fused product qkv [batch * M][ld] (query heads, key heads, value heads), queries see the keys up
-// to their own position.  grid (query tiles, H, batch), longest first; two tiles of keys in shared memory.
+// to their own position.  grid (query tiles, H, batch), longest first; two tiles of keys per group in shared memory.
 template <int HD>
-constexpr size_t am_prompt_smem() { return (size_t)2 * 2 * AM_KEYS * HD * 2; }
+constexpr size_t am_prompt_smem() { return (size_t)AM_SHARES * 2 * 2 * AM_KEYS * HD * 2; }
 
 template <typename T, int HD>
-__global__ void __launch_bounds__(AM_THREADS) prompt_attention_kernel(const T* __restrict__ qkv, T* __restrict__ out, int M, int H, int HKV, int ld, float scale) {
+__global__ void __launch_bounds__(AM_P_THREADS) prompt_attention_kernel(const T* __restrict__ qkv, T* __restrict__ out, int M, int H, int HKV, int ld, float scale) {
     extern __shared__ __align__(128) unsigned char am_smem[];
     constexpr uint32_t TILE = AM_KEYS * HD * 2;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x & (AM_THREADS - 1), lane = tid & 31, warp = threadIdx.x >> 5, group = warp >> 2;
     const int qt = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, hk = h / (H / HKV);
     const T* base = qkv + (size_t)blockIdx.z * M * ld;
     const T *k = base + (size_t)(H + hk) * HD, *v = k + (size_t)HKV * HD;
-    const uint32_t s0 = smem_u32(am_smem);
+    const uint32_t s0 = smem_u32(am_smem) + (uint32_t)group * 4 * TILE;
     pdl_launch_dependents();
     pdl_wait();
     auto fetch = [&](int t) {                               // rows past the end repeat the last one; no query looks at them
-        const uint32_t dst = s0 + (uint32_t)(t & 1) * 2 * TILE;
+        const uint32_t dst = s0 + (uint32_t)(t >> 1 & 1) * 2 * TILE;
 #pragma unroll
         for (int i = 0; i < AM_KEYS * HD / 8 / AM_THREADS; ++i) {
             const int e = tid + i * AM_THREADS, r = e / (HD / 8), c = e % (HD / 8);
@@ -178,21 +207,23 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_kernel(const T* _
         }
         am_commit();
     };
-    fetch(0);
-    const int r0 = qt * AM_KEYS + warp * 16 + (lane >> 2), r1 = r0 + 8;
+    if (group <= qt) fetch(group);
+    const int r0 = qt * AM_KEYS + (warp & 3) * 16 + (lane >> 2), r1 = r0 + 8;
     AmQueries<T, HD> w;
     w.load(base + (size_t)min(r0, M - 1) * ld + (size_t)h * HD, base + (size_t)min(r1, M - 1) * ld + (size_t)h * HD, lane);
 #pragma unroll 1
-    for (int t = 0; t <= qt; ++t) {
-        if (t < qt) {
-            fetch(t + 1);
+    for (int t = group; t <= qt; t += AM_SHARES) {
+        if (t + AM_SHARES <= qt) {
+            fetch(t + AM_SHARES);
             am_wait<1>();
         } else am_wait<0>();
-        __syncthreads();
-        const uint32_t ks = s0 + (uint32_t)(t & 1) * 2 * TILE;
+        am_group_sync(group);
+        const uint32_t ks = s0 + (uint32_t)(t >> 1 & 1) * 2 * TILE;
         w.template tile<AM_KEYS>(ks, ks + TILE, r0 - t * AM_KEYS, r1 - t * AM_KEYS, scale, lane);
-        __syncthreads();                                    // the tile has been read before the next but one overwrites it
+        am_group_sync(group);                               // the tile has been read before the next but one overwrites it
     }
+    am_join(w.o, w.mx, w.sum, (float*)am_smem, warp, lane);
+    if (group) return;
     w.finish();
     const float i0 = 1.f / w.sum[0], i1 = 1.f / w.sum[1];
     T* y = out + ((size_t)blockIdx.z * M) * ((size_t)H * HD) + (size_t)h * HD + 2 * (lane & 3);
@@ -207,7 +238,7 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_kernel(const T* _
 // 2^-27 of it), every product as the six of theirs that count, the products of a kind summed in accumulators of their own
 // because the tensor core cuts small terms off beside large ones.  Six MMAs take 48 clocks where 64 of FMA would be needed, and
 // read shared memory a fifth as often: the CUDA-core version of this kernel was bound by those reads.
-// Measured, 256 positions of 32 / 8 heads of 64: AM_F32_BEFORE -> AM_F32_AFTER us.
+// Measured, 256 positions of 32 / 8 heads of 64: 37 -> 15 us (23 with one group of warps).
 #define AM_F32_KEYS 32
 __device__ __forceinline__ void am_split(float a, float b, uint32_t (&w)[3]) {
 #pragma unroll
@@ -229,23 +260,24 @@ __device__ __forceinline__ void am_mma6(float (&d)[3][4], const uint32_t (&a0)[4
 }
 // two tiles of keys and values as they are, one as pieces
 template <int HD>
-constexpr size_t am_f32_smem() { return (size_t)AM_F32_KEYS * HD * (2 * 2 * 4 + 2 * 3 * 2); }
+constexpr size_t am_f32_smem() { return (size_t)AM_SHARES * AM_F32_KEYS * HD * (2 * 2 * 4 + 2 * 3 * 2); }
 
 template <int HD>
-__global__ void __launch_bounds__(AM_THREADS) prompt_attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, int M, int H, int HKV, int ld, float scale) {
+__global__ void __launch_bounds__(AM_P_THREADS) prompt_attention_f32_kernel(const float* __restrict__ qkv, float* __restrict__ out, int M, int H, int HKV, int ld, float scale) {
     extern __shared__ __align__(128) unsigned char am_smem[];
     constexpr int KT = AM_F32_KEYS, NC = KT * HD / 8 / AM_THREADS;          // chunks of eight values per thread
     constexpr uint32_t RAW = KT * HD * 4, PL = KT * HD * 2;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t4 = lane & 3;
+    const int tid = threadIdx.x & (AM_THREADS - 1), lane = tid & 31, warp = threadIdx.x >> 5, group = warp >> 2, t4 = lane & 3;
     const int qt = gridDim.x - 1 - blockIdx.x, q0 = qt * AM_KEYS, h = blockIdx.y, hk = h / (H / HKV);
     const float* base = qkv + (size_t)blockIdx.z * M * ld;
     const float *k = base + (size_t)(H + hk) * HD, *v = k + (size_t)HKV * HD;
-    const uint32_t s0 = smem_u32(am_smem), ps = s0 + 4 * RAW;
+    unsigned char* mem = am_smem + group * (4 * RAW + 6 * PL);
+    const uint32_t s0 = smem_u32(mem), ps = s0 + 4 * RAW;
     pdl_launch_dependents();
     pdl_wait();
     // a thread turns the chunks that it has fetched itself
     auto fetch = [&](int t) {
-        const uint32_t dst = s0 + (uint32_t)(t & 1) * 2 * RAW;
+        const uint32_t dst = s0 + (uint32_t)(t >> 1 & 1) * 2 * RAW;
 #pragma unroll
         for (int i = 0; i < NC; ++i) {
             const int e = tid + i * AM_THREADS;
@@ -255,8 +287,9 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_f32_kernel(const 
         }
         am_commit();
     };
-    fetch(0);
-    const int r0 = q0 + warp * 16 + (lane >> 2), r1 = r0 + 8;
+    const int n = min(q0 + AM_KEYS - 1, M - 1) / KT + 1;
+    if (group < n) fetch(group);
+    const int r0 = q0 + (warp & 3) * 16 + (lane >> 2), r1 = r0 + 8;
     uint32_t q[3][HD / 16][4];
     {
         const float *a = base + (size_t)min(r0, M - 1) * ld + (size_t)h * HD + 2 * t4, *b = base + (size_t)min(r1, M - 1) * ld + (size_t)h * HD + 2 * t4;
@@ -273,14 +306,13 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_f32_kernel(const 
     float o[HD / 8][4], mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.f, 0.f};          // mx: in units of log2
 #pragma unroll
     for (int j = 0; j < HD / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    const int n = min(q0 + AM_KEYS - 1, M - 1) / KT + 1;
 #pragma unroll 1
-    for (int t = 0; t < n; ++t) {
-        if (t + 1 < n) {
-            fetch(t + 1);
+    for (int t = group; t < n; t += AM_SHARES) {
+        if (t + AM_SHARES < n) {
+            fetch(t + AM_SHARES);
             am_wait<1>();
         } else am_wait<0>();
-        const unsigned char* raw = am_smem + (t & 1) * 2 * RAW;
+        const unsigned char* raw = mem + (t >> 1 & 1) * 2 * RAW;
 #pragma unroll
         for (int i = 0; i < 2 * NC; ++i) {
             const int e = tid + (i >> 1) * AM_THREADS;
@@ -289,10 +321,10 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_f32_kernel(const 
             am_split(lo.x, lo.y, w[0]), am_split(lo.z, lo.w, w[1]), am_split(hi.x, hi.y, w[2]), am_split(hi.z, hi.w, w[3]);
 #pragma unroll
             for (int pl = 0; pl < 3; ++pl)
-                *(uint4*)(am_smem + 4 * RAW + (3 * (i & 1) + pl) * PL + am_chunk<HD>(e / (HD / 8), e % (HD / 8))) = make_uint4(w[0][pl], w[1][pl], w[2][pl], w[3][pl]);
+                *(uint4*)(mem + 4 * RAW + (3 * (i & 1) + pl) * PL + am_chunk<HD>(e / (HD / 8), e % (HD / 8))) = make_uint4(w[0][pl], w[1][pl], w[2][pl], w[3][pl]);
         }
-        __syncthreads();
-        if (t * KT <= q0 + warp * 16 + 15) {                   // else no query of this warp sees any of the tile
+        am_group_sync(group);
+        if (t * KT <= q0 + (warp & 3) * 16 + 15) {                   // else no query of this warp sees any of the tile
             float s[KT / 8][4];
 #pragma unroll
             for (int j = 0; j < KT / 8; j += 2) {              // two sums of each kind side by side
@@ -360,8 +392,10 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_f32_kernel(const 
                     for (int i = 0; i < 4; ++i) o[2 * c + x][i] = fmaf(o[2 * c + x][i], f[i >> 1], acc[x][0][i] + (acc[x][1][i] + acc[x][2][i]));
             }
         }
-        __syncthreads();
+        am_group_sync(group);
     }
+    am_join(o, mx, sum, (float*)am_smem, warp, lane);
+    if (group) return;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
@@ -378,7 +412,7 @@ __global__ void __launch_bounds__(AM_THREADS) prompt_attention_f32_kernel(const 
 // ---- a decode step: one new token a sequence.  Its key and value go from the fused product into position `len` of the caches
 // ([sequence][key head][position][HD]), and its query heads attend to positions 0 .. len.  grid (parts, key heads, sequences), a cluster
 // of `parts` blocks for the keys of one head of one sequence; each warp goes through tiles of 8 KB of keys and values, two of
-// them on the way.  The warps' results are put together in shared memory, the blocks' through the cluster's.
+// them on the way.  Bound by reading the caches: 5.2 TB/s at 60 sequences of 8 heads (126 MB).  The warps' results are put together in shared memory, the blocks' through the cluster's.
 template <int HD>
 constexpr size_t am_decode_smem() { return (size_t)(AM_THREADS / 32) * AM_RING * 8192; }
 

@@ -1781,17 +1781,17 @@ constexpr float LOG2E = 1.44269504f;
 template <int HD>
 int causal_f32(const void* qkv, void* out, int batch, int rows, int heads, int kv_heads, cudaStream_t st) {
     static std::once_flag once[64];
-    return launch_attention(prompt_attention_f32_kernel<HD>, once, dim3((unsigned)((rows + AM_KEYS - 1) / AM_KEYS), (unsigned)heads, (unsigned)batch), AM_THREADS,
+    return launch_attention(prompt_attention_f32_kernel<HD>, once, dim3((unsigned)((rows + AM_KEYS - 1) / AM_KEYS), (unsigned)heads, (unsigned)batch), AM_P_THREADS,
                             am_f32_smem<HD>(), 1, st, (const float*)qkv, (float*)out, rows, heads, kv_heads, (heads + 2 * kv_heads) * HD, LOG2E / sqrtf((float)HD));
 }
 template <typename T, int HD>
 int causal_16bit(const void* qkv, void* out, int batch, int rows, int heads, int kv_heads, cudaStream_t st) {
     static std::once_flag once[64];
-    return launch_attention(prompt_attention_kernel<T, HD>, once, dim3((unsigned)((rows + AM_KEYS - 1) / AM_KEYS), (unsigned)heads, (unsigned)batch), AM_THREADS,
+    return launch_attention(prompt_attention_kernel<T, HD>, once, dim3((unsigned)((rows + AM_KEYS - 1) / AM_KEYS), (unsigned)heads, (unsigned)batch), AM_P_THREADS,
                             am_prompt_smem<HD>(), 1, st, (const T*)qkv, (T*)out, rows, heads, kv_heads, (heads + 2 * kv_heads) * HD, LOG2E / sqrtf((float)HD));
 }
 // A cluster of up to eight blocks per key head, as many as still fit two to an SM, with 128 keys each at least.  (Twice as many blocks than
-// that, in a second wave: 11 us instead of AM_DECODE_US at 16 sequences of 1024 keys, 8 key heads of 64.)
+// that, in a second wave: 11 us instead of 7.5 at 16 sequences of 1024 keys, 8 key heads of 64.)
 template <typename T, int HD>
 int decode_16bit(const void* qkv, void* k, void* v, void* out, int rows, int heads, int kv_heads, int len, int64_t seq_step, int64_t head_step, int sms, cudaStream_t st) {
     static std::once_flag once[64];
