@@ -325,13 +325,44 @@ struct Workspace {
 // and never less than the 255 of their issue.  A tile's epilogue is hidden behind the next one except at the end, or where
 // there is no room for two sets of accumulators.  In a tile that `parts` blocks share the last one to arrive reads the other
 // parts, a round trip to L2 for every sixteen rows of each, 3000 clocks in all at least.
+// A cluster of C blocks per tile: every block's units, then what goes to the other blocks and the adding-up of its own share, 2000
+// clocks at least.  A launch that holds more than half of the SMs keeps the next one's blocks, one to an SM, from starting up
+// beside it: 3000 clocks (2048 x 8192, 20 rows: 7.1 us as 64 blocks of 32 rows, 9.2 as 128 of 16).
 struct MmPlan {
-    int Nt, m_tiles, split;
+    int Nt, m_tiles, split, cluster;
     double clocks;
 };
+constexpr int MM_SMEM = 227 * 1024, MM_RAW_UNITS = 4;
+// shared memory that is left for units of B
+int mm_b_bytes(int nt, int cluster) {
+    const int parts = cluster > 1 ? cluster * ((nt / 16 + cluster - 1) / cluster) * 8192 : 0;
+    return std::min(192 * 1024, MM_SMEM - 1024 - 512 - MM_RAW_UNITS * MM_UNIT_BYTES - parts);
+}
+// clusters of `cluster` blocks that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a GPU is made of
+int mm_clusters(int cluster, int sms) {
+    static std::atomic<int> known[9];
+    int n = known[cluster].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(sms / cluster * cluster));
+        cfg.blockDim = dim3(MM_THREADS);
+        cfg.dynamicSmemBytes = MM_SMEM;
+        cudaLaunchAttribute at[1] = {};
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)cluster, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+        cfg.attrs = at, cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, mma_spmm_kernel, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = -1;                                  // no device: no clusters
+        }
+        known[cluster].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
 int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
 MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
-    MmPlan best{0, 0, 0, 0};
+    MmPlan best{0, 0, 0, 1, 0};
     const int kbu = (kb + MM_UK - 1) / MM_UK;
     for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
         const int mt = (rows + nt - 1) / nt;
@@ -339,11 +370,17 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
         const double tiles = (double)n_tiles * mt, units = tiles * kbu;
         const double slice = std::max(255.0, 2.5 * planes * nt), epilogue = nt / 16 * 350.0;
         const bool two = 2 * planes * nt <= MM_A_COL;
-        const double whole = std::ceil(tiles / sms) * (kb * slice + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
+        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? 3000.0 : 0.0; };
+        const double whole = crowd(tiles) + std::ceil(tiles / sms) * (kb * slice + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
-        const double split = std::ceil(units / blocks) * MM_UK * slice + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
-        if (best.Nt == 0 || whole < best.clocks) best = MmPlan{nt, mt, 0, whole};
-        if (split < best.clocks) best = MmPlan{nt, mt, 1, split};
+        const double split = crowd(blocks) + std::ceil(units / blocks) * MM_UK * slice + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
+        if (best.Nt == 0 || whole < best.clocks) best = MmPlan{nt, mt, 0, 1, whole};
+        if (split < best.clocks) best = MmPlan{nt, mt, 1, 1, split};
+        for (int c = 2; c <= 8 && c <= kbu; c *= 2) {
+            if (mm_b_bytes(nt, c) < 2 * planes * nt * 128 * MM_UK || mm_clusters(c, sms) < tiles) continue;
+            const double shared = (kbu + c - 1) / c * MM_UK * slice + 2000.0 + nt / 16 * 100.0 + (nt / 16 + c - 1) / c * 350.0 + crowd(tiles * c);
+            if (shared < best.clocks) best = MmPlan{nt, mt, 2, c, shared};
+        }
         if (nt >= rows) break;
     }
     return best;
@@ -423,7 +460,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     p.status = w.status;
     p.M = rows, p.K = w.inners, p.N = w.columns;
     p.KB = w.kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
-    p.n_tiles = w.n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split;
+    p.n_tiles = w.n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split, p.cluster = plan.cluster;
     p.P = x.planes;
     p.epilogue = o.epilogue, p.y_ld = o.ld, p.plane_y = o.plane;
     p.y_step_n = o.col_major ? o.ld : 1, p.y_step_m = o.col_major ? 1 : o.ld;
@@ -433,10 +470,10 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
         if (wide && o.col_major && (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0) p.out = o.dtype == TLLM_F32 ? MM_OUT_F32_COL4 : MM_OUT_I32_COL4;
         if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && w.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
     }
-    // rings: four units of bit tiles, and as many of B as 192 KiB hold (three at 128 columns of D, two at 192)
-    p.R = 4;
+    // rings: four units of bit tiles, and as many of B as there is room for (three at 128 columns of D, two at 192 or in a cluster)
+    p.R = MM_RAW_UNITS;
     const int b_unit = x.planes * p.Nt * 128 * MM_UK;
-    p.SB = std::min(MM_MAX_STAGES, 192 * 1024 / b_unit);
+    p.SB = std::min(MM_MAX_STAGES, mm_b_bytes(p.Nt, p.cluster) / b_unit);
     p.mul4 = 4, p.mul16 = 16;
     const uint32_t fmt = x.bf16 ? 1u : 0u;
     // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B formats (bits 7-9, 10-12), both K-major,
@@ -447,18 +484,18 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     CUtensorMap map;
     int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, rows, x.planes, x.pitch, (size_t)x.plane_rows * x.pitch, p.Nt);
     if (rc) return rc;
-    const size_t smem = 1024 + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512;
-    if (smem > 227 * 1024) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
+    const size_t smem = 1024 + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512 + (p.split == 2 ? (size_t)p.cluster * ((p.Nt / 16 + p.cluster - 1) / p.cluster) * 8192 : 0);
+    if (smem > MM_SMEM || p.SB < 2) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
     static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[w.device & 63], [&] { err = cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+    std::call_once(once[w.device & 63], [&] { err = cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
     CU_TRY(err);
     // never more blocks than items: the hand-over between the blocks that share a tile counts on every block in a
     // tile's range of owners holding at least one unit of it
-    const long long items = (long long)p.n_tiles * p.m_tiles * (p.split ? p.KBU : 1);
+    const long long items = (long long)p.n_tiles * p.m_tiles * (p.split == 1 ? p.KBU : p.cluster);
     const int grid = (int)(items < w.sms ? items : w.sms);
     Workspace ws;
-    if ((p.Nt <= MM_OWN_NT && w.partial) || !p.split) p.partial = w.partial;
+    if ((p.Nt <= MM_OWN_NT && w.partial) || p.split != 1) p.partial = w.partial;
     else {
         rc = ws.take(w.device, (size_t)2 * grid * MM_TILE_N * p.Nt * sizeof(float), st);
         if (rc) return rc;
@@ -469,9 +506,16 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     cfg.blockDim = dim3(MM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1] = {pdl_attribute()};
+    cudaLaunchAttribute at[2] = {};
+    int n_at = 0;
+    if (w.pdl) at[n_at++] = pdl_attribute();
+    if (p.split == 2) {
+        at[n_at].id = cudaLaunchAttributeClusterDimension;
+        at[n_at].val.clusterDim.x = (unsigned)p.cluster, at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
+        ++n_at;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = w.pdl ? 1 : 0;
+    cfg.numAttrs = (unsigned)n_at;
     CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, *w.map, p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
@@ -746,7 +790,7 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
     return TLLM_OK;
 }
 
-// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 4 us of start-up and hand-over, the plan's
+// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 2.4 us of start-up, the plan's
 // clocks at 1.8 GHz, and 3 us for planes that have to be made first.
 double bt_model_us(int inners, int columns, int sms, int x_dtype, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
@@ -758,7 +802,7 @@ double mm_tiles_model_us(int inners, int columns, int sms, bool direct, int x_dt
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += 4.0 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms).clocks / 1800.0 + (direct ? 0.0 : 3.0);
+        t += 2.4 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms).clocks / 1800.0 + (direct ? 0.0 : 3.0);
     return t;
 }
 // which of the two: true = decode in registers

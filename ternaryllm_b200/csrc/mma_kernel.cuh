@@ -33,6 +33,9 @@
 // cut into equal contiguous ranges, one per block.  Tiles that straddle two or more blocks are summed in block order by the
 // last block to arrive, which makes the result independent of scheduling; a block does its two shared tiles first, so that
 // this adding-up hides behind the tiles it has to itself.
+// With few tiles a third way: a cluster of two, four or eight blocks cuts the units of one tile.  Each block sends its sums of the rows
+// that another one is to write straight into that one's shared memory, so that a hand-over costs one trip between SMs, not
+// partial sums to L2, a counter and partial sums back, and every block adds and writes a share of the tile.
 //
 // Every wait is bounded (see bounded_wait); on a time-out the block raises its abort flag, every role leaves
 // its loop, tensor memory is released and the status word reports the failure.
@@ -78,7 +81,8 @@ struct MmParams {
     int KBU;                  // ceil(KB / 4): units per tile
     int n_tiles, m_tiles;
     int Nt;                   // activation rows per tile; planes * Nt is the MMA's N
-    int split;                // 1: equal unit ranges, tiles may be shared; 0: whole tiles
+    int split;                // 0: whole tiles; 1: equal unit ranges, tiles may be shared; 2: a cluster per tile
+    int cluster;              // blocks per tile, split 2
     int P;                    // planes of X
     int out;                  // MM_OUT_*
     int epilogue, y_ld;       // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
@@ -221,6 +225,22 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(pred));
     return pred != 0;
 }
+
+// ---- clusters (split 2) ----------------------------------------------------------------------------------
+__device__ __forceinline__ void mm_cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of this block's shared location in block `rank`
+__device__ __forceinline__ uint32_t mm_peer(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void mm_st_peer(uint32_t addr, float a, float b, float c, float d) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void mm_arrive_peer(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 // column (of the 32 of a quarter tile) that lane `lane` of tensor memory's quarter holds
 __device__ __forceinline__ int mm_column(int lane) { return ((lane >> 1) & 1) * 16 + (lane & 1) * 8 + (lane >> 2); }
@@ -373,9 +393,13 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     // ---- this block's unit range -----------------------------------------------------------------------
     const int G = (int)gridDim.x, cta = (int)blockIdx.x, KBU = p.KBU, KB = p.KB, tiles = p.n_tiles * p.m_tiles;
     const long long total = (long long)tiles * KBU;
-    const int u0 = p.split ? (int)(total * cta / G) : (int)((long long)tiles * cta / G) * KBU;
-    const int u1 = p.split ? (int)(total * (cta + 1) / G) : (int)((long long)tiles * (cta + 1) / G) * KBU;
-    if (u0 >= u1) return;
+    const bool clustered = p.split == 2;
+    const int C = clustered ? p.cluster : 1, rank = clustered ? cta % C : 0;
+    int u0, u1;
+    if (clustered) u0 = cta / C * KBU + KBU * rank / C, u1 = cta / C * KBU + KBU * (rank + 1) / C;
+    else if (p.split) u0 = (int)(total * cta / G), u1 = (int)(total * (cta + 1) / G);
+    else u0 = (int)((long long)tiles * cta / G) * KBU, u1 = (int)((long long)tiles * (cta + 1) / G) * KBU;
+    if (u0 >= u1) return;                  // never in a cluster: KBU >= C
     const MmSegs segs(u0, u1, KBU);
 
     // ---- shared memory ---------------------------------------------------------------------------------
@@ -385,8 +409,8 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     const int Nt = p.Nt;
     const uint32_t acc_cols = (uint32_t)(p.P * Nt), b_slice = acc_cols * 128u, b_unit = MM_UK * b_slice;
     const uint32_t b_base = base, r_base = b_base + SB * b_unit;
-    const uint32_t bar_base = r_base + R * MM_UNIT_BYTES;
-    volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 52);   // [0] tensor-memory address, [1] abort
+    const uint32_t bar_base = r_base + R * MM_UNIT_BYTES, part_base = bar_base + 512u;      // part_base: the cluster's parts, [block][rows / 16][4][128] x 16 bytes
+    volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 56);   // [0] tensor-memory address, [1] abort
     volatile int* abort_flag = flags + 1;
 #define A_FULL(s) (bar_base + 8u * (uint32_t)(s))
 #define A_EMPTY(s) (bar_base + 8u * (8u + (uint32_t)(s)))
@@ -396,6 +420,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 #define RAW_EMPTY(r) (bar_base + 8u * (40u + (uint32_t)(r)))
 #define ACC_FULL(a) (bar_base + 8u * (48u + (uint32_t)(a)))
 #define ACC_EMPTY(a) (bar_base + 8u * (50u + (uint32_t)(a)))
+#define PART_FULL(q) (bar_base + 8u * (52u + (uint32_t)(q)))
 
     if (tid == 0) {
         for (int s = 0; s < MM_MAX_STAGES; ++s) {
@@ -410,12 +435,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             mbar_init(ACC_FULL(a), 1);
             mbar_init(ACC_EMPTY(a), 4);    // the four epilogue warps
         }
+        for (int q = 0; q < 4; ++q) mbar_init(PART_FULL(q), (uint32_t)max(C - 1, 1));   // the same warp of the other blocks
         flags[0] = 0;
         flags[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    __syncthreads();
+    if (clustered) mm_cluster_sync();      // the others' barriers exist
+    else __syncthreads();
     if (warp == 1) tmem_alloc(smem_u32((const void*)flags), 512);
     tc_fence_before();
     __syncthreads();
@@ -608,7 +635,44 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             };
             bool sum = false;                    // this block adds up the parts of a shared tile
             int cf = 0, cl = 0;
-            if (!full) {
+            if (clustered) {
+                // sixteen c of the rows is block c % C's to write
+                const int sixteens = Nt / 16, own = (sixteens + C - 1) / C;
+                for (int c = 0; c < sixteens; ++c) {
+                    const int o = c % C;
+                    if (o == rank) continue;
+                    float f[16];
+                    load16(16 * c, f);
+                    const uint32_t to = mm_peer(part_base + (uint32_t)(((rank * own + c / C) * 4) * 128 + nl) * 16u, (uint32_t)o);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) mm_st_peer(to + (uint32_t)t * 2048u, f[4 * t], f[4 * t + 1], f[4 * t + 2], f[4 * t + 3]);
+                }
+                __syncwarp();
+                if (lane < C && lane != rank && lane < sixteens) mm_arrive_peer(mm_peer(PART_FULL(q), (uint32_t)lane));
+                if (rank < sixteens) {
+                    MM_WAIT(PART_FULL(q), 0u);
+                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    mm_with_out(p, [&](auto out, auto silu) {
+                        uint32_t at0 = part_base + (uint32_t)nl * 16u;
+                        for (int c = rank; c < sixteens; c += C, at0 += 8192u) {
+                            float f[16];
+                            load16(16 * c, f);                          // its own part, then the others in block order
+                            uint32_t at = at0;
+#pragma unroll 1
+                            for (int cc = 0; cc < C; ++cc, at += (uint32_t)own * 8192u)
+                                if (cc != rank) {
+#pragma unroll
+                                    for (int t = 0; t < 4; ++t) {
+                                        const uint4 x = ld_shared_v4(at + (uint32_t)t * 2048u);
+                                        f[4 * t] += __uint_as_float(x.x), f[4 * t + 1] += __uint_as_float(x.y), f[4 * t + 2] += __uint_as_float(x.z), f[4 * t + 3] += __uint_as_float(x.w);
+                                    }
+                                }
+                            if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, mt * Nt + 16 * c);
+                            else mm_emit<decltype(out)::value>(p, f, n, mt * Nt + 16 * c);
+                        }
+                    });
+                }
+            } else if (!full) {
                 // The last of the blocks that share this tile to arrive adds the partial sums, in block order.  Each epilogue warp owns 32
                 // columns of the tile and runs the hand-over for them by itself.  The last block's own part stays in tensor memory;
                 // a block that finds all the others there already does not even write it.
@@ -636,7 +700,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     __threadfence();
                 }
             }
-            if (full || sum) {
+            if (!clustered && (full || sum)) {
                 // A part lies in its block's slot 0, except that the first block may have come from an earlier tile.
                 const float* part0 = p.partial + (size_t)(2 * cf + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * cf + 2) * slot_floats + nl * 4;
@@ -684,6 +748,7 @@ done:
         tmem_dealloc(tmem, 512);
     }
     if (tid == 0 && flags[1]) atomicExch(p.status, MM_ERR_WAIT);
+    if (clustered) mm_cluster_sync();      // nobody leaves while the others may still write to its shared memory
 #undef A_FULL
 #undef A_EMPTY
 #undef B_FULL
@@ -692,6 +757,7 @@ done:
 #undef RAW_EMPTY
 #undef ACC_FULL
 #undef ACC_EMPTY
+#undef PART_FULL
 }
 #undef MM_WAIT
 #undef MM_ADVANCE

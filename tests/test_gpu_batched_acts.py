@@ -10,7 +10,7 @@ import torch
 
 import oracle
 from conftest import random_ternary
-from ternaryllm_b200 import PackedMLP, PackedWeight
+from ternaryllm_b200 import PackedMLP, PackedWeight, _lib
 
 pytestmark = pytest.mark.gpu
 DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16, "i8": torch.int8}
@@ -82,4 +82,28 @@ def test_calls_with_a_workspace_replay_from_a_graph():
         g.replay()
         want = oracle.dense_f64(xs, w)
         assert np.array_equal(Y.double().cpu().numpy(), want) and np.array_equal(Z.double().cpu().numpy(), 2 * want)
+    pw.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("K,N", [(512, 256), (1000, 130), (2048, 2048), (4352, 257), (2100, 3900), (1024, 9000), (7000, 128)])
+def test_few_tiles(K, N, dtype):
+    """Products of few tiles, which clusters of two, four and eight blocks share: exact on integers, row- and column-major, at
+    row counts around the sixteens that a cluster divides among its blocks."""
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    w = torch.randint(-1, 2, (K, N), generator=g, device="cuda", dtype=torch.int8)
+    pw = PackedWeight.from_dense(w.cpu().numpy())
+    prev = _lib.lib().tllm_set_mma_min_rows(1 if dtype != "f32" else -1)
+    try:
+        for M in (1, 16, 17, 33, 48, 64, 80, 128, 131, 200, 256):
+            X = torch.randint(-16, 17, (M, K), generator=g, device="cuda").to(DT[dtype])
+            want = X.double() @ w.double()
+            out = torch.full((M, N), -1, dtype=torch.float32, device="cuda")
+            assert torch.equal(pw.matmul(X, out=out).double(), want), M
+            out.fill_(-1)
+            assert torch.equal(pw.matmul(X, out=out).double(), want), M
+            assert float((pw.matmul(X).double() - want).abs().max()) <= {"f32": 0.0, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dtype] * float(want.abs().max())
+        pw.check()
+    finally:
+        _lib.lib().tllm_set_mma_min_rows(prev)
     pw.close()
