@@ -325,9 +325,11 @@ struct Workspace {
 // and never less than the 255 of their issue.  A tile's epilogue is hidden behind the next one except at the end, or where
 // there is no room for two sets of accumulators.  In a tile that `parts` blocks share the last one to arrive reads the other
 // parts, a round trip to L2 for every sixteen rows of each, 3000 clocks in all at least.
+// The first unit of activations takes 12 clocks a row to arrive.
 // A cluster of C blocks per tile: every block's units, then what goes to the other blocks and the adding-up of its own share, 2000
 // clocks at least.  A launch that holds more than half of the SMs keeps the next one's blocks, one to an SM, from starting up
-// beside it: 3000 clocks (2048 x 8192, 20 rows: 7.1 us as 64 blocks of 32 rows, 9.2 as 128 of 16).
+// beside it: 3000 clocks (2048 x 8192, 20 rows: 8.3 us as 64 blocks of 32 rows, 9.2 as 128 of 16); 1000 behind the kernel that makes
+// planes, which starts in between.
 struct MmPlan {
     int Nt, m_tiles, split, cluster;
     double clocks;
@@ -368,18 +370,18 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
         const int mt = (rows + nt - 1) / nt;
         if (mt > MM_MAX_M_TILES) continue;
         const double tiles = (double)n_tiles * mt, units = tiles * kbu;
-        const double slice = std::max(255.0, 2.5 * planes * nt), epilogue = nt / 16 * 350.0;
+        const double slice = std::max(255.0, 2.5 * planes * nt), epilogue = nt / 16 * 350.0, fill = 12.0 * planes * nt;
         const bool two = 2 * planes * nt <= MM_A_COL;
-        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? 3000.0 : 0.0; };
+        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (planes == 1 ? 3000.0 : 1000.0) : 0.0; };
         const double whole = crowd(tiles) + std::ceil(tiles / sms) * (kb * slice + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
         const double split = crowd(blocks) + std::ceil(units / blocks) * MM_UK * slice + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
-        if (best.Nt == 0 || whole < best.clocks) best = MmPlan{nt, mt, 0, 1, whole};
-        if (split < best.clocks) best = MmPlan{nt, mt, 1, 1, split};
+        if (best.Nt == 0 || whole + fill < best.clocks) best = MmPlan{nt, mt, 0, 1, whole + fill};
+        if (split + fill < best.clocks) best = MmPlan{nt, mt, 1, 1, split + fill};
         for (int c = 2; c <= 8 && c <= kbu; c *= 2) {
             if (mm_b_bytes(nt, c) < 2 * planes * nt * 128 * MM_UK || mm_clusters(c, sms) < tiles) continue;
             const double shared = (kbu + c - 1) / c * MM_UK * slice + 2000.0 + nt / 16 * 100.0 + (nt / 16 + c - 1) / c * 350.0 + crowd(tiles * c);
-            if (shared < best.clocks) best = MmPlan{nt, mt, 2, c, shared};
+            if (shared + fill < best.clocks) best = MmPlan{nt, mt, 2, c, shared + fill};
         }
         if (nt >= rows) break;
     }
