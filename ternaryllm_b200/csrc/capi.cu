@@ -793,7 +793,7 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
 }
 
 // Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 2.4 us of start-up, the plan's
-// clocks at 1.8 GHz, and 3 us for planes that have to be made first.
+// clocks at 1.8 GHz, and 5 us for planes that have to be made first.
 double bt_model_us(int inners, int columns, int sms, int x_dtype, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
@@ -804,7 +804,7 @@ double mm_tiles_model_us(int inners, int columns, int sms, bool direct, int x_dt
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += 2.4 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms).clocks / 1800.0 + (direct ? 0.0 : 3.0);
+        t += 2.4 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms).clocks / 1800.0 + (direct ? 0.0 : 5.0);
     return t;
 }
 // which of the two: true = decode in registers
@@ -822,8 +822,9 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
     // int8 sums are exact in fp32 while K * 128 stays within 2^24
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
-        // very sparse weights: the index lists are shorter than two bits an entry (the gather model is a fifth low at 90 % zeros)
-        if (rows <= 4 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_GATHER;
+        // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (4096 x 11008, 90 % zeros, 5.6 us
+        // against 6.6).  The gather model is a fifth low there, and twice too low where there are few columns.
+        if (rows == 1 && w->lay.columns >= 4096 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_GATHER;
         return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
     if (nb && mm) return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
