@@ -705,32 +705,32 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 const float* part0 = p.partial + (size_t)(2 * cf + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * cf + 2) * slot_floats + nl * 4;
                 mm_with_out(p, [&](auto out, auto silu) {
-                for (int c16 = 0; c16 < Nt; c16 += 16) {
-                    float f[16];
-                    if (full) load16(c16, f);
-                    else {
+                    for (int c16 = 0; c16 < Nt; c16 += 16) {
+                        float f[16];
+                        if (full) load16(c16, f);
+                        else {
 #pragma unroll
-                        for (int t = 0; t < 16; ++t) f[t] = 0.f;
-                        const float* ps = part0 + (size_t)c16 * MM_TILE_N;
-                        for (int cc = cf; cc <= cl; ++cc) {
-                            if (cc == cta) {
-                                float mine[16];
-                                load16(c16, mine);
+                            for (int t = 0; t < 16; ++t) f[t] = 0.f;
+                            const float* ps = part0 + (size_t)c16 * MM_TILE_N;
+                            for (int cc = cf; cc <= cl; ++cc) {
+                                if (cc == cta) {
+                                    float mine[16];
+                                    load16(c16, mine);
 #pragma unroll
-                                for (int t = 0; t < 16; ++t) f[t] += mine[t];
-                            } else {
-                                float4 x[4];
+                                    for (int t = 0; t < 16; ++t) f[t] += mine[t];
+                                } else {
+                                    float4 x[4];
 #pragma unroll
-                                for (int t = 0; t < 4; ++t) x[t] = __ldcg((const float4*)(ps + (size_t)(4 * t) * MM_TILE_N));
+                                    for (int t = 0; t < 4; ++t) x[t] = __ldcg((const float4*)(ps + (size_t)(4 * t) * MM_TILE_N));
 #pragma unroll
-                                for (int t = 0; t < 4; ++t) f[4 * t] += x[t].x, f[4 * t + 1] += x[t].y, f[4 * t + 2] += x[t].z, f[4 * t + 3] += x[t].w;
+                                    for (int t = 0; t < 4; ++t) f[4 * t] += x[t].x, f[4 * t + 1] += x[t].y, f[4 * t + 2] += x[t].z, f[4 * t + 3] += x[t].w;
+                                }
+                                ps = rest + (size_t)(cc - cf) * 2 * slot_floats + (size_t)c16 * MM_TILE_N;
                             }
-                            ps = rest + (size_t)(cc - cf) * 2 * slot_floats + (size_t)c16 * MM_TILE_N;
                         }
+                        if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, mt * Nt + c16);
+                        else mm_emit<decltype(out)::value>(p, f, n, mt * Nt + c16);
                     }
-                    if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, mt * Nt + c16);
-                    else mm_emit<decltype(out)::value>(p, f, n, mt * Nt + c16);
-                }
                 });
             }
             tc_fence_before();
