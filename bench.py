@@ -166,7 +166,7 @@ def spmv_records(torch, device, peak_hbm, quick=False):
     rng = np.random.default_rng(12345)
     out = {"sweep": [], "other_configs": []}
 
-    KERNELS = {"gather": "gather (index lists)", "mma": "tensor core (two-bit tiles)", "nibble": "decode tensor core (four-bit planes by TMA)"}
+    KERNELS = {"gather": "gather (index lists)", "mma": "tensor core (two-bit tiles)", "bits": "register decoder (two-bit tiles)", "nibble": "decode tensor core (four-bit planes by TMA)"}
 
     def pin(which):
         """auto = the library's cost model; gather / nibble = that kernel for every call it can take"""
@@ -174,11 +174,11 @@ def spmv_records(torch, device, peak_hbm, quick=False):
         L.tllm_set_nibble_max_rows({"auto": -1, "gather": 0, "nibble": 64}[which])
 
     def counters():
-        return L.tllm_mma_launch_count(), L.tllm_nibble_launch_count()
+        return L.tllm_mma_launch_count(), L.tllm_nibble_launch_count(), L.tllm_bits_launch_count()
 
     def ran_since(c0):
-        m1, n1 = counters()
-        names = ([KERNELS["mma"]] if m1 > c0[0] else []) + ([KERNELS["nibble"]] if n1 > c0[1] else [])
+        m1, n1, b1 = counters()
+        names = ([KERNELS["bits"]] if b1 > c0[2] else []) + ([KERNELS["mma"]] if m1 - c0[0] > b1 - c0[2] else []) + ([KERNELS["nibble"]] if n1 > c0[1] else [])
         return " + ".join(names) if names else KERNELS["gather"]
 
     def product(K, N, S, M, dtype=torch.float16, seed0=1000, check=True, pins=("auto",)):
@@ -208,10 +208,10 @@ def spmv_records(torch, device, peak_hbm, quick=False):
         recs = []
         for which in pins:
             pin(which)
-            m0, n0 = L.tllm_mma_launch_count(), L.tllm_nibble_launch_count()
+            m0, n0, b0 = counters()
             step()
             torch.cuda.synchronize()
-            kern = "mma" if L.tllm_mma_launch_count() > m0 else ("nibble" if L.tllm_nibble_launch_count() > n0 else "gather")
+            kern = "bits" if L.tllm_bits_launch_count() > b0 else ("mma" if L.tllm_mma_launch_count() > m0 else ("nibble" if L.tllm_nibble_launch_count() > n0 else "gather"))
             err = None
             if check:
                 ref = (X.double() @ torch.tensor(w0, device=device).double()) * scales[0]
@@ -223,7 +223,7 @@ def spmv_records(torch, device, peak_hbm, quick=False):
             us /= R
             for p in packed:
                 p.check()
-            wbytes = {"mma": info["bit_tile_bytes"], "nibble": info["nibble_bytes"], "gather": info["stream_bytes"] + info["meta_bytes"]}[kern]
+            wbytes = {"mma": info["bit_tile_bytes"], "bits": info["bit_tile_bytes"], "nibble": info["nibble_bytes"], "gather": info["stream_bytes"] + info["meta_bytes"]}[kern]
             bphys = wbytes + e * M * (K + N)
             recs.append({"K": K, "N": N, "zeros": S, "rows": M, "choice": which, "kernel": KERNELS[kern], "us_per_launch": us,
                          "algorithmic_GBps": balg / us / 1e3, "frac": balg / us / 1e3 / peak_hbm, "physical_bytes": int(bphys),

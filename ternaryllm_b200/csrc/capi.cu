@@ -58,6 +58,7 @@ static size_t dtype_size(int dt) {
 // tensor-core kernel, n > 0 = from n activation rows on.  TLLM_MMA_MIN_ROWS sets the initial value.
 static std::atomic<int> g_mm_min_rows{-2};
 static std::atomic<int64_t> g_mm_launches{0};
+static std::atomic<int64_t> g_bits_launches{0};
 static int mm_min_rows() {
     int v = g_mm_min_rows.load(std::memory_order_relaxed);
     if (v == -2) {
@@ -788,6 +789,7 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
         const int rc = bits_launch(p, w.sms, w.device, st);
         if (rc) return rc;
     }
+    g_bits_launches.fetch_add((rows + per - 1) / per, std::memory_order_relaxed);
     if (rows > 4) g_mm_launches.fetch_add((rows + per - 1) / per, std::memory_order_relaxed);   // counted with the batched products
     return TLLM_OK;
 }
@@ -1147,6 +1149,7 @@ extern "C" {
 const char* tllm_last_error(void) { return g_err.c_str(); }
 int tllm_version(void) { return 200; }
 int64_t tllm_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+int64_t tllm_bits_launch_count(void) { return g_bits_launches.load(std::memory_order_relaxed); }
 int64_t tllm_mma_launch_count(void) { return g_mm_launches.load(std::memory_order_relaxed); }
 int tllm_set_mma_min_rows(int rows) {
     const int prev = mm_min_rows();

@@ -44,7 +44,7 @@ def main(argv=None) -> int:
     packed = [PackedWeight.from_dense(w, scale=0.03125, device=dev, no_bit_tiles=0 if a.kernel in ("auto", "mma") else 1) for w in ws]
     X = torch.randn((a.rows, a.K), device=dev).to(dt)
     Y = torch.empty((a.rows, a.N), device=dev, dtype=torch.float32 if a.rows <= 64 else dt)
-    n0, g0, m0 = L.tllm_nibble_launch_count(), L.tllm_launch_count(), L.tllm_mma_launch_count()
+    n0, g0, m0, b0 = L.tllm_nibble_launch_count(), L.tllm_launch_count(), L.tllm_mma_launch_count(), L.tllm_bits_launch_count()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     for r in range(a.rounds):
         if r == a.rounds - 1:
@@ -59,7 +59,7 @@ def main(argv=None) -> int:
     ref = (X[:rows_checked].double() @ torch.tensor(ws[-1], device=dev).double()) * 0.03125
     err = float((Y[:rows_checked].double() - ref).abs().max() / ref.abs().max())
     info = packed[0].info
-    which = "nibble" if L.tllm_nibble_launch_count() > n0 else ("mma" if L.tllm_mma_launch_count() > m0 else "gather")
+    which = "bits" if L.tllm_bits_launch_count() > b0 else "nibble" if L.tllm_nibble_launch_count() > n0 else ("mma" if L.tllm_mma_launch_count() > m0 else "gather")
     print(f"{which} kernel, {L.tllm_launch_count() - g0} launches, x[{a.rows},{a.K}] {a.dtype}, W[{a.K},{a.N}] {a.zeros:.0%} zeros: "
           f"{e0.elapsed_time(e1) * 1e3 / len(packed):.2f} us per launch (eager, last round), rel err {err:.2e}; per weight: "
           f"index stream {info['stream_bytes'] + info['meta_bytes']} B, four-bit planes {info['nibble_bytes']} B, "
