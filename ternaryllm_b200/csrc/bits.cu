@@ -19,7 +19,12 @@ int launch(const BitsParams& p, int grid, size_t smem, int device, cudaStream_t 
     auto kern = bits_spmm_kernel<XT, NB, GR, ASYNC>;
     static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+    std::call_once(once[device & 63], [&] {
+        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        // An SM changes its split of L1 and shared memory only while it is idle: with the split left to each kernel, the next launch's blocks go
+        // two to an SM where there happens to be room (fp16 MLP, one row, 4096 / 11008: 29 us instead of 18).
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    });
     BT_TRY(err);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
@@ -57,7 +62,7 @@ int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device,
 // activations anew.
 namespace {
 struct BitsPlan {
-    int nb, own, own_more, split_log, per_pass, gr, pairs;     // pairs: pairs of slices a warp goes through, all passes together
+    int nb, own, own_more, split_log, per_pass, passes, gr, pairs;     // pairs: pairs of slices a warp goes through, all passes together
 };
 BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
     BitsPlan q;
@@ -66,7 +71,7 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
     const int most = q.nb > 1 ? 2 : 3, own = q.own + (q.own_more ? 1 : 0);
     q.split_log = own <= most ? 0 : own <= 2 * most ? 1 : 2;
     const int split = 1 << q.split_log, passes = (own + split * most - 1) / (split * most), kparts = BT_WARPS / split;
-    q.per_pass = (own + passes - 1) / passes;
+    q.passes = passes, q.per_pass = (own + passes - 1) / passes;
     q.gr = (q.per_pass + split - 1) / split;
     q.pairs = ((kb + 1) / 2 + kparts - 1) / kparts * passes;
     return q;
@@ -74,11 +79,11 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 }  // namespace
 
 // Microseconds of a launch: a chain of 2 us, and per pair of slices that a warp goes through what it takes sixteen warps to fetch and
-// turn the activations and to decode and multiply the columns.  Measured at 1 to 16 rows of 2048 x 2048 .. 8192 x 10240.
+// turn the activations and to decode and multiply the columns, more of it where the activations are fetched once a pass.  Measured at 1 to 16 rows of 2048 x 2048 .. 8192 x 10240.
 double bits_estimate_us(int x_dtype, int rows, int columns, int kb, int sms) {
     const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
     const double step = x_dtype == TLLM_F32 ? q.nb * (0.6 + 0.18 * q.gr) : 0.25 + q.nb * (0.15 + 0.2 * q.gr);
-    return 2.0 + q.pairs * step;
+    return 2.0 + q.pairs * (step + (q.passes > 1 ? 0.15 : 0.0));
 }
 
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {

@@ -827,6 +827,10 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
         // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (4096 x 11008, 90 % zeros, 5.6 us
         // against 6.6).  The gather model is a fifth low there, and twice too low where there are few columns.
         if (rows == 1 && w->lay.columns >= 4096 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_GATHER;
+        // A weight so wide that a block of the register decoder makes several passes: four bits an entry, which no thread touches, are read
+        // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4).  The model is 8 % high there.
+        if (nb && rows <= 8 && x_dtype != TLLM_F32 &&
+            0.92 * nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_NIBBLE;
         return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
     if (nb && mm) return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
