@@ -42,6 +42,7 @@ namespace tllm {
 
 #define BT_WARPS 16
 #define BT_SMEM_SHARED (112u * 1024u)   // two blocks of this size share an SM
+#define BT_SMEM_ALONE (116u * 1024u)    // two of this do not
 #define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks)
 #define BT_MASK 0xC000C000u             // the two codes at the top of a word's halves: 16-bit floats 0 / +-2
 
