@@ -347,14 +347,14 @@ __global__ void __launch_bounds__(RMS_MAX_THREADS) add_rmsnorm_kernel(T* x, cons
     float keep[KEEP][8], gain[KEEP][8];
     float ss = 0.f;
     pdl_launch_dependents();
-    if (weight) {                       // does not depend on the preceding kernel
+    pdl_wait();                         // weight is a caller's buffer too: the preceding kernel may have written it
+    if (weight) {                       // on the way together with x and delta
 #pragma unroll
         for (int k = 0; k < KEEP; ++k) {
             const int vi = threadIdx.x + k * nt;
             if (vi < nvec) RmsVec<T>::load(weight + (size_t)vi * N, gain[k]);
         }
     }
-    pdl_wait();
     auto first_pass = [&](int vi, float (&v)[8]) {
         float d[8];
         RmsVec<T>::load(x + row + (size_t)vi * N, v);
