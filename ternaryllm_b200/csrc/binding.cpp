@@ -10,6 +10,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -308,16 +309,17 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     BINDING_CATCH
 }
 
-// ter_spmm(X, row_idx, col_off, tile_idx | None, batch, rows, columns, inners, uniformed, padded, scale, out | None, tile_k) -> tensor
+// ter_spmm(X, row_idx, col_off, tile_idx | None, batch, rows, columns, inners, uniformed, padded, scale, out | None, tile_k, prepare) -> tensor
+// prepare: outside a stream capture the arrays are repacked first (tllm_ter_spmm_prepare), once every check has passed
 PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-    NEED_ARGS(13, "ter_spmm")
+    NEED_ARGS(14, "ter_spmm")
     BINDING_TRY
     const at::Tensor *xp = tensor_of(a[0]), *ip = tensor_of(a[1]), *op = tensor_of(a[2]);
     long long batch, rows, columns, inners, tile_k;
     if (!int_of(a[4], &batch) || !int_of(a[5], &rows) || !int_of(a[6], &columns) || !int_of(a[7], &inners) || !int_of(a[12], &tile_k)) return nullptr;
-    const int uniformed = PyObject_IsTrue(a[8]), padded = PyObject_IsTrue(a[9]);
+    const int uniformed = PyObject_IsTrue(a[8]), padded = PyObject_IsTrue(a[9]), prepare = PyObject_IsTrue(a[13]);
     const double scale = PyFloat_AsDouble(a[10]);
-    if (uniformed < 0 || padded < 0 || (scale == -1.0 && PyErr_Occurred())) return nullptr;
+    if (uniformed < 0 || padded < 0 || prepare < 0 || (scale == -1.0 && PyErr_Occurred())) return nullptr;
     const at::Tensor* three[3] = {xp, ip, op};
     const char* names[3] = {"X", "row indices", "col offsets"};
     for (int i = 0; i < 3; ++i)
@@ -357,6 +359,15 @@ PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const int16_t* idx = (const int16_t*)ip->const_data_ptr();
         const int32_t* off = (const int32_t*)op->const_data_ptr();
         int rc;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (prepare) C10_CUDA_CHECK(cudaStreamIsCapturing((cudaStream_t)st, &capture));
+        if (prepare && capture == cudaStreamCaptureStatusNone) {
+            DeviceScope there(ip->get_device());
+            Py_BEGIN_ALLOW_THREADS
+            rc = tllm_ter_spmm_prepare(idx, off, (int)columns, (int)inners, (int)tile_k);
+            Py_END_ALLOW_THREADS
+            if (rc) return raise_rc("ter_spmm.prepare", rc);
+        }
         Py_BEGIN_ALLOW_THREADS
         rc = tllm_ter_spmm(X, xcode, layout, idx, off, tile_ptr, Y, ycode, (int)batch, (int)rows, (int)columns, (int)inners, (int)tile_k, (float)scale,
                            uniformed, padded, st);
@@ -379,7 +390,7 @@ PyMethodDef methods[] = {
     {"decode_attention", (PyCFunction)(void (*)(void))decode_attention, METH_FASTCALL, "decode_attention(qkv, k_cache, v_cache, heads, len)"},
     {"causal_attention", (PyCFunction)(void (*)(void))causal_attention, METH_FASTCALL, "causal_attention(qkv, batch, rows, heads, kv_heads, head_dim)"},
     {"ter_spmm", (PyCFunction)(void (*)(void))ter_spmm, METH_FASTCALL,
-     "ter_spmm(X, row_idx, col_off, tile_idx, batch, rows, columns, inners, uniformed, padded, scale, out, tile_k)"},
+     "ter_spmm(X, row_idx, col_off, tile_idx, batch, rows, columns, inners, uniformed, padded, scale, out, tile_k, prepare)"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", "per-call path of ternaryllm_b200 (see csrc/binding.cpp)", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -103,13 +103,8 @@ def ter_spmm(X, w_tiled_merged_row_indice, w_tiled_merged_col_offset, w_col_tile
     """
     if tile_k is None:
         tile_k = tile_size_for(inners)
-    if AUTO_PREPARE and batch_size != 0 and w_tiled_merged_row_indice.is_cuda and w_tiled_merged_col_offset.is_cuda:
-        import torch
-
-        if not torch.cuda.is_current_stream_capturing():
-            prepare(w_tiled_merged_row_indice, w_tiled_merged_col_offset, columns, inners, tile_k)
     return _lib.binding().ter_spmm(X, w_tiled_merged_row_indice, w_tiled_merged_col_offset, w_col_tile_indices, batch_size, rows, columns,
-                                   inners, uniformed, padded, scale, out, tile_k)
+                                   inners, uniformed, padded, scale, out, tile_k, AUTO_PREPARE)
 
 
 def prepare(w_tiled_merged_row_indice, w_tiled_merged_col_offset, columns, inners, tile_k=None):
