@@ -292,9 +292,14 @@ int ws_pool(int device, cudaMemPool_t* out) {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
         cudaMemPool_t pool = nullptr;
-        CU_TRY(cudaMemPoolCreate(&pool, &props));
+        // the first call may come under stream capture, where making a pool is refused unless the thread says that it does not mind
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CU_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
         uint64_t keep = WS_KEEP_BYTES;
-        CU_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        cudaError_t made = cudaMemPoolCreate(&pool, &props);
+        if (made == cudaSuccess) made = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        CU_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+        CU_TRY(made);
         g_ws_pool[device] = pool;
     }
     *out = g_ws_pool[device];
