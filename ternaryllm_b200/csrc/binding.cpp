@@ -10,6 +10,8 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/Parallel.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -17,10 +19,7 @@
 
 #include <cuda_runtime.h>
 
-#include <map>
-#include <mutex>
 #include <string>
-#include <vector>
 
 #include "../../include/tllm.h"
 
@@ -133,87 +132,41 @@ PyObject* matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     BINDING_CATCH
 }
 
-// ---- page-locked result buffers ------------------------------------------------------------------------------------
-// A result that the GPU writes into page-locked memory arrives at the speed of the bus (4 MB in 86 us; 237 us into pageable
-// memory, and its pages have to be faulted in first), but making page-locked memory is slow (4 MB: 3.8 ms).  Freed buffers are
-// therefore kept, by size class, up to KEEP bytes in all, for later results of any handle; what is beyond that is freed at
-// once, and results of more than LARGEST bytes are not page-locked at all.
-class HostPool {
-  public:
-    static constexpr size_t KEEP = 64u << 20, LARGEST = 16u << 20;
-    void* take(size_t bytes, size_t* cls) {
-        size_t c = 4096;
-        while (c < bytes) c <<= 1;
-        *cls = c;
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            auto& v = free_[c];
-            if (!v.empty()) {
-                void* p = v.back();
-                v.pop_back();
-                kept_ -= c;
-                return p;
-            }
-        }
-        void* p = nullptr;
-        if (cudaHostAlloc(&p, c, cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        return p;
-    }
-    void give(void* p, size_t cls) {
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            if (kept_ + cls <= KEEP) {
-                free_[cls].push_back(p);
-                kept_ += cls;
-                return;
-            }
-        }
-        cudaFreeHost(p);
-    }
-
-  private:
-    std::mutex mu_;
-    std::map<size_t, std::vector<void*>> free_;
-    size_t kept_ = 0;
-};
-HostPool& host_pool() {
-    static HostPool* pool = new HostPool();      // never destroyed: results may outlive the module
-    return *pool;
-}
-
-// matmul_host(handle, x, x_code, x_col_major, rows, y_rows, y_columns, y_code, y_col_major, device) -> CPU tensor [y_rows, y_columns]
-// x: a C-contiguous buffer.  Copies in, runs, copies out, synchronises.
+// matmul_host(handle, x, x_code, x_col_major, rows, y, y_code, y_col_major, device): x and y are C-contiguous buffers, y writable
+// and of rows * columns elements.  Copies in, runs, copies out, synchronises.
+//
+// A result arrives in page-locked memory at the speed of the bus (4 MB in 86 us) and in pageable memory at that of the one
+// thread that the driver copies it with (257).  Results of some size therefore come through a block of torch's page-locked cache,
+// from which torch's threads copy them (144 with sixteen of them, 210 with four, 309 with two); the block is back in the cache when the
+// call returns, and only calls that run at the same time need more than one.
+constexpr int64_t STAGE_FROM = 256 << 10, STAGE_TO = 16 << 20;
 PyObject* matmul_host(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-    NEED_ARGS(10, "matmul_host")
+    NEED_ARGS(9, "matmul_host")
     BINDING_TRY
-    long long v[10];
-    for (int i = 0; i < 10; ++i)
-        if (i != 1 && !int_of(a[i], &v[i])) return nullptr;
-    Py_buffer x;
-    if (PyObject_GetBuffer(a[1], &x, PyBUF_C_CONTIGUOUS) != 0) return nullptr;
-    struct Release {
-        Py_buffer* b;
-        ~Release() { PyBuffer_Release(b); }
-    } release{&x};
-    const at::ScalarType yt = v[7] == TLLM_F16 ? at::kHalf : v[7] == TLLM_I32 ? at::kInt : at::kFloat;
-    const size_t bytes = (size_t)v[5] * v[6] * at::elementSize(yt);
-    const auto opts = at::TensorOptions().dtype(yt).device(at::kCPU);
-    at::Tensor y;
-    size_t cls = 0;
-    DeviceScope scope((c10::DeviceIndex)v[9]);
-    void* p = bytes && bytes <= HostPool::LARGEST ? host_pool().take(bytes, &cls) : nullptr;
-    if (p) y = at::from_blob(p, {v[5], v[6]}, [p, cls](void*) { host_pool().give(p, cls); }, opts);
-    else y = at::empty({v[5], v[6]}, opts);
-    void* Y = y.data_ptr();
+    long long v[9];
+    for (int i = 0; i < 9; ++i)
+        if (i != 1 && i != 5 && !int_of(a[i], &v[i])) return nullptr;
+    struct Buffer {
+        Py_buffer b{};
+        bool held = false;
+        bool get(PyObject* o, int flags) { return held = PyObject_GetBuffer(o, &b, flags) == 0; }
+        ~Buffer() {
+            if (held) PyBuffer_Release(&b);
+        }
+    } x, y;
+    if (!x.get(a[1], PyBUF_C_CONTIGUOUS) || !y.get(a[5], PyBUF_C_CONTIGUOUS | PyBUF_WRITABLE)) return nullptr;
+    DeviceScope scope((c10::DeviceIndex)v[8]);
+    const int64_t bytes = y.b.len;
+    c10::DataPtr stage;
+    if (bytes >= STAGE_FROM && bytes <= STAGE_TO && at::get_num_threads() >= 4) stage = at::getHostAllocator(at::kCUDA)->allocate((size_t)bytes);
+    void* out = stage.get() ? stage.get() : y.b.buf;
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = tllm_spmm_host((tllm_weight*)v[0], x.buf, (int)v[2], v[3] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR, (int)v[4], Y, (int)v[7], v[8] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR);
+    rc = tllm_spmm_host((tllm_weight*)v[0], x.b.buf, (int)v[2], v[3] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR, (int)v[4], out, (int)v[6], v[7] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR);
     Py_END_ALLOW_THREADS
     if (rc) return raise_rc("tllm_spmm_host", rc);
-    return THPVariable_Wrap(std::move(y));
+    if (stage.get()) at::from_blob(y.b.buf, {bytes}, at::kByte).copy_(at::from_blob(out, {bytes}, at::kByte));
+    Py_RETURN_NONE;
     BINDING_CATCH
 }
 
@@ -385,7 +338,7 @@ PyObject* ter_spmm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 PyMethodDef methods[] = {
     {"matmul", (PyCFunction)(void (*)(void))matmul, METH_FASTCALL, "matmul(handle, x, out, col_major, device, inners, columns)"},
     {"matmul_host", (PyCFunction)(void (*)(void))matmul_host, METH_FASTCALL,
-     "matmul_host(handle, x, x_code, x_col_major, rows, y_rows, y_columns, y_code, y_col_major, device)"},
+     "matmul_host(handle, x, x_code, x_col_major, rows, y, y_code, y_col_major, device)"},
     {"mlp_forward", (PyCFunction)(void (*)(void))mlp_forward, METH_FASTCALL, "mlp_forward(handle, x, out, h, hidden)"},
     {"decode_attention", (PyCFunction)(void (*)(void))decode_attention, METH_FASTCALL, "decode_attention(qkv, k_cache, v_cache, heads, len)"},
     {"causal_attention", (PyCFunction)(void (*)(void))causal_attention, METH_FASTCALL, "causal_attention(qkv, batch, rows, heads, kv_heads, head_dim)"},

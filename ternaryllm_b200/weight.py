@@ -128,8 +128,9 @@ class PackedWeight:
         rows = x.shape[1] if col_major else x.shape[0]
         if x.ndim != 2 or x.shape[0 if col_major else 1] != c[3]:
             raise RuntimeError(f"activation has {x.shape} but the weight has {c[3]} inners")
-        y_rows, y_cols = (c[4], rows) if y_col_major else (rows, c[4])
-        return _lib.binding().matmul_host(c[1], x, code, bool(col_major), rows, y_rows, y_cols, _lib.I32 if code == _lib.I8 else code, bool(y_col_major), c[2]).numpy()
+        y = np.empty((c[4], rows) if y_col_major else (rows, c[4]), np.int32 if code == _lib.I8 else x.dtype)
+        _lib.binding().matmul_host(c[1], x, code, bool(col_major), rows, y, _lib.I32 if code == _lib.I8 else code, bool(y_col_major), c[2])
+        return y
 
     def close(self):
         if self._h:

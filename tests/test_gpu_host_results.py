@@ -1,7 +1,8 @@
-"""matmul_host: results in page-locked buffers that come back to a pool, both layouts, every kernel that can serve the call.
-Exact on integers; results that are still held must not be overwritten by later calls."""
+"""matmul_host: both layouts, every kernel that can serve the call.  Exact on integers; results that are still held must not be
+overwritten by later calls, and are ordinary numpy arrays of their own memory."""
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from conftest import random_ternary
@@ -32,4 +33,28 @@ def test_layouts_and_lifetime(dtype, pin):
             assert np.array_equal(y.astype(np.float64), want)
     finally:
         _lib.lib().tllm_set_mma_min_rows(prev)
+        pw.close()
+
+
+@pytest.mark.parametrize("threads", [1, 8])                     # one: no page-locked block in between
+def test_results_are_ordinary_arrays(threads):
+    """Pageable memory of their own: a copy of one to the GPU has read its source when it returns, even with non_blocking=True,
+    so that the array may be dropped or written at once; and a program that keeps many of them locks no memory."""
+    rng = np.random.default_rng(2)
+    K, N, M = 256, 2048, 512                                    # 4 MB a result
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w)
+    xs = [rng.integers(-3, 4, size=(M, K)).astype(np.float32) for _ in range(3)]
+    before = torch.get_num_threads()
+    torch.set_num_threads(threads)
+    try:
+        for x in xs:
+            y = pw.matmul_host(x)
+            assert y.flags.owndata and y.flags.c_contiguous and y.flags.writeable
+            assert not torch.from_numpy(y).is_pinned()
+        on_gpu = [torch.from_numpy(pw.matmul_host(x)).to("cuda", non_blocking=True) for x in xs]
+        for x, y in zip(xs, on_gpu):
+            assert np.array_equal(y.double().cpu().numpy(), oracle.dense_f64(x.astype(np.float64), w))
+    finally:
+        torch.set_num_threads(before)
         pw.close()
