@@ -31,11 +31,13 @@
 // Precision.  fp16 / bf16 activations are multiplied as they are; int8 becomes fp16 (exact); an fp32 value is cut into
 // three bf16 values of eight significant bits each (truncation, so the three add up to it exactly), three columns of B
 // whose sums are added at the end.  W is 0 / +-2 (the factor two is taken back with the scale), products are exact, sums
-// are fp32; integer activations give exact sums below 2^24.
+// are fp32; integer activations give exact sums below 2^24.  A sum that is not finite is taken again entry by entry
+// (column_sum.cuh).  fp32 values below 2^-110 lose the bits under 2^-133, the last place of a bf16 value.
 #pragma once
 #include <type_traits>
 
 #include "bittile_format.h"
+#include "column_sum.cuh"
 #include "kernels.cuh"
 
 namespace tllm {
@@ -213,6 +215,14 @@ __device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, 
 #pragma unroll
         for (int i = 0; i < 8; ++i) b[i] = w[i];
     }
+}
+
+// column n of row m, entry by entry, for a sum that is not finite
+template <int XT>
+__device__ __noinline__ float bt_column_sum(const BitsParams& p, int n, int m) {
+    return column_sum((const uint32_t*)p.bits, n, p.K, p.KB, false, [&](int k) {
+        return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + k : (size_t)k * p.x_ld + m);
+    });
 }
 
 // A warp multiplies up to GR groups of sixteen columns by NB blocks of eight columns of B (activation rows; fp32: pieces of
@@ -410,15 +420,18 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                     for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
             }
             const int n = (c0 + q0 + j) * 16 + c;
+            const float sc = p.epilogue && (c & 1) ? p.scale2 : p.scale;
+            float y = v * sc;
+            if (XT != TLLM_I8 && __builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
             if (p.epilogue == 0) {
                 if (valid && n < p.N) {
                     const size_t at = (size_t)m * p.y_step_m + (size_t)n * p.y_step_n;
-                    if (p.y_dtype == TLLM_I32) ((int*)p.Y)[at] = (int)(v * 0.5f);
-                    else store_out(p.Y, p.y_dtype, at, v * p.scale);
+                    if (XT == TLLM_I8) ((int*)p.Y)[at] = (int)(v * 0.5f);
+                    else store_out(p.Y, p.y_dtype, at, y);
                 }
             } else {
-                const float u = __shfl_xor_sync(0xffffffffu, v, 1);
-                if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(v * p.scale, u * p.scale2));
+                const float u = __shfl_xor_sync(0xffffffffu, y, 1);
+                if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(y, u));
             }
         }
     }

@@ -168,7 +168,7 @@ struct BitsView {
     float* partial;               // 2 * sms hand-over slots for row tiles of up to MM_OWN_NT, or NULL
     unsigned int* counters;       // n_tiles * MM_MAX_M_TILES * 4, zero between launches
     int* status;
-    bool pdl;                     // the weight was there before the preceding kernel in the stream: the product may start beside it
+    bool lists;                   // made from lists by the preceding kernel: the product may not start beside it; else the tiles were there before
 };
 
 struct tllm_mlp {
@@ -254,7 +254,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 BitsView bits_view(const tllm_weight* w) {
-    return BitsView{w->d_bits, &w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, true};
+    return BitsView{w->d_bits, &w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, false};
 }
 
 // true when TMA can read the activations where they are (rows on 16 bytes; a box is 64 values wide)
@@ -449,6 +449,7 @@ struct MmActs {
     bool bf16;
     int planes, plane_rows;
     size_t pitch;
+    int finite;              // MmParams::finite
 };
 struct MmOut {
     void* Y;
@@ -488,6 +489,9 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     // N / 8 in bits 17-22, M / 16 in bits 24-28
     p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(x.planes * p.Nt >> 3) << 17) | ((uint32_t)(MM_TILE_N >> 4) << 24);
     p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
+    p.finite = x.finite;
+    p.bits = (const uint32_t*)w.bits, p.X = (const unsigned short*)x.base, p.bf16 = x.bf16;
+    p.ld_x = (long long)(x.pitch / 2), p.plane_x = x.plane_rows * p.ld_x;
 
     CUtensorMap map;
     int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, rows, x.planes, x.pitch, (size_t)x.plane_rows * x.pitch, p.Nt);
@@ -516,7 +520,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     cfg.stream = st;
     cudaLaunchAttribute at[2] = {};
     int n_at = 0;
-    if (w.pdl) at[n_at++] = pdl_attribute();
+    if (!w.lists) at[n_at++] = pdl_attribute();
     if (p.split == 2) {
         at[n_at].id = cudaLaunchAttributeClusterDimension;
         at[n_at].val.clusterDim.x = (unsigned)p.cluster, at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
@@ -534,7 +538,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
 int run_mm_planes(const BitsView& w, const unsigned short* planes, int plane_rows, size_t pitch, int rows, void* Y, int y_dtype, int y_ld, float scale, cudaStream_t st) {
     const int per = MM_MAX_M_TILES * mm_max_nt(3);
     for (int r0 = 0; r0 < rows; r0 += per) {
-        const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch}, std::min(rows - r0, per),
+        const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch, 1}, std::min(rows - r0, per),
                                  MmOut{(char*)Y + (size_t)r0 * y_ld * dtype_size(y_dtype), y_dtype, y_ld, 0, scale, 0.f, false, false, 0}, st);
         if (rc) return rc;
     }
@@ -548,6 +552,7 @@ int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const bool direct = mm_direct(w.inners, X, x_dtype, x_layout, x_ld);
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
+    const int finite = x_dtype == TLLM_I8 ? 0 : !direct || w.lists ? 1 : x_dtype == TLLM_BF16 ? 2 : 0;
     Workspace ws;
     if (!direct) {
         const int rc = ws.take(w.device, (size_t)planes * std::min(rows, per) * stage_pad(K) * 2, st);
@@ -556,7 +561,7 @@ int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld
     for (int r0 = 0; r0 < rows; r0 += per) {
         const int m = std::min(rows - r0, per);
         const char* xp = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
-        MmActs a{xp, x_dtype == TLLM_BF16 || x_dtype == TLLM_F32, planes, m, (size_t)x_ld * 2};
+        MmActs a{xp, x_dtype == TLLM_BF16 || x_dtype == TLLM_F32, planes, m, (size_t)x_ld * 2, finite};
         if (!direct) {
             const int rc = run_stage(xp, x_dtype, x_layout, x_ld, m, K, (unsigned short*)ws.ptr, st);
             if (rc) return rc;
@@ -778,7 +783,7 @@ int bt_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? BT_MAX_ROWS /
 int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
              float scale2, cudaStream_t st, bool y_col = false) {
     BitsParams p{};
-    p.pdl = w.pdl;
+    p.pdl = !w.lists;
     p.bits = w.bits;
     p.x_dtype = x_dtype, p.x_layout = x_layout, p.x_ld = x_ld;
     p.y_dtype = y_dtype, p.epilogue = epilogue;
@@ -1112,7 +1117,7 @@ int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, 
     rc = encode_bits_map(&map, bits, n_tiles, kb);
     if (rc) return rc;
     // not beside the preceding kernel: that is the one that writes the tiles
-    const BitsView view{(const uint4*)bits, &map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, false};
+    const BitsView view{(const uint4*)bits, &map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, true};
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const bool one = x_layout == TLLM_ROW_MAJOR && (long long)batch * rows <= 0x7fffffffLL;      // the batch is contiguous: one product
     const int parts = one ? 1 : batch, m = one ? batch * rows : rows, x_ld = x_layout == TLLM_ROW_MAJOR ? inners : rows;

@@ -44,6 +44,7 @@
 
 #include <type_traits>
 
+#include "column_sum.cuh"
 #include "kernels.cuh"
 
 namespace tllm {
@@ -92,6 +93,14 @@ struct MmParams {
     uint32_t idesc;           // tcgen05 instruction descriptor
     uint32_t mul4, mul16;     // 4 and 16
     float scale, scale2;      // half the product's scales: the decoded weights are 0 / +-2
+    // Sums that are not finite (column_sum.cuh).  0: stored as they are (int8, where there are none; fp16 read in place, which 0 / +-2 cannot
+    // overflow); 1: taken again from the rows that a column uses; 2: the same over every row, 0 * Inf = NaN included (bf16 read
+    // in place).
+    int finite;
+    const uint32_t* bits;     // the bit tiles, and X where TMA reads it: plane_x elements from plane to plane, ld_x from row to row
+    const unsigned short* X;
+    long long plane_x, ld_x;
+    bool bf16;
 };
 
 // ---- tcgen05 / TMA wrappers ------------------------------------------------------------------------------
@@ -324,6 +333,12 @@ __device__ __forceinline__ void mm_emit(const MmParams& p, const float (&f)[16],
         }
     }
 }
+// An fp32 value as bf16 values of eight significant bits: the upper half of `w` is the next one, and what is left after it is exact.  Inf
+// and NaN are the first value, with zeros behind them (Inf - Inf would be NaN).
+__device__ __forceinline__ uint32_t mm_first_piece(uint32_t w) { return (w & 0x7FFFFFFFu) > 0x7F800000u ? w | 0x00400000u : w; }
+__device__ __forceinline__ uint32_t mm_next_piece(uint32_t w) {
+    return (w & 0x7F800000u) == 0x7F800000u ? 0u : __float_as_uint(__uint_as_float(w) - __uint_as_float(w & 0xFFFF0000u));
+}
 // Gate and up columns sit in neighbouring lanes: the even one takes row t, the odd one row t + 1.
 template <int OUT>
 __device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)[16], int n, int m) {
@@ -345,11 +360,11 @@ __device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)
     } else if constexpr (OUT == MM_OUT_PLANES) {
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            uint32_t w = __float_as_uint(y[t]);
+            uint32_t w = mm_first_piece(__float_as_uint(y[t]));
 #pragma unroll
             for (int pl = 0; pl < 3; ++pl) {
                 if (ok && row + 2 * t < p.M) ((unsigned short*)p.Y)[(size_t)pl * p.plane_y + at + t * step] = (unsigned short)(w >> 16);
-                w = __float_as_uint(__uint_as_float(w) - __uint_as_float(w & 0xFFFF0000u));
+                w = mm_next_piece(w);
             }
         }
     } else {
@@ -358,6 +373,50 @@ __device__ __forceinline__ void mm_emit_silu(const MmParams& p, const float (&f)
             const unsigned short w = mm_16bit<OUT == MM_OUT_BF16>(y[t]);
             if (ok && row + 2 * t < p.M) ((unsigned short*)p.Y)[at + t * step] = w;
         }
+    }
+}
+
+// Which of sixteen sums are not finite: none, nearly always, and then one multiply-add each is all it costs.
+__device__ __forceinline__ uint32_t mm_not_finite(const MmParams& p, const float (&f)[16]) {
+    if (p.finite == 0) return 0u;
+    float z[4] = {};
+#pragma unroll
+    for (int t = 0; t < 16; ++t) z[t & 3] = fmaf(f[t], 0.f, z[t & 3]);      // 0, or NaN from the first Inf or NaN on
+    uint32_t bad = 0u;
+    if (z[0] + z[1] + z[2] + z[3] != 0.f)
+#pragma unroll
+        for (int t = 0; t < 16; ++t) bad |= finite_sum(f[t]) ? 0u : 1u << t;
+    return bad;
+}
+__device__ __noinline__ float mm_column_sum(const MmParams& p, int n, int m) {
+    return column_sum(p.bits, n, p.K, p.KB, p.finite == 2, [&](int k) {
+        float v = 0.f;
+        for (int pl = p.P - 1; pl >= 0; --pl) {
+            const unsigned short x = __ldcg(p.X + (size_t)pl * p.plane_x + (size_t)m * p.ld_x + k);
+            v += p.bf16 ? __bfloat162float(__ushort_as_bfloat16(x)) : __half2float(__ushort_as_half(x));
+        }
+        return v;
+    });
+}
+// Stores those of rows m .. m + 15 of column n again, behind the stores of the whole warp.  Of a gate and an up column either may be the
+// one, so both are summed.
+__device__ __noinline__ void mm_store_again(const MmParams& p, uint32_t bad, int n, int m) {
+    const bool half = p.out == MM_OUT_F16 || p.out == MM_OUT_F16_PAIRS, bf16 = p.out == MM_OUT_BF16 || p.out == MM_OUT_BF16_PAIRS;
+    for (; bad; bad &= bad - 1) {
+        const int row = m + __ffs(bad) - 1;
+        if (n >= p.N || row >= p.M) continue;
+        float y;
+        size_t at;
+        if (p.epilogue == 0) y = mm_column_sum(p, n, row) * (2.f * p.scale), at = (size_t)n * p.y_step_n + (size_t)row * p.y_step_m;
+        else {
+            if ((n | 1) >= p.N) continue;
+            y = silu_mul(mm_column_sum(p, n & ~1, row) * (2.f * p.scale), mm_column_sum(p, n | 1, row) * (2.f * p.scale2));
+            at = (size_t)row * p.y_ld + (n >> 1);
+        }
+        if (p.out == MM_OUT_PLANES) {
+            uint32_t w = mm_first_piece(__float_as_uint(y));
+            for (int pl = 0; pl < 3; ++pl, w = mm_next_piece(w)) ((unsigned short*)p.Y)[(size_t)pl * p.plane_y + at] = (unsigned short)(w >> 16);
+        } else store_out(p.Y, half ? TLLM_F16 : bf16 ? TLLM_BF16 : TLLM_F32, at, y);
     }
 }
 
@@ -633,6 +692,15 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     for (int t = 0; t < 16; ++t) f[t] += __uint_as_float(v[t]) + __uint_as_float(u[t]);
                 }
             };
+            auto finish16 = [&](auto out, auto silu, const float (&f)[16], int n, int m) {
+                const uint32_t bad = mm_not_finite(p, f);
+                if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, m);
+                else mm_emit<decltype(out)::value>(p, f, n, m);
+                if (__any_sync(0xffffffffu, bad)) {
+                    __syncwarp();
+                    mm_store_again(p, bad, n, m);
+                }
+            };
             bool sum = false;                    // this block adds up the parts of a shared tile
             int cf = 0, cl = 0;
             if (clustered) {
@@ -667,8 +735,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                                         f[4 * t] += __uint_as_float(x.x), f[4 * t + 1] += __uint_as_float(x.y), f[4 * t + 2] += __uint_as_float(x.z), f[4 * t + 3] += __uint_as_float(x.w);
                                     }
                                 }
-                            if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, mt * Nt + 16 * c);
-                            else mm_emit<decltype(out)::value>(p, f, n, mt * Nt + 16 * c);
+                            finish16(out, silu, f, n, mt * Nt + 16 * c);
                         }
                     });
                 }
@@ -728,8 +795,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                                 ps = rest + (size_t)(cc - cf) * 2 * slot_floats + (size_t)c16 * MM_TILE_N;
                             }
                         }
-                        if constexpr (decltype(silu)::value) mm_emit_silu<decltype(out)::value>(p, f, n, mt * Nt + c16);
-                        else mm_emit<decltype(out)::value>(p, f, n, mt * Nt + c16);
+                        finish16(out, silu, f, n, mt * Nt + c16);
                     }
                 });
             }
@@ -775,7 +841,7 @@ __device__ __forceinline__ void stage_eight(const StageParams& p, const uint32_t
     constexpr int PL = XT == TLLM_F32 ? 3 : 1;
     uint32_t v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = w[i];
+    for (int i = 0; i < 8; ++i) v[i] = XT == TLLM_F32 ? mm_first_piece(w[i]) : w[i];
 #pragma unroll
     for (int pl = 0; pl < PL; ++pl) {
         uint32_t o[4];
@@ -789,7 +855,7 @@ __device__ __forceinline__ void stage_eight(const StageParams& p, const uint32_t
         *(uint4*)(p.out + ((size_t)pl * p.M + m) * p.k_pad + k) = make_uint4(o[0], o[1], o[2], o[3]);
         if (XT == TLLM_F32) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) - __uint_as_float(v[i] & 0xFFFF0000u));   // exact
+            for (int i = 0; i < 8; ++i) v[i] = mm_next_piece(v[i]);
         }
     }
 }
