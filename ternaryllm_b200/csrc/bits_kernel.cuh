@@ -236,6 +236,9 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     extern __shared__ __align__(128) unsigned char bt_smem[];
     using Act = BitsAct<XT>;
     constexpr bool BF16 = XT == TLLM_BF16 || XT == TLLM_F32;
+    // The tensor core cuts bits off its running sum at every MMA: fp32 sums leave it after the eight of a pair of slices (gate and up of a
+    // 2560 / 6912 MLP, 8 rows, h = silu(gate) * up: off by 1.4e-7 with a warp's 40 MMAs in one sum, 1.1e-7 now).
+    constexpr bool PARTS = XT == TLLM_F32;
     constexpr int CPR = 8 * Act::E, RPI = 32 / CPR, KPC = 16 / Act::E;     // chunks per row (and pair of slices), rows per warp copy, values per chunk
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
@@ -361,6 +364,15 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                 advance();
             }
             cp_commit();
+            float part[GR][NB][4];                                   // fp32: the sums of this pair of slices
+            if constexpr (PARTS) {
+#pragma unroll
+                for (int j = 0; j < GR; ++j)
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) part[j][nb][k] = 0.f;
+            }
 #pragma unroll 1
             for (uint32_t h = 0; h < 2; ++h) {
                 uint32_t bf[NB][8];
@@ -379,12 +391,20 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                             const uint32_t a0 = a[j].x & BT_MASK, a1 = a[j].y & BT_MASK, a2 = (a[j].x * m4) & BT_MASK, a3 = (a[j].y * m4) & BT_MASK;
                             if (s < 3) a[j].x *= m16, a[j].y *= m16;
 #pragma unroll
-                            for (int nb = 0; nb < NB; ++nb) mma_16816<BF16>(acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                            for (int nb = 0; nb < NB; ++nb) mma_16816<BF16>(PARTS ? part[j][nb] : acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
                         }
                 };
                 // a warp's share of a pass is GR groups or one less (or none: GR = 1)
                 if constexpr (GR > 1) half(std::integral_constant<int, 0>{}, std::integral_constant<int, GR - 1>{});
                 if (mine == GR) half(std::integral_constant<int, GR - 1>{}, std::integral_constant<int, GR>{});
+            }
+            if constexpr (PARTS) {
+#pragma unroll
+                for (int j = 0; j < GR; ++j)
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[j][nb][k] += part[j][nb][k];
             }
             if (++cs == S) cs = 0;
         }

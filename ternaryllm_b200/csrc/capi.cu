@@ -377,16 +377,18 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
         if (mt > MM_MAX_M_TILES) continue;
         const double tiles = (double)n_tiles * mt, units = tiles * kbu;
         const double slice = std::max(255.0, 2.5 * planes * nt), epilogue = nt / 16 * 350.0, fill = 12.0 * planes * nt;
-        const bool two = 2 * planes * nt <= MM_A_COL;
+        const bool two = mm_acc_sets(planes, nt) == 2;
+        // legs of fp32 sums: where there is one set of accumulators the MMAs wait while the epilogue reads it
+        const auto legs = [&](double u) { return two || planes == 1 ? 0.0 : (std::ceil(u / MM_LEG) - 1) * (500 + nt / 16 * 150.0); };
         const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (planes == 1 ? 3000.0 : 1000.0) : 0.0; };
-        const double whole = crowd(tiles) + std::ceil(tiles / sms) * (kb * slice + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
+        const double whole = crowd(tiles) + std::ceil(tiles / sms) * (kb * slice + legs(kbu) + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
-        const double split = crowd(blocks) + std::ceil(units / blocks) * MM_UK * slice + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
+        const double split = crowd(blocks) + std::ceil(units / blocks) * MM_UK * slice + legs(std::min(units / blocks, (double)kbu)) + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
         if (best.Nt == 0 || whole + fill < best.clocks) best = MmPlan{nt, mt, 0, 1, whole + fill};
         if (split + fill < best.clocks) best = MmPlan{nt, mt, 1, 1, split + fill};
         for (int c = 2; c <= 8 && c <= kbu; c *= 2) {
             if (mm_b_bytes(nt, c) < 2 * planes * nt * 128 * MM_UK || mm_clusters(c, sms) < tiles) continue;
-            const double shared = (kbu + c - 1) / c * MM_UK * slice + 2000.0 + nt / 16 * 100.0 + (nt / 16 + c - 1) / c * 350.0 + crowd(tiles * c);
+            const double shared = (kbu + c - 1) / c * MM_UK * slice + legs((kbu + c - 1) / c) + 2000.0 + nt / 16 * 100.0 + (nt / 16 + c - 1) / c * 350.0 + crowd(tiles * c);
             if (shared + fill < best.clocks) best = MmPlan{nt, mt, 2, c, shared + fill};
         }
         if (nt >= rows) break;
@@ -471,6 +473,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     p.KB = w.kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
     p.n_tiles = w.n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split, p.cluster = plan.cluster;
     p.P = x.planes;
+    p.leg = x.planes > 1 ? MM_LEG : 1 << 24;
     p.epilogue = o.epilogue, p.y_ld = o.ld, p.plane_y = o.plane;
     p.y_step_n = o.col_major ? o.ld : 1, p.y_step_m = o.col_major ? 1 : o.ld;
     p.out = o.planes ? MM_OUT_PLANES : o.dtype == TLLM_F32 ? MM_OUT_F32 : o.dtype == TLLM_I32 ? MM_OUT_I32 : o.dtype == TLLM_F16 ? MM_OUT_F16 : MM_OUT_BF16;

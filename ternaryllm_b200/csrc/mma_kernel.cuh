@@ -56,6 +56,11 @@ namespace tllm {
 #define MM_A_UNITS 2                  // ring of expanded units in tensor memory: 128 columns each, behind 256 columns of accumulators
 #define MM_A_COL 256
 #define MM_MAX_STAGES 8
+// Units of a leg.  The tensor core cuts bits off its running sum at every MMA, always toward zero, so that a sum of many MMAs comes out too
+// small: by 3.6e-7 of the result for fp32 activations of the spread that a gated MLP makes and 432 MMAs, where fp32 additions
+// rounded to nearest are off by 7e-8.  The sums of fp32 activations therefore leave the accumulators after every 64 MMAs and
+// are added up in fp32: 8e-8.
+#define MM_LEG 4
 #define MM_THREADS (23 * 32)
 #define MM_MAX_COLS 192               // columns of D of a tile = planes * Nt, Nt (activation rows) a multiple of sixteen
 #define MM_OWN_NT 64                  // a handle's own hand-over scratch is for tiles of up to this many rows
@@ -90,6 +95,7 @@ struct MmParams {
     long long y_step_n, y_step_m;   // elements from column to column and from row to row (epilogue 0)
     long long plane_y;        // MM_OUT_PLANES: elements from plane to plane
     int SB, R;                // ring lengths: units of B, units of bit tiles
+    int leg;                  // units that are summed in the tensor core before the sum goes on in fp32 (MM_LEG)
     uint32_t idesc;           // tcgen05 instruction descriptor
     uint32_t mul4, mul16;     // 4 and 16
     float scale, scale2;      // half the product's scales: the decoded weights are 0 / +-2
@@ -148,6 +154,47 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         : "r"(taddr)
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "f"(v[0]), "f"(v[1]),
+        "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+        : "memory");
+}
+// sixteen columns of the calling warp's lanes at each of two places, one wait for both; added up
+__device__ __forceinline__ void tmem_sum16(uint32_t at, uint32_t at2, float (&f)[16]) {
+    uint32_t v[16], u[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+        : "r"(at), "r"(at2)
+        : "memory");
+#pragma unroll
+    for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]) + __uint_as_float(u[t]);
+}
+// sixteen columns of D (rows of X) of this lane's column of W, the planes added up, the small ones first
+__device__ __forceinline__ void mm_load16(uint32_t at, int nt, int planes, float (&f)[16]) {
+    uint32_t v[16];
+    if (planes == 1) {
+        tmem_ld16(at, v);
+#pragma unroll
+        for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]);
+    } else {
+        tmem_sum16(at + (uint32_t)nt, at + (uint32_t)(2 * nt), f);
+        tmem_ld16(at, v);
+#pragma unroll
+        for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]) + f[t];
+    }
+}
+__device__ __forceinline__ void mm_add16(uint32_t at, float (&f)[16]) {
+    uint32_t v[16];
+    tmem_ld16(at, v);
+#pragma unroll
+    for (int t = 0; t < 16; ++t) f[t] += __uint_as_float(v[t]);
 }
 // 2-D tiled TMA load into this block's own shared memory: coordinates are (element along K, activation row)
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -444,6 +491,8 @@ __device__ __forceinline__ void mm_with_out(const MmParams& p, F f) {
     }
 }
 
+__host__ __device__ __forceinline__ uint32_t mm_acc_sets(int planes, int nt) { return (2 * planes + (planes > 1 ? 1 : 0)) * nt <= MM_A_COL ? 2u : 1u; }
+
 __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap,
                                                                  const __grid_constant__ MmParams p) {
     extern __shared__ unsigned char mm_smem[];
@@ -507,7 +556,8 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = (uint32_t)flags[0];
-    const uint32_t accs = 2u * acc_cols <= MM_A_COL ? 2u : 1u;
+    // one or two sets of accumulators, and behind them, for fp32 activations, the sum of the legs so far
+    const uint32_t accs = mm_acc_sets(p.P, Nt), run_col = accs * acc_cols;
     pdl_launch_dependents();
 
     // Every role walks the same list of segments.
@@ -566,16 +616,18 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         const uint32_t b_lo0 = (b_base >> 4) & 0x3FFFu;
         uint32_t sa = 0, saph = 0, sb = 0, sbph = 0, a = 0, aph = 0;
         for (int i = 0; i < segs.n; ++i) {
-            int tile, ua, ub, sl;
+            int tile, ua, ub, sl, left = 0;
             segs.get(i, tile, ua, ub, sl);
-            MM_WAIT(ACC_EMPTY(a), aph ^ 1u);
-            tc_fence_after();
-            const uint32_t d = tmem + a * acc_cols;
-            uint32_t acc = 0;
+            uint32_t d = 0, acc = 0;
             MM_WAIT(A_FULL(sa), saph);
             MM_WAIT(B_FULL(sb), sbph);
             tc_fence_after();
             for (int ku = ua; ku < ub; ++ku) {
+                if (left == 0) {                             // a leg starts
+                    MM_WAIT(ACC_EMPTY(a), aph ^ 1u);
+                    tc_fence_after();
+                    d = tmem + a * acc_cols, acc = 0, left = min(p.leg, ub - ku);
+                }
                 const int nk = min(MM_UK, KB - ku * MM_UK);
                 const uint32_t at = tmem + MM_A_COL + sa * (MM_UK * 32u), b_lo = b_lo0 + sb * (b_unit >> 4), sb0 = sb, sa0 = sa;
                 // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
@@ -609,10 +661,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 }
                 __syncwarp();
                 acc = 1;
+                if (--left == 0) {
+                    if (elect_one()) umma_commit(ACC_FULL(a));
+                    __syncwarp();
+                    MM_ADVANCE(a, aph, accs);
+                }
             }
-            if (elect_one()) umma_commit(ACC_FULL(a));
-            __syncwarp();
-            MM_ADVANCE(a, aph, accs);
         }
     } else if (warp >= 7) {
         // ---- decoders: a warp expands slice h of every unit, 32 columns of W, into its 32 lanes of tensor memory.  Lane 4g + u
@@ -671,26 +725,36 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
             const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
+            const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
+            // all legs but the last join the sum in tensor memory
+            bool legs = false;
+            for (int left = ub - ua; left > p.leg; left -= p.leg) {
+                MM_WAIT(ACC_FULL(a), aph);
+                tc_fence_after();
+                for (int c16 = 0; c16 < Nt; c16 += 16) {
+                    float f[16];
+                    mm_load16(lanes + a * acc_cols + (uint32_t)c16, Nt, p.P, f);
+                    if (legs) mm_add16(lanes + run_col + (uint32_t)c16, f);
+                    tmem_st16(lanes + run_col + (uint32_t)c16, f);
+                }
+                tmem_wait_st();
+                legs = true;
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ACC_EMPTY(a));
+                MM_ADVANCE(a, aph, accs);
+            }
             MM_WAIT(ACC_FULL(a), aph);
             tc_fence_after();
             const bool full = ua == 0 && ub == KBU;
-            const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + a * acc_cols;
+            const uint32_t taddr = lanes + a * acc_cols;
             const size_t slot_floats = (size_t)MM_TILE_N * Nt;
             float* slot = p.partial + (size_t)(2 * cta + sl) * slot_floats + nl * 4;
             const int n = nt * MM_TILE_N + ncol;
             // sixteen accumulator columns (rows of X) of this lane's column of W
             auto load16 = [&](int c16, float (&f)[16]) {
-                uint32_t v[16];
-                tmem_ld16(taddr + (uint32_t)c16, v);
-#pragma unroll
-                for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]);
-                if (p.P > 1) {
-                    uint32_t u[16];
-                    tmem_ld16(taddr + (uint32_t)(Nt + c16), v);
-                    tmem_ld16(taddr + (uint32_t)(2 * Nt + c16), u);
-#pragma unroll
-                    for (int t = 0; t < 16; ++t) f[t] += __uint_as_float(v[t]) + __uint_as_float(u[t]);
-                }
+                mm_load16(taddr + (uint32_t)c16, Nt, p.P, f);
+                if (legs) mm_add16(lanes + run_col + (uint32_t)c16, f);
             };
             auto finish16 = [&](auto out, auto silu, const float (&f)[16], int n, int m) {
                 const uint32_t bad = mm_not_finite(p, f);
