@@ -9,12 +9,12 @@
 #include <atomic>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/tllm.h"
 #include "bstream_format.h"
 #include "column_lists.h"
+#include "util.h"
 
 namespace {
 
@@ -259,13 +259,7 @@ const char* bs_pack_dense(const int8_t* w, int inners, int columns, const tllm_p
                 while (B.stream.size() % 512) B.stream.push_back(0);
             }
         };
-        unsigned nthreads = std::thread::hardware_concurrency();
-        nthreads = std::max(1u, std::min(nthreads, 32u));
-        nthreads = std::min<unsigned>(nthreads, (unsigned)L.num_ctas);
-        std::vector<std::thread> pool;
-        for (unsigned i = 1; i < nthreads; ++i) pool.emplace_back(work);
-        work();
-        for (std::thread& th : pool) th.join();
+        tllm::on_threads((unsigned)L.num_ctas, work);
         if (too_big.load()) {
             col_blocks = std::min((columns + 1) / 2, std::max(col_blocks + 1, (int)((int64_t)col_blocks * 3 / 2)));
             continue;

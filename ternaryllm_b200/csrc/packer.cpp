@@ -11,7 +11,6 @@
 #include <cstring>
 #include <numeric>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/tllm.h"
@@ -390,7 +389,7 @@ extern "C" int tllm_ternarize(const float* w, int inners, int columns, float thr
 }
 
 // ---------------------------------------------------------------------------------------------------
-// bit tiles: the dense two-bit copy the tensor-core kernel reads (layout: tstream_format.h)
+// bit tiles: the dense two-bit copy the tensor-core kernel reads (layout: bittile_format.h)
 // ---------------------------------------------------------------------------------------------------
 void mm_pack_bits(const int8_t* w, int inners, int columns, std::vector<uint32_t>* bits, int* n_tiles, int* kb_out) {
     const int NT = (columns + 127) / 128, KB = (inners + 63) / 64;
@@ -413,11 +412,7 @@ void mm_pack_bits(const int8_t* w, int inners, int columns, std::vector<uint32_t
             }
         }
     };
-    const unsigned nthreads = std::min<unsigned>(std::max(1u, std::min(std::thread::hardware_concurrency(), 32u)), (unsigned)NT);
-    std::vector<std::thread> pool;
-    for (unsigned i = 1; i < nthreads; ++i) pool.emplace_back(work);
-    work();
-    for (std::thread& th : pool) th.join();
+    tllm::on_threads((unsigned)NT, work);
     *n_tiles = NT;
     *kb_out = KB;
 }
@@ -535,12 +530,7 @@ void nb_pack_dense(const int8_t* w, int inners, int columns, NbHostImage* out) {
             }
         }
     };
-    unsigned nthreads = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
-    nthreads = std::min<unsigned>(nthreads, (unsigned)tiles);
-    std::vector<std::thread> pool;
-    for (unsigned i = 1; i < nthreads; ++i) pool.emplace_back(work);
-    work();
-    for (std::thread& th : pool) th.join();
+    tllm::on_threads((unsigned)tiles, work);
 }
 
 bool nb_unpack_dense(const NbHostImage& img, int8_t* w) {

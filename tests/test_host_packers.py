@@ -4,6 +4,8 @@ tile-stream packer round-trips and keeps the invariants its kernel relies on."""
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -270,3 +272,26 @@ def test_ternarize_matches_the_numpy_restatement(mode):
     # the scale minimises |w - s*t| over s for the chosen t
     kept = t != 0
     assert abs(s - np.abs(w[kept]).mean()) <= 1e-6 * s
+
+
+THREADLESS = """
+import resource, sys
+import numpy as np
+sys.path.insert(0, "tests")
+import test_host_packers as t
+from conftest import random_ternary
+w = random_ternary(np.random.default_rng(1), 512, 512, 0.5)
+assert t._roundtrip(w)[0] == 0
+pages = int(open("/proc/self/statm").read().split()[0])
+room = pages * resource.getpagesize() + (6 << 20)              # less than the stack of one thread
+resource.setrlimit(resource.RLIMIT_AS, (room, room))
+rc, out, info = t._roundtrip(w)
+assert rc == 0 and np.array_equal(out, w)
+print("ok")
+"""
+
+
+def test_packers_without_a_second_thread():
+    """Where the system gives no more threads, the packers run on the caller's: nothing is thrown through the C entry."""
+    r = subprocess.run([sys.executable, "-c", THREADLESS], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stderr[-1000:])
