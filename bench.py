@@ -178,7 +178,7 @@ def spmv_records(torch, device, peak_hbm, quick=False):
 
     def ran_since(c0):
         m1, n1, b1 = counters()
-        names = ([KERNELS["bits"]] if b1 > c0[2] else []) + ([KERNELS["mma"]] if m1 - c0[0] > b1 - c0[2] else []) + ([KERNELS["nibble"]] if n1 > c0[1] else [])
+        names = ([KERNELS["bits"]] if b1 > c0[2] else []) + ([KERNELS["mma"]] if m1 > c0[0] else []) + ([KERNELS["nibble"]] if n1 > c0[1] else [])
         return " + ".join(names) if names else KERNELS["gather"]
 
     def product(K, N, S, M, dtype=torch.float16, seed0=1000, check=True, pins=("auto",)):
@@ -385,11 +385,11 @@ def decoder_bench(torch, dist, world, rank, device, steps, warmup, sparsities, b
                     x, pending = layers[i % nsets](x, pending)
                 result["y"] = layers[0].finish(x, pending)
 
-            n0, m0, d0 = L.tllm_launch_count(), L.tllm_mma_launch_count(), L.tllm_nibble_launch_count()
+            n0, m0, d0, b0 = L.tllm_launch_count(), L.tllm_mma_launch_count(), L.tllm_nibble_launch_count(), L.tllm_bits_launch_count()
             step()
             torch.cuda.synchronize()
             launches, tensor_launches = L.tllm_launch_count() - n0, L.tllm_mma_launch_count() - m0
-            decode_tc_launches = L.tllm_nibble_launch_count() - d0
+            decode_tc_launches, decoder_launches = L.tllm_nibble_launch_count() - d0, L.tllm_bits_launch_count() - b0
             assert torch.isfinite(result["y"].float()).all()
             graph = capture(torch, step)
             y = result["y"]                           # the tensor the captured step writes
@@ -426,7 +426,7 @@ def decoder_bench(torch, dist, world, rank, device, steps, warmup, sparsities, b
                 ms, dt_e2e = float(t[0]), float(t[1])
             rec = {"zeros": S, "batch": batch, "tokens_per_s": batch / (ms * 1e-3), "ms_per_step": ms, "steps": nsteps,
                    "e2e_tokens_per_s": batch / dt_e2e, "launches_per_step": int(launches), "tensor_core_launches_per_step": int(tensor_launches),
-                   "decode_tensor_core_launches_per_step": int(decode_tc_launches),
+                   "decode_tensor_core_launches_per_step": int(decode_tc_launches), "register_decoder_launches_per_step": int(decoder_launches),
                    "weight_sets": nsets, "algorithmic_weight_GBps_per_rank": alg_local / (ms * 1e-3) / 1e9, "parity_rel_err": parity,
                    "h2d_bytes_per_step": batch * d["hidden"] * 2, "d2h_bytes_per_step": batch * d["hidden"] * 2}
             if headline is None:
@@ -436,7 +436,8 @@ def decoder_bench(torch, dist, world, rank, device, steps, warmup, sparsities, b
                 balg_launch = layers[0].alg_bytes_local / per_layer
                 rec["products_only"] = {"us_per_launch": us_launch, "launches_per_layer": per_layer, "algorithmic_bytes_per_launch": balg_launch,
                                         "algorithmic_GBps": balg_launch / us_launch / 1e3,
-                                        "kernel": "nibble_spmm_kernel" if decode_tc_launches else ("mma_spmm_kernel" if tensor_launches else "bstream_spmm_kernel")}
+                                        "kernel": " + ".join(name for name, ran in (("bits_spmm_kernel", decoder_launches), ("nibble_spmm_kernel", decode_tc_launches),
+                                                                                    ("mma_spmm_kernel", tensor_launches)) if ran) or "bstream_spmm_kernel"}
             records.append(rec)
             note(f"{S:.0%} zeros, batch {batch}: {rec['tokens_per_s']:.1f} tokens/s ({ms:.2f} ms/step)")
             del graph

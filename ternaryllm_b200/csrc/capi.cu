@@ -803,7 +803,6 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
         if (rc) return rc;
     }
     g_bits_launches.fetch_add((rows + per - 1) / per, std::memory_order_relaxed);
-    if (rows > 4) g_mm_launches.fetch_add((rows + per - 1) / per, std::memory_order_relaxed);   // counted with the batched products
     return TLLM_OK;
 }
 

@@ -163,20 +163,30 @@ def test_crossover_setting_and_fallbacks():
 
 
 def test_cost_model_dispatch():
-    """Default setting: one row always gathers; many rows of a matrix dense enough go to the tensor cores; a
-    90 %-sparse matrix keeps a few rows on the gather kernel (its index lists are shorter than the dense copy)."""
+    """Default setting, by the launches of each kernel: one row of a wide, 90 %-sparse weight goes to the gather kernel (its index
+    lists are shorter than two bits an entry) and a few rows of any weight to the register decoder; many rows go to the
+    batched tensor-core kernel; a few 16-bit rows of a weight so wide that the decoder makes several passes go to the kernel on
+    four-bit planes."""
     L = _lib.lib()
     L.tllm_set_mma_min_rows(-1)
     rng = np.random.default_rng(15)
-    K, N = 4096, 2816
-    for s, rows_gather, rows_tensor in ((0.5, (1,), (8, 64, 300)), (0.9, (1, 2, 4), (64, 300))):
+
+    def launches():
+        return np.array([L.tllm_bits_launch_count(), L.tllm_mma_launch_count(), L.tllm_nibble_launch_count(), L.tllm_launch_count()])
+
+    for K, N, s, want in ((4096, 2816, 0.5, {1: "bits", 2: "bits", 4: "bits", 8: "bits", 64: "mma", 300: "mma"}),
+                          (4096, 2816, 0.9, {1: "bits", 4: "bits", 64: "mma", 300: "mma"}),
+                          (4096, 11008, 0.95, {1: "gather", 4: "bits", 300: "mma"}),
+                          (8192, 28672, 0.5, {1: "nibble", 300: "mma"})):
         w = random_ternary(rng, K, N, s)
         pw = PackedWeight.from_dense(w)
-        for M in rows_gather + rows_tensor:
+        Wd = torch.tensor(w, device=dev()).double()
+        for M, kernel in want.items():
             X = torch.tensor(rng.integers(-4, 5, size=(M, K)).astype(np.float32), dtype=torch.bfloat16, device=dev())
             Y = torch.empty((M, N), dtype=torch.float32, device=dev())
-            n0 = mma_launches()
+            n0 = launches()
             pw.matmul(X, out=Y)
-            assert (mma_launches() - n0 == 1) == (M in rows_tensor), (s, M)
-            assert np.array_equal(Y.double().cpu().numpy(), oracle.dense_f64(X.double().cpu().numpy(), w, 1.0))
+            n = launches() - n0
+            assert n[3] == 1 and list(n[:3]) == [kernel == "bits", kernel == "mma", kernel == "nibble"], (K, N, s, M, kernel, n)
+            assert torch.equal(Y.double(), X.double() @ Wd)
         pw.close()
