@@ -57,6 +57,8 @@ __device__ __forceinline__ uint32_t am_pack(float lo, float hi) {
         return *(const uint32_t*)&h;
     }
 }
+// What the exponents are taken from: the maximum, or 0 as long as every score was -Inf (and their weights 0, not Inf - Inf)
+__device__ __forceinline__ float am_base(float m) { return m == -INFINITY ? 0.f : m; }
 // 16-byte chunk c of row r of a tile whose rows hold HD values
 template <int HD>
 __device__ __forceinline__ uint32_t am_chunk(int r, int c) { return (uint32_t)(r * (HD * 2) + ((c ^ (r & 7)) << 4)); }
@@ -122,14 +124,14 @@ struct AmQueries {
             m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, x));
             m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, x));
         }
-        const float f0 = exp2f(mx[0] - m0), f1 = exp2f(mx[1] - m1);
+        const float b0 = am_base(m0), b1 = am_base(m1), f0 = exp2f(mx[0] - b0), f1 = exp2f(mx[1] - b1);
         mx[0] = m0, mx[1] = m1;
         sum[0] *= f0, sum[1] *= f1;
 #pragma unroll
         for (int j = 0; j < HD / 8; ++j) o[j][0] *= f0, o[j][1] *= f0, o[j][2] *= f1, o[j][3] *= f1;
 #pragma unroll
         for (int j = 0; j < KT / 8; ++j) {
-            s[j][0] = exp2f(s[j][0] - m0), s[j][1] = exp2f(s[j][1] - m0), s[j][2] = exp2f(s[j][2] - m1), s[j][3] = exp2f(s[j][3] - m1);
+            s[j][0] = exp2f(s[j][0] - b0), s[j][1] = exp2f(s[j][1] - b0), s[j][2] = exp2f(s[j][2] - b1), s[j][3] = exp2f(s[j][3] - b1);
             sum[0] += s[j][0] + s[j][1], sum[1] += s[j][2] + s[j][3];
         }
 #pragma unroll
@@ -171,7 +173,7 @@ __device__ __forceinline__ void am_join(float (&o)[N][4], float (&mx)[2], float 
         float f[2], g[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const float m1 = at[32 * (N * 4 + r)], m = fmaxf(mx[r], m1);         // the first group has seen key 0
+            const float m1 = at[32 * (N * 4 + r)], m = am_base(fmaxf(mx[r], m1));
             f[r] = exp2f(mx[r] - m), g[r] = exp2f(m1 - m);
             sum[r] = sum[r] * f[r] + at[32 * (N * 4 + 2 + r)] * g[r];
         }
@@ -358,13 +360,14 @@ __global__ void __launch_bounds__(AM_P_THREADS) prompt_attention_f32_kernel(cons
                 m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
                 m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
                 m = fmaxf(mx[r], m * scale);
-                f[r] = exp2f(mx[r] - m);
+                const float base = am_base(m);
+                f[r] = exp2f(mx[r] - base);
                 mx[r] = m;
                 sum[r] *= f[r];
 #pragma unroll
                 for (int j = 0; j < KT / 8; ++j)
 #pragma unroll
-                    for (int i = 2 * r; i < 2 * r + 2; ++i) sum[r] += s[j][i] = exp2f(fmaf(s[j][i], scale, -m));
+                    for (int i = 2 * r; i < 2 * r + 2; ++i) sum[r] += s[j][i] = exp2f(fmaf(s[j][i], scale, -base));
             }
             uint32_t p[3][KT / 16][4];
 #pragma unroll

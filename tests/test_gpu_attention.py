@@ -48,6 +48,31 @@ def test_decode(B, H, KV, D, n, dtype):
     assert float((y.double() - ref).abs().max()) <= (1e-5 + eps) * float(ref.abs().max()) + eps * float(wv.abs().max())
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_keys_that_score_minus_infinity(dtype):
+    """Finite queries and keys whose product is past the range of fp32: such a key has no weight, also where a row has seen no other
+    yet, a whole tile of them or both groups' first tiles.  The fp64 scores of these keys are below the others by 1e39."""
+    dt, eps = DT[dtype]
+    B, M, H, KV, D, far = 1, 200, 4, 2, 64, 130
+    qkv = torch.randn((M, (H + 2 * KV) * D), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).to(dt)
+    qkv[:, 0:H * D:D] = 2.0e19
+    qkv[:, H * D:(H + KV) * D:D] = 0
+    qkv[:far, H * D:(H + KV) * D:D] = -1.0e20
+    y = _lib.binding().causal_attention(qkv, B, M, H, KV, D)
+    ref = reference(qkv, B, M, H, KV, D)
+    assert float((y[far:].double() - ref[far:]).abs().max()) <= (1e-5 + eps) * float(ref.abs().max()) + eps * float(qkv[:, (H + KV) * D:].abs().max())
+    if dtype == "bf16":
+        q, rows = 5, 3                                                             # the decode step: 130 such keys, then others
+        kc, vc = (torch.randn((rows, KV, M + 1, D), device="cuda", generator=torch.Generator(device="cuda").manual_seed(q)).to(dt) for _ in range(2))
+        kc[:, :, :, 0] = 0
+        kc[:, :, :far, 0] = -1.0e20
+        x = qkv[M - rows:].contiguous()
+        got = _lib.binding().decode_attention(x, kc, vc, H, M)
+        s = x[:, :H * D].double().view(rows, KV, H // KV, D) @ kc.double().transpose(2, 3) / D ** 0.5
+        want = (s.softmax(-1) @ vc.double()).reshape(rows, H * D)
+        assert float((got.double() - want).abs().max()) <= (1e-5 + eps) * float(want.abs().max()) + eps * float(vc.abs().max())
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 def test_module_agrees_with_the_stock_core(dtype):
     dt, eps = DT[dtype]
