@@ -73,7 +73,7 @@ class LlamaTernaryAttention(nn.Module):
         """Whether a plain causal prompt goes to the library's one-launch attention, which reads the q | k | v product as it lies.
         fp32: always, the stock path is a dozen launches.  16-bit: while it takes less than the host needs for the stock path's launches
         (40 us: 14 us here at 512 positions of 16 heads of 128, 39 at 1024); the kernels behind that are faster on long prompts."""
-        if self.head_dim not in (64, 128) or bsz > 65535:
+        if self.head_dim not in (64, 128) or bsz > 65535 or torch.is_autocast_enabled("cuda"):      # autocast chooses the stock core's type
             return False
         return dtype == torch.float32 or bsz * q_len * q_len * self.num_heads * self.head_dim <= _OWN_CORE_16BIT
 

@@ -85,3 +85,14 @@ def test_module_agrees_with_the_stock_core(dtype):
         stock = m(x)[0]
     # 16-bit: the stock core rounds its probabilities and the two products round q | k | v and the result
     assert float((own - stock).abs().max()) <= (2e-5 + 8 * eps) * float(stock.abs().max())
+
+
+def test_module_under_autocast():
+    """The stock core computes in autocast's type and hands that on; so does a prompt that the library's kernel would take."""
+    cfg = TernaryConfig(hidden_size=512, num_attention_heads=8, num_key_value_heads=2, sparsity=0.7)
+    m = LlamaTernaryAttention(cfg, scales=(0.03,) * 4, generator=torch.Generator().manual_seed(0)).eval()
+    x = torch.randn((2, 45, 512), device="cuda")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.float16):
+        y = m(x)[0]
+        m._own_core = lambda *a: False
+        assert torch.equal(y, m(x)[0]) and y.dtype == torch.float16
