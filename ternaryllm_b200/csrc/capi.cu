@@ -71,8 +71,7 @@ static int mm_min_rows() {
 }
 // Cost model measured on B200 (CUDA-graph replays of back-to-back products, weights streamed from HBM), microseconds:
 // a gather launch of up to four rows costs about GATHER_FIXED + nnz * g(rows padded to 1, 2, 4), more rows take
-// ceil(rows / 4) launches; the batched tensor-core kernel about 9.8 + 0.205e-6 per matrix entry whatever the row count
-// up to 64; the decode tensor-core kernel is modelled below.  Every call goes to the kernel the model finds fastest.
+// ceil(rows / 4) launches; the decode tensor-core kernel is modelled below, the two kernels on bit tiles beside theirs.
 static const double GATHER_FIXED_US = 2.9;
 static const double GATHER_PS_PER_NNZ[3] = {0.48, 0.68, 1.35};
 // The decode tensor-core kernel: -1 = cost model, 0 = never, n > 0 = always for calls of up to n rows.
@@ -105,11 +104,6 @@ static double nibble_model_us(int64_t entries, int rows, int rows_per_launch) {
         t += NR_FIXED_US[i] + entries * 1e-6 * NR_US_PER_MENTRY[i];
     }
     return t;
-}
-static double mm_model_us(int64_t entries, int rows) { return 9.8 + entries * 0.205e-6 * (rows <= 64 ? 1.0 : rows / 64.0); }
-static bool mm_model_prefers_tensor(int64_t nnz, int64_t entries, int rows) {
-    if (rows < 2) return false;
-    return mm_model_us(entries, rows) < gather_model_us(nnz, rows);
 }
 
 }  // namespace tllm
@@ -263,14 +257,10 @@ bool mm_direct(int inners, const void* X, int x_dtype, int x_layout, int x_ld) {
            inners >= MM_TILE_K;
 }
 
-// true when the tensor-core kernel is pinned, or the cost model of the older kernels prefers it, for fp16 / bf16 row-major
-// activations whose rows TMA can address
-bool mm_usable(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows) {
-    if (!w->d_bits || !mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld) || tensor_map_encoder() == nullptr) return false;
+// true when the batched tensor-core kernel is pinned: for fp16 / bf16 row-major activations whose rows TMA can address
+bool mm_pinned(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows) {
     const int thr = mm_min_rows();
-    if (thr == 0) return false;
-    if (thr > 0) return rows >= thr;
-    return mm_model_prefers_tensor(w->lay.nnz, (int64_t)w->lay.inners * w->lay.columns, rows);
+    return thr > 0 && rows >= thr && w->d_bits && mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld) && tensor_map_encoder() != nullptr;
 }
 
 // ---- workspace of one call ---------------------------------------------------------------------------------------------
@@ -347,9 +337,9 @@ int mm_b_bytes(int nt, int cluster) {
     return std::min(192 * 1024, MM_SMEM - 1024 - 512 - MM_RAW_UNITS * MM_UNIT_BYTES - parts);
 }
 // clusters of `cluster` blocks that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a GPU is made of
-int mm_clusters(int cluster, int sms) {
-    static std::atomic<int> known[9];
-    int n = known[cluster].load(std::memory_order_relaxed);
+int mm_clusters(int cluster, int sms, int device) {
+    static std::atomic<int> known[64][9];
+    int n = device < 64 ? known[device][cluster].load(std::memory_order_relaxed) : 0;
     if (n == 0) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(sms / cluster * cluster));
@@ -362,14 +352,14 @@ int mm_clusters(int cluster, int sms) {
         if (cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, mma_spmm_kernel, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
-            n = -1;                                  // no device: no clusters
+            return 0;                                // no clusters for this call; the next one asks again
         }
-        known[cluster].store(n, std::memory_order_relaxed);
+        if (device < 64) known[device][cluster].store(n, std::memory_order_relaxed);
     }
     return n;
 }
 int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
-MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
+MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
     MmPlan best{0, 0, 0, 1, 0};
     const int kbu = (kb + MM_UK - 1) / MM_UK;
     for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
@@ -387,7 +377,7 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms) {
         if (best.Nt == 0 || whole + fill < best.clocks) best = MmPlan{nt, mt, 0, 1, whole + fill};
         if (split + fill < best.clocks) best = MmPlan{nt, mt, 1, 1, split + fill};
         for (int c = 2; c <= 8 && c <= kbu; c *= 2) {
-            if (mm_b_bytes(nt, c) < 2 * planes * nt * 128 * MM_UK || mm_clusters(c, sms) < tiles) continue;
+            if (mm_b_bytes(nt, c) < 2 * planes * nt * 128 * MM_UK || mm_clusters(c, sms, device) < tiles) continue;
             const double shared = (kbu + c - 1) / c * MM_UK * slice + legs((kbu + c - 1) / c) + 2000.0 + nt / 16 * 100.0 + (nt / 16 + c - 1) / c * 350.0 + crowd(tiles * c);
             if (shared + fill < best.clocks) best = MmPlan{nt, mt, 2, c, shared + fill};
         }
@@ -464,7 +454,7 @@ struct MmOut {
 
 // rows [0, rows) of `x` (at most MM_MAX_M_TILES tiles) in one launch of the tensor-core kernel
 int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cudaStream_t st) {
-    const MmPlan plan = mm_plan(rows, x.planes, w.n_tiles, w.kb, w.sms);
+    const MmPlan plan = mm_plan(rows, x.planes, w.n_tiles, w.kb, w.sms, w.device);
     MmParams p{};
     p.Y = o.Y;
     p.counters = w.counters;
@@ -814,25 +804,25 @@ double bt_model_us(int inners, int columns, int sms, int x_dtype, int rows) {
     for (int r0 = 0; r0 < rows; r0 += per) t += bits_estimate_us(x_dtype, std::min(rows - r0, per), columns, (inners + 63) / 64, sms);
     return t;
 }
-double mm_tiles_model_us(int inners, int columns, int sms, bool direct, int x_dtype, int rows) {
+double mm_tiles_model_us(int inners, int columns, int sms, int device, bool direct, int x_dtype, int rows) {
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += 2.4 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms).clocks / 1800.0 + (direct ? 0.0 : 5.0);
+        t += 2.4 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).clocks / 1800.0 + (direct ? 0.0 : 5.0);
     return t;
 }
 // which of the two: true = decode in registers
-bool bits_prefer_registers(int inners, int columns, int sms, bool direct, int x_dtype, int rows) {
+bool bits_prefer_registers(int inners, int columns, int sms, int device, bool direct, int x_dtype, int rows) {
     if (rows == 1) return true;
     if (rows > 8 * BT_MAX_ROWS) return false;
-    return bt_model_us(inners, columns, sms, x_dtype, rows) <= mm_tiles_model_us(inners, columns, sms, direct, x_dtype, rows);
+    return bt_model_us(inners, columns, sms, x_dtype, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
 KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_ld, int rows) {
-    const bool nb = nb_usable(w, x_dtype, x_layout, rows), mm = mm_usable(w, X, x_dtype, x_layout, x_ld, rows);
+    const bool nb = nb_usable(w, x_dtype, x_layout, rows);
     if (nb && g_nb_max_rows.load(std::memory_order_relaxed) > 0) return KERNEL_NIBBLE;     // pinned
-    if (mm && mm_min_rows() > 0) return KERNEL_MMA;                                         // pinned
+    if (mm_pinned(w, X, x_dtype, x_layout, x_ld, rows)) return KERNEL_MMA;
     const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
     // int8 sums are exact in fp32 while K * 128 stays within 2^24
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
@@ -843,10 +833,9 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
         // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4).  The model is 8 % high there.
         if (nb && rows <= 8 && x_dtype != TLLM_F32 &&
             0.92 * nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_NIBBLE;
-        return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
+        return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, w->device, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
-    if (nb && mm) return mm_model_us(entries, rows) < nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) ? KERNEL_MMA : KERNEL_NIBBLE;
-    return nb ? KERNEL_NIBBLE : (mm ? KERNEL_MMA : KERNEL_GATHER);
+    return nb ? KERNEL_NIBBLE : KERNEL_GATHER;           // no bit tiles, or the kernels on them switched off
 }
 
 // K-tiles whose activation tables one launch keeps in shared memory at the same time (the rest follow, one barrier-
@@ -1126,7 +1115,7 @@ int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, 
     for (int b = 0; b < parts; ++b) {
         const char* xp = (const char*)X + (size_t)b * rows * inners * xe;
         char* yp = (char*)Y + (size_t)b * rows * columns * ye;
-        if (bits_prefer_registers(inners, columns, sms, mm_direct(inners, xp, x_dtype, x_layout, x_ld), x_dtype, m))
+        if (bits_prefer_registers(inners, columns, sms, dev, mm_direct(inners, xp, x_dtype, x_layout, x_ld), x_dtype, m))
             rc = run_bits(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
         else rc = run_mm(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
         if (rc) return rc;
