@@ -170,12 +170,13 @@ struct tllm_mlp {
     tllm_weight* down = nullptr;
     int hidden = 0, inter = 0;
     float s_gate = 1.f, s_up = 1.f;
-    void* d_h = nullptr;
+    void* d_h = nullptr;              // never replaced: graphs that were captured with it hold its address
     size_t h_cap = 0;
-    // staging for the host-buffer entry point
+    // staging for the host-buffer entry point, grown as needed
     void* d_x = nullptr;
     void* d_y = nullptr;
-    size_t x_cap = 0, y_cap = 0;
+    void* d_hh = nullptr;
+    size_t x_cap = 0, y_cap = 0, hh_cap = 0;
 };
 
 namespace {
@@ -1694,6 +1695,7 @@ int tllm_mlp_destroy(tllm_mlp* m) {
     cudaFree(m->d_h);
     cudaFree(m->d_x);
     cudaFree(m->d_y);
+    cudaFree(m->d_hh);
     delete m;
     return TLLM_OK;
 }
@@ -1757,7 +1759,7 @@ int tllm_mlp_forward_host(tllm_mlp* m, void* X, int x_dtype, int x_layout, int r
     if (rc) return rc;
     rc = ensure(&m->d_y, &m->y_cap, xb, false);
     if (rc) return rc;
-    rc = ensure(&m->d_h, &m->h_cap, hb, false);
+    rc = ensure(&m->d_hh, &m->hh_cap, hb, false);
     if (rc) return rc;
     // a column-major caller ([hidden][rows], rows contiguous) is turned on the host: the block itself is row-major
     const bool turn = x_layout == TLLM_COL_MAJOR && rows > 1;
@@ -1770,10 +1772,10 @@ int tllm_mlp_forward_host(tllm_mlp* m, void* X, int x_dtype, int x_layout, int r
         if (H) th.resize(hb);
     }
     CU_TRY(cudaMemcpyAsync(m->d_x, hx, xb, cudaMemcpyHostToDevice, w->own_stream));
-    rc = tllm_mlp_forward(m, m->d_x, x_dtype, rows, m->d_y, m->d_h, w->own_stream);
+    rc = tllm_mlp_forward(m, m->d_x, x_dtype, rows, m->d_y, m->d_hh, w->own_stream);
     if (rc) return rc;
     CU_TRY(cudaMemcpyAsync(hx, m->d_y, xb, cudaMemcpyDeviceToHost, w->own_stream));
-    if (H) CU_TRY(cudaMemcpyAsync(turn ? (void*)th.data() : H, m->d_h, hb, cudaMemcpyDeviceToHost, w->own_stream));
+    if (H) CU_TRY(cudaMemcpyAsync(turn ? (void*)th.data() : H, m->d_hh, hb, cudaMemcpyDeviceToHost, w->own_stream));
     CU_TRY(cudaMemcpyAsync(w->h_status, w->d_status, sizeof(int), cudaMemcpyDeviceToHost, w->own_stream));
     CU_TRY(cudaStreamSynchronize(w->own_stream));
     if (turn) {
