@@ -273,7 +273,7 @@ class TernaryDecoderLayerTP(nn.Module):
     def attention(self, qkv, M):
         # one launch instead of two copies, a flash kernel and its reduction; the stock core takes what it is not built for
         if self.dtype in (torch.float16, torch.bfloat16) and self.hd in (64, 128) and self.hq <= 16 * self.hkv and qkv.is_cuda and \
-                not torch.is_autocast_enabled("cuda"):
+                self.k_cache.is_contiguous() and self.v_cache.is_contiguous() and not torch.is_autocast_enabled("cuda"):
             return _lib.binding().decode_attention(qkv, self.k_cache, self.v_cache, self.hq, self.kv_len)
         q, k, v = qkv.split([self.hq * self.hd, self.hkv * self.hd, self.hkv * self.hd], dim=1)
         q = q.view(M, self.hq, 1, self.hd)

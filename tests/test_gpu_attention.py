@@ -4,7 +4,7 @@ rounding of the result (eps of it) and of the probabilities (each off by eps of 
 import pytest
 import torch
 
-from ternaryllm_b200 import LlamaTernaryAttention, TernaryConfig, _lib
+from ternaryllm_b200 import LlamaTernaryAttention, TernaryConfig, TernaryDecoderLayerTP, _lib
 
 pytestmark = pytest.mark.gpu
 DT = {"f32": (torch.float32, 0.0), "f16": (torch.float16, 2.0 ** -11), "bf16": (torch.bfloat16, 2.0 ** -8)}
@@ -96,3 +96,15 @@ def test_module_under_autocast():
         y = m(x)[0]
         m._own_core = lambda *a: False
         assert torch.equal(y, m(x)[0]) and y.dtype == torch.float16
+
+
+def test_layer_with_caches_in_another_order():
+    """Caches that are views of another layout (positions first) go to the stock core, as the contiguous ones do to the kernel."""
+    layer = TernaryDecoderLayerTP(512, 1024, 8, 8, 64, 0.5, 1, 0, torch.device("cuda"), kv_len=40, max_batch=3, reduce="nccl")
+    qkv = torch.randn((3, 24 * 64), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).bfloat16()
+    want = layer.attention(qkv, 3)
+    k, v = layer.k_cache, layer.v_cache
+    layer.k_cache, layer.v_cache = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (k, v))
+    got = layer.attention(qkv, 3)
+    assert torch.equal(layer.k_cache, k) and torch.equal(layer.v_cache, v)
+    assert float((got - want).abs().max()) <= 4 * 2.0 ** -8 * float(want.abs().max())      # probabilities and results rounded by each
