@@ -267,7 +267,8 @@ bool mm_pinned(const tllm_weight* w, const void* X, int x_dtype, int x_layout, i
 // ---- workspace of one call ---------------------------------------------------------------------------------------------
 // Stream-ordered allocations from a pool of the library's own (one per device): a call takes what it needs, frees it behind its
 // last kernel in stream order, and the next call on the stream gets the same memory without a synchronisation.  The pool
-// is thread-safe, keeps at most WS_KEEP_BYTES across synchronisations and is trimmed to nothing when the last handle goes.
+// is thread-safe, keeps at most WS_KEEP_BYTES across synchronisations and is trimmed to nothing when the last handle goes, or, where
+// there never was one, by tllm_ter_spmm_forget(NULL, NULL).
 constexpr uint64_t WS_KEEP_BYTES = 256ull << 20;
 std::mutex g_ws_mu;
 cudaMemPool_t g_ws_pool[64] = {};
@@ -1214,6 +1215,7 @@ int tllm_ter_spmm_forget(const int16_t* row_idx, const int32_t* col_off) {
         }
     }
     for (tllm_weight* w : dead) tllm_weight_destroy(w);
+    if (!row_idx && !col_off && g_handles.load(std::memory_order_relaxed) == 0) ws_trim();      // calls on arrays as they are need no handle
     return (int)dead.size();
 }
 
@@ -1571,8 +1573,8 @@ int tllm_spmm_host(tllm_weight* w, const void* X, int x_dtype, int x_layout, int
 // Some callers run where device allocation is off the table: a serving loop whose memory pool was carved up
 // at start-up and is policed for late cudaMalloc calls, code that executes under a framework allocator it
 // must not bypass, or a latency-critical path where an allocation (which may synchronise the device) is not
-// acceptable.  tllm_spmm itself allocates nothing either, but the handle it uses had its split-K scratch
-// allocated with cudaMalloc when it was created.  This entry point does not use that scratch: partial sums
+// acceptable.  tllm_spmm takes a stream-ordered workspace for some calls, and the handle it uses had its split-K scratch
+// allocated with cudaMalloc when it was created.  This entry point uses neither: partial sums
 // and arrival counters live in the fixed array below, which every GPU that loads this library carries until
 // the process exits.  Its size is the limit on what one call may ask for.  (The 4-byte status word stays the
 // handle's own -- it exists since the handle was created -- so that tllm_weight_check reports a kernel that

@@ -1,12 +1,15 @@
 """ter_spmm on the reference's arrays with enough rows: the lists are turned into two-bit tiles on the device first
 (csrc/lists_kernel.cuh).  Pinned by the oracle's product on the arrays themselves, exact on integers; lists that bit tiles
 cannot hold (an entry named twice, a pair that cancels across lists) fall back to the per-column kernel inside the same call."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 import oracle
-from conftest import random_ternary
+from conftest import ROOT, random_ternary
 from ternaryllm_b200 import _lib, ter_spmm
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +98,28 @@ def test_lists_that_bit_tiles_cannot_hold():
             boff[column, tile, 3] = factor
             same_as_the_arrays_say(idx, boff.reshape(off.shape))
     same_as_the_arrays_say(idx, differs=False)
+
+
+GIVEN_BACK = """
+import numpy as np, torch
+from ternaryllm_b200 import ter_spmm
+K, N, T, M = 4096, 8192, 512, 1024                    # 8 MB of tiles, 25 MB of planes
+w = np.zeros((K, N), np.int32)
+w[::5], w[3::5] = 1, -1
+idx, off, _ = ter_spmm.convert_to_ter_tiled_mcsc(w, N, K, int((w == 1).sum()), int((w == -1).sum()), T, False, 4, as_numpy=True)
+ri, co = torch.tensor(idx.astype(np.int16), device="cuda"), torch.tensor(off.astype(np.int32), device="cuda")
+x, y = torch.ones((1, M, K), device="cuda"), torch.empty((1, M, N), device="cuda")
+for _ in range(2):
+    ter_spmm.ter_spmm(x, ri, co, None, 1, M, N, K, False, False, tile_k=T, out=y)
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    ter_spmm.forget()
+    assert torch.cuda.mem_get_info()[0] - held >= 24 << 20, (held, torch.cuda.mem_get_info()[0])
+print("ok")
+"""
+
+
+def test_workspaces_are_given_back():
+    """Without a handle in the process, forget() with no arguments gives back what the pool of workspaces holds."""
+    r = subprocess.run([sys.executable, "-c", GIVEN_BACK], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr[-2000:]
