@@ -914,7 +914,7 @@ int run_gather(tllm_weight* w, const void* X, int x_dtype, int x_layout, int x_l
 
 // [rows][columns] -> [columns][ld], elements of e bytes, on the device
 int turn_out(const void* src, void* dst, int rows, int columns, int ld, int e, cudaStream_t st) {
-    const dim3 grid((columns + 31) / 32, (rows + 31) / 32), block(32, 8);
+    const dim3 grid((columns + 31) / 32, std::min((rows - 1) / 32 + 1, 65535)), block(32, 8);
     if (e == 4) turn_kernel<uint32_t><<<grid, block, 0, st>>>((const uint32_t*)src, (uint32_t*)dst, rows, columns, ld);
     else turn_kernel<uint16_t><<<grid, block, 0, st>>>((const uint16_t*)src, (uint16_t*)dst, rows, columns, ld);
     CU_TRY(cudaGetLastError());

@@ -229,18 +229,22 @@ __global__ void __launch_bounds__(256) mcsc_spmm_if_kernel(const void* __restric
     }
 }
 
-// dst[c][r] = src[r][c] (ld elements from c to c), 32 x 32 tiles through shared memory; block (32, 8)
+// dst[c][r] = src[r][c] (ld elements from c to c), 32 x 32 tiles through shared memory; block (32, 8).  A grid is at most 65535 blocks
+// high: a block takes every gridDim.y-th tile of rows.
 template <typename T>
 __global__ void __launch_bounds__(256) turn_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int columns, int ld) {
     __shared__ T tile[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, x = threadIdx.x;
+    const int c0 = blockIdx.x * 32, x = threadIdx.x;
+    for (long long r0 = blockIdx.y * 32LL; r0 < rows; r0 += gridDim.y * 32LL) {
 #pragma unroll
-    for (int i = threadIdx.y; i < 32; i += 8)
-        if (r0 + i < rows && c0 + x < columns) tile[i][x] = src[(size_t)(r0 + i) * columns + c0 + x];
-    __syncthreads();
+        for (int i = threadIdx.y; i < 32; i += 8)
+            if (r0 + i < rows && c0 + x < columns) tile[i][x] = src[(size_t)(r0 + i) * columns + c0 + x];
+        __syncthreads();
 #pragma unroll
-    for (int i = threadIdx.y; i < 32; i += 8)
-        if (c0 + i < columns && r0 + x < rows) dst[(size_t)(c0 + i) * ld + r0 + x] = tile[x][i];
+        for (int i = threadIdx.y; i < 32; i += 8)
+            if (c0 + i < columns && r0 + x < rows) dst[(size_t)(c0 + i) * ld + r0 + x] = tile[x][i];
+        __syncthreads();                             // the tile has been read
+    }
 }
 
 // g[i] = silu(g[i]) * u[i]

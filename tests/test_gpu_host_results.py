@@ -58,3 +58,22 @@ def test_results_are_ordinary_arrays(threads):
     finally:
         torch.set_num_threads(before)
         pw.close()
+
+
+def test_more_rows_than_a_grid_is_high():
+    """Column-major results that are turned on the device (here behind a bias): one row more than 65535 tiles
+    of 32."""
+    rng = np.random.default_rng(4)
+    K, N, M = 16, 3, 65535 * 32 + 1
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w)
+    x = rng.integers(-3, 4, size=(M, K)).astype(np.float16)
+    bias = np.array([1.0, -2.0, 5.0], np.float16)
+    want = (x.astype(np.float32) @ w.astype(np.float32)).T + bias[:, None].astype(np.float32)
+    y = np.empty((N, M), np.float16)
+    try:
+        rc = _lib.lib().tllm_spmm_host_bias(pw._h, _lib.np_ptr(x), _lib.F16, _lib.ROW_MAJOR, M, _lib.np_ptr(bias), _lib.np_ptr(y), _lib.F16, _lib.COL_MAJOR)
+        assert rc == 0, _lib.lib().tllm_last_error()
+        assert np.array_equal(y.astype(np.float32), want)
+    finally:
+        pw.close()
