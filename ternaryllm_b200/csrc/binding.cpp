@@ -11,6 +11,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/Parallel.h>
+#include <ATen/RedispatchFunctions.h>
 #include <ATen/core/CachingHostAllocator.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -165,7 +166,10 @@ PyObject* matmul_host(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     rc = tllm_spmm_host((tllm_weight*)v[0], x.b.buf, (int)v[2], v[3] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR, (int)v[4], out, (int)v[6], v[7] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR);
     Py_END_ALLOW_THREADS
     if (rc) return raise_rc("tllm_spmm_host", rc);
-    if (stage.get()) at::from_blob(y.b.buf, {bytes}, at::kByte).copy_(at::from_blob(out, {bytes}, at::kByte));
+    if (stage.get()) {                               // straight to the CPU's copy: a dispatch mode of the caller's has no part in it
+        at::Tensor to = at::from_blob(y.b.buf, {bytes}, at::kByte);
+        at::redispatch::copy_(c10::DispatchKeySet(c10::DispatchKey::CPU), to, at::from_blob(out, {bytes}, at::kByte));
+    }
     Py_RETURN_NONE;
     BINDING_CATCH
 }

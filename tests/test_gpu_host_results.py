@@ -60,6 +60,26 @@ def test_results_are_ordinary_arrays(threads):
         pw.close()
 
 
+def test_results_under_a_dispatch_mode():
+    """The call works on numpy arrays: what intercepts torch's operations has nothing to do with it."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    rng = np.random.default_rng(3)
+    K, N, M = 96, 1024, 256                                     # 1 MB: through the page-locked block
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w)
+    x = rng.integers(-3, 4, size=(M, K)).astype(np.float32)
+    before = torch.get_num_threads()
+    torch.set_num_threads(8)
+    try:
+        with FakeTensorMode():
+            y = pw.matmul_host(x)
+        assert np.array_equal(y.astype(np.float64), oracle.dense_f64(x.astype(np.float64), w))
+    finally:
+        torch.set_num_threads(before)
+        pw.close()
+
+
 def test_more_rows_than_a_grid_is_high():
     """Column-major results that are turned on the device (here behind a bias): one row more than 65535 tiles
     of 32."""
