@@ -271,9 +271,10 @@ class TernaryDecoderLayerTP(nn.Module):
         self._part2 = torch.empty((max_batch, hidden), dtype=torch.float32, device=self.device)   # down projection's
 
     def attention(self, qkv, M):
-        # one launch instead of two copies, a flash kernel and its reduction; the stock core takes what it is not built for
+        # one launch instead of two copies, a flash kernel and its reduction; the stock core takes what it is not built for, and caches
+        # that go on behind the new position (it attends to all that they hold)
         if self.dtype in (torch.float16, torch.bfloat16) and self.hd in (64, 128) and self.hq <= 16 * self.hkv and qkv.is_cuda and \
-                self.k_cache.is_contiguous() and self.v_cache.is_contiguous() and not torch.is_autocast_enabled("cuda"):
+                self.k_cache.shape[2] == self.kv_len + 1 and self.k_cache.is_contiguous() and self.v_cache.is_contiguous() and not torch.is_autocast_enabled("cuda"):
             return _lib.binding().decode_attention(qkv, self.k_cache, self.v_cache, self.hq, self.kv_len)
         q, k, v = qkv.split([self.hq * self.hd, self.hkv * self.hd, self.hkv * self.hd], dim=1)
         q = q.view(M, self.hq, 1, self.hd)

@@ -108,3 +108,17 @@ def test_layer_with_caches_in_another_order():
     got = layer.attention(qkv, 3)
     assert torch.equal(layer.k_cache, k) and torch.equal(layer.v_cache, v)
     assert float((got - want).abs().max()) <= 4 * 2.0 ** -8 * float(want.abs().max())      # probabilities and results rounded by each
+
+
+def test_layer_with_a_cache_longer_than_its_length():
+    """The layer attends to every position that its caches hold; the one-launch kernel, which stops at the new one, is for caches that end there."""
+    layer = TernaryDecoderLayerTP(512, 1024, 8, 8, 64, 0.5, 1, 0, torch.device("cuda"), kv_len=40, max_batch=3, reduce="nccl")
+    layer.kv_len = 20
+    qkv = torch.randn((3, 24 * 64), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).bfloat16()
+    got = layer.attention(qkv, 3)
+    q, k, v = (t.view(3, 8, 64) for t in qkv.split(512, 1))
+    assert torch.equal(layer.k_cache[:, :, 20], k) and torch.equal(layer.v_cache[:, :, 20], v)
+    s = (layer.k_cache.double() @ q.double()[..., None]).squeeze(-1) / 8
+    want = (s.softmax(-1)[:, :, None] @ layer.v_cache.double()).reshape(3, 512)
+    # probabilities off by eps of themselves, the result rounded once
+    assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * (float(want.abs().max()) + float(layer.v_cache.abs().max()))
