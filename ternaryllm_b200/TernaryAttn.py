@@ -28,7 +28,7 @@ from .TernaryLinear import TernaryLinear
 from .weight import PackedWeight
 
 
-_OWN_CORE_16BIT = 704 * 704 * 2048      # positions^2 * heads * head_dim
+_OWN_CORE_16BIT, _OWN_CORE_CAPTURED = 1.82e9, 0.5e9      # heads * head_dim * positions * (positions + 192), positions in whole tiles of 64
 
 
 def _rotate_half(x):
@@ -70,12 +70,21 @@ class LlamaTernaryAttention(nn.Module):
         return pw
 
     def _own_core(self, dtype, bsz, q_len) -> bool:
-        """Whether a plain causal prompt goes to the library's one-launch attention, which reads the q | k | v product as it lies.
-        fp32: always, the stock path is a dozen launches.  16-bit: while it takes less than the host needs for the stock path's launches
-        (40 us: 14 us here at 512 positions of 16 heads of 128, 39 at 1024); the kernels behind that are faster on long prompts."""
+        """Whether a plain causal prompt goes to the library's one-launch attention, which reads the q | k | v product as it lies.  Its
+        time goes with the tiles of 64 queries and keys, whole or not, and what a block costs besides (three tiles).
+        fp32: the stock path is a dozen launches (heads repeated) or one kernel as fast as this one; not for many prompts of a few positions
+        (1024 of 8 positions, 16 / 4 heads of 64: 387 us here, 287 there; 200 of one: 71 and 133).
+        16-bit: while it takes less than the host needs for the stock path's launches (28 us: 25 and 28 here at 832 positions of 32 heads
+        of 64 and 16 of 128; 256 prompts of 16 positions, 16 heads of 128: 111 here, 55 there).  Captured launches cost the host nothing
+        when they run, and the stock kernels are the faster ones from fewer tiles on (16 heads of 128: 320 positions 9.3 us here, 11.4
+        there; 4 prompts of 256 14.9 and 9.4)."""
         if self.head_dim not in (64, 128) or bsz > 65535 or torch.is_autocast_enabled("cuda"):      # autocast chooses the stock core's type
             return False
-        return dtype == torch.float32 or bsz * q_len * q_len * self.num_heads * self.head_dim <= _OWN_CORE_16BIT
+        if dtype == torch.float32:
+            return q_len >= 16 or bsz * self.num_heads <= 4096
+        m = -(-q_len // 64) * 64
+        work = bsz * self.num_heads * self.head_dim * m * (m + 192)
+        return work <= (_OWN_CORE_CAPTURED if work > _OWN_CORE_CAPTURED and torch.cuda.is_current_stream_capturing() else _OWN_CORE_16BIT)
 
     def forward(self, hidden_states: torch.Tensor, attention_mask: Optional[torch.Tensor] = None,
                 position_embeddings: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,

@@ -87,6 +87,31 @@ def test_module_agrees_with_the_stock_core(dtype):
     assert float((own - stock).abs().max()) <= (2e-5 + 8 * eps) * float(stock.abs().max())
 
 
+# many short prompts, which leave most of a tile empty, and longer ones under capture were slower on the library's kernel than on the stock core
+@pytest.mark.parametrize("dtype, B, M, captured, own", [("f16", 1, 832, False, True), ("f16", 256, 16, False, False), ("f16", 1, 300, True, True), ("f16", 4, 256, True, False),
+                                                        ("f16", 4, 256, False, True), ("f32", 1024, 8, False, False), ("f32", 128, 1, False, True), ("f32", 2, 300, True, True)])
+def test_core_of_the_module(dtype, B, M, captured, own):
+    dt, eps = DT[dtype]
+    cfg = TernaryConfig(hidden_size=2048, num_attention_heads=16, num_key_value_heads=16, sparsity=0.9)
+    m = LlamaTernaryAttention(cfg, scales=(0.03,) * 4, generator=torch.Generator().manual_seed(0)).eval()
+    x = torch.randn((B, M, 2048), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).to(dt)
+    calls, core = [], _lib.binding()
+    seen = type("Seen", (), {"matmul": core.matmul, "causal_attention": staticmethod(lambda *a: calls.append(1) or core.causal_attention(*a))})
+    with torch.no_grad(), pytest.MonkeyPatch.context() as patch:
+        y = m(x)[0]
+        patch.setattr(_lib, "binding", lambda: seen)
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = m(x)[0]
+            graph.replay()
+        else:
+            got = m(x)[0]
+    assert len(calls) == own
+    # either core: probabilities, the core's result and the product's rounded by each
+    assert float((got - y).abs().max()) <= (2e-5 + 8 * eps) * float(y.abs().max())
+
+
 def test_module_under_autocast():
     """The stock core computes in autocast's type and hands that on; so does a prompt that the library's kernel would take."""
     cfg = TernaryConfig(hidden_size=512, num_attention_heads=8, num_key_value_heads=2, sparsity=0.7)
