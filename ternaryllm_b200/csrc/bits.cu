@@ -81,15 +81,24 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 
 // Microseconds of a launch: a chain of 2 us, and per pair of slices that a warp goes through what it takes sixteen warps to fetch and
 // turn the activations and to decode and multiply the columns, more of it where the activations are fetched once a pass.  Measured at 1 to 16 rows of 2048 x 2048 .. 8192 x 10240.
-double bits_estimate_us(int x_dtype, int rows, int columns, int kb, int sms) {
+// Activations that cp.async cannot read pass through registers with every pair, and the blocks wait for them: 2.7 us a pair where 16 rows of
+// fp16 start anywhere (bytes 1.6, 8 rows of fp32 2.4), and element by element from a column-major X, by all blocks
+// from the same lines (16 rows of fp16, 4096 x 11008: 227 us; the batched kernel behind its planes 18.5).  Measured over the
+// same sizes, 1 to 16 rows.
+double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
     const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
-    const double step = x_dtype == TLLM_F32 ? q.nb * (0.6 + 0.18 * q.gr) : 0.25 + q.nb * (0.15 + 0.2 * q.gr);
+    const bool f32 = x_dtype == TLLM_F32, i8 = x_dtype == TLLM_I8;
+    double step = f32 ? q.nb * (0.6 + 0.18 * q.gr) : 0.25 + q.nb * (0.15 + 0.2 * q.gr);
+    const double groups = (columns + 15) / 16;               // of few columns few blocks read X
+    if (access == BITS_ROWS) step += std::min(1.0, 0.6 + groups / 256) * (f32 ? 0.6 + 0.23 * rows : i8 ? 0.7 + 0.055 * rows : 0.35 + 0.15 * rows);
+    else if (access == BITS_COLUMNS)
+        step += std::min(1.0, 0.1 + groups / 128) * (i8 ? 1.6 + 0.5 * rows : (f32 ? 1.7 : 1.1) * rows * (rows <= 4 ? 0.65 : 1.0));
     return 2.0 + q.pairs * (step + (q.passes > 1 ? 0.15 : 0.0));
 }
 
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
-    const bool async = p.x_layout == TLLM_ROW_MAJOR && (uintptr_t)p.X % 16 == 0 && (size_t)p.x_ld * e % 16 == 0;
+    const bool async = bits_access(p.X, p.x_dtype, p.x_layout, p.x_ld) == BITS_ROWS16;
     const BitsPlan q = bits_plan(p.x_dtype, p.M, p.N, p.KB, sms);
     const int nb = q.nb, gr = q.gr, grid = sms, kparts = BT_WARPS >> q.split_log, cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, pairs = q.pairs;
     p.own = q.own, p.own_more = q.own_more, p.split_log = q.split_log, p.per_pass = q.per_pass;

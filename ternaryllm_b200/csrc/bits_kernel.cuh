@@ -459,7 +459,14 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
 
 // one launch of up to BT_MAX_ROWS rows (half of it fp32); fills in everything from `own` to `mul16` (bits.cu)
 int bits_launch(BitsParams& p, int sms, int device, void* stream);
+// How it reads X: rows on 16 bytes (cp.async), rows that start anywhere, or a column-major X
+enum BitsAccess { BITS_ROWS16, BITS_ROWS, BITS_COLUMNS };
+inline BitsAccess bits_access(const void* X, int x_dtype, int x_layout, int x_ld) {
+    const int e = x_dtype == TLLM_F32 ? 4 : x_dtype == TLLM_I8 ? 1 : 2;
+    if (x_layout != TLLM_ROW_MAJOR) return BITS_COLUMNS;
+    return (uintptr_t)X % 16 == 0 && (size_t)x_ld * e % 16 == 0 ? BITS_ROWS16 : BITS_ROWS;
+}
 // its time, for the choice between kernels
-double bits_estimate_us(int x_dtype, int rows, int columns, int kb, int sms);
+double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms);
 
 }  // namespace tllm

@@ -800,10 +800,10 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
 
 // Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 2.4 us of start-up, the plan's
 // clocks at 1.8 GHz, and 5 us for planes that have to be made first.
-double bt_model_us(int inners, int columns, int sms, int x_dtype, int rows) {
+double bt_model_us(int inners, int columns, int sms, int x_dtype, BitsAccess access, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
-    for (int r0 = 0; r0 < rows; r0 += per) t += bits_estimate_us(x_dtype, std::min(rows - r0, per), columns, (inners + 63) / 64, sms);
+    for (int r0 = 0; r0 < rows; r0 += per) t += bits_estimate_us(x_dtype, access, std::min(rows - r0, per), columns, (inners + 63) / 64, sms);
     return t;
 }
 double mm_tiles_model_us(int inners, int columns, int sms, int device, bool direct, int x_dtype, int rows) {
@@ -814,10 +814,10 @@ double mm_tiles_model_us(int inners, int columns, int sms, int device, bool dire
     return t;
 }
 // which of the two: true = decode in registers
-bool bits_prefer_registers(int inners, int columns, int sms, int device, bool direct, int x_dtype, int rows) {
-    if (rows == 1) return true;
+bool bits_prefer_registers(int inners, int columns, int sms, int device, bool direct, int x_dtype, BitsAccess access, int rows) {
+    if (rows == 1 && access == BITS_ROWS16) return true;
     if (rows > 8 * BT_MAX_ROWS) return false;
-    return bt_model_us(inners, columns, sms, x_dtype, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, rows);
+    return bt_model_us(inners, columns, sms, x_dtype, access, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
@@ -828,14 +828,24 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
     // int8 sums are exact in fp32 while K * 128 stays within 2^24
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
+        const int inners = w->lay.inners, columns = w->lay.columns, sms = w->mm_grid;
+        const BitsAccess access = bits_access(X, x_dtype, x_layout, x_ld);
+        const double bits = bt_model_us(inners, columns, sms, x_dtype, BITS_ROWS16, rows), gather = gather_model_us(w->lay.nnz, rows);
         // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (4096 x 11008, 90 % zeros, 5.6 us
         // against 6.6).  The gather model is a fifth low there, and twice too low where there are few columns.
-        if (rows == 1 && w->lay.columns >= 4096 && 1.25 * gather_model_us(w->lay.nnz, rows) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_GATHER;
+        if (rows == 1 && columns >= 4096 && 1.25 * gather < bits) return KERNEL_GATHER;
+        // Two rows of int8 too, which the gather kernel reads in either layout (column-major, 2048 x 8192, 70 % zeros: 6.6 us; decoded in
+        // registers 11.9; and 8192 x 28672, 90 % zeros: 22 against 35 by rows).  Its sums are exact as well.
+        if (x_dtype == TLLM_I8 && rows <= 2 && columns >= 4096 &&
+            1.35 * gather < std::min(bt_model_us(inners, columns, sms, x_dtype, access, rows), mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, rows)))
+            return KERNEL_GATHER;
         // A weight so wide that a block of the register decoder makes several passes: four bits an entry, which no thread touches, are read
-        // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4).  The model is 8 % high there.
-        if (nb && rows <= 8 && x_dtype != TLLM_F32 &&
-            0.92 * nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) < bt_model_us(w->lay.inners, w->lay.columns, w->mm_grid, x_dtype, rows)) return KERNEL_NIBBLE;
-        return bits_prefer_registers(w->lay.inners, w->lay.columns, w->mm_grid, w->device, mm_direct(w->lay.inners, X, x_dtype, x_layout, x_ld), x_dtype, rows) ? KERNEL_BITS : KERNEL_MMA;
+        // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4).  The model is 8 % high there.  More than
+        // one launch's rows (4) have to start on 16 bytes: its planes are made from X element by element else (28672 x 8192, eight rows:
+        // 82 us, the batched kernel 43).
+        const int per = nb_rows_per_launch(x_dtype);
+        if (nb && rows <= 8 && x_dtype != TLLM_F32 && (rows <= per || access == BITS_ROWS16) && 0.92 * nibble_model_us(entries, rows, per) < bits) return KERNEL_NIBBLE;
+        return bits_prefer_registers(inners, columns, sms, w->device, mm_direct(inners, X, x_dtype, x_layout, x_ld), x_dtype, access, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
     return nb ? KERNEL_NIBBLE : KERNEL_GATHER;           // no bit tiles, or the kernels on them switched off
 }
@@ -1117,7 +1127,7 @@ int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, 
     for (int b = 0; b < parts; ++b) {
         const char* xp = (const char*)X + (size_t)b * rows * inners * xe;
         char* yp = (char*)Y + (size_t)b * rows * columns * ye;
-        if (bits_prefer_registers(inners, columns, sms, dev, mm_direct(inners, xp, x_dtype, x_layout, x_ld), x_dtype, m))
+        if (bits_prefer_registers(inners, columns, sms, dev, mm_direct(inners, xp, x_dtype, x_layout, x_ld), x_dtype, bits_access(xp, x_dtype, x_layout, x_ld), m))
             rc = run_bits(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
         else rc = run_mm(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
         if (rc) return rc;
@@ -1508,6 +1518,7 @@ int tllm_spmm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows
     rc = check_device(w, "tllm_spmm");
     if (rc) return rc;
     const BsLayout& L = w->lay;
+    if (rows == 1) x_layout = TLLM_ROW_MAJOR;        // the same memory
     const int x_ld = x_layout == TLLM_ROW_MAJOR ? L.inners : rows;
     return run_product(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, L.columns, 0, w->scale, 0.f, (cudaStream_t)stream);
 }
@@ -1535,6 +1546,7 @@ int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout
     }
     // A column-major result leaves the kernels in that layout; a bias is added to rows first.
     const bool y_col = y_layout != TLLM_ROW_MAJOR && rows > 1;
+    if (rows == 1) x_layout = TLLM_ROW_MAJOR;
     const int x_ld = x_layout == TLLM_ROW_MAJOR ? L.inners : rows;
     void* out = w->d_y;
     if (!bias) {

@@ -190,3 +190,30 @@ def test_cost_model_dispatch():
             assert n[3] == 1 and list(n[:3]) == [kernel == "bits", kernel == "mma", kernel == "nibble"], (K, N, s, M, kernel, n)
             assert torch.equal(Y.double(), X.double() @ Wd)
         pw.close()
+
+
+# Default setting, activations that the register decoder cannot read by asynchronous copies:
+# each of these was slower there by a factor of 1.5 to 12.
+@pytest.mark.parametrize("K, N, s, dtype, calls", [
+    (2048, 2048, 0.5, torch.float16, {("columns", 2): "bits", ("columns", 16): "mma", ("offset", 8): "bits", ("offset", 64): "mma"}),
+    (2048, 8192, 0.7, torch.float32, {("columns", 1): "bits", ("columns", 8): "mma", ("offset", 16): "mma", ("rows", 4): "bits"}),
+    (2048, 8192, 0.7, torch.int8, {("columns", 2): "gather", ("rows", 2): "bits", ("columns", 16): "mma"})])
+def test_cost_model_by_layout(K, N, s, dtype, calls):
+    L = _lib.lib()
+    L.tllm_set_mma_min_rows(-1)
+    rng = np.random.default_rng(16)
+    w = random_ternary(rng, K, N, s)
+    pw = PackedWeight.from_dense(w)
+    Wd = torch.tensor(w, device=dev()).double()
+    for (layout, M), kernel in calls.items():
+        X = torch.tensor(rng.integers(-4, 5, size=(M, K)), device=dev()).to(dtype)
+        x = X.t().contiguous() if layout == "columns" else X
+        if layout == "offset":                                        # rows that start on no multiple of 16 bytes
+            x = torch.empty(M * K + 1, dtype=dtype, device=dev())[1:].view(M, K).copy_(X)
+        counts = lambda: np.array([L.tllm_bits_launch_count(), L.tllm_mma_launch_count(), L.tllm_nibble_launch_count()])
+        n0 = counts()
+        Y = pw.matmul(x, col_major=layout == "columns", out=torch.empty((M, N), dtype=torch.int32 if dtype == torch.int8 else torch.float32, device=dev()))
+        n = counts() - n0
+        assert list(n > 0) == [kernel == "bits", kernel == "mma", kernel == "nibble"], (layout, M, kernel, n)
+        assert torch.equal(Y.double(), X.double() @ Wd)
+    pw.close()
