@@ -572,11 +572,14 @@ int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld
 int nb_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? NB_ROWS / 8 : NB_ROWS / 4; }
 
 // true when the decode tensor-core kernel can and should take this call
+bool nb_fits(const tllm_weight* w, int x_dtype, int x_layout) {
+    return w->d_nib && (x_dtype == TLLM_F16 || x_dtype == TLLM_BF16 || x_dtype == TLLM_F32) && x_layout == TLLM_ROW_MAJOR && mm_min_rows() != 0 &&
+           g_nb_max_rows.load(std::memory_order_relaxed) != 0;
+}
+// pinned, or ahead of the gather kernel
 bool nb_usable(const tllm_weight* w, int x_dtype, int x_layout, int rows) {
-    if (!w->d_nib || (x_dtype != TLLM_F16 && x_dtype != TLLM_BF16 && x_dtype != TLLM_F32) || x_layout != TLLM_ROW_MAJOR) return false;
-    if (mm_min_rows() == 0) return false;
+    if (!nb_fits(w, x_dtype, x_layout)) return false;
     const int thr = g_nb_max_rows.load(std::memory_order_relaxed);
-    if (thr == 0) return false;
     if (thr > 0) return rows <= thr;
     const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
     return nibble_model_us(entries, rows, nb_rows_per_launch(x_dtype)) < gather_model_us(w->lay.nnz, rows);
@@ -840,11 +843,17 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
             1.35 * gather < std::min(bt_model_us(inners, columns, sms, x_dtype, access, rows), mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, rows)))
             return KERNEL_GATHER;
         // A weight so wide that a block of the register decoder makes several passes: four bits an entry, which no thread touches, are read
-        // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4).  The model is 8 % high there.  More than
-        // one launch's rows (4) have to start on 16 bytes: its planes are made from X element by element else (28672 x 8192, eight rows:
-        // 82 us, the batched kernel 43).
+        // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4; one or two rows of fp32 28.4 and 32.7
+        // against 47 and 49, with the same error).  The model is 8 % high there.  More than one launch's rows (4, fp32 2) have to start on 16
+        // bytes: its planes are made from X element by element else (28672 x 8192, eight rows: 82 us, the batched kernel 43).  Of fp32 these
+        // compete with the batched kernel (four rows 34 us against 46, eight 40), over a K that is not too long: 28672 x 8192 57 against 46.
         const int per = nb_rows_per_launch(x_dtype);
-        if (nb && rows <= 8 && x_dtype != TLLM_F32 && (rows <= per || access == BITS_ROWS16) && 0.92 * nibble_model_us(entries, rows, per) < bits) return KERNEL_NIBBLE;
+        if (nb_fits(w, x_dtype, x_layout) && rows <= 8 && (rows <= per || access == BITS_ROWS16)) {
+            const double nibble = nibble_model_us(entries, rows, per);
+            if (x_dtype == TLLM_F32 && rows > per) {
+                if (inners <= 16384 && nibble < std::min(bits, mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, rows))) return KERNEL_NIBBLE;
+            } else if ((nb || x_dtype == TLLM_F32) && 0.92 * nibble < bits) return KERNEL_NIBBLE;
+        }
         return bits_prefer_registers(inners, columns, sms, w->device, mm_direct(inners, X, x_dtype, x_layout, x_ld), x_dtype, access, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
     return nb ? KERNEL_NIBBLE : KERNEL_GATHER;           // no bit tiles, or the kernels on them switched off

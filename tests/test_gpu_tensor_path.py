@@ -192,12 +192,13 @@ def test_cost_model_dispatch():
         pw.close()
 
 
-# Default setting, activations that the register decoder cannot read by asynchronous copies:
+# Default setting, activations that the register decoder cannot read by asynchronous copies, or (fp32, wide weight) reads three times:
 # each of these was slower there by a factor of 1.5 to 12.
 @pytest.mark.parametrize("K, N, s, dtype, calls", [
     (2048, 2048, 0.5, torch.float16, {("columns", 2): "bits", ("columns", 16): "mma", ("offset", 8): "bits", ("offset", 64): "mma"}),
     (2048, 8192, 0.7, torch.float32, {("columns", 1): "bits", ("columns", 8): "mma", ("offset", 16): "mma", ("rows", 4): "bits"}),
-    (2048, 8192, 0.7, torch.int8, {("columns", 2): "gather", ("rows", 2): "bits", ("columns", 16): "mma"})])
+    (2048, 8192, 0.7, torch.int8, {("columns", 2): "gather", ("rows", 2): "bits", ("columns", 16): "mma"}),
+    (8192, 28672, 0.5, torch.float32, {("rows", 1): "nibble", ("offset", 1): "nibble", ("rows", 2): "nibble", ("rows", 5): "nibble", ("offset", 5): "mma", ("columns", 1): "nibble", ("rows", 64): "mma"})])
 def test_cost_model_by_layout(K, N, s, dtype, calls):
     L = _lib.lib()
     L.tllm_set_mma_min_rows(-1)
