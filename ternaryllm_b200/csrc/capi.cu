@@ -318,30 +318,33 @@ struct Workspace {
     }
 };
 
-// How a product of `rows` rows (in `planes` planes) is cut: row tiles of Nt rows each, whole tiles or equal ranges of units, chosen
-// by an estimate in SM clocks.  A slice of 64 rows of W is four MMAs of 128 x (planes * Nt) x 16, 2.5 clocks a column (measured)
-// and never less than the 255 of their issue.  A tile's epilogue is hidden behind the next one except at the end, or where
-// there is no room for two sets of accumulators.  In a tile that `parts` blocks share the last one to arrive reads the other
-// parts, a round trip to L2 for every sixteen rows of each, 3000 clocks in all at least.
-// The first unit of activations takes 12 clocks a row to arrive.
-// A cluster of C blocks per tile: every block's units, then what goes to the other blocks and the adding-up of its own share, 2000
-// clocks at least.  A launch that holds more than half of the SMs keeps the next one's blocks, one to an SM, from starting up
-// beside it: 3000 clocks (2048 x 8192, 20 rows: 8.3 us as 64 blocks of 32 rows, 9.2 as 128 of 16); 1000 behind the kernel that makes
-// planes, which starts in between.
+// How a product of `rows` rows (in `planes` planes) is cut: row tiles of Nt rows each, and whole tiles, equal ranges of units, or a
+// cluster per tile; by one block or by a pair of blocks.  Chosen by an estimate in SM clocks, fitted to 1400 plans of 9 weights from
+// 512 x 512 to 5120 x 15360 and 20 to 2048 rows (6 % off in the mean, and the plan it picks 1.3 % slower than the best).
+// A unit is eight MMAs of 128 x (planes * Nt) x 16.  With a pair they take little more than their own time, 4.3 clocks a column.  A block by
+// itself takes as long up to 256 columns as its shared memory needs to write and read the activations: 600 clocks and 2.2 a column.
+// Neither takes less than the 750 of decoding a unit.  A tile's epilogue is hidden behind the next one where that takes longer.
+// In a tile that `parts` blocks share the last one to arrive reads the other parts, a round trip to L2 for every sixteen rows of each.
+// A cluster of C blocks per tile: every block's units, then what goes to the other blocks and the adding-up of its own share.
+// A launch that holds more than half of the SMs keeps the next one's blocks, one to an SM, from starting up beside it.
 struct MmPlan {
     int Nt, m_tiles, split, cluster;
+    int cg;                  // blocks that share a tile's MMAs: 1, or 2 (a pair: 256 columns of W, half of the activations in each block)
     double clocks;
 };
-constexpr int MM_SMEM = 227 * 1024, MM_RAW_UNITS = 4;
-// shared memory that is left for units of B
-int mm_b_bytes(int nt, int cluster) {
+constexpr int MM_SMEM = 227 * 1024;
+// shared memory beside the units of B: bit tiles, barriers, a cluster's parts, the sum of the legs of three planes
+int mm_other_bytes(int nt, int planes, int cluster) {
     const int parts = cluster > 1 ? cluster * ((nt / 16 + cluster - 1) / cluster) * 8192 : 0;
-    return std::min(192 * 1024, MM_SMEM - 1024 - 512 - MM_RAW_UNITS * MM_UNIT_BYTES - parts);
+    return 1024 + 512 + MM_RAW_UNITS * MM_UNIT_BYTES + parts + (planes > 1 ? nt * 512 : 0);
 }
-// clusters of `cluster` blocks that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a GPU is made of
-int mm_clusters(int cluster, int sms, int device) {
+// clusters of `cluster` blocks (cg = 2: pairs) that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a
+// GPU is made of
+int mm_clusters(int cluster, int cg, int sms, int device) {
     static std::atomic<int> known[64][9];
-    int n = device < 64 ? known[device][cluster].load(std::memory_order_relaxed) : 0;
+    const int slot = cg == 2 ? 1 : cluster;
+    auto kern = cg == 2 ? mma_spmm_kernel<2> : mma_spmm_kernel<1>;
+    int n = device < 64 ? known[device][slot].load(std::memory_order_relaxed) : 0;
     if (n == 0) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(sms / cluster * cluster));
@@ -351,37 +354,39 @@ int mm_clusters(int cluster, int sms, int device) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned)cluster, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
         cfg.attrs = at, cfg.numAttrs = 1;
-        if (cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, mma_spmm_kernel, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             return 0;                                // no clusters for this call; the next one asks again
         }
-        if (device < 64) known[device][cluster].store(n, std::memory_order_relaxed);
+        if (device < 64) known[device][slot].store(n, std::memory_order_relaxed);
     }
     return n;
 }
 int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
 MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
-    MmPlan best{0, 0, 0, 1, 0};
-    const int kbu = (kb + MM_UK - 1) / MM_UK;
+    MmPlan best{0, 0, 0, 1, 1, 0};
+    const int kbu = (kb + MM_UK - 1) / MM_UK, pairs = n_tiles > 1 ? mm_clusters(2, 2, sms, device) : 0;
+    const bool one = planes == 1;
+    const auto take = [&](int nt, int mt, int split, int c, int cg, double clocks) {
+        if (best.Nt == 0 || clocks < best.clocks) best = MmPlan{nt, mt, split, c, cg, clocks};
+    };
     for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
-        const int mt = (rows + nt - 1) / nt;
+        const int mt = (rows + nt - 1) / nt, cols = planes * nt, sixteens = nt / 16;
         if (mt > MM_MAX_M_TILES) continue;
-        const double tiles = (double)n_tiles * mt, units = tiles * kbu;
-        const double slice = std::max(255.0, 2.5 * planes * nt), epilogue = nt / 16 * 350.0, fill = 12.0 * planes * nt;
-        const bool two = mm_acc_sets(planes, nt) == 2;
-        // legs of fp32 sums: where there is one set of accumulators the MMAs wait while the epilogue reads it
-        const auto legs = [&](double u) { return two || planes == 1 ? 0.0 : (std::ceil(u / MM_LEG) - 1) * (500 + nt / 16 * 150.0); };
-        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (planes == 1 ? 3000.0 : 1000.0) : 0.0; };
-        const double whole = crowd(tiles) + std::ceil(tiles / sms) * (kb * slice + legs(kbu) + (two ? 0.0 : epilogue)) + (two ? epilogue : 0.0);
-        const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu, blocks / tiles + 1.0);
-        const double split = crowd(blocks) + std::ceil(units / blocks) * MM_UK * slice + legs(std::min(units / blocks, (double)kbu)) + 3000.0 + 3 * epilogue + nt / 16 * 1000.0 * (parts - 1);
-        if (best.Nt == 0 || whole + fill < best.clocks) best = MmPlan{nt, mt, 0, 1, whole + fill};
-        if (split + fill < best.clocks) best = MmPlan{nt, mt, 1, 1, split + fill};
-        for (int c = 2; c <= 8 && c <= kbu; c *= 2) {
-            if (mm_b_bytes(nt, c) < 2 * planes * nt * 128 * MM_UK || mm_clusters(c, sms, device) < tiles) continue;
-            const double shared = (kbu + c - 1) / c * MM_UK * slice + legs((kbu + c - 1) / c) + 2000.0 + nt / 16 * 100.0 + (nt / 16 + c - 1) / c * 350.0 + crowd(tiles * c);
-            if (shared + fill < best.clocks) best = MmPlan{nt, mt, 2, c, shared + fill};
+        const double piece = one ? 780.0 : 1700.0, epilogue = sixteens * piece, legs = one ? 0.0 : ((kbu + MM_LEG - 1) / MM_LEG - 1) * sixteens * 300.0;
+        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (one ? 2600.0 : 4000.0) : 0.0; };
+        for (int cg = 1; cg <= 2; ++cg) {
+            const double groups = cg == 1 ? sms : pairs, tiles = (double)((n_tiles + cg - 1) / cg) * mt, units = tiles * kbu;
+            if (groups <= 0 || nt % (16 * cg) != 0) continue;
+            const double unit = std::max(750.0, cg == 1 ? 600.0 + 2.2 * cols : 130.0 + 4.3 * cols), extra = cg == 1 ? 0.0 : 1400.0;
+            take(nt, mt, 0, 1, cg, extra + (std::ceil(tiles / groups) - 1) * std::max(kbu * unit, epilogue + legs) + kbu * unit + epilogue + crowd(tiles * cg));
+            const double blocks = std::min(units, groups), parts = std::min((double)kbu, blocks / tiles + 1.0);
+            take(nt, mt, 1, 1, cg, extra + std::ceil(units / blocks) * unit + 3600.0 + 2.8 * epilogue + sixteens * 580.0 * (parts - 1) + crowd(blocks * cg));
+            for (int c = 2; cg == 1 && c <= 8 && c <= kbu; c *= 2) {
+                if (MM_SMEM - mm_other_bytes(nt, planes, c) < 2 * cols * 128 * MM_UK || mm_clusters(c, 1, sms, device) < tiles) continue;
+                take(nt, mt, 2, c, 1, (kbu + c - 1) / c * unit + 3600.0 + sixteens * 400.0 + (sixteens + c - 1) / c * piece + crowd(tiles * c));
+            }
         }
         if (nt >= rows) break;
     }
@@ -474,33 +479,33 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
         if (wide && o.col_major && (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0) p.out = o.dtype == TLLM_F32 ? MM_OUT_F32_COL4 : MM_OUT_I32_COL4;
         if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && w.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
     }
-    // rings: four units of bit tiles, and as many of B as there is room for (three at 128 columns of D, two at 192 or in a cluster)
-    p.R = MM_RAW_UNITS;
-    const int b_unit = x.planes * p.Nt * 128 * MM_UK;
-    p.SB = std::min(MM_MAX_STAGES, mm_b_bytes(p.Nt, p.cluster) / b_unit);
+    const int cg = plan.cg, b_unit = x.planes * p.Nt / cg * 128 * MM_UK, other = mm_other_bytes(p.Nt, x.planes, p.cluster);
+    p.SB = std::min(MM_MAX_STAGES, (MM_SMEM - other) / b_unit);
     p.mul4 = 4, p.mul16 = 16;
     const uint32_t fmt = x.bf16 ? 1u : 0u;
     // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B formats (bits 7-9, 10-12), both K-major,
     // N / 8 in bits 17-22, M / 16 in bits 24-28
-    p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(x.planes * p.Nt >> 3) << 17) | ((uint32_t)(MM_TILE_N >> 4) << 24);
+    p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(x.planes * p.Nt >> 3) << 17) | ((uint32_t)(cg * MM_TILE_N >> 4) << 24);
     p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
     p.finite = x.finite;
     p.bits = (const uint32_t*)w.bits, p.X = (const unsigned short*)x.base, p.bf16 = x.bf16;
     p.ld_x = (long long)(x.pitch / 2), p.plane_x = x.plane_rows * p.ld_x;
 
     CUtensorMap map;
-    int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, rows, x.planes, x.pitch, (size_t)x.plane_rows * x.pitch, p.Nt);
+    int rc = encode_rows_map(&map, x.base, x.bf16, w.inners, rows, x.planes, x.pitch, (size_t)x.plane_rows * x.pitch, p.Nt / cg);
     if (rc) return rc;
-    const size_t smem = 1024 + (size_t)p.SB * b_unit + (size_t)p.R * MM_UNIT_BYTES + 512 + (p.split == 2 ? (size_t)p.cluster * ((p.Nt / 16 + p.cluster - 1) / p.cluster) * 8192 : 0);
+    const size_t smem = (size_t)other + (size_t)p.SB * b_unit;
     if (smem > MM_SMEM || p.SB < 2) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
-    static std::once_flag once[64];
+    auto kern = cg == 2 ? mma_spmm_kernel<2> : mma_spmm_kernel<1>;
+    static std::once_flag once[2][64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[w.device & 63], [&] { err = cudaFuncSetAttribute(mma_spmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
+    std::call_once(once[cg - 1][w.device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
     CU_TRY(err);
     // never more blocks than items: the hand-over between the blocks that share a tile counts on every block in a
     // tile's range of owners holding at least one unit of it
-    const long long items = (long long)p.n_tiles * p.m_tiles * (p.split == 1 ? p.KBU : p.cluster);
-    const int grid = (int)(items < w.sms ? items : w.sms);
+    const long long items = (long long)((p.n_tiles + cg - 1) / cg) * p.m_tiles * (p.split == 1 ? p.KBU : p.cluster);
+    const long long most = cg == 2 ? mm_clusters(2, 2, w.sms, w.device) : w.sms;
+    const int grid = (int)std::min(items, most) * cg;
     Workspace ws;
     if ((p.Nt <= MM_OWN_NT && w.partial) || p.split != 1) p.partial = w.partial;
     else {
@@ -516,14 +521,14 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     cudaLaunchAttribute at[2] = {};
     int n_at = 0;
     if (!w.lists) at[n_at++] = pdl_attribute();
-    if (p.split == 2) {
+    if (p.split == 2 || cg == 2) {
         at[n_at].id = cudaLaunchAttributeClusterDimension;
-        at[n_at].val.clusterDim.x = (unsigned)p.cluster, at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
+        at[n_at].val.clusterDim.x = (unsigned)(cg == 2 ? 2 : p.cluster), at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
         ++n_at;
     }
     cfg.attrs = at;
     cfg.numAttrs = (unsigned)n_at;
-    CU_TRY(cudaLaunchKernelEx(&cfg, mma_spmm_kernel, map, *w.map, p));
+    CU_TRY(cudaLaunchKernelEx(&cfg, kern, map, *w.map, p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
@@ -801,8 +806,8 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
     return TLLM_OK;
 }
 
-// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 2.4 us of start-up, the plan's
-// clocks at 1.8 GHz, and 5 us for planes that have to be made first.
+// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 3.1 us of start-up, or 4.9 behind the kernel
+// that makes planes, and the plan's clocks at 1.85 GHz.
 double bt_model_us(int inners, int columns, int sms, int x_dtype, BitsAccess access, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
@@ -813,7 +818,7 @@ double mm_tiles_model_us(int inners, int columns, int sms, int device, bool dire
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += 2.4 + mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).clocks / 1800.0 + (direct ? 0.0 : 5.0);
+        t += mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).clocks / 1850.0 + (direct ? 3.1 : 4.9);
     return t;
 }
 // which of the two: true = decode in registers

@@ -17,20 +17,25 @@
 // of 2048 x 2048); D's planes are added in the epilogue, the small ones first.  (The tensor core truncates its sums: with the
 // planes in one accumulator every step would cut bits, 1e-5 of the result at K = 4096 against 1e-7.)
 //
-// One persistent block per SM, twenty-three warps:
-//   warp 0        streams this block's range of bit tiles into a shared-memory ring (TMA)
-//   warp 1        owns tensor memory and issues tcgen05.mma (one lane)
+// One persistent block per SM, alone or as one of a pair, twenty-three warps:
+//   warp 0        streams this block's range of bit tiles into a shared-memory ring (TMA, one thread)
+//   warp 1        owns tensor memory and issues tcgen05.mma (one thread; a pair's second block has none)
 //   warps 2..5    epilogue: tensor memory -> registers -> Y (or partial sums)
-//   warp 6        loads the activation slices by TMA
-//   warps 7..22   decoders: bit tile -> tensor memory, one slice of 32 columns per warp and unit (a warp can only write the 32
+//   warp 6        loads the activation slices by TMA (one thread)
+//   warps 7..22   decoders: bit tile -> tensor memory, one slice of 32 columns per warp and second unit (a warp can only write the 32
 //                 lanes of tensor memory that its number modulo 4 selects)
-// A unit is four consecutive slices of K: the issuer's waits, commits and loop cost 500 clocks whatever it issues in between, and an
-// MMA 40 to issue, so that sixteen MMAs of 128 x 128 x 16 (1270 clocks) hide it and eight do not (measured at 5120 x 15360, 2048
-// rows: 285 us with two slices per unit, 183 with the MMAs alone).  A has a ring of two units (256 columns of tensor memory;
-// the accumulators have the other 256: two of them where they fit, so that the epilogue of one tile runs beside the next),
-// B one of units.
+// A unit is two consecutive slices of K.  What bounds a launch of many tiles is that the tensor core is never without an MMA:
+//   * one thread issues (13 clocks an MMA), and it finds the next unit's operands ready: A has a ring of two or four units in tensor memory
+//     beside two sets of accumulators, so that the sums of one tile (fp32: of one leg) leave while the next one's MMAs run; the decoders have
+//     the values in registers when a place is free;
+//   * a pair of blocks shares the MMAs (tcgen05 cta_group::2): 256 columns of W, 128 in each block's tensor memory, by Nt activation
+//     rows, half of them in each block's shared memory.  For a block by itself writing and reading the activations takes all of the
+//     128 bytes that its shared memory moves per clock.
+// An MMA of N columns then takes 0.52 N + 13 to 25 clocks, the latter while decoders write to tensor memory.  Measured against a unit of four
+// slices, one block per tile, a warp that elects a lane per MMA and one set of accumulators for three planes: 2048 rows of 5120 x 15360
+// bf16 235 us (276; both at the power cap), 256 rows of fp32 2048 x 16384 44 us (56), 2048 x 8192 28 us (36).
 // Work is either whole output tiles or, where those would leave SMs idle, the flattened list of (output tile, unit) pairs
-// cut into equal contiguous ranges, one per block.  Tiles that straddle two or more blocks are summed in block order by the
+// cut into equal contiguous ranges, one per block or pair.  Tiles that straddle two or more blocks are summed in block order by the
 // last block to arrive, which makes the result independent of scheduling; a block does its two shared tiles first, so that
 // this adding-up hides behind the tiles it has to itself.
 // With few tiles a third way: a cluster of two, four or eight blocks cuts the units of one tile.  Each block sends its sums of the rows
@@ -50,17 +55,16 @@
 namespace tllm {
 
 #define MM_TILE_N 128                 // output columns per tile  (the MMA's M)
-#define MM_TILE_K 64                  // rows of W per slice      (four MMAs of K = 16); a unit is four slices
-#define MM_UNIT_BYTES 8192            // bit tiles of one unit: eight groups of sixteen columns, 1024 bytes each
-#define MM_UK 4
-#define MM_A_UNITS 2                  // ring of expanded units in tensor memory: 128 columns each, behind 256 columns of accumulators
-#define MM_A_COL 256
+#define MM_TILE_K 64                  // rows of W per slice      (four MMAs of K = 16); a unit is two slices
+#define MM_UNIT_BYTES 4096            // bit tiles of one unit: eight groups of sixteen columns, 512 bytes each
+#define MM_UK 2
+#define MM_RAW_UNITS 8                // ring of bit tiles: a power of two, at most MM_MAX_STAGES
 #define MM_MAX_STAGES 8
 // Units of a leg.  The tensor core cuts bits off its running sum at every MMA, always toward zero, so that a sum of many MMAs comes out too
 // small: by 3.6e-7 of the result for fp32 activations of the spread that a gated MLP makes and 432 MMAs, where fp32 additions
 // rounded to nearest are off by 7e-8.  The sums of fp32 activations therefore leave the accumulators after every 64 MMAs and
 // are added up in fp32: 8e-8.
-#define MM_LEG 4
+#define MM_LEG 8
 #define MM_THREADS (23 * 32)
 #define MM_MAX_COLS 192               // columns of D of a tile = planes * Nt, Nt (activation rows) a multiple of sixteen
 #define MM_OWN_NT 64                  // a handle's own hand-over scratch is for tiles of up to this many rows
@@ -84,7 +88,7 @@ struct MmParams {
     int* status;
     int M, K, N;
     int KB;                   // ceil(K / 64): slices
-    int KBU;                  // ceil(KB / 4): units per tile
+    int KBU;                  // ceil(KB / 2): units per tile
     int n_tiles, m_tiles;
     int Nt;                   // activation rows per tile; planes * Nt is the MMA's N
     int split;                // 0: whole tiles; 1: equal unit ranges, tiles may be shared; 2: a cluster per tile
@@ -94,7 +98,7 @@ struct MmParams {
     int epilogue, y_ld;       // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
     long long y_step_n, y_step_m;   // elements from column to column and from row to row (epilogue 0)
     long long plane_y;        // MM_OUT_PLANES: elements from plane to plane
-    int SB, R;                // ring lengths: units of B, units of bit tiles
+    int SB;                   // ring length: units of B
     int leg;                  // units that are summed in the tensor core before the sum goes on in fp32 (MM_LEG)
     uint32_t idesc;           // tcgen05 instruction descriptor
     uint32_t mul4, mul16;     // 4 and 16
@@ -112,24 +116,39 @@ struct MmParams {
 // ---- tcgen05 / TMA wrappers ------------------------------------------------------------------------------
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// CG: blocks that the tensor core works for at a time, 1 or 2 (a pair); a warp of each of them allocates and releases
+template <int CG = 1>
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (CG == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
 }
+template <int CG = 1>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+    if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem], issued by one thread; A: lane = row, 32-bit column c = values 2c, 2c + 1 of K.  B is given by the
 // low word of its shared-memory descriptor (start address >> 4; the upper word -- K-major, 128-byte swizzle, eight-row
-// groups 1024 bytes apart, version 1 -- is a constant).
+// groups 1024 bytes apart, version 1 -- is a constant).  CG = 2: D and A at the same columns of both blocks' tensor memory, 128 rows each;
+// B's rows half in this block's shared memory and half at the same place of the other's.
+template <int CG>
 __device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "mov.b64 db, {%2, %5};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(d),
-        "r"(a), "r"(b_lo | (1u << 16)), "r"(idesc), "r"(accumulate), "r"(0x40004040u)
-        : "memory");
+#define MM_UMMA(group)                                                                   \
+    asm volatile(                                                                        \
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"                                      \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                      \
+        "mov.b64 db, {%2, %5};\n\t"                                                      \
+        "tcgen05.mma.cta_group::" group ".kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(d), \
+        "r"(a), "r"(b_lo | (1u << 16)), "r"(idesc), "r"(accumulate), "r"(0x40004040u)     \
+        : "memory")
+    if (CG == 1) MM_UMMA("1");
+    else MM_UMMA("2");
+#undef MM_UMMA
 }
 // 32 columns of the calling warp's 32 lanes
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
@@ -142,9 +161,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// the barrier receives one arrival when every MMA issued so far by this thread has completed
+// the barrier (CG = 2: that of both blocks) receives one arrival when every MMA issued so far by this thread has completed
+template <int CG = 1>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    if (CG == 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3)
+                     : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
@@ -155,55 +178,66 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "f"(v[0]), "f"(v[1]),
-        "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
-        : "memory");
-}
-// sixteen columns of the calling warp's lanes at each of two places, one wait for both; added up
-__device__ __forceinline__ void tmem_sum16(uint32_t at, uint32_t at2, float (&f)[16]) {
-    uint32_t v[16], u[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
-          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-        : "r"(at), "r"(at2)
-        : "memory");
-#pragma unroll
-    for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]) + __uint_as_float(u[t]);
-}
-// sixteen columns of D (rows of X) of this lane's column of W, the planes added up, the small ones first
+// sixteen columns of D (rows of X) of this lane's column of W, the planes (nt columns apart) added up, the small ones first
 __device__ __forceinline__ void mm_load16(uint32_t at, int nt, int planes, float (&f)[16]) {
-    uint32_t v[16];
     if (planes == 1) {
+        uint32_t v[16];
         tmem_ld16(at, v);
 #pragma unroll
         for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]);
     } else {
-        tmem_sum16(at + (uint32_t)nt, at + (uint32_t)(2 * nt), f);
-        tmem_ld16(at, v);
+        float g[16], h[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%48];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%49];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%50];\n\t"
+            "tcgen05.wait::ld.sync.aligned;"
+            : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]), "=f"(f[8]), "=f"(f[9]), "=f"(f[10]), "=f"(f[11]),
+              "=f"(f[12]), "=f"(f[13]), "=f"(f[14]), "=f"(f[15]), "=f"(g[0]), "=f"(g[1]), "=f"(g[2]), "=f"(g[3]), "=f"(g[4]), "=f"(g[5]), "=f"(g[6]), "=f"(g[7]),
+              "=f"(g[8]), "=f"(g[9]), "=f"(g[10]), "=f"(g[11]), "=f"(g[12]), "=f"(g[13]), "=f"(g[14]), "=f"(g[15]), "=f"(h[0]), "=f"(h[1]), "=f"(h[2]), "=f"(h[3]),
+              "=f"(h[4]), "=f"(h[5]), "=f"(h[6]), "=f"(h[7]), "=f"(h[8]), "=f"(h[9]), "=f"(h[10]), "=f"(h[11]), "=f"(h[12]), "=f"(h[13]), "=f"(h[14]), "=f"(h[15])
+            : "r"(at), "r"(at + (uint32_t)nt), "r"(at + (uint32_t)(2 * nt))
+            : "memory");
 #pragma unroll
-        for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]) + f[t];
+        for (int t = 0; t < 16; ++t) f[t] += g[t] + h[t];
     }
 }
-__device__ __forceinline__ void mm_add16(uint32_t at, float (&f)[16]) {
-    uint32_t v[16];
-    tmem_ld16(at, v);
+// the sum of the legs so far: sixteen values of this thread, 512 bytes apart in shared memory
+__device__ __forceinline__ void mm_add_run(uint32_t at, float (&f)[16]) {
 #pragma unroll
-    for (int t = 0; t < 16; ++t) f[t] += __uint_as_float(v[t]);
+    for (int t = 0; t < 16; ++t) {
+        float r;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(r) : "r"(at + (uint32_t)t * 512u) : "memory");
+        f[t] += r;
+    }
 }
-// 2-D tiled TMA load into this block's own shared memory: coordinates are (element along K, activation row)
+__device__ __forceinline__ void mm_store_run(uint32_t at, const float (&f)[16]) {
+#pragma unroll
+    for (int t = 0; t < 16; ++t) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)t * 512u), "f"(f[t]) : "memory");
+}
+// 2-D tiled TMA load into this block's own shared memory: coordinates are (element along K, activation row).  CG = 2: `bar` may be
+// the other block's of the pair.
+template <int CG = 1>
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    if (CG == 2) {
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                     "l"(map), "r"(bar), "r"(c0), "r"(c1)
+                     : "memory");
+        return;
+    }
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
                  "l"(map), "r"(bar), "r"(c0), "r"(c1)
                  : "memory");
 }
 // coordinates (element along K, activation row, plane)
+template <int CG = 1>
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    if (CG == 2) {
+        asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                     "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+                     : "memory");
+        return;
+    }
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
                  "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
                  : "memory");
@@ -257,10 +291,14 @@ __device__ __forceinline__ bool bounded_spin(uint32_t bar, uint32_t parity, vola
     }
 }
 
-// waiting roles are parked (bounded_wait): spinning ones took issue slots from the epilogue
+// waiting roles are parked (bounded_wait): spinning ones took issue slots from the epilogue; only the thread that issues MMAs spins
 #define MM_WAIT(bar, par)                             \
     do {                                                    \
         if (!bounded_wait((bar), (par), abort_flag)) goto done; \
+    } while (0)
+#define MM_SPIN(bar, par)                                       \
+    do {                                                        \
+        if (!bounded_spin((bar), (par), abort_flag)) goto done; \
     } while (0)
 // ring position and the parity of its current round
 #define MM_ADVANCE(idx, ph, n) \
@@ -296,6 +334,9 @@ __device__ __forceinline__ uint32_t mm_peer(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mm_st_peer(uint32_t addr, float a, float b, float c, float d) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
+// An arrival at the barrier of a pair's first block: what it stands for is tensor memory, which the tcgen05 waits and fences before it
+// have taken care of.  (With release.cluster it waited for the thread's other writes too: 2500 clocks.)
+__device__ __forceinline__ void mm_arrive_first(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mm_peer(bar, 0u)) : "memory"); }
 __device__ __forceinline__ void mm_arrive_peer(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 // column (of the 32 of a quarter tile) that lane `lane` of tensor memory's quarter holds
@@ -491,17 +532,21 @@ __device__ __forceinline__ void mm_with_out(const MmParams& p, F f) {
     }
 }
 
-__host__ __device__ __forceinline__ uint32_t mm_acc_sets(int planes, int nt) { return (2 * planes + (planes > 1 ? 1 : 0)) * nt <= MM_A_COL ? 2u : 1u; }
+// Tensor memory: two sets of accumulators, and behind them the ring of expanded units, 64 columns each: four, or two beside
+// accumulators of more than 128 columns.
+__host__ __device__ __forceinline__ uint32_t mm_a_units_log(uint32_t acc_cols) { return acc_cols <= 128 ? 2u : 1u; }
 
+template <int CG>
 __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap,
                                                                  const __grid_constant__ MmParams p) {
     extern __shared__ unsigned char mm_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // ---- this block's unit range -----------------------------------------------------------------------
-    const int G = (int)gridDim.x, cta = (int)blockIdx.x, KBU = p.KBU, KB = p.KB, tiles = p.n_tiles * p.m_tiles;
+    // ---- the unit range of this block or pair ------------------------------------------------------------
+    const int G = (int)gridDim.x / CG, cta = (int)blockIdx.x / CG, member = CG == 2 ? (int)blockIdx.x & 1 : 0;
+    const int KBU = p.KBU, KB = p.KB, tiles = (p.n_tiles + CG - 1) / CG * p.m_tiles;
     const long long total = (long long)tiles * KBU;
-    const bool clustered = p.split == 2;
+    const bool clustered = CG == 1 && p.split == 2;
     const int C = clustered ? p.cluster : 1, rank = clustered ? cta % C : 0;
     int u0, u1;
     if (clustered) u0 = cta / C * KBU + KBU * rank / C, u1 = cta / C * KBU + KBU * (rank + 1) / C;
@@ -513,11 +558,17 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     // ---- shared memory ---------------------------------------------------------------------------------
     const uint32_t raw0 = smem_u32(mm_smem);
     const uint32_t base = (raw0 + 1023u) & ~1023u;                 // swizzled tiles need 1024-byte alignment
-    const uint32_t SB = (uint32_t)p.SB, R = (uint32_t)p.R;
+    const uint32_t SB = (uint32_t)p.SB, R = MM_RAW_UNITS;
     const int Nt = p.Nt;
-    const uint32_t acc_cols = (uint32_t)(p.P * Nt), b_slice = acc_cols * 128u, b_unit = MM_UK * b_slice;
+    const uint32_t acc_cols = (uint32_t)(p.P * Nt), b_slice = acc_cols / CG * 128u, b_unit = MM_UK * b_slice;
     const uint32_t b_base = base, r_base = b_base + SB * b_unit;
     const uint32_t bar_base = r_base + R * MM_UNIT_BYTES, part_base = bar_base + 512u;      // part_base: the cluster's parts, [block][rows / 16][4][128] x 16 bytes
+    const uint32_t run_base = part_base + (clustered ? (uint32_t)(C * ((Nt / 16 + C - 1) / C)) * 8192u : 0u);      // fp32: the sum of the legs so far, [row][128]
+    const uint32_t a_log = mm_a_units_log(acc_cols), a_mask = (1u << a_log) - 1u;
+    // Where the ring of expanded units has two places, each of their slices has barriers of its own, so that it is filled again while the
+    // other three are multiplied (5120 x 15360, 2048 rows in tiles of 192: 198 us, 227 with one pair of barriers a unit); with four places
+    // there is time enough, and fewer barriers are faster (2048 x 8192, 32 rows: 8.8 us against 9.6).
+    const uint32_t fine = a_log == 1u ? 1u : 0u;
     volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 56);   // [0] tensor-memory address, [1] abort
     volatile int* abort_flag = flags + 1;
 #define A_FULL(s) (bar_base + 8u * (uint32_t)(s))
@@ -532,16 +583,16 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 
     if (tid == 0) {
         for (int s = 0; s < MM_MAX_STAGES; ++s) {
-            mbar_init(A_FULL(s), 16);      // the decoder warps
+            mbar_init(A_FULL(s), (fine ? 4 : 8) * CG);      // the decoder warps of a slice or unit (of a pair: at the first block)
             mbar_init(A_EMPTY(s), 1);      // tcgen05.commit
             mbar_init(B_FULL(s), 1);       // the TMA thread's expect_tx arrival
             mbar_init(B_EMPTY(s), 1);      // tcgen05.commit
             mbar_init(RAW_FULL(s), 1);
-            mbar_init(RAW_EMPTY(s), 16);   // the decoder warps
+            mbar_init(RAW_EMPTY(s), 8);    // half of the decoder warps
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(ACC_FULL(a), 1);
-            mbar_init(ACC_EMPTY(a), 4);    // the four epilogue warps
+            mbar_init(ACC_EMPTY(a), 4 * CG);    // the four epilogue warps
         }
         for (int q = 0; q < 4; ++q) mbar_init(PART_FULL(q), (uint32_t)max(C - 1, 1));   // the same warp of the other blocks
         flags[0] = 0;
@@ -549,148 +600,133 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (clustered) mm_cluster_sync();      // the others' barriers exist
+    if (CG == 2 || clustered) mm_cluster_sync();      // the others' barriers exist
     else __syncthreads();
-    if (warp == 1) tmem_alloc(smem_u32((const void*)flags), 512);
+    if (warp == 1) tmem_alloc<CG>(smem_u32((const void*)flags), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = (uint32_t)flags[0];
-    // one or two sets of accumulators, and behind them, for fp32 activations, the sum of the legs so far
-    const uint32_t accs = mm_acc_sets(p.P, Nt), run_col = accs * acc_cols;
+    const uint32_t a_base = tmem + (a_log == 2u ? 256u : 384u);
     pdl_launch_dependents();
 
-    // Every role walks the same list of segments.
+    // Every role walks the same list of segments.  The producers and the issuer are one thread each: with the whole warp in the loop and a
+    // lane elected per block of instructions, eight MMAs and two commits took 220 clocks to issue, by one thread 105.
     if (warp == 0) {
         // ---- bit-tile producer: the weights do not depend on the preceding kernel, so this starts at once.  A tile's eight groups
-        // of sixteen columns are eight streams along K; the tensor map sees them as eight rows, and one box of 8 x 1024 bytes is
+        // of sixteen columns are eight streams along K; the tensor map sees them as eight rows, and one box of 8 x 512 bytes is
         // a unit.  (Eight bulk copies instead, one per lane, took 820 clocks a unit to issue.)
-        uint32_t r = 0, rph = 0;
-        for (int i = 0; i < segs.n; ++i) {
-            int tile, ua, ub, sl;
-            segs.get(i, tile, ua, ub, sl);
-            const int row0 = tile / p.m_tiles * 8;
-            for (int ku = ua; ku < ub; ++ku) {
-                MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
-                if (elect_one()) {
+        if (elect_one()) {
+            uint32_t r = 0, rph = 0;
+            for (int i = 0; i < segs.n; ++i) {
+                int tile, ua, ub, sl;
+                segs.get(i, tile, ua, ub, sl);
+                const int row0 = (tile / p.m_tiles * CG + member) * 8;
+                for (int ku = ua; ku < ub; ++ku) {
+                    MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
                     mbar_expect_tx(RAW_FULL(r), MM_UNIT_BYTES);          // past the end of K the box is filled with zeros, which count
                     tma_load_2d(r_base + r * MM_UNIT_BYTES, &wmap, ku * (MM_UK * 64), row0, RAW_FULL(r));
+                    MM_ADVANCE(r, rph, R);
                 }
-                __syncwarp();
-                MM_ADVANCE(r, rph, R);
             }
         }
     } else if (warp == 6) {
-        // ---- activation producer: a unit is four TMA boxes (all planes of a slice each) on one barrier (whole warp converged, one elected lane per
-        // instruction: addresses and coordinates then are warp-uniform values)
-        pdl_wait();
-        uint32_t b = 0, bph = 0;
-        for (int i = 0; i < segs.n; ++i) {
-            int tile, ua, ub, sl;
-            segs.get(i, tile, ua, ub, sl);
-            const int row0 = (tile % p.m_tiles) * Nt;
-            for (int ku = ua; ku < ub; ++ku) {
-                const int nk = min(MM_UK, KB - ku * MM_UK);
-                MM_WAIT(B_EMPTY(b), bph ^ 1u);
-                if (elect_one()) {
-                    mbar_expect_tx(B_FULL(b), (uint32_t)nk * b_slice);
-                    // (three planes as three boxes a slice would be twelve instructions to issue; one plane as a box of three dimensions
+        // ---- activation producer: a unit is two TMA boxes (all planes of a slice each) on one barrier
+        if (elect_one()) {
+            pdl_wait();
+            uint32_t b = 0, bph = 0;
+            const int rows = Nt / CG;                             // of a pair each block fetches half of the rows, for the first block's barrier
+            for (int i = 0; i < segs.n; ++i) {
+                int tile, ua, ub, sl;
+                segs.get(i, tile, ua, ub, sl);
+                const int row0 = (tile % p.m_tiles) * Nt + member * rows;
+                for (int ku = ua; ku < ub; ++ku) {
+                    const bool two = ku * MM_UK + 1 < KB;
+                    MM_WAIT(B_EMPTY(b), bph ^ 1u);
+                    const uint32_t full = CG == 1 ? B_FULL(b) : mm_peer(B_FULL(b), 0u), to = b_base + b * b_unit;
+                    if (member == 0) mbar_expect_tx(B_FULL(b), (two ? 2u : 1u) * CG * b_slice);
+                    // (three planes as three boxes a slice would be six instructions to issue; one plane as a box of three dimensions
                     // measured 4 % slower than one of two)
                     if (p.P == 1) {
-#pragma unroll
-                        for (int h = 0; h < MM_UK; ++h)
-                            if (h < nk) tma_load_2d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * MM_UK + h) * MM_TILE_K, row0, B_FULL(b));
+                        tma_load_2d<CG>(to, &tmap, ku * (MM_UK * MM_TILE_K), row0, full);
+                        if (two) tma_load_2d<CG>(to + b_slice, &tmap, ku * (MM_UK * MM_TILE_K) + MM_TILE_K, row0, full);
                     } else {
-#pragma unroll
-                        for (int h = 0; h < MM_UK; ++h)
-                            if (h < nk) tma_load_3d(b_base + b * b_unit + (uint32_t)h * b_slice, &tmap, (ku * MM_UK + h) * MM_TILE_K, row0, 0, B_FULL(b));
+                        tma_load_3d<CG>(to, &tmap, ku * (MM_UK * MM_TILE_K), row0, 0, full);
+                        if (two) tma_load_3d<CG>(to + b_slice, &tmap, ku * (MM_UK * MM_TILE_K) + MM_TILE_K, row0, 0, full);
                     }
+                    MM_ADVANCE(b, bph, SB);
                 }
-                __syncwarp();
-                MM_ADVANCE(b, bph, SB);
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer (whole warp converged, one elected lane per instruction)
-        const uint32_t idesc = p.idesc;
-        const uint32_t b_lo0 = (b_base >> 4) & 0x3FFFu;
-        uint32_t sa = 0, saph = 0, sb = 0, sbph = 0, a = 0, aph = 0;
-        for (int i = 0; i < segs.n; ++i) {
-            int tile, ua, ub, sl, left = 0;
-            segs.get(i, tile, ua, ub, sl);
-            uint32_t d = 0, acc = 0;
-            MM_WAIT(A_FULL(sa), saph);
-            MM_WAIT(B_FULL(sb), sbph);
-            tc_fence_after();
-            for (int ku = ua; ku < ub; ++ku) {
-                if (left == 0) {                             // a leg starts
-                    MM_WAIT(ACC_EMPTY(a), aph ^ 1u);
-                    tc_fence_after();
-                    d = tmem + a * acc_cols, acc = 0, left = min(p.leg, ub - ku);
-                }
-                const int nk = min(MM_UK, KB - ku * MM_UK);
-                const uint32_t at = tmem + MM_A_COL + sa * (MM_UK * 32u), b_lo = b_lo0 + sb * (b_unit >> 4), sb0 = sb, sa0 = sa;
-                // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
-                if (elect_one()) {
-#pragma unroll
-                    for (uint32_t h = 0; h < MM_UK - 1; ++h)
-                        if ((int)h < nk) {
-#pragma unroll
-                            for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
-                                umma_f16_ts(d, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, (h | k4) == 0 ? acc : 1u);
-                        }
-                }
-                __syncwarp();
-                MM_ADVANCE(sb, sbph, SB);
-                MM_ADVANCE(sa, saph, MM_A_UNITS);
-                // what comes next is waited for before the last slice goes out: the tensor core works on what is queued meanwhile
-                if (ku + 1 < ub) {
-                    MM_WAIT(A_FULL(sa), saph);
-                    MM_WAIT(B_FULL(sb), sbph);
-                    tc_fence_after();
-                }
-                if (elect_one()) {
-                    if (nk == MM_UK) {
-                        constexpr uint32_t h = MM_UK - 1;
-#pragma unroll
-                        for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4)
-                            umma_f16_ts(d, at + 32u * h + 8u * k4, b_lo + h * (b_slice >> 4) + 2u * k4, idesc, 1u);
+        // ---- MMA issuer; of a pair the first block's.  Nothing but the MMAs' own time lies between two of them as long as the next unit's
+        // operands are there: the tensor core has some in its queue while this thread looks.
+        if (member == 0 && elect_one()) {
+            const uint32_t idesc = p.idesc, b_lo0 = (b_base >> 4) & 0x3FFFu;
+            uint32_t u = 0, sb = 0, sbph = 0, a = 0, aph = 0;
+            for (int i = 0; i < segs.n; ++i) {
+                int tile, ua, ub, sl, left = 0;
+                segs.get(i, tile, ua, ub, sl);
+                uint32_t d = 0, acc = 0;
+                for (int ku = ua; ku < ub; ++ku, ++u) {
+                    const uint32_t sa = u & a_mask, saph = (u >> a_log) & 1u;
+                    MM_SPIN(A_FULL(sa << fine), saph);
+                    MM_SPIN(B_FULL(sb), sbph);
+                    if (left == 0) {                             // a leg starts
+                        MM_SPIN(ACC_EMPTY(a), aph ^ 1u);
+                        d = tmem + a * acc_cols, acc = 0, left = min(p.leg, ub - ku);
                     }
-                    umma_commit(B_EMPTY(sb0));
-                    umma_commit(A_EMPTY(sa0));
-                }
-                __syncwarp();
-                acc = 1;
-                if (--left == 0) {
-                    if (elect_one()) umma_commit(ACC_FULL(a));
-                    __syncwarp();
-                    MM_ADVANCE(a, aph, accs);
+                    tc_fence_after();
+                    const uint32_t at = a_base + sa * (MM_UK * 32u), b_lo = b_lo0 + sb * (b_unit >> 4);
+                    // 16 values = 8 columns of A, 32 bytes = 2 descriptor address units of B
+#pragma unroll
+                    for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4) umma_f16_ts<CG>(d, at + 8u * k4, b_lo + 2u * k4, idesc, k4 == 0 ? acc : 1u);
+                    if (fine) {
+                        umma_commit<CG>(A_EMPTY(2u * sa));
+                        MM_SPIN(A_FULL(2u * sa + 1u), saph);
+                        tc_fence_after();
+                    }
+                    if (ku * MM_UK + 1 < KB) {
+#pragma unroll
+                        for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4) umma_f16_ts<CG>(d, at + 32u + 8u * k4, b_lo + (b_slice >> 4) + 2u * k4, idesc, 1u);
+                    }
+                    umma_commit<CG>(A_EMPTY(fine ? 2u * sa + 1u : sa));
+                    umma_commit<CG>(B_EMPTY(sb));
+                    MM_ADVANCE(sb, sbph, SB);
+                    acc = 1;
+                    if (--left == 0) {
+                        umma_commit<CG>(ACC_FULL(a));
+                        MM_ADVANCE(a, aph, 2u);
+                    }
                 }
             }
         }
     } else if (warp >= 7) {
-        // ---- decoders: a warp expands slice h of every unit, 32 columns of W, into its 32 lanes of tensor memory.  Lane 4g + u
-        // holds column 16 * (u >> 1) + 8 * (u & 1) + g of them (see mm_column).
-        const int q = warp & 3, h = (warp - 7) >> 2;
+        // ---- decoders: eight warps take the even units and eight the odd ones, and a warp expands 32 columns of W of one slice into its 32
+        // lanes of tensor memory.  Lane 4g + u holds column 16 * (u >> 1) + 8 * (u & 1) + g of them (see mm_column).  The values are in
+        // registers before the place in the ring is free: from there on they are a store away.
+        const int q = warp & 3, h = ((warp - 7) >> 2) & 1;
+        const uint32_t mine = (uint32_t)(warp - 7) >> 3;
         const uint32_t g = (uint32_t)lane >> 2, u = (uint32_t)lane & 3u;
-        const uint32_t raw_lane = (uint32_t)(2 * q + (u >> 1)) * 1024u + (uint32_t)(h >> 1) * 512u;
-        const uint32_t a_lane = tmem + MM_A_COL + ((uint32_t)(q * 32) << 16) + (uint32_t)h * 32u;
+        const uint32_t raw_lane = r_base + (uint32_t)(2 * q + (u >> 1)) * 512u;
+        const uint32_t a_lane = a_base + ((uint32_t)(q * 32) << 16) + (uint32_t)h * 32u;
         uint32_t m4, m16;
         asm volatile("mov.b32 %0, %2;\n\tmov.b32 %1, %3;" : "=r"(m4), "=r"(m16) : "r"(p.mul4), "r"(p.mul16));
-        uint32_t sa = 0, saph = 0, r = 0, rph = 0;
+        uint32_t n = 0;                                       // units so far
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
-            for (int ku = ua; ku < ub; ++ku) {
+            for (int ku = ua; ku < ub; ++ku, ++n) {
+                if ((n & 1u) != mine) continue;
                 const int slice = ku * MM_UK + h;
-                const uint32_t at = r_base + r * MM_UNIT_BYTES + raw_lane;
-                MM_WAIT(RAW_FULL(r), rph);
-                uint32_t w[4];
+                const uint32_t r = n & (R - 1u), at = raw_lane + r * MM_UNIT_BYTES, sa = n & a_mask, bar = fine ? 2u * sa + (uint32_t)h : sa;
+                MM_WAIT(RAW_FULL(r), (n / R) & 1u);
+                uint32_t w[4] = {};
                 if ((slice | 1) < KB) {
 #pragma unroll
                     for (int t = 0; t < 4; ++t) {
                         uint32_t lo, hi;
-                        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(at + (uint32_t)mm_chunk((int)g, t) * 16u + (uint32_t)(h & 1) * 8u) : "memory");
+                        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(at + (uint32_t)mm_chunk((int)g, t) * 16u + (uint32_t)h * 8u) : "memory");
                         w[t] = u & 1u ? hi : lo;
                     }
                 } else if (slice < KB) {                      // an odd last slice
@@ -698,22 +734,23 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     for (int t = 0; t < 4; ++t)
                         asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[t]) : "r"(at + (4u * g + (uint32_t)t) * 8u + (u & 1u) * 4u) : "memory");
                 }
+                uint32_t o[32];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) mm_decode_word(w[t], m4, m16, o + 8 * t);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(RAW_EMPTY(r));
-                MM_WAIT(A_EMPTY(sa), saph ^ 1u);
+                MM_WAIT(A_EMPTY(bar), ((n >> a_log) & 1u) ^ 1u);
                 if (slice < KB) {
                     tc_fence_after();
-                    uint32_t o[32];
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) mm_decode_word(w[t], m4, m16, o + 8 * t);
                     tmem_st32(a_lane + sa * (MM_UK * 32u), o);
                     tmem_wait_st();
                     tc_fence_before();
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(A_FULL(sa));
-                MM_ADVANCE(sa, saph, MM_A_UNITS);
-                MM_ADVANCE(r, rph, R);
+                if (lane == 0) {
+                    if (CG == 1) mbar_arrive(A_FULL(bar));
+                    else mm_arrive_first(A_FULL(bar));
+                }
             }
         }
     } else {
@@ -721,40 +758,46 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         const int q = warp & 3, nl = q * 32 + lane, ncol = q * 32 + mm_column(lane);
         pdl_wait();
         uint32_t a = 0, aph = 0;
+        const auto acc_free = [&](uint32_t bar) {
+            if (CG == 1) mbar_arrive(bar);
+            else mm_arrive_first(bar);
+        };
+        // Columns of D: rows [0, Nt / 2) of X of each plane, which a pair's first block holds, and then the other's.
+        const int rows = Nt / CG;
+        const auto column = [&](int c16) { return (uint32_t)(CG == 2 && c16 >= rows ? c16 + (p.P - 1) * rows : c16); };
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
-            const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
-            const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
-            // all legs but the last join the sum in tensor memory
+            const int mt = tile % p.m_tiles, nt = tile / p.m_tiles * CG + member;      // nt: this block's tile of 128 columns; the last of an odd number has no pair
+            const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16), run = run_base + (uint32_t)nl * 4u;
+            // all legs but the last join the sum in shared memory
             bool legs = false;
             for (int left = ub - ua; left > p.leg; left -= p.leg) {
                 MM_WAIT(ACC_FULL(a), aph);
                 tc_fence_after();
                 for (int c16 = 0; c16 < Nt; c16 += 16) {
                     float f[16];
-                    mm_load16(lanes + a * acc_cols + (uint32_t)c16, Nt, p.P, f);
-                    if (legs) mm_add16(lanes + run_col + (uint32_t)c16, f);
-                    tmem_st16(lanes + run_col + (uint32_t)c16, f);
+                    mm_load16(lanes + a * acc_cols + column(c16), rows, p.P, f);
+                    if (legs) mm_add_run(run + (uint32_t)c16 * 512u, f);
+                    mm_store_run(run + (uint32_t)c16 * 512u, f);
                 }
-                tmem_wait_st();
                 legs = true;
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(ACC_EMPTY(a));
-                MM_ADVANCE(a, aph, accs);
+                if (lane == 0) acc_free(ACC_EMPTY(a));
+                MM_ADVANCE(a, aph, 2u);
             }
             MM_WAIT(ACC_FULL(a), aph);
             tc_fence_after();
             const bool full = ua == 0 && ub == KBU;
             const uint32_t taddr = lanes + a * acc_cols;
             const size_t slot_floats = (size_t)MM_TILE_N * Nt;
-            float* slot = p.partial + (size_t)(2 * cta + sl) * slot_floats + nl * 4;
+            float* slot = p.partial + (size_t)(2 * (cta * CG + member) + sl) * slot_floats + nl * 4;
             const int n = nt * MM_TILE_N + ncol;
             // sixteen accumulator columns (rows of X) of this lane's column of W
             auto load16 = [&](int c16, float (&f)[16]) {
-                mm_load16(taddr + (uint32_t)c16, Nt, p.P, f);
-                if (legs) mm_add16(lanes + run_col + (uint32_t)c16, f);
+                mm_load16(taddr + column(c16), rows, p.P, f);
+                if (legs) mm_add_run(run + (uint32_t)c16 * 512u, f);
             };
             auto finish16 = [&](auto out, auto silu, const float (&f)[16], int n, int m) {
                 const uint32_t bad = mm_not_finite(p, f);
@@ -803,13 +846,13 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                         }
                     });
                 }
-            } else if (!full) {
+            } else if (!full && (CG == 1 || nt < p.n_tiles)) {
                 // The last of the blocks that share this tile to arrive adds the partial sums, in block order.  Each epilogue warp owns 32
                 // columns of the tile and runs the hand-over for them by itself.  The last block's own part stays in tensor memory;
                 // a block that finds all the others there already does not even write it.
                 const long long first_unit = (long long)tile * KBU, last_unit = first_unit + KBU - 1;
                 cf = (int)(((first_unit + 1) * G + total - 1) / total - 1), cl = (int)(((last_unit + 1) * G + total - 1) / total - 1);
-                unsigned int* ctr = p.counters + (size_t)tile * 4 + q;
+                unsigned int* ctr = p.counters + ((size_t)nt * p.m_tiles + mt) * 4 + q;
                 const unsigned int others = (unsigned int)(cl - cf);
                 unsigned int there = 0;
                 if (lane == 0) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(there) : "l"(ctr) : "memory");
@@ -831,10 +874,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     __threadfence();
                 }
             }
-            if (!clustered && (full || sum)) {
+            if (!clustered && (full || sum) && (CG == 1 || nt < p.n_tiles)) {
                 // A part lies in its block's slot 0, except that the first block may have come from an earlier tile.
-                const float* part0 = p.partial + (size_t)(2 * cf + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
-                const float* rest = p.partial + (size_t)(2 * cf + 2) * slot_floats + nl * 4;
+                const float* part0 = p.partial + (size_t)(2 * (cf * CG + member) + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
+                const float* rest = p.partial + (size_t)(2 * ((cf + 1) * CG + member)) * slot_floats + nl * 4;
                 mm_with_out(p, [&](auto out, auto silu) {
                     for (int c16 = 0; c16 < Nt; c16 += 16) {
                         float f[16];
@@ -856,7 +899,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 #pragma unroll
                                     for (int t = 0; t < 4; ++t) f[4 * t] += x[t].x, f[4 * t + 1] += x[t].y, f[4 * t + 2] += x[t].z, f[4 * t + 3] += x[t].w;
                                 }
-                                ps = rest + (size_t)(cc - cf) * 2 * slot_floats + (size_t)c16 * MM_TILE_N;
+                                ps = rest + (size_t)(cc - cf) * 2 * CG * slot_floats + (size_t)c16 * MM_TILE_N;
                             }
                         }
                         finish16(out, silu, f, n, mt * Nt + c16);
@@ -865,17 +908,18 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ACC_EMPTY(a));
-            MM_ADVANCE(a, aph, accs);
+            if (lane == 0) acc_free(ACC_EMPTY(a));
+            MM_ADVANCE(a, aph, 2u);
         }
     }
 done:
     __syncwarp();
     tc_fence_before();
-    __syncthreads();
+    if (CG == 2) mm_cluster_sync();        // the pair's MMAs read both blocks' shared and tensor memory
+    else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, 512);
+        tmem_dealloc<CG>(tmem, 512);
     }
     if (tid == 0 && flags[1]) atomicExch(p.status, MM_ERR_WAIT);
     if (clustered) mm_cluster_sync();      // nobody leaves while the others may still write to its shared memory
@@ -890,6 +934,7 @@ done:
 #undef PART_FULL
 }
 #undef MM_WAIT
+#undef MM_SPIN
 #undef MM_ADVANCE
 
 // ---- activations as planes of 16-bit values for the kernel above: rows of k_pad values, zero beyond K ------------------

@@ -87,6 +87,26 @@ def test_tolerance_on_gaussian_activations_and_agreement_with_the_gather_kernel(
     pw.close()
 
 
+# Sizes that go to pairs of blocks: whole tiles and shared ones, two and four places in the ring of expanded units, odd numbers of slices and
+# of column tiles, ragged rows, columns and K, several legs of fp32.
+@pytest.mark.parametrize("M,K,N,dtype", [(500, 1000, 8192, "bf16"), (1500, 2056, 1500, "f16"), (300, 2056, 8192, "bf16"), (2000, 130, 8192, "f16"),
+                                         (130, 4100, 3333, "f32"), (1000, 4100, 640, "f32"), (1000, 448, 8192, "f32"), (500, 4100, 2500, "f32")])
+def test_exact_on_pairs_of_blocks(M, K, N, dtype):
+    rng = np.random.default_rng(M + K)
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w, scale=1.0)
+    x = torch.tensor(rng.integers(-4, 5, size=(M, K)), dtype=torch.float64, device=dev())
+    n0 = mma_launches()
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device=dev())
+    L = _lib.lib()
+    L.tllm_set_mma_min_rows(-1)                       # the library's choice, fp32 as well
+    pw.matmul(x.to({"f32": torch.float32, **DT}[dtype]), out=y)
+    assert mma_launches() > n0, "the call did not run on the tensor-core kernel"
+    assert torch.equal(y.double(), x @ torch.tensor(w, device=dev()).double())
+    pw.check()
+    pw.close()
+
+
 def test_repeated_calls_and_row_counts_share_the_split_scratch():
     """Back-to-back launches with different row counts on one handle (programmatic dependent launch lets the
     next kernel start before the previous one has drained): counters and partial sums must not leak."""
