@@ -243,7 +243,9 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
     const int KB = p.KB, KP = (KB + 1) >> 1, D = p.depth, S = p.slots, M = p.M, SL = p.split_log;
-    const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = warp & ((1 << SL) - 1);
+    // Which share of the columns: the shares may differ by a group, and every scheduler (warp modulo 4) gets some of each, so that none has
+    // all of the larger ones (8192 x 10240, one row: 10.95 us, 11.83 with share = warp modulo shares; 4096 x 11008 6.5 and 6.9).
+    const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = (SL == 1 ? warp ^ (warp >> 2) : warp + (warp >> 2)) & ((1 << SL) - 1);
     const int np = kw < KP ? (KP - kw + kstep - 1) >> klog : 0;      // pairs of this warp: kw, kw + kstep, ...
     const uint32_t ring = smem_u32(bt_smem) + (uint32_t)warp * (uint32_t)S * p.slot_bytes;
     float* red = (float*)(bt_smem + (size_t)BT_WARPS * S * p.slot_bytes);          // [warp][group][column of B][20] partial sums
