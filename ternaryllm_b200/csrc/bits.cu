@@ -49,6 +49,9 @@ int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device,
     if (nb == 1 && gr == 3) return launch<XT, 1, 3, ASYNC>(p, grid, smem, device, st);
     if (nb == 2 && gr == 1) return launch<XT, 2, 1, ASYNC>(p, grid, smem, device, st);
     if (nb == 2 && gr == 2) return launch<XT, 2, 2, ASYNC>(p, grid, smem, device, st);
+    if constexpr (XT == TLLM_I8) {
+        if (nb == 4 && gr == 1) return launch<XT, 4, 1, ASYNC>(p, grid, smem, device, st);
+    }
     if constexpr (XT == TLLM_F32) {
         if (nb == 3 && gr == 1) return launch<XT, 3, 1, ASYNC>(p, grid, smem, device, st);
         if (nb == 3 && gr == 2) return launch<XT, 3, 2, ASYNC>(p, grid, smem, device, st);
@@ -68,8 +71,10 @@ struct BitsPlan {
 BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
     BitsPlan q;
     const int cols = x_dtype == TLLM_F32 ? 3 * rows : rows, groups = (columns + 15) / 16;     // fp32: three bf16 columns a row
-    q.nb = (cols + 7) / 8, q.own = groups / sms, q.own_more = groups % sms;
-    const int most = q.nb > 1 ? 2 : 3, own = q.own + (q.own_more ? 1 : 0);
+    q.nb = (cols + 7) / 8;
+    if (x_dtype == TLLM_I8 && q.nb > 2) q.nb = 4;
+    q.own = groups / sms, q.own_more = groups % sms;
+    const int most = q.nb == 4 ? 1 : q.nb > 1 ? 2 : 3, own = q.own + (q.own_more ? 1 : 0);
     q.split_log = own <= most ? 0 : own <= 2 * most ? 1 : 2;
     const int split = 1 << q.split_log, passes = (own + split * most - 1) / (split * most), kparts = BT_WARPS / split;
     q.passes = passes, q.per_pass = (own + passes - 1) / passes;
@@ -88,7 +93,7 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
     const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
     const bool f32 = x_dtype == TLLM_F32, i8 = x_dtype == TLLM_I8;
-    double step = f32 ? q.nb * (0.6 + 0.18 * q.gr) : 0.25 + q.nb * (0.15 + 0.2 * q.gr);
+    double step = f32 ? q.nb * (0.6 + 0.18 * q.gr) : !i8 ? 0.25 + q.nb * (0.15 + 0.2 * q.gr) : q.nb == 4 ? 1.15 : 0.1 + q.nb * (0.02 + 0.16 * q.gr);
     const double groups = (columns + 15) / 16;               // of few columns few blocks read X
     if (access == BITS_ROWS) step += std::min(1.0, 0.6 + groups / 256) * (f32 ? 0.6 + 0.23 * rows : i8 ? 0.7 + 0.055 * rows : 0.35 + 0.15 * rows);
     else if (access == BITS_COLUMNS)

@@ -25,10 +25,13 @@
 //   2048 x 2048    1 row  2.3 (gather 3.9)      8 rows  2.6 (batched 11.5)
 //   4096 x 11008   1 row  6.2 (gather 8.3, 75 % zeros; four-bit planes 10.5)   8 rows  7.0 (17.2)   16 rows 13.3 (19.5)
 //   8192 x 10240   1 row 10.8 (four-bit planes 15.4)     8 rows 12.1 (22.7)
+// int8: seven instructions instead of fifteen decode sixteen entries, and two MMAs (m16n8k32) replace four:
+//   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 6.9 in one launch (9.3 in two)
+//   8192 x 10240   1 row  7.6 (12.0)             16 rows 15 (22)
 // Of the 6.2 us, 3.3 are there without any decode or MMA (launch chain, activations from L2, sums); the rest is instruction
 // issue, 0.55 per scheduler and clock.
 //
-// Precision.  fp16 / bf16 activations are multiplied as they are; int8 becomes fp16 (exact); an fp32 value is cut into
+// Precision.  fp16 / bf16 activations are multiplied as they are; int8 as int8 with int32 sums (exact); an fp32 value is cut into
 // three bf16 values of eight significant bits each (truncation, so the three add up to it exactly), three columns of B
 // whose sums are added at the end.  W is 0 / +-2 (the factor two is taken back with the scale), products are exact, sums
 // are fp32; integer activations give exact sums below 2^24.  A sum that is not finite is taken again entry by entry
@@ -45,8 +48,9 @@ namespace tllm {
 #define BT_WARPS 16
 #define BT_SMEM_SHARED (112u * 1024u)   // two blocks of this size share an SM
 #define BT_SMEM_ALONE (116u * 1024u)    // two of this do not
-#define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks)
+#define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks; int8: 32, four)
 #define BT_MASK 0xC000C000u             // the two codes at the top of a word's halves: 16-bit floats 0 / +-2
+#define BT_MASK8 0xC0C0C0C0u            // the four at the top of its bytes: 0 / +-64
 
 struct BitsParams {
     const uint4* bits;
@@ -88,6 +92,11 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_16832(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -181,9 +190,10 @@ template <int XT>
 __device__ __forceinline__ uint32_t bt_lane_chunk(uint32_t t, uint32_t m) { return bt_chunk<XT>(t * BitsAct<XT>::E, m) * 16u; }
 // The lane's sixteen activations of slice h (rows 16t .. 16t+15) -> the eight words of a B fragment (word p = rows 2p, 2p+1);
 // `at` is the address of the lane's first chunk of slice 0.  fp32: the `piece`-th of the three bf16 values that add up to
-// each of them.
+// each of them.  int8: four words, word s = rows 8+2s, 2s, 9+2s, 2s+1, which is where the codes stand that a shift by 2s brings to the
+// top of a word's bytes.
 template <int XT>
-__device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, uint32_t (&b)[8]) {
+__device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, uint32_t (&b)[XT == TLLM_I8 ? 4 : 8]) {
     constexpr uint32_t CS = BitsAct<XT>::E;
     uint32_t w[4 * CS];
     const uint32_t a0 = XT == TLLM_I8 ? at ^ (h * 64u) : at + h * (CS * 64u);
@@ -204,13 +214,7 @@ __device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, 
         for (int i = 0; i < 8; ++i) b[i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x7632);
     } else if constexpr (XT == TLLM_I8) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t u = w[i >> 1] ^ 0x80808080u;                                     // 0..255: x + 128
-            const uint32_t v = __byte_perm(u, 0x64646464u, i & 1 ? 0x4342 : 0x4140);        // fp16 1024 + (x + 128)
-            const uint32_t bias = 0x64806480u;                                              // 1152 twice
-            const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&bias));
-            b[i] = *reinterpret_cast<const uint32_t*>(&d);
-        }
+        for (int i = 0; i < 4; ++i) b[i] = __byte_perm(w[i >> 1], w[2 + (i >> 1)], i & 1 ? 0x3726 : 0x1504);
     } else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) b[i] = w[i];
@@ -235,7 +239,8 @@ template <int XT, int NB, int GR, bool ASYNC>
 __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_spmm_kernel(const __grid_constant__ BitsParams p) {
     extern __shared__ __align__(128) unsigned char bt_smem[];
     using Act = BitsAct<XT>;
-    constexpr bool BF16 = XT == TLLM_BF16 || XT == TLLM_F32;
+    constexpr bool BF16 = XT == TLLM_BF16 || XT == TLLM_F32, I8 = XT == TLLM_I8;
+    using Sum = typename std::conditional<I8, int, float>::type;
     // The tensor core cuts bits off its running sum at every MMA: fp32 sums leave it after the eight of a pair of slices (gate and up of a
     // 2560 / 6912 MLP, 8 rows, h = silu(gate) * up: off by 1.4e-7 with a warp's 40 MMAs in one sum, 1.1e-7 now).
     constexpr bool PARTS = XT == TLLM_F32;
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = (SL == 1 ? warp ^ (warp >> 2) : warp + (warp >> 2)) & ((1 << SL) - 1);
     const int np = kw < KP ? (KP - kw + kstep - 1) >> klog : 0;      // pairs of this warp: kw, kw + kstep, ...
     const uint32_t ring = smem_u32(bt_smem) + (uint32_t)warp * (uint32_t)S * p.slot_bytes;
-    float* red = (float*)(bt_smem + (size_t)BT_WARPS * S * p.slot_bytes);          // [warp][group][column of B][20] partial sums
+    Sum* red = (Sum*)(bt_smem + (size_t)BT_WARPS * S * p.slot_bytes);          // [warp][group][column of B][20] partial sums
     const uint32_t group_bytes = (uint32_t)KB * 256u;
     pdl_launch_dependents();
     // There is a block for every SM even where there are fewer groups: with free SMs the next launch's blocks would be placed
@@ -347,13 +352,13 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
 #pragma unroll 1
     for (int q0 = 0; q0 < own; q0 += p.per_pass) {
         const int ng = min(p.per_pass, own - q0), w0 = (ng * cw) >> SL, mine = ((ng * (cw + 1)) >> SL) - w0;    // this warp's groups of the pass
-        float acc[GR][NB][4];
+        Sum acc[GR][NB][4];
 #pragma unroll
         for (int j = 0; j < GR; ++j)
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[j][nb][i] = 0.f;
+                for (int i = 0; i < 4; ++i) acc[j][nb][i] = 0;
 #pragma unroll 1
         for (int i = 0; i < np; ++i) {
             cp_wait(D - 1);
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
             }
 #pragma unroll 1
             for (uint32_t h = 0; h < 2; ++h) {
-                uint32_t bf[NB][8];
+                uint32_t bf[NB][I8 ? 4 : 8];
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) bt_fragment<XT>(slot + bat[nb], h, bpiece[nb], bf[nb]);
                 auto half = [&](auto first, auto end) {              // groups [lo, hi) of the warp
@@ -386,14 +391,19 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
 #pragma unroll
                     for (int j = lo; j < hi; ++j) a[j] = bt_lds64(slot + (uint32_t)j * 512u + wchunk + h * 8u);
                     // consecutive MMAs go to different accumulators: a chain of dependent ones costs their full latency each
+                    constexpr int MMAS = I8 ? 2 : 4;
+                    constexpr uint32_t MASK = I8 ? BT_MASK8 : BT_MASK;
 #pragma unroll
-                    for (int s = 0; s < 4; ++s)
+                    for (int s = 0; s < MMAS; ++s)
 #pragma unroll
                         for (int j = lo; j < hi; ++j) {
-                            const uint32_t a0 = a[j].x & BT_MASK, a1 = a[j].y & BT_MASK, a2 = (a[j].x * m4) & BT_MASK, a3 = (a[j].y * m4) & BT_MASK;
-                            if (s < 3) a[j].x *= m16, a[j].y *= m16;
+                            const uint32_t a0 = a[j].x & MASK, a1 = a[j].y & MASK, a2 = (a[j].x * m4) & MASK, a3 = (a[j].y * m4) & MASK;
+                            if (s < MMAS - 1) a[j].x *= m16, a[j].y *= m16;
 #pragma unroll
-                            for (int nb = 0; nb < NB; ++nb) mma_16816<BF16>(PARTS ? part[j][nb] : acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                            for (int nb = 0; nb < NB; ++nb) {
+                                if constexpr (I8) mma_16832(acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                                else mma_16816<BF16>(PARTS ? part[j][nb] : acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                            }
                         }
                 };
                 // a warp's share of a pass is GR groups or one less (or none: GR = 1)
@@ -418,7 +428,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
 #pragma unroll
         for (int j = 0; j < GR; ++j)
             if (j < mine) {
-                float* r = red + (size_t)kw * kw_step + (w0 + j) * MC * 20 + g;
+                Sum* r = red + (size_t)kw * kw_step + (w0 + j) * MC * 20 + g;
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
                     const int m = nb * 8 + 2 * t;
@@ -433,24 +443,25 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
         for (int i0 = warp * 2; i0 < ng * M; i0 += BT_WARPS * 2) {
             const int idx = i0 + (lane >> 4), j = M > 1 ? (int)__umulhi((uint32_t)idx, p.m_inv) : idx, m = idx - j * M;
             const bool valid = idx < ng * M;
-            float v = 0.f;
+            Sum v = 0;
             if (valid) {
-                const float* r = red + (j * MC + m * Act::P) * 20 + c;
+                const Sum* r = red + (j * MC + m * Act::P) * 20 + c;
 #pragma unroll
                 for (int pc = Act::P - 1; pc >= 0; --pc)            // fp32: the small pieces first
 #pragma unroll 4
                     for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
             }
             const int n = (c0 + q0 + j) * 16 + c;
+            const size_t at = (size_t)m * p.y_step_m + (size_t)n * p.y_step_n;
+            if constexpr (I8) {                                      // an exact multiple of 64
+                if (valid && n < p.N) ((int*)p.Y)[at] = v >> 6;
+                continue;
+            }
             const float sc = p.epilogue && (c & 1) ? p.scale2 : p.scale;
             float y = v * sc;
-            if (XT != TLLM_I8 && __builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
+            if (__builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
             if (p.epilogue == 0) {
-                if (valid && n < p.N) {
-                    const size_t at = (size_t)m * p.y_step_m + (size_t)n * p.y_step_n;
-                    if (XT == TLLM_I8) ((int*)p.Y)[at] = (int)(v * 0.5f);
-                    else store_out(p.Y, p.y_dtype, at, y);
-                }
+                if (valid && n < p.N) store_out(p.Y, p.y_dtype, at, y);
             } else {
                 const float u = __shfl_xor_sync(0xffffffffu, y, 1);
                 if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(y, u));

@@ -780,8 +780,8 @@ int run_nb(tllm_weight* w, const void* X, int x_dtype, int x_ld, int rows, void*
 }
 
 // ---- two-bit tiles decoded in registers ----------------------------------------------------------------------------
-// rows one launch takes: 16, fp32 (three bf16 values each) 8
-int bt_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? BT_MAX_ROWS / 2 : BT_MAX_ROWS; }
+// rows one launch takes: 16, fp32 (three bf16 values each) 8, int8 32
+int bt_rows_per_launch(int x_dtype) { return x_dtype == TLLM_F32 ? BT_MAX_ROWS / 2 : x_dtype == TLLM_I8 ? BT_MAX_ROWS * 2 : BT_MAX_ROWS; }
 
 int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld, int rows, void* Y, int y_dtype, int y_ld, int epilogue, float scale,
              float scale2, cudaStream_t st, bool y_col = false) {

@@ -58,6 +58,21 @@ def test_exact_on_integer_activations(K, N, s, dtype):
     pw.close()
 
 
+# int8 sums are int32: the largest values of one sign, at the row counts around the blocks of eight, sixteen and thirty-two rows
+@pytest.mark.parametrize("M", [8, 9, 15, 16, 17, 31, 32, 33])
+@pytest.mark.parametrize("K,N", [(64, 16), (130, 517), (8200, 40)])
+def test_int8_extremes(K, N, M):
+    w = random_ternary(np.random.default_rng(M), K, N, 0.3)
+    w[:, 0], w[:, 1] = 1, -1
+    pw = PackedWeight.from_dense(w)
+    x = torch.randint(-128, 128, (M, K), dtype=torch.int8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(K))
+    x[0], x[-1] = -128, 127
+    want = x.double() @ torch.tensor(w, device="cuda").double()
+    assert torch.equal(pw.matmul(x).double(), want)
+    assert torch.equal(pw.matmul(x.t().contiguous(), col_major=True).double(), want)
+    pw.close()
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
 def test_gaussian_activations_and_result_types(dtype):
     rng = np.random.default_rng(5)
