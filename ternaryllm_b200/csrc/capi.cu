@@ -162,7 +162,8 @@ struct BitsView {
     float* partial;               // 2 * sms hand-over slots for row tiles of up to MM_OWN_NT, or NULL
     unsigned int* counters;       // n_tiles * MM_MAX_M_TILES * 4, zero between launches
     int* status;
-    bool lists;                   // made from lists by the preceding kernel: the product may not start beside it; else the tiles were there before
+    bool lists;                   // made from lists by the preceding kernel: the product has to wait for it; else the tiles were there before
+    bool fresh;                   // lists: nothing has been launched since
 };
 
 struct tllm_mlp {
@@ -249,7 +250,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 BitsView bits_view(const tllm_weight* w) {
-    return BitsView{w->d_bits, &w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, false};
+    return BitsView{w->d_bits, &w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, false, false};
 }
 
 // true when TMA can read the activations where they are (rows on 16 bytes; a box is 64 values wide)
@@ -426,8 +427,8 @@ cudaLaunchAttribute pdl_attribute() {
 
 int stage_pad(int k) { return (k + 63) / 64 * 64; }
 
-int run_stage(const void* X, int x_dtype, int x_layout, int x_ld, int rows, int K, unsigned short* out, cudaStream_t st) {
-    StageParams q{X, out, x_dtype, x_layout, x_ld, rows, K, stage_pad(K)};
+int run_stage(const void* X, int x_dtype, int x_layout, int x_ld, int rows, int K, unsigned short* out, bool late, cudaStream_t st) {
+    StageParams q{X, out, x_dtype, x_layout, x_ld, rows, K, stage_pad(K), late};
     void (*kern)(StageParams) = x_dtype == TLLM_F32 ? stage_acts_kernel<TLLM_F32> : x_dtype == TLLM_I8 ? stage_acts_kernel<TLLM_I8> : stage_acts_kernel<TLLM_F16>;
     cudaLaunchConfig_t cfg{};
     const long long blocks = x_layout == TLLM_ROW_MAJOR ? ((long long)rows * (q.k_pad / 8) + 255) / 256 : (long long)(q.k_pad / 64) * ((rows + 31) / 32);
@@ -489,6 +490,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     p.scale = o.scale * 0.5f, p.scale2 = o.scale2 * 0.5f;          // the decoded weights are +-2
     p.finite = x.finite;
     p.bits = (const uint32_t*)w.bits, p.X = (const unsigned short*)x.base, p.bf16 = x.bf16;
+    p.wait_bits = w.lists;
     p.ld_x = (long long)(x.pitch / 2), p.plane_x = x.plane_rows * p.ld_x;
 
     CUtensorMap map;
@@ -520,7 +522,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     cfg.stream = st;
     cudaLaunchAttribute at[2] = {};
     int n_at = 0;
-    if (!w.lists) at[n_at++] = pdl_attribute();
+    at[n_at++] = pdl_attribute();
     if (p.split == 2 || cg == 2) {
         at[n_at].id = cudaLaunchAttributeClusterDimension;
         at[n_at].val.clusterDim.x = (unsigned)(cg == 2 ? 2 : p.cluster), at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
@@ -563,7 +565,7 @@ int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld
         const char* xp = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
         MmActs a{xp, x_dtype == TLLM_BF16 || x_dtype == TLLM_F32, planes, m, (size_t)x_ld * 2, finite};
         if (!direct) {
-            const int rc = run_stage(xp, x_dtype, x_layout, x_ld, m, K, (unsigned short*)ws.ptr, st);
+            const int rc = run_stage(xp, x_dtype, x_layout, x_ld, m, K, (unsigned short*)ws.ptr, w.fresh && r0 == 0, st);
             if (rc) return rc;
             a.base = ws.ptr, a.pitch = (size_t)stage_pad(K) * 2;
         }
@@ -1098,9 +1100,15 @@ int run_mcsc(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, c
     const dim3 grid((columns + 7) / 8, (rows + MCSC_ROWS - 1) / MCSC_ROWS, batch);
 #define MCSC_ARGS rows, columns, inners, tile_k, scale
     if (flags) {
-        if (x_dtype == TLLM_I8)
-            mcsc_spmm_if_kernel<int, MCSC_ROWS><<<blocks, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, MCSC_ARGS, flags, nflags);
-        else mcsc_spmm_if_kernel<float, MCSC_ROWS><<<blocks, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, MCSC_ARGS, flags, nflags);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1] = {pdl_attribute()};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        auto kern = x_dtype == TLLM_I8 ? mcsc_spmm_if_kernel<int, MCSC_ROWS> : mcsc_spmm_if_kernel<float, MCSC_ROWS>;
+        CU_TRY(cudaLaunchKernelEx(&cfg, kern, X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, MCSC_ARGS, flags, nflags));
     } else {
         if (grid.y > 65535) return fail(TLLM_ERR_ARG, "tllm_ter_spmm: too many rows for one call");
         if (x_dtype == TLLM_I8) mcsc_spmm_kernel<int, MCSC_ROWS><<<grid, 256, 0, st>>>(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, MCSC_ARGS);
@@ -1127,14 +1135,19 @@ int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, 
     uint32_t* bits = (uint32_t*)ws.ptr;
     unsigned int* counters = (unsigned int*)((char*)ws.ptr + bits_bytes);
     int* flags = (int*)(counters + counter_words);          // one per group of columns, then the status word of the product
-    lists_to_bits_kernel<<<(unsigned)groups, LB_THREADS, 0, st>>>(row_idx, col_off, bits, counters, (int)counter_words, flags, columns, inners, tile_k, kb);
-    CU_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)groups);
+    cfg.blockDim = dim3(LB_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1] = {pdl_attribute()};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU_TRY(cudaLaunchKernelEx(&cfg, lists_to_bits_kernel, row_idx, col_off, bits, counters, (int)counter_words, flags, columns, inners, tile_k, kb));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     CUtensorMap map;
     rc = encode_bits_map(&map, bits, n_tiles, kb);
     if (rc) return rc;
-    // not beside the preceding kernel: that is the one that writes the tiles
-    const BitsView view{(const uint4*)bits, &map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, true};
+    BitsView view{(const uint4*)bits, &map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, true, true};
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const bool one = x_layout == TLLM_ROW_MAJOR && (long long)batch * rows <= 0x7fffffffLL;      // the batch is contiguous: one product
     const int parts = one ? 1 : batch, m = one ? batch * rows : rows, x_ld = x_layout == TLLM_ROW_MAJOR ? inners : rows;
@@ -1145,6 +1158,7 @@ int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, 
             rc = run_bits(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
         else rc = run_mm(view, xp, x_dtype, x_layout, x_ld, m, yp, y_dtype, columns, 0, scale, 0.f, st);
         if (rc) return rc;
+        view.fresh = false;
     }
     // lists that two bits an entry cannot hold (an entry named twice) are computed as before
     return run_mcsc(X, x_dtype, x_layout, row_idx, col_off, Y, y_dtype, batch, rows, columns, inners, tile_k, scale, flags, groups + 1, 2 * sms, st);

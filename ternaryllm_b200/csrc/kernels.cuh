@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(256) mcsc_spmm_if_kernel(const void* __restric
                                                             const int16_t* __restrict__ idx, const int32_t* __restrict__ off,
                                                             void* __restrict__ Y, int y_dtype, int B, int M, int N, int K, int T, float scale, const int* flags,
                                                             int nflags) {
+    pdl_launch_dependents();
+    pdl_wait();
     int any = 0;
     for (int i = threadIdx.x; i < nflags; i += blockDim.x) any |= __ldcg(flags + i);
     if (!__syncthreads_or(any)) return;

@@ -111,6 +111,7 @@ struct MmParams {
     const unsigned short* X;
     long long plane_x, ld_x;
     bool bf16;
+    bool wait_bits;           // the bit tiles are the work of a kernel that may not have finished
 };
 
 // ---- tcgen05 / TMA wrappers ------------------------------------------------------------------------------
@@ -617,6 +618,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         // of sixteen columns are eight streams along K; the tensor map sees them as eight rows, and one box of 8 x 512 bytes is
         // a unit.  (Eight bulk copies instead, one per lane, took 820 clocks a unit to issue.)
         if (elect_one()) {
+            if (p.wait_bits) pdl_wait();
             uint32_t r = 0, rph = 0;
             for (int i = 0; i < segs.n; ++i) {
                 int tile, ua, ub, sl;
@@ -943,6 +945,7 @@ struct StageParams {
     unsigned short* out;      // [planes][M][k_pad]
     int x_dtype, x_layout, x_ld;
     int M, K, k_pad;
+    bool late;                // neither X nor `out` has to do with the preceding kernel: it is waited for at the end
 };
 // eight consecutive values of one row -> 16 bytes of each plane
 template <int XT>
@@ -980,7 +983,7 @@ __device__ __forceinline__ uint32_t stage_load(const void* X, size_t at) {
 template <int XT>
 __global__ void __launch_bounds__(256) stage_acts_kernel(const __grid_constant__ StageParams p) {
     pdl_launch_dependents();
-    pdl_wait();
+    if (!p.late) pdl_wait();
     uint32_t w[8];
     if (p.x_layout == TLLM_ROW_MAJOR) {
         const long long per_row = p.k_pad / 8, i = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -1012,6 +1015,7 @@ __global__ void __launch_bounds__(256) stage_acts_kernel(const __grid_constant__
         for (int j = 0; j < 8; ++j) w[j] = tile[k8 + j][m];
         if (m0 + m < p.M) stage_eight<XT>(p, w, m0 + m, kt * 64 + k8);
     }
+    if (p.late) pdl_wait();           // so that whoever waits for this kernel has waited for that one too
 }
 
 }  // namespace tllm
