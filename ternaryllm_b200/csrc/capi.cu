@@ -17,6 +17,7 @@
 #include "kernels.cuh"
 #include "lists_kernel.cuh"
 #include "mma_kernel.cuh"
+#include "mma_units4_kernel.cuh"
 #include "nibble_format.h"
 #include "nibble_kernel.cuh"
 #include "nibble_rows_kernel.cuh"
@@ -135,7 +136,7 @@ struct tllm_weight {
     float* d_mm_partial = nullptr;
     unsigned int* d_mm_counters = nullptr;
     size_t bits_bytes = 0;
-    CUtensorMap bits_map;
+    CUtensorMap bits_map[2];
     int mm_n_tiles = 0, mm_kb = 0, mm_grid = 0;
     // decode tensor-core kernel: transposed four-bit copy of W, its tensor map, schedule and hand-over scratch
     uint8_t* d_nib = nullptr;
@@ -157,7 +158,7 @@ struct tllm_weight {
 // What the two kernels that read bit tiles need of a weight: a handle's, or one made for a single call (tllm_ter_spmm).
 struct BitsView {
     const uint4* bits;
-    const CUtensorMap* map;
+    const CUtensorMap* map;       // bit tiles in boxes of a unit: [0] two slices, [1] four (mma_units4_kernel)
     int inners, columns, n_tiles, kb, sms, device;
     float* partial;               // 2 * sms hand-over slots for row tiles of up to MM_OWN_NT, or NULL
     unsigned int* counters;       // n_tiles * MM_MAX_M_TILES * 4, zero between launches
@@ -250,7 +251,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 BitsView bits_view(const tllm_weight* w) {
-    return BitsView{w->d_bits, &w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, false, false};
+    return BitsView{w->d_bits, w->bits_map, w->lay.inners, w->lay.columns, w->mm_n_tiles, w->mm_kb, w->mm_grid, w->device, w->d_mm_partial, w->d_mm_counters, w->d_status, false, false};
 }
 
 // true when TMA can read the activations where they are (rows on 16 bytes; a box is 64 values wide)
@@ -319,37 +320,43 @@ struct Workspace {
     }
 };
 
-// How a product of `rows` rows (in `planes` planes) is cut: row tiles of Nt rows each, and whole tiles, equal ranges of units, or a
-// cluster per tile; by one block or by a pair of blocks.  Chosen by an estimate in SM clocks, fitted to 1400 plans of 9 weights from
-// 512 x 512 to 5120 x 15360 and 20 to 2048 rows (6 % off in the mean, and the plan it picks 1.3 % slower than the best).
-// A unit is eight MMAs of 128 x (planes * Nt) x 16.  With a pair they take little more than their own time, 4.3 clocks a column.  A block by
-// itself takes as long up to 256 columns as its shared memory needs to write and read the activations: 600 clocks and 2.2 a column.
-// Neither takes less than the 750 of decoding a unit.  A tile's epilogue is hidden behind the next one where that takes longer.
+// How a product of `rows` rows (in `planes` planes) is cut: by which of the two kernels, row tiles of Nt rows each, and whole tiles, equal
+// ranges of units, or a cluster per tile; by one block or by a pair of blocks.  Chosen by estimates, fitted to 1700 plans of 11 weights from
+// 512 x 512 to 5120 x 15360 and 20 to 2048 rows (6 % off in the mean, and the plan that is picked 1.6 % slower than the best).
+// Units of two slices, in SM clocks: eight MMAs of 128 x (planes * Nt) x 16.  With a pair they take little more than their own time, 4.3 a
+// column.  A block by itself takes as long as its shared memory needs to write and read the activations: 630 clocks and 2.4 a column.
+// Neither takes less than the 780 of decoding a unit.  A tile's epilogue is hidden behind the next one where that takes longer.
+// Units of four slices: a slice is four MMAs, 2.5 clocks a column and never less than the 255 of their issue; where there is no room for two
+// sets of accumulators a tile's epilogue and legs are not hidden; the first unit of activations takes 12 clocks a row to arrive.
 // In a tile that `parts` blocks share the last one to arrive reads the other parts, a round trip to L2 for every sixteen rows of each.
 // A cluster of C blocks per tile: every block's units, then what goes to the other blocks and the adding-up of its own share.
 // A launch that holds more than half of the SMs keeps the next one's blocks, one to an SM, from starting up beside it.
 struct MmPlan {
     int Nt, m_tiles, split, cluster;
     int cg;                  // blocks that share a tile's MMAs: 1, or 2 (a pair: 256 columns of W, half of the activations in each block)
-    double clocks;
+    bool units4;             // mma_units4_kernel
+    double us;
+    double model;            // for the choice between kernels, whose other side was fitted beside it
 };
 constexpr int MM_SMEM = 227 * 1024;
 // shared memory beside the units of B: bit tiles, barriers, a cluster's parts, the sum of the legs of three planes
-int mm_other_bytes(int nt, int planes, int cluster) {
+int mm_other_bytes(int nt, int planes, int cluster, bool units4) {
     const int parts = cluster > 1 ? cluster * ((nt / 16 + cluster - 1) / cluster) * 8192 : 0;
-    return 1024 + 512 + MM_RAW_UNITS * MM_UNIT_BYTES + parts + (planes > 1 ? nt * 512 : 0);
+    return 1024 + 512 + (units4 ? MS_RAW_UNITS * MS_UNIT_BYTES : MM_RAW_UNITS * MM_UNIT_BYTES) + parts + (planes > 1 && !units4 ? nt * 512 : 0);
 }
+using MmKernel = void (*)(CUtensorMap, CUtensorMap, MmParams);
+MmKernel mm_kernel(int cg, bool units4) { return units4 ? mma_units4_kernel : cg == 2 ? mma_spmm_kernel<2> : mma_spmm_kernel<1>; }
 // clusters of `cluster` blocks (cg = 2: pairs) that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a
 // GPU is made of
-int mm_clusters(int cluster, int cg, int sms, int device) {
-    static std::atomic<int> known[64][9];
-    const int slot = cg == 2 ? 1 : cluster;
-    auto kern = cg == 2 ? mma_spmm_kernel<2> : mma_spmm_kernel<1>;
+int mm_clusters(int cluster, int cg, bool units4, int sms, int device) {
+    static std::atomic<int> known[64][18];
+    const int slot = (units4 ? 9 : 0) + (cg == 2 ? 1 : cluster);
+    const MmKernel kern = mm_kernel(cg, units4);
     int n = device < 64 ? known[device][slot].load(std::memory_order_relaxed) : 0;
     if (n == 0) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(sms / cluster * cluster));
-        cfg.blockDim = dim3(MM_THREADS);
+        cfg.blockDim = dim3(units4 ? MS_THREADS : MM_THREADS);
         cfg.dynamicSmemBytes = MM_SMEM;
         cudaLaunchAttribute at[1] = {};
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -366,32 +373,60 @@ int mm_clusters(int cluster, int cg, int sms, int device) {
 }
 int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
 MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
-    MmPlan best{0, 0, 0, 1, 1, 0};
-    const int kbu = (kb + MM_UK - 1) / MM_UK, pairs = n_tiles > 1 ? mm_clusters(2, 2, sms, device) : 0;
+    MmPlan best{0, 0, 0, 1, 1, false, 0, 0};
     const bool one = planes == 1;
-    const auto take = [&](int nt, int mt, int split, int c, int cg, double clocks) {
-        if (best.Nt == 0 || clocks < best.clocks) best = MmPlan{nt, mt, split, c, cg, clocks};
+    const auto take = [&](int nt, int mt, int split, int c, int cg, double us) {
+        if (best.Nt == 0 || us < best.us) best = MmPlan{nt, mt, split, c, cg, false, us, us};
     };
+    const int kbu = (kb + MM_UK - 1) / MM_UK, kbu4 = (kb + MS_UK - 1) / MS_UK, pairs = n_tiles > 1 ? mm_clusters(2, 2, false, sms, device) : 0;
+    MmPlan four{0, 0, 0, 1, 1, true, 0, 0};          // us: clocks, until the loop is done
     for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
-        const int mt = (rows + nt - 1) / nt, cols = planes * nt, sixteens = nt / 16;
+        const int mt = (rows + nt - 1) / nt, cols = planes * nt, sixteens = nt / 16, turns = (sixteens + 1) / 2;     // turns: sixteens of an epilogue warp
         if (mt > MM_MAX_M_TILES) continue;
-        const double piece = one ? 780.0 : 1700.0, epilogue = sixteens * piece, legs = one ? 0.0 : ((kbu + MM_LEG - 1) / MM_LEG - 1) * sixteens * 300.0;
-        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (one ? 2600.0 : 4000.0) : 0.0; };
+        // units of two slices
+        const double piece = one ? 940.0 : 2100.0, epilogue = turns * piece, legs = one ? 0.0 : ((kbu + MM_LEG - 1) / MM_LEG - 1) * turns * 300.0;
+        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (one ? 2400.0 : 3000.0) : 0.0; };
+        const auto us = [&](double clocks) { return ((one ? 5700.0 : 8900.0) + clocks) / 1850.0; };
         for (int cg = 1; cg <= 2; ++cg) {
             const double groups = cg == 1 ? sms : pairs, tiles = (double)((n_tiles + cg - 1) / cg) * mt, units = tiles * kbu;
             if (groups <= 0 || nt % (16 * cg) != 0) continue;
-            const double unit = std::max(750.0, cg == 1 ? 600.0 + 2.2 * cols : 130.0 + 4.3 * cols), extra = cg == 1 ? 0.0 : 1400.0;
-            take(nt, mt, 0, 1, cg, extra + (std::ceil(tiles / groups) - 1) * std::max(kbu * unit, epilogue + legs) + kbu * unit + epilogue + crowd(tiles * cg));
+            const double unit = std::max(780.0, cg == 1 ? 630.0 + 2.36 * cols : 150.0 + 4.34 * cols), extra = cg == 1 ? 0.0 : 1300.0;
+            take(nt, mt, 0, 1, cg, us(extra + (std::ceil(tiles / groups) - 1) * std::max(kbu * unit, epilogue + legs) + kbu * unit + epilogue + crowd(tiles * cg)));
             const double blocks = std::min(units, groups), parts = std::min((double)kbu, blocks / tiles + 1.0);
-            take(nt, mt, 1, 1, cg, extra + std::ceil(units / blocks) * unit + 3600.0 + 2.8 * epilogue + sixteens * 580.0 * (parts - 1) + crowd(blocks * cg));
+            take(nt, mt, 1, 1, cg, us(extra + std::ceil(units / blocks) * unit + 4900.0 + (one ? 2.7 : 3.1) * epilogue + turns * 630.0 * (parts - 1) + crowd(blocks * cg)));
             for (int c = 2; cg == 1 && c <= 8 && c <= kbu; c *= 2) {
-                if (MM_SMEM - mm_other_bytes(nt, planes, c) < 2 * cols * 128 * MM_UK || mm_clusters(c, 1, sms, device) < tiles) continue;
-                take(nt, mt, 2, c, 1, (kbu + c - 1) / c * unit + 3600.0 + sixteens * 400.0 + (sixteens + c - 1) / c * piece + crowd(tiles * c));
+                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols * 128 * MM_UK || mm_clusters(c, 1, false, sms, device) < tiles) continue;
+                take(nt, mt, 2, c, 1, us((kbu + c - 1) / c * unit + 3400.0 + sixteens * 600.0 + ((sixteens + c - 1) / c + 1) / 2 * piece + crowd(tiles * c)));
             }
+        }
+        // units of four slices
+        const double tiles = (double)n_tiles * mt, units = tiles * kbu4;
+        const double slice = std::max(255.0, 2.5 * cols), epilogue4 = sixteens * 350.0, fill = 12.0 * cols;
+        const bool two = ms_acc_sets(planes, nt) == 2;
+        const auto legs4 = [&](double u) { return two || one ? 0.0 : (std::ceil(u / MS_LEG) - 1) * (500 + sixteens * 150.0); };
+        const auto crowd4 = [&](double blocks) { return 2 * blocks > sms ? (one ? 3000.0 : 1000.0) : 0.0; };
+        const auto take4 = [&](int split, int c, double clocks) {
+            if (four.Nt == 0 || clocks + fill < four.us) four = MmPlan{nt, mt, split, c, 1, true, clocks + fill, 0};
+        };
+        take4(0, 1, crowd4(tiles) + std::ceil(tiles / sms) * (kb * slice + legs4(kbu4) + (two ? 0.0 : epilogue4)) + (two ? epilogue4 : 0.0));
+        const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu4, blocks / tiles + 1.0);
+        take4(1, 1, crowd4(blocks) + std::ceil(units / blocks) * MS_UK * slice + legs4(std::min(units / blocks, (double)kbu4)) + 3000.0 + 3 * epilogue4 + sixteens * 1000.0 * (parts - 1));
+        for (int c = 2; c <= 8 && c <= kbu4; c *= 2) {
+            if (MM_SMEM - mm_other_bytes(nt, planes, c, true) < 2 * cols * 128 * MS_UK || mm_clusters(c, 1, true, sms, device) < tiles) continue;
+            take4(2, c, (kbu4 + c - 1) / c * MS_UK * slice + legs4((kbu4 + c - 1) / c) + 2000.0 + sixteens * 100.0 + (sixteens + c - 1) / c * 350.0 + crowd4(tiles * c));
         }
         if (nt >= rows) break;
     }
-    return best;
+    if (four.Nt != 0) {                // what calls of these clocks took, 196 of them
+        const double k = four.us / 1000.0, sixteens = four.Nt / 16;
+        four.model = 2.4 + four.us / 1800.0 + (one ? 0.0 : 5.0);
+        four.us = one ? (four.split == 2 ? 5.6 + 0.6 * k : 3.5 + 0.64 * k + 0.1 * sixteens)
+                      : four.split == 0 ? 4.9 + 0.87 * k - 0.22 * sixteens : four.split == 1 ? 1.7 + 0.83 * k + 1.37 * sixteens : 6.1 + 0.96 * k - 0.86 * sixteens;
+    }
+    // Of short launches the estimates are not good enough to tell a few per cent, and units of four slices are the faster ones nearly always.
+    const bool two = four.Nt == 0 || best.us * (!one ? 1.1 : best.us < 35.0 ? 1.15 : 1.0) <= four.us;
+    best.model = four.Nt == 0 ? best.us : std::min(four.model, best.us);
+    return two ? best : four;
 }
 
 // X as planes of rows of K values (one plane: two dimensions); a box is 64 values of box_rows rows of every plane
@@ -407,11 +442,11 @@ int encode_rows_map(CUtensorMap* map, const void* base, bool bf16, int k, int ro
     return TLLM_OK;
 }
 
-// bit tiles as rows = groups of sixteen columns of KB * 64 words; a box is a unit: eight groups x four slices
-int encode_bits_map(CUtensorMap* map, const void* bits, int n_tiles, int kb) {
+// bit tiles as rows = groups of sixteen columns of KB * 64 words; a box is a unit: eight groups x two or four slices
+int encode_bits_map(CUtensorMap* map, const void* bits, int n_tiles, int kb, int slices) {
     const cuuint64_t dims[2] = {(cuuint64_t)kb * 64, (cuuint64_t)n_tiles * 8};
     const cuuint64_t strides[1] = {(cuuint64_t)kb * 256};
-    const cuuint32_t box[2] = {MM_UK * 64, 8}, estr[2] = {1, 1};
+    const cuuint32_t box[2] = {(cuuint32_t)slices * 64, 8}, estr[2] = {1, 1};
     const CUresult cr = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(bits), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fail(TLLM_ERR_CUDA, "cuTensorMapEncodeTiled (bit tiles) failed with code %d", (int)cr);
@@ -468,10 +503,11 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     p.counters = w.counters;
     p.status = w.status;
     p.M = rows, p.K = w.inners, p.N = w.columns;
-    p.KB = w.kb, p.KBU = (p.KB + MM_UK - 1) / MM_UK;
+    const int uk = plan.units4 ? MS_UK : MM_UK;
+    p.KB = w.kb, p.KBU = (p.KB + uk - 1) / uk;
     p.n_tiles = w.n_tiles, p.m_tiles = plan.m_tiles, p.Nt = plan.Nt, p.split = plan.split, p.cluster = plan.cluster;
     p.P = x.planes;
-    p.leg = x.planes > 1 ? MM_LEG : 1 << 24;
+    p.leg = x.planes > 1 ? (plan.units4 ? MS_LEG : MM_LEG) : 1 << 24;
     p.epilogue = o.epilogue, p.y_ld = o.ld, p.plane_y = o.plane;
     p.y_step_n = o.col_major ? o.ld : 1, p.y_step_m = o.col_major ? 1 : o.ld;
     p.out = o.planes ? MM_OUT_PLANES : o.dtype == TLLM_F32 ? MM_OUT_F32 : o.dtype == TLLM_I32 ? MM_OUT_I32 : o.dtype == TLLM_F16 ? MM_OUT_F16 : MM_OUT_BF16;
@@ -480,7 +516,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
         if (wide && o.col_major && (uintptr_t)o.Y % 16 == 0 && o.ld % 4 == 0) p.out = o.dtype == TLLM_F32 ? MM_OUT_F32_COL4 : MM_OUT_I32_COL4;
         if (!wide && !o.col_major && (uintptr_t)o.Y % 4 == 0 && o.ld % 2 == 0 && w.columns % MM_TILE_N == 0) p.out += MM_OUT_F16_PAIRS - MM_OUT_F16;
     }
-    const int cg = plan.cg, b_unit = x.planes * p.Nt / cg * 128 * MM_UK, other = mm_other_bytes(p.Nt, x.planes, p.cluster);
+    const int cg = plan.cg, b_unit = x.planes * p.Nt / cg * 128 * uk, other = mm_other_bytes(p.Nt, x.planes, p.cluster, plan.units4);
     p.SB = std::min(MM_MAX_STAGES, (MM_SMEM - other) / b_unit);
     p.mul4 = 4, p.mul16 = 16;
     const uint32_t fmt = x.bf16 ? 1u : 0u;
@@ -498,15 +534,15 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     if (rc) return rc;
     const size_t smem = (size_t)other + (size_t)p.SB * b_unit;
     if (smem > MM_SMEM || p.SB < 2) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
-    auto kern = cg == 2 ? mma_spmm_kernel<2> : mma_spmm_kernel<1>;
-    static std::once_flag once[2][64];
+    const MmKernel kern = mm_kernel(cg, plan.units4);
+    static std::once_flag once[3][64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[cg - 1][w.device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
+    std::call_once(once[plan.units4 ? 2 : cg - 1][w.device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
     CU_TRY(err);
     // never more blocks than items: the hand-over between the blocks that share a tile counts on every block in a
     // tile's range of owners holding at least one unit of it
     const long long items = (long long)((p.n_tiles + cg - 1) / cg) * p.m_tiles * (p.split == 1 ? p.KBU : p.cluster);
-    const long long most = cg == 2 ? mm_clusters(2, 2, w.sms, w.device) : w.sms;
+    const long long most = cg == 2 ? mm_clusters(2, 2, false, w.sms, w.device) : w.sms;
     const int grid = (int)std::min(items, most) * cg;
     Workspace ws;
     if ((p.Nt <= MM_OWN_NT && w.partial) || p.split != 1) p.partial = w.partial;
@@ -517,7 +553,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(MM_THREADS);
+    cfg.blockDim = dim3(plan.units4 ? MS_THREADS : MM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[2] = {};
@@ -530,7 +566,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     }
     cfg.attrs = at;
     cfg.numAttrs = (unsigned)n_at;
-    CU_TRY(cudaLaunchKernelEx(&cfg, kern, map, *w.map, p));
+    CU_TRY(cudaLaunchKernelEx(&cfg, kern, map, w.map[plan.units4 ? 1 : 0], p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
     return TLLM_OK;
@@ -808,8 +844,8 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
     return TLLM_OK;
 }
 
-// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: 3.1 us of start-up, or 4.9 behind the kernel
-// that makes planes, and the plan's clocks at 1.85 GHz.
+// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: the plan's, and 5 us for one plane that has to be
+// made first.
 double bt_model_us(int inners, int columns, int sms, int x_dtype, BitsAccess access, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
@@ -820,7 +856,7 @@ double mm_tiles_model_us(int inners, int columns, int sms, int device, bool dire
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).clocks / 1850.0 + (direct ? 3.1 : 4.9);
+        t += mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).model + (direct || planes > 1 ? 0.0 : 5.0);
     return t;
 }
 // which of the two: true = decode in registers
@@ -1003,7 +1039,8 @@ int upload_bit_tiles(tllm_weight* w, const std::vector<uint32_t>& bits, int sms)
     CU_TRY(cudaMalloc(&w->d_bits, w->bits_bytes));
     CU_TRY(cudaMemcpy(w->d_bits, bits.data(), w->bits_bytes, cudaMemcpyHostToDevice));
     if (tensor_map_encoder() != nullptr) {
-        const int rc = encode_bits_map(&w->bits_map, w->d_bits, w->mm_n_tiles, w->mm_kb);
+        int rc = encode_bits_map(&w->bits_map[0], w->d_bits, w->mm_n_tiles, w->mm_kb, MM_UK);
+        if (!rc) rc = encode_bits_map(&w->bits_map[1], w->d_bits, w->mm_n_tiles, w->mm_kb, MS_UK);
         if (rc) return rc;
     }
     const size_t partial_bytes = (size_t)2 * sms * MM_TILE_N * MM_OWN_NT * sizeof(float);
@@ -1144,10 +1181,11 @@ int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, 
     cfg.numAttrs = 1;
     CU_TRY(cudaLaunchKernelEx(&cfg, lists_to_bits_kernel, row_idx, col_off, bits, counters, (int)counter_words, flags, columns, inners, tile_k, kb));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    CUtensorMap map;
-    rc = encode_bits_map(&map, bits, n_tiles, kb);
+    CUtensorMap map[2];
+    rc = encode_bits_map(&map[0], bits, n_tiles, kb, MM_UK);
+    if (!rc) rc = encode_bits_map(&map[1], bits, n_tiles, kb, MS_UK);
     if (rc) return rc;
-    BitsView view{(const uint4*)bits, &map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, true, true};
+    BitsView view{(const uint4*)bits, map, inners, columns, n_tiles, kb, sms, dev, nullptr, counters, flags + groups, true, true};
     const size_t xe = dtype_size(x_dtype), ye = dtype_size(y_dtype);
     const bool one = x_layout == TLLM_ROW_MAJOR && (long long)batch * rows <= 0x7fffffffLL;      // the batch is contiguous: one product
     const int parts = one ? 1 : batch, m = one ? batch * rows : rows, x_ld = x_layout == TLLM_ROW_MAJOR ? inners : rows;

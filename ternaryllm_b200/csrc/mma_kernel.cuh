@@ -17,12 +17,14 @@
 // of 2048 x 2048); D's planes are added in the epilogue, the small ones first.  (The tensor core truncates its sums: with the
 // planes in one accumulator every step would cut bits, 1e-5 of the result at K = 4096 against 1e-7.)
 //
-// One persistent block per SM, alone or as one of a pair, twenty-three warps:
+// One persistent block per SM, alone or as one of a pair, twenty-seven warps (and one that has nothing to do):
 //   warp 0        streams this block's range of bit tiles into a shared-memory ring (TMA, one thread)
 //   warp 1        owns tensor memory and issues tcgen05.mma (one thread; a pair's second block has none)
-//   warps 2..5    epilogue: tensor memory -> registers -> Y (or partial sums)
-//   warp 6        loads the activation slices by TMA (one thread)
-//   warps 7..22   decoders: bit tile -> tensor memory, one slice of 32 columns per warp and second unit (a warp can only write the 32
+//   warp 2        loads the activation slices by TMA (one thread)
+//   warps 4..11   epilogue: tensor memory -> registers -> Y (or partial sums), four warps for every other sixteen rows (one warp per
+//                 scheduler waits most of its time: 1700 clocks for sixteen rows of three planes, 780 of one; fp32 MLP module of 256 rows,
+//                 2048 / 8192: 84 us with four warps, 74 with eight)
+//   warps 12..27  decoders: bit tile -> tensor memory, one slice of 32 columns per warp and second unit (a warp can only write the 32
 //                 lanes of tensor memory that its number modulo 4 selects)
 // A unit is two consecutive slices of K.  What bounds a launch of many tiles is that the tensor core is never without an MMA:
 //   * one thread issues (13 clocks an MMA), and it finds the next unit's operands ready: A has a ring of two or four units in tensor memory
@@ -65,7 +67,7 @@ namespace tllm {
 // rounded to nearest are off by 7e-8.  The sums of fp32 activations therefore leave the accumulators after every 64 MMAs and
 // are added up in fp32: 8e-8.
 #define MM_LEG 8
-#define MM_THREADS (23 * 32)
+#define MM_THREADS (28 * 32)
 #define MM_MAX_COLS 192               // columns of D of a tile = planes * Nt, Nt (activation rows) a multiple of sixteen
 #define MM_OWN_NT 64                  // a handle's own hand-over scratch is for tiles of up to this many rows
 #define MM_MAX_M_TILES 16             // row tiles of one launch
@@ -187,20 +189,22 @@ __device__ __forceinline__ void mm_load16(uint32_t at, int nt, int planes, float
 #pragma unroll
         for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]);
     } else {
-        float g[16], h[16];
+        float g[16];
         asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%48];\n\t"
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%49];\n\t"
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%50];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
             "tcgen05.wait::ld.sync.aligned;"
-            : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]), "=f"(f[8]), "=f"(f[9]), "=f"(f[10]), "=f"(f[11]),
-              "=f"(f[12]), "=f"(f[13]), "=f"(f[14]), "=f"(f[15]), "=f"(g[0]), "=f"(g[1]), "=f"(g[2]), "=f"(g[3]), "=f"(g[4]), "=f"(g[5]), "=f"(g[6]), "=f"(g[7]),
-              "=f"(g[8]), "=f"(g[9]), "=f"(g[10]), "=f"(g[11]), "=f"(g[12]), "=f"(g[13]), "=f"(g[14]), "=f"(g[15]), "=f"(h[0]), "=f"(h[1]), "=f"(h[2]), "=f"(h[3]),
-              "=f"(h[4]), "=f"(h[5]), "=f"(h[6]), "=f"(h[7]), "=f"(h[8]), "=f"(h[9]), "=f"(h[10]), "=f"(h[11]), "=f"(h[12]), "=f"(h[13]), "=f"(h[14]), "=f"(h[15])
-            : "r"(at), "r"(at + (uint32_t)nt), "r"(at + (uint32_t)(2 * nt))
+            : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]), "=f"(f[8]), "=f"(f[9]), "=f"(f[10]),
+              "=f"(f[11]), "=f"(f[12]), "=f"(f[13]), "=f"(f[14]), "=f"(f[15]), "=f"(g[0]), "=f"(g[1]), "=f"(g[2]), "=f"(g[3]), "=f"(g[4]), "=f"(g[5]),
+              "=f"(g[6]), "=f"(g[7]), "=f"(g[8]), "=f"(g[9]), "=f"(g[10]), "=f"(g[11]), "=f"(g[12]), "=f"(g[13]), "=f"(g[14]), "=f"(g[15])
+            : "r"(at + (uint32_t)nt), "r"(at + (uint32_t)(2 * nt))
             : "memory");
 #pragma unroll
-        for (int t = 0; t < 16; ++t) f[t] += g[t] + h[t];
+        for (int t = 0; t < 16; ++t) f[t] += g[t];
+        uint32_t v[16];                                       // (not with the other two: forty-eight registers at a time were too many)
+        tmem_ld16(at, v);
+#pragma unroll
+        for (int t = 0; t < 16; ++t) f[t] = __uint_as_float(v[t]) + f[t];
     }
 }
 // the sum of the legs so far: sixteen values of this thread, 512 bytes apart in shared memory
@@ -570,7 +574,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     // other three are multiplied (5120 x 15360, 2048 rows in tiles of 192: 198 us, 227 with one pair of barriers a unit); with four places
     // there is time enough, and fewer barriers are faster (2048 x 8192, 32 rows: 8.8 us against 9.6).
     const uint32_t fine = a_log == 1u ? 1u : 0u;
-    volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 56);   // [0] tensor-memory address, [1] abort
+    volatile int* flags = (volatile int*)(mm_smem + (bar_base - raw0) + 8 * 60);   // [0] tensor-memory address, [1] abort
     volatile int* abort_flag = flags + 1;
 #define A_FULL(s) (bar_base + 8u * (uint32_t)(s))
 #define A_EMPTY(s) (bar_base + 8u * (8u + (uint32_t)(s)))
@@ -593,9 +597,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(ACC_FULL(a), 1);
-            mbar_init(ACC_EMPTY(a), 4 * CG);    // the four epilogue warps
+            mbar_init(ACC_EMPTY(a), 8 * CG);    // the epilogue warps
         }
-        for (int q = 0; q < 4; ++q) mbar_init(PART_FULL(q), (uint32_t)max(C - 1, 1));   // the same warp of the other blocks
+        for (int q = 0; q < 8; ++q) mbar_init(PART_FULL(q), (uint32_t)max(C - 1, 1));   // the same warp of the other blocks
         flags[0] = 0;
         flags[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -632,7 +636,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 }
             }
         }
-    } else if (warp == 6) {
+    } else if (warp == 2) {
         // ---- activation producer: a unit is two TMA boxes (all planes of a slice each) on one barrier
         if (elect_one()) {
             pdl_wait();
@@ -703,12 +707,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 }
             }
         }
-    } else if (warp >= 7) {
+    } else if (warp >= 12) {
         // ---- decoders: eight warps take the even units and eight the odd ones, and a warp expands 32 columns of W of one slice into its 32
         // lanes of tensor memory.  Lane 4g + u holds column 16 * (u >> 1) + 8 * (u & 1) + g of them (see mm_column).  The values are in
         // registers before the place in the ring is free: from there on they are a store away.
-        const int q = warp & 3, h = ((warp - 7) >> 2) & 1;
-        const uint32_t mine = (uint32_t)(warp - 7) >> 3;
+        const int q = warp & 3, h = ((warp - 12) >> 2) & 1;
+        const uint32_t mine = (uint32_t)(warp - 12) >> 3;
         const uint32_t g = (uint32_t)lane >> 2, u = (uint32_t)lane & 3u;
         const uint32_t raw_lane = r_base + (uint32_t)(2 * q + (u >> 1)) * 512u;
         const uint32_t a_lane = a_base + ((uint32_t)(q * 32) << 16) + (uint32_t)h * 32u;
@@ -755,9 +759,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 }
             }
         }
-    } else {
-        // ---- epilogue (warps 2..5): a warp may read the 32 tensor-memory lanes selected by warp % 4
-        const int q = warp & 3, nl = q * 32 + lane, ncol = q * 32 + mm_column(lane);
+    } else if (warp >= 4) {
+        // ---- epilogue: a warp may read the 32 tensor-memory lanes selected by warp % 4; of the sixteens of rows it has every other one (of
+        // those that a block of a cluster writes, too)
+        const int q = warp & 3, odd = (warp >> 2) - 1, nl = q * 32 + lane, ncol = q * 32 + mm_column(lane);
         pdl_wait();
         uint32_t a = 0, aph = 0;
         const auto acc_free = [&](uint32_t bar) {
@@ -777,7 +782,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             for (int left = ub - ua; left > p.leg; left -= p.leg) {
                 MM_WAIT(ACC_FULL(a), aph);
                 tc_fence_after();
-                for (int c16 = 0; c16 < Nt; c16 += 16) {
+                for (int c16 = 16 * odd; c16 < Nt; c16 += 32) {
                     float f[16];
                     mm_load16(lanes + a * acc_cols + column(c16), rows, p.P, f);
                     if (legs) mm_add_run(run + (uint32_t)c16 * 512u, f);
@@ -817,7 +822,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 const int sixteens = Nt / 16, own = (sixteens + C - 1) / C;
                 for (int c = 0; c < sixteens; ++c) {
                     const int o = c % C;
-                    if (o == rank) continue;
+                    if (o == rank || ((c / C) & 1) != odd) continue;
                     float f[16];
                     load16(16 * c, f);
                     const uint32_t to = mm_peer(part_base + (uint32_t)(((rank * own + c / C) * 4) * 128 + nl) * 16u, (uint32_t)o);
@@ -825,13 +830,13 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     for (int t = 0; t < 4; ++t) mm_st_peer(to + (uint32_t)t * 2048u, f[4 * t], f[4 * t + 1], f[4 * t + 2], f[4 * t + 3]);
                 }
                 __syncwarp();
-                if (lane < C && lane != rank && lane < sixteens) mm_arrive_peer(mm_peer(PART_FULL(q), (uint32_t)lane));
+                if (lane < C && lane != rank && lane < sixteens) mm_arrive_peer(mm_peer(PART_FULL(4 * odd + q), (uint32_t)lane));
                 if (rank < sixteens) {
-                    MM_WAIT(PART_FULL(q), 0u);
+                    MM_WAIT(PART_FULL(4 * odd + q), 0u);
                     asm volatile("fence.acq_rel.cluster;" ::: "memory");
                     mm_with_out(p, [&](auto out, auto silu) {
-                        uint32_t at0 = part_base + (uint32_t)nl * 16u;
-                        for (int c = rank; c < sixteens; c += C, at0 += 8192u) {
+                        uint32_t at0 = part_base + (uint32_t)nl * 16u + (uint32_t)odd * 8192u;
+                        for (int c = rank + odd * C; c < sixteens; c += 2 * C, at0 += 16384u) {
                             float f[16];
                             load16(16 * c, f);                          // its own part, then the others in block order
                             uint32_t at = at0;
@@ -856,11 +861,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 cf = (int)(((first_unit + 1) * G + total - 1) / total - 1), cl = (int)(((last_unit + 1) * G + total - 1) / total - 1);
                 unsigned int* ctr = p.counters + ((size_t)nt * p.m_tiles + mt) * 4 + q;
                 const unsigned int others = (unsigned int)(cl - cf);
+                const uint32_t field = 16u * (uint32_t)odd;      // the two warps of a column count in halves of one word
                 unsigned int there = 0;
                 if (lane == 0) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(there) : "l"(ctr) : "memory");
-                sum = __shfl_sync(0xffffffffu, there, 0) == others;
+                sum = (__shfl_sync(0xffffffffu, there, 0) >> field & 0xFFFFu) == others;
                 if (!sum) {
-                    for (int c16 = 0; c16 < Nt; c16 += 16) {
+                    for (int c16 = 16 * odd; c16 < Nt; c16 += 32) {
                         float f[16];
                         load16(c16, f);
 #pragma unroll
@@ -868,11 +874,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     }
                     __threadfence();
                     __syncwarp();
-                    if (lane == 0) there = atomicAdd(ctr, 1u);
-                    sum = __shfl_sync(0xffffffffu, there, 0) == others;
+                    if (lane == 0) there = atomicAdd(ctr, 1u << field);
+                    sum = (__shfl_sync(0xffffffffu, there, 0) >> field & 0xFFFFu) == others;
                 }
                 if (sum) {
-                    if (lane == 0) *ctr = 0;
+                    if (lane == 0) atomicAnd(ctr, ~(0xFFFFu << field));
                     __threadfence();
                 }
             }
@@ -881,7 +887,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 const float* part0 = p.partial + (size_t)(2 * (cf * CG + member) + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * ((cf + 1) * CG + member)) * slot_floats + nl * 4;
                 mm_with_out(p, [&](auto out, auto silu) {
-                    for (int c16 = 0; c16 < Nt; c16 += 16) {
+                    for (int c16 = 16 * odd; c16 < Nt; c16 += 32) {
                         float f[16];
                         if (full) load16(c16, f);
                         else {
@@ -935,9 +941,6 @@ done:
 #undef ACC_EMPTY
 #undef PART_FULL
 }
-#undef MM_WAIT
-#undef MM_SPIN
-#undef MM_ADVANCE
 
 // ---- activations as planes of 16-bit values for the kernel above: rows of k_pad values, zero beyond K ------------------
 struct StageParams {
