@@ -93,7 +93,7 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
     const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
     const bool f32 = x_dtype == TLLM_F32, i8 = x_dtype == TLLM_I8;
-    double step = f32 ? q.nb * (0.6 + 0.18 * q.gr) : !i8 || access != BITS_ROWS16 ? 0.25 + q.nb * (0.15 + 0.2 * q.gr) : q.nb == 4 ? 1.15 : 0.1 + q.nb * (0.02 + 0.16 * q.gr);
+    double step = f32 ? q.nb * (0.6 + 0.18 * q.gr) : !i8 || access != BITS_ROWS16 ? 0.25 + q.nb * (0.15 + 0.2 * q.gr) : q.nb == 4 ? 1.3 : 0.1 + q.nb * (0.02 + 0.16 * q.gr);
     const double groups = (columns + 15) / 16;               // of few columns few blocks read X
     if (access == BITS_ROWS) step += std::min(1.0, 0.6 + groups / 256) * (f32 ? 0.6 + 0.23 * rows : i8 ? 0.7 + 0.055 * rows : 0.35 + 0.15 * rows);
     else if (access == BITS_COLUMNS)

@@ -372,13 +372,19 @@ int mm_clusters(int cluster, int cg, bool units4, int sms, int device) {
     return n;
 }
 int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
-MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
+// asked: false where the device did not say how many clusters fit
+MmPlan mm_make_plan(int rows, int planes, int n_tiles, int kb, int sms, int device, bool* asked) {
+    const auto clusters = [&](int c, int cg, bool units4) {
+        const int n = mm_clusters(c, cg, units4, sms, device);
+        if (n == 0) *asked = false;
+        return n;
+    };
     MmPlan best{0, 0, 0, 1, 1, false, 0, 0};
     const bool one = planes == 1;
     const auto take = [&](int nt, int mt, int split, int c, int cg, double us) {
         if (best.Nt == 0 || us < best.us) best = MmPlan{nt, mt, split, c, cg, false, us, us};
     };
-    const int kbu = (kb + MM_UK - 1) / MM_UK, kbu4 = (kb + MS_UK - 1) / MS_UK, pairs = n_tiles > 1 ? mm_clusters(2, 2, false, sms, device) : 0;
+    const int kbu = (kb + MM_UK - 1) / MM_UK, kbu4 = (kb + MS_UK - 1) / MS_UK, pairs = n_tiles > 1 ? clusters(2, 2, false) : 0;
     MmPlan four{0, 0, 0, 1, 1, true, 0, 0};          // us: clocks, until the loop is done
     for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
         const int mt = (rows + nt - 1) / nt, cols = planes * nt, sixteens = nt / 16, turns = (sixteens + 1) / 2;     // turns: sixteens of an epilogue warp
@@ -395,7 +401,7 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
             const double blocks = std::min(units, groups), parts = std::min((double)kbu, blocks / tiles + 1.0);
             take(nt, mt, 1, 1, cg, us(extra + std::ceil(units / blocks) * unit + 4900.0 + (one ? 2.7 : 3.1) * epilogue + turns * 630.0 * (parts - 1) + crowd(blocks * cg)));
             for (int c = 2; cg == 1 && c <= 8 && c <= kbu; c *= 2) {
-                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols * 128 * MM_UK || mm_clusters(c, 1, false, sms, device) < tiles) continue;
+                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols * 128 * MM_UK || clusters(c, 1, false) < tiles) continue;
                 take(nt, mt, 2, c, 1, us((kbu + c - 1) / c * unit + 3400.0 + sixteens * 600.0 + ((sixteens + c - 1) / c + 1) / 2 * piece + crowd(tiles * c)));
             }
         }
@@ -412,7 +418,7 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu4, blocks / tiles + 1.0);
         take4(1, 1, crowd4(blocks) + std::ceil(units / blocks) * MS_UK * slice + legs4(std::min(units / blocks, (double)kbu4)) + 3000.0 + 3 * epilogue4 + sixteens * 1000.0 * (parts - 1));
         for (int c = 2; c <= 8 && c <= kbu4; c *= 2) {
-            if (MM_SMEM - mm_other_bytes(nt, planes, c, true) < 2 * cols * 128 * MS_UK || mm_clusters(c, 1, true, sms, device) < tiles) continue;
+            if (MM_SMEM - mm_other_bytes(nt, planes, c, true) < 2 * cols * 128 * MS_UK || clusters(c, 1, true) < tiles) continue;
             take4(2, c, (kbu4 + c - 1) / c * MS_UK * slice + legs4((kbu4 + c - 1) / c) + 2000.0 + sixteens * 100.0 + (sixteens + c - 1) / c * 350.0 + crowd4(tiles * c));
         }
         if (nt >= rows) break;
@@ -427,6 +433,21 @@ MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
     const bool two = four.Nt == 0 || best.us * (!one ? 1.1 : best.us < 35.0 ? 1.15 : 1.0) <= four.us;
     best.model = four.Nt == 0 ? best.us : std::min(four.model, best.us);
     return two ? best : four;
+}
+// The plan depends on these sizes alone; a thread keeps those of the last sizes it asked for (making one takes 0.1 to 1 us of a call that takes 4).
+MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
+    struct Known {
+        int rows, planes, n_tiles, kb, sms, device;
+        MmPlan plan;
+    };
+    static thread_local Known known[64];
+    const uint32_t h = ((uint32_t)rows * 31u + (uint32_t)n_tiles) * 31u + (uint32_t)kb * 4u + (uint32_t)planes;
+    Known& e = known[(h * 2654435761u) >> 26];
+    if (e.rows == rows && e.planes == planes && e.n_tiles == n_tiles && e.kb == kb && e.sms == sms && e.device == device) return e.plan;
+    bool asked = true;
+    const MmPlan plan = mm_make_plan(rows, planes, n_tiles, kb, sms, device, &asked);
+    if (asked) e = Known{rows, planes, n_tiles, kb, sms, device, plan};
+    return plan;
 }
 
 // X as planes of rows of K values (one plane: two dimensions); a box is 64 values of box_rows rows of every plane
@@ -845,7 +866,7 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
 }
 
 // Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: the plan's, and 5 us for one plane that has to be
-// made first.
+// made first (of int8 3.5: 64 rows of 4096 x 4096 take 11.7 us there, 14.3 in two launches of the register decoder).
 double bt_model_us(int inners, int columns, int sms, int x_dtype, BitsAccess access, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
@@ -856,7 +877,7 @@ double mm_tiles_model_us(int inners, int columns, int sms, int device, bool dire
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).model + (direct || planes > 1 ? 0.0 : 5.0);
+        t += mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).model + (direct || planes > 1 ? 0.0 : x_dtype == TLLM_I8 ? 3.5 : 5.0);
     return t;
 }
 // which of the two: true = decode in registers
