@@ -244,6 +244,11 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     // The tensor core cuts bits off its running sum at every MMA: fp32 sums leave it after the eight of a pair of slices (gate and up of a
     // 2560 / 6912 MLP, 8 rows, h = silu(gate) * up: off by 1.4e-7 with a warp's 40 MMAs in one sum, 1.1e-7 now).
     constexpr bool PARTS = XT == TLLM_F32;
+    // Whether a result's address is computed before its sum is looked at.  It decides how ptxas allots the registers of the whole kernel (64 of them
+    // in most instances), and so the time of every call.  Computed late: 2048 x 2048, eight rows of fp16 2.61 us (early 3.15), of fp32 4.41
+    // (4.49); 1003 x 517, three rows of bf16 2.62 (2.77).  Early: 8192 x 10240, one row of bf16 10.3 us (late 10.6); 4096 x 11008, eight of fp16
+    // 6.89 (6.98).
+    constexpr bool EARLY = GR == 3 && ASYNC && Act::E == 2;
     constexpr int CPR = 8 * Act::E, RPI = 32 / CPR, KPC = 16 / Act::E;     // chunks per row (and pair of slices), rows per warp copy, values per chunk
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
@@ -452,16 +457,18 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                     for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
             }
             const int n = (c0 + q0 + j) * 16 + c;
-            const size_t at = (size_t)m * p.y_step_m + (size_t)n * p.y_step_n;
+            const auto address = [&] { return (size_t)m * p.y_step_m + (size_t)n * p.y_step_n; };
             if constexpr (I8) {                                      // an exact multiple of 64
-                if (valid && n < p.N) ((int*)p.Y)[at] = v >> 6;
+                if (valid && n < p.N) ((int*)p.Y)[address()] = v >> 6;
                 continue;
             }
+            size_t at = 0;
+            if constexpr (EARLY) at = address();
             const float sc = p.epilogue && (c & 1) ? p.scale2 : p.scale;
             float y = v * sc;
             if (__builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
             if (p.epilogue == 0) {
-                if (valid && n < p.N) store_out(p.Y, p.y_dtype, at, y);
+                if (valid && n < p.N) store_out(p.Y, p.y_dtype, EARLY ? at : address(), y);
             } else {
                 const float u = __shfl_xor_sync(0xffffffffu, y, 1);
                 if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(y, u));
