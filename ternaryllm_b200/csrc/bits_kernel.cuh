@@ -254,8 +254,9 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
     const int KB = p.KB, KP = (KB + 1) >> 1, D = p.depth, S = p.slots, M = p.M, SL = p.split_log;
     // Which share of the columns: the shares may differ by a group, and every scheduler (warp modulo 4) gets some of each, so that none has
-    // all of the larger ones (8192 x 10240, one row: 10.95 us, 11.83 with share = warp modulo shares; 4096 x 11008 6.5 and 6.9).
-    const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = (SL == 1 ? warp ^ (warp >> 2) : warp + (warp >> 2)) & ((1 << SL) - 1);
+    // all of the larger ones (8192 x 10240, one row of bf16: 10.2 us, 11.5 with share = warp modulo shares; 4096 x 11008, fp16 6.0 and 6.5).  One
+    // expression for two and for four shares: with a choice between two every call got slower (2048 x 8192, eight rows of fp32 8.03 us, 7.85 now).
+    const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = (warp + (warp >> 2)) & ((1 << SL) - 1);
     const int np = kw < KP ? (KP - kw + kstep - 1) >> klog : 0;      // pairs of this warp: kw, kw + kstep, ...
     const uint32_t ring = smem_u32(bt_smem) + (uint32_t)warp * (uint32_t)S * p.slot_bytes;
     Sum* red = (Sum*)(bt_smem + (size_t)BT_WARPS * S * p.slot_bytes);          // [warp][group][column of B][20] partial sums
