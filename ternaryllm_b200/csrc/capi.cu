@@ -539,6 +539,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     }
     const int cg = plan.cg, b_unit = x.planes * p.Nt / cg * 128 * uk, other = mm_other_bytes(p.Nt, x.planes, p.cluster, plan.units4);
     p.SB = std::min(MM_MAX_STAGES, (MM_SMEM - other) / b_unit);
+    p.R = MS_RAW_UNITS;
     p.mul4 = 4, p.mul16 = 16;
     const uint32_t fmt = x.bf16 ? 1u : 0u;
     // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B formats (bits 7-9, 10-12), both K-major,

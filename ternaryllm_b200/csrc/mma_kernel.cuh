@@ -101,6 +101,7 @@ struct MmParams {
     long long y_step_n, y_step_m;   // elements from column to column and from row to row (epilogue 0)
     long long plane_y;        // MM_OUT_PLANES: elements from plane to plane
     int SB;                   // ring length: units of B
+    int R;                    // mma_units4_kernel: ring length, units of bit tiles (MS_RAW_UNITS)
     int leg;                  // units that are summed in the tensor core before the sum goes on in fp32 (MM_LEG)
     uint32_t idesc;           // tcgen05 instruction descriptor
     uint32_t mul4, mul16;     // 4 and 16

@@ -86,7 +86,9 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
     // ---- shared memory ---------------------------------------------------------------------------------
     const uint32_t raw0 = smem_u32(mm_smem);
     const uint32_t base = (raw0 + 1023u) & ~1023u;                 // swizzled tiles need 1024-byte alignment
-    const uint32_t SB = (uint32_t)p.SB, R = MS_RAW_UNITS;
+    // The length of the ring of bit tiles is a parameter: as a constant ptxas allots other registers, and stores of results get slower (998 rows of
+    // int8 on 320 x 7296 20.5 us, 19.5 so; 500 rows of fp32 on 312 x 12480 31.3 and 28.7; 192 rows of fp16 on 4096 x 4096 13.9 and 13.6).
+    const uint32_t SB = (uint32_t)p.SB, R = (uint32_t)p.R;
     const int Nt = p.Nt;
     const uint32_t acc_cols = (uint32_t)(p.P * Nt), b_slice = acc_cols * 128u, b_unit = MS_UK * b_slice;
     const uint32_t b_base = base, r_base = b_base + SB * b_unit;
