@@ -84,21 +84,32 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 }
 }  // namespace
 
-// Microseconds of a launch: a chain of 2 us, and per pair of slices that a warp goes through what it takes sixteen warps to fetch and
-// turn the activations and to decode and multiply the columns, more of it where the activations are fetched once a pass.  Measured at 1 to 16 rows of 2048 x 2048 .. 8192 x 10240.
-// Activations that cp.async cannot read pass through registers with every pair, and the blocks wait for them: 2.7 us a pair where 16 rows of
-// fp16 start anywhere (bytes 1.6, 8 rows of fp32 2.4), and element by element from a column-major X, by all blocks
-// from the same lines (16 rows of fp16, 4096 x 11008: 227 us; the batched kernel behind its planes 18.5).  Measured over the
-// same sizes, 1 to 16 rows.
+// Microseconds of a launch: its start, more of it the more of the sixteen warps have work; per pair of slices that a warp goes through what it takes
+// sixteen warps to fetch and turn the activations and to decode and multiply the columns, more of it where the activations are fetched once a
+// pass; and the results.  Fitted to 5000 launches on 100 weights from 256 x 256 to 8192 x 10240, 1 to 64 rows: 4 to 7 % off in the mean.  A column-major
+// X is read element by element, by all blocks from the same lines (16 rows of fp16, 4096 x 11008: 227 us; the batched kernel behind its planes
+// 18.5), less where a short K leaves warps without work; what that takes depends on the addresses more than on anything here: 20 % off.
 double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
+    struct Cost {
+        double start, warps, step, nb, nb_gr, fetch, row, few, results;     // few: share of fetch and row where blocks are few, at least
+    };
+    static const Cost costs[3][3] = {       // fp32, 16 bits, int8; rows on 16 bytes, rows, columns
+        {{0.8, 1.5, 0.95, 0.08, 0.18, 0, 0, 0, 0}, {0.75, 1.6, 0.5, 0.2, 0.11, 0.42, 0.325, 0.74, 0.14}, {0.5, 1.8, 0, 0, 0.2, 0, 1.4, 0.5, 1.08}},
+        {{1.2, 0.6, 0.53, 0, 0.18, 0, 0, 0, 0.075}, {1.2, 0.75, 0.26, 0, 0.13, 0.56, 0.147, 0.73, 0.18}, {0.5, 0.4, 0.7, 0.14, 0.19, 4.3, 0.46, 0.34, 0.82}},
+        {{1.3, 0.4, 0.44, 0, 0.1, 0, 0, 0, 0.053}, {1.2, 0.9, 0.06, 0.11, 0.07, 0.7, 0.062, 0.68, 0.19}, {0.5, 0, 0, 1.5, 0, 5.1, 0.1, 0.14, 1.2}}};
+    static const double int8_four[3] = {1.02, 0.8, 7.5}, few_rows[3][2] = {{0.75, 1.0}, {0.25, 0.54}, {0.45, 0.48}};     // a step of four blocks of columns of B; columns, up to two and four rows
+    if (access == BITS_COLUMNS && rows == 1) access = BITS_ROWS;             // the same addresses
     const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
-    const bool f32 = x_dtype == TLLM_F32, i8 = x_dtype == TLLM_I8;
-    double step = f32 ? q.nb * (0.6 + 0.18 * q.gr) : !i8 || access != BITS_ROWS16 ? 0.25 + q.nb * (0.15 + 0.2 * q.gr) : q.nb == 4 ? 1.3 : 0.1 + q.nb * (0.02 + 0.16 * q.gr);
-    const double groups = (columns + 15) / 16;               // of few columns few blocks read X
-    if (access == BITS_ROWS) step += std::min(1.0, 0.6 + groups / 256) * (f32 ? 0.6 + 0.23 * rows : i8 ? 0.7 + 0.055 * rows : 0.35 + 0.15 * rows);
-    else if (access == BITS_COLUMNS)
-        step += std::min(1.0, 0.1 + groups / 128) * (i8 ? 1.6 + 0.5 * rows : (f32 ? 1.7 : 1.1) * rows * (rows <= 4 ? 0.65 : 1.0));
-    return 2.0 + q.pairs * (step + (q.passes > 1 ? 0.15 : 0.0));
+    const int type = x_dtype == TLLM_F32 ? 0 : x_dtype == TLLM_I8 ? 2 : 1, kp = (kb + 1) / 2;
+    const Cost& c = costs[type][access];
+    const double groups = (columns + 15) / 16;
+    double step = type == 2 && q.nb == 4 ? int8_four[access] : c.step + q.nb * (c.nb + c.nb_gr * q.gr);
+    if (type == 0 && access == BITS_ROWS16 && q.nb == 3) step += 0.23;
+    double fetch = (c.fetch + c.row * rows) * std::min(1.0, c.few + groups / (access == BITS_COLUMNS ? 128 : 256));
+    if (access == BITS_COLUMNS) fetch *= std::min(1.0, 0.3 + 0.0875 * kp) * (rows <= 2 ? few_rows[type][0] : rows <= 4 ? few_rows[type][1] : 1.0);
+    const double each = (double)kp / (BT_WARPS >> q.split_log);             // pairs of a warp and pass, in the mean
+    const double pairs = q.passes > 1 ? (q.pairs + q.passes * each) / 2 : q.pairs;        // a warp that has one less goes on with the next pass
+    return c.start + c.warps * std::min(1.0, each) + pairs * (step + fetch) + c.results * groups * rows / 1000;
 }
 
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {

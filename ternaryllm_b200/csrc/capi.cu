@@ -321,22 +321,25 @@ struct Workspace {
 };
 
 // How a product of `rows` rows (in `planes` planes) is cut: by which of the two kernels, row tiles of Nt rows each, and whole tiles, equal
-// ranges of units, or a cluster per tile; by one block or by a pair of blocks.  Chosen by estimates, fitted to 1700 plans of 11 weights from
-// 512 x 512 to 5120 x 15360 and 20 to 2048 rows (6 % off in the mean, and the plan that is picked 1.6 % slower than the best).
-// Units of two slices, in SM clocks: eight MMAs of 128 x (planes * Nt) x 16.  With a pair they take little more than their own time, 4.3 a
-// column.  A block by itself takes as long as its shared memory needs to write and read the activations: 630 clocks and 2.4 a column.
-// Neither takes less than the 780 of decoding a unit.  A tile's epilogue is hidden behind the next one where that takes longer.
-// Units of four slices: a slice is four MMAs, 2.5 clocks a column and never less than the 255 of their issue; where there is no room for two
-// sets of accumulators a tile's epilogue and legs are not hidden; the first unit of activations takes 12 clocks a row to arrive.
+// ranges of units, or a cluster per tile; by one block or by a pair of blocks.  Chosen by one estimate of what the call takes, microseconds, the
+// kernel that makes planes included (`staged`: most of the product's start hides behind it); the choice between this product and the other kernels
+// goes by the same figure.  Fitted to 21000 measured plans (100 weights from 256 x 256 to 8192 x 10240, 8 to 2048 rows, one plane and three): 3 % off
+// in the mean.  (Separate estimates for the two choices, fitted to fewer and larger calls, picked plans 2 % slower than the best measured in the
+// mean, now 0.5; 24 rows of fp16 on 1280 x 465 took 7.5 us where units of four slices take 5.7.)  In clocks of 1.85 GHz:
+// Units of two slices: eight MMAs of 128 x (planes * Nt) x 16.  A block by itself takes as long as its shared memory needs to write and read the
+// activations, a pair half of that; neither takes less than the 700 to 780 of decoding a unit.  A tile's epilogue is hidden behind the next one where
+// that takes longer.
+// Units of four slices: a slice never takes less than 250; where there is no room for two sets of accumulators a tile's epilogue and legs are not
+// hidden.
 // In a tile that `parts` blocks share the last one to arrive reads the other parts, a round trip to L2 for every sixteen rows of each.
 // A cluster of C blocks per tile: every block's units, then what goes to the other blocks and the adding-up of its own share.
-// A launch that holds more than half of the SMs keeps the next one's blocks, one to an SM, from starting up beside it.
+// A million results take half a microsecond to store, a million activations as much to turn into planes.
+// A launch that holds more than half of the SMs, or of the clusters that fit, keeps the next one's blocks, one to an SM, from starting up beside it.
 struct MmPlan {
     int Nt, m_tiles, split, cluster;
     int cg;                  // blocks that share a tile's MMAs: 1, or 2 (a pair: 256 columns of W, half of the activations in each block)
     bool units4;             // mma_units4_kernel
     double us;
-    double model;            // for the choice between kernels, whose other side was fitted beside it
 };
 constexpr int MM_SMEM = 227 * 1024;
 // shared memory beside the units of B: bit tiles, barriers, a cluster's parts, the sum of the legs of three planes
@@ -372,81 +375,77 @@ int mm_clusters(int cluster, int cg, bool units4, int sms, int device) {
     return n;
 }
 int mm_max_nt(int planes) { return planes == 1 ? MM_MAX_COLS : MM_MAX_COLS / 3; }
-// asked: false where the device did not say how many clusters fit
-MmPlan mm_make_plan(int rows, int planes, int n_tiles, int kb, int sms, int device, bool* asked) {
+// staged: planes made by the preceding kernel from rows (MM_FROM_ROWS) or columns (MM_FROM_COLUMNS).  asked: false where the device did not say how
+// many clusters fit.
+enum { MM_READY, MM_FROM_ROWS, MM_FROM_COLUMNS };
+MmPlan mm_make_plan(int rows, int planes, int staged, int n_tiles, int kb, int sms, int device, bool* asked) {
     const auto clusters = [&](int c, int cg, bool units4) {
         const int n = mm_clusters(c, cg, units4, sms, device);
         if (n == 0) *asked = false;
         return n;
     };
-    MmPlan best{0, 0, 0, 1, 1, false, 0, 0};
+    MmPlan best{0, 0, 0, 1, 1, false, 0};
     const bool one = planes == 1;
-    const auto take = [&](int nt, int mt, int split, int c, int cg, double us) {
-        if (best.Nt == 0 || us < best.us) best = MmPlan{nt, mt, split, c, cg, false, us, us};
+    const auto take = [&](int nt, int mt, int split, int c, int cg, bool units4, double start, double clocks) {
+        const double us = start + clocks / 1850.0;
+        if (best.Nt == 0 || us < best.us) best = MmPlan{nt, mt, split, c, cg, units4, us};
     };
+    const double crowded = staged == MM_FROM_ROWS ? 900.0 : staged ? 2200.0 : 2500.0;
+    const double results = (double)rows * n_tiles * MM_TILE_N / 1e6, planes_us = staged ? 0.55 * rows * kb * MM_TILE_K / 1e6 : 0.0;
+    const double start2 = (!staged ? 1.3 : one ? 5.1 : 5.2) + 0.6 * results + planes_us, start4 = (!staged ? 1.7 : one ? 5.3 : 5.6) + 0.4 * results + planes_us;
     const int kbu = (kb + MM_UK - 1) / MM_UK, kbu4 = (kb + MS_UK - 1) / MS_UK, pairs = n_tiles > 1 ? clusters(2, 2, false) : 0;
-    MmPlan four{0, 0, 0, 1, 1, true, 0, 0};          // us: clocks, until the loop is done
     for (int nt = 16; nt <= mm_max_nt(planes); nt += 16) {
         const int mt = (rows + nt - 1) / nt, cols = planes * nt, sixteens = nt / 16, turns = (sixteens + 1) / 2;     // turns: sixteens of an epilogue warp
         if (mt > MM_MAX_M_TILES) continue;
         // units of two slices
-        const double piece = one ? 940.0 : 2100.0, epilogue = turns * piece, legs = one ? 0.0 : ((kbu + MM_LEG - 1) / MM_LEG - 1) * turns * 300.0;
-        const auto crowd = [&](double blocks) { return 2 * blocks > sms ? (one ? 2400.0 : 3000.0) : 0.0; };
-        const auto us = [&](double clocks) { return ((one ? 5700.0 : 8900.0) + clocks) / 1850.0; };
+        const double piece = one ? 740.0 : 1240.0, epilogue = 2000.0 + turns * piece, legs = one ? 0.0 : ((kbu + MM_LEG - 1) / MM_LEG - 1) * turns * 2000.0;
+        const auto crowd = [&](double held, double fit) { return 2 * held > fit ? crowded : 0.0; };
         for (int cg = 1; cg <= 2; ++cg) {
             const double groups = cg == 1 ? sms : pairs, tiles = (double)((n_tiles + cg - 1) / cg) * mt, units = tiles * kbu;
             if (groups <= 0 || nt % (16 * cg) != 0) continue;
-            const double unit = std::max(780.0, cg == 1 ? 630.0 + 2.36 * cols : 150.0 + 4.34 * cols), extra = cg == 1 ? 0.0 : 1300.0;
-            take(nt, mt, 0, 1, cg, us(extra + (std::ceil(tiles / groups) - 1) * std::max(kbu * unit, epilogue + legs) + kbu * unit + epilogue + crowd(tiles * cg)));
+            const double unit = cg == 1 ? std::max(706.0, 500.0 + 3.36 * cols) : std::max(780.0, 240.0 + 3.23 * cols), extra = cg == 1 ? 0.0 : 1590.0;
+            take(nt, mt, 0, 1, cg, false, start2, extra + (std::ceil(tiles / groups) - 1) * std::max(kbu * unit, epilogue + legs) + kbu * unit + epilogue + crowd(tiles * cg, sms));
             const double blocks = std::min(units, groups), parts = std::min((double)kbu, blocks / tiles + 1.0);
-            take(nt, mt, 1, 1, cg, us(extra + std::ceil(units / blocks) * unit + 4900.0 + (one ? 2.7 : 3.1) * epilogue + turns * 630.0 * (parts - 1) + crowd(blocks * cg)));
+            take(nt, mt, 1, 1, cg, false, start2, extra + std::ceil(units / blocks) * unit + 7170.0 + turns * (4.4 * piece + 320.0 * (parts - 1)) + crowd(blocks * cg, sms));
             for (int c = 2; cg == 1 && c <= 8 && c <= kbu; c *= 2) {
-                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols * 128 * MM_UK || clusters(c, 1, false) < tiles) continue;
-                take(nt, mt, 2, c, 1, us((kbu + c - 1) / c * unit + 3400.0 + sixteens * 600.0 + ((sixteens + c - 1) / c + 1) / 2 * piece + crowd(tiles * c)));
+                const int fit = clusters(c, 1, false);
+                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols * 128 * MM_UK || fit < tiles) continue;
+                take(nt, mt, 2, c, 1, false, start2, (kbu + c - 1) / c * unit + 6900.0 + sixteens * 400.0 + ((sixteens + c - 1) / c + 1) / 2 * piece + crowd(tiles, fit));
             }
         }
         // units of four slices
         const double tiles = (double)n_tiles * mt, units = tiles * kbu4;
-        const double slice = std::max(255.0, 2.5 * cols), epilogue4 = sixteens * 350.0, fill = 12.0 * cols;
+        const double slice = std::max(245.0, one ? 200.0 + 1.26 * cols : 195.0 + 1.8 * cols), piece4 = one ? 520.0 : 580.0, epilogue4 = 1510.0 + sixteens * piece4;
         const bool two = ms_acc_sets(planes, nt) == 2;
         const auto legs4 = [&](double u) { return two || one ? 0.0 : (std::ceil(u / MS_LEG) - 1) * (500 + sixteens * 150.0); };
-        const auto crowd4 = [&](double blocks) { return 2 * blocks > sms ? (one ? 3000.0 : 1000.0) : 0.0; };
-        const auto take4 = [&](int split, int c, double clocks) {
-            if (four.Nt == 0 || clocks + fill < four.us) four = MmPlan{nt, mt, split, c, 1, true, clocks + fill, 0};
-        };
-        take4(0, 1, crowd4(tiles) + std::ceil(tiles / sms) * (kb * slice + legs4(kbu4) + (two ? 0.0 : epilogue4)) + (two ? epilogue4 : 0.0));
+        const double tile = kb * slice + legs4(kbu4);
+        take(nt, mt, 0, 1, 1, true, start4, tile + epilogue4 + (std::ceil(tiles / sms) - 1) * (two ? std::max(tile, epilogue4) : tile + epilogue4) + crowd(tiles, sms));
         const double blocks = std::min(units, (double)sms), parts = std::min((double)kbu4, blocks / tiles + 1.0);
-        take4(1, 1, crowd4(blocks) + std::ceil(units / blocks) * MS_UK * slice + legs4(std::min(units / blocks, (double)kbu4)) + 3000.0 + 3 * epilogue4 + sixteens * 1000.0 * (parts - 1));
+        take(nt, mt, 1, 1, 1, true, start4,
+             std::ceil(units / blocks) * MS_UK * slice + legs4(std::min(units / blocks, (double)kbu4)) + 3000.0 + sixteens * (8 * piece4 + 520.0 * (parts - 1)) + crowd(blocks, sms));
         for (int c = 2; c <= 8 && c <= kbu4; c *= 2) {
-            if (MM_SMEM - mm_other_bytes(nt, planes, c, true) < 2 * cols * 128 * MS_UK || clusters(c, 1, true) < tiles) continue;
-            take4(2, c, (kbu4 + c - 1) / c * MS_UK * slice + legs4((kbu4 + c - 1) / c) + 2000.0 + sixteens * 100.0 + (sixteens + c - 1) / c * 350.0 + crowd4(tiles * c));
+            const int fit = clusters(c, 1, true);
+            if (MM_SMEM - mm_other_bytes(nt, planes, c, true) < 2 * cols * 128 * MS_UK || fit < tiles) continue;
+            take(nt, mt, 2, c, 1, true, start4, (kbu4 + c - 1) / c * MS_UK * slice + legs4((kbu4 + c - 1) / c) + 5110.0 + sixteens * 470.0 + (sixteens + c - 1) / c * piece4 + crowd(tiles, fit));
         }
         if (nt >= rows) break;
     }
-    if (four.Nt != 0) {                // what calls of these clocks took, 196 of them
-        const double k = four.us / 1000.0, sixteens = four.Nt / 16;
-        four.model = 2.4 + four.us / 1800.0 + (one ? 0.0 : 5.0);
-        four.us = one ? (four.split == 2 ? 5.6 + 0.6 * k : 3.5 + 0.64 * k + 0.1 * sixteens)
-                      : four.split == 0 ? 4.9 + 0.87 * k - 0.22 * sixteens : four.split == 1 ? 1.7 + 0.83 * k + 1.37 * sixteens : 6.1 + 0.96 * k - 0.86 * sixteens;
-    }
-    // Of short launches the estimates are not good enough to tell a few per cent, and units of four slices are the faster ones nearly always.
-    const bool two = four.Nt == 0 || best.us * (!one ? 1.1 : best.us < 35.0 ? 1.15 : 1.0) <= four.us;
-    best.model = four.Nt == 0 ? best.us : std::min(four.model, best.us);
-    return two ? best : four;
+    return best;
 }
 // The plan depends on these sizes alone; a thread keeps those of the last sizes it asked for (making one takes 0.1 to 1 us of a call that takes 4).
-MmPlan mm_plan(int rows, int planes, int n_tiles, int kb, int sms, int device) {
+MmPlan mm_plan(int rows, int planes, int staged, int n_tiles, int kb, int sms, int device) {
     struct Known {
         int rows, planes, n_tiles, kb, sms, device;
+        int staged;
         MmPlan plan;
     };
     static thread_local Known known[64];
-    const uint32_t h = ((uint32_t)rows * 31u + (uint32_t)n_tiles) * 31u + (uint32_t)kb * 4u + (uint32_t)planes;
+    const uint32_t h = ((uint32_t)rows * 31u + (uint32_t)n_tiles) * 31u + (uint32_t)kb * 16u + (uint32_t)planes * 4u + (uint32_t)staged;
     Known& e = known[(h * 2654435761u) >> 26];
-    if (e.rows == rows && e.planes == planes && e.n_tiles == n_tiles && e.kb == kb && e.sms == sms && e.device == device) return e.plan;
+    if (e.rows == rows && e.planes == planes && e.staged == staged && e.n_tiles == n_tiles && e.kb == kb && e.sms == sms && e.device == device) return e.plan;
     bool asked = true;
-    const MmPlan plan = mm_make_plan(rows, planes, n_tiles, kb, sms, device, &asked);
-    if (asked) e = Known{rows, planes, n_tiles, kb, sms, device, plan};
+    const MmPlan plan = mm_make_plan(rows, planes, staged, n_tiles, kb, sms, device, &asked);
+    if (asked) e = Known{rows, planes, n_tiles, kb, sms, device, staged, plan};
     return plan;
 }
 
@@ -506,6 +505,7 @@ struct MmActs {
     int planes, plane_rows;
     size_t pitch;
     int finite;              // MmParams::finite
+    int staged;              // mm_plan
 };
 struct MmOut {
     void* Y;
@@ -518,7 +518,7 @@ struct MmOut {
 
 // rows [0, rows) of `x` (at most MM_MAX_M_TILES tiles) in one launch of the tensor-core kernel
 int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cudaStream_t st) {
-    const MmPlan plan = mm_plan(rows, x.planes, w.n_tiles, w.kb, w.sms, w.device);
+    const MmPlan plan = mm_plan(rows, x.planes, x.staged, w.n_tiles, w.kb, w.sms, w.device);
     MmParams p{};
     p.Y = o.Y;
     p.counters = w.counters;
@@ -598,7 +598,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
 int run_mm_planes(const BitsView& w, const unsigned short* planes, int plane_rows, size_t pitch, int rows, void* Y, int y_dtype, int y_ld, float scale, cudaStream_t st) {
     const int per = MM_MAX_M_TILES * mm_max_nt(3);
     for (int r0 = 0; r0 < rows; r0 += per) {
-        const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch, 1}, std::min(rows - r0, per),
+        const int rc = launch_mm(w, MmActs{(const char*)planes + (size_t)r0 * pitch, true, 3, plane_rows, pitch, 1, MM_FROM_ROWS}, std::min(rows - r0, per),
                                  MmOut{(char*)Y + (size_t)r0 * y_ld * dtype_size(y_dtype), y_dtype, y_ld, 0, scale, 0.f, false, false, 0}, st);
         if (rc) return rc;
     }
@@ -621,7 +621,7 @@ int run_mm(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_ld
     for (int r0 = 0; r0 < rows; r0 += per) {
         const int m = std::min(rows - r0, per);
         const char* xp = (const char*)X + (x_layout == TLLM_ROW_MAJOR ? (size_t)r0 * x_ld : (size_t)r0) * xe;
-        MmActs a{xp, x_dtype == TLLM_BF16 || x_dtype == TLLM_F32, planes, m, (size_t)x_ld * 2, finite};
+        MmActs a{xp, x_dtype == TLLM_BF16 || x_dtype == TLLM_F32, planes, m, (size_t)x_ld * 2, finite, direct ? MM_READY : x_layout == TLLM_ROW_MAJOR ? MM_FROM_ROWS : MM_FROM_COLUMNS};
         if (!direct) {
             const int rc = run_stage(xp, x_dtype, x_layout, x_ld, m, K, (unsigned short*)ws.ptr, w.fresh && r0 == 0, st);
             if (rc) return rc;
@@ -866,26 +866,25 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
     return TLLM_OK;
 }
 
-// Cost models of the two kernels that read the two-bit tiles, microseconds.  Batched: the plan's, and 5 us for one plane that has to be
-// made first (of int8 3.5: 64 rows of 4096 x 4096 take 11.7 us there, 14.3 in two launches of the register decoder).
+// Cost models of the two kernels that read the two-bit tiles, microseconds.
 double bt_model_us(int inners, int columns, int sms, int x_dtype, BitsAccess access, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
     double t = 0;
     for (int r0 = 0; r0 < rows; r0 += per) t += bits_estimate_us(x_dtype, access, std::min(rows - r0, per), columns, (inners + 63) / 64, sms);
     return t;
 }
-double mm_tiles_model_us(int inners, int columns, int sms, int device, bool direct, int x_dtype, int rows) {
-    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes);
-    double t = 0;
+double mm_tiles_model_us(int inners, int columns, int sms, int device, bool direct, int x_dtype, BitsAccess access, int rows) {
+    const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes), staged = direct ? MM_READY : access == BITS_COLUMNS ? MM_FROM_COLUMNS : MM_FROM_ROWS;
+    double t = access == BITS_COLUMNS ? 0.1 + 1.3 * rows * inners / 1e6 : 0.0;        // columns take longer to turn into planes
     for (int r0 = 0; r0 < rows; r0 += per)
-        t += mm_plan(std::min(rows - r0, per), planes, (columns + 127) / 128, (inners + 63) / 64, sms, device).model + (direct || planes > 1 ? 0.0 : x_dtype == TLLM_I8 ? 3.5 : 5.0);
+        t += mm_plan(std::min(rows - r0, per), planes, staged, (columns + 127) / 128, (inners + 63) / 64, sms, device).us;
     return t;
 }
 // which of the two: true = decode in registers
 bool bits_prefer_registers(int inners, int columns, int sms, int device, bool direct, int x_dtype, BitsAccess access, int rows) {
     if (rows == 1 && access == BITS_ROWS16) return true;
     if (rows > 8 * BT_MAX_ROWS) return false;
-    return bt_model_us(inners, columns, sms, x_dtype, access, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, rows);
+    return bt_model_us(inners, columns, sms, x_dtype, access, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, access, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
@@ -899,24 +898,26 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
         const int inners = w->lay.inners, columns = w->lay.columns, sms = w->mm_grid;
         const BitsAccess access = bits_access(X, x_dtype, x_layout, x_ld);
         const double bits = bt_model_us(inners, columns, sms, x_dtype, BITS_ROWS16, rows), gather = gather_model_us(w->lay.nnz, rows);
-        // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (4096 x 11008, 90 % zeros, 5.6 us
-        // against 6.6).  The gather model is a fifth low there, and twice too low where there are few columns.
-        if (rows == 1 && columns >= 4096 && 1.25 * gather < bits) return KERNEL_GATHER;
+        const int per = nb_rows_per_launch(x_dtype);
+        const bool nibbles = nb_fits(w, x_dtype, x_layout) && rows <= 8 && (rows <= per || access == BITS_ROWS16);
+        const double nibble = nibbles ? nibble_model_us(entries, rows, per) : 1e9;
+        // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (8192 x 28672, 90 % zeros, fp16: 22 us against 30;
+        // 4096 x 11008, fp32: 6.1 against 8.7).
+        // The gather model is a fifth low there, two fifths where rows start anywhere, and twice too low where there are few columns.
+        if (rows == 1 && columns >= 4096 && 1.45 * gather < std::min(bits, nibble)) return KERNEL_GATHER;
         // Two rows of int8 too, which the gather kernel reads in either layout (column-major, 2048 x 8192, 70 % zeros: 6.6 us; decoded in
         // registers 11.9; and 8192 x 28672, 90 % zeros: 22 against 35 by rows).  Its sums are exact as well.
         if (x_dtype == TLLM_I8 && rows <= 2 && columns >= 4096 &&
-            1.35 * gather < std::min(bt_model_us(inners, columns, sms, x_dtype, access, rows), mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, rows)))
+            1.35 * gather < std::min(bt_model_us(inners, columns, sms, x_dtype, access, rows), mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, access, rows)))
             return KERNEL_GATHER;
         // A weight so wide that a block of the register decoder makes several passes: four bits an entry, which no thread touches, are read
         // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4; one or two rows of fp32 28.4 and 32.7
         // against 47 and 49, with the same error).  The model is 8 % high there.  More than one launch's rows (4, fp32 2) have to start on 16
         // bytes: its planes are made from X element by element else (28672 x 8192, eight rows: 82 us, the batched kernel 43).  Of fp32 these
         // compete with the batched kernel (four rows 34 us against 46, eight 40), over a K that is not too long: 28672 x 8192 57 against 46.
-        const int per = nb_rows_per_launch(x_dtype);
-        if (nb_fits(w, x_dtype, x_layout) && rows <= 8 && (rows <= per || access == BITS_ROWS16)) {
-            const double nibble = nibble_model_us(entries, rows, per);
+        if (nibbles) {
             if (x_dtype == TLLM_F32 && rows > per) {
-                if (inners <= 16384 && nibble < std::min(bits, mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, rows))) return KERNEL_NIBBLE;
+                if (inners <= 16384 && nibble < std::min(bits, mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, access, rows))) return KERNEL_NIBBLE;
             } else if ((nb || x_dtype == TLLM_F32) && 0.92 * nibble < bits) return KERNEL_NIBBLE;
         }
         return bits_prefer_registers(inners, columns, sms, w->device, mm_direct(inners, X, x_dtype, x_layout, x_ld), x_dtype, access, rows) ? KERNEL_BITS : KERNEL_MMA;
