@@ -59,6 +59,7 @@ static size_t dtype_size(int dt) {
 // tensor-core kernel, n > 0 = from n activation rows on.  TLLM_MMA_MIN_ROWS sets the initial value.
 static std::atomic<int> g_mm_min_rows{-2};
 static std::atomic<int64_t> g_mm_launches{0};
+static thread_local int g_mm_last_plan[5];      // of this thread's last launch: tllm_mma_last_plan
 static std::atomic<int64_t> g_bits_launches{0};
 static int mm_min_rows() {
     int v = g_mm_min_rows.load(std::memory_order_relaxed);
@@ -591,6 +592,8 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     CU_TRY(cudaLaunchKernelEx(&cfg, kern, map, w.map[plan.units4 ? 1 : 0], p));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     g_mm_launches.fetch_add(1, std::memory_order_relaxed);
+    const int cut[5] = {uk, cg, p.split, p.cluster, p.Nt};
+    std::memcpy(g_mm_last_plan, cut, sizeof cut);
     return TLLM_OK;
 }
 
@@ -1257,6 +1260,11 @@ int tllm_version(void) { return 200; }
 int64_t tllm_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 int64_t tllm_bits_launch_count(void) { return g_bits_launches.load(std::memory_order_relaxed); }
 int64_t tllm_mma_launch_count(void) { return g_mm_launches.load(std::memory_order_relaxed); }
+int tllm_mma_last_plan(int plan[5]) {
+    if (!plan || g_mm_last_plan[0] == 0) return fail(TLLM_ERR_ARG, "tllm_mma_last_plan: %s", plan ? "this thread has launched none" : "plan is NULL");
+    std::memcpy(plan, g_mm_last_plan, sizeof g_mm_last_plan);
+    return TLLM_OK;
+}
 int tllm_set_mma_min_rows(int rows) {
     const int prev = mm_min_rows();
     g_mm_min_rows.store(rows < 0 ? -1 : rows, std::memory_order_relaxed);

@@ -4,6 +4,8 @@ An activation touches the columns whose weight there is not zero, as in the prod
 NaN, and every other column is as if it were not there.  Only a product of many rows of 16-bit activations that are read in place
 multiplies the zeros too (0 * Inf = NaN).  The reference is the same sum in fp64; finite sums are held to the bounds of the other tests,
 1e-5 of the row's largest finite output."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -71,6 +73,22 @@ def test_product(K, N, M, dtype):
     check(out, product(X, w, dense=dtype != "f32" and not decoded), 1e-5)
     pw.matmul(X.t().contiguous(), out=out, col_major=True)     # through planes where it is batched
     check(out, product(X, w), 1e-5)
+    pw.check()
+    pw.close()
+
+
+# pairs of blocks, whole tiles and ranges of units, read in place (the zeros count) and through planes
+@pytest.mark.parametrize("M,K,N,dtype,cut,dense", [(2177, 792, 1635, "bf16", 0, True), (2177, 792, 1635, "f16", 0, True), (2127, 778, 1854, "bf16", 0, False),
+                                                   (880, 1085, 138, "f32", 0, False), (232, 6512, 2337, "f32", 1, False)])
+def test_pairs_of_blocks(M, K, N, dtype, cut, dense):
+    w = weights(K, N, 0.6, K)
+    pw = PackedWeight.from_dense(w)
+    X = special_rows(torch.randn((M, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).to(DT[dtype]), 4.0e4 if dtype == "f16" else 2.5e38)
+    out = torch.empty((M, N), device="cuda")
+    pw.matmul(X, out=out)
+    plan = (ctypes.c_int * 5)()
+    assert _lib.lib().tllm_mma_last_plan(plan) == 0 and tuple(plan)[:3] == (2, 2, cut), tuple(plan)
+    check(out, product(X, w, dense=dense), 1e-5)
     pw.check()
     pw.close()
 

@@ -6,6 +6,8 @@ ternaryLLM_GPU/csrc/ter_spmm_kernel.cuh:106-308), so the pin is the oracle's den
 integer-valued activations (every product and every partial sum is an integer below 2^24, so the order of the
 sums cannot matter), and within 1e-3 of the largest output on N(0,1) activations.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -87,11 +89,27 @@ def test_tolerance_on_gaussian_activations_and_agreement_with_the_gather_kernel(
     pw.close()
 
 
-# Sizes that go to pairs of blocks: whole tiles and shared ones, two and four places in the ring of expanded units, odd numbers of slices and
-# of column tiles, ragged rows, columns and K, several legs of fp32.
-@pytest.mark.parametrize("M,K,N,dtype", [(500, 1000, 8192, "bf16"), (1500, 2056, 1500, "f16"), (300, 2056, 8192, "bf16"), (2000, 130, 8192, "f16"),
-                                         (130, 4100, 3333, "f32"), (1000, 4100, 640, "f32"), (1000, 448, 8192, "f32"), (500, 4100, 2500, "f32")])
-def test_exact_on_pairs_of_blocks(M, K, N, dtype):
+def mma_plan():
+    """Of the calling thread's last launch: slices of a unit, blocks that share an MMA, cut (0 tiles, 1 ranges of units, 2 clusters), blocks of a
+    cluster, rows of a tile."""
+    plan = (ctypes.c_int * 5)()
+    assert _lib.lib().tllm_mma_last_plan(plan) == 0
+    return tuple(plan)
+
+
+# The forms of the kernel with units of two slices: blocks that share an MMA, cut, blocks of a cluster, whether a tile has more than 128 columns of
+# D (two places in the ring of expanded units, else four).  Even and odd numbers of column tiles (of the last one a pair's second block has
+# none), one slice and many, odd ones, activations that TMA reads in place and that it does not (K not a multiple of eight, fp32), several legs of fp32.
+@pytest.mark.parametrize("M,K,N,dtype,blocks,cut,cluster,wide", [
+    (160, 2424, 9902, "f16", 2, 0, 1, True), (2177, 792, 1635, "bf16", 2, 0, 1, True), (2127, 778, 1854, "f16", 2, 0, 1, True),
+    (880, 1085, 138, "f32", 2, 0, 1, True), (799, 1009, 263, "f32", 2, 0, 1, True),
+    (2178, 208, 8140, "bf16", 2, 1, 1, True), (1577, 312, 14154, "f16", 2, 1, 1, True), (2204, 65, 9729, "bf16", 2, 1, 1, True),
+    (1801, 144, 8836, "f16", 2, 1, 1, False), (1905, 88, 13945, "bf16", 2, 1, 1, False),
+    (551, 7944, 414, "f32", 2, 1, 1, True), (232, 6512, 2337, "f32", 2, 1, 1, True),
+    (342, 256, 200, "f16", 1, 0, 1, False), (1906, 64, 539, "bf16", 1, 0, 1, True), (591, 348, 1800, "f32", 1, 0, 1, True),
+    (1862, 80, 6850, "f16", 1, 1, 1, False), (2191, 64, 6630, "bf16", 1, 1, 1, True), (800, 5910, 294, "f32", 1, 1, 1, True),
+    (784, 1985, 411, "f32", 1, 2, 2, True), (1567, 2319, 277, "bf16", 1, 2, 4, True), (221, 4424, 268, "f32", 1, 2, 8, True)])
+def test_exact_on_units_of_two_slices(M, K, N, dtype, blocks, cut, cluster, wide):
     rng = np.random.default_rng(M + K)
     w = random_ternary(rng, K, N, 0.5)
     pw = PackedWeight.from_dense(w, scale=1.0)
@@ -100,8 +118,11 @@ def test_exact_on_pairs_of_blocks(M, K, N, dtype):
     y = torch.full((M, N), float("nan"), dtype=torch.float32, device=dev())
     L = _lib.lib()
     L.tllm_set_mma_min_rows(-1)                       # the library's choice, fp32 as well
-    pw.matmul(x.to({"f32": torch.float32, **DT}[dtype]), out=y)
-    assert mma_launches() > n0, "the call did not run on the tensor-core kernel"
+    for _ in range(2):                                # the second launch starts beside the first one
+        pw.matmul(x.to({"f32": torch.float32, **DT}[dtype]), out=y)
+    assert mma_launches() == n0 + 2, "the call did not run on the tensor-core kernel"
+    plan = mma_plan()
+    assert plan[:4] == (2, blocks, cut, cluster) and (plan[4] * (3 if dtype == "f32" else 1) > 128) == wide, plan
     assert torch.equal(y.double(), x @ torch.tensor(w, device=dev()).double())
     pw.check()
     pw.close()
