@@ -114,6 +114,7 @@ double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, i
 
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
+    if (p.x_dtype == TLLM_I8 && p.K >= BT_MAX_INT8_K) return fail(TLLM_ERR_ARG, "bits_launch: int8 over %d inners does not fit into 32-bit sums", p.K);
     const bool async = bits_access(p.X, p.x_dtype, p.x_layout, p.x_ld) == BITS_ROWS16;
     const BitsPlan q = bits_plan(p.x_dtype, p.M, p.N, p.KB, sms);
     const int nb = q.nb, gr = q.gr, grid = sms, kparts = BT_WARPS >> q.split_log, cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, pairs = q.pairs;

@@ -31,7 +31,8 @@
 // Of the 6.2 us, 3.3 are there without any decode or MMA (launch chain, activations from L2, sums); the rest is instruction
 // issue, 0.55 per scheduler and clock.
 //
-// Precision.  fp16 / bf16 activations are multiplied as they are; int8 as int8 with int32 sums (exact); an fp32 value is cut into
+// Precision.  fp16 / bf16 activations are multiplied as they are; int8 as int8 with int32 sums of +-64 * x
+// (exact below BT_MAX_INT8_K inners); an fp32 value is cut into
 // three bf16 values of eight significant bits each (truncation, so the three add up to it exactly), three columns of B
 // whose sums are added at the end.  W is 0 / +-2 (the factor two is taken back with the scale), products are exact, sums
 // are fp32; integer activations give exact sums below 2^24.  A sum that is not finite is taken again entry by entry
@@ -51,6 +52,7 @@ namespace tllm {
 #define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks; int8: 32, four)
 #define BT_MASK 0xC000C000u             // the two codes at the top of a word's halves: 16-bit floats 0 / +-2
 #define BT_MASK8 0xC0C0C0C0u            // the four at the top of its bytes: 0 / +-64
+#define BT_MAX_INT8_K (1 << 18)         // int8: 64 * 128 * K has to stay below 2^31
 
 struct BitsParams {
     const uint4* bits;
@@ -478,7 +480,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     }
 }
 
-// one launch of up to BT_MAX_ROWS rows (half of it fp32); fills in everything from `own` to `mul16` (bits.cu)
+// one launch of up to BT_MAX_ROWS rows (half of it fp32, twice int8); fills in everything from `own` to `mul16` (bits.cu)
 int bits_launch(BitsParams& p, int sms, int device, void* stream);
 // How it reads X: rows on 16 bytes (cp.async), rows that start anywhere, or a column-major X
 enum BitsAccess { BITS_ROWS16, BITS_ROWS, BITS_COLUMNS };

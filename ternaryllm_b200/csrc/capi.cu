@@ -896,7 +896,8 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     if (nb && g_nb_max_rows.load(std::memory_order_relaxed) > 0) return KERNEL_NIBBLE;     // pinned
     if (mm_pinned(w, X, x_dtype, x_layout, x_ld, rows)) return KERNEL_MMA;
     const int64_t entries = (int64_t)w->lay.inners * w->lay.columns;
-    // int8 sums are exact in fp32 while K * 128 stays within 2^24
+    // int8: the batched kernel's fp32 sums are exact while K * 128 stays within 2^24; the register decoder's int32 sums of 64 * x while K stays below
+    // 2^18 (BT_MAX_INT8_K), which this bound takes care of too
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
         const int inners = w->lay.inners, columns = w->lay.columns, sms = w->mm_grid;
         const BitsAccess access = bits_access(X, x_dtype, x_layout, x_ld);

@@ -73,6 +73,34 @@ def test_int8_extremes(K, N, M):
     pw.close()
 
 
+# Four blocks of columns of B in registers, rows on 16 bytes: several pairs of slices per warp, slots that are used again, the columns cut two and
+# four ways.
+@pytest.mark.parametrize("M", [17, 24, 31, 32])
+@pytest.mark.parametrize("K,N", [(2048, 8192), (4096, 4096)])
+def test_int8_of_32_rows_in_registers(K, N, M):
+    w = random_ternary(np.random.default_rng(M), K, N, 0.3)
+    w[:, 0], w[:, N - 1] = 1, -1
+    pw = PackedWeight.from_dense(w)
+    x = torch.randint(-128, 128, (M, K), dtype=torch.int8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(K))
+    x[0], x[-1] = -128, 127
+    assert torch.equal(decoded(pw.matmul, x).double(), x.double() @ torch.tensor(w, device="cuda").double())
+    pw.close()
+
+
+# the largest K that int8 takes here: sums of 2^24, accumulators of +-64 * 2^24
+def test_int8_of_the_largest_k():
+    K, N = 131072, 24
+    w = random_ternary(np.random.default_rng(0), K, N, 0.3)
+    w[:, 0], w[:, N - 1] = 1, -1
+    pw = PackedWeight.from_dense(w)
+    for value in (-128, 127):
+        x = torch.full((1, K), value, dtype=torch.int8, device="cuda")
+        assert torch.equal(decoded(pw.matmul, x).double(), x.double() @ torch.tensor(w, device="cuda").double())
+        x = x.expand(8, K).contiguous()
+        assert torch.equal(pw.matmul(x).double(), x.double() @ torch.tensor(w, device="cuda").double())
+    pw.close()
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
 def test_gaussian_activations_and_result_types(dtype):
     rng = np.random.default_rng(5)
