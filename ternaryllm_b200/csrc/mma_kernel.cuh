@@ -71,6 +71,8 @@ namespace tllm {
 #define MM_MAX_COLS 192               // columns of D of a tile = planes * Nt, Nt (activation rows) a multiple of sixteen
 #define MM_OWN_NT 64                  // a handle's own hand-over scratch is for tiles of up to this many rows
 #define MM_MAX_M_TILES 16             // row tiles of one launch
+static_assert(MM_RAW_UNITS <= MM_MAX_STAGES && (MM_RAW_UNITS & (MM_RAW_UNITS - 1)) == 0, "as many barriers as places; positions are masked");
+static_assert(MM_MAX_STAGES == 8, "the barriers of the rings lie eight apart in shared memory");
 // what a result is stored as
 #define MM_OUT_F32 0
 #define MM_OUT_I32 1

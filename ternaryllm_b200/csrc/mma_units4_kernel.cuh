@@ -21,6 +21,8 @@ namespace tllm {
 #define MS_A_COL 256
 #define MS_LEG 4
 #define MS_THREADS (23 * 32)
+static_assert(MS_RAW_UNITS <= MM_MAX_STAGES && MS_A_UNITS <= MM_MAX_STAGES, "as many barriers as places");
+static_assert(MS_A_COL + MS_A_UNITS * MS_UK * 32 <= 512, "the ring of expanded units lies in tensor memory");
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
     asm volatile(
