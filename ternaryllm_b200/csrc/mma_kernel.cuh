@@ -343,8 +343,10 @@ __device__ __forceinline__ void mm_st_peer(uint32_t addr, float a, float b, floa
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 // An arrival at the barrier of a pair's first block: what it stands for is tensor memory, which the tcgen05 waits and fences before it
-// have taken care of.  (With release.cluster it waited for the thread's other writes too: 2500 clocks.)
-__device__ __forceinline__ void mm_arrive_first(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mm_peer(bar, 0u)) : "memory"); }
+// have taken care of, so that nothing has to be released with it.  (With release.cluster it waited for the thread's other writes too: 2500 clocks.)
+__device__ __forceinline__ void mm_arrive_first(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mm_peer(bar, 0u)) : "memory");
+}
 __device__ __forceinline__ void mm_arrive_peer(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 // column (of the 32 of a quarter tile) that lane `lane` of tensor memory's quarter holds
