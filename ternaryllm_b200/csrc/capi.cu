@@ -1185,8 +1185,9 @@ int run_mcsc(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, c
 }
 
 // Whether the arrays are turned into bit tiles first, on every call.  The per-column kernel reads the lists again for every four
-// rows: 27 us a time at 2048 x 8192, 80 % zeros, fp32; the conversion and what follows it cost 15 us and 1.2e-6 us an entry
-// (35 us there, 57 with 256 rows).  The two meet at about 6e6 entries times passes.
+// rows; the conversion and the kernels behind it cost 13 to 24 us at least.  2048 x 8192, 80 % zeros, fp32: 5 rows 24 us turned into tiles, 41 per
+// column; 256 rows 39 and 1393.  The two meet at about 6e6 entries times passes: 24 rows of fp32 17.5 us and 16.6 on 1024 x 1024, 14.7 and 14.9 on
+// 512 x 2048 (bf16 16.8 and 18.7, 13.3 and 16.7), 9 rows on 2048 x 1024, half zeros, 24.8 and 26.0.
 bool lists_worth_converting(long long entries, int rows) { return rows > MCSC_ROWS && entries * ((rows + MCSC_ROWS - 1) / MCSC_ROWS) >= 6000000; }
 
 int run_lists(const void* X, int x_dtype, int x_layout, const int16_t* row_idx, const int32_t* col_off, void* Y, int y_dtype, int batch, int rows, int columns,

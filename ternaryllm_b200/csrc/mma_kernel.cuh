@@ -35,7 +35,7 @@
 //     128 bytes that its shared memory moves per clock.
 // An MMA of N columns then takes 0.52 N + 13 to 25 clocks, the latter while decoders write to tensor memory.  Measured against a unit of four
 // slices, one block per tile, a warp that elects a lane per MMA and one set of accumulators for three planes: 2048 rows of 5120 x 15360
-// bf16 235 us (276; both at the power cap), 256 rows of fp32 2048 x 16384 44 us (56), 2048 x 8192 28 us (36).
+// bf16 233 us (276; both at the power cap), 256 rows of fp32 2048 x 16384 42 us with its planes (55), 2048 x 8192 28 us (36).
 // Work is either whole output tiles or, where those would leave SMs idle, the flattened list of (output tile, unit) pairs
 // cut into equal contiguous ranges, one per block or pair.  Tiles that straddle two or more blocks are summed in block order by the
 // last block to arrive, which makes the result independent of scheduling; a block does its two shared tiles first, so that

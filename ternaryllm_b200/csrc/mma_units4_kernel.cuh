@@ -2,8 +2,8 @@
 //
 // Where a block has a handful of units, what counts is the time from its start to its first MMA and from its last one to the result, and how many
 // barriers are passed between; sixteen decoder warps expand a whole unit at a time, four warps store, and a block has twenty-three warps to start.
-// mma_kernel.cuh feeds the tensor core better and starts later (20 to 32 rows of 2048 x 2048: 6.9 us here, 7.7 there; 192 rows of
-// 4096 x 4096: 14.8 and 16.4; but 256 rows of fp32 2048 x 16384: 56 and 41, 2048 rows of 5120 x 15360: 276 and 235).  mm_plan has an
+// mma_kernel.cuh feeds the tensor core better and starts later (24 rows of fp16 on 2048 x 2048: 5.6 us here, 6.3 there; 256 rows on 4096 x 4096
+// 15.1 and 16.5; but 256 rows of fp32 on 4096 x 11008, planes included, 67 and 52; 2048 rows of 5120 x 15360 276 and 233).  mm_plan has an
 // estimate of either.
 //
 // Roles: warp 0 bit tiles and warp 6 activations by TMA, warp 1 MMAs (one thread each), warps 2..5 epilogue, warps 7..22 decoders.  A has a ring of

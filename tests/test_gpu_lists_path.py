@@ -31,10 +31,10 @@ def kernels():
     return np.array([L.tllm_launch_count(), L.tllm_bits_launch_count() + L.tllm_mma_launch_count()])
 
 
-# one slice, odd slices, tiles of many sizes, several images per block (K > 8192; of tiles that end with them and of one that does not),
-# no full tile of columns; each with the fewest rows that are turned into bit tiles (entries * ceil(rows / 4) >= 6e6), and one block of four fewer
+# one slice, odd slices, tiles of many sizes, several images per block (K > 2048: one row more, a slice more, several more; of tiles that end with
+# them and of one that does not), no full tile of columns; each with the fewest rows that are turned into bit tiles (entries * ceil(rows / 4) >= 6e6), and one block of four fewer
 @pytest.mark.parametrize("K,N,T,s", [(40, 3, 16, 0.3), (64, 16, 64, 0.5), (200, 130, 64, 0.6), (1000, 70, 256, 0.5), (2048, 300, 256, 0.9), (9000, 40, 512, 0.6),
-                                     (8256, 20, 100, 0.5)])
+                                     (8256, 20, 100, 0.5), (2049, 36, 256, 0.5), (2112, 50, 512, 0.6)])
 @pytest.mark.parametrize("padding", [0, 4])
 def test_exact_on_integer_activations(K, N, T, s, padding):
     rng = np.random.default_rng(K + N)
