@@ -48,7 +48,9 @@ METRIC = "ternary_llama70b_shape_decode_tokens_per_s"
 DEC = dict(hidden=8192, ffn=28672, heads=64, kv_heads=8, head_dim=128, layers=80, kv_len=1024)
 # DRAM bytes per launch of the decode kernel from an ncu capture of the headline product (dram__bytes_read.sum +
 # dram__bytes_write.sum); refreshed whenever the kernel or the format changes
-NCU_TRAFFIC = {"bytes": 14.03e6, "source": "ncu, profiles/bstream_spmm_decode_4096x11008_s75_m1.md"}
+# DRAM bytes of a launch of the decode product's headline workload, where ncu has counted them, by the kernel that runs it
+NCU_TRAFFIC = {"bits_spmm_kernel": {"bytes": 11.3e6, "source": "ncu (bytes read), profiles/two_bit_kernels_and_attention.md"},
+               "bstream_spmm_kernel<float,1>": {"bytes": 14.03e6, "source": "ncu, profiles/bstream_spmm_decode_4096x11008_s75_m1.md"}}
 
 
 def algorithmic_bytes(nnz: int, K: int, N: int, M: int, e: int) -> int:
@@ -653,14 +655,16 @@ def main():
         }
         if spmv is not None:
             h = spmv["headline"]
+            ran = {"decode": "nibble_spmm_kernel", "register": "bits_spmm_kernel", "tensor": "mma_spmm_kernel / mma_units4_kernel"}.get(h["kernel"].split()[0], "bstream_spmm_kernel<float,1>")
+            traffic = NCU_TRAFFIC.get(ran, {"bytes": None, "source": f"not counted for {ran}"})
             line["roofline"] = {"bound": "hbm", "achieved": h["algorithmic_GBps"], "peak": peak, "unit": "GB/s", "frac": h["frac"],
                                 "frac_physical": h["frac_physical"], "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback 6650 GB/s",
-                                "kernel": "nibble_spmm_kernel" if h["kernel"].startswith("decode") else "bstream_spmm_kernel<float,1>",
+                                "kernel": ran,
                                 "kernel_choice": "the library's cost model (the times of the gather and the decode tensor-core kernel, each pinned, are under spmv.headline.by_kernel)",
                                 "us_per_launch": h["us_per_launch"],
                                 "workload": f"decode product x[1,{K_IN}] fp16, W[{K_IN},{N_OUT}] 75% zeros, {h['weights_in_rotation']} weights in rotation (larger than L2)",
                                 "algorithmic_bytes_per_launch": h["algorithmic_bytes"], "physical_bytes_per_launch": h["physical_bytes"],
-                                "traffic": NCU_TRAFFIC["bytes"], "traffic_source": NCU_TRAFFIC["source"]}
+                                "traffic": traffic["bytes"], "traffic_source": traffic["source"]}
             line["spmv"] = spmv
         po = headline.get("products_only")
         if po:
