@@ -23,12 +23,12 @@
 //
 // Measured, fp16, CUDA-graph chain of distinct weights from HBM (us; before = the fastest of the other kernels):
 //   2048 x 2048    1 row  2.3 (gather 3.9)      8 rows  2.6 (batched 11.5)
-//   4096 x 11008   1 row  6.2 (gather 8.3, 75 % zeros; four-bit planes 10.5)   8 rows  7.0 (17.2)   16 rows 13.3 (19.5)
+//   4096 x 11008   1 row  6.0 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  7.0 (17.2)   16 rows 11.8 (19.5)
 //   8192 x 10240   1 row 10.8 (four-bit planes 15.4)     8 rows 12.1 (22.7)
 // int8: seven instructions instead of fifteen decode sixteen entries, and two MMAs (m16n8k32) replace four:
 //   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 6.9 in one launch (9.3 in two)
 //   8192 x 10240   1 row  7.6 (12.0)             16 rows 15 (22)
-// Of the 6.2 us, 3.3 are there without any decode or MMA (launch chain, activations from L2, sums); the rest is instruction
+// Of the 6.0 us, 3.3 are there without any decode or MMA (launch chain, activations from L2, sums); the rest is instruction
 // issue, 0.55 per scheduler and clock.
 //
 // Precision.  fp16 / bf16 activations are multiplied as they are; int8 as int8 with int32 sums of +-64 * x
