@@ -15,9 +15,9 @@ namespace {
         if (e_ != cudaSuccess) return fail(TLLM_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_)); \
     } while (0)
 
-template <int XT, int NB, int GR, bool ASYNC>
+template <int XT, int NB, int GR, bool ASYNC, bool SHARED>
 int launch(const BitsParams& p, int grid, size_t smem, int device, cudaStream_t st) {
-    auto kern = bits_spmm_kernel<XT, NB, GR, ASYNC>;
+    auto kern = bits_spmm_kernel<XT, NB, GR, ASYNC, SHARED>;
     static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
     std::call_once(once[device & 63], [&] {
@@ -42,19 +42,19 @@ int launch(const BitsParams& p, int grid, size_t smem, int device, cudaStream_t 
     return TLLM_OK;
 }
 
-template <int XT, bool ASYNC>
+template <int XT, bool ASYNC, bool SHARED>
 int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device, cudaStream_t st) {
-    if (nb == 1 && gr == 1) return launch<XT, 1, 1, ASYNC>(p, grid, smem, device, st);
-    if (nb == 1 && gr == 2) return launch<XT, 1, 2, ASYNC>(p, grid, smem, device, st);
-    if (nb == 1 && gr == 3) return launch<XT, 1, 3, ASYNC>(p, grid, smem, device, st);
-    if (nb == 2 && gr == 1) return launch<XT, 2, 1, ASYNC>(p, grid, smem, device, st);
-    if (nb == 2 && gr == 2) return launch<XT, 2, 2, ASYNC>(p, grid, smem, device, st);
+    if (nb == 1 && gr == 1) return launch<XT, 1, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+    if (nb == 1 && gr == 2) return launch<XT, 1, 2, ASYNC, SHARED>(p, grid, smem, device, st);
+    if (nb == 1 && gr == 3) return launch<XT, 1, 3, ASYNC, SHARED>(p, grid, smem, device, st);
+    if (nb == 2 && gr == 1) return launch<XT, 2, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+    if (nb == 2 && gr == 2) return launch<XT, 2, 2, ASYNC, SHARED>(p, grid, smem, device, st);
     if constexpr (XT == TLLM_I8) {
-        if (nb == 4 && gr == 1) return launch<XT, 4, 1, ASYNC>(p, grid, smem, device, st);
+        if (nb == 4 && gr == 1) return launch<XT, 4, 1, ASYNC, SHARED>(p, grid, smem, device, st);
     }
     if constexpr (XT == TLLM_F32) {
-        if (nb == 3 && gr == 1) return launch<XT, 3, 1, ASYNC>(p, grid, smem, device, st);
-        if (nb == 3 && gr == 2) return launch<XT, 3, 2, ASYNC>(p, grid, smem, device, st);
+        if (nb == 3 && gr == 1) return launch<XT, 3, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+        if (nb == 3 && gr == 2) return launch<XT, 3, 2, ASYNC, SHARED>(p, grid, smem, device, st);
     }
     return fail(TLLM_ERR_ARG, "bits_launch: no kernel for %d x %d", nb, gr);
 }
@@ -81,6 +81,18 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
     q.gr = (q.per_pass + split - 1) / split;
     q.pairs = ((kb + 1) / 2 + kparts - 1) / kparts * passes;
     return q;
+}
+// Whether the warps of a block share X in shared memory, loaded once a row by the TMA unit (rows that start anywhere and columns: by all threads),
+// or each fetches its own pairs of slices of it.  Sharing saves what every part of a split, and every pass, would fetch again; a block's
+// barrier and the later start cost 0.2 to 0.5 us, which a warp of a few pairs does not win back.  (16 rows of fp16 on 4096 x 11008 9.7 us, 12.1 apart;
+// one on 8192 x 10240 9.3 and 10.3; 32 rows of int8 on 2048 x 8192 5.8 and 6.8, but 4.2 and 3.8 on 768 x 6912; 16 of fp16 on 2048 x 2048,
+// no split, 3.1 and 2.7.  Two rows of fp16 on odd addresses, 2048 x 16384, 5.5 and 7.8; two columns of fp32 on 4096 x 11008 9.5 and 16.4.)
+bool bits_share(int x_dtype, bool async, const BitsPlan& q, int kp, int rows) {
+    if (q.passes > 1) return true;
+    if (!async) return q.split_log > 0 || (kp <= 10 && rows >= 8);
+    const bool two_bytes = x_dtype == TLLM_F16 || x_dtype == TLLM_BF16;
+    if (q.split_log == 2) return q.pairs > 2;
+    return q.split_log == 1 && (q.pairs > 4 || (q.pairs == 4 && two_bytes) || (q.pairs > 1 && (q.nb == 3 || (q.nb == 2 && two_bytes))));
 }
 }  // namespace
 
@@ -115,29 +127,45 @@ double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, i
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
     if (p.x_dtype == TLLM_I8 && p.K >= BT_MAX_INT8_K) return fail(TLLM_ERR_ARG, "bits_launch: int8 over %d inners does not fit into 32-bit sums", p.K);
-    const bool async = bits_access(p.X, p.x_dtype, p.x_layout, p.x_ld) == BITS_ROWS16;
+    const bool async = bits_access(p.X, p.x_dtype, p.x_layout, p.x_ld) == BITS_ROWS16 && (size_t)p.K * e % 16 == 0;
     const BitsPlan q = bits_plan(p.x_dtype, p.M, p.N, p.KB, sms);
     const int nb = q.nb, gr = q.gr, grid = sms, kparts = BT_WARPS >> q.split_log, cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, pairs = q.pairs;
     p.own = q.own, p.own_more = q.own_more, p.split_log = q.split_log, p.per_pass = q.per_pass;
     p.mul4 = 4, p.mul16 = 16;
     p.m_inv = (uint32_t)(((1ull << 32) + p.M - 1) / p.M);
-    p.slot_bytes = (uint32_t)(gr * 512 + p.M * 128 * e);
-    // Pairs in flight: as many as a warp has to fetch and half of the shared memory holds (so that the next launch fits
-    // beside this one); where not even two fit there, up to all of it.
+    const int kp = (p.KB + 1) / 2;
     const size_t red = (size_t)kparts * p.per_pass * cols * 80;
-    auto slots = [&](int d) { return pairs <= d ? pairs : d + 1; };
-    auto total = [&](int d) { return (size_t)BT_WARPS * slots(d) * p.slot_bytes + red; };
+    // Shared memory: X for all warps together, or a warp's pairs of it beside those of W.  Of these as many in flight as a warp has to fetch and as
+    // there is room for: in half of the shared memory, so that the next launch fits beside this one, unless the launch is one of some length
+    // or does not fit there; then in all of it.
+    bool share = bits_share(p.x_dtype, async, q, kp, p.M);
+    const auto pitch = [&](int n) { return (size_t)n * 128 * e + (e == 1 ? 64 : e == 2 ? 16 : 32); };
+    const auto chunk = [&](int n) { return share ? (p.M * pitch(std::min(n, kp)) + 127) / 128 * 128 : 0; };
+    const auto slots = [&](int d) { return pairs <= d ? pairs : d + 1; };
+    const auto slot = [&] { return (uint32_t)(gr * 512 + (share ? 0 : p.M * 128 * e)); };
+    const auto total = [&](int d) { return p.x_chunks * chunk(p.x_pairs) + (size_t)BT_WARPS * slots(d) * slot() + red + BT_BAR_BYTES; };
+    const int least = std::min(pairs, 2);
+    p.x_chunks = kp > 16 && (size_t)p.M * p.K * e > 16384 ? 2 : 1;
+    p.x_pairs = p.x_chunks == 1 ? (kp + 15) / 16 * 16 : ((kp + 1) / 2 + 15) / 16 * 16;
+    if (share && total(least) > BT_SMEM_ALL) share = false;
+    p.slot_bytes = slot();
+    const size_t limit = pairs > 4 || total(least) > BT_SMEM_SHARED ? BT_SMEM_ALL : BT_SMEM_SHARED;
     p.depth = 8;
-    while (p.depth > 1 && (p.depth / 2 >= pairs || total(p.depth) > BT_SMEM_SHARED)) p.depth /= 2;
-    if (p.depth == 1 && pairs > 1 && total(2) <= 220u * 1024u) p.depth = 2;
+    while (p.depth > 1 && (p.depth / 2 >= pairs || total(p.depth) > limit)) p.depth /= 2;
     p.slots = slots(p.depth);
+    p.x_pitch = (uint32_t)pitch(std::min(p.x_pairs, kp)), p.x_bytes = (uint32_t)chunk(p.x_pairs);
+    p.ring_at = p.x_chunks * p.x_bytes;
+    p.red_at = p.ring_at + (uint32_t)BT_WARPS * p.slots * p.slot_bytes;
+    p.bar_at = p.red_at + (uint32_t)red;
     // A launch of some length keeps an SM to itself: behind one that does not fit beside it, its blocks would start two to an SM while
     // others wait (fp16 MLP, four rows, 4096 / 11008: 24 us instead of 19).
     size_t smem = total(p.depth);
     if (pairs > 4) smem = std::max(smem, (size_t)BT_SMEM_ALONE);
     if (smem > 227u * 1024u) return fail(TLLM_ERR_ARG, "bits_launch: %zu bytes of shared memory", smem);
     cudaStream_t st = (cudaStream_t)stream;
-#define BT_PICK(XT) (async ? pick<XT, true>(p, nb, gr, grid, smem, device, st) : pick<XT, false>(p, nb, gr, grid, smem, device, st))
+#define BT_PICK(XT)                                                                                                               \
+    (async ? share ? pick<XT, true, true>(p, nb, gr, grid, smem, device, st) : pick<XT, true, false>(p, nb, gr, grid, smem, device, st) \
+           : share ? pick<XT, false, true>(p, nb, gr, grid, smem, device, st) : pick<XT, false, false>(p, nb, gr, grid, smem, device, st))
     switch (p.x_dtype) {
         case TLLM_F32: return BT_PICK(TLLM_F32);
         case TLLM_F16: return BT_PICK(TLLM_F16);

@@ -13,8 +13,11 @@
 //   * a block owns whole columns (groups of sixteen, dealt out evenly) over all of K; its sixteen warps cut K, and the
 //     columns two or four ways where it owns many: no scratch, no counters, no second pass over global memory.  The warps'
 //     partial sums meet in shared memory and are added in warp order, so results do not depend on scheduling;
-//   * W and X travel by cp.async, several pairs of slices ahead, into slots that belong to one warp: no block barrier in
+//   * W travels by cp.async, several pairs of slices ahead, into slots that belong to one warp: no block barrier in
 //     the main loop, and W is in flight before the preceding kernel has finished (griddepcontrol.wait);
+//   * X travels the same way, each warp its own pairs of slices; or, where several warps would fetch the same ones (the columns cut two or four ways, several
+//     passes), whole, once, for all warps of the block (SHARED; bits_share in bits.cu has the rule and its figures): as much of it as of W went
+//     through L2 four times over (16 rows of fp16 on 2048 x 16384: 64 KB of X a block, fetched four times, for 57 KB of W);
 //   * sixteen warps (four per scheduler hide the latency of shared-memory load -> decode -> MMA; with two per scheduler the
 //     loop issued 0.49 instructions per clock) of <= 64 registers, so that the next launch's block fits beside this one
 //     and starts streaming;
@@ -23,13 +26,15 @@
 //
 // Measured, fp16, CUDA-graph chain of distinct weights from HBM (us; before = the fastest of the other kernels):
 //   2048 x 2048    1 row  2.3 (gather 3.9)      8 rows  2.6 (batched 11.5)
-//   4096 x 11008   1 row  6.0 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  7.0 (17.2)   16 rows 11.8 (19.5)
-//   8192 x 10240   1 row 10.8 (four-bit planes 15.4)     8 rows 12.1 (22.7)
+//   4096 x 11008   1 row  5.6 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  6.6 (17.2)   16 rows  9.7 (19.5)
+//   8192 x 10240   1 row  9.3 (four-bit planes 15.4)     8 rows 10.9 (22.7)
+// fp32: three MMAs per eight rows, whose values a lane cuts into all three pieces at once (BY_PIECE; each block of columns of B by itself 4.5, 8.0 and 11.5):
+//   2048 x 2048    8 rows  3.7      4096 x 4096    8 rows  6.6       8192 x 2048    8 rows  8.8
 // int8: seven instructions instead of fifteen decode sixteen entries, and two MMAs (m16n8k32) replace four:
-//   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 6.9 in one launch (9.3 in two)
-//   8192 x 10240   1 row  7.6 (12.0)             16 rows 15 (22)
-// Of the 6.0 us, 3.3 are there without any decode or MMA (launch chain, activations from L2, sums); the rest is instruction
-// issue, 0.55 per scheduler and clock.
+//   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 5.8 in one launch (9.3 in two)
+//   8192 x 10240   1 row  6.9 (12.0)             16 rows 12.3 (22)
+// Of the 9.3 us of 8192 x 10240, 5.4 are there without decode and MMAs; masks and MMAs, which hardly overlap, take 65 to 70 clocks of a scheduler per
+// 1024 entries (53 with the same instructions and nothing to wait for).
 //
 // Precision.  fp16 / bf16 activations are multiplied as they are; int8 as int8 with int32 sums of +-64 * x
 // (exact below BT_MAX_INT8_K inners); an fp32 value is cut into
@@ -52,12 +57,16 @@ namespace tllm {
 #define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks; int8: 32, four)
 #define BT_MASK 0xC000C000u             // the two codes at the top of a word's halves: 16-bit floats 0 / +-2
 #define BT_MASK8 0xC0C0C0C0u            // the four at the top of its bytes: 0 / +-64
+#define BT_SMEM_ALL (226u * 1024u)
+#define BT_BAR_BYTES 32u                // two barriers, and whether a wait ran out
+#define BT_ERR_WAIT 3                   // status word: a bounded wait ran out
 #define BT_MAX_INT8_K (1 << 18)         // int8: 64 * 128 * K has to stay below 2^31
 
 struct BitsParams {
     const uint4* bits;
     const void* X;
     void* Y;
+    int* status;
     int x_dtype, x_layout, x_ld;   // row-major X: elements between rows; column-major X: elements between k
     int y_dtype, epilogue;         // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
     long long y_step_n, y_step_m;  // elements from column to column and from row to row of Y
@@ -65,8 +74,11 @@ struct BitsParams {
     int own, own_more;             // groups of sixteen columns per block; the first own_more blocks have one more
     int per_pass;                  // groups per pass (<= split * GR)
     int split_log;                 // the warps cut the block's columns 1 << split_log ways (1, 2 or 4); 16 >> split_log warps cut K
-    int slots, depth;              // pairs of slices a warp has room for, pairs in flight (1, 2, 4 or 8; < slots unless no slot is used twice)
-    uint32_t slot_bytes;           // shared memory of one pair of slices: GR * 512 + M * 128 * E
+    int slots, depth;              // pairs of slices of W a warp has room for, pairs in flight (1, 2, 4 or 8; < slots unless no slot is used twice)
+    uint32_t slot_bytes;           // shared memory of one pair of slices: GR * 512, and of X, unless it is shared, M * 128 * E
+    int x_pairs, x_chunks;         // X shared by the warps: pairs of slices of a chunk (a multiple of sixteen), one chunk or two
+    uint32_t x_pitch, x_bytes;     // shared memory of a row of a chunk, and of a chunk
+    uint32_t ring_at, red_at, bar_at;      // where W, the partial sums and the barriers lie
     uint32_t m_inv;                // ceil(2^32 / M): idx / M = umulhi(idx, m_inv) for M > 1
     uint32_t mul4, mul16;          // 4 and 16
     bool pdl;                      // host: launch beside the preceding kernel
@@ -105,6 +117,10 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+// `bytes` (a multiple of 16) of a row by the TMA unit
+__device__ __forceinline__ void bt_load_row(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // waits until at most `left` of the newest groups are in flight (7, 3, 1 or 0)
@@ -193,15 +209,20 @@ __device__ __forceinline__ uint32_t bt_lane_chunk(uint32_t t, uint32_t m) { retu
 // The lane's sixteen activations of slice h (rows 16t .. 16t+15) -> the eight words of a B fragment (word p = rows 2p, 2p+1);
 // `at` is the address of the lane's first chunk of slice 0.  fp32: the `piece`-th of the three bf16 values that add up to
 // each of them.  int8: four words, word s = rows 8+2s, 2s, 9+2s, 2s+1, which is where the codes stand that a shift by 2s brings to the
-// top of a word's bytes.
-template <int XT>
+// top of a word's bytes.  IN_ORDER: the chunks follow one another; else they lie where bt_chunk says.
+template <int XT, bool IN_ORDER>
+__device__ __forceinline__ uint4 bt_load_chunk(uint32_t at, uint32_t h, uint32_t c) {
+    constexpr uint32_t CS = BitsAct<XT>::E;
+    if (IN_ORDER) return bt_lds128(at + h * (CS * 64u) + c * 16u);
+    return bt_lds128((XT == TLLM_I8 ? at ^ (h * 64u) : at + h * (CS * 64u)) ^ (c * 16u));
+}
+template <int XT, bool IN_ORDER>
 __device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, uint32_t (&b)[XT == TLLM_I8 ? 4 : 8]) {
     constexpr uint32_t CS = BitsAct<XT>::E;
     uint32_t w[4 * CS];
-    const uint32_t a0 = XT == TLLM_I8 ? at ^ (h * 64u) : at + h * (CS * 64u);
 #pragma unroll
     for (uint32_t c = 0; c < CS; ++c) {
-        const uint4 v = bt_lds128(a0 ^ (c * 16u));
+        const uint4 v = bt_load_chunk<XT, IN_ORDER>(at, h, c);
         w[4 * c] = v.x, w[4 * c + 1] = v.y, w[4 * c + 2] = v.z, w[4 * c + 3] = v.w;
     }
     if constexpr (XT == TLLM_F32) {
@@ -222,6 +243,23 @@ __device__ __forceinline__ void bt_fragment(uint32_t at, uint32_t h, int piece, 
         for (int i = 0; i < 8; ++i) b[i] = w[i];
     }
 }
+// fp32: all three pieces, as fragments of three blocks of columns of B; the values are read and cut once
+template <bool IN_ORDER>
+__device__ __forceinline__ void bt_pieces(uint32_t at, uint32_t h, uint32_t (&b)[3][8]) {
+#pragma unroll
+    for (uint32_t c = 0; c < 4; ++c) {
+        const uint4 v = bt_load_chunk<TLLM_F32, IN_ORDER>(at, h, c);
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            b[p][2 * c] = __byte_perm(w[0], w[1], 0x7632), b[p][2 * c + 1] = __byte_perm(w[2], w[3], 0x7632);
+            if (p < 2) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) - __uint_as_float(w[i] & 0xFFFF0000u));
+            }
+        }
+    }
+}
 
 // column n of row m, entry by entry, for a sum that is not finite
 template <int XT>
@@ -233,11 +271,12 @@ __device__ __noinline__ float bt_column_sum(const BitsParams& p, int n, int m) {
 
 // A warp multiplies up to GR groups of sixteen columns by NB blocks of eight columns of B (activation rows; fp32: pieces of
 // rows).  A block with more than split * GR groups makes several passes.
-// ASYNC: the rows of X start on 16 bytes and are copied by cp.async; otherwise they pass through registers.
+// ASYNC: the rows of X start on 16 bytes and are a multiple of 16 bytes long; otherwise they pass through registers.
+// SHARED: X lies in shared memory once for all warps, else each has its own pairs of slices.
 //
 // The code is kept short (rolled loops, no divisions): a warp of a small product runs the loop body once or twice, and then
 // fetching instructions costs more than executing them.
-template <int XT, int NB, int GR, bool ASYNC>
+template <int XT, int NB, int GR, bool ASYNC, bool SHARED>
 __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_spmm_kernel(const __grid_constant__ BitsParams p) {
     extern __shared__ __align__(128) unsigned char bt_smem[];
     using Act = BitsAct<XT>;
@@ -246,12 +285,10 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     // The tensor core cuts bits off its running sum at every MMA: fp32 sums leave it after the eight of a pair of slices (gate and up of a
     // 2560 / 6912 MLP, 8 rows, h = silu(gate) * up: off by 1.4e-7 with a warp's 40 MMAs in one sum, 1.1e-7 now).
     constexpr bool PARTS = XT == TLLM_F32;
-    // Whether a result's address is computed before its sum is looked at.  It decides how ptxas allots the registers of the whole kernel (64 of them
-    // in most instances), and so the time of every call.  Computed late: 2048 x 2048, eight rows of fp16 2.61 us (early 3.15), of fp32 4.41
-    // (4.49); 1003 x 517, three rows of bf16 2.62 (2.77).  Early: 8192 x 10240, one row of bf16 10.3 us (late 10.6); 4096 x 11008, eight of fp16
-    // 6.89 (6.98).
-    constexpr bool EARLY = GR == 3 && ASYNC && Act::E == 2;
-    constexpr int CPR = 8 * Act::E, RPI = 32 / CPR, KPC = 16 / Act::E;     // chunks per row (and pair of slices), rows per warp copy, values per chunk
+    // Columns of B: piece of row m is column 3 m + piece; with three blocks of them block `piece` has column m, so that a lane cuts the values of one
+    // row and has all of its columns.
+    constexpr bool BY_PIECE = XT == TLLM_F32 && NB == 3;
+    constexpr uint32_t PAIR = 128u * Act::E;                               // bytes of a row in a pair of slices
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
     const int KB = p.KB, KP = (KB + 1) >> 1, D = p.depth, S = p.slots, M = p.M, SL = p.split_log;
@@ -260,9 +297,12 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     // expression for two and for four shares: with a choice between two every call got slower (2048 x 8192, eight rows of fp32 8.03 us, 7.85 now).
     const int kw = warp >> SL, klog = 4 - SL, kstep = 1 << klog, cw = (warp + (warp >> 2)) & ((1 << SL) - 1);
     const int np = kw < KP ? (KP - kw + kstep - 1) >> klog : 0;      // pairs of this warp: kw, kw + kstep, ...
-    const uint32_t ring = smem_u32(bt_smem) + (uint32_t)warp * (uint32_t)S * p.slot_bytes;
-    Sum* red = (Sum*)(bt_smem + (size_t)BT_WARPS * S * p.slot_bytes);          // [warp][group][column of B][20] partial sums
+    const uint32_t smem = smem_u32(bt_smem), ring = smem + p.ring_at + (uint32_t)warp * (uint32_t)S * p.slot_bytes;
+    Sum* red = (Sum*)(bt_smem + p.red_at);                           // [warp][group][column of B][20] partial sums
+    const uint32_t bars = smem + p.bar_at;
+    volatile int* abort_flag = (volatile int*)(bt_smem + p.bar_at + 16);
     const uint32_t group_bytes = (uint32_t)KB * 256u;
+#define BT_FULL(i) (bars + 8u * (uint32_t)(i))           // X's chunks, 0 and 1
     pdl_launch_dependents();
     // There is a block for every SM even where there are fewer groups: with free SMs the next launch's blocks would be placed
     // two to an SM there (8192 x 2048, one row: 10.5 us instead of 5), so the spare ones hold their place until it is settled.
@@ -272,7 +312,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     }
 
     // A pass covers groups [q0, q0 + n) of the block; this warp's share is [n * cw / split, n * (cw + 1) / split) of them.
-    // ---- copies: the warp's step s (its pairs in order, pass after pass) goes to slot s % S ---------------------------
+    // ---- copies of W: the warp's step s (its pairs in order, pass after pass) goes to slot s % S ----------------------
     const char* wsrc;                                                // first group of the pass being fetched, this warp's next pair
     uint32_t last;                                                   // offset of the last group from it
     int fpass = 0, fi = 0, fs = 0;                                   // next copy: first group of the pass, pair, slot
@@ -304,7 +344,29 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
         }
         if (++fs == S) fs = 0;
     };
-    // X: the lanes copy whole rows, 16 bytes each (the caller's pair i of this warp)
+    open_pass();
+#pragma unroll 1
+    for (int s = 0; s < D; ++s) {                                    // W does not depend on the preceding kernel
+        if (fpass < own && np) {
+            copy_w(ring + (uint32_t)fs * p.slot_bytes);
+            advance();
+            if (SHARED) cp_commit();
+        } else if (SHARED) cp_commit();
+    }
+    const int pre_pass = fpass, pre_i = fi;
+    if (SHARED) {
+        if (tid == 0) {
+            mbar_init(BT_FULL(0), ASYNC ? M : BT_WARPS * 32);
+            mbar_init(BT_FULL(1), ASYNC ? M : BT_WARPS * 32);
+            *abort_flag = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncthreads();
+    }
+
+    // ---- X, of one warp's pair: the lanes copy whole rows, 16 bytes each
+    constexpr int CPR = 8 * Act::E, RPI = 32 / CPR, KPC = 16 / Act::E;     // chunks per row (and pair of slices), rows per warp copy, values per chunk
     const uint32_t xm = (uint32_t)lane / CPR, xch = (uint32_t)lane % CPR;
     auto copy_x = [&](int i, uint32_t slot) {
         const int k = (kw + (i << klog)) * 128 + (int)xch * KPC;
@@ -323,16 +385,36 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
             }
         }
     };
-    open_pass();
+    // ---- X, of all warps: whole, in one chunk of x_pairs pairs of slices or in two that arrive one after the other.  (Rows are x_pitch bytes apart,
+    // 16 (fp32: 32, int8: 64) more than a multiple of 128, so that the lanes of a fragment read different banks.)
+    auto load_x = [&](int chunk) {
+        const int k0 = chunk * p.x_pairs * 128, k1 = min(k0 + p.x_pairs * 128, KP * 128);      // zero past the end of K
+        const uint32_t to = smem + (uint32_t)chunk * p.x_bytes;
+        if (ASYNC) {
+            if (warp == BT_WARPS - 1 && lane < M) {                  // a lane per row
+                const uint32_t row = to + (uint32_t)lane * p.x_pitch, bytes = (uint32_t)(min(k1, p.K) - k0) * Act::E;
+                for (uint32_t z = bytes; z < (uint32_t)(k1 - k0) * Act::E; z += 16u) bt_sts128(row + z, make_uint4(0u, 0u, 0u, 0u));
+                mbar_expect_tx(BT_FULL(chunk), bytes);
+                bt_load_row(row, (const char*)p.X + ((size_t)lane * p.x_ld + k0) * Act::E, bytes, BT_FULL(chunk));
+            }
+        } else {
+            const bool rows = p.x_layout == TLLM_ROW_MAJOR;
+            const uint32_t per_row = (uint32_t)(k1 - k0) * Act::E / 16u, inner = rows ? per_row : (uint32_t)M;
 #pragma unroll 1
-    for (int s = 0; s < D; ++s)                                     // W does not depend on the preceding kernel
-        if (fpass < own && np) {
-            copy_w(ring + (uint32_t)fs * p.slot_bytes);
-            advance();
+            for (uint32_t i = (uint32_t)tid; i < per_row * (uint32_t)M; i += BT_WARPS * 32) {
+                const uint32_t hi = i / inner, lo = i - hi * inner, m = rows ? hi : lo, c = rows ? lo : hi;
+                const int k = k0 + (int)c * (16 / Act::E);
+                bt_sts128(to + m * p.x_pitch + c * 16u, rows ? bt_load_unaligned((const char*)p.X + (size_t)m * p.x_ld * Act::E, k * Act::E, p.K * Act::E)
+                                                             : bt_load_strided<Act::E>(p.X, (int)m, k, p.K, (size_t)p.x_ld));
+            }
+            mbar_arrive_n(BT_FULL(chunk), 1u);
         }
-    const int pre_pass = fpass, pre_i = fi;
+    };
     pdl_wait();
-    {
+    if (SHARED) {
+        load_x(0);
+        if (p.x_chunks > 1) load_x(1);
+    } else {
         int i = 0, pass = 0;
 #pragma unroll 1
         for (int s = 0; s < D; ++s) {
@@ -349,14 +431,15 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     int bpiece[NB];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
-        const uint32_t c = (uint32_t)(nb * 8 + g), m = min(c / Act::P, (uint32_t)M - 1u);
+        const uint32_t c = (uint32_t)(nb * 8 + g), m = min(BY_PIECE ? (uint32_t)g : c / Act::P, (uint32_t)M - 1u);
         bpiece[nb] = (int)(c % Act::P);
-        bat[nb] = GR * 512u + m * (CPR * 16u) + bt_lane_chunk<XT>((uint32_t)t, m);
+        bat[nb] = SHARED ? smem + (uint32_t)kw * PAIR + m * p.x_pitch + (uint32_t)t * (16u * Act::E) : GR * 512u + m * PAIR + bt_lane_chunk<XT>((uint32_t)t, m);
     }
     // Multipliers in registers: a shift by an immediate would run on the ALU pipe, which the ANDs already fill.
     uint32_t m4, m16;
     asm volatile("mov.b32 %0, %2;\n\tmov.b32 %1, %3;" : "=r"(m4), "=r"(m16) : "r"(p.mul4), "r"(p.mul16));
     int cs = 0;                                                      // slot being consumed
+    bool ok = true;
 #pragma unroll 1
     for (int q0 = 0; q0 < own; q0 += p.per_pass) {
         const int ng = min(p.per_pass, own - q0), w0 = (ng * cw) >> SL, mine = ((ng * (cw + 1)) >> SL) - w0;    // this warp's groups of the pass
@@ -367,66 +450,78 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
             for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[j][nb][i] = 0;
+        int left = np;                                               // pairs of the pass
 #pragma unroll 1
-        for (int i = 0; i < np; ++i) {
-            cp_wait(D - 1);
-            __syncwarp();                                            // other lanes' chunks of X are here, and they have read the slot before
-            const uint32_t slot = ring + (uint32_t)cs * p.slot_bytes;
-            if (fpass < own) {                                       // into the slot that was consumed one step ago
-                const uint32_t dst = ring + (uint32_t)fs * p.slot_bytes;
-                copy_w(dst);
-                copy_x(fi, dst);
-                advance();
-            }
-            cp_commit();
-            float part[GR][NB][4];                                   // fp32: the sums of this pair of slices
-            if constexpr (PARTS) {
-#pragma unroll
-                for (int j = 0; j < GR; ++j)
-#pragma unroll
-                    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) part[j][nb][k] = 0.f;
-            }
+        for (int chunk = 0; chunk < (SHARED ? p.x_chunks : 1); ++chunk) {
+            if (SHARED) ok = ok && bounded_wait(BT_FULL(chunk), 0u, abort_flag);
+            uint32_t xat = (uint32_t)chunk * p.x_bytes;
+            int here = SHARED ? min(left, p.x_pairs >> klog) : np;
+            left -= here;
 #pragma unroll 1
-            for (uint32_t h = 0; h < 2; ++h) {
-                uint32_t bf[NB][I8 ? 4 : 8];
+            for (; here > 0; --here, xat += (uint32_t)kstep * PAIR) {
+                cp_wait(D - 1);
+                __syncwarp();                                        // other lanes' chunks of W are here, and they have read the slot before
+                const uint32_t slot = ring + (uint32_t)cs * p.slot_bytes;
+                if (fpass < own) {                                   // into the slot that was consumed one step ago
+                    const uint32_t dst = ring + (uint32_t)fs * p.slot_bytes;
+                    copy_w(dst);
+                    if (!SHARED) copy_x(fi, dst);
+                    advance();
+                }
+                cp_commit();
+                if (!SHARED) xat = slot;
+                float part[GR][NB][4];                               // fp32: the sums of this pair of slices
+                if constexpr (PARTS) {
 #pragma unroll
-                for (int nb = 0; nb < NB; ++nb) bt_fragment<XT>(slot + bat[nb], h, bpiece[nb], bf[nb]);
-                auto half = [&](auto first, auto end) {              // groups [lo, hi) of the warp
-                    constexpr int lo = decltype(first)::value, hi = decltype(end)::value;
-                    uint2 a[GR];
+                    for (int j = 0; j < GR; ++j)
 #pragma unroll
-                    for (int j = lo; j < hi; ++j) a[j] = bt_lds64(slot + (uint32_t)j * 512u + wchunk + h * 8u);
-                    // consecutive MMAs go to different accumulators: a chain of dependent ones costs their full latency each
-                    constexpr int MMAS = I8 ? 2 : 4;
-                    constexpr uint32_t MASK = I8 ? BT_MASK8 : BT_MASK;
+                        for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                    for (int s = 0; s < MMAS; ++s)
+                            for (int k = 0; k < 4; ++k) part[j][nb][k] = 0.f;
+                }
+#pragma unroll 1
+                for (uint32_t h = 0; h < 2; ++h) {
+                    uint32_t bf[NB][I8 ? 4 : 8];
+                    if constexpr (BY_PIECE) bt_pieces<SHARED>(bat[0] + xat, h, bf);
+                    else {
 #pragma unroll
-                        for (int j = lo; j < hi; ++j) {
-                            const uint32_t a0 = a[j].x & MASK, a1 = a[j].y & MASK, a2 = (a[j].x * m4) & MASK, a3 = (a[j].y * m4) & MASK;
-                            if (s < MMAS - 1) a[j].x *= m16, a[j].y *= m16;
+                        for (int nb = 0; nb < NB; ++nb) bt_fragment<XT, SHARED>(bat[nb] + xat, h, bpiece[nb], bf[nb]);
+                    }
+                    auto half = [&](auto first, auto end) {          // groups [lo, hi) of the warp
+                        constexpr int lo = decltype(first)::value, hi = decltype(end)::value;
+                        uint2 a[GR];
 #pragma unroll
-                            for (int nb = 0; nb < NB; ++nb) {
-                                if constexpr (I8) mma_16832(acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
-                                else mma_16816<BF16>(PARTS ? part[j][nb] : acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                        for (int j = lo; j < hi; ++j) a[j] = bt_lds64(slot + (uint32_t)j * 512u + wchunk + h * 8u);
+                        // consecutive MMAs go to different accumulators: a chain of dependent ones costs their full latency each
+                        constexpr int MMAS = I8 ? 2 : 4;
+                        constexpr uint32_t MASK = I8 ? BT_MASK8 : BT_MASK;
+#pragma unroll
+                        for (int s = 0; s < MMAS; ++s)
+#pragma unroll
+                            for (int j = lo; j < hi; ++j) {
+                                const uint32_t a0 = a[j].x & MASK, a1 = a[j].y & MASK, a2 = (a[j].x * m4) & MASK, a3 = (a[j].y * m4) & MASK;
+                                if (s < MMAS - 1) a[j].x *= m16, a[j].y *= m16;
+#pragma unroll
+                                for (int nb = 0; nb < NB; ++nb) {
+                                    if constexpr (I8) mma_16832(acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                                    else mma_16816<BF16>(PARTS ? part[j][nb] : acc[j][nb], a0, a1, a2, a3, bf[nb][2 * s], bf[nb][2 * s + 1]);
+                                }
                             }
-                        }
-                };
-                // a warp's share of a pass is GR groups or one less (or none: GR = 1)
-                if constexpr (GR > 1) half(std::integral_constant<int, 0>{}, std::integral_constant<int, GR - 1>{});
-                if (mine == GR) half(std::integral_constant<int, GR - 1>{}, std::integral_constant<int, GR>{});
+                    };
+                    // a warp's share of a pass is GR groups or one less (or none: GR = 1)
+                    if constexpr (GR > 1) half(std::integral_constant<int, 0>{}, std::integral_constant<int, GR - 1>{});
+                    if (mine == GR) half(std::integral_constant<int, GR - 1>{}, std::integral_constant<int, GR>{});
+                }
+                if constexpr (PARTS) {
+#pragma unroll
+                    for (int j = 0; j < GR; ++j)
+#pragma unroll
+                        for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) acc[j][nb][k] += part[j][nb][k];
+                }
+                if (++cs == S) cs = 0;
             }
-            if constexpr (PARTS) {
-#pragma unroll
-                for (int j = 0; j < GR; ++j)
-#pragma unroll
-                    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) acc[j][nb][k] += part[j][nb][k];
-            }
-            if (++cs == S) cs = 0;
         }
         // ---- sum over the warps that share columns: lane (g, t) holds columns g, g + 8 of W for columns 2t, 2t + 1 of B (20
         // floats apart: no bank conflicts)
@@ -439,9 +534,9 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                 Sum* r = red + (size_t)kw * kw_step + (w0 + j) * MC * 20 + g;
 #pragma unroll
                 for (int nb = 0; nb < NB; ++nb) {
-                    const int m = nb * 8 + 2 * t;
+                    const int m = BY_PIECE ? 6 * t + nb : nb * 8 + 2 * t, m1 = m + (BY_PIECE ? 3 : 1);
                     if (m < MC) r[m * 20] = acc[j][nb][0], r[m * 20 + 8] = acc[j][nb][2];
-                    if (m + 1 < MC) r[(m + 1) * 20] = acc[j][nb][1], r[(m + 1) * 20 + 8] = acc[j][nb][3];
+                    if (m1 < MC) r[m1 * 20] = acc[j][nb][1], r[m1 * 20 + 8] = acc[j][nb][3];
                 }
             }
         __syncthreads();
@@ -460,24 +555,25 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                     for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
             }
             const int n = (c0 + q0 + j) * 16 + c;
+            // (computed where it is used: before the sum it made ptxas allot other registers, 2048 x 2048, eight rows of fp16 3.15 us instead of 2.61)
             const auto address = [&] { return (size_t)m * p.y_step_m + (size_t)n * p.y_step_n; };
             if constexpr (I8) {                                      // an exact multiple of 64
                 if (valid && n < p.N) ((int*)p.Y)[address()] = v >> 6;
                 continue;
             }
-            size_t at = 0;
-            if constexpr (EARLY) at = address();
             const float sc = p.epilogue && (c & 1) ? p.scale2 : p.scale;
             float y = v * sc;
             if (__builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
             if (p.epilogue == 0) {
-                if (valid && n < p.N) store_out(p.Y, p.y_dtype, EARLY ? at : address(), y);
+                if (valid && n < p.N) store_out(p.Y, p.y_dtype, address(), y);
             } else {
                 const float u = __shfl_xor_sync(0xffffffffu, y, 1);
                 if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(y, u));
             }
         }
     }
+    if (!ok) atomicExch(p.status, BT_ERR_WAIT);
+#undef BT_FULL
 }
 
 // one launch of up to BT_MAX_ROWS rows (half of it fp32, twice int8); fills in everything from `own` to `mul16` (bits.cu)

@@ -850,7 +850,7 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
              float scale2, cudaStream_t st, bool y_col = false) {
     BitsParams p{};
     p.pdl = !w.lists;
-    p.bits = w.bits;
+    p.bits = w.bits, p.status = w.status;
     p.x_dtype = x_dtype, p.x_layout = x_layout, p.x_ld = x_ld;
     p.y_dtype = y_dtype, p.epilogue = epilogue;
     p.y_step_n = y_col ? y_ld : 1, p.y_step_m = y_col ? 1 : y_ld;

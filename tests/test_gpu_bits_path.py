@@ -73,6 +73,29 @@ def test_int8_extremes(K, N, M):
     pw.close()
 
 
+# Activations that all warps of a block share: columns cut two and four ways and several passes (groups of sixteen columns per SM), X in one chunk and in two
+# (16 and 17, 32 and 33 pairs of slices), ends of K inside a slice, fewer pairs than warps; rows on 16 bytes, on odd addresses and columns.
+@pytest.mark.parametrize("groups", [3, 5, 7, 13])
+@pytest.mark.parametrize("dtype,M,K", [("f16", 1, 4104), ("f16", 8, 4096), ("bf16", 8, 4232), ("bf16", 16, 2048), ("f16", 16, 2184), ("f32", 6, 2048), ("f32", 7, 2180),
+                                       ("f32", 8, 4228), ("f32", 1, 4100), ("i8", 1, 4112), ("i8", 9, 2192), ("i8", 32, 4096), ("i8", 17, 1168), ("f16", 8, 1000)])
+def test_shared_activations(dtype, M, K, groups):
+    rng = np.random.default_rng(K + groups)
+    N = 16 * groups * torch.cuda.get_device_properties(0).multi_processor_count - 5
+    w = torch.randint(-1, 2, (K, N), dtype=torch.int8, generator=torch.Generator().manual_seed(K))
+    pw = PackedWeight.from_dense(w.numpy())
+    top = 127 if dtype in ("i8", "bf16") else 512
+    X = torch.tensor(rng.integers(-top, top + 1, size=(M, K)), dtype=DT[dtype], device="cuda")
+    want = X.double() @ w.cuda().double()
+    out = torch.empty((M, N), dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+    buf = torch.zeros(M * K + 1, dtype=DT[dtype], device="cuda")
+    buf[1:] = X.reshape(-1)
+    for x, kw in ((X, {}), (buf[1:].view(M, K), {}), (X.t().contiguous(), {"col_major": True})):
+        out.fill_(-1)
+        assert torch.equal(pw.matmul(x, out=out, **kw).double(), want)
+    pw.check()
+    pw.close()
+
+
 # Four blocks of columns of B in registers, rows on 16 bytes: several pairs of slices per warp, slots that are used again, the columns cut two and
 # four ways.
 @pytest.mark.parametrize("M", [17, 24, 31, 32])
