@@ -133,7 +133,8 @@ int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     p.own = q.own, p.own_more = q.own_more, p.split_log = q.split_log, p.per_pass = q.per_pass;
     p.mul4 = 4, p.mul16 = 16;
     p.m_inv = (uint32_t)(((1ull << 32) + p.M - 1) / p.M);
-    const int kp = (p.KB + 1) / 2;
+    const int kp = (p.KB + 1) / 2, ye = p.y_dtype == TLLM_F32 || p.y_dtype == TLLM_I32 ? 4 : 2;
+    p.y_wide = p.epilogue == 0 && p.y_step_n == 1 && p.y_step_m % 4 == 0 && p.N % 4 == 0 && (uintptr_t)p.Y % (4 * ye) == 0;
     const size_t red = (size_t)kparts * p.per_pass * cols * 80;
     // Shared memory: X for all warps together, or a warp's pairs of it beside those of W.  Of these as many in flight as a warp has to fetch and as
     // there is room for: in half of the shared memory, so that the next launch fits beside this one, unless the launch is one of some length

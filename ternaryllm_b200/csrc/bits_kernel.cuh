@@ -26,13 +26,13 @@
 //
 // Measured, fp16, CUDA-graph chain of distinct weights from HBM (us; before = the fastest of the other kernels):
 //   2048 x 2048    1 row  2.3 (gather 3.9)      8 rows  2.6 (batched 11.5)
-//   4096 x 11008   1 row  5.6 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  6.6 (17.2)   16 rows  9.7 (19.5)
-//   8192 x 10240   1 row  9.3 (four-bit planes 15.4)     8 rows 10.9 (22.7)
+//   4096 x 11008   1 row  5.7 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  6.4 (17.2)   16 rows  9.2 (19.5)
+//   8192 x 10240   1 row  9.3 (four-bit planes 15.4)     8 rows 10.7 (22.7)
 // fp32: three MMAs per eight rows, whose values a lane cuts into all three pieces at once (BY_PIECE; each block of columns of B by itself 4.5, 8.0 and 11.5):
 //   2048 x 2048    8 rows  3.7      4096 x 4096    8 rows  6.6       8192 x 2048    8 rows  8.8
 // int8: seven instructions instead of fifteen decode sixteen entries, and two MMAs (m16n8k32) replace four:
-//   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 5.8 in one launch (9.3 in two)
-//   8192 x 10240   1 row  6.9 (12.0)             16 rows 12.3 (22)
+//   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 5.4 in one launch (9.3 in two)
+//   8192 x 10240   1 row  6.9 (12.0)             16 rows 11.8 (22)
 // Of the 9.3 us of 8192 x 10240, 5.4 are there without decode and MMAs; masks and MMAs, which hardly overlap, take 65 to 70 clocks of a scheduler per
 // 1024 entries (53 with the same instructions and nothing to wait for).
 //
@@ -70,6 +70,7 @@ struct BitsParams {
     int x_dtype, x_layout, x_ld;   // row-major X: elements between rows; column-major X: elements between k
     int y_dtype, epilogue;         // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
     long long y_step_n, y_step_m;  // elements from column to column and from row to row of Y
+    bool y_wide;                   // four neighbouring columns are one store
     int M, K, N, KB;               // KB = ceil(K / 64) slices
     int own, own_more;             // groups of sixteen columns per block; the first own_more blocks have one more
     int per_pass;                  // groups per pass (<= split * GR)
@@ -261,12 +262,42 @@ __device__ __forceinline__ void bt_pieces(uint32_t at, uint32_t h, uint32_t (&b)
     }
 }
 
+// elements at .. at + 3, which lie on a multiple of their size
+__device__ __forceinline__ void store_four(void* Y, int dtype, size_t at, const float (&v)[4]) {
+    if (dtype == TLLM_F32) {
+        *(float4*)((float*)Y + at) = make_float4(v[0], v[1], v[2], v[3]);
+        return;
+    }
+    uint32_t w[2];
+    if (dtype == TLLM_F16) {
+        const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
+        w[0] = *reinterpret_cast<const uint32_t*>(&a), w[1] = *reinterpret_cast<const uint32_t*>(&b);
+    } else {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+        w[0] = *reinterpret_cast<const uint32_t*>(&a), w[1] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    *(uint2*)((unsigned short*)Y + at) = make_uint2(w[0], w[1]);
+}
 // column n of row m, entry by entry, for a sum that is not finite
 template <int XT>
 __device__ __noinline__ float bt_column_sum(const BitsParams& p, int n, int m) {
     return column_sum((const uint32_t*)p.bits, n, p.K, p.KB, false, [&](int k) {
         return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + k : (size_t)k * p.x_ld + m);
     });
+}
+// Columns n .. n + 3 of row m again, entry by entry, where one of their sums is not finite (behind the stores of the others, so that next to no register has
+// to live through the call: with the sums kept for it the kernels of 64 registers took half as long again).
+template <int XT>
+__device__ __noinline__ void bt_store_again(const BitsParams& p, int n, int m) {
+    const auto sum = [&](int c) {                                    // (a call of bt_column_sum from here cost the callers registers)
+        return column_sum((const uint32_t*)p.bits, c, p.K, p.KB, false, [&](int k) {
+            return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + k : (size_t)k * p.x_ld + m);
+        });
+    };
+    for (int c = n; c < min(n + 4, p.N); ++c) {
+        if (p.epilogue == 0) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (size_t)c * p.y_step_n, sum(c) * (2.f * p.scale));
+        else if (!(c & 1) && c + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (c >> 1), silu_mul(sum(c) * (2.f * p.scale), sum(c + 1) * (2.f * p.scale2)));
+    }
 }
 
 // A warp multiplies up to GR groups of sixteen columns by NB blocks of eight columns of B (activation rows; fp32: pieces of
@@ -288,6 +319,9 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     // Columns of B: piece of row m is column 3 m + piece; with three blocks of them block `piece` has column m, so that a lane cuts the values of one
     // row and has all of its columns.
     constexpr bool BY_PIECE = XT == TLLM_F32 && NB == 3;
+    // Which of the two ways to add up the warps' sums there is: instances of 64 registers have no room for both (2048 x 2048, eight rows of fp16 2.6 us with
+    // one of them, 3.2 with both).
+    constexpr bool TIGHT = NB == 1 && ASYNC, WIDE = !TIGHT || SHARED || GR > 1, HALF = !TIGHT || !WIDE;
     constexpr uint32_t PAIR = 128u * Act::E;                               // bytes of a row in a pair of slices
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
@@ -540,36 +574,83 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
                 }
             }
         __syncthreads();
-        // half a warp per group and row; idx = group * M + row
-        const int c = lane & 15;
+        // Sums of the warps' sums; idx = group * M + row.  Up to thirty-two of them: half a warp each, a column per thread.
+        if (HALF && (!WIDE || ng * M <= BT_WARPS * 2)) {
+            const int c = lane & 15;
 #pragma unroll 1
-        for (int i0 = warp * 2; i0 < ng * M; i0 += BT_WARPS * 2) {
-            const int idx = i0 + (lane >> 4), j = M > 1 ? (int)__umulhi((uint32_t)idx, p.m_inv) : idx, m = idx - j * M;
-            const bool valid = idx < ng * M;
-            Sum v = 0;
-            if (valid) {
-                const Sum* r = red + (j * MC + m * Act::P) * 20 + c;
+            for (int i0 = warp * 2; i0 < ng * M; i0 += BT_WARPS * 2) {
+                const int idx = i0 + (lane >> 4), j = M > 1 ? (int)__umulhi((uint32_t)idx, p.m_inv) : idx, m = idx - j * M;
+                const bool valid = idx < ng * M;
+                Sum v = 0;
+                if (valid) {
+                    const Sum* r = red + (j * MC + m * Act::P) * 20 + c;
 #pragma unroll
-                for (int pc = Act::P - 1; pc >= 0; --pc)            // fp32: the small pieces first
+                    for (int pc = Act::P - 1; pc >= 0; --pc)        // fp32: the small pieces first
 #pragma unroll 4
-                    for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
+                        for (int w = 0; w < kstep; ++w) v += r[w * kw_step + pc * 20];
+                }
+                const int n = (c0 + q0 + j) * 16 + c;
+                if constexpr (I8) {                                  // an exact multiple of 64
+                    if (valid && n < p.N) ((int*)p.Y)[(size_t)m * p.y_step_m + (size_t)n * p.y_step_n] = v >> 6;
+                    continue;
+                }
+                const float sc = p.epilogue && (c & 1) ? p.scale2 : p.scale;
+                float y = v * sc;
+                if (__builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
+                if (p.epilogue == 0) {
+                    // (the address is computed here: before the sum it made ptxas allot other registers, 2048 x 2048, eight rows of fp16 3.15 us instead of 2.61)
+                    if (valid && n < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (size_t)n * p.y_step_n, y);
+                } else {
+                    const float u = __shfl_xor_sync(0xffffffffu, y, 1);
+                    if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(y, u));
+                }
             }
+            continue;
+        }
+        if constexpr (!WIDE) continue;
+        // More: four columns per thread.  (With a column per thread the loop went round four times as often, each time a chain of some 600 clocks: 16 rows of
+        // fp16 on 2048 x 16384 7.2 us, 6.5 so; 32 of int8 9.7 and 8.7.)
+#pragma unroll 1
+        for (int i = tid; i < ng * M * 4; i += BT_WARPS * 32) {
+            const int idx = i >> 2, c = (i & 3) * 4, j = M > 1 ? (int)__umulhi((uint32_t)idx, p.m_inv) : idx, m = idx - j * M;
+            Sum v[4] = {};
+            const Sum* r = red + (j * MC + m * Act::P) * 20 + c;
+#pragma unroll
+            for (int pc = Act::P - 1; pc >= 0; --pc)
+#pragma unroll 4
+                for (int w = 0; w < kstep; ++w) {
+                    Sum x[4];
+                    *(uint4*)x = *(const uint4*)(r + w * kw_step + pc * 20);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[k] += x[k];
+                }
             const int n = (c0 + q0 + j) * 16 + c;
-            // (computed where it is used: before the sum it made ptxas allot other registers, 2048 x 2048, eight rows of fp16 3.15 us instead of 2.61)
-            const auto address = [&] { return (size_t)m * p.y_step_m + (size_t)n * p.y_step_n; };
-            if constexpr (I8) {                                      // an exact multiple of 64
-                if (valid && n < p.N) ((int*)p.Y)[address()] = v >> 6;
+            size_t at = (size_t)m * p.y_step_m + (size_t)n * p.y_step_n;
+            if constexpr (I8) {                                      // exact multiples of 64
+                if (p.y_wide && n < p.N) *(int4*)((int*)p.Y + at) = make_int4(v[0] >> 6, v[1] >> 6, v[2] >> 6, v[3] >> 6);
+                else
+#pragma unroll
+                    for (int k = 0; k < 4; ++k, at += p.y_step_n)
+                        if (n + k < p.N) ((int*)p.Y)[at] = v[k] >> 6;
                 continue;
             }
-            const float sc = p.epilogue && (c & 1) ? p.scale2 : p.scale;
-            float y = v * sc;
-            if (__builtin_expect(!finite_sum(v), 0)) y = bt_column_sum<XT>(p, min(n, p.N - 1), m) * (2.f * sc);
+            float z = 0.f;                                           // 0, or NaN from the first Inf or NaN on
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z = fmaf((float)v[k], 0.f, z);
             if (p.epilogue == 0) {
-                if (valid && n < p.N) store_out(p.Y, p.y_dtype, address(), y);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] *= p.scale;
+                if (p.y_wide && n < p.N) store_four(p.Y, p.y_dtype, at, (float(&)[4])v);
+                else
+#pragma unroll
+                    for (int k = 0; k < 4; ++k, at += p.y_step_n)
+                        if (n + k < p.N) store_out(p.Y, p.y_dtype, at, v[k]);
             } else {
-                const float u = __shfl_xor_sync(0xffffffffu, y, 1);
-                if (valid && !(c & 1) && n + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (n >> 1), silu_mul(y, u));
+                at = (size_t)m * p.y_step_m + (n >> 1);
+                if (n + 1 < p.N) store_out(p.Y, p.y_dtype, at, silu_mul(v[0] * p.scale, v[1] * p.scale2));
+                if (n + 3 < p.N) store_out(p.Y, p.y_dtype, at + 1, silu_mul(v[2] * p.scale, v[3] * p.scale2));
             }
+            if (__builtin_expect(z != 0.f, 0)) bt_store_again<XT>(p, n, m);
         }
     }
     if (!ok) atomicExch(p.status, BT_ERR_WAIT);

@@ -96,6 +96,33 @@ def test_shared_activations(dtype, M, K, groups):
     pw.close()
 
 
+# Results added up a column per thread and four per thread, stored together and one by one: around thirty-two (group, row) pairs per block, N a multiple of four and
+# not, Y on 16 bytes and not, sums that are not finite among the four
+@pytest.mark.parametrize("dtype", list(DT))
+@pytest.mark.parametrize("M,groups", [(8, 3), (8, 4), (8, 5), (1, 9), (16, 2), (16, 3), (32, 1), (32, 2)])
+def test_sums_of_the_warps(dtype, M, groups):
+    K, N = 520, 16 * groups * torch.cuda.get_device_properties(0).multi_processor_count
+    gen = torch.Generator().manual_seed(M)
+    for n in (N, N - 4, N - 6):
+        w = torch.randint(-1, 2, (K, n), dtype=torch.int8, generator=gen)
+        w[0] = 0
+        w[0, 5], w[0, n - 1] = 1, -1
+        pw = PackedWeight.from_dense(w.numpy())
+        X = torch.randint(-64, 65, (M, K), generator=gen).to(DT[dtype]).cuda()
+        want = X.double() @ w.cuda().double()
+        out = torch.full((M * n + 1,), -1, dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+        for y in (out[:-1].view(M, n), out[1:].view(M, n)):
+            assert torch.equal(pw.matmul(X, out=y).double(), want)
+        if dtype != "i8":
+            X[M - 1, 0] = float("inf")
+            want[M - 1, 5], want[M - 1, n - 1] = float("inf"), -float("inf")
+            got = pw.matmul(X, out=out[:-1].view(M, n)).double()
+            same = want.clone()
+            if not torch.equal(got, same):                           # many rows of 16-bit activations multiply the zeros too: 0 * Inf
+                assert dtype != "f32" and M > 8 and torch.equal(torch.isnan(got[M - 1]), ~torch.isinf(want[M - 1])) and torch.equal(got[:-1], want[:-1])
+        pw.close()
+
+
 # Four blocks of columns of B in registers, rows on 16 bytes: several pairs of slices per warp, slots that are used again, the columns cut two and
 # four ways.
 @pytest.mark.parametrize("M", [17, 24, 31, 32])
