@@ -70,6 +70,7 @@ SIGNATURES = {
     "tllm_weight_check": (_I, [_P]),
     "tllm_spmm": (_I, [_P, _P, _I, _I, _I, _P, _I, _P]),
     "tllm_spmm_host": (_I, [_P, _P, _I, _I, _I, _P, _I, _I]),
+    "tllm_spmm_host_parts": (_I, [_P, _P, _I, _I, _I, _P, _I, _I, _I, _P, _P]),
     "tllm_spmm_host_bias": (_I, [_P, _P, _I, _I, _I, _P, _P, _I, _I]),
     "tllm_spmm_static_scratch": (_I, [_P, _P, _I, _I, _I, _P, _I, _P]),
     "tllm_mlp_create": (_I, [_P, _P, _P, _I, _I, _F, _F, _F, _P, _P]),

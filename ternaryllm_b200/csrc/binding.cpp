@@ -20,6 +20,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <exception>
 #include <string>
 
 #include "../../include/tllm.h"
@@ -60,6 +62,12 @@ struct DeviceScope {
     explicit DeviceScope(c10::DeviceIndex device) {
         if (c10::cuda::current_device() != device) g.set_index(device);
     }
+};
+
+// the interpreter is free for other threads until the end of the scope, exceptions included
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
 };
 
 std::string shape_text(const at::Tensor& t) {
@@ -136,11 +144,17 @@ PyObject* matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // matmul_host(handle, x, x_code, x_col_major, rows, y, y_code, y_col_major, device): x and y are C-contiguous buffers, y writable
 // and of rows * columns elements.  Copies in, runs, copies out, synchronises.
 //
-// A result arrives in page-locked memory at the speed of the bus (4 MB in 86 us) and in pageable memory at that of the one
-// thread that the driver copies it with (257).  Results of some size therefore come through a block of torch's page-locked cache,
-// from which torch's threads copy them (144 with sixteen of them, 210 with four, 309 with two); the block is back in the cache when the
-// call returns, and only calls that run at the same time need more than one.
-constexpr int64_t STAGE_FROM = 256 << 10, STAGE_TO = 16 << 20;
+// The bus moves page-locked memory at 50 GB/s; what is pageable goes through the one thread that the driver copies it with (1 MB in 82 us instead of 20,
+// a result of 4 MB in 257 instead of 86).  Buffers of some size therefore go through blocks of torch's page-locked cache, which torch's threads
+// fill and empty, a result piece by piece while the next one is on the bus; the blocks are back in the cache when the call returns, and only
+// calls that run at the same time need more than two.  (256 columns of fp32, 1024 x 4096, sixteen threads: 214 us, 288 with only the result staged, and
+// in one piece; 2048 x 8192 377 and 504.  Pieces of 1 MB 217 and 383, of 2 MB 236 and 417.)
+constexpr int64_t STAGE_X_FROM = 128 << 10, STAGE_FROM = 256 << 10, STAGE_TO = 16 << 20, STAGE_PART = 512 << 10;
+// straight to the CPU's copy: a dispatch mode of the caller's has no part in it
+void copy_bytes(char* to, const char* from, int64_t n) {
+    at::Tensor t = at::from_blob(to, {n}, at::kByte);
+    at::redispatch::copy_(c10::DispatchKeySet(c10::DispatchKey::CPU), t, at::from_blob(const_cast<char*>(from), {n}, at::kByte));
+}
 PyObject* matmul_host(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     NEED_ARGS(9, "matmul_host")
     BINDING_TRY
@@ -157,19 +171,39 @@ PyObject* matmul_host(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     } x, y;
     if (!x.get(a[1], PyBUF_C_CONTIGUOUS) || !y.get(a[5], PyBUF_C_CONTIGUOUS | PyBUF_WRITABLE)) return nullptr;
     DeviceScope scope((c10::DeviceIndex)v[8]);
-    const int64_t bytes = y.b.len;
-    c10::DataPtr stage;
-    if (bytes >= STAGE_FROM && bytes <= STAGE_TO && at::get_num_threads() >= 4) stage = at::getHostAllocator(at::kCUDA)->allocate((size_t)bytes);
-    void* out = stage.get() ? stage.get() : y.b.buf;
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = tllm_spmm_host((tllm_weight*)v[0], x.b.buf, (int)v[2], v[3] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR, (int)v[4], out, (int)v[6], v[7] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR);
-    Py_END_ALLOW_THREADS
-    if (rc) return raise_rc("tllm_spmm_host", rc);
-    if (stage.get()) {                               // straight to the CPU's copy: a dispatch mode of the caller's has no part in it
-        at::Tensor to = at::from_blob(y.b.buf, {bytes}, at::kByte);
-        at::redispatch::copy_(c10::DispatchKeySet(c10::DispatchKey::CPU), to, at::from_blob(out, {bytes}, at::kByte));
+    const int64_t bytes = y.b.len, x_bytes = x.b.len;
+    const bool threads = at::get_num_threads() >= 4;
+    c10::DataPtr x_stage, y_stage;
+    if (threads && x_bytes >= STAGE_X_FROM && x_bytes <= STAGE_TO) x_stage = at::getHostAllocator(at::kCUDA)->allocate((size_t)x_bytes);
+    if (threads && bytes >= STAGE_FROM && bytes <= STAGE_TO) y_stage = at::getHostAllocator(at::kCUDA)->allocate((size_t)bytes);
+    struct Result {
+        char *to, *from;
+        std::exception_ptr failed;
+    } out{(char*)y.b.buf, (char*)y_stage.get(), nullptr};
+    const auto ready = [](void* a, size_t b, size_t e) {
+        Result* r = (Result*)a;
+        try {
+            copy_bytes(r->to + b, r->from + b, (int64_t)(e - b));
+        } catch (...) {
+            r->failed = std::current_exception();
+        }
+    };
+    int rc = 0;
+    {
+        NoGil no_gil;
+        const void* X = x.b.buf;
+        if (x_stage.get()) {
+            copy_bytes((char*)x_stage.get(), (const char*)X, x_bytes);
+            X = x_stage.get();
+        }
+        const int xl = v[3] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR, yl = v[7] ? TLLM_COL_MAJOR : TLLM_ROW_MAJOR;
+        if (out.from) {
+            const int parts = (int)std::min<int64_t>(TLLM_HOST_PARTS, (bytes + STAGE_PART - 1) / STAGE_PART);
+            rc = tllm_spmm_host_parts((tllm_weight*)v[0], X, (int)v[2], xl, (int)v[4], out.from, (int)v[6], yl, parts, ready, &out);
+        } else rc = tllm_spmm_host((tllm_weight*)v[0], X, (int)v[2], xl, (int)v[4], out.to, (int)v[6], yl);
     }
+    if (rc) return raise_rc("tllm_spmm_host", rc);
+    if (out.failed) std::rethrow_exception(out.failed);
     Py_RETURN_NONE;
     BINDING_CATCH
 }

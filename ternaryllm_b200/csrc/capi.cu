@@ -132,6 +132,7 @@ struct tllm_weight {
     int* h_status = nullptr;        // pinned copy of the status word, read back with every host-buffer call
     size_t x_cap = 0, y_cap = 0, bias_cap = 0;
     cudaStream_t own_stream = nullptr;
+    cudaEvent_t part_event[TLLM_HOST_PARTS] = {};       // tllm_spmm_host_parts: a piece of the result has arrived
     // tensor-core kernel: dense two-bit copy of W and its split scratch
     uint4* d_bits = nullptr;
     float* d_mm_partial = nullptr;
@@ -1465,6 +1466,8 @@ int tllm_weight_destroy(tllm_weight* w) {
     cudaFree(w->d_y);
     cudaFree(w->d_bias);
     if (w->h_status) cudaFreeHost(w->h_status);
+    for (cudaEvent_t e : w->part_event)
+        if (e) cudaEventDestroy(e);
     if (w->own_stream) cudaStreamDestroy(w->own_stream);
     delete w;
     if (g_handles.fetch_sub(1, std::memory_order_relaxed) == 1) ws_trim();
@@ -1622,7 +1625,8 @@ int tllm_spmm(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows
     return run_product(w, X, x_dtype, x_layout, x_ld, rows, Y, y_dtype, L.columns, 0, w->scale, 0.f, (cudaStream_t)stream);
 }
 
-int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows, const void* bias, void* Y, int y_dtype, int y_layout) {
+static int spmm_host(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows, const void* bias, void* Y, int y_dtype, int y_layout, int parts,
+                     void (*ready)(void*, size_t, size_t), void* arg) {
     if (!w || !X || !Y) return fail(TLLM_ERR_ARG, "tllm_spmm_host: NULL pointer");
     if (rows <= 0) return fail(TLLM_ERR_ARG, "tllm_spmm_host: rows must be positive");
     int rc = check_types(x_dtype, y_dtype, "tllm_spmm_host");
@@ -1637,6 +1641,13 @@ int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout
     if (r) return r;
     r = ensure(&w->d_y, &w->y_cap, yb, false);
     if (r) return r;
+    // With page-locked buffers the copies are still under way when something fails behind them: they end before the caller has its buffers back.
+    struct Drain {
+        cudaStream_t st;
+        ~Drain() {
+            if (st) cudaStreamSynchronize(st);
+        }
+    } drain{w->own_stream};
     CU_TRY(cudaMemcpyAsync(w->d_x, X, xb, cudaMemcpyHostToDevice, w->own_stream));
     if (bias) {
         r = ensure(&w->d_bias, &w->bias_cap, (size_t)L.columns * dtype_size(y_dtype), false);
@@ -1666,14 +1677,37 @@ int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout
         out = ws.ptr;
     }
     CU_TRY(cudaMemcpyAsync(w->h_status, w->d_status, sizeof(int), cudaMemcpyDeviceToHost, w->own_stream));
-    CU_TRY(cudaMemcpyAsync(Y, out, yb, cudaMemcpyDeviceToHost, w->own_stream));
+    if (!ready) CU_TRY(cudaMemcpyAsync(Y, out, yb, cudaMemcpyDeviceToHost, w->own_stream));
+    else {
+        const auto from = [&](int i) { return i == parts ? yb : yb / parts * i / 4096 * 4096; };
+        for (int i = 0; i < parts; ++i) {
+            if (!w->part_event[i]) CU_TRY(cudaEventCreateWithFlags(&w->part_event[i], cudaEventDisableTiming));
+            CU_TRY(cudaMemcpyAsync((char*)Y + from(i), (const char*)out + from(i), from(i + 1) - from(i), cudaMemcpyDeviceToHost, w->own_stream));
+            CU_TRY(cudaEventRecord(w->part_event[i], w->own_stream));
+        }
+        for (int i = 0; i < parts; ++i) {
+            CU_TRY(cudaEventSynchronize(w->part_event[i]));
+            ready(arg, from(i), from(i + 1));
+        }
+    }
+    drain.st = nullptr;
     CU_TRY(cudaStreamSynchronize(w->own_stream));
     // the status word came back with the result; only a non-zero one needs the (synchronising) full check
     return *w->h_status ? tllm_weight_check(w) : TLLM_OK;
 }
 
+int tllm_spmm_host_bias(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows, const void* bias, void* Y, int y_dtype, int y_layout) {
+    return spmm_host(w, X, x_dtype, x_layout, rows, bias, Y, y_dtype, y_layout, 1, nullptr, nullptr);
+}
+
 int tllm_spmm_host(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows, void* Y, int y_dtype, int y_layout) {
-    return tllm_spmm_host_bias(w, X, x_dtype, x_layout, rows, nullptr, Y, y_dtype, y_layout);
+    return spmm_host(w, X, x_dtype, x_layout, rows, nullptr, Y, y_dtype, y_layout, 1, nullptr, nullptr);
+}
+
+int tllm_spmm_host_parts(tllm_weight* w, const void* X, int x_dtype, int x_layout, int rows, void* Y, int y_dtype, int y_layout, int parts,
+                         void (*ready)(void* arg, size_t from, size_t to), void* arg) {
+    if (!ready || parts < 1 || parts > TLLM_HOST_PARTS) return fail(TLLM_ERR_ARG, "tllm_spmm_host_parts: 1 to %d parts and a function", TLLM_HOST_PARTS);
+    return spmm_host(w, X, x_dtype, x_layout, rows, nullptr, Y, y_dtype, y_layout, parts, ready, arg);
 }
 
 }  // extern "C"

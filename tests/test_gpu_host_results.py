@@ -97,3 +97,23 @@ def test_more_rows_than_a_grid_is_high():
         assert np.array_equal(y.astype(np.float32), want)
     finally:
         pw.close()
+
+
+# results in one piece, several, as many as there are, ragged last ones, and too large to be staged; activations staged and not; threads that copy and none
+@pytest.mark.parametrize("threads", [1, 8])
+@pytest.mark.parametrize("M,K,N", [(64, 512, 1024), (33, 1000, 2051), (131, 257, 1111), (256, 300, 3001), (301, 1024, 3500), (512, 64, 8200)])
+def test_staged_buffers(M, K, N, threads):
+    rng = np.random.default_rng(N)
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w)
+    before = torch.get_num_threads()
+    torch.set_num_threads(threads)
+    try:
+        for dtype in (np.float32, np.float16, np.int8):
+            x = rng.integers(-3, 4, size=(M, K)).astype(dtype)
+            want = x.astype(np.float32) @ w.astype(np.float32)
+            assert np.array_equal(pw.matmul_host(x).astype(np.float32), want)
+            assert np.array_equal(pw.matmul_host(np.ascontiguousarray(x.T), col_major=True, y_col_major=True).astype(np.float32), want.T)
+    finally:
+        torch.set_num_threads(before)
+        pw.close()
