@@ -350,13 +350,13 @@ int mm_other_bytes(int nt, int planes, int cluster, bool units4) {
     return 1024 + 512 + (units4 ? MS_RAW_UNITS * MS_UNIT_BYTES : MM_RAW_UNITS * MM_UNIT_BYTES) + parts + (planes > 1 && !units4 ? nt * 512 : 0);
 }
 using MmKernel = void (*)(CUtensorMap, CUtensorMap, MmParams);
-MmKernel mm_kernel(int cg, bool units4) { return units4 ? mma_units4_kernel : cg == 2 ? mma_spmm_kernel<2> : mma_spmm_kernel<1>; }
-// clusters of `cluster` blocks (cg = 2: pairs) that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a
+MmKernel mm_kernel(int cg, bool units4, bool pairs) { return units4 ? mma_units4_kernel : cg == 1 ? mma_spmm_kernel<1> : pairs ? mma_spmm_kernel<2, true> : mma_spmm_kernel<2>; }
+// clusters of `cluster` blocks (cg = 2: of one, two or four pairs) that fit on the device at a time: they do not span the groups of 16 to 20 SMs that a
 // GPU is made of
 int mm_clusters(int cluster, int cg, bool units4, int sms, int device) {
     static std::atomic<int> known[64][18];
-    const int slot = (units4 ? 9 : 0) + (cg == 2 ? 1 : cluster);
-    const MmKernel kern = mm_kernel(cg, units4);
+    const int slot = (units4 ? 9 : 0) + (cg == 2 ? cluster - 1 : cluster);      // 2, 4, 8; pairs 1, 3, 7
+    const MmKernel kern = mm_kernel(cg, units4, cg == 2 && cluster > 2);
     int n = device < 64 ? known[device][slot].load(std::memory_order_relaxed) : 0;
     if (n == 0) {
         cudaLaunchConfig_t cfg{};
@@ -409,10 +409,12 @@ MmPlan mm_make_plan(int rows, int planes, int staged, int n_tiles, int kb, int s
             take(nt, mt, 0, 1, cg, false, start2, extra + (std::ceil(tiles / groups) - 1) * std::max(kbu * unit, epilogue + legs) + kbu * unit + epilogue + crowd(tiles * cg, sms));
             const double blocks = std::min(units, groups), parts = std::min((double)kbu, blocks / tiles + 1.0);
             take(nt, mt, 1, 1, cg, false, start2, extra + std::ceil(units / blocks) * unit + 7170.0 + turns * (4.4 * piece + 320.0 * (parts - 1)) + crowd(blocks * cg, sms));
-            for (int c = 2; cg == 1 && c <= 8 && c <= kbu; c *= 2) {
-                const int fit = clusters(c, 1, false);
-                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols * 128 * MM_UK || fit < tiles) continue;
-                take(nt, mt, 2, c, 1, false, start2, (kbu + c - 1) / c * unit + 6900.0 + sixteens * 400.0 + ((sixteens + c - 1) / c + 1) / 2 * piece + crowd(tiles, fit));
+            for (int c = 2; c * cg <= 8 && c <= kbu; c *= 2) {
+                const int fit = clusters(c * cg, cg, false);
+                // pairs: not where the last ones' second blocks would do nothing, nor for a few units, which do not pay for their start
+                if (cg == 2 && (n_tiles % 2 != 0 || kbu < 16 * c)) continue;
+                if (MM_SMEM - mm_other_bytes(nt, planes, c, false) < 2 * cols / cg * 128 * MM_UK || fit < tiles) continue;
+                take(nt, mt, 2, c, cg, false, start2, extra + (kbu + c - 1) / c * unit + 6900.0 + sixteens * 400.0 + ((sixteens + c - 1) / c + 1) / 2 * piece + crowd(tiles, fit));
             }
         }
         // units of four slices
@@ -558,16 +560,19 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     if (rc) return rc;
     const size_t smem = (size_t)other + (size_t)p.SB * b_unit;
     if (smem > MM_SMEM || p.SB < 2) return fail(TLLM_ERR_ARG, "tensor-core kernel: ring configuration needs %zu bytes of shared memory", smem);
-    const MmKernel kern = mm_kernel(cg, plan.units4);
-    static std::once_flag once[3][64];
+    const MmKernel kern = mm_kernel(cg, plan.units4, p.split == 2);
+    static std::once_flag once[4][64];
     cudaError_t err = cudaSuccess;
-    std::call_once(once[plan.units4 ? 2 : cg - 1][w.device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
+    std::call_once(once[plan.units4 ? 2 : cg == 2 && p.split == 2 ? 3 : cg - 1][w.device & 63], [&] { err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM); });
     CU_TRY(err);
     // never more blocks than items: the hand-over between the blocks that share a tile counts on every block in a
     // tile's range of owners holding at least one unit of it
     const long long items = (long long)((p.n_tiles + cg - 1) / cg) * p.m_tiles * (p.split == 1 ? p.KBU : p.cluster);
-    const long long most = cg == 2 ? mm_clusters(2, 2, false, w.sms, w.device) : w.sms;
-    const int grid = (int)std::min(items, most) * cg;
+    const long long most = p.split == 2 ? items : cg == 2 ? mm_clusters(2, 2, false, w.sms, w.device) : w.sms;      // (the plan has seen that a launch's clusters fit)
+    const int groups = (int)std::min(items, most), grid = groups * cg, dealt = p.split == 0 ? (p.n_tiles + cg - 1) / cg * p.m_tiles : (p.n_tiles + cg - 1) / cg * p.m_tiles * p.KBU;
+    p.share = dealt / groups, p.share_more = dealt % groups, p.g_inv = mm_inverse((uint32_t)groups);
+    p.kbu_inv = mm_inverse((uint32_t)p.KBU), p.mt_inv = mm_inverse((uint32_t)p.m_tiles);
+    p.cluster_log = p.cluster == 8 ? 3 : p.cluster / 2;
     Workspace ws;
     if ((p.Nt <= MM_OWN_NT && w.partial) || p.split != 1) p.partial = w.partial;
     else {
@@ -585,7 +590,7 @@ int launch_mm(const BitsView& w, const MmActs& x, int rows, const MmOut& o, cuda
     at[n_at++] = pdl_attribute();
     if (p.split == 2 || cg == 2) {
         at[n_at].id = cudaLaunchAttributeClusterDimension;
-        at[n_at].val.clusterDim.x = (unsigned)(cg == 2 ? 2 : p.cluster), at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
+        at[n_at].val.clusterDim.x = (unsigned)(cg * (p.split == 2 ? p.cluster : 1)), at[n_at].val.clusterDim.y = 1, at[n_at].val.clusterDim.z = 1;
         ++n_at;
     }
     cfg.attrs = at;

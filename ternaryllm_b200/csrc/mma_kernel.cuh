@@ -40,9 +40,10 @@
 // cut into equal contiguous ranges, one per block or pair.  Tiles that straddle two or more blocks are summed in block order by the
 // last block to arrive, which makes the result independent of scheduling; a block does its two shared tiles first, so that
 // this adding-up hides behind the tiles it has to itself.
-// With few tiles a third way: a cluster of two, four or eight blocks cuts the units of one tile.  Each block sends its sums of the rows
-// that another one is to write straight into that one's shared memory, so that a hand-over costs one trip between SMs, not
-// partial sums to L2, a counter and partial sums back, and every block adds and writes a share of the tile.
+// With few tiles a third way: a cluster of two, four or eight blocks, or of two or four pairs, cuts the units of one tile.  Each block sends its sums
+// of the rows that another one is to write straight into that one's shared memory, so that a hand-over costs one trip between SMs, not
+// partial sums to L2, a counter and partial sums back, and every block adds and writes a share of the tile.  (A block of a pair deals with
+// the blocks of the other pairs that have its 128 columns.  256 rows of fp32 on 8192 x 2048: 26.6 us, 31.2 in equal ranges of units.)
 //
 // Every wait is bounded (see bounded_wait); on a time-out the block raises its abort flag, every role leaves
 // its loop, tensor memory is released and the status word reports the failure.
@@ -96,7 +97,11 @@ struct MmParams {
     int n_tiles, m_tiles;
     int Nt;                   // activation rows per tile; planes * Nt is the MMA's N
     int split;                // 0: whole tiles; 1: equal unit ranges, tiles may be shared; 2: a cluster per tile
-    int cluster;              // blocks per tile, split 2
+    int cluster;              // blocks (CG = 2: pairs) per tile, split 2
+    // How the work is dealt out (split 0: tiles, 1: units): every one of the G blocks or pairs has `share`, `share_more` of them one more; and what divisions by
+    // G, KBU and m_tiles multiply with (mm_div).  (64-bit divisions in the kernel took 1500 clocks before its first copy, and again at every shared tile.)
+    int share, share_more, cluster_log;
+    uint32_t g_inv, kbu_inv, mt_inv;
     int P;                    // planes of X
     int out;                  // MM_OUT_*
     int epilogue, y_ld;       // epilogue 1: columns are (gate, up) pairs, Y[c / 2] = silu(g * scale) * (u * scale2)
@@ -167,12 +172,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// the barrier (CG = 2: that of both blocks) receives one arrival when every MMA issued so far by this thread has completed
+// the barrier (CG = 2: that of the cluster's blocks `both`) receives one arrival when every MMA issued so far by this thread has completed
 template <int CG = 1>
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t both = 3u) {
     if (CG == 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
     else
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)both)
                      : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
@@ -299,6 +304,27 @@ __device__ __forceinline__ bool bounded_spin(uint32_t bar, uint32_t parity, vola
     }
 }
 
+// a wait for the first phase of a barrier at which other blocks arrive behind their writes to this one's shared memory (with a fence behind a wait that acquires
+// for the block alone, 950 clocks)
+__device__ __forceinline__ bool mm_wait_cluster(uint32_t bar, volatile int* abort_flag) {
+    const long long t0 = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar)
+            : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > TLLM_WAIT_LIMIT_CLOCKS) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
 // waiting roles are parked (bounded_wait): spinning ones took issue slots from the epilogue; only the thread that issues MMAs spins
 #define MM_WAIT(bar, par)                             \
     do {                                                    \
@@ -329,9 +355,22 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- clusters (split 2) ----------------------------------------------------------------------------------
-__device__ __forceinline__ void mm_cluster_sync() {
+__device__ __forceinline__ void mm_cluster_arrive() {
     __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mm_cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mm_cluster_sync() {
+    mm_cluster_arrive();
+    mm_cluster_wait();
+}
+// barriers made by this thread, for the other blocks' arrivals and for the TMA unit's
+__device__ __forceinline__ void mm_fence_barriers() {
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 // address of this block's shared location in block `rank`
 __device__ __forceinline__ uint32_t mm_peer(uint32_t addr, uint32_t rank) {
@@ -344,19 +383,36 @@ __device__ __forceinline__ void mm_st_peer(uint32_t addr, float a, float b, floa
 }
 // An arrival at the barrier of a pair's first block: what it stands for is tensor memory, which the tcgen05 waits and fences before it
 // have taken care of, so that nothing has to be released with it.  (With release.cluster it waited for the thread's other writes too: 2500 clocks.)
-__device__ __forceinline__ void mm_arrive_first(uint32_t bar) {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mm_peer(bar, 0u)) : "memory");
+__device__ __forceinline__ void mm_arrive_first(uint32_t bar, uint32_t first) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mm_peer(bar, first)) : "memory");
 }
 __device__ __forceinline__ void mm_arrive_peer(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 // column (of the 32 of a quarter tile) that lane `lane` of tensor memory's quarter holds
 __device__ __forceinline__ int mm_column(int lane) { return ((lane >> 1) & 1) * 16 + (lane & 1) * 8 + (lane >> 2); }
 
+// a / d, inv = ceil(2^32 / d)
+__host__ __device__ __forceinline__ uint32_t mm_inverse(uint32_t d) { return d == 1 ? 0u : 0xFFFFFFFFu / d + 1u; }
+__device__ __forceinline__ int mm_div(int a, int d, uint32_t inv) {
+    if (d == 1) return a;
+    const uint32_t q = __umulhi((uint32_t)a, inv);
+    return (int)(q * (uint32_t)d > (uint32_t)a ? q - 1u : q);
+}
+// first tile or unit of block or pair c of G
+__device__ __forceinline__ int mm_share(const MmParams& p, int c, int G) { return c * p.share + mm_div(c * p.share_more, G, p.g_inv); }
+// whose unit u is (split 1)
+__device__ __forceinline__ int mm_owner(const MmParams& p, int u, int G, int total) {
+    int c = min(G - 1, (int)((float)u * (float)G / (float)total));
+    while (c + 1 < G && mm_share(p, c + 1, G) <= u) ++c;
+    while (mm_share(p, c, G) > u) --c;
+    return c;
+}
+
 // The segments of a block's unit range [u0, u1): one per output tile it touches; the first and the last, which other blocks may
 // share, come first.
 struct MmSegs {
     int u0, u1, KBU, t0, n;
-    __device__ __forceinline__ MmSegs(int a, int b, int kbu) : u0(a), u1(b), KBU(kbu), t0(a / kbu), n((b - 1) / kbu - a / kbu + 1) {}
+    __device__ __forceinline__ MmSegs(int a, int b, int kbu, uint32_t inv) : u0(a), u1(b), KBU(kbu), t0(mm_div(a, kbu, inv)), n(mm_div(b - 1, kbu, inv) - t0 + 1) {}
     // segment i: its tile, the tile's units [ua, ub), and which of the block's two slots a partial sum goes to
     __device__ __forceinline__ void get(int i, int& tile, int& ua, int& ub, int& slot) const {
         const int j = i < 2 ? (i ? n - 1 : 0) : i - 1;
@@ -364,6 +420,23 @@ struct MmSegs {
         const int f = tile * KBU;
         ua = max(u0 - f, 0), ub = min(u1 - f, KBU);
         slot = j ? 1 : 0;
+    }
+};
+
+// the units of those segments one after the other, for the thread that loads bit tiles
+struct MmBitsRange {
+    const MmSegs& segs;
+    const MmParams& p;
+    int cg, member, i = 0, ku = 0, ub = 0, row0 = 0;
+    __device__ __forceinline__ MmBitsRange(const MmSegs& s, const MmParams& q, int c, int m) : segs(s), p(q), cg(c), member(m) { open(); }
+    __device__ __forceinline__ bool left() const { return i < segs.n; }
+    __device__ __forceinline__ void next() {
+        if (++ku == ub && ++i < segs.n) open();
+    }
+    __device__ __forceinline__ void open() {
+        int tile, slot;
+        segs.get(i, tile, ku, ub, slot);
+        row0 = (mm_div(tile, p.m_tiles, p.mt_inv) * cg + member) * 8;
     }
 };
 
@@ -546,7 +619,9 @@ __device__ __forceinline__ void mm_with_out(const MmParams& p, F f) {
 // accumulators of more than 128 columns.
 __host__ __device__ __forceinline__ uint32_t mm_a_units_log(uint32_t acc_cols) { return acc_cols <= 128 ? 2u : 1u; }
 
-template <int CG>
+// PAIRS: pairs of blocks (CG = 2) in clusters of several; an instance of its own, since with the place of a pair in its cluster as a variable the others took
+// 3 to 7 % longer (512 rows of fp16 on 2048 x 16384 34.5 us, 32.4 with constants)
+template <int CG, bool PAIRS = false>
 __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap wmap,
                                                                  const __grid_constant__ MmParams p) {
     extern __shared__ unsigned char mm_smem[];
@@ -555,15 +630,18 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     // ---- the unit range of this block or pair ------------------------------------------------------------
     const int G = (int)gridDim.x / CG, cta = (int)blockIdx.x / CG, member = CG == 2 ? (int)blockIdx.x & 1 : 0;
     const int KBU = p.KBU, KB = p.KB, tiles = (p.n_tiles + CG - 1) / CG * p.m_tiles;
-    const long long total = (long long)tiles * KBU;
-    const bool clustered = CG == 1 && p.split == 2;
-    const int C = clustered ? p.cluster : 1, rank = clustered ? cta % C : 0;
+    const int total = tiles * KBU;
+    const bool clustered = PAIRS || (CG == 1 && p.split == 2);
+    const int C = clustered ? p.cluster : 1, rank = clustered ? cta & (C - 1) : 0;
+    const uint32_t first = PAIRS ? (uint32_t)(rank * CG) : 0u, both = 3u << first;              // the pair's blocks in the cluster
     int u0, u1;
-    if (clustered) u0 = cta / C * KBU + KBU * rank / C, u1 = cta / C * KBU + KBU * (rank + 1) / C;
-    else if (p.split) u0 = (int)(total * cta / G), u1 = (int)(total * (cta + 1) / G);
-    else u0 = (int)((long long)tiles * cta / G) * KBU, u1 = (int)((long long)tiles * (cta + 1) / G) * KBU;
+    if (clustered) u0 = (cta >> p.cluster_log) * KBU, u1 = u0 + (KBU * (rank + 1) >> p.cluster_log), u0 += KBU * rank >> p.cluster_log;
+    else {
+        u0 = mm_share(p, cta, G), u1 = mm_share(p, cta + 1, G);
+        if (!p.split) u0 *= KBU, u1 *= KBU;
+    }
     if (u0 >= u1) return;                  // never in a cluster: KBU >= C
-    const MmSegs segs(u0, u1, KBU);
+    const MmSegs segs(u0, u1, KBU, p.kbu_inv);
 
     // ---- shared memory ---------------------------------------------------------------------------------
     const uint32_t raw0 = smem_u32(mm_smem);
@@ -591,28 +669,51 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 #define ACC_EMPTY(a) (bar_base + 8u * (50u + (uint32_t)(a)))
 #define PART_FULL(q) (bar_base + 8u * (52u + (uint32_t)(q)))
 
-    if (tid == 0) {
-        for (int s = 0; s < MM_MAX_STAGES; ++s) {
-            mbar_init(A_FULL(s), (fine ? 4 : 8) * CG);      // the decoder warps of a slice or unit (of a pair: at the first block)
-            mbar_init(A_EMPTY(s), 1);      // tcgen05.commit
-            mbar_init(B_FULL(s), 1);       // the TMA thread's expect_tx arrival
-            mbar_init(B_EMPTY(s), 1);      // tcgen05.commit
-            mbar_init(RAW_FULL(s), 1);
-            mbar_init(RAW_EMPTY(s), 8);    // half of the decoder warps
+    // Start: warp 0 has the first bit tiles on their way as soon as their barriers exist, warp 1 takes tensor memory, warps 2 and 3 make the other
+    // barriers, a thread each, and one barrier of the block or cluster ends it.  (One thread making sixty barriers, then tensor memory, then the first copies took
+    // 4000 to 4600 clocks to here, 2500 in mma_units4_kernel, and 2800 more to the first expanded slice; with 64-bit divisions gone as well, and the
+    // cluster waited for later, us before / now: 24 rows of fp32 on 2048 x 2048 10.4 / 9.4, 256 on 2048 x 8192 24.8 / 24.0, 256 of fp16 on
+    // 512 x 3000 6.4 / 6.1.)
+    MmBitsRange load(segs, p, CG, member);
+    if (warp == 0) {
+        if (lane < 16) mbar_init(RAW_FULL(lane), lane < 8 ? 1 : 8);             // RAW_EMPTY: half of the decoder warps
+        mm_fence_barriers();
+        __syncwarp();
+        // The weights do not depend on the preceding kernel.  A tile's eight groups of sixteen columns are eight streams along K; the tensor map sees them
+        // as eight rows, and one box of 8 x 512 bytes is a unit; past the end of K it is filled with zeros, which count.  (Eight bulk copies
+        // instead, one per lane, took 820 clocks a unit to issue.)
+        if (!p.wait_bits && elect_one())
+            for (uint32_t r = 0; r < R && load.left(); ++r, load.next()) {
+                mbar_expect_tx(RAW_FULL(r), MM_UNIT_BYTES);
+                tma_load_2d(r_base + r * MM_UNIT_BYTES, &wmap, load.ku * (MM_UK * 64), load.row0, RAW_FULL(r));
+            }
+        __syncwarp();
+    } else if (warp == 1) {
+        tmem_alloc<CG>(smem_u32((const void*)flags), 512);
+    } else if (warp < 4) {
+        const int i = tid - 64;                                                // the order of the names above
+        if (i < 60 && (i < 32 || i >= 48)) {
+            const int n = i < 8 ? (fine ? 4 : 8) * CG                          // the decoder warps of a slice or unit (of a pair: at the first block)
+                        : i < 16 ? 1                                           // tcgen05.commit
+                        : i < 24 ? 1                                           // the TMA thread's expect_tx arrival
+                        : i < 50 ? 1                                           // tcgen05.commit
+                        : i < 52 ? 8 * CG                                      // the epilogue warps
+                                 : max(C - 1, 1);                              // the same warp of the other blocks
+            mbar_init(bar_base + 8u * (uint32_t)i, (uint32_t)n);
         }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(ACC_FULL(a), 1);
-            mbar_init(ACC_EMPTY(a), 8 * CG);    // the epilogue warps
+        if (i == 63) {
+            flags[1] = 0;
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap) : "memory");
         }
-        for (int q = 0; q < 8; ++q) mbar_init(PART_FULL(q), (uint32_t)max(C - 1, 1));   // the same warp of the other blocks
-        flags[0] = 0;
-        flags[1] = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mm_fence_barriers();
     }
-    if (CG == 2 || clustered) mm_cluster_sync();      // the others' barriers exist
-    else __syncthreads();
-    if (warp == 1) tmem_alloc<CG>(smem_u32((const void*)flags), 512);
+    // The other blocks' barriers are waited for where they are needed (join): blocks of a cluster start up to 1300 clocks apart, and the first tiles are expanded
+    // meanwhile.
+    if (CG == 2 || clustered) mm_cluster_arrive();
+    bool joined = CG == 1 && !clustered;
+    const auto join = [&] {
+        if (!joined) mm_cluster_wait(), joined = true;
+    };
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -623,26 +724,21 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     // Every role walks the same list of segments.  The producers and the issuer are one thread each: with the whole warp in the loop and a
     // lane elected per block of instructions, eight MMAs and two commits took 220 clocks to issue, by one thread 105.
     if (warp == 0) {
-        // ---- bit-tile producer: the weights do not depend on the preceding kernel, so this starts at once.  A tile's eight groups
-        // of sixteen columns are eight streams along K; the tensor map sees them as eight rows, and one box of 8 x 512 bytes is
-        // a unit.  (Eight bulk copies instead, one per lane, took 820 clocks a unit to issue.)
+        // ---- bit-tile producer, behind the first round of its ring
         if (elect_one()) {
-            if (p.wait_bits) pdl_wait();
             uint32_t r = 0, rph = 0;
-            for (int i = 0; i < segs.n; ++i) {
-                int tile, ua, ub, sl;
-                segs.get(i, tile, ua, ub, sl);
-                const int row0 = (tile / p.m_tiles * CG + member) * 8;
-                for (int ku = ua; ku < ub; ++ku) {
-                    MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
-                    mbar_expect_tx(RAW_FULL(r), MM_UNIT_BYTES);          // past the end of K the box is filled with zeros, which count
-                    tma_load_2d(r_base + r * MM_UNIT_BYTES, &wmap, ku * (MM_UK * 64), row0, RAW_FULL(r));
-                    MM_ADVANCE(r, rph, R);
-                }
+            if (p.wait_bits) pdl_wait();
+            else rph = 1u;
+            for (; load.left(); load.next()) {
+                MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
+                mbar_expect_tx(RAW_FULL(r), MM_UNIT_BYTES);
+                tma_load_2d(r_base + r * MM_UNIT_BYTES, &wmap, load.ku * (MM_UK * 64), load.row0, RAW_FULL(r));
+                MM_ADVANCE(r, rph, R);
             }
         }
     } else if (warp == 2) {
         // ---- activation producer: a unit is two TMA boxes (all planes of a slice each) on one barrier
+        if (CG == 2) join();
         if (elect_one()) {
             pdl_wait();
             uint32_t b = 0, bph = 0;
@@ -650,11 +746,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             for (int i = 0; i < segs.n; ++i) {
                 int tile, ua, ub, sl;
                 segs.get(i, tile, ua, ub, sl);
-                const int row0 = (tile % p.m_tiles) * Nt + member * rows;
+                const int row0 = (tile - mm_div(tile, p.m_tiles, p.mt_inv) * p.m_tiles) * Nt + member * rows;
                 for (int ku = ua; ku < ub; ++ku) {
                     const bool two = ku * MM_UK + 1 < KB;
                     MM_WAIT(B_EMPTY(b), bph ^ 1u);
-                    const uint32_t full = CG == 1 ? B_FULL(b) : mm_peer(B_FULL(b), 0u), to = b_base + b * b_unit;
+                    const uint32_t full = CG == 1 ? B_FULL(b) : mm_peer(B_FULL(b), first), to = b_base + b * b_unit;
                     if (member == 0) mbar_expect_tx(B_FULL(b), (two ? 2u : 1u) * CG * b_slice);
                     // (three planes as three boxes a slice would be six instructions to issue; one plane as a box of three dimensions
                     // measured 4 % slower than one of two)
@@ -672,6 +768,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     } else if (warp == 1) {
         // ---- MMA issuer; of a pair the first block's.  Nothing but the MMAs' own time lies between two of them as long as the next unit's
         // operands are there: the tensor core has some in its queue while this thread looks.
+        if (CG == 2) join();
         if (member == 0 && elect_one()) {
             const uint32_t idesc = p.idesc, b_lo0 = (b_base >> 4) & 0x3FFFu;
             uint32_t u = 0, sb = 0, sbph = 0, a = 0, aph = 0;
@@ -693,7 +790,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4) umma_f16_ts<CG>(d, at + 8u * k4, b_lo + 2u * k4, idesc, k4 == 0 ? acc : 1u);
                     if (fine) {
-                        umma_commit<CG>(A_EMPTY(2u * sa));
+                        umma_commit<CG>(A_EMPTY(2u * sa), both);
                         MM_SPIN(A_FULL(2u * sa + 1u), saph);
                         tc_fence_after();
                     }
@@ -701,12 +798,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
 #pragma unroll
                         for (uint32_t k4 = 0; k4 < MM_TILE_K / 16; ++k4) umma_f16_ts<CG>(d, at + 32u + 8u * k4, b_lo + (b_slice >> 4) + 2u * k4, idesc, 1u);
                     }
-                    umma_commit<CG>(A_EMPTY(fine ? 2u * sa + 1u : sa));
-                    umma_commit<CG>(B_EMPTY(sb));
+                    umma_commit<CG>(A_EMPTY(fine ? 2u * sa + 1u : sa), both);
+                    umma_commit<CG>(B_EMPTY(sb), both);
                     MM_ADVANCE(sb, sbph, SB);
                     acc = 1;
                     if (--left == 0) {
-                        umma_commit<CG>(ACC_FULL(a));
+                        umma_commit<CG>(ACC_FULL(a), both);
                         MM_ADVANCE(a, aph, 2u);
                     }
                 }
@@ -724,6 +821,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         uint32_t m4, m16;
         asm volatile("mov.b32 %0, %2;\n\tmov.b32 %1, %3;" : "=r"(m4), "=r"(m16) : "r"(p.mul4), "r"(p.mul16));
         uint32_t n = 0;                                       // units so far
+        if (CG == 2) join();                                  // (in the loop, behind the first unit's values, it cost every unit 1 %)
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
@@ -760,7 +858,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 __syncwarp();
                 if (lane == 0) {
                     if (CG == 1) mbar_arrive(A_FULL(bar));
-                    else mm_arrive_first(A_FULL(bar));
+                    else mm_arrive_first(A_FULL(bar), first);
                 }
             }
         }
@@ -768,11 +866,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         // ---- epilogue: a warp may read the 32 tensor-memory lanes selected by warp % 4; of the sixteens of rows it has every other one (of
         // those that a block of a cluster writes, too)
         const int q = warp & 3, odd = (warp >> 2) - 1, nl = q * 32 + lane, ncol = q * 32 + mm_column(lane);
+        join();
         pdl_wait();
         uint32_t a = 0, aph = 0;
         const auto acc_free = [&](uint32_t bar) {
             if (CG == 1) mbar_arrive(bar);
-            else mm_arrive_first(bar);
+            else mm_arrive_first(bar, first);
         };
         // Columns of D: rows [0, Nt / 2) of X of each plane, which a pair's first block holds, and then the other's.
         const int rows = Nt / CG;
@@ -780,7 +879,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
-            const int mt = tile % p.m_tiles, nt = tile / p.m_tiles * CG + member;      // nt: this block's tile of 128 columns; the last of an odd number has no pair
+            const int ct = mm_div(tile, p.m_tiles, p.mt_inv), mt = tile - ct * p.m_tiles, nt = ct * CG + member;      // nt: this block's tile of 128 columns; the last of an odd number has no pair
             const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16), run = run_base + (uint32_t)nl * 4u;
             // all legs but the last join the sum in shared memory
             bool legs = false;
@@ -830,15 +929,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                     if (o == rank || ((c / C) & 1) != odd) continue;
                     float f[16];
                     load16(16 * c, f);
-                    const uint32_t to = mm_peer(part_base + (uint32_t)(((rank * own + c / C) * 4) * 128 + nl) * 16u, (uint32_t)o);
+                    const uint32_t to = mm_peer(part_base + (uint32_t)(((rank * own + c / C) * 4) * 128 + nl) * 16u, (uint32_t)(o * CG + member));
 #pragma unroll
                     for (int t = 0; t < 4; ++t) mm_st_peer(to + (uint32_t)t * 2048u, f[4 * t], f[4 * t + 1], f[4 * t + 2], f[4 * t + 3]);
                 }
                 __syncwarp();
-                if (lane < C && lane != rank && lane < sixteens) mm_arrive_peer(mm_peer(PART_FULL(4 * odd + q), (uint32_t)lane));
+                if (lane < C && lane != rank && lane < sixteens) mm_arrive_peer(mm_peer(PART_FULL(4 * odd + q), (uint32_t)(lane * CG + member)));
                 if (rank < sixteens) {
-                    MM_WAIT(PART_FULL(4 * odd + q), 0u);
-                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    if (!mm_wait_cluster(PART_FULL(4 * odd + q), abort_flag)) goto done;
                     mm_with_out(p, [&](auto out, auto silu) {
                         uint32_t at0 = part_base + (uint32_t)nl * 16u + (uint32_t)odd * 8192u;
                         for (int c = rank + odd * C; c < sixteens; c += 2 * C, at0 += 16384u) {
@@ -854,7 +952,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                                         f[4 * t] += __uint_as_float(x.x), f[4 * t + 1] += __uint_as_float(x.y), f[4 * t + 2] += __uint_as_float(x.z), f[4 * t + 3] += __uint_as_float(x.w);
                                     }
                                 }
-                            finish16(out, silu, f, n, mt * Nt + 16 * c);
+                            if (CG == 1 || nt < p.n_tiles) finish16(out, silu, f, n, mt * Nt + 16 * c);
                         }
                     });
                 }
@@ -862,8 +960,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
                 // The last of the blocks that share this tile to arrive adds the partial sums, in block order.  Each epilogue warp owns 32
                 // columns of the tile and runs the hand-over for them by itself.  The last block's own part stays in tensor memory;
                 // a block that finds all the others there already does not even write it.
-                const long long first_unit = (long long)tile * KBU, last_unit = first_unit + KBU - 1;
-                cf = (int)(((first_unit + 1) * G + total - 1) / total - 1), cl = (int)(((last_unit + 1) * G + total - 1) / total - 1);
+                cf = mm_owner(p, tile * KBU, G, total), cl = mm_owner(p, tile * KBU + KBU - 1, G, total);
                 unsigned int* ctr = p.counters + ((size_t)nt * p.m_tiles + mt) * 4 + q;
                 const unsigned int others = (unsigned int)(cl - cf);
                 const uint32_t field = 16u * (uint32_t)odd;      // the two warps of a column count in halves of one word
@@ -889,7 +986,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
             }
             if (!clustered && (full || sum) && (CG == 1 || nt < p.n_tiles)) {
                 // A part lies in its block's slot 0, except that the first block may have come from an earlier tile.
-                const float* part0 = p.partial + (size_t)(2 * (cf * CG + member) + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
+                const float* part0 = p.partial + (size_t)(2 * (cf * CG + member) + (!full && mm_share(p, cf, G) >= tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * ((cf + 1) * CG + member)) * slot_floats + nl * 4;
                 mm_with_out(p, [&](auto out, auto silu) {
                     for (int c16 = 16 * odd; c16 < Nt; c16 += 32) {
@@ -927,6 +1024,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) mma_spmm_kernel(const __grid_co
     }
 done:
     __syncwarp();
+    join();
     tc_fence_before();
     if (CG == 2) mm_cluster_sync();        // the pair's MMAs read both blocks' shared and tensor memory
     else __syncthreads();

@@ -75,15 +75,17 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
 
     // ---- this block's unit range -----------------------------------------------------------------------
     const int G = (int)gridDim.x, cta = (int)blockIdx.x, KBU = p.KBU, KB = p.KB, tiles = p.n_tiles * p.m_tiles;
-    const long long total = (long long)tiles * KBU;
+    const int total = tiles * KBU;
     const bool clustered = p.split == 2;
-    const int C = clustered ? p.cluster : 1, rank = clustered ? cta % C : 0;
+    const int C = clustered ? p.cluster : 1, rank = clustered ? cta & (C - 1) : 0;
     int u0, u1;
-    if (clustered) u0 = cta / C * KBU + KBU * rank / C, u1 = cta / C * KBU + KBU * (rank + 1) / C;
-    else if (p.split) u0 = (int)(total * cta / G), u1 = (int)(total * (cta + 1) / G);
-    else u0 = (int)((long long)tiles * cta / G) * KBU, u1 = (int)((long long)tiles * (cta + 1) / G) * KBU;
+    if (clustered) u0 = (cta >> p.cluster_log) * KBU, u1 = u0 + (KBU * (rank + 1) >> p.cluster_log), u0 += KBU * rank >> p.cluster_log;
+    else {
+        u0 = mm_share(p, cta, G), u1 = mm_share(p, cta + 1, G);
+        if (!p.split) u0 *= KBU, u1 *= KBU;
+    }
     if (u0 >= u1) return;                  // never in a cluster: KBU >= C
-    const MmSegs segs(u0, u1, KBU);
+    const MmSegs segs(u0, u1, KBU, p.kbu_inv);
 
     // ---- shared memory ---------------------------------------------------------------------------------
     const uint32_t raw0 = smem_u32(mm_smem);
@@ -107,28 +109,42 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
 #define ACC_EMPTY(a) (bar_base + 8u * (50u + (uint32_t)(a)))
 #define PART_FULL(q) (bar_base + 8u * (52u + (uint32_t)(q)))
 
-    if (tid == 0) {
-        for (int s = 0; s < MM_MAX_STAGES; ++s) {
-            mbar_init(A_FULL(s), 16);      // the decoder warps
-            mbar_init(A_EMPTY(s), 1);      // tcgen05.commit
-            mbar_init(B_FULL(s), 1);       // the TMA thread's expect_tx arrival
-            mbar_init(B_EMPTY(s), 1);      // tcgen05.commit
-            mbar_init(RAW_FULL(s), 1);
-            mbar_init(RAW_EMPTY(s), 16);   // the decoder warps
+    // Start, as in mma_kernel.cuh: the first bit tiles on their way, tensor memory and the other barriers beside one another.
+    MmBitsRange load(segs, p, 1, 0);
+    if (warp == 0) {
+        if (lane < 16) mbar_init(RAW_FULL(lane), lane < 8 ? 1 : 16);            // RAW_EMPTY: the decoder warps
+        mm_fence_barriers();
+        __syncwarp();
+        // The weights do not depend on the preceding kernel, unless that is the one that makes them.  A unit is one box of 8 x 1024 bytes; past the end
+        // of K it is filled with zeros, which count.
+        if (!p.wait_bits && elect_one())
+            for (uint32_t r = 0; r < R && load.left(); ++r, load.next()) {
+                mbar_expect_tx(RAW_FULL(r), MS_UNIT_BYTES);
+                tma_load_2d(r_base + r * MS_UNIT_BYTES, &wmap, load.ku * (MS_UK * 64), load.row0, RAW_FULL(r));
+            }
+        __syncwarp();
+    } else if (warp == 1) {
+        tmem_alloc(smem_u32((const void*)flags), 512);
+    } else if (warp < 4) {
+        const int i = tid - 64;                                                // the order of the names above
+        if (i < 56 && (i < 32 || i >= 48)) {
+            const int n = i < 8 ? 16                                           // the decoder warps
+                        : i < 50 ? 1                                           // tcgen05.commit; B_FULL: the TMA thread's expect_tx arrival
+                        : i < 52 ? 4                                           // the four epilogue warps
+                                 : max(C - 1, 1);                              // the same warp of the other blocks
+            mbar_init(bar_base + 8u * (uint32_t)i, (uint32_t)n);
         }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(ACC_FULL(a), 1);
-            mbar_init(ACC_EMPTY(a), 4);    // the four epilogue warps
+        if (i == 63) {
+            flags[1] = 0;
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap) : "memory");
         }
-        for (int q = 0; q < 4; ++q) mbar_init(PART_FULL(q), (uint32_t)max(C - 1, 1));   // the same warp of the other blocks
-        flags[0] = 0;
-        flags[1] = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mm_fence_barriers();
     }
-    if (clustered) mm_cluster_sync();      // the others' barriers exist
-    else __syncthreads();
-    if (warp == 1) tmem_alloc(smem_u32((const void*)flags), 512);
+    if (clustered) mm_cluster_arrive();    // the others' barriers are waited for where they are needed
+    bool joined = !clustered;
+    const auto join = [&] {
+        if (!joined) mm_cluster_wait(), joined = true;
+    };
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -139,21 +155,16 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
 
     // Every role walks the same list of segments.
     if (warp == 0) {
-        // ---- bit-tile producer: the weights do not depend on the preceding kernel (unless that is the one that makes them), so this starts at
-        // once.  A unit is one box of 8 x 1024 bytes.
+        // ---- bit-tile producer, behind the first round of its ring
         if (elect_one()) {
-            if (p.wait_bits) pdl_wait();
             uint32_t r = 0, rph = 0;
-            for (int i = 0; i < segs.n; ++i) {
-                int tile, ua, ub, sl;
-                segs.get(i, tile, ua, ub, sl);
-                const int row0 = tile / p.m_tiles * 8;
-                for (int ku = ua; ku < ub; ++ku) {
-                    MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
-                    mbar_expect_tx(RAW_FULL(r), MS_UNIT_BYTES);          // past the end of K the box is filled with zeros, which count
-                    tma_load_2d(r_base + r * MS_UNIT_BYTES, &wmap, ku * (MS_UK * 64), row0, RAW_FULL(r));
-                    MM_ADVANCE(r, rph, R);
-                }
+            if (p.wait_bits) pdl_wait();
+            else rph = 1u;
+            for (; load.left(); load.next()) {
+                MM_WAIT(RAW_EMPTY(r), rph ^ 1u);
+                mbar_expect_tx(RAW_FULL(r), MS_UNIT_BYTES);
+                tma_load_2d(r_base + r * MS_UNIT_BYTES, &wmap, load.ku * (MS_UK * 64), load.row0, RAW_FULL(r));
+                MM_ADVANCE(r, rph, R);
             }
         }
     } else if (warp == 6) {
@@ -164,7 +175,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
             for (int i = 0; i < segs.n; ++i) {
                 int tile, ua, ub, sl;
                 segs.get(i, tile, ua, ub, sl);
-                const int row0 = (tile % p.m_tiles) * Nt;
+                const int row0 = (tile - mm_div(tile, p.m_tiles, p.mt_inv) * p.m_tiles) * Nt;
                 for (int ku = ua; ku < ub; ++ku) {
                     const int nk = min(MS_UK, KB - ku * MS_UK);
                     MM_WAIT(B_EMPTY(b), bph ^ 1u);
@@ -268,12 +279,13 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
     } else {
         // ---- epilogue (warps 2..5): a warp may read the 32 tensor-memory lanes selected by warp % 4
         const int q = warp & 3, nl = q * 32 + lane, ncol = q * 32 + mm_column(lane);
+        join();
         pdl_wait();
         uint32_t a = 0, aph = 0;
         for (int i = 0; i < segs.n; ++i) {
             int tile, ua, ub, sl;
             segs.get(i, tile, ua, ub, sl);
-            const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
+            const int nt = mm_div(tile, p.m_tiles, p.mt_inv), mt = tile - nt * p.m_tiles;
             const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
             // all legs but the last join the sum in tensor memory
             bool legs = false;
@@ -331,8 +343,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
                 __syncwarp();
                 if (lane < C && lane != rank && lane < sixteens) mm_arrive_peer(mm_peer(PART_FULL(q), (uint32_t)lane));
                 if (rank < sixteens) {
-                    MM_WAIT(PART_FULL(q), 0u);
-                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    if (!mm_wait_cluster(PART_FULL(q), abort_flag)) goto done;
                     mm_with_out(p, [&](auto out, auto silu) {
                         uint32_t at0 = part_base + (uint32_t)nl * 16u;
                         for (int c = rank; c < sixteens; c += C, at0 += 8192u) {
@@ -356,8 +367,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
                 // The last of the blocks that share this tile to arrive adds the partial sums, in block order.  Each epilogue warp owns 32
                 // columns of the tile and runs the hand-over for them by itself.  The last block's own part stays in tensor memory;
                 // a block that finds all the others there already does not even write it.
-                const long long first_unit = (long long)tile * KBU, last_unit = first_unit + KBU - 1;
-                cf = (int)(((first_unit + 1) * G + total - 1) / total - 1), cl = (int)(((last_unit + 1) * G + total - 1) / total - 1);
+                cf = mm_owner(p, tile * KBU, G, total), cl = mm_owner(p, tile * KBU + KBU - 1, G, total);
                 unsigned int* ctr = p.counters + (size_t)tile * 4 + q;
                 const unsigned int others = (unsigned int)(cl - cf);
                 unsigned int there = 0;
@@ -382,7 +392,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
             }
             if (!clustered && (full || sum)) {
                 // A part lies in its block's slot 0, except that the first block may have come from an earlier tile.
-                const float* part0 = p.partial + (size_t)(2 * cf + (!full && total * cf / G >= (long long)tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
+                const float* part0 = p.partial + (size_t)(2 * cf + (!full && mm_share(p, cf, G) >= tile * KBU ? 0 : 1)) * slot_floats + nl * 4;
                 const float* rest = p.partial + (size_t)(2 * cf + 2) * slot_floats + nl * 4;
                 mm_with_out(p, [&](auto out, auto silu) {
                     for (int c16 = 0; c16 < Nt; c16 += 16) {
@@ -420,6 +430,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) mma_units4_kernel(const __grid_
     }
 done:
     __syncwarp();
+    join();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

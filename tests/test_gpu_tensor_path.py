@@ -129,6 +129,29 @@ def test_exact_on_units_of_two_slices(M, K, N, dtype, blocks, cut, cluster, wide
     pw.close()
 
 
+# Clusters of two and four pairs of blocks: one plane and three, ragged K, rows and columns, int8, gate and up; launches one behind the other
+@pytest.mark.parametrize("M,K,N,dtype,cluster", [(256, 8192, 2048, "f32", 2), (100, 4160, 4096, "f32", 2), (512, 8300, 1000, "f32", 2), (400, 8300, 500, "f32", 4),
+                                                 (700, 12352, 2048, "f16", 2), (700, 12352, 2041, "i8", 2)])
+def test_exact_on_clusters_of_pairs(M, K, N, dtype, cluster):
+    gen = torch.Generator().manual_seed(K + N)
+    w = torch.randint(-1, 2, (K, N), dtype=torch.int8, generator=gen)
+    pw = PackedWeight.from_dense(w.numpy(), scale=1.0)
+    L = _lib.lib()
+    L.tllm_set_mma_min_rows(-1)
+    X = torch.randint(-4, 5, (M, K), generator=gen).to({"f32": torch.float32, "f16": torch.float16, "i8": torch.int8}[dtype]).cuda()
+    want = X.double() @ w.cuda().double()
+    out = torch.full((M, N), -1, dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+    for x, kw in ((X, {}), (X, {}), (X.t().contiguous(), {"col_major": True})):
+        pw.matmul(x, out=out, **kw)
+        plan = mma_plan()
+        assert plan[1:3] != (2, 2) or plan[3] == cluster, plan
+        if not kw:
+            assert plan[:4] == (2, 2, 2, cluster), plan
+        assert torch.equal(out.double(), want)
+    pw.check()
+    pw.close()
+
+
 def test_repeated_calls_and_row_counts_share_the_split_scratch():
     """Back-to-back launches with different row counts on one handle (programmatic dependent launch lets the
     next kernel start before the previous one has drained): counters and partial sums must not leak."""
