@@ -124,6 +124,14 @@ double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, i
     return c.start + c.warps * std::min(1.0, each) + pairs * (step + fetch) + c.results * groups * rows / 1000;
 }
 
+// What a launch takes of that estimate where the warps share X (columns cut two and four ways; three blocks of fp32 columns of B are cut once): over
+// 4800 drawn products of 1 to 100 rows.
+double bits_shared_part(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
+    static const double part[3][2] = {{0.96, 0.86}, {0.86, 0.72}, {0.6, 0.45}};
+    const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
+    return (q.split_log ? part[access][q.split_log - 1] : 1.0) * (x_dtype == TLLM_F32 && q.nb == 3 ? 0.93 : 1.0);
+}
+
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
     if (p.x_dtype == TLLM_I8 && p.K >= BT_MAX_INT8_K) return fail(TLLM_ERR_ARG, "bits_launch: int8 over %d inners does not fit into 32-bit sums", p.K);

@@ -668,5 +668,6 @@ inline BitsAccess bits_access(const void* X, int x_dtype, int x_layout, int x_ld
 }
 // its time, for the choice between kernels
 double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms);
+double bits_shared_part(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms);
 
 }  // namespace tllm

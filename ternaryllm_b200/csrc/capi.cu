@@ -893,7 +893,10 @@ double mm_tiles_model_us(int inners, int columns, int sms, int device, bool dire
 bool bits_prefer_registers(int inners, int columns, int sms, int device, bool direct, int x_dtype, BitsAccess access, int rows) {
     if (rows == 1 && access == BITS_ROWS16) return true;
     if (rows > 8 * BT_MAX_ROWS) return false;
-    return bt_model_us(inners, columns, sms, x_dtype, access, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, access, rows);
+    // Both estimates are from before the decoder's warps shared X and the batched kernels started earlier.  (Loss against the faster of the two over 4800 drawn
+    // products: 0.4 to 0.8 % for rows on 16 bytes, as before; rows anywhere 0.8 %, 1.2 without; columns 1.6 %, 3.5.)
+    const double part = bits_shared_part(x_dtype, access, std::min(rows, bt_rows_per_launch(x_dtype)), columns, (inners + 63) / 64, sms);
+    return part * bt_model_us(inners, columns, sms, x_dtype, access, rows) <= (direct ? 0.985 : 0.95) * mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, access, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
