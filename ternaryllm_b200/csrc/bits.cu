@@ -61,9 +61,8 @@ int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device,
 
 }  // namespace
 
-// How a product is cut.  One pass over the widest block's columns if GR = 3 (two for more than eight columns of B: 64 and 128
-// registers) and a split of up to four allow it; the narrowest split that does, because every part of a split fetches the
-// activations anew.
+// How a product is cut.  One pass over the widest block's columns if GR = 3 (two for more than eight columns of B) and a split of up to four allow it; the
+// narrowest split that does, because every part of a split reads the activations anew.
 namespace {
 struct BitsPlan {
     int nb, own, own_more, split_log, per_pass, passes, gr, pairs;     // pairs: pairs of slices a warp goes through, all passes together
@@ -145,8 +144,7 @@ int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     p.y_wide = p.epilogue == 0 && p.y_step_n == 1 && p.y_step_m % 4 == 0 && p.N % 4 == 0 && (uintptr_t)p.Y % (4 * ye) == 0;
     const size_t red = (size_t)kparts * p.per_pass * cols * 80;
     // Shared memory: X for all warps together, or a warp's pairs of it beside those of W.  Of these as many in flight as a warp has to fetch and as
-    // there is room for: in half of the shared memory, so that the next launch fits beside this one, unless the launch is one of some length
-    // or does not fit there; then in all of it.
+    // there is room for.
     bool share = bits_share(p.x_dtype, async, q, kp, p.M);
     const auto pitch = [&](int n) { return (size_t)n * 128 * e + (e == 1 ? 64 : e == 2 ? 16 : 32); };
     const auto chunk = [&](int n) { return share ? (p.M * pitch(std::min(n, kp)) + 127) / 128 * 128 : 0; };
@@ -158,18 +156,18 @@ int bits_launch(BitsParams& p, int sms, int device, void* stream) {
     p.x_pairs = p.x_chunks == 1 ? (kp + 15) / 16 * 16 : ((kp + 1) / 2 + 15) / 16 * 16;
     if (share && total(least) > BT_SMEM_ALL) share = false;
     p.slot_bytes = slot();
-    const size_t limit = pairs > 4 || total(least) > BT_SMEM_SHARED ? BT_SMEM_ALL : BT_SMEM_SHARED;
     p.depth = 8;
-    while (p.depth > 1 && (p.depth / 2 >= pairs || total(p.depth) > limit)) p.depth /= 2;
+    while (p.depth > 1 && (p.depth / 2 >= pairs || total(p.depth) > BT_SMEM_ALL)) p.depth /= 2;
     p.slots = slots(p.depth);
     p.x_pitch = (uint32_t)pitch(std::min(p.x_pairs, kp)), p.x_bytes = (uint32_t)chunk(p.x_pairs);
     p.ring_at = p.x_chunks * p.x_bytes;
     p.red_at = p.ring_at + (uint32_t)BT_WARPS * p.slots * p.slot_bytes;
     p.bar_at = p.red_at + (uint32_t)red;
-    // A launch of some length keeps an SM to itself: behind one that does not fit beside it, its blocks would start two to an SM while
-    // others wait (fp16 MLP, four rows, 4096 / 11008: 24 us instead of 19).
-    size_t smem = total(p.depth);
-    if (pairs > 4) smem = std::max(smem, (size_t)BT_SMEM_ALONE);
+    // A launch keeps an SM to itself.  With room for two blocks, those of the next launch came two to an SM as often as not, while other SMs waited: 4096 x 11008,
+    // one row of fp16, called 400 times one after the other, 8.0 us in the median (5.9 to 8.2), alone 6.0 (6.0 to 6.1); an MLP of 2048 / 5632,
+    // four rows, 10.7 and 8.5; 8192 x 2048, one row, in a graph 5.0 and 4.0.  What it costs is the next launch's start beside this one: 2048 x 16384,
+    // one row, in a graph 4.7 and 5.1.
+    const size_t smem = std::max(total(p.depth), (size_t)BT_SMEM_ALONE);
     if (smem > 227u * 1024u) return fail(TLLM_ERR_ARG, "bits_launch: %zu bytes of shared memory", smem);
     cudaStream_t st = (cudaStream_t)stream;
 #define BT_PICK(XT)                                                                                                               \

@@ -19,21 +19,20 @@
 //     passes), whole, once, for all warps of the block (SHARED; bits_share in bits.cu has the rule and its figures): as much of it as of W went
 //     through L2 four times over (16 rows of fp16 on 2048 x 16384: 64 KB of X a block, fetched four times, for 57 KB of W);
 //   * sixteen warps (four per scheduler hide the latency of shared-memory load -> decode -> MMA; with two per scheduler the
-//     loop issued 0.49 instructions per clock) of <= 64 registers, so that the next launch's block fits beside this one
-//     and starts streaming;
+//     loop issued 0.49 instructions per clock), one block to an SM (bits_launch);
 //   * the shifts of the decode are multiplications by a value in a register: they run on the FMA pipe beside the ANDs on the
 //     ALU pipe, both of which take two clocks per warp instruction.
 //
 // Measured, fp16, CUDA-graph chain of distinct weights from HBM (us; before = the fastest of the other kernels):
-//   2048 x 2048    1 row  2.3 (gather 3.9)      8 rows  2.6 (batched 11.5)
-//   4096 x 11008   1 row  5.7 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  6.4 (17.2)   16 rows  9.2 (19.5)
-//   8192 x 10240   1 row  9.3 (four-bit planes 15.4)     8 rows 10.7 (22.7)
+//   2048 x 2048    1 row  2.1 (gather 3.9)      8 rows  2.3 (batched 11.5)
+//   4096 x 11008   1 row  5.6 (gather 8.2, 75 % zeros; four-bit planes 10.5)   8 rows  6.0 (17.2)   16 rows  9.2 (19.5)
+//   8192 x 10240   1 row  8.8 (four-bit planes 15.4)     8 rows 10.2 (22.7)
 // fp32: three MMAs per eight rows, whose values a lane cuts into all three pieces at once (BY_PIECE; each block of columns of B by itself 4.5, 8.0 and 11.5):
 //   2048 x 2048    8 rows  3.7      4096 x 4096    8 rows  6.6       8192 x 2048    8 rows  8.8
 // int8: seven instructions instead of fifteen decode sixteen entries, and two MMAs (m16n8k32) replace four:
 //   2048 x 8192    1 row  2.7 (as fp16 3.5)      32 rows 5.4 in one launch (9.3 in two)
-//   8192 x 10240   1 row  6.9 (12.0)             16 rows 11.8 (22)
-// Of the 9.3 us of 8192 x 10240, 5.4 are there without decode and MMAs; masks and MMAs, which hardly overlap, take 65 to 70 clocks of a scheduler per
+//   8192 x 10240   1 row  6.6 (12.0)             16 rows 11.8 (22)
+// Of the 8.8 us of 8192 x 10240, 5.4 are there without decode and MMAs; masks and MMAs, which hardly overlap, take 65 to 70 clocks of a scheduler per
 // 1024 entries (53 with the same instructions and nothing to wait for).
 //
 // Precision.  fp16 / bf16 activations are multiplied as they are; int8 as int8 with int32 sums of +-64 * x
@@ -52,8 +51,7 @@
 namespace tllm {
 
 #define BT_WARPS 16
-#define BT_SMEM_SHARED (112u * 1024u)   // two blocks of this size share an SM
-#define BT_SMEM_ALONE (116u * 1024u)    // two of this do not
+#define BT_SMEM_ALONE (116u * 1024u)    // two blocks of this size do not share an SM
 #define BT_MAX_ROWS 16                  // rows of one launch (NB = 2 blocks of eight columns of B; fp32: 8 rows, three blocks; int8: 32, four)
 #define BT_MASK 0xC000C000u             // the two codes at the top of a word's halves: 16-bit floats 0 / +-2
 #define BT_MASK8 0xC0C0C0C0u            // the four at the top of its bytes: 0 / +-64
@@ -285,8 +283,8 @@ __device__ __noinline__ float bt_column_sum(const BitsParams& p, int n, int m) {
         return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + k : (size_t)k * p.x_ld + m);
     });
 }
-// Columns n .. n + 3 of row m again, entry by entry, where one of their sums is not finite (behind the stores of the others, so that next to no register has
-// to live through the call: with the sums kept for it the kernels of 64 registers took half as long again).
+// Columns n .. n + 3 of row m again, entry by entry, where one of their sums is not finite: behind the stores of the others, so that next to no register has
+// to live through the call.
 template <int XT>
 __device__ __noinline__ void bt_store_again(const BitsParams& p, int n, int m) {
     const auto sum = [&](int c) {                                    // (a call of bt_column_sum from here cost the callers registers)
@@ -308,7 +306,7 @@ __device__ __noinline__ void bt_store_again(const BitsParams& p, int n, int m) {
 // The code is kept short (rolled loops, no divisions): a warp of a small product runs the loop body once or twice, and then
 // fetching instructions costs more than executing them.
 template <int XT, int NB, int GR, bool ASYNC, bool SHARED>
-__global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_spmm_kernel(const __grid_constant__ BitsParams p) {
+__global__ void __launch_bounds__(BT_WARPS * 32, 1) bits_spmm_kernel(const __grid_constant__ BitsParams p) {
     extern __shared__ __align__(128) unsigned char bt_smem[];
     using Act = BitsAct<XT>;
     constexpr bool BF16 = XT == TLLM_BF16 || XT == TLLM_F32, I8 = XT == TLLM_I8;
@@ -319,9 +317,6 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
     // Columns of B: piece of row m is column 3 m + piece; with three blocks of them block `piece` has column m, so that a lane cuts the values of one
     // row and has all of its columns.
     constexpr bool BY_PIECE = XT == TLLM_F32 && NB == 3;
-    // Which of the two ways to add up the warps' sums there is: instances of 64 registers have no room for both (2048 x 2048, eight rows of fp16 2.6 us with
-    // one of them, 3.2 with both).
-    constexpr bool TIGHT = NB == 1 && ASYNC, WIDE = !TIGHT || SHARED || GR > 1, HALF = !TIGHT || !WIDE;
     constexpr uint32_t PAIR = 128u * Act::E;                               // bytes of a row in a pair of slices
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, c0 = b * p.own + min(b, p.own_more), own = p.own + (b < p.own_more);
@@ -575,7 +570,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
             }
         __syncthreads();
         // Sums of the warps' sums; idx = group * M + row.  Up to thirty-two of them: half a warp each, a column per thread.
-        if (HALF && (!WIDE || ng * M <= BT_WARPS * 2)) {
+        if (ng * M <= BT_WARPS * 2) {
             const int c = lane & 15;
 #pragma unroll 1
             for (int i0 = warp * 2; i0 < ng * M; i0 += BT_WARPS * 2) {
@@ -607,7 +602,6 @@ __global__ void __launch_bounds__(BT_WARPS * 32, NB == 1 && ASYNC ? 2 : 1) bits_
             }
             continue;
         }
-        if constexpr (!WIDE) continue;
         // More: four columns per thread.  (With a column per thread the loop went round four times as often, each time a chain of some 600 clocks: 16 rows of
         // fp16 on 2048 x 16384 7.2 us, 6.5 so; 32 of int8 9.7 and 8.7.)
 #pragma unroll 1
