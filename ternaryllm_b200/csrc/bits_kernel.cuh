@@ -283,18 +283,25 @@ __device__ __noinline__ float bt_column_sum(const BitsParams& p, int n, int m) {
         return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + k : (size_t)k * p.x_ld + m);
     });
 }
-// Columns n .. n + 3 of row m again, entry by entry, where one of their sums is not finite: behind the stores of the others, so that next to no register has
-// to live through the call.
+// Those of columns n .. n + 3 of row m again, entry by entry, whose sums (v0 .. v3) are not finite: behind the stores of all four, so that next to no register
+// has to live through the call.  A finite sum keeps its bits.
 template <int XT>
-__device__ __noinline__ void bt_store_again(const BitsParams& p, int n, int m) {
-    const auto sum = [&](int c) {                                    // (a call of bt_column_sum from here cost the callers registers)
-        return column_sum((const uint32_t*)p.bits, c, p.K, p.KB, false, [&](int k) {
-            return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + k : (size_t)k * p.x_ld + m);
-        });
+__device__ __noinline__ void bt_store_again(const BitsParams& p, int n, int m, float v0, float v1, float v2, float v3) {
+    const auto result = [&](int k, float v, float sc) {              // (a call of bt_column_sum from here cost the callers registers)
+        if (finite_sum(v)) return v * sc;
+        return column_sum((const uint32_t*)p.bits, n + k, p.K, p.KB, false, [&](int i) {
+                   return load_act_f32_cg(p.X, XT, p.x_layout == TLLM_ROW_MAJOR ? (size_t)m * p.x_ld + i : (size_t)i * p.x_ld + m);
+               }) * (2.f * sc);
     };
-    for (int c = n; c < min(n + 4, p.N); ++c) {
-        if (p.epilogue == 0) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (size_t)c * p.y_step_n, sum(c) * (2.f * p.scale));
-        else if (!(c & 1) && c + 1 < p.N) store_out(p.Y, p.y_dtype, (size_t)m * p.y_step_m + (c >> 1), silu_mul(sum(c) * (2.f * p.scale), sum(c + 1) * (2.f * p.scale2)));
+#pragma unroll 1
+    for (int k = 0; k < 4 && n + k < p.N; k += 2, v0 = v2, v1 = v3) {
+        size_t at = (size_t)m * p.y_step_m;
+        if (p.epilogue == 0) {
+            at += (size_t)(n + k) * p.y_step_n;
+            if (!finite_sum(v0)) store_out(p.Y, p.y_dtype, at, result(k, v0, p.scale));
+            if (n + k + 1 < p.N && !finite_sum(v1)) store_out(p.Y, p.y_dtype, at + p.y_step_n, result(k + 1, v1, p.scale));
+        } else if (n + k + 1 < p.N && !(finite_sum(v0) && finite_sum(v1)))
+            store_out(p.Y, p.y_dtype, at + ((n + k) >> 1), silu_mul(result(k, v0, p.scale), result(k + 1, v1, p.scale2)));
     }
 }
 
@@ -632,19 +639,20 @@ __global__ void __launch_bounds__(BT_WARPS * 32, 1) bits_spmm_kernel(const __gri
 #pragma unroll
             for (int k = 0; k < 4; ++k) z = fmaf((float)v[k], 0.f, z);
             if (p.epilogue == 0) {
+                float y[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) v[k] *= p.scale;
-                if (p.y_wide && n < p.N) store_four(p.Y, p.y_dtype, at, (float(&)[4])v);
+                for (int k = 0; k < 4; ++k) y[k] = v[k] * p.scale;
+                if (p.y_wide && n < p.N) store_four(p.Y, p.y_dtype, at, y);
                 else
 #pragma unroll
                     for (int k = 0; k < 4; ++k, at += p.y_step_n)
-                        if (n + k < p.N) store_out(p.Y, p.y_dtype, at, v[k]);
+                        if (n + k < p.N) store_out(p.Y, p.y_dtype, at, y[k]);
             } else {
                 at = (size_t)m * p.y_step_m + (n >> 1);
                 if (n + 1 < p.N) store_out(p.Y, p.y_dtype, at, silu_mul(v[0] * p.scale, v[1] * p.scale2));
                 if (n + 3 < p.N) store_out(p.Y, p.y_dtype, at + 1, silu_mul(v[2] * p.scale, v[3] * p.scale2));
             }
-            if (__builtin_expect(z != 0.f, 0)) bt_store_again<XT>(p, n, m);
+            if (__builtin_expect(z != 0.f, 0)) bt_store_again<XT>(p, n, m, v[0], v[1], v[2], v[3]);
         }
     }
     if (!ok) atomicExch(p.status, BT_ERR_WAIT);

@@ -120,3 +120,48 @@ def test_fused_mlp(M):
     assert torch.isfinite(want[:3]).any(1).all() and not torch.isfinite(want[:3]).all(1).any()
     check(mlp.forward(X), want, 1e-5 + 2.0 ** -22)
     mlp.close()
+
+
+# Four columns a thread add up the warps' sums (more than thirty-two of them a block): the ones beside a sum that is not finite keep every bit
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_neighbours_of_a_sum_that_is_not_finite(dtype):
+    M, K = 8, 1000
+    N = 16 * 5 * torch.cuda.get_device_properties(0).multi_processor_count - 6
+    w = random_ternary(np.random.default_rng(1), K, N, 0.5)
+    w[7] = 0
+    w[7, 1::5] = 1                                             # 2 * 2.5e38 is past the range of fp32 inside the kernel
+    pw = PackedWeight.from_dense(w)
+    X = torch.randn((M, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).to(DT[dtype])
+    X[:, 7] = 0
+    L = _lib.lib()
+    b0 = L.tllm_bits_launch_count()
+    plain = pw.matmul(X, out=torch.empty((M, N), device="cuda"))
+    X[:, 7] = 2.5e38
+    got = pw.matmul(X, out=torch.empty((M, N), device="cuda"))
+    assert L.tllm_bits_launch_count() == b0 + 2
+    used = torch.zeros(N, dtype=torch.bool)
+    used[1::5] = True
+    assert torch.equal(got[:, ~used], plain[:, ~used])
+    check(got, product(X, w), 1e-5)
+    pw.close()
+
+
+# the same for pairs of gate and up columns: h comes back through a second product that takes one entry a column
+def test_neighbours_of_a_gate_that_is_not_finite():
+    M, hidden, inter = 8, 1000, 34 * torch.cuda.get_device_properties(0).multi_processor_count + 6
+    wg, wu = random_ternary(np.random.default_rng(1), hidden, inter, 0.5), random_ternary(np.random.default_rng(2), hidden, inter, 0.5)
+    wg[7], wu[7] = 0, 0
+    wg[7, 1::5] = 1
+    mlp = PackedMLP(wg, wu, np.eye(inter, hidden, dtype=np.int8), 0.05, 0.04, 1.0)
+    X = torch.randn((M, hidden), device="cuda", generator=torch.Generator(device="cuda").manual_seed(0))
+    X[:, 7] = 0
+    L = _lib.lib()
+    b0 = L.tllm_bits_launch_count()
+    plain = mlp.forward(X).clone()
+    X[:, 7] = 2.5e38
+    got = mlp.forward(X)
+    assert L.tllm_bits_launch_count() >= b0 + 2
+    used = torch.zeros(hidden, dtype=torch.bool)
+    used[1::5] = True
+    assert torch.equal(got[:, ~used], plain[:, ~used]) and not torch.equal(got[:, used], plain[:, used])
+    mlp.close()
