@@ -39,6 +39,7 @@ SIGNATURES = {
     "tllm_launch_count": (_L, []),
     "tllm_mma_launch_count": (_L, []),
     "tllm_mma_last_plan": (_I, [_P]),
+    "tllm_bits_last_plan": (_I, [_P]),
     "tllm_bits_launch_count": (_L, []),
     "tllm_set_mma_min_rows": (_I, [_I]),
     "tllm_set_nibble_max_rows": (_I, [_I]),

@@ -1,6 +1,7 @@
 // bits.cu -- instantiations and launches of bits_spmm_kernel (bits_kernel.cuh), in a translation unit of their own so that
 // they compile beside the rest.
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 
 #include "bits_kernel.cuh"
@@ -64,6 +65,7 @@ int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device,
 // How a product is cut.  One pass over the widest block's columns if GR = 3 (two for more than eight columns of B) and a split of up to four allow it; the
 // narrowest split that does, because every part of a split reads the activations anew.
 namespace {
+int dtype_bytes(int x_dtype) { return x_dtype == TLLM_F32 ? 4 : x_dtype == TLLM_I8 ? 1 : 2; }
 struct BitsPlan {
     int nb, own, own_more, split_log, per_pass, passes, gr, pairs;     // pairs: pairs of slices a warp goes through, all passes together
 };
@@ -92,6 +94,36 @@ bool bits_share(int x_dtype, bool async, const BitsPlan& q, int kp, int rows) {
     const bool two_bytes = x_dtype == TLLM_F16 || x_dtype == TLLM_BF16;
     if (q.split_log == 2) return q.pairs > 2;
     return q.split_log == 1 && (q.pairs > 4 || (q.pairs == 4 && two_bytes) || (q.pairs > 1 && (q.nb == 3 || (q.nb == 2 && two_bytes))));
+}
+// The whole cut of a launch.  Shared memory: X for all warps together, or a warp's pairs of it beside those of W.  Of these as many in flight as a warp has to
+// fetch and as there is room for.
+struct BitsCut : BitsPlan {
+    bool async, share;             // X by rows that start on 16 bytes and are a multiple of them long; whether the warps share it
+    int x_chunks, x_pairs, depth, slots;
+    uint32_t x_pitch, slot_bytes, ring_at, red_at, bar_at, smem;
+};
+BitsCut bits_cut(int x_dtype, BitsAccess access, int rows, int inners, int columns, int sms) {
+    const int e = dtype_bytes(x_dtype), kb = (inners + 63) / 64, kp = (kb + 1) / 2;
+    BitsCut q{bits_plan(x_dtype, rows, columns, kb, sms)};
+    q.async = access == BITS_ROWS16 && (size_t)inners * e % 16 == 0;
+    q.share = bits_share(x_dtype, q.async, q, kp, rows);
+    const uint32_t red = (uint32_t)(BT_WARPS >> q.split_log) * q.per_pass * (x_dtype == TLLM_F32 ? 3 * rows : rows) * 80;
+    q.x_pitch = (uint32_t)kp * 128 * e + (e == 1 ? 64 : e == 2 ? 16 : 32);
+    const auto all_x = [&] { return q.share ? ((size_t)rows * q.x_pitch + 127) / 128 * 128 : 0; };
+    const auto slots = [&](int d) { return q.pairs <= d ? q.pairs : d + 1; };
+    const auto slot = [&] { return (uint32_t)(q.gr * 512 + (q.share ? 0 : rows * 128 * e)); };
+    const auto total = [&](int d) { return all_x() + (size_t)BT_WARPS * slots(d) * slot() + red + BT_BAR_BYTES; };
+    if (q.share && total(std::min(q.pairs, 2)) > BT_SMEM_ALL) q.share = false;
+    q.x_chunks = kp > 16 && (size_t)rows * inners * e > 16384 ? 2 : 1;
+    q.x_pairs = q.x_chunks == 1 ? (kp + 15) / 16 * 16 : ((kp + 1) / 2 + 15) / 16 * 16;
+    q.depth = 8;
+    while (q.depth > 1 && (q.depth / 2 >= q.pairs || total(q.depth) > BT_SMEM_ALL)) q.depth /= 2;
+    q.slots = slots(q.depth), q.slot_bytes = slot();
+    q.ring_at = (uint32_t)all_x();
+    q.red_at = q.ring_at + (uint32_t)BT_WARPS * q.slots * q.slot_bytes;
+    q.bar_at = q.red_at + red;
+    q.smem = q.bar_at + BT_BAR_BYTES;
+    return q;
 }
 }  // namespace
 
@@ -131,48 +163,31 @@ double bits_shared_part(int x_dtype, BitsAccess access, int rows, int columns, i
     return (q.split_log ? part[access][q.split_log - 1] : 1.0) * (x_dtype == TLLM_F32 && q.nb == 3 ? 0.93 : 1.0);
 }
 
+thread_local int bits_last_plan[6];
+
 int bits_launch(BitsParams& p, int sms, int device, void* stream) {
-    const int e = p.x_dtype == TLLM_F32 ? 4 : p.x_dtype == TLLM_I8 ? 1 : 2;
     if (p.x_dtype == TLLM_I8 && p.K >= BT_MAX_INT8_K) return fail(TLLM_ERR_ARG, "bits_launch: int8 over %d inners does not fit into 32-bit sums", p.K);
-    const bool async = bits_access(p.X, p.x_dtype, p.x_layout, p.x_ld) == BITS_ROWS16 && (size_t)p.K * e % 16 == 0;
-    const BitsPlan q = bits_plan(p.x_dtype, p.M, p.N, p.KB, sms);
-    const int nb = q.nb, gr = q.gr, grid = sms, kparts = BT_WARPS >> q.split_log, cols = p.x_dtype == TLLM_F32 ? 3 * p.M : p.M, pairs = q.pairs;
+    const BitsCut q = bits_cut(p.x_dtype, bits_access(p.X, p.x_dtype, p.x_layout, p.x_ld), p.M, p.K, p.N, sms);
+    const int nb = q.nb, gr = q.gr, grid = sms, ye = p.y_dtype == TLLM_F32 || p.y_dtype == TLLM_I32 ? 4 : 2;
     p.own = q.own, p.own_more = q.own_more, p.split_log = q.split_log, p.per_pass = q.per_pass;
+    p.depth = q.depth, p.slots = q.slots, p.slot_bytes = q.slot_bytes;
+    p.x_pairs = q.x_pairs, p.x_chunks = q.x_chunks, p.x_pitch = q.x_pitch, p.x_chunk = (uint32_t)q.x_pairs * 128u * (uint32_t)dtype_bytes(p.x_dtype);
+    p.ring_at = q.ring_at, p.red_at = q.red_at, p.bar_at = q.bar_at;
     p.mul4 = 4, p.mul16 = 16;
     p.m_inv = (uint32_t)(((1ull << 32) + p.M - 1) / p.M);
-    const int kp = (p.KB + 1) / 2, ye = p.y_dtype == TLLM_F32 || p.y_dtype == TLLM_I32 ? 4 : 2;
     p.y_wide = p.epilogue == 0 && p.y_step_n == 1 && p.y_step_m % 4 == 0 && p.N % 4 == 0 && (uintptr_t)p.Y % (4 * ye) == 0;
-    const size_t red = (size_t)kparts * p.per_pass * cols * 80;
-    // Shared memory: X for all warps together, or a warp's pairs of it beside those of W.  Of these as many in flight as a warp has to fetch and as
-    // there is room for.
-    bool share = bits_share(p.x_dtype, async, q, kp, p.M);
-    const auto pitch = [&](int n) { return (size_t)n * 128 * e + (e == 1 ? 64 : e == 2 ? 16 : 32); };
-    const auto chunk = [&](int n) { return share ? (p.M * pitch(std::min(n, kp)) + 127) / 128 * 128 : 0; };
-    const auto slots = [&](int d) { return pairs <= d ? pairs : d + 1; };
-    const auto slot = [&] { return (uint32_t)(gr * 512 + (share ? 0 : p.M * 128 * e)); };
-    const auto total = [&](int d) { return p.x_chunks * chunk(p.x_pairs) + (size_t)BT_WARPS * slots(d) * slot() + red + BT_BAR_BYTES; };
-    const int least = std::min(pairs, 2);
-    p.x_chunks = kp > 16 && (size_t)p.M * p.K * e > 16384 ? 2 : 1;
-    p.x_pairs = p.x_chunks == 1 ? (kp + 15) / 16 * 16 : ((kp + 1) / 2 + 15) / 16 * 16;
-    if (share && total(least) > BT_SMEM_ALL) share = false;
-    p.slot_bytes = slot();
-    p.depth = 8;
-    while (p.depth > 1 && (p.depth / 2 >= pairs || total(p.depth) > BT_SMEM_ALL)) p.depth /= 2;
-    p.slots = slots(p.depth);
-    p.x_pitch = (uint32_t)pitch(std::min(p.x_pairs, kp)), p.x_bytes = (uint32_t)chunk(p.x_pairs);
-    p.ring_at = p.x_chunks * p.x_bytes;
-    p.red_at = p.ring_at + (uint32_t)BT_WARPS * p.slots * p.slot_bytes;
-    p.bar_at = p.red_at + (uint32_t)red;
     // A launch keeps an SM to itself.  With room for two blocks, those of the next launch came two to an SM as often as not, while other SMs waited: 4096 x 11008,
     // one row of fp16, called 400 times one after the other, 8.0 us in the median (5.9 to 8.2), alone 6.0 (6.0 to 6.1); an MLP of 2048 / 5632,
     // four rows, 10.7 and 8.5; 8192 x 2048, one row, in a graph 5.0 and 4.0.  What it costs is the next launch's start beside this one: 2048 x 16384,
     // one row, in a graph 4.7 and 5.1.
-    const size_t smem = std::max(total(p.depth), (size_t)BT_SMEM_ALONE);
-    if (smem > 227u * 1024u) return fail(TLLM_ERR_ARG, "bits_launch: %zu bytes of shared memory", smem);
+    const uint32_t smem = std::max(q.smem, BT_SMEM_ALONE);
+    if (smem > 227u * 1024u) return fail(TLLM_ERR_ARG, "bits_launch: %u bytes of shared memory", smem);
+    const int cut[6] = {gr, nb, 1 << q.split_log, q.passes, q.share ? q.x_chunks : 0, q.depth};
+    std::memcpy(bits_last_plan, cut, sizeof cut);
     cudaStream_t st = (cudaStream_t)stream;
 #define BT_PICK(XT)                                                                                                               \
-    (async ? share ? pick<XT, true, true>(p, nb, gr, grid, smem, device, st) : pick<XT, true, false>(p, nb, gr, grid, smem, device, st) \
-           : share ? pick<XT, false, true>(p, nb, gr, grid, smem, device, st) : pick<XT, false, false>(p, nb, gr, grid, smem, device, st))
+    (q.async ? q.share ? pick<XT, true, true>(p, nb, gr, grid, smem, device, st) : pick<XT, true, false>(p, nb, gr, grid, smem, device, st) \
+             : q.share ? pick<XT, false, true>(p, nb, gr, grid, smem, device, st) : pick<XT, false, false>(p, nb, gr, grid, smem, device, st))
     switch (p.x_dtype) {
         case TLLM_F32: return BT_PICK(TLLM_F32);
         case TLLM_F16: return BT_PICK(TLLM_F16);

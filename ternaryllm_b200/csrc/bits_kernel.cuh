@@ -76,7 +76,7 @@ struct BitsParams {
     int slots, depth;              // pairs of slices of W a warp has room for, pairs in flight (1, 2, 4 or 8; < slots unless no slot is used twice)
     uint32_t slot_bytes;           // shared memory of one pair of slices: GR * 512, and of X, unless it is shared, M * 128 * E
     int x_pairs, x_chunks;         // X shared by the warps: pairs of slices of a chunk (a multiple of sixteen), one chunk or two
-    uint32_t x_pitch, x_bytes;     // shared memory of a row of a chunk, and of a chunk
+    uint32_t x_pitch, x_chunk;     // shared memory of a row, and of the first chunk of it
     uint32_t ring_at, red_at, bar_at;      // where W, the partial sums and the barriers lie
     uint32_t m_inv;                // ceil(2^32 / M): idx / M = umulhi(idx, m_inv) for M > 1
     uint32_t mul4, mul16;          // 4 and 16
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, 1) bits_spmm_kernel(const __gri
     // 16 (fp32: 32, int8: 64) more than a multiple of 128, so that the lanes of a fragment read different banks.)
     auto load_x = [&](int chunk) {
         const int k0 = chunk * p.x_pairs * 128, k1 = min(k0 + p.x_pairs * 128, KP * 128);      // zero past the end of K
-        const uint32_t to = smem + (uint32_t)chunk * p.x_bytes;
+        const uint32_t to = smem + (uint32_t)chunk * p.x_chunk;
         if (ASYNC) {
             if (warp == BT_WARPS - 1 && lane < M) {                  // a lane per row
                 const uint32_t row = to + (uint32_t)lane * p.x_pitch, bytes = (uint32_t)(min(k1, p.K) - k0) * Act::E;
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32, 1) bits_spmm_kernel(const __gri
 #pragma unroll 1
         for (int chunk = 0; chunk < (SHARED ? p.x_chunks : 1); ++chunk) {
             if (SHARED) ok = ok && bounded_wait(BT_FULL(chunk), 0u, abort_flag);
-            uint32_t xat = (uint32_t)chunk * p.x_bytes;
+            uint32_t xat = (uint32_t)chunk * p.x_chunk;
             int here = SHARED ? min(left, p.x_pairs >> klog) : np;
             left -= here;
 #pragma unroll 1
@@ -659,8 +659,10 @@ __global__ void __launch_bounds__(BT_WARPS * 32, 1) bits_spmm_kernel(const __gri
 #undef BT_FULL
 }
 
-// one launch of up to BT_MAX_ROWS rows (half of it fp32, twice int8); fills in everything from `own` to `mul16` (bits.cu)
+// one launch of up to BT_MAX_ROWS rows (half of it fp32, twice int8); fills in y_wide and everything from `own` to `mul16` (bits.cu)
 int bits_launch(BitsParams& p, int sms, int device, void* stream);
+// how this thread's last launch was cut (tllm_bits_last_plan)
+extern thread_local int bits_last_plan[6];
 // How it reads X: rows on 16 bytes (cp.async), rows that start anywhere, or a column-major X
 enum BitsAccess { BITS_ROWS16, BITS_ROWS, BITS_COLUMNS };
 inline BitsAccess bits_access(const void* X, int x_dtype, int x_layout, int x_ld) {

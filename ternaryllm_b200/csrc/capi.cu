@@ -1276,6 +1276,11 @@ int tllm_mma_last_plan(int plan[5]) {
     std::memcpy(plan, g_mm_last_plan, sizeof g_mm_last_plan);
     return TLLM_OK;
 }
+int tllm_bits_last_plan(int plan[6]) {
+    if (!plan || bits_last_plan[0] == 0) return fail(TLLM_ERR_ARG, "tllm_bits_last_plan: %s", plan ? "this thread has launched none" : "plan is NULL");
+    std::memcpy(plan, bits_last_plan, sizeof bits_last_plan);
+    return TLLM_OK;
+}
 int tllm_set_mma_min_rows(int rows) {
     const int prev = mm_min_rows();
     g_mm_min_rows.store(rows < 0 ? -1 : rows, std::memory_order_relaxed);

@@ -4,6 +4,8 @@ oracle, through the calls that reach it by default: few activation rows of any t
 Integer-valued activations are exact (products and partial sums are integers below 2^24); on N(0,1) the fp32 sums of
 exact products stay within 1e-5 of the largest output, the bound the other tensor-core kernels are held to.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -23,6 +25,12 @@ def decoded(call, *args, **kw):
     y = call(*args, **kw)
     assert L.tllm_bits_launch_count() - b0 == L.tllm_launch_count() - n0 > 0
     return y
+
+
+def bits_plan():
+    plan = (ctypes.c_int * 6)()
+    assert _lib.lib().tllm_bits_last_plan(plan) == 0
+    return tuple(plan)
 
 
 # one slice, an odd last slice, K and N multiples of nothing (rows of X on odd addresses), fewer pairs of slices than
@@ -92,6 +100,24 @@ def test_shared_activations(dtype, M, K, groups):
     for x, kw in ((X, {}), (buf[1:].view(M, K), {}), (X.t().contiguous(), {"col_major": True})):
         out.fill_(-1)
         assert torch.equal(pw.matmul(x, out=out, **kw).double(), want)
+    pw.check()
+    pw.close()
+
+
+# Shared activations take the room of what they hold, not of chunks rounded up to sixteen pairs of slices: K just above 4096 and 2048, up to the last row that fits
+@pytest.mark.parametrize("dtype,M,K,N", [("f16", 12, 5120, 5120), ("bf16", 13, 5120, 10240), ("bf16", 14, 5120, 5120), ("bf16", 16, 4224, 11008), ("f32", 6, 5120, 5120), ("f32", 8, 2304, 8192),
+                                         ("i8", 32, 4224, 8192), ("i8", 32, 5120, 5120)])
+def test_shared_activations_as_they_fit(dtype, M, K, N):
+    rng = np.random.default_rng(K)
+    w = torch.randint(-1, 2, (K, N), dtype=torch.int8, generator=torch.Generator().manual_seed(N))
+    pw = PackedWeight.from_dense(w.numpy())
+    top = 127 if dtype in ("i8", "bf16") else 512
+    X = torch.tensor(rng.integers(-top, top + 1, size=(M, K)), dtype=DT[dtype], device="cuda")
+    out = torch.empty((M, N), dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+    for _ in range(2):
+        out.fill_(-1)
+        assert torch.equal(decoded(pw.matmul, X, out=out).double(), X.double() @ w.cuda().double())
+        assert bits_plan()[4] == 2
     pw.check()
     pw.close()
 
