@@ -171,24 +171,19 @@ __device__ __forceinline__ uint4 bt_load_unaligned(const char* row, int off, int
     }
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
-// the same sixteen bytes of a column-major X (elements of one row are x_ld apart)
+// The same sixteen bytes of a column-major X (elements of one row are x_ld apart).  All loads are issued, past the end of K that of the last element again: with a
+// condition each, sixteen of them wait for one another's predicates (two rows of int8, 2048 x 2048: 4.5 us, 4.0 so; 2048 x 8192 5.3 and 4.3).
 template <int E>
 __device__ __forceinline__ uint4 bt_load_strided(const void* X, int m, int k, int K, size_t ld) {
-    uint32_t o[4];
+    constexpr int COUNT = 16 / E;
+    uint32_t x[COUNT], o[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t v = 0;
-#pragma unroll
-        for (int j = 0; j < 4 / E; ++j) {
-            const int kk = k + i * (4 / E) + j;
-            if (kk < K) {
-                const size_t at = (size_t)kk * ld + m;
-                const uint32_t x = E == 4 ? __ldcg((const unsigned int*)X + at) : E == 2 ? (uint32_t)__ldcg((const unsigned short*)X + at) : (uint32_t)__ldcg((const unsigned char*)X + at);
-                v |= x << (8 * E * j);
-            }
-        }
-        o[i] = v;
+    for (int i = 0; i < COUNT; ++i) {
+        const size_t at = (size_t)min(k + i, K - 1) * ld + m;
+        x[i] = E == 4 ? __ldcg((const unsigned int*)X + at) : E == 2 ? (uint32_t)__ldcg((const unsigned short*)X + at) : (uint32_t)__ldcg((const unsigned char*)X + at);
     }
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) o[i * E / 4] |= (k + i < K ? x[i] : 0u) << (8 * E * i % 32);
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
