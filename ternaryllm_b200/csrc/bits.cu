@@ -88,9 +88,15 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 // barrier and the later start cost 0.2 to 0.5 us, which a warp of a few pairs does not win back.  (16 rows of fp16 on 4096 x 11008 9.7 us, 12.1 apart;
 // one on 8192 x 10240 9.3 and 10.3; 32 rows of int8 on 2048 x 8192 5.8 and 6.8, but 4.2 and 3.8 on 768 x 6912; 16 of fp16 on 2048 x 2048,
 // no split, 3.1 and 2.7.  Two rows of fp16 on odd addresses, 2048 x 16384, 5.5 and 7.8; two columns of fp32 on 4096 x 11008 9.5 and 16.4.)
-bool bits_share(int x_dtype, bool async, const BitsPlan& q, int kp, int rows) {
+// Without a split the warps of rows and columns that start anywhere fetch nothing twice.  Shared, their loads of columns lie beside one another, and all 512 threads
+// take part where K is short.  (Apart and shared, columns: nine of int8 on 1344 x 1152 12.1 and 7.2, seven of fp16 on 1183 x 332 5.5 and 3.7, four of fp32 on
+// 616 x 3880 5.6 and 4.4; odd addresses: 24 rows of int8 on 1615 x 2056 5.8 and 4.9, six of fp16 on 440 x 4480 3.4 and 2.8, seven of fp32 on 216 x 1792
+// 4.9 and 3.5.  Up to four columns of int8 over a short K lose 6 %, two of fp16 3 %, rows of fp32 over a longer K 4 %.)
+bool bits_share(int x_dtype, BitsAccess access, bool async, const BitsPlan& q, int kp, int rows) {
     if (q.passes > 1) return true;
-    if (!async) return q.split_log > 0 || (kp <= 10 && rows >= 8);
+    if (!async && q.split_log > 0) return true;
+    if (access == BITS_COLUMNS) return rows > 4 || kp > 16 || (rows > 2 ? x_dtype != TLLM_I8 : x_dtype == TLLM_F32 && kp <= 10);
+    if (!async) return x_dtype == TLLM_I8 || (x_dtype == TLLM_F32 ? rows > 2 && kp <= 10 : rows > 2 || kp > 10);
     const bool two_bytes = x_dtype == TLLM_F16 || x_dtype == TLLM_BF16;
     if (q.split_log == 2) return q.pairs > 2;
     return q.split_log == 1 && (q.pairs > 4 || (q.pairs == 4 && two_bytes) || (q.pairs > 1 && (q.nb == 3 || (q.nb == 2 && two_bytes))));
@@ -106,7 +112,7 @@ BitsCut bits_cut(int x_dtype, BitsAccess access, int rows, int inners, int colum
     const int e = dtype_bytes(x_dtype), kb = (inners + 63) / 64, kp = (kb + 1) / 2;
     BitsCut q{bits_plan(x_dtype, rows, columns, kb, sms)};
     q.async = access == BITS_ROWS16 && (size_t)inners * e % 16 == 0;
-    q.share = bits_share(x_dtype, q.async, q, kp, rows);
+    q.share = bits_share(x_dtype, access, q.async, q, kp, rows);
     const uint32_t red = (uint32_t)(BT_WARPS >> q.split_log) * q.per_pass * (x_dtype == TLLM_F32 ? 3 * rows : rows) * 80;
     q.x_pitch = (uint32_t)kp * 128 * e + (e == 1 ? 64 : e == 2 ? 16 : 32);
     const auto all_x = [&] { return q.share ? ((size_t)rows * q.x_pitch + 127) / 128 * 128 : 0; };

@@ -122,6 +122,26 @@ def test_shared_activations_as_they_fit(dtype, M, K, N):
     pw.close()
 
 
+# Columns, and rows on odd addresses, that the warps share although no split fetches them twice: a K of one pair of slices to a warp, of fewer and of more of them,
+# in one chunk and in two
+@pytest.mark.parametrize("dtype,M,K,N,columns,chunks", [("i8", 9, 1344, 1152, True, 1), ("i8", 5, 900, 811, True, 1), ("i8", 2, 2188, 640, True, 1), ("bf16", 5, 1728, 2304, True, 1), ("f16", 3, 896, 811, True, 1),
+                                                        ("f16", 4, 2376, 1043, True, 2), ("f32", 3, 720, 1024, True, 1), ("f32", 2, 1192, 384, True, 1), ("i8", 24, 1827, 1280, False, 1), ("i8", 1, 4104, 333, False, 1),
+                                                        ("f16", 7, 2376, 2048, False, 2), ("bf16", 5, 768, 4864, False, 1), ("f16", 2, 1480, 640, False, 1), ("f32", 4, 516, 320, False, 1)])
+def test_shared_without_a_split(dtype, M, K, N, columns, chunks):
+    gen = torch.Generator().manual_seed(K)
+    w = torch.randint(-1, 2, (K, N), dtype=torch.int8, generator=gen)
+    pw = PackedWeight.from_dense(w.numpy())
+    X = torch.randint(-127, 128, (M, K), generator=gen).to(DT[dtype]).cuda()
+    buf = torch.zeros(M * K + 1, dtype=DT[dtype], device="cuda")
+    buf[1:] = X.reshape(-1)
+    x = X.t().contiguous() if columns else buf[1:].view(M, K)
+    out = torch.full((M, N), -1, dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+    assert torch.equal(decoded(pw.matmul, x, out=out, col_major=columns).double(), X.double() @ w.cuda().double())
+    assert bits_plan()[2:5] == (1, 1, chunks)
+    pw.check()
+    pw.close()
+
+
 # Results added up a column per thread and four per thread, stored together and one by one: around thirty-two (group, row) pairs per block, N a multiple of four and
 # not, Y on 16 bytes and not, sums that are not finite among the four
 @pytest.mark.parametrize("dtype", list(DT))
