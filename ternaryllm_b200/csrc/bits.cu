@@ -63,7 +63,7 @@ int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device,
 }  // namespace
 
 // How a product is cut.  One pass over the widest block's columns if GR = 3 (two for more than eight columns of B) and a split of up to four allow it; the
-// narrowest split that does, because every part of a split reads the activations anew.
+// narrowest split that does: every part of a split fetches the activations anew, or reads the shared ones again, and adds up fewer warps' sums.
 namespace {
 int dtype_bytes(int x_dtype) { return x_dtype == TLLM_F32 ? 4 : x_dtype == TLLM_I8 ? 1 : 2; }
 struct BitsPlan {
@@ -133,40 +133,31 @@ BitsCut bits_cut(int x_dtype, BitsAccess access, int rows, int inners, int colum
 }
 }  // namespace
 
-// Microseconds of a launch: its start, more of it the more of the sixteen warps have work; per pair of slices that a warp goes through what it takes
-// sixteen warps to fetch and turn the activations and to decode and multiply the columns, more of it where the activations are fetched once a
-// pass; and the results.  Fitted to 5000 launches on 100 weights from 256 x 256 to 8192 x 10240, 1 to 64 rows: 4 to 7 % off in the mean.  A column-major
-// X is read element by element, by all blocks from the same lines (16 rows of fp16, 4096 x 11008: 227 us; the batched kernel behind its planes
-// 18.5), less where a short K leaves warps without work; what that takes depends on the addresses more than on anything here: 20 % off.
-double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
+// Microseconds of a launch as bits_cut makes it: its start, more of it the more of the sixteen warps have work; per pair of slices that a warp goes through a step
+// of its own and what every block of columns of B and group of columns adds; the results; and the activations, of every pair again or, shared,
+// of all of K once.  Fitted to 18000 products of 1 to 100 rows on 281 weights from 256 x 256 to 28672 x 8192 in graphs: 7 to 11 % off for rows; up to four
+// columns and more of them apart, 8 to 22 %, since the addresses decide there.
+double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int inners, int columns, int sms) {
     struct Cost {
-        double start, warps, step, nb, nb_gr, fetch, row, few, results;     // few: share of fetch and row where blocks are few, at least
+        double start, warps, step, groups, results, fetch, fetch_row;       // fetch and fetch_row, not shared: a row of a pair, less of it where blocks are few, and in any case
     };
-    static const Cost costs[3][3] = {       // fp32, 16 bits, int8; rows on 16 bytes, rows, columns
-        {{0.8, 1.5, 0.95, 0.08, 0.18, 0, 0, 0, 0}, {0.75, 1.6, 0.5, 0.2, 0.11, 0.42, 0.325, 0.74, 0.14}, {0.5, 1.8, 0, 0, 0.2, 0, 1.4, 0.5, 1.08}},
-        {{1.2, 0.6, 0.53, 0, 0.18, 0, 0, 0, 0.075}, {1.2, 0.75, 0.26, 0, 0.13, 0.56, 0.147, 0.73, 0.18}, {0.5, 0.4, 0.7, 0.14, 0.19, 4.3, 0.46, 0.34, 0.82}},
-        {{1.3, 0.4, 0.44, 0, 0.1, 0, 0, 0, 0.053}, {1.2, 0.9, 0.06, 0.11, 0.07, 0.7, 0.062, 0.68, 0.19}, {0.5, 0, 0, 1.5, 0, 5.1, 0.1, 0.14, 1.2}}};
-    static const double int8_four[3] = {1.02, 0.8, 7.5}, few_rows[3][2] = {{0.75, 1.0}, {0.25, 0.54}, {0.45, 0.48}};     // a step of four blocks of columns of B; columns, up to two and four rows
-    if (access == BITS_COLUMNS && rows == 1) access = BITS_ROWS;             // the same addresses
-    const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
-    const int type = x_dtype == TLLM_F32 ? 0 : x_dtype == TLLM_I8 ? 2 : 1, kp = (kb + 1) / 2;
-    const Cost& c = costs[type][access];
-    const double groups = (columns + 15) / 16;
-    double step = type == 2 && q.nb == 4 ? int8_four[access] : c.step + q.nb * (c.nb + c.nb_gr * q.gr);
-    if (type == 0 && access == BITS_ROWS16 && q.nb == 3) step += 0.23;
-    double fetch = (c.fetch + c.row * rows) * std::min(1.0, c.few + groups / (access == BITS_COLUMNS ? 128 : 256));
-    if (access == BITS_COLUMNS) fetch *= std::min(1.0, 0.3 + 0.0875 * kp) * (rows <= 2 ? few_rows[type][0] : rows <= 4 ? few_rows[type][1] : 1.0);
-    const double each = (double)kp / (BT_WARPS >> q.split_log);             // pairs of a warp and pass, in the mean
+    static const Cost costs[2][3][4] = {     // warps apart, sharing X; fp32, 16 bits, int8; rows on 16 bytes, rows, more than four columns, up to four
+        {{{0.977, 0.904, 1.05, 0.145, 0, 0, 0}, {1.18, 0.781, 0.947, 0.238, 0.22, 0.0149, 0.242}, {0, 0, 0, 0.091, 5.77, 0, 1.7}, {0, 1.65, 0, 0.11, 1.25, 0.137, 1.01}},
+         {{1.02, 0.499, 0.565, 0.189, 0.0258, 0, 0}, {0.706, 1.02, 0.953, 0.141, 0.227, 0.0336, 0.13}, {0, 0, 0, 1.08, 3.86, 0, 0.693}, {0.0118, 0.88, 1.69, 0.0865, 0.374, 0.235, 0.0594}},
+         {{1.24, 0.431, 0.179, 0.191, 0.0162, 0, 0}, {0, 2.76, 0.725, 0.137, 0.275, 0.0184, 0.0558}, {0, 0, 0.527, 1.09, 2.7, 0.0458, 0.225}, {0, 2.87, 1.34, 0.0302, 0, 0.608, 0}}},
+        {{{0, 1.1, 1.56, 0, 0.155, 0, 0.00279}, {1.45, 0.457, 0.946, 0.0593, 0.109, 0.0652, 0.0205}, {1.88, 0.783, 0.715, 0.113, 0.0789, 0.162, 0}, {2.09, 0.0933, 0.311, 0.311, 0.203, 0.0455, 0.0179}},
+         {{0, 1.54, 0.655, 0.0522, 0.0795, 0.021, 0}, {1.53, 0.266, 0.496, 0.127, 0.0427, 0.0157, 0.0107}, {1.94, 1.57, 0, 0.294, 0, 0.144, 0}, {2.53, 0, 0.156, 0.297, 0.23, 0.0298, 0.0127}},
+         {{2.05, 0.0528, 0.516, 0.0124, 0.0579, 0.00903, 0}, {1.65, 0.145, 0.309, 0.0754, 0.042, 0.0128, 0.00552}, {2.67, 1.06, 0, 0.239, 0, 0.166, 0}, {3.88, 0, 0, 0.337, 0.0102, 0.0042, 0.0139}}}};
+    const BitsCut q = bits_cut(x_dtype, access, rows, inners, columns, sms);
+    const int type = x_dtype == TLLM_F32 ? 0 : x_dtype == TLLM_I8 ? 2 : 1, how = access == BITS_COLUMNS ? (rows > 4 ? 2 : 3) : q.async ? 0 : 1;
+    const Cost& c = costs[q.share][type][how];
+    const double groups = (columns + 15) / 16, kp = ((inners + 63) / 64 + 1) / 2, each = kp / (BT_WARPS >> q.split_log);      // each: pairs of a warp and pass, in the mean
     const double pairs = q.passes > 1 ? (q.pairs + q.passes * each) / 2 : q.pairs;        // a warp that has one less goes on with the next pass
-    return c.start + c.warps * std::min(1.0, each) + pairs * (step + fetch) + c.results * groups * rows / 1000;
-}
-
-// What a launch takes of that estimate where the warps share X (columns cut two and four ways; three blocks of fp32 columns of B are cut once): over
-// 4800 drawn products of 1 to 100 rows.
-double bits_shared_part(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms) {
-    static const double part[3][2] = {{0.96, 0.86}, {0.86, 0.72}, {0.6, 0.45}};
-    const BitsPlan q = bits_plan(x_dtype, rows, columns, kb, sms);
-    return (q.split_log ? part[access][q.split_log - 1] : 1.0) * (x_dtype == TLLM_F32 && q.nb == 3 ? 0.93 : 1.0);
+    const double fetch = q.share ? kp * (c.fetch + c.fetch_row * rows) : pairs * rows * (c.fetch * std::min(1.0, groups / (access == BITS_COLUMNS ? 128 : 256)) + c.fetch_row);
+    // What columns take depends on the addresses (five of fp16 on 512 x 2568 9.7 us, four 5.6 before the warps shared them), so that they are priced above the mean, most
+    // where every block reads all of X: of 6400 calls 60 became slower by more than 5 % with these prices in the place of the ones before, 202 without.
+    const double doubt = access != BITS_COLUMNS ? 1.0 : rows <= 4 || columns < 1280 || q.split_log == 2 ? 1.1 : q.split_log == 1 ? 1.3 : 1.5;
+    return doubt * (c.start + c.warps * std::min(1.0, each) + pairs * (c.step + c.groups * q.nb * q.gr) + c.results * groups * rows / 1000 + fetch);
 }
 
 thread_local int bits_last_plan[6];

@@ -666,7 +666,6 @@ inline BitsAccess bits_access(const void* X, int x_dtype, int x_layout, int x_ld
     return (uintptr_t)X % 16 == 0 && (size_t)x_ld * e % 16 == 0 ? BITS_ROWS16 : BITS_ROWS;
 }
 // its time, for the choice between kernels
-double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms);
-double bits_shared_part(int x_dtype, BitsAccess access, int rows, int columns, int kb, int sms);
+double bits_estimate_us(int x_dtype, BitsAccess access, int rows, int inners, int columns, int sms);
 
 }  // namespace tllm

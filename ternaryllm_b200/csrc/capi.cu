@@ -878,25 +878,24 @@ int run_bits(const BitsView& w, const void* X, int x_dtype, int x_layout, int x_
 // Cost models of the two kernels that read the two-bit tiles, microseconds.
 double bt_model_us(int inners, int columns, int sms, int x_dtype, BitsAccess access, int rows) {
     const int per = bt_rows_per_launch(x_dtype);
-    double t = 0;
-    for (int r0 = 0; r0 < rows; r0 += per) t += bits_estimate_us(x_dtype, access, std::min(rows - r0, per), columns, (inners + 63) / 64, sms);
-    return t;
+    const auto us = [&](int m) { return bits_estimate_us(x_dtype, access, m, inners, columns, sms); };
+    return (rows >= per ? rows / per * us(per) : 0.0) + (rows % per ? us(rows % per) : 0.0);
 }
 double mm_tiles_model_us(int inners, int columns, int sms, int device, bool direct, int x_dtype, BitsAccess access, int rows) {
     const int planes = x_dtype == TLLM_F32 ? 3 : 1, per = MM_MAX_M_TILES * mm_max_nt(planes), staged = direct ? MM_READY : access == BITS_COLUMNS ? MM_FROM_COLUMNS : MM_FROM_ROWS;
     double t = access == BITS_COLUMNS ? 0.1 + 1.3 * rows * inners / 1e6 : 0.0;        // columns take longer to turn into planes
     for (int r0 = 0; r0 < rows; r0 += per)
         t += mm_plan(std::min(rows - r0, per), planes, staged, (columns + 127) / 128, (inners + 63) / 64, sms, device).us;
-    return t;
+    // (the plans' figures are from before the batched kernels started earlier; in the mean of 6000 products not far from the decoder's time)
+    return t * (direct ? 0.94 : access == BITS_COLUMNS ? 0.91 : 0.89);
 }
 // which of the two: true = decode in registers
 bool bits_prefer_registers(int inners, int columns, int sms, int device, bool direct, int x_dtype, BitsAccess access, int rows) {
     if (rows == 1 && access == BITS_ROWS16) return true;
     if (rows > 8 * BT_MAX_ROWS) return false;
-    // Both estimates are from before the decoder's warps shared X and the batched kernels started earlier.  (Loss against the faster of the two over 4800 drawn
-    // products: 0.4 to 0.8 % for rows on 16 bytes, as before; rows anywhere 0.8 %, 1.2 without; columns 1.6 %, 3.5.)
-    const double part = bits_shared_part(x_dtype, access, std::min(rows, bt_rows_per_launch(x_dtype)), columns, (inners + 63) / 64, sms);
-    return part * bt_model_us(inners, columns, sms, x_dtype, access, rows) <= (direct ? 0.985 : 0.95) * mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, access, rows);
+    // (Against the fastest kernel over 18000 drawn products, by type, access and 1, 2 to 4, 5 to 16 and more rows: mean loss 0 to 1 % for rows, 0 to 4 % for columns; 0 to 6 and
+    // 0 to 16 % with estimates that counted on shared activations whether or not a launch shares them, and on those of the kernels before.)
+    return bt_model_us(inners, columns, sms, x_dtype, access, rows) <= mm_tiles_model_us(inners, columns, sms, device, direct, x_dtype, access, rows);
 }
 
 enum KernelChoice { KERNEL_GATHER, KERNEL_MMA, KERNEL_NIBBLE, KERNEL_BITS };
@@ -910,28 +909,30 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
     if (w->d_bits && mm_min_rows() == -1 && (x_dtype != TLLM_I8 || w->lay.inners <= 131072) && tensor_map_encoder() != nullptr) {
         const int inners = w->lay.inners, columns = w->lay.columns, sms = w->mm_grid;
         const BitsAccess access = bits_access(X, x_dtype, x_layout, x_ld);
-        const double bits = bt_model_us(inners, columns, sms, x_dtype, BITS_ROWS16, rows), gather = gather_model_us(w->lay.nnz, rows);
+        const double bits = bt_model_us(inners, columns, sms, x_dtype, access, rows), gather = gather_model_us(w->lay.nnz, rows);
         const int per = nb_rows_per_launch(x_dtype);
         const bool nibbles = nb_fits(w, x_dtype, x_layout) && rows <= 8 && (rows <= per || access == BITS_ROWS16);
         const double nibble = nibbles ? nibble_model_us(entries, rows, per) : 1e9;
-        // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (8192 x 28672, 90 % zeros, fp16: 22 us against 30;
-        // 4096 x 11008, fp32: 6.1 against 8.7).
-        // The gather model is a fifth low there, two fifths where rows start anywhere, and twice too low where there are few columns.
-        if (rows == 1 && columns >= 4096 && 1.45 * gather < std::min(bits, nibble)) return KERNEL_GATHER;
-        // Two rows of int8 too, which the gather kernel reads in either layout (column-major, 2048 x 8192, 70 % zeros: 6.6 us; decoded in
-        // registers 11.9; and 8192 x 28672, 90 % zeros: 22 against 35 by rows).  Its sums are exact as well.
-        if (x_dtype == TLLM_I8 && rows <= 2 && columns >= 4096 &&
-            1.35 * gather < std::min(bt_model_us(inners, columns, sms, x_dtype, access, rows), mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, access, rows)))
+        const auto tiles = [&] { return mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, access, rows); };
+        // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (13456 x 9088, 90 % zeros, fp32: 13.1 us against 19.0; 4096 x 11008,
+        // 95 % zeros, fp16 5.0 against 6.1).  The gather model is 0.2 too low up to K = 4096, 0.5 to 0.9 (and thrice 1.2) beyond, 0.6 and more for rows on odd addresses.
+        // Two rows of int8 too, which the gather kernel reads in either layout, with sums that are exact as well (column-major, 21504 x 5828, 90 % zeros:
+        // 16.6 us against 25.8); two columns over a short K as before the decoder's warps shared them (2048 x 8192, 70 % zeros: 6.0 us, 4.3 decoded).
+        const bool short_k = inners <= 4096;
+        if (columns >= 4096 && rows == 1 && (short_k && access == BITS_ROWS16 ? 1.3 : 1.85) * gather < std::min(bits, nibble)) return KERNEL_GATHER;
+        if (columns >= 4096 && rows == 2 && x_dtype == TLLM_I8 &&
+            (short_k && access == BITS_COLUMNS && w->lay.nnz * 3 < entries ? 0.97 : 1.6) * gather < std::min(bits, tiles()))
             return KERNEL_GATHER;
         // A weight so wide that a block of the register decoder makes several passes: four bits an entry, which no thread touches, are read
-        // faster (8192 x 28672, one row of bf16: 27.0 us against 32.0; eight rows 32.2 against 36.4; one or two rows of fp32 28.4 and 32.7
-        // against 47 and 49, with the same error).  The model is 8 % high there.  More than one launch's rows (4, fp32 2) have to start on 16
+        // faster (10056 x 15232, one row of fp32 21.2 us against 24.5; two on 22720 x 7680 25.7 against 30.8).  The model is 8 % high for 16 bits and 10 to 20 % low for fp32 and for
+        // rows on odd addresses.  More than one launch's rows (4, fp32 2) have to start on 16
         // bytes: its planes are made from X element by element else (28672 x 8192, eight rows: 82 us, the batched kernel 43).  Of fp32 these
-        // compete with the batched kernel (four rows 34 us against 46, eight 40), over a K that is not too long: 28672 x 8192 57 against 46.
+        // compete with the batched kernel (three rows on 5120 x 23512 20.1 us against 24.9, on 2240 x 23936 12.8 against 18.6), over a K that is not too
+        // long: 28672 x 8192 57 against 46.
         if (nibbles) {
             if (x_dtype == TLLM_F32 && rows > per) {
-                if (inners <= 16384 && nibble < std::min(bits, mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, access, rows))) return KERNEL_NIBBLE;
-            } else if ((nb || x_dtype == TLLM_F32) && 0.92 * nibble < bits) return KERNEL_NIBBLE;
+                if (inners <= 16384 && 0.95 * nibble < std::min(bits, tiles())) return KERNEL_NIBBLE;
+            } else if ((nb || x_dtype == TLLM_F32) && (x_dtype == TLLM_F32 || access != BITS_ROWS16 ? 1.2 : 0.92) * nibble < bits) return KERNEL_NIBBLE;
         }
         return bits_prefer_registers(inners, columns, sms, w->device, mm_direct(inners, X, x_dtype, x_layout, x_ld), x_dtype, access, rows) ? KERNEL_BITS : KERNEL_MMA;
     }

@@ -283,3 +283,20 @@ def test_cost_model_by_layout(K, N, s, dtype, calls):
         assert list(n > 0) == [kernel == "bits", kernel == "mma", kernel == "nibble"], (layout, M, kernel, n)
         assert torch.equal(Y.double(), X.double() @ Wd)
     pw.close()
+
+
+# The price of the register decoder is that of the form it is launched in: shared activations that do not fit are not counted on
+@pytest.mark.parametrize("M, K, N, dtype, kernel", [(16, 4888, 13696, torch.float16, "mma"), (14, 4888, 13696, torch.float16, "bits"), (16, 5120, 15360, torch.bfloat16, "mma"), (12, 5120, 15360, torch.bfloat16, "bits"),
+                                                    (16, 8192, 10240, torch.bfloat16, "mma"), (8, 8192, 10240, torch.bfloat16, "bits")])
+def test_choice_by_the_form_that_is_launched(M, K, N, dtype, kernel):
+    L = _lib.lib()
+    L.tllm_set_mma_min_rows(-1)
+    gen = torch.Generator().manual_seed(K)
+    w = torch.randint(-1, 2, (K, N), dtype=torch.int8, generator=gen)
+    pw = PackedWeight.from_dense(w.numpy())
+    X = torch.randint(-8, 9, (M, K), generator=gen).to(dtype).to(dev())
+    b0, m0 = L.tllm_bits_launch_count(), L.tllm_mma_launch_count()
+    Y = pw.matmul(X, out=torch.empty((M, N), dtype=torch.float32, device=dev()))
+    assert (L.tllm_bits_launch_count() > b0, L.tllm_mma_launch_count() > m0) == (kernel == "bits", kernel == "mma")
+    assert torch.equal(Y.double(), X.double() @ w.to(dev()).double())
+    pw.close()
