@@ -43,18 +43,23 @@ int launch(const BitsParams& p, int grid, size_t smem, int device, cudaStream_t 
     return TLLM_OK;
 }
 
+// Rows on 16 bytes are shared only where the columns are cut (bits_share), which leaves a warp two groups or more, of four blocks of columns of B one.
 template <int XT, bool ASYNC, bool SHARED>
 int pick(const BitsParams& p, int nb, int gr, int grid, size_t smem, int device, cudaStream_t st) {
-    if (nb == 1 && gr == 1) return launch<XT, 1, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+    if constexpr (!ASYNC || !SHARED) {
+        if (nb == 1 && gr == 1) return launch<XT, 1, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+        if (nb == 2 && gr == 1) return launch<XT, 2, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+        if constexpr (XT == TLLM_F32) {
+            if (nb == 3 && gr == 1) return launch<XT, 3, 1, ASYNC, SHARED>(p, grid, smem, device, st);
+        }
+    }
     if (nb == 1 && gr == 2) return launch<XT, 1, 2, ASYNC, SHARED>(p, grid, smem, device, st);
     if (nb == 1 && gr == 3) return launch<XT, 1, 3, ASYNC, SHARED>(p, grid, smem, device, st);
-    if (nb == 2 && gr == 1) return launch<XT, 2, 1, ASYNC, SHARED>(p, grid, smem, device, st);
     if (nb == 2 && gr == 2) return launch<XT, 2, 2, ASYNC, SHARED>(p, grid, smem, device, st);
     if constexpr (XT == TLLM_I8) {
         if (nb == 4 && gr == 1) return launch<XT, 4, 1, ASYNC, SHARED>(p, grid, smem, device, st);
     }
     if constexpr (XT == TLLM_F32) {
-        if (nb == 3 && gr == 1) return launch<XT, 3, 1, ASYNC, SHARED>(p, grid, smem, device, st);
         if (nb == 3 && gr == 2) return launch<XT, 3, 2, ASYNC, SHARED>(p, grid, smem, device, st);
     }
     return fail(TLLM_ERR_ARG, "bits_launch: no kernel for %d x %d", nb, gr);
