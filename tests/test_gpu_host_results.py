@@ -1,5 +1,7 @@
 """matmul_host: both layouts, every kernel that can serve the call.  Exact on integers; results that are still held must not be
 overwritten by later calls, and are ordinary numpy arrays of their own memory."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -117,3 +119,30 @@ def test_staged_buffers(M, K, N, threads):
     finally:
         torch.set_num_threads(before)
         pw.close()
+
+
+# Pieces of a result in the order of their bytes, more of them than it has blocks of 4096 bytes too; a refused call reports none
+def test_results_in_pieces():
+    L = _lib.lib()
+    rng = np.random.default_rng(3)
+    K, N = 128, 520
+    w = random_ternary(rng, K, N, 0.5)
+    pw = PackedWeight.from_dense(w)
+    seen = []
+    ready = C.CFUNCTYPE(None, C.c_void_p, C.c_size_t, C.c_size_t)(lambda arg, begin, end: seen.append((begin, end)))
+    for M in (1, 9, 64):
+        x = rng.integers(-3, 4, size=(M, K)).astype(np.float32)
+        y = np.full((M, N), -1, np.float32)
+
+        def call(parts, rows=M, y_type=_lib.F32, function=ready):
+            seen.clear()
+            return L.tllm_spmm_host_parts(pw._h, x.ctypes.data, _lib.F32, _lib.ROW_MAJOR, rows, y.ctypes.data, y_type, _lib.ROW_MAJOR, parts, C.cast(function, C.c_void_p), None)
+
+        for parts in (1, 3, 8):
+            y[:] = -1
+            assert call(parts) == 0 and len(seen) == parts
+            assert [b for b, _ in seen] == [0] + [e for _, e in seen[:-1]] and seen[-1][1] == y.nbytes
+            assert np.array_equal(y, oracle.dense_f64(x.astype(np.float64), w))
+        assert call(0) != 0 and call(9) != 0 and call(2, rows=0) != 0 and call(2, y_type=77) != 0 and not seen
+        assert call(2, function=None) != 0
+    pw.close()
