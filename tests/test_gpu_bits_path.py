@@ -142,6 +142,79 @@ def test_shared_without_a_split(dtype, M, K, N, columns, chunks):
     pw.close()
 
 
+# The forms of shared activations, each by the plan of its launch: columns cut two and four ways, one pass and more of them, X in one chunk and in two; rows on 16
+# bytes, on odd addresses and columns
+@pytest.mark.parametrize("access,dtype,M,K,groups,split,passes,chunks", [
+    ("rows", "f16", 8, 4096, 5, 2, 1, 2), ("rows", "bf16", 8, 4232, 7, 4, 1, 2), ("rows", "bf16", 16, 2048, 5, 4, 1, 1), ("rows", "f16", 8, 4096, 13, 4, 2, 2), ("rows", "f32", 6, 2048, 5, 4, 1, 1),
+    ("rows", "f32", 7, 2180, 5, 4, 1, 2), ("rows", "f32", 8, 1160, 3, 2, 1, 1), ("rows", "f32", 5, 520, 13, 4, 2, 1), ("rows", "i8", 32, 4096, 3, 4, 1, 2), ("rows", "i8", 32, 4096, 5, 4, 2, 2),
+    ("rows", "i8", 17, 1168, 7, 4, 2, 1), ("rows", "i8", 9, 2192, 13, 4, 2, 2), ("rows", "f16", 1, 4104, 5, 2, 1, 1),
+    ("offset", "f16", 8, 4096, 5, 2, 1, 2), ("offset", "f16", 8, 1000, 7, 4, 1, 1), ("offset", "f16", 4, 1003, 13, 4, 2, 1), ("offset", "bf16", 12, 1000, 5, 4, 1, 1), ("offset", "f32", 4, 1016, 3, 2, 1, 1),
+    ("offset", "f32", 5, 520, 7, 4, 1, 1), ("offset", "i8", 8, 4100, 13, 4, 2, 2), ("offset", "i8", 17, 1168, 5, 4, 2, 1), ("offset", "i8", 16, 1040, 13, 4, 2, 1),
+    ("columns", "f16", 4, 1003, 5, 2, 1, 1), ("columns", "f16", 8, 1000, 13, 4, 2, 1), ("columns", "bf16", 12, 1000, 7, 4, 1, 1), ("columns", "f16", 8, 4096, 13, 4, 2, 2), ("columns", "f32", 5, 520, 5, 4, 1, 1),
+    ("columns", "f32", 4, 1016, 7, 4, 1, 1), ("columns", "f32", 2, 4100, 5, 2, 1, 2), ("columns", "i8", 8, 4100, 13, 4, 2, 2)])
+def test_forms_of_shared_activations(access, dtype, M, K, groups, split, passes, chunks):
+    gen = torch.Generator().manual_seed(K + groups)
+    N = 16 * groups * torch.cuda.get_device_properties(0).multi_processor_count - 5
+    w = torch.randint(-1, 2, (K, N), dtype=torch.int8, generator=gen)
+    pw = PackedWeight.from_dense(w.numpy())
+    top = 127 if dtype in ("i8", "bf16") else 512
+    X = torch.randint(-top, top + 1, (M, K), generator=gen).to(DT[dtype]).cuda()
+    buf = torch.zeros(M * K + 1, dtype=DT[dtype], device="cuda")
+    buf[1:] = X.reshape(-1)
+    x = {"rows": X, "offset": buf[1:].view(M, K), "columns": X.t().contiguous()}[access]
+    want = X.double() @ w.cuda().double()
+    out = torch.empty((M, N), dtype=torch.int32 if dtype == "i8" else torch.float32, device="cuda")
+    for _ in range(2):
+        out.fill_(-1)
+        assert torch.equal(decoded(pw.matmul, x, out=out, col_major=access == "columns").double(), want)
+        assert bits_plan()[2:5] == (split, passes, chunks)
+    pw.check()
+    pw.close()
+
+
+# Four columns per thread with results of 16 bits, stored together and one by one, one of the four not finite and none
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("M,groups", [(8, 5), (16, 3)])
+def test_sums_of_the_warps_in_16_bits(dtype, M, groups):
+    K, sms = 120, torch.cuda.get_device_properties(0).multi_processor_count      # sums of up to 120 are exact in both types
+    gen = torch.Generator().manual_seed(M)
+    for n in (16 * groups * sms, 16 * groups * sms - 4, 16 * groups * sms - 6):
+        w = torch.randint(-1, 2, (K, n), dtype=torch.int8, generator=gen)
+        w[0] = 0
+        w[0, 5], w[0, n - 1] = 1, -1
+        pw = PackedWeight.from_dense(w.numpy())
+        X = torch.randint(-1, 2, (M, K), generator=gen).to(DT[dtype]).cuda()
+        want = X.double() @ w.cuda().double()
+        out = torch.full((M * n + 1,), -1, dtype=DT[dtype], device="cuda")
+        for y in (out[:-1].view(M, n), out[1:].view(M, n)):
+            assert torch.equal(decoded(pw.matmul, X, out=y).double(), want)
+        X[M - 1, 0] = float("inf")
+        want[M - 1, 5], want[M - 1, n - 1] = float("inf"), -float("inf")
+        for y in (out[:-1].view(M, n), out[1:].view(M, n)):
+            y.fill_(-1)
+            assert torch.equal(decoded(pw.matmul, X, out=y).double(), want)
+        pw.close()
+
+
+# Gate and up columns that four-column threads add up: more than thirty-two (group, row) pairs a block
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("M", [6, 8])
+def test_wide_fused_mlp(dtype, M):
+    rng = np.random.default_rng(M)
+    hidden, inter = 264, 40 * torch.cuda.get_device_properties(0).multi_processor_count + 2
+    wg, wu, wd = (random_ternary(rng, *shape, 0.6) for shape in ((hidden, inter), (hidden, inter), (inter, hidden)))
+    mlp = PackedMLP(wg, wu, wd, 0.021, 0.034, 0.027)
+    X = torch.tensor(rng.standard_normal((M, hidden)), dtype=DT[dtype], device="cuda")
+    ref = oracle.mlp_f64(X.double().cpu().numpy(), wg, wu, wd, 0.021, 0.034, 0.027, h_round={"f32": 3, "f16": 1, "bf16": 2}[dtype])
+    L = _lib.lib()
+    b0 = L.tllm_bits_launch_count()
+    got = mlp.forward(X)
+    assert L.tllm_bits_launch_count() > b0
+    err = np.max(np.abs(got.double().cpu().numpy() - ref)) / np.max(np.abs(ref))
+    assert err <= 1e-5 + {"f32": 2.0 ** -22, "f16": 2.0 ** -10, "bf16": 2.0 ** -7}[dtype], err          # as in test_fused_mlp
+    mlp.close()
+
+
 # Results added up a column per thread and four per thread, stored together and one by one: around thirty-two (group, row) pairs per block, N a multiple of four and
 # not, Y on 16 bytes and not, sums that are not finite among the four
 @pytest.mark.parametrize("dtype", list(DT))
