@@ -915,24 +915,28 @@ KernelChoice choose_kernel(const tllm_weight* w, const void* X, int x_dtype, int
         const double nibble = nibbles ? nibble_model_us(entries, rows, per) : 1e9;
         const auto tiles = [&] { return mm_tiles_model_us(inners, columns, sms, w->device, false, x_dtype, access, rows); };
         // One row of a large, very sparse weight: the index lists are shorter than two bits an entry (13456 x 9088, 90 % zeros, fp32: 13.1 us against 19.0; 4096 x 11008,
-        // 95 % zeros, fp16 5.0 against 6.1).  The gather model is 0.2 too low up to K = 4096, 0.5 to 0.9 (and thrice 1.2) beyond, 0.6 and more for rows on odd addresses.
+        // 95 % zeros, fp16 5.0 against 6.1; 8192 x 57344, 90 % zeros, bf16 34.5 against 44.7).  The gather model is 0.2 too low up to K = 4096, beyond that 0.4 to 0.6 for
+        // the largest weights and 0.5 to 0.9 (thrice more) for others, and 0.6 or more for rows on odd addresses.
         // Two rows of int8 too, which the gather kernel reads in either layout, with sums that are exact as well (column-major, 21504 x 5828, 90 % zeros:
         // 16.6 us against 25.8); two columns over a short K as before the decoder's warps shared them (2048 x 8192, 70 % zeros: 6.0 us, 4.3 decoded).
         const bool short_k = inners <= 4096;
-        if (columns >= 4096 && rows == 1 && (short_k && access == BITS_ROWS16 ? 1.3 : 1.85) * gather < std::min(bits, nibble)) return KERNEL_GATHER;
+        const double gather_times = short_k && access == BITS_ROWS16 ? 1.3 : entries > 150000000 ? 1.6 : 1.85;
+        if (columns >= 4096 && rows == 1 && gather_times * gather < std::min(bits, nibble)) return KERNEL_GATHER;
         if (columns >= 4096 && rows == 2 && x_dtype == TLLM_I8 &&
             (short_k && access == BITS_COLUMNS && w->lay.nnz * 3 < entries ? 0.97 : 1.6) * gather < std::min(bits, tiles()))
             return KERNEL_GATHER;
-        // A weight so wide that a block of the register decoder makes several passes: four bits an entry, which no thread touches, are read
-        // faster (10056 x 15232, one row of fp32 21.2 us against 24.5; two on 22720 x 7680 25.7 against 30.8).  The model is 8 % high for 16 bits and 10 to 20 % low for fp32 and for
-        // rows on odd addresses.  More than one launch's rows (4, fp32 2) have to start on 16
-        // bytes: its planes are made from X element by element else (28672 x 8192, eight rows: 82 us, the batched kernel 43).  Of fp32 these
-        // compete with the batched kernel (three rows on 5120 x 23512 20.1 us against 24.9, on 2240 x 23936 12.8 against 18.6), over a K that is not too
-        // long: 28672 x 8192 57 against 46.
+        // Four bits an entry, which no thread touches.  16 bits: where a block of the register decoder makes several passes (more than twelve groups of sixteen columns to an SM)
+        // the two are level (8192 x 28672, one row of bf16 26.9 us, 26.5 decoded); with more rows, more columns or a longer K the decoder is ahead (eight rows
+        // 32.1 and 27.4; 8192 x 57344, one row 46.4 and 44.8; 28672 x 8192 31.1 and 24.2).  fp32: faster than the three pieces in registers (8192 x 28672, one row
+        // 27.1 and 38.4; 10056 x 15232 21.2 and 24.5).  The model is 10 to 20 % low for fp32 and for rows on odd addresses.  More than one launch's rows (4, fp32 2)
+        // have to start on 16 bytes: its planes are made from X element by element else (28672 x 8192, eight rows: 82 us, the batched kernel 43).  Of fp32
+        // these compete with the batched kernel (three rows on 5120 x 23512 20.1 us against 24.9, on 2240 x 23936 12.8 against 18.6), over a K that is
+        // not too long: 28672 x 8192, four rows 59 against 40.
         if (nibbles) {
             if (x_dtype == TLLM_F32 && rows > per) {
                 if (inners <= 16384 && 0.95 * nibble < std::min(bits, tiles())) return KERNEL_NIBBLE;
-            } else if ((nb || x_dtype == TLLM_F32) && (x_dtype == TLLM_F32 || access != BITS_ROWS16 ? 1.2 : 0.92) * nibble < bits) return KERNEL_NIBBLE;
+            } else if (x_dtype == TLLM_F32 ? 1.2 * nibble < bits : nb && columns > 12 * 16 * sms && (access == BITS_ROWS16 ? 0.92 : 1.2) * nibble < bits)
+                return KERNEL_NIBBLE;
         }
         return bits_prefer_registers(inners, columns, sms, w->device, mm_direct(inners, X, x_dtype, x_layout, x_ld), x_dtype, access, rows) ? KERNEL_BITS : KERNEL_MMA;
     }
