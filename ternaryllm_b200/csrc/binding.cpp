@@ -150,10 +150,16 @@ PyObject* matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // calls that run at the same time need more than two.  (256 columns of fp32, 1024 x 4096, sixteen threads: 214 us, 288 with only the result staged, and
 // in one piece; 2048 x 8192 377 and 504.  Pieces of 1 MB 217 and 383, of 2 MB 236 and 417.)
 constexpr int64_t STAGE_X_FROM = 128 << 10, STAGE_FROM = 256 << 10, STAGE_TO = 16 << 20, STAGE_PART = 512 << 10;
-// straight to the CPU's copy: a dispatch mode of the caller's has no part in it
+// Straight to the CPU's copy: a dispatch mode of the caller's has no part in it.  torch deals out equal numbers of elements, 32768 or more to a thread, so that bytes
+// would start anywhere for five to seven threads: these get elements as wide as leave work for four of them.  (64 rows of fp32, 4096 x 512: 97 us, 119 to 132 in bytes, 128
+// unstaged; 64 on 2048 x 2048 89, 95 to 105, 107.  Twelve threads are better off with bytes.)
 void copy_bytes(char* to, const char* from, int64_t n) {
-    at::Tensor t = at::from_blob(to, {n}, at::kByte);
-    at::redispatch::copy_(c10::DispatchKeySet(c10::DispatchKey::CPU), t, at::from_blob(const_cast<char*>(from), {n}, at::kByte));
+    const int threads = at::get_num_threads();
+    int64_t e = threads > 4 && threads < 8 ? 8 : 1;
+    while (e > 1 && (n / e < 4 * 32768 || ((uintptr_t)to | (uintptr_t)from | (uintptr_t)n) % e != 0)) e /= 2;
+    const at::ScalarType type = e == 8 ? at::kLong : e == 4 ? at::kInt : e == 2 ? at::kShort : at::kByte;
+    at::Tensor t = at::from_blob(to, {n / e}, type);
+    at::redispatch::copy_(c10::DispatchKeySet(c10::DispatchKey::CPU), t, at::from_blob(const_cast<char*>(from), {n / e}, type));
 }
 PyObject* matmul_host(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     NEED_ARGS(9, "matmul_host")

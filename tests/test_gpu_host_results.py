@@ -146,3 +146,24 @@ def test_results_in_pieces():
         assert call(0) != 0 and call(9) != 0 and call(2, rows=0) != 0 and call(2, y_type=77) != 0 and not seen
         assert call(2, function=None) != 0
     pw.close()
+
+
+# Staged copies are dealt out in elements of one to eight bytes: sizes that are multiples of eight and not, above and below the least that is staged
+@pytest.mark.parametrize("threads", [4, 5, 6, 7, 12])
+@pytest.mark.parametrize("dtype", [np.float32, np.float16, np.int8])
+def test_staging_by_threads(dtype, threads):
+    rng = np.random.default_rng(4)
+    before = torch.get_num_threads()
+    torch.set_num_threads(threads)
+    try:
+        for M, K, N in ((64, 4096, 512), (255, 1001, 1037), (511, 515, 2051)):
+            w = random_ternary(rng, K, N, 0.5)
+            pw = PackedWeight.from_dense(w)
+            x = rng.integers(-1, 2, size=(M, K)).astype(dtype)
+            want = x.astype(np.float32) @ w.astype(np.float32)          # exact: sums below 4097
+            y = pw.matmul_host(x)
+            assert np.array_equal(y, want.astype(np.float16) if dtype == np.float16 else want)
+            assert np.array_equal(pw.matmul_host(np.ascontiguousarray(x.T), col_major=True, y_col_major=True), y.T)
+            pw.close()
+    finally:
+        torch.set_num_threads(before)
