@@ -46,11 +46,9 @@ K_IN, N_OUT = 4096, 11008
 L2_BYTES = 126 * 1024 * 1024
 METRIC = "ternary_llama70b_shape_decode_tokens_per_s"
 DEC = dict(hidden=8192, ffn=28672, heads=64, kv_heads=8, head_dim=128, layers=80, kv_len=1024)
-# DRAM bytes per launch of the decode kernel from an ncu capture of the headline product (dram__bytes_read.sum +
-# dram__bytes_write.sum); refreshed whenever the kernel or the format changes
 # DRAM bytes of a launch of the decode product's headline workload, where ncu has counted them, by the kernel that runs it
-NCU_TRAFFIC = {"bits_spmm_kernel": {"bytes": 11.3e6, "source": "ncu (bytes read), profiles/two_bit_kernels_and_attention.md"},
-               "bstream_spmm_kernel<float,1>": {"bytes": 14.03e6, "source": "ncu, profiles/bstream_spmm_decode_4096x11008_s75_m1.md"}}
+NCU_TRAFFIC = {"bits_spmm_kernel": {"bytes": 11.3e6, "source": "ncu, dram__bytes_read.sum"},
+               "bstream_spmm_kernel<float,1>": {"bytes": 14.03e6, "source": "ncu, dram__bytes_read.sum + dram__bytes_write.sum"}}
 
 
 def algorithmic_bytes(nnz: int, K: int, N: int, M: int, e: int) -> int:
