@@ -94,7 +94,7 @@ BitsPlan bits_plan(int x_dtype, int rows, int columns, int kb, int sms) {
 // one on 8192 x 10240 9.3 and 10.3; 32 rows of int8 on 2048 x 8192 5.8 and 6.8, but 4.2 and 3.8 on 768 x 6912; 16 of fp16 on 2048 x 2048,
 // no split, 3.1 and 2.7.  Two rows of fp16 on odd addresses, 2048 x 16384, 5.5 and 7.8; two columns of fp32 on 4096 x 11008 9.5 and 16.4.)
 // Without a split the warps of rows and columns that start anywhere fetch nothing twice.  Shared, their loads of columns lie beside one another, and all 512 threads
-// take part where K is short.  (Apart and shared, columns: nine of int8 on 1344 x 1152 12.1 and 7.2, seven of fp16 on 1183 x 332 5.5 and 3.7, four of fp32 on
+// take part where K is short.  (Apart and shared, columns: nine of int8 on 1344 x 1152 12.1 and 6.5, seven of fp16 on 1183 x 332 5.5 and 3.7, four of fp32 on
 // 616 x 3880 5.6 and 4.4; odd addresses: 24 rows of int8 on 1615 x 2056 5.8 and 4.9, six of fp16 on 440 x 4480 3.4 and 2.8, seven of fp32 on 216 x 1792
 // 4.9 and 3.5.  Up to four columns of int8 over a short K lose 6 %, two of fp16 3 %, rows of fp32 over a longer K 4 %.)
 bool bits_share(int x_dtype, BitsAccess access, bool async, const BitsPlan& q, int kp, int rows) {

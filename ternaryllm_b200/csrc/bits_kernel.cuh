@@ -16,8 +16,9 @@
 //   * W travels by cp.async, several pairs of slices ahead, into slots that belong to one warp: no block barrier in
 //     the main loop, and W is in flight before the preceding kernel has finished (griddepcontrol.wait);
 //   * X travels the same way, each warp its own pairs of slices; or, where several warps would fetch the same ones (the columns cut two or four ways, several
-//     passes), whole, once, for all warps of the block (SHARED; bits_share in bits.cu has the rule and its figures): as much of it as of W went
-//     through L2 four times over (16 rows of fp16 on 2048 x 16384: 64 KB of X a block, fetched four times, for 57 KB of W);
+//     passes) or a warp's loads would lie apart (most calls by columns or on odd addresses), whole, once, for all warps of the block (SHARED; bits_share has the
+//     rule and its figures): as much of it as of W went through L2 four times over (16 rows of fp16 on 2048 x 16384: 64 KB of X a block, fetched four
+//     times, for 57 KB of W);
 //   * sixteen warps (four per scheduler hide the latency of shared-memory load -> decode -> MMA; with two per scheduler the
 //     loop issued 0.49 instructions per clock), one block to an SM (bits_launch);
 //   * the shifts of the decode are multiplications by a value in a register: they run on the FMA pipe beside the ANDs on the
